@@ -1,0 +1,48 @@
+// The launches of the cluster row sampler (a translation unit of its own: it is compiled beside the others).
+#include <cuda_runtime.h>
+
+#include "host.cuh"
+#include "sample_cluster.cuh"
+
+namespace lm {
+
+// Blocks per row of the cluster kernel: as many as keep every SM busy (16 needs an opt-in; a GPU processing cluster holds one such
+// cluster, so 8 rows), slices of at least 2048 logits.
+static int cluster_blocks(int64_t rows, int64_t vocab, int sms) {
+  int c = rows <= 8 ? 16 : rows * 8 <= sms ? 8 : rows * 4 <= sms ? 4 : rows * 2 <= sms ? 2 : 1;
+  while (c > 1 && vocab < 2048LL * c) c >>= 1;
+  return c;
+}
+
+template <bool F32, bool CACHED, int kPerSM>
+static int launch_cluster(const SampleDev& P, int C, size_t smem, int instance, cudaStream_t st) {
+  const void* fn = reinterpret_cast<const void*>(sample_cluster_kernel<F32, CACHED, kClusterBlock, kPerSM>);
+  const int rc = ensure_dynamic_smem(static_cast<KernelSlot>(kSlotCluster + instance), fn, smem, true);
+  if (rc != LM_OK) return rc;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(P.rows) * static_cast<unsigned>(C)); cfg.blockDim = dim3(kClusterBlock); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(C); attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = C > 1 ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, sample_cluster_kernel<F32, CACHED, kClusterBlock, kPerSM>, P, C);
+  return e == cudaSuccess ? LM_OK : cuda_fail(e);
+}
+
+int sample_clusters(const SampleDev& P, int sms, cudaStream_t st) {
+  const int C = cluster_blocks(P.rows, P.vocab, sms);
+  const size_t per = (static_cast<size_t>((P.vocab + 14) / 8) + C - 1) / C;    // chunks of a slice, for any alignment of the row
+  const bool pen = P.history != nullptr && P.hist_len > 0;
+  const size_t head = cluster_smem_head(), marks = pen ? (per + 15) / 16 * 16 : 0;
+  const size_t generic = sizeof(GenericSmem) + (pen ? static_cast<size_t>((P.vocab + 31) / 32) * 4 : 0) + 16;
+  constexpr size_t kMost = 227 * 1024;
+  const bool cached = head + per * 32 + marks <= kMost && C > 1;             // (a block per row reads its row from L2: two of them share an SM)
+  size_t smem = head + (cached ? per * 32 : 0) + marks;
+  if (smem < generic) smem = generic;
+  const bool f32 = P.dtype == LM_DTYPE_F32, two = static_cast<long long>(P.rows) * C > sms && smem <= kMost / 2 - 1024;   // two blocks per SM
+  if (cached) return f32 ? launch_cluster<true, true, 1>(P, C, smem, 0, st) : launch_cluster<false, true, 1>(P, C, smem, 1, st);
+  if (two) return f32 ? launch_cluster<true, false, 2>(P, C, smem, 2, st) : launch_cluster<false, false, 2>(P, C, smem, 3, st);
+  return f32 ? launch_cluster<true, false, 1>(P, C, smem, 4, st) : launch_cluster<false, false, 1>(P, C, smem, 5, st);
+}
+
+}  // namespace lm

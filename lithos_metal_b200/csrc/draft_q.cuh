@@ -54,7 +54,7 @@ struct DraftQDev {
   const uint32_t* state; int t_max, g;                   // optional StepState: seed and step come from it; a done state ends the launch
 };
 
-__global__ void __launch_bounds__(kDraftQBlock, 1) draft_q_kernel(DraftQDev P) {
+static __global__ void __launch_bounds__(kDraftQBlock, 1) draft_q_kernel(DraftQDev P) {
   extern __shared__ __align__(16) float dq_smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, G = gridDim.x, b = blockIdx.x;
   constexpr int kWarps = kDraftQBlock / 32;

@@ -10,7 +10,7 @@
 
 namespace lm {
 
-constexpr int kMaxSweeps = LM_MAX_VOCAB / (kBlock * kChunk) + 1;
+constexpr int kMaxSweeps = LM_MAX_VOCAB / (512 * kChunk) + 1;   // blocks of 512 threads or more
 
 struct DrawSmem {
   uint64_t scratch[32];
@@ -64,17 +64,17 @@ __device__ __forceinline__ uint32_t kept_chunk(const RowView& rv, int c, float t
 // the block, one look at the sweep that holds it). Every thread of the block calls; every thread gets the token (-1 if the kept
 // set has no weight).
 // The kept set's total fixed-point weight. Every thread of the block calls; every thread gets the total.
-__device__ uint64_t kept_weight_total(const RowView& rv, float tau, float vmax, float temperature, DrawSmem& d) {
+static __device__ uint64_t kept_weight_total(const RowView& rv, float tau, float vmax, float temperature, DrawSmem& d) {
   const int tid = threadIdx.x;
   const int n_chunks = (rv.vocab + kChunk - 1) / kChunk;
-  const int n_sweeps = (n_chunks + kBlock - 1) / kBlock;
+  const int n_sweeps = (n_chunks + static_cast<int>(blockDim.x) - 1) / static_cast<int>(blockDim.x);
   const float c2 = exp2_scale(temperature);
   const uint32_t tc = ceil_bf16_code(tau);
   const uint32_t tau2 = tc | (tc << 16);
   uint64_t mine = 0ull;
   for (int it = 0; it < n_sweeps; it++) {
     float z[kChunk];
-    const uint32_t mask = kept_chunk(rv, it * kBlock + tid, tau, tau2, z);
+    const uint32_t mask = kept_chunk(rv, it * static_cast<int>(blockDim.x) + tid, tau, tau2, z);
     if (mask) {
 #pragma unroll
       for (int e = 0; e < kChunk; e++) if ((mask >> e) & 1u) mine += weight_q40(z[e], vmax, c2);
@@ -83,10 +83,10 @@ __device__ uint64_t kept_weight_total(const RowView& rv, float tau, float vmax, 
   return block_sum_u64(mine, d.scratch);
 }
 
-__device__ int draw_inverse_cdf(const RowView& rv, float tau, float vmax, float temperature, float u, DrawSmem& d, uint64_t* out_total = nullptr) {
+static __device__ int draw_inverse_cdf(const RowView& rv, float tau, float vmax, float temperature, float u, DrawSmem& d, uint64_t* out_total = nullptr) {
   const int tid = threadIdx.x;
   const int n_chunks = (rv.vocab + kChunk - 1) / kChunk;
-  const int n_sweeps = (n_chunks + kBlock - 1) / kBlock;
+  const int n_sweeps = (n_chunks + static_cast<int>(blockDim.x) - 1) / static_cast<int>(blockDim.x);
   const float c2 = exp2_scale(temperature);
   const uint32_t tc = ceil_bf16_code(tau);
   const uint32_t tau2 = tc | (tc << 16);
@@ -101,11 +101,11 @@ __device__ int draw_inverse_cdf(const RowView& rv, float tau, float vmax, float 
   for (int level = 0; level < 4; level++) {
     const int shift = 24 - 8 * level;
     const uint32_t hi_mask = level == 0 ? 0u : (0xFFFFFFFFu << (shift + 8));
-    for (int i = tid; i < 256; i += kBlock) d.wbin[i] = 0ull;
+    for (int i = tid; i < 256; i += static_cast<int>(blockDim.x)) d.wbin[i] = 0ull;
     __syncthreads();
     for (int it = 0; it < n_sweeps; it++) {
       float z[kChunk];
-      const uint32_t mask = kept_chunk(rv, it * kBlock + tid, tau, tau2, z);
+      const uint32_t mask = kept_chunk(rv, it * static_cast<int>(blockDim.x) + tid, tau, tau2, z);
       if (!mask) continue;
 #pragma unroll
       for (int e = 0; e < kChunk; e++) if ((mask >> e) & 1u) {
@@ -129,11 +129,11 @@ __device__ int draw_inverse_cdf(const RowView& rv, float tau, float vmax, float 
   const uint64_t each = weight_q40(v, vmax, c2);
   const uint32_t want = each ? static_cast<uint32_t>((target - before) / each) : 0u;   // 0-based rank by index among the logits equal to v
   // ---- how many of them every sweep of the block holds
-  for (int i = tid; i < n_sweeps; i += kBlock) d.sweep_total[i] = 0ull;
+  for (int i = tid; i < n_sweeps; i += static_cast<int>(blockDim.x)) d.sweep_total[i] = 0ull;
   __syncthreads();
   for (int it = 0; it < n_sweeps; it++) {
     float z[kChunk];
-    const uint32_t mask = kept_chunk(rv, it * kBlock + tid, tau, tau2, z);
+    const uint32_t mask = kept_chunk(rv, it * static_cast<int>(blockDim.x) + tid, tau, tau2, z);
     uint32_t n = 0u;
     if (mask) {
 #pragma unroll
@@ -157,7 +157,7 @@ __device__ int draw_inverse_cdf(const RowView& rv, float tau, float vmax, float 
   const int it = d.found_sweep;
   if (it >= 0) {
     const uint32_t local = static_cast<uint32_t>(d.found_base);          // the (local)-th match, in index order, within this sweep
-    const int c = it * kBlock + tid;
+    const int c = it * static_cast<int>(blockDim.x) + tid;
     float z[kChunk];
     const uint32_t mask = kept_chunk(rv, c, tau, tau2, z);
     uint32_t hit = 0u;
@@ -175,7 +175,7 @@ __device__ int draw_inverse_cdf(const RowView& rv, float tau, float vmax, float 
 }
 
 // The Gumbel-max draw; *near_tie is set when another candidate lies within 4e-6 of the winning key.
-__device__ int draw_gumbel(const RowView& rv, float tau, float temperature, uint64_t seed, uint32_t step, uint32_t t_id, DrawSmem& d, bool* near_tie) {
+static __device__ int draw_gumbel(const RowView& rv, float tau, float temperature, uint64_t seed, uint32_t step, uint32_t t_id, DrawSmem& d, bool* near_tie) {
   const int tid = threadIdx.x;
   const int n_chunks = (rv.vocab + kChunk - 1) / kChunk;
   const float inv_t32 = __double2float_rn(1.0 / static_cast<double>(temperature));
@@ -183,7 +183,7 @@ __device__ int draw_gumbel(const RowView& rv, float tau, float temperature, uint
   const uint32_t tau2 = tc | (tc << 16);
   uint64_t b1 = 0ull;
   float second = -INFINITY;
-  for (int c = tid; c < n_chunks; c += kBlock) {
+  for (int c = tid; c < n_chunks; c += static_cast<int>(blockDim.x)) {
     float z[kChunk];
     const uint32_t mask = kept_chunk(rv, c, tau, tau2, z);
     if (!mask) continue;

@@ -1,0 +1,65 @@
+// What the translation units of the library share on the host side: the error text, the device's size, shared-memory grants.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <cstdio>
+#include <mutex>
+
+#include "../../include/lithos_b200.h"
+
+namespace lm {
+
+inline thread_local char g_cuda_error[256] = "";
+
+inline int cuda_fail(cudaError_t e) {
+  std::snprintf(g_cuda_error, sizeof(g_cuda_error), "%s: %s", cudaGetErrorName(e), cudaGetErrorString(e));
+  return LM_E_CUDA;
+}
+
+inline int sm_count(int* out) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return cuda_fail(e);
+  static thread_local int cached_dev = -1, cached = 0;
+  if (cached_dev != dev) {
+    e = cudaDeviceGetAttribute(&cached, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return cuda_fail(e);
+    cached_dev = dev;
+  }
+  *out = cached;
+  return LM_OK;
+}
+
+// Kernels that need more than 48 KB of dynamic shared memory must be told so once per device (the attribute belongs to the
+// device's copy of the function); remembered per device and kernel, raised when a call needs more.
+enum KernelSlot { kSlotFast, kSlotTopk, kSlotGeneric, kSlotVocabLocal, kSlotVerify, kSlotVerifyStats, kSlotDraftQ, kSlotTileFinish, kSlotSlice, kSlotSliceSmall, kSlotSliceTiny, kSlotSlicedMerge, kSlotHead, kSlotCluster,
+                  kSlotCount = kSlotCluster + 6 };   // (the cluster kernel has six instances)
+
+inline int ensure_dynamic_smem(KernelSlot slot, const void* func, size_t bytes, bool large_clusters = false) {
+  if (bytes <= 48 * 1024 && !large_clusters) return LM_OK;
+  constexpr int kMaxDevices = 64;
+  static std::mutex mutex;
+  static size_t granted[kMaxDevices][kSlotCount] = {};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return cuda_fail(e);
+  std::lock_guard<std::mutex> lock(mutex);
+  const bool tracked = dev >= 0 && dev < kMaxDevices;
+  if (tracked && bytes <= granted[dev][slot]) return LM_OK;
+  e = cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+  if (e != cudaSuccess) return cuda_fail(e);
+  if (large_clusters) {                                                     // clusters of up to 16 blocks
+    e = cudaFuncSetAttribute(func, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return cuda_fail(e);
+  }
+  if (tracked) granted[dev][slot] = bytes;
+  return LM_OK;
+}
+
+inline size_t align256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
+
+struct SampleDev;
+// cluster.cu: one row per thread-block cluster, every row of the call.
+int sample_clusters(const SampleDev& P, int sms, cudaStream_t st);
+
+}  // namespace lm

@@ -3,11 +3,11 @@
 #include <cuda_runtime.h>
 
 #include <cmath>
-#include <cstdio>
 #include <cstring>
 #include <mutex>
 
 #include "common.cuh"
+#include "host.cuh"
 #include "sample_generic.cuh"
 #include "sample_hist.cuh"
 #include "sample_topk.cuh"
@@ -78,51 +78,9 @@ __global__ void __launch_bounds__(kBlock, 1) sample_generic_kernel(SampleDev P, 
 // handle for cudaGetSymbolAddress; the kernels get the device address that call returns.
 static __device__ __align__(256) ArgmaxWs g_argmax_static_ws[LM_ARGMAX_STATIC_MAX_ROWS];
 
-thread_local char g_cuda_error[256] = "";
-
-static int cuda_fail(cudaError_t e) {
-  std::snprintf(g_cuda_error, sizeof(g_cuda_error), "%s: %s", cudaGetErrorName(e), cudaGetErrorString(e));
-  return LM_E_CUDA;
-}
-
 constexpr int kOverlapRowsPerSM = 5;    // up to this many rows per SM the two sampler kernels run side by side (lm_sample)
 constexpr int kAloneRowsPerSM = 2;      // ... and up to this many the histogram kernel's blocks have their SM to themselves
 constexpr size_t kAloneSmemBytes = 140 * 1024;   // more than an SM's shared memory less a block of the top-k kernel
-
-static int sm_count(int* out) {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return cuda_fail(e);
-  static thread_local int cached_dev = -1, cached = 0;
-  if (cached_dev != dev) {
-    e = cudaDeviceGetAttribute(&cached, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return cuda_fail(e);
-    cached_dev = dev;
-  }
-  *out = cached;
-  return LM_OK;
-}
-
-// Kernels that need more than 48 KB of dynamic shared memory must be told so once per device (the attribute belongs to the
-// device's copy of the function); remembered per device and kernel, raised when a call needs more.
-enum KernelSlot { kSlotFast, kSlotTopk, kSlotGeneric, kSlotVocabLocal, kSlotVerify, kSlotVerifyStats, kSlotDraftQ, kSlotTileFinish, kSlotSlice, kSlotSliceSmall, kSlotSliceTiny, kSlotSlicedMerge, kSlotHead, kSlotCount };
-
-static int ensure_dynamic_smem(KernelSlot slot, const void* func, size_t bytes) {
-  if (bytes <= 48 * 1024) return LM_OK;
-  constexpr int kMaxDevices = 64;
-  static std::mutex mutex;
-  static size_t granted[kMaxDevices][kSlotCount] = {};
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return cuda_fail(e);
-  std::lock_guard<std::mutex> lock(mutex);
-  const bool tracked = dev >= 0 && dev < kMaxDevices;
-  if (tracked && bytes <= granted[dev][slot]) return LM_OK;
-  e = cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
-  if (e != cudaSuccess) return cuda_fail(e);
-  if (tracked) granted[dev][slot] = bytes;
-  return LM_OK;
-}
 
 static bool sample_has_penalties(const lm_sample_args* a) {
   return a->history != nullptr && a->hist_len > 0 && !(a->repetition_penalty == 1.0f && a->presence_penalty == 0.0f);
@@ -145,7 +103,6 @@ static SampleDev sample_dev(const lm_sample_args* a) {
   return P;
 }
 
-static size_t align256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
 
 }  // namespace lm
 
@@ -351,9 +308,14 @@ int lm_sample(const lm_sample_args* a) {
   }
   const bool fast = a->dtype == LM_DTYPE_BF16 && a->out_stats == nullptr && a->out_probs == nullptr && a->vocab <= kHistMaxVocab &&
                     (a->vocab % kChunk) == 0 && (!pen || a->hist_len <= 65536);
+  const int limit = static_cast<int>((a->flags >> 8) & 0xFFu);
+  if (fast && (!a->workspace || (reinterpret_cast<uintptr_t>(a->workspace) & 255u) || a->workspace_bytes < lm_workspace_bytes(a->rows, a->vocab)))
+    return LM_E_WORKSPACE;
+  // A row per cluster: every row the streaming kernels below do not take (binary32, ragged vocabularies, statistics), and batches too
+  // small to fill the GPU with a block per row. A call that limits its blocks stays below.
+  if (limit == 0 && a->vocab > 0 && (!fast || a->rows * 4 <= sms) && (!pen || a->hist_len <= 65536) && a->rows <= 0x7FFFFFFF / 16)
+    return sample_clusters(P, sms, st);
   if (fast) {
-    if (!a->workspace || (reinterpret_cast<uintptr_t>(a->workspace) & 255u) || a->workspace_bytes < lm_workspace_bytes(a->rows, a->vocab))
-      return LM_E_WORKSPACE;
     const size_t rows_bytes = align256(static_cast<size_t>(a->rows) * sizeof(uint32_t));
     char* ws = static_cast<char*>(a->workspace) + align256(static_cast<size_t>(a->rows) * sizeof(ArgmaxWs));
     int* redo = reinterpret_cast<int*>(ws);                                // rows for the generic kernel
@@ -366,7 +328,6 @@ int lm_sample(const lm_sample_args* a) {
     rc = ensure_dynamic_smem(kSlotFast, reinterpret_cast<const void*>(sample_hist_kernel), hist_smem);
     if (rc == LM_OK) rc = ensure_dynamic_smem(kSlotTopk, reinterpret_cast<const void*>(sample_topk_kernel), sizeof(TopkSmem));
     if (rc != LM_OK) return rc;
-    const int limit = static_cast<int>((a->flags >> 8) & 0xFFu);
     const bool topk = !(a->flags & LM_FLAG_EXACT_ONLY) && a->vocab >= kTopkMinVocab && (a->top_k != nullptr || (a->top_k_s >= 1 && a->top_k_s <= kTopkMaxK)) &&
                       (a->temperature != nullptr || a->temperature_s > 0.0f) && (!pen || a->hist_len <= kTopkHist);
     {

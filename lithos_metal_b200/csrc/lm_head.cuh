@@ -50,7 +50,7 @@ __device__ __forceinline__ uint16_t f32_to_bf16_rn(float f) {                // 
   return static_cast<uint16_t>((u + 0x7FFFu + ((u >> 16) & 1u)) >> 16);
 }
 
-__global__ void __launch_bounds__(kHeadThreads) lm_head_kernel(HeadDev P) {
+static __global__ void __launch_bounds__(kHeadThreads) lm_head_kernel(HeadDev P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint16_t* xs = reinterpret_cast<uint16_t*>(smem_raw);                    // [kHeadRows][H + kHeadPad] BF16, rows beyond P.rows zero
   __shared__ float s_part[kHeadRows][kHeadWarps];

@@ -62,15 +62,15 @@ __device__ __forceinline__ double softmass(float z, float vmax, double inv_t) {
 
 // Histogram pass over the elements whose key matches `prefix` in the bits above this level's digit.
 template <bool MASS>
-__device__ void hist_pass(const RowView& rv, int level, uint32_t prefix, float vmax, double inv_t, GenericSmem& s) {
+static __device__ void hist_pass(const RowView& rv, int level, uint32_t prefix, float vmax, double inv_t, GenericSmem& s) {
   const int tid = threadIdx.x, lane = tid & 31;
-  for (int i = tid; i < kBins; i += kBlock) s.cnt[i] = 0;
-  if (MASS) for (int i = tid; i < kBins * kReplicas; i += kBlock) s.mass[i] = 0.0;
+  for (int i = tid; i < kBins; i += static_cast<int>(blockDim.x)) s.cnt[i] = 0;
+  if (MASS) for (int i = tid; i < kBins * kReplicas; i += static_cast<int>(blockDim.x)) s.mass[i] = 0.0;
   __syncthreads();
   const int shift = 24 - 8 * level;
   const uint32_t hi_mask = level == 0 ? 0u : (0xFFFFFFFFu << (shift + 8));
   const int n_chunks = (rv.vocab + kChunk - 1) / kChunk;
-  for (int c = tid; c < n_chunks; c += kBlock) {
+  for (int c = tid; c < n_chunks; c += static_cast<int>(blockDim.x)) {
     float z[kChunk];
     const int n = load_chunk(rv, c, z);
 #pragma unroll
@@ -91,7 +91,7 @@ __device__ void hist_pass(const RowView& rv, int level, uint32_t prefix, float v
 // from the running totals in s.sel_base_*. Leaves the selected bin in the return value and the running totals
 // strictly above it in s.sel_base_c / s.sel_base_m. `cnt`/`mass` are per-bin arrays of kBins entries.
 template <bool BY_MASS>
-__device__ int select_bin(const uint32_t* cnt, const double* mass, uint32_t k_target, double m_target, GenericSmem& s) {
+static __device__ int select_bin(const uint32_t* cnt, const double* mass, uint32_t k_target, double m_target, GenericSmem& s) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) { s.sel_pos = kBins; s.last_pos = -1; }
   __syncthreads();
@@ -138,7 +138,7 @@ __device__ __forceinline__ void fold_mass(GenericSmem& s) {
 }
 
 // One row, start to finish. All threads of the block call it with the same arguments.
-__device__ void sample_row_generic(const SampleDev& P, int row, GenericSmem& s, uint32_t* pen_bits) {
+static __device__ void sample_row_generic(const SampleDev& P, int row, GenericSmem& s, uint32_t* pen_bits) {
   const int tid = threadIdx.x;
   const int V = P.vocab;
   const float T = P.temperature ? P.temperature[row] : P.temperature_s;
@@ -168,10 +168,10 @@ __device__ void sample_row_generic(const SampleDev& P, int row, GenericSmem& s, 
   // ---- the row's distinct history ids as a bitmap ----------------------------------------------------------
   if (P.history != nullptr && P.hist_len > 0 && !(P.rho == 1.0f && P.pi == 0.0f)) {
     const int words = (V + 31) / 32;
-    for (int i = tid; i < words; i += kBlock) pen_bits[i] = 0u;
+    for (int i = tid; i < words; i += static_cast<int>(blockDim.x)) pen_bits[i] = 0u;
     __syncthreads();
     const int32_t* h = P.history + static_cast<int64_t>(row) * P.hist_stride;
-    for (int i = tid; i < P.hist_len; i += kBlock) {
+    for (int i = tid; i < P.hist_len; i += static_cast<int>(blockDim.x)) {
       const int id = __ldg(h + i);
       if (id >= 0 && id < V) atomicOr(&pen_bits[id >> 5], 1u << (id & 31));
     }
@@ -182,7 +182,7 @@ __device__ void sample_row_generic(const SampleDev& P, int row, GenericSmem& s, 
   // ---- pass A: the maximum and its lowest index --------------------------------------------------------------
   uint64_t best = 0ull;
   bool nan = false;
-  for (int c = tid; c < n_chunks; c += kBlock) {
+  for (int c = tid; c < n_chunks; c += static_cast<int>(blockDim.x)) {
     float z[kChunk];
     const int n = load_chunk(rv, c, z);
 #pragma unroll
@@ -200,7 +200,7 @@ __device__ void sample_row_generic(const SampleDev& P, int row, GenericSmem& s, 
   if (T == 0.0f) {                                                       // greedy
     if (P.out_probs) {
       float* pr = P.out_probs + static_cast<int64_t>(row) * P.probs_stride;
-      for (int i = tid; i < V; i += kBlock) pr[i] = (i == arg) ? 1.0f : 0.0f;
+      for (int i = tid; i < V; i += static_cast<int>(blockDim.x)) pr[i] = (i == arg) ? 1.0f : 0.0f;
     }
     if (tid == 0) {
       P.out_tokens[row] = arg;
@@ -244,7 +244,7 @@ __device__ void sample_row_generic(const SampleDev& P, int row, GenericSmem& s, 
     double total = 0.0;
     if (in_topk) {                                                       // the mass of the top-k set
       double m = 0.0;
-      for (int c = tid; c < n_chunks; c += kBlock) {
+      for (int c = tid; c < n_chunks; c += static_cast<int>(blockDim.x)) {
         float z[kChunk];
         const int n = load_chunk(rv, c, z);
 #pragma unroll
@@ -292,7 +292,7 @@ __device__ void sample_row_generic(const SampleDev& P, int row, GenericSmem& s, 
   double kept_mass = 0.0;
   if (need_mass) {
     double m = 0.0;
-    for (int c = tid; c < n_chunks; c += kBlock) {
+    for (int c = tid; c < n_chunks; c += static_cast<int>(blockDim.x)) {
       float z[kChunk];
       const int n = load_chunk(rv, c, z);
 #pragma unroll
@@ -316,7 +316,7 @@ __device__ void sample_row_generic(const SampleDev& P, int row, GenericSmem& s, 
   // ---- outputs ----------------------------------------------------------------------------------------------------
   if (P.out_probs) {
     float* pr = P.out_probs + static_cast<int64_t>(row) * P.probs_stride;
-    for (int c = tid; c < n_chunks; c += kBlock) {
+    for (int c = tid; c < n_chunks; c += static_cast<int>(blockDim.x)) {
       float z[kChunk];
       const int n = load_chunk(rv, c, z);
       for (int e = 0; e < n; e++) pr[c * kChunk + e] = (z[e] >= tau) ? static_cast<float>(softmass(z[e], vmax, inv_t) / kept_mass) : 0.0f;

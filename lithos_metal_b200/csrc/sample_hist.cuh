@@ -134,7 +134,7 @@ __device__ __forceinline__ uint32_t cnt_of_pos(const HistSmem& s, uint32_t p) {
 __device__ __forceinline__ float penalised_value(uint32_t code, float rho, float pi) { return canon_zero(penalise(hcode_val(code), rho, pi)); }
 
 // One logit that the fast path of the pass does not take: an exact zero, -inf, or a code outside the window.
-__device__ __noinline__ void hist_add_slow(HistSmem& s, uint32_t code) {
+static __device__ __noinline__ void hist_add_slow(HistSmem& s, uint32_t code) {
   const uint32_t slot = slot_of_code(code);
   if (slot != 0xFFFFFFFFu) atomicAdd(&s.hist[slot >> 1], (slot & 1u) ? 0x10000u : 1u);
   else if ((code & 0x7FFFu) == 0u) atomicAdd(&s.cz, 1u);
@@ -200,7 +200,7 @@ __device__ __forceinline__ double b_mass_range(const HistSmem& s, uint32_t j0, u
 // totals (counts, and masses when MASS) are in s.g_cnt / s.g_mass. Every thread calls. Results: s.res_tau, and the running
 // totals s.res_cum_c / s.res_cum_m including every logit equal to res_tau, s.res_excl_m excluding them.
 template <bool BY_MASS, bool MASS>
-__device__ void hist_walk(HistSmem& s, uint32_t k_target, double m_target, float vmax, double inv_t) {
+static __device__ void hist_walk(HistSmem& s, uint32_t k_target, double m_target, float vmax, double inv_t) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // -- level 1: the group. One group per thread, inclusive scan in walk order.
   uint32_t c = 0u, ci = 0u; double m = 0.0, mi = 0.0;
@@ -326,7 +326,7 @@ __device__ __forceinline__ uint32_t equal_mask8(const uint4 q, uint32_t code2, b
 // COUNT them -- segments of 256 logits from whichever end is nearer, a batch of kBatchSegs per barrier, packed 16-bit compares
 // against v's raw code, the penalised logits equal to v as per-segment corrections (s.seg_fix) -- and the warp that holds the
 // segment locates the token. Every thread calls; every thread gets the token (-1: the kept set has no weight).
-__device__ int hist_draw_inverse_cdf(const SampleDev& P, HistSmem& s, const uint32_t* pen, const uint16_t* rowp, int n_chunks, float tau, float vmax, float T, float u,
+static __device__ int hist_draw_inverse_cdf(const SampleDev& P, HistSmem& s, const uint32_t* pen, const uint16_t* rowp, int n_chunks, float tau, float vmax, float T, float u,
                                      uint64_t* out_total, bool total_only = false) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const float c2 = exp2_scale(T);
@@ -522,7 +522,7 @@ __device__ int hist_draw_inverse_cdf(const SampleDev& P, HistSmem& s, const uint
 // The Gumbel-max draw over the kept set (monolith/nn/sampling_ref.py:55-62; kernels/common/sample.metal:164-198): the sweeps
 // skip the penalised positions (bitmap), whose values come from the list afterwards. *near_tie: another key within 4e-6 of the
 // winner's. Every thread calls; every thread gets the token.
-__device__ int hist_draw_gumbel(const SampleDev& P, HistSmem& s, const uint32_t* pen, const uint16_t* rowp, int n_chunks, float tau, float T, uint32_t t_id, bool* near_tie) {
+static __device__ int hist_draw_gumbel(const SampleDev& P, HistSmem& s, const uint32_t* pen, const uint16_t* rowp, int n_chunks, float tau, float T, uint32_t t_id, bool* near_tie) {
   const int tid = threadIdx.x;
   const float inv_t32 = __double2float_rn(1.0 / static_cast<double>(T));
   const uint32_t tc = hceil_code(tau), tau2 = tc | (tc << 16);
@@ -569,7 +569,7 @@ __device__ int hist_draw_gumbel(const SampleDev& P, HistSmem& s, const uint32_t*
 // ---- one row ---------------------------------------------------------------------------------------------------------------------
 // Every thread of the block calls with the same arguments. `pen`: the block's bitmap area. `next`: the row this block takes
 // after this one (-1: none), whose history is pulled into L2 meanwhile. A row the kernel cannot take is appended to `redo`.
-__device__ void sample_row_hist(const SampleDev& P, int row, int next, HistSmem& s, uint32_t* pen, int* redo, int* n_redo) {
+static __device__ void sample_row_hist(const SampleDev& P, int row, int next, HistSmem& s, uint32_t* pen, int* redo, int* n_redo) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int V = P.vocab;
   const float T = P.temperature ? P.temperature[row] : P.temperature_s;
@@ -912,7 +912,7 @@ __device__ void sample_row_hist(const SampleDev& P, int row, int next, HistSmem&
 // stride; a block always holds the item after its current one too, so that it can pull that row's history into L2 while it
 // works. With a row list (written by the top-k kernel: the rows it left) the items are entries of the list, without one they
 // are the rows themselves.
-__global__ void __launch_bounds__(kHB, 2) sample_hist_kernel(SampleDev P, const int* list, const int* n_list, int* next_item, int* redo, int* n_redo) {
+static __global__ void __launch_bounds__(kHB, 2) sample_hist_kernel(SampleDev P, const int* list, const int* n_list, int* next_item, int* redo, int* n_redo) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   HistSmem& s = *reinterpret_cast<HistSmem*>(smem_raw);
   uint32_t* pen = reinterpret_cast<uint32_t*>(smem_raw + ((sizeof(HistSmem) + 15) & ~static_cast<size_t>(15)));

@@ -66,7 +66,7 @@ __host__ __device__ inline size_t slice_smem_bytes(int slice_len) { return slice
 // bits on the monotone keys. (BF16 logits have no key bits below those; for binary32 logits the few values that share the upper
 // 22 bits with the k-th largest pass the bound too, which the merge sorts out.)
 template <int B>
-__device__ uint32_t slice_kth_key(const float* vals, int n, uint32_t k, uint32_t* bins, uint64_t* scratch, uint32_t* pick) {
+static __device__ uint32_t slice_kth_key(const float* vals, int n, uint32_t k, uint32_t* bins, uint64_t* scratch, uint32_t* pick) {
   const int tid = threadIdx.x;
   uint32_t prefix = 0u, above = 0u;
 #pragma unroll 1
@@ -101,7 +101,7 @@ __device__ uint32_t slice_kth_key(const float* vals, int n, uint32_t k, uint32_t
 }
 
 template <int B>
-__global__ void __launch_bounds__(B) slice_local_kernel(SliceDev P) {
+static __global__ void __launch_bounds__(B) slice_local_kernel(SliceDev P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float* vals = reinterpret_cast<float*>(smem_raw);
   uint32_t* marks = reinterpret_cast<uint32_t*>(smem_raw + slice_marks_offset(P.slice_len));
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(B) slice_local_kernel(SliceDev P) {
 }
 
 // The merge of the sliced path: one block per row. Launched with programmatic stream serialization behind slice_local_kernel.
-__global__ void __launch_bounds__(kVpMaxCandidates, 1) sliced_merge_kernel(VpMergeDev M, SampleDev P) {
+static __global__ void __launch_bounds__(kVpMaxCandidates, 1) sliced_merge_kernel(VpMergeDev M, SampleDev P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ VpMergeSmem s;
   asm volatile("griddepcontrol.wait;" ::: "memory");                      // the records are complete behind this

@@ -60,7 +60,7 @@ __device__ __forceinline__ uint32_t f32_to_bf16_code(float f) {            // ro
 
 // The value key of the k-th largest entry (k >= 1, k <= n) of list[0 .. n): a 4 x 8-bit radix descent on the 32-bit monotone
 // value keys, counting in shared memory. Every thread of the block calls; hist: 256 counters; pick: 2 words.
-__device__ uint32_t tile_kth_key(const unsigned long long* list, int n, int k, uint32_t* hist, uint32_t* pick) {
+static __device__ uint32_t tile_kth_key(const unsigned long long* list, int n, int k, uint32_t* hist, uint32_t* pick) {
   uint32_t prefix = 0u, above = 0u;                                       // `above`: entries whose key is larger than every key with this prefix
   for (int level = 0; level < 4; level++) {
     const int shift = 24 - 8 * level;
@@ -85,7 +85,7 @@ __device__ uint32_t tile_kth_key(const unsigned long long* list, int n, int k, u
 }
 
 // Keeps the entries of list[0 .. n) whose value key is >= min_key, in their order; returns how many. Every thread calls.
-__device__ int tile_filter(unsigned long long* list, int n, uint32_t min_key, uint32_t* warp_cnt) {
+static __device__ int tile_filter(unsigned long long* list, int n, uint32_t min_key, uint32_t* warp_cnt) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   int out = 0;
   for (int i0 = 0; i0 < n; i0 += blockDim.x) {                            // a batch is read completely before any of it is written
@@ -108,7 +108,7 @@ __device__ int tile_filter(unsigned long long* list, int n, uint32_t min_key, ui
 // of the block calls with the same arguments. scratch: 256 + 2 + 32 words and 32 doubles of shared memory (TileScratch).
 struct TileScratch { uint32_t hist[256]; uint32_t pick[2]; uint32_t warp_cnt[32]; double warp_d[32]; double warp_p[32]; uint64_t warp_m[32]; uint32_t n_now; };
 
-__device__ void tile_consume_row(TileRow* st, unsigned long long* list, const uint16_t* codes, int cols, int col0, float temperature, int top_k,
+static __device__ void tile_consume_row(TileRow* st, unsigned long long* list, const uint16_t* codes, int cols, int col0, float temperature, int top_k,
                                  const uint32_t* pen_bits, float rho, float pi, TileScratch& t) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
   if (st->flags & kTileDeclined) return;
@@ -211,7 +211,7 @@ __device__ void tile_consume_row(TileRow* st, unsigned long long* list, const ui
 }
 
 // A tile that lies in memory: one block per row. FP32 tiles are rounded to BF16 first (what lm_head stores).
-__global__ void __launch_bounds__(kTileBlock) tile_consume_kernel(TileDev P) {
+static __global__ void __launch_bounds__(kTileBlock) tile_consume_kernel(TileDev P) {
   __shared__ TileScratch t;
   __shared__ uint16_t codes[kTileMaxCols];
   const int row = blockIdx.x;
@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(kTileBlock) tile_consume_kernel(TileDev P) {
 }
 
 // Clears the rows' states and, with a history, builds each row's bitmap of distinct history ids. One block per row.
-__global__ void __launch_bounds__(kTileBlock) tile_begin_kernel(TileDev P) {
+static __global__ void __launch_bounds__(kTileBlock) tile_begin_kernel(TileDev P) {
   const int row = blockIdx.x;
   if (row >= P.rows) return;
   if (threadIdx.x < sizeof(TileRow) / 8) reinterpret_cast<unsigned long long*>(P.rows_state + row)[threadIdx.x] = 0ull;
@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(kTileBlock) tile_begin_kernel(TileDev P) {
 
 // The rows' tokens from their states and lists: a last compaction to what the exact phases hold, the candidates into shared
 // memory with their code bins, then topk_finish. A row that cannot be finished here gets token -1 and LM_STATUS_TILE_DECLINED.
-__global__ void __launch_bounds__(kTB, kTopkPerSM) tile_finish_kernel(SampleDev P, TileRow* states, unsigned long long* lists) {
+static __global__ void __launch_bounds__(kTB, kTopkPerSM) tile_finish_kernel(SampleDev P, TileRow* states, unsigned long long* lists) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   TopkSmem& c = *reinterpret_cast<TopkSmem*>(smem_raw);
   __shared__ TileScratch t;

@@ -121,19 +121,19 @@ __device__ __forceinline__ bool topk_row_eligible(const SampleDev& P, int row) {
 }
 
 // The rows that are not the top-k kernel's, listed for the histogram kernel (one thread per row).
-__global__ void sample_classify_kernel(SampleDev P, int* list, int* n_list) {
+static __global__ void sample_classify_kernel(SampleDev P, int* list, int* n_list) {
   apply_step_state(P);
   const int row = blockIdx.x * blockDim.x + threadIdx.x;
   if (row < P.rows && !topk_row_eligible(P, row)) list[atomicAdd(n_list, 1)] = row;
 }
 
 struct TopkSmem;
-__device__ bool topk_finish(const SampleDev& P, int row, TopkSmem& c, uint32_t cut_code, const RowMass& zm);
+static __device__ bool topk_finish(const SampleDev& P, int row, TopkSmem& c, uint32_t cut_code, const RowMass& zm);
 
 // One row. Every thread of the block calls with the same arguments; returns true when the row is finished, false when the
 // histogram kernel has to take it (nothing has been written then).
 // `next` is the row this block takes afterwards (-1: none): its sample and history are pulled into L2 meanwhile.
-__device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem& c) {
+static __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem& c) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int V = P.vocab;
   const float T = P.temperature ? P.temperature[row] : P.temperature_s;
@@ -417,7 +417,7 @@ __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem& c) {
 // how many of them have BF16 code cut_code + b, c.wide set if one lies beyond the bins. `zm` is what is known about the mass of
 // the WHOLE row. Every thread of the block calls with the same arguments; returns true when the row is finished (token, tau
 // and status written), false when the exact path has to take it (nothing has been written then).
-__device__ bool topk_finish(const SampleDev& P, int row, TopkSmem& c, uint32_t cut_code, const RowMass& zm) {
+static __device__ bool topk_finish(const SampleDev& P, int row, TopkSmem& c, uint32_t cut_code, const RowMass& zm) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const float T = P.temperature ? P.temperature[row] : P.temperature_s;
   const int top_k = P.top_k ? P.top_k[row] : P.top_k_s;
@@ -630,7 +630,7 @@ __device__ bool topk_finish(const SampleDev& P, int row, TopkSmem& c, uint32_t c
 // Rows are handed out through a counter in the workspace (counters[0], zeroed by the host before the launch): a block takes
 // the next row, passes over it if it is not this kernel's (listing it if `list_others`), and else either finishes it or appends it to `list` (length in
 // counters[1]) for the histogram kernel. The order of the list varies from run to run; what is computed per row does not.
-__global__ void __launch_bounds__(kTB, kTopkPerSM) sample_topk_kernel(SampleDev P, int* list, int* counters, int list_others) {
+static __global__ void __launch_bounds__(kTB, kTopkPerSM) sample_topk_kernel(SampleDev P, int* list, int* counters, int list_others) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   TopkSmem& c = *reinterpret_cast<TopkSmem*>(smem_raw);
   __shared__ int item[2];                                                   // the row in hand and the one after it

@@ -70,7 +70,7 @@ struct AcceptDev {
 //   lanes k <= acc  hold the k-th token to commit (accepted draft, or the pick after the last accepted one), test it against the
 //                   stop tokens, and, up to the first stop token, publish it in ring slot head + k
 //   lane 0          writes the log entry and moves the state on
-__device__ void round_close(const AcceptDev& p) {
+static __device__ void round_close(const AcceptDev& p) {
   const int lane = threadIdx.x & 31;
   StepStateView st{p.state, p.t_max, p.g};
   if (st.done()) return;
@@ -127,7 +127,7 @@ __device__ void round_close(const AcceptDev& p) {
   }
 }
 
-__global__ void accept_scan_kernel(AcceptDev p) {
+static __global__ void accept_scan_kernel(AcceptDev p) {
   if (blockIdx.x == 0 && threadIdx.x < 32) round_close(p);
 }
 
@@ -140,7 +140,7 @@ struct SelectDev {
 // length L comes from the confidences (mode 0: the confident prefix, by vote; mode 1: the length with the best expected tokens
 // per unit cost, a running product that lane 0 forms in the reference's order; mode 2: a fixed length); lanes k < L then stage
 // draft k as pending token k + 1 behind the anchor. One warp.
-__global__ void verify_select_kernel(SelectDev p) {
+static __global__ void verify_select_kernel(SelectDev p) {
   if (blockIdx.x != 0 || threadIdx.x >= 32) return;
   const uint32_t lane = threadIdx.x;
   StepStateView st{p.state, p.t_max, p.g};
@@ -201,7 +201,7 @@ struct AdvanceDev { const int32_t* token; uint32_t* state; int t_max, g; unsigne
 
 // Closes a step that verified nothing: the last row's token is the step's token. The lanes share the stop-token test (one list
 // entry each per vote); lane 0 publishes the token and moves the state on. One warp.
-__global__ void advance_kernel(AdvanceDev p) {
+static __global__ void advance_kernel(AdvanceDev p) {
   if (blockIdx.x != 0 || threadIdx.x >= 32) return;
   const int lane = threadIdx.x;
   StepStateView st{p.state, p.t_max, p.g};
@@ -247,7 +247,7 @@ __device__ __forceinline__ float lane_dot_bf16(const uint16_t* row, const float*
   return acc;
 }
 
-__global__ void confidence_kernel(ConfDev p) {
+static __global__ void confidence_kernel(ConfDev p) {
   const int lane = threadIdx.x & 31, k = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (k >= p.gamma) return;
   if (p.state) { StepStateView st{p.state, p.t_max, p.g}; if (st.done()) return; }

@@ -34,7 +34,7 @@ struct VpLocalDev {
   int cap; unsigned char* records; int64_t record_bytes;
 };
 
-__global__ void __launch_bounds__(kBlock, 1) vocab_local_kernel(VpLocalDev P) {
+static __global__ void __launch_bounds__(kBlock, 1) vocab_local_kernel(VpLocalDev P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   GenericSmem& s = *reinterpret_cast<GenericSmem*>(smem_raw);
   __shared__ uint32_t s_n, s_ninf;
@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(kBlock, 1) vocab_local_kernel(VpLocalDev P) {
 // inside the k-th key's bin.
 // B threads, all of them call; bins: kSelectBins words, scratch: 32 words, pick: 3 words of shared memory.
 template <int B, int PER>
-__device__ uint32_t kth_key_bound_in_span(const uint32_t (&keys)[PER], uint32_t k, uint32_t lo_key, uint32_t hi_key, uint32_t limit,
+static __device__ uint32_t kth_key_bound_in_span(const uint32_t (&keys)[PER], uint32_t k, uint32_t lo_key, uint32_t hi_key, uint32_t limit,
                                           uint32_t* bins, uint64_t* scratch, uint32_t* pick) {
   const int tid = threadIdx.x;
   const uint32_t span = hi_key - lo_key;
@@ -206,8 +206,11 @@ __device__ __forceinline__ const unsigned char* merge_record(const VpMergeDev& P
   return P.records + (static_cast<int64_t>(shard) * P.rows + row) * P.record_bytes;
 }
 
-template <int E>
-__device__ void merge_tail_one_warp(const VpMergeDev& P, int row, VpMergeSmem& s, int N, float T, int top_k, float top_p, float min_p, double inv_t,
+// The ordered candidates of a row and what is known about it, where they do not lie in a VpMergeSmem (sample_cluster.cuh).
+struct MergeTail { const unsigned long long* key; float vmax; double z_total; int amb; };
+
+template <int E, class Smem>
+static __device__ void merge_tail_one_warp(const VpMergeDev& P, int row, Smem& s, int N, float T, int top_k, float top_p, float min_p, double inv_t,
                                     uint32_t status0) {
   const int lane = threadIdx.x & 31;
   unsigned long long key[E]; bool valid[E]; float val[E]; int idx[E]; uint32_t hi[E];
@@ -336,7 +339,7 @@ __device__ void merge_tail_one_warp(const VpMergeDev& P, int row, VpMergeSmem& s
       kept_weight = warp_sum_u64(ws);
     }
   }
-  if (lane == 0) {
+  if (lane == 0 && P.out_tokens) {
     P.out_tokens[row] = token;
     if (P.out_tau) P.out_tau[row] = tau;
     if (P.out_status) P.out_status[row] = status;
@@ -348,7 +351,7 @@ __device__ void merge_tail_one_warp(const VpMergeDev& P, int row, VpMergeSmem& s
 // One row of the merge. Every thread of the block (kVpMaxCandidates threads) calls with the same arguments; returns false when
 // the row's records overflowed and the caller asked to hand such rows on (P.hand_on): nothing has been written then.
 // The host has checked shards <= kVpMaxShards and cap <= kVpPerThread * (kVpMaxCandidates / shards).
-__device__ bool vocab_merge_row(const VpMergeDev& P, int row, VpMergeSmem& s) {
+static __device__ bool vocab_merge_row(const VpMergeDev& P, int row, VpMergeSmem& s) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const float T = P.temperature ? P.temperature[row] : P.temperature_s;
   int top_k = P.top_k ? P.top_k[row] : P.top_k_s;
@@ -579,7 +582,7 @@ __device__ bool vocab_merge_row(const VpMergeDev& P, int row, VpMergeSmem& s) {
   return true;
 }
 
-__global__ void __launch_bounds__(kVpMaxCandidates, 1) vocab_merge_kernel(VpMergeDev P) {
+static __global__ void __launch_bounds__(kVpMaxCandidates, 1) vocab_merge_kernel(VpMergeDev P) {
   __shared__ VpMergeSmem s;
   for (int row = blockIdx.x; row < P.rows; row += gridDim.x) vocab_merge_row(P, row, s);
 }

@@ -1,0 +1,129 @@
+"""The cluster row sampler (one row per thread-block cluster): what the streaming kernels do not take -- binary32 rows, ragged
+vocabularies and misaligned rows, statistics and probabilities -- and batches too small to fill the GPU with a block per row.
+Tokens and thresholds are the oracle's, bit for bit; probabilities and masses are binary32 roundings of FP64 sums (1e-6)."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+import lithos_metal_b200 as lm
+
+pytestmark = pytest.mark.gpu
+
+
+def _tensor(host):
+    return torch.from_numpy(host.view(np.int16)).cuda().view(torch.bfloat16) if host.dtype == np.uint16 else torch.from_numpy(host).cuda()
+
+
+def _check(x, host, knobs, *, draw, history=None, rho=1.0, pi=0.0, seed=3, step=5, row_offset=0, exact_only=False, topp_in_topk=False, stats=False):
+    rows = x.shape[0]
+    u = np.random.default_rng(seed + 7).random(rows).astype(np.float32)
+    dev = {k: torch.from_numpy(np.ascontiguousarray(v)).cuda() if isinstance(v, np.ndarray) else v for k, v in knobs.items()}
+    p = lm.SamplingParams(seed=seed, draw=draw, repetition_penalty=rho, presence_penalty=pi, exact_only=exact_only, topp_in_topk=topp_in_topk, **dev)
+    r = lm.sample(x, p, history=None if history is None else torch.from_numpy(history).cuda(), uniforms=torch.from_numpy(u).cuda(), step=step,
+                  row_offset=row_offset, return_tau=True, return_status=True, return_stats=stats, return_probs=stats, return_vmax=True)
+    tok, tau, st = oracle.sample_batch(host, history=history, repetition_penalty=rho, presence_penalty=pi, draw=draw, uniforms=u, seed=seed, step=step,
+                                       row_offset=row_offset, topp_in_topk=topp_in_topk, n_threads=8, **knobs)
+    status = r.status.cpu().numpy()
+    np.testing.assert_array_equal(r.tau.cpu().numpy(), tau)
+    assert np.all((r.tokens.cpu().numpy() == tok) | ((status & 4) != 0)), np.nonzero(r.tokens.cpu().numpy() != tok)
+    if stats:
+        np.testing.assert_allclose(r.stats.cpu().numpy(), st, rtol=1e-6)
+        pr = r.probs.cpu().numpy().astype(np.float64)
+        np.testing.assert_allclose(pr.sum(-1), 1.0, rtol=1e-5)
+        z = oracle.bf16_to_f32(host) if host.dtype == np.uint16 else host
+        for i in range(rows):
+            zi = z[i] if history is None else oracle.apply_penalties(z[i], history[i], rho, pi)
+            t = knobs["temperature"][i] if isinstance(knobs["temperature"], np.ndarray) else knobs["temperature"]
+            e = np.where(zi >= tau[i], np.exp((zi.astype(np.float64) - float(zi.max())) / np.float64(np.float32(t))), 0.0)
+            np.testing.assert_allclose(pr[i], e / e.sum(), rtol=1e-6, atol=1e-40)
+    return r, status
+
+
+def _mixed(rng, rows, top_ks=(0, 1, 20, 50, 1000)):
+    return dict(temperature=rng.uniform(0.3, 1.5, rows).astype(np.float32), top_k=rng.choice(np.array(top_ks, np.int32), rows),
+                top_p=rng.uniform(0.7, 1.02, rows).astype(np.float32), min_p=rng.choice(np.array([0.0, 0.0, 0.03], np.float32), rows))
+
+
+# rows choose the blocks per row (16 / 8 / 4 / 2 / 1), vocabularies the edges of chunks (8), of the smallest slices (2048) and of the
+# blocks' sweeps (8192 logits), views the alignment of the rows
+@pytest.mark.parametrize("rows,vocab", [(1, 151936), (8, 40001), (9, 16385), (19, 8191), (38, 50257), (75, 4099), (150, 2049), (3, 1), (5, 9), (2, 262139)])
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("draw", ["inverse_cdf", "gumbel"])
+def test_rows_and_sizes(rows, vocab, dtype, draw):
+    rng = np.random.default_rng(rows * 7 + vocab)
+    z = (rng.standard_normal((rows, vocab)) * 2).astype(np.float32)
+    host = oracle.f32_to_bf16(z) if dtype == "bf16" else z
+    hist = rng.integers(-3, vocab + 3, (rows, 300)).astype(np.int32)
+    _check(_tensor(host), host, _mixed(rng, rows), draw=draw, history=hist, rho=1.2, pi=0.3, row_offset=11)
+    wide = np.zeros((rows, vocab + 5), host.dtype)                          # a view with an offset: another alignment for every row
+    wide[:, 3:3 + vocab] = host
+    _check(_tensor(wide)[:, 3:3 + vocab], host, _mixed(rng, rows, (0,)), draw=draw)
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("rows", [2, 40])
+def test_statistics_and_probabilities(dtype, rows):
+    rng = np.random.default_rng(rows)
+    z = (rng.standard_normal((rows, 30011)) * 2).astype(np.float32)
+    host = oracle.f32_to_bf16(z) if dtype == "bf16" else z
+    hist = rng.integers(0, 30011, (rows, 100)).astype(np.int32)
+    knobs = _mixed(rng, rows)
+    _, status = _check(_tensor(host), host, knobs, draw="gumbel", history=hist, rho=1.1, pi=0.5, stats=True)
+    assert np.all(status & 1)                                              # reported for such calls, whoever serves them
+    _check(_tensor(host), host, dict(temperature=0.9, top_k=0, top_p=0.0, min_p=0.0), draw="inverse_cdf", stats=True)
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+def test_without_lists_of_the_top_k(dtype):
+    """Crossing bins for everything: a top_k beyond the list, and exact_only; top-p inside the top-k set."""
+    rng = np.random.default_rng(5)
+    z = (rng.standard_normal((6, 65543)) * 2).astype(np.float32)
+    host = oracle.f32_to_bf16(z) if dtype == "bf16" else z
+    for kw in (dict(), dict(exact_only=True), dict(topp_in_topk=True), dict(exact_only=True, topp_in_topk=True)):
+        for draw in ("inverse_cdf", "gumbel"):
+            _, status = _check(_tensor(host), host, _mixed(rng, 6, (3, 700, 1500, 5000)), draw=draw, **kw)
+            assert np.count_nonzero(status & 1) <= 1
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+def test_rows_that_are_handed_on_and_degenerate_rows(dtype):
+    V = 40000
+    rng = np.random.default_rng(9)
+    z = (rng.standard_normal((8, V)) * 2).astype(np.float32)
+    z[0] = 1.5                                                              # every logit equal: no list holds the bin
+    z[1, 100:] = -np.inf                                                    # a masked row
+    z[2, ::2] = -1e9                                                        # masked by a large negative number
+    z[3, 5:4000] = 9.0                                                      # more ties at the top than a list holds
+    z[4] *= 300.0                                                           # nearly greedy
+    z[5] *= 1e-3                                                            # nearly uniform
+    z[6, 17] = 80.0                                                         # one logit far above the rest
+    host = oracle.f32_to_bf16(z) if dtype == "bf16" else z
+    for draw in ("inverse_cdf", "gumbel"):
+        for k in (0, 30, 2000):
+            knobs = dict(temperature=np.full(8, 0.8, np.float32), top_k=np.full(8, k, np.int32), top_p=np.full(8, 0.9, np.float32), min_p=np.zeros(8, np.float32))
+            knobs["temperature"][7] = 0.0
+            _check(_tensor(host), host, knobs, draw=draw)
+    x = _tensor(host).clone()
+    x[2, 77] = float("nan"); x[3, 9] = float("inf")
+    r = lm.sample(x, lm.SamplingParams(temperature=0.8, top_p=0.9, seed=1), return_status=True)
+    st = r.status.cpu().numpy()
+    assert st[2] & 2 and st[2] & 1 and st[3] & 1 and not np.any(st[[1, 4, 5, 6, 7]] & 3)
+
+
+def test_a_top_p_boundary_inside_the_error_bound_is_decided_in_fp64():
+    """top_p placed on (and a hair beside) an exact boundary of the cumulative mass: the coarse sums hand the decision to the fine ones."""
+    rng = np.random.default_rng(21)
+    rows = []
+    z0 = oracle.bf16_to_f32(oracle.f32_to_bf16((rng.standard_normal(60000) * 2).astype(np.float32)))
+    vals, counts = np.unique(z0.astype(np.float64), return_counts=True)
+    vals, counts = vals[::-1], counts[::-1]
+    cum = np.cumsum(counts * np.exp(vals - vals[0]))
+    for i in (40, 200, 600):
+        for d in (0.0, 1e-8, -1e-8, 1e-7, -1e-7, 1e-6, -1e-6, 1e-5, -1e-5):
+            rows.append(np.float32(cum[i] / cum[-1] * (1.0 + d)))
+    n = len(rows)
+    for host in (np.tile(oracle.f32_to_bf16(z0), (n, 1)), np.tile(z0, (n, 1))):
+        for k in (0, 1000):
+            knobs = dict(temperature=1.0, top_k=np.full(n, k, np.int32), top_p=np.array(rows, np.float32), min_p=0.0)
+            _check(_tensor(host), host, knobs, draw="inverse_cdf")
