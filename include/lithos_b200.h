@@ -54,10 +54,11 @@ extern "C" {
 /* lm_sample_args.flags */
 #define LM_FLAG_TOPP_IN_TOPK 1u /* top-p over the top-k set's renormalised mass (the Hugging Face warpers' order) */
 #define LM_FLAG_EXACT_ONLY 2u /* skip the one-pass candidate kernel for rows with a top_k: every row takes the histogram path (same results) */
+#define LM_FLAG_TOKENS_I64 4u /* lm_sample: out_tokens points to int64_t entries (what the reference's sampler modules return) */
 #define LM_FLAG_GRID_LIMIT(n) (((uint32_t)(n) & 0xFFu) << 8) /* at most n thread blocks (0 = one per SM): leaves SMs to other streams */
 
 /* per-row status bits written to lm_sample_args.out_status (optional) */
-#define LM_STATUS_GENERIC_PATH 1u /* the row was handled by the generic multi-pass path */
+#define LM_STATUS_GENERIC_PATH 1u /* the row was handled by the generic multi-pass path, or the call asked for statistics or probabilities */
 #define LM_STATUS_NAN 2u          /* the row holds a NaN: results for the row are unspecified */
 #define LM_STATUS_NEAR_TIE 4u     /* Gumbel draw: best and second-best key closer than 4e-6 (float32 log is library-specific) */
 #define LM_STATUS_TOPP_EDGE 8u    /* top-p: cumulative mass within 1e-12 (relative) of the target at the boundary */
@@ -145,24 +146,21 @@ LM_API int lm_sample(const lm_sample_args* args);
 LM_API int lm_argmax(const void* logits, int32_t dtype, int64_t rows, int64_t vocab, int64_t row_stride, int32_t* out_tokens,
               void* workspace, size_t workspace_bytes, void* stream);
 
+/* The same with int64_t tokens, as GreedySampler.forward returns them. No workspace. */
+LM_API int lm_argmax_i64(const void* logits, int32_t dtype, int64_t rows, int64_t vocab, int64_t row_stride, int64_t* out_tokens, void* stream);
+
 /*
- * lm_argmax with its scratch inside the library: for callers that cannot allocate device memory.
+ * lm_argmax without the workspace arguments: for callers that cannot allocate device memory.
  *
  * Has no counterpart in lithos-metal (whose programs size every buffer at compile time). Some hosts of this library
  * are handed tensors and a stream and nothing else: a runtime plug-in called from a frozen decode loop, a step
  * that runs while the engine's allocator is locked or while a memory budget is already spent, code that must not
- * call cudaMalloc because cudaMalloc synchronises the device. They cannot create the workspace lm_argmax needs when it
- * splits rows over several thread blocks, so this entry point keeps that workspace in a fixed device array that is
- * part of the library image: LM_ARGMAX_STATIC_MAX_ROWS entries of 16 bytes (64 KiB), resident on every GPU that
- * loads the library for as long as the process lives.
+ * call cudaMalloc because cudaMalloc synchronises the device. (lm_argmax itself needs no scratch any more either: the
+ * blocks that share a row meet in one another's shared memory. Its workspace arguments are not read.)
  *
  *   - same arguments and result as lm_argmax, minus the workspace; rows > LM_ARGMAX_STATIC_MAX_ROWS returns LM_E_UNSUPPORTED;
  *   - it allocates nothing: no cudaMalloc / cudaFree and no allocating library call, on any call;
- *   - the first call on each device looks up the array's device address (cudaGetSymbolAddress, with that device
- *     current) and remembers it; make that first call before starting a stream capture;
- *   - every call uses the same array and clears the part it needs on the given stream before the kernel runs, so
- *     calls on one stream may follow each other freely, but two calls that can overlap on the GPU (different
- *     streams without an ordering between them, or different host threads) race on it: order them yourself.
+ *   - calls on different streams or from different host threads do not disturb one another.
  */
 #define LM_ARGMAX_STATIC_MAX_ROWS 4096
 LM_API int lm_argmax_static(const void* logits, int32_t dtype, int64_t rows, int64_t vocab, int64_t row_stride, int32_t* out_tokens, void* stream);

@@ -3,6 +3,8 @@ object is missing and cannot be built, importing the binding raises."""
 from __future__ import annotations
 
 import ctypes as C
+import importlib
+import importlib.util
 import os
 
 from . import build as _build
@@ -117,10 +119,11 @@ class HeadArgs(C.Structure):
     ]
 
 
-EXPORTS = ["lm_head", "lm_accept_scan", "lm_verify_select", "lm_advance", "lm_step_state_bytes", "lm_sample", "lm_argmax", "lm_argmax_static", "lm_vocab_local", "lm_vocab_merge", "lm_vocab_record_bytes", "lm_vocab_candidate_cap", "lm_vocab_pieces", "lm_verify", "lm_draft_q", "lm_confidence", "lm_tile_state_bytes", "lm_tile_begin", "lm_tile_consume", "lm_tile_finish", "lm_workspace_bytes", "lm_verify_workspace_bytes", "lm_uniform01", "lm_abi_version",
+EXPORTS = ["lm_head", "lm_accept_scan", "lm_verify_select", "lm_advance", "lm_step_state_bytes", "lm_sample", "lm_argmax", "lm_argmax_i64", "lm_argmax_static", "lm_vocab_local", "lm_vocab_merge", "lm_vocab_record_bytes", "lm_vocab_candidate_cap", "lm_vocab_pieces", "lm_verify", "lm_draft_q", "lm_confidence", "lm_tile_state_bytes", "lm_tile_begin", "lm_tile_consume", "lm_tile_finish", "lm_workspace_bytes", "lm_verify_workspace_bytes", "lm_uniform01", "lm_abi_version",
            "lm_error_string", "lm_last_cuda_error", "lm_device_sm_count"]
 
 _lib = None
+_host = None
 
 
 def library_path() -> str:
@@ -153,6 +156,8 @@ def lib():
         L.lm_draft_q.argtypes = [C.POINTER(DraftQArgs)]
         L.lm_argmax.restype = C.c_int
         L.lm_argmax.argtypes = [C.c_void_p, C.c_int32, C.c_int64, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p]
+        L.lm_argmax_i64.restype = C.c_int
+        L.lm_argmax_i64.argtypes = [C.c_void_p, C.c_int32, C.c_int64, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p]
         L.lm_argmax_static.restype = C.c_int
         L.lm_argmax_static.argtypes = [C.c_void_p, C.c_int32, C.c_int64, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p]
         L.lm_vocab_local.restype = L.lm_vocab_merge.restype = C.c_int
@@ -184,6 +189,23 @@ def lib():
             raise RuntimeError("lithos_metal_b200: ABI version mismatch between the binding and the shared object")
         _lib = L
     return _lib
+
+
+def host():
+    """The native call path (csrc/host_ext.cpp), handed the addresses of the loaded library's functions and the types it returns."""
+    global _host
+    if _host is None:
+        L = lib()
+        spec = importlib.util.spec_from_file_location("lithos_host", _build.HOST_OUT)
+        if not os.path.exists(_build.HOST_OUT):
+            raise RuntimeError(f"lithos_metal_b200: native host layer {_build.HOST_OUT} is missing; run `python -m lithos_metal_b200.build`")
+        m = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(m)
+        sampler, verify = (importlib.import_module(f"{__package__}.{n}") for n in ("sampler", "verify"))
+        names = ("lm_sample", "lm_argmax", "lm_argmax_i64", "lm_verify", "lm_draft_q", "lm_head", "lm_workspace_bytes", "lm_verify_workspace_bytes")
+        m.init({n: C.cast(getattr(L, n), C.c_void_p).value for n in names}, sampler.SamplingParams, sampler.SampleOutput, verify.DraftQ, check, sampler._workspace)
+        _host = m
+    return _host
 
 
 class LithosError(RuntimeError):

@@ -1,7 +1,8 @@
 """Builds the CUDA library in-tree: ``lithos_metal_b200/_lib/liblithos_b200.so`` for sm_100a with nvcc.
 
 ``python -m lithos_metal_b200.build`` (or :func:`build`). The shared object has a plain C ABI (include/lithos_b200.h);
-it is loaded with ctypes, so no Python headers and no torch headers are involved.
+it is loaded with ctypes, so no Python headers and no torch headers are involved. Beside it ``lithos_host.so``, a CPython extension
+(csrc/host_ext.cpp, g++ with torch's headers): the Python layer's calls without the cost of ctypes.
 """
 from __future__ import annotations
 
@@ -9,12 +10,15 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 SRC_DIR = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "_lib", "liblithos_b200.so")
+HOST_OUT = os.path.join(HERE, "_lib", "lithos_host.so")   # the native call path of the Python layer (CPython extension)
+HOST_SOURCE = "host_ext.cpp"
 SOURCES = ["lithos_b200.cu", "cluster.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-fvisibility=hidden",
               "--fmad=true", "-Xptxas", "-v", "-cudart", "shared"]
@@ -32,10 +36,21 @@ def _nvcc() -> str:
     raise RuntimeError("nvcc not found: the CUDA library cannot be built")
 
 
+def _host_command():
+    """g++ on the CPython extension: it reads tensors through torch's headers and links against the torch that is installed."""
+    import torch
+    base = os.path.join(os.path.dirname(torch.__file__))
+    inc = [os.path.join(base, "include"), os.path.join(base, "include", "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"],
+           os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")]
+    return [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            *[f"-isystem{d}" for d in inc], "-o", HOST_OUT, os.path.join(SRC_DIR, HOST_SOURCE), "-L", os.path.join(base, "lib"),
+            "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10"]
+
+
 def _stale() -> bool:
-    if not os.path.exists(OUT):
+    if not os.path.exists(OUT) or not os.path.exists(HOST_OUT):
         return True
-    t = os.path.getmtime(OUT)
+    t = min(os.path.getmtime(OUT), os.path.getmtime(HOST_OUT))
     deps = [os.path.join(SRC_DIR, f) for f in os.listdir(SRC_DIR)] + [os.path.join(ROOT, "include", "lithos_b200.h"), os.path.abspath(__file__)]
     return any(os.path.getmtime(d) > t for d in deps)
 
@@ -50,9 +65,10 @@ def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(os.path.dirname(OUT), exist_ok=True)
     cmds = [[_nvcc(), *NVCC_FLAGS, *EXTRA_FLAGS.get(src, []), "-I", os.path.join(ROOT, "include"), "-c", "-o", os.path.join(os.path.dirname(OUT), os.path.splitext(src)[0] + ".o"),
              os.path.join(SRC_DIR, src)] for src in SOURCES]
+    cmds.append(_host_command())
     with ThreadPoolExecutor(len(cmds)) as pool:                             # the translation units side by side
         done = list(pool.map(_run, cmds))
-    cmds.append([_nvcc(), "-shared", "-cudart", "shared", "-o", OUT, *[c[c.index("-o") + 1] for c in cmds]])
+    cmds.append([_nvcc(), "-shared", "-cudart", "shared", "-o", OUT, *[c[c.index("-o") + 1] for c in cmds[:len(SOURCES)]]])
     if all(r.returncode == 0 for r in done):
         done.append(_run(cmds[-1]))
     log = os.path.join(os.path.dirname(OUT), "build.log")
@@ -63,7 +79,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if verbose or failed:
         print(text)
     if failed:
-        raise RuntimeError(f"nvcc failed; see {log}")
+        raise RuntimeError(f"the build failed; see {log}")
     return OUT
 
 

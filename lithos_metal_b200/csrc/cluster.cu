@@ -1,15 +1,16 @@
 // The launches of the cluster row sampler (a translation unit of its own: it is compiled beside the others).
 #include <cuda_runtime.h>
 
+#include "argmax.cuh"
 #include "host.cuh"
 #include "sample_cluster.cuh"
 
 namespace lm {
 
-// Blocks per row of the cluster kernel: as many as keep every SM busy (16 needs an opt-in; a GPU processing cluster holds one such
-// cluster, so 8 rows), slices of at least 2048 logits.
+// Blocks per row of the cluster kernels: as many as keep every SM busy (16 needs an opt-in; seven such clusters of blocks with an SM
+// each are resident at once, fifteen of eight), slices of at least 2048 logits.
 static int cluster_blocks(int64_t rows, int64_t vocab, int sms) {
-  int c = rows <= 8 ? 16 : rows * 8 <= sms ? 8 : rows * 4 <= sms ? 4 : rows * 2 <= sms ? 2 : 1;
+  int c = rows * 20 <= sms ? 16 : rows * 8 <= sms ? 8 : rows * 4 <= sms ? 4 : rows * 2 <= sms ? 2 : 1;
   while (c > 1 && vocab < 2048LL * c) c >>= 1;
   return c;
 }
@@ -43,6 +44,29 @@ int sample_clusters(const SampleDev& P, int sms, cudaStream_t st) {
   if (cached) return f32 ? launch_cluster<true, true, 1>(P, C, smem, 0, st) : launch_cluster<false, true, 1>(P, C, smem, 1, st);
   if (two) return f32 ? launch_cluster<true, false, 2>(P, C, smem, 2, st) : launch_cluster<false, false, 2>(P, C, smem, 3, st);
   return f32 ? launch_cluster<true, false, 1>(P, C, smem, 4, st) : launch_cluster<false, false, 1>(P, C, smem, 5, st);
+}
+
+template <bool F32>
+static int launch_argmax(const void* logits, int rows, int vocab, int64_t row_stride, int32_t* out32, int64_t* out64, int C, cudaStream_t st) {
+  const int rc = ensure_dynamic_smem(static_cast<KernelSlot>(kSlotArgmax + (F32 ? 1 : 0)), reinterpret_cast<const void*>(argmax_cluster_kernel<F32>), 1, true);
+  if (rc != LM_OK) return rc;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(rows) * static_cast<unsigned>(C)); cfg.blockDim = dim3(kArgmaxThreads); cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(C); attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = C > 1 ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, argmax_cluster_kernel<F32>, logits, vocab, row_stride, out32, out64, C);
+  return e == cudaSuccess ? LM_OK : cuda_fail(e);
+}
+
+int argmax_clusters(const void* logits, int dtype, int rows, int vocab, int64_t row_stride, int32_t* out32, int64_t* out64, cudaStream_t st) {
+  int sms = 0;
+  const int rc = sm_count(&sms);
+  if (rc != LM_OK) return rc;
+  const int C = cluster_blocks(rows, vocab, 2 * sms);                       // (two of these blocks share an SM easily)
+  return dtype == LM_DTYPE_F32 ? launch_argmax<true>(logits, rows, vocab, row_stride, out32, out64, C, st)
+                               : launch_argmax<false>(logits, rows, vocab, row_stride, out32, out64, C, st);
 }
 
 }  // namespace lm

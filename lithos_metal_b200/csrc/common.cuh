@@ -244,6 +244,11 @@ __device__ __forceinline__ uint64_t block_exclusive_scan_u64(uint64_t v, uint64_
   return warp_base + incl - v;
 }
 
+// A row's token, 32 or 64 bits wide.
+__device__ __forceinline__ void store_token(int32_t* out, uint32_t flags, int row, int token) {
+  if (flags & LM_FLAG_TOKENS_I64) reinterpret_cast<int64_t*>(out)[row] = token; else out[row] = token;
+}
+
 // Packed (value, index) for argmax with ties -> lowest index: larger packed value wins.
 __device__ __forceinline__ uint64_t pack_best(float v, uint32_t idx) { return (static_cast<uint64_t>(fkey(v)) << 32) | (0xFFFFFFFFu - idx); }
 __device__ __forceinline__ uint32_t best_index(uint64_t p) { return 0xFFFFFFFFu - static_cast<uint32_t>(p); }

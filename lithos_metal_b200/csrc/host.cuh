@@ -33,7 +33,8 @@ inline int sm_count(int* out) {
 // Kernels that need more than 48 KB of dynamic shared memory must be told so once per device (the attribute belongs to the
 // device's copy of the function); remembered per device and kernel, raised when a call needs more.
 enum KernelSlot { kSlotFast, kSlotTopk, kSlotGeneric, kSlotVocabLocal, kSlotVerify, kSlotVerifyStats, kSlotDraftQ, kSlotTileFinish, kSlotSlice, kSlotSliceSmall, kSlotSliceTiny, kSlotSlicedMerge, kSlotHead, kSlotCluster,
-                  kSlotCount = kSlotCluster + 6 };   // (the cluster kernel has six instances)
+                  kSlotArgmax = kSlotCluster + 6,   // (the cluster kernel has six instances, the argmax kernel two)
+                  kSlotCount = kSlotArgmax + 2 };
 
 inline int ensure_dynamic_smem(KernelSlot slot, const void* func, size_t bytes, bool large_clusters = false) {
   if (bytes <= 48 * 1024 && !large_clusters) return LM_OK;
@@ -61,5 +62,6 @@ inline size_t align256(size_t x) { return (x + 255) & ~static_cast<size_t>(255);
 struct SampleDev;
 // cluster.cu: one row per thread-block cluster, every row of the call.
 int sample_clusters(const SampleDev& P, int sms, cudaStream_t st);
+int argmax_clusters(const void* logits, int dtype, int rows, int vocab, int64_t row_stride, int32_t* out32, int64_t* out64, cudaStream_t st);
 
 }  // namespace lm

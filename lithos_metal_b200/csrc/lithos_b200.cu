@@ -23,43 +23,6 @@ namespace lm {
 
 static_assert(kBlock == 512 || kBlock == 1024, "the row kernels are written for 512 or 1024 threads per block");
 
-// ---- greedy argmax: rows x splits blocks, packed (value, lowest index) maxima meet in the workspace --------------
-constexpr int kArgmaxBlock = 512;
-
-struct ArgmaxWs { unsigned long long best; unsigned arrivals; unsigned pad; };   // one per row, zero when idle
-
-__global__ void __launch_bounds__(kArgmaxBlock) argmax_kernel(const void* logits, int dtype, int rows, int vocab, int64_t row_stride, int splits,
-                                                             int32_t* out_tokens, ArgmaxWs* ws) {
-  __shared__ uint64_t scratch[32];
-  const int row = blockIdx.y, split = blockIdx.x, tid = threadIdx.x;
-  RowView rv;
-  rv.dtype = dtype; rv.vocab = vocab; rv.pen = nullptr; rv.rho = 1.0f; rv.pi = 0.0f;
-  rv.row = static_cast<const char*>(logits) + static_cast<size_t>(row) * static_cast<size_t>(row_stride) * (dtype == LM_DTYPE_BF16 ? 2 : 4);
-  rv.aligned = (reinterpret_cast<uintptr_t>(rv.row) & 15u) == 0;
-  const int n_chunks = (vocab + kChunk - 1) / kChunk;
-  uint64_t best = 0ull;
-  for (int c = split * kArgmaxBlock + tid; c < n_chunks; c += splits * kArgmaxBlock) {
-    float z[kChunk];
-    const int n = load_chunk(rv, c, z);
-#pragma unroll
-    for (int e = 0; e < kChunk; e++) if (e < n) {
-      const uint64_t p = pack_best(z[e], static_cast<uint32_t>(c * kChunk + e));
-      best = p > best ? p : best;
-    }
-  }
-  best = block_max_u64(best, scratch);
-  if (tid != 0) return;
-  if (splits == 1) { out_tokens[row] = best ? static_cast<int>(best_index(best)) : -1; return; }
-  if (best) atomicMax(&ws[row].best, static_cast<unsigned long long>(best));
-  __threadfence();
-  if (atomicAdd(&ws[row].arrivals, 1u) == static_cast<unsigned>(splits) - 1u) {   // the last block of the row
-    __threadfence();
-    const unsigned long long b = atomicExch(&ws[row].best, 0ull);
-    ws[row].arrivals = 0u;
-    out_tokens[row] = b ? static_cast<int>(best_index(b)) : -1;
-  }
-}
-
 // ---- the generic sampler: one block per row, grid-stride over rows, or over the rows an earlier kernel listed ---------------
 __global__ void __launch_bounds__(kBlock, 1) sample_generic_kernel(SampleDev P, const int* list, const int* n_list) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -73,10 +36,6 @@ __global__ void __launch_bounds__(kBlock, 1) sample_generic_kernel(SampleDev P, 
     __syncthreads();
   }
 }
-
-// Scratch of lm_argmax_static: a fixed array in the library image (zero at load). In host code this name is only a
-// handle for cudaGetSymbolAddress; the kernels get the device address that call returns.
-static __device__ __align__(256) ArgmaxWs g_argmax_static_ws[LM_ARGMAX_STATIC_MAX_ROWS];
 
 constexpr int kOverlapRowsPerSM = 5;    // up to this many rows per SM the two sampler kernels run side by side (lm_sample)
 constexpr int kAloneRowsPerSM = 2;      // ... and up to this many the histogram kernel's blocks have their SM to themselves
@@ -137,9 +96,9 @@ float lm_uniform01(uint64_t seed, uint32_t step, uint32_t t, uint32_t index) { r
 size_t lm_workspace_bytes(int64_t rows, int64_t vocab) {
   (void)vocab;
   if (rows < 0) rows = 0;
-  // argmax partials | rows for the generic kernel | rows that are not the top-k kernel's | rows the top-k kernel left | counters
+  // (16 bytes a row, free) | rows for the generic kernel | rows that are not the top-k kernel's | rows the top-k kernel left | counters
   //   | the slice records of a call of a few rows
-  return align256(static_cast<size_t>(rows) * sizeof(ArgmaxWs)) + 3 * align256(static_cast<size_t>(rows) * sizeof(uint32_t)) + 256 + kSlicedWsBytes;
+  return align256(static_cast<size_t>(rows) * 16) + 3 * align256(static_cast<size_t>(rows) * sizeof(uint32_t)) + 256 + kSlicedWsBytes;
 }
 
 size_t lm_verify_workspace_bytes(int32_t n_draft, int64_t vocab) {
@@ -149,70 +108,34 @@ size_t lm_verify_workspace_bytes(int32_t n_draft, int64_t vocab) {
   return align256(sizeof(VerifyWs)) + align256(sizeof(DraftQWs));
 }
 
-int lm_argmax(const void* logits, int32_t dtype, int64_t rows, int64_t vocab, int64_t row_stride, int32_t* out_tokens, void* workspace,
-              size_t workspace_bytes, void* stream) {
+static int argmax_args_ok(const void* logits, int32_t dtype, int64_t rows, int64_t vocab, int64_t row_stride, const void* out_tokens) {
   if (rows < 0 || vocab < 0 || (dtype != LM_DTYPE_BF16 && dtype != LM_DTYPE_F32)) return LM_E_INVALID;
   if (rows == 0) return LM_OK;
   if (!logits || !out_tokens || row_stride < vocab) return LM_E_INVALID;
   if (vocab > LM_MAX_VOCAB || rows > 65535 * 32) return LM_E_UNSUPPORTED;
-  int sms = 0;
-  int rc = sm_count(&sms);
-  if (rc != LM_OK) return rc;
-  const int n_chunks = static_cast<int>((vocab + kChunk - 1) / kChunk);
-  // enough blocks to cover the machine twice; a block needs at least one sweep of work
-  int splits = static_cast<int>((2 * sms + rows - 1) / rows);
-  const int max_splits = (n_chunks + kArgmaxBlock - 1) / kArgmaxBlock;
-  if (splits > max_splits) splits = max_splits;
-  if (splits < 1) splits = 1;
-  if (splits > 1 && (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 255u) || workspace_bytes < lm_workspace_bytes(rows, vocab)))
-    return LM_E_WORKSPACE;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (splits > 1) {
-    // one entry per row, zero when the kernel starts. A workspace that also served lm_sample with another row count holds that
-    // call's row lists where these entries lie, so they are cleared here rather than trusted.
-    const cudaError_t e = cudaMemsetAsync(workspace, 0, static_cast<size_t>(rows) * sizeof(ArgmaxWs), st);
-    if (e != cudaSuccess) return cuda_fail(e);
-  }
-  for (int64_t r0 = 0; r0 < rows; r0 += 65535) {                          // gridDim.y limit
-    const int nr = static_cast<int>(rows - r0 < 65535 ? rows - r0 : 65535);
-    const size_t esz = dtype == LM_DTYPE_BF16 ? 2 : 4;
-    argmax_kernel<<<dim3(splits, nr), kArgmaxBlock, 0, st>>>(static_cast<const char*>(logits) + static_cast<size_t>(r0) * row_stride * esz, dtype, nr,
-                                                            static_cast<int>(vocab), row_stride, splits, out_tokens + r0,
-                                                            static_cast<ArgmaxWs*>(workspace) + r0);
-  }
-  const cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? LM_OK : cuda_fail(e);
+  return LM_OK;
 }
 
-// The allocation-free variant of lm_argmax: the same kernel, its workspace in g_argmax_static_ws.
+int lm_argmax(const void* logits, int32_t dtype, int64_t rows, int64_t vocab, int64_t row_stride, int32_t* out_tokens, void* workspace,
+              size_t workspace_bytes, void* stream) {
+  (void)workspace; (void)workspace_bytes;                                   // (the blocks of a row meet in shared memory)
+  const int rc = argmax_args_ok(logits, dtype, rows, vocab, row_stride, out_tokens);
+  if (rc != LM_OK || rows == 0) return rc;
+  return argmax_clusters(logits, dtype, static_cast<int>(rows), static_cast<int>(vocab), row_stride, out_tokens, nullptr, static_cast<cudaStream_t>(stream));
+}
+
+int lm_argmax_i64(const void* logits, int32_t dtype, int64_t rows, int64_t vocab, int64_t row_stride, int64_t* out_tokens, void* stream) {
+  const int rc = argmax_args_ok(logits, dtype, rows, vocab, row_stride, out_tokens);
+  if (rc != LM_OK || rows == 0) return rc;
+  return argmax_clusters(logits, dtype, static_cast<int>(rows), static_cast<int>(vocab), row_stride, nullptr, out_tokens, static_cast<cudaStream_t>(stream));
+}
+
+// lm_argmax needs no scratch any more; the row limit of the fixed array it once had is part of the interface.
 int lm_argmax_static(const void* logits, int32_t dtype, int64_t rows, int64_t vocab, int64_t row_stride, int32_t* out_tokens, void* stream) {
-  if (rows < 0 || vocab < 0 || (dtype != LM_DTYPE_BF16 && dtype != LM_DTYPE_F32)) return LM_E_INVALID;
-  if (rows == 0) return LM_OK;
-  if (!logits || !out_tokens || row_stride < vocab) return LM_E_INVALID;
-  if (rows > LM_ARGMAX_STATIC_MAX_ROWS || vocab > LM_MAX_VOCAB) return LM_E_UNSUPPORTED;   // beyond the fixed scratch
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return cuda_fail(e);
-  // set-up, once per device, with that device current: the device address of the scratch array
-  constexpr int kMaxDevices = 64;
-  static void* ws_addr[kMaxDevices] = {nullptr};
-  static std::mutex ws_mutex;
-  if (dev < 0 || dev >= kMaxDevices) return LM_E_UNSUPPORTED;
-  void* ws = nullptr;
-  {
-    std::lock_guard<std::mutex> lock(ws_mutex);
-    if (ws_addr[dev] == nullptr) {
-      void* p = nullptr;
-      e = cudaGetSymbolAddress(&p, g_argmax_static_ws);
-      if (e != cudaSuccess) return cuda_fail(e);
-      ws_addr[dev] = p;
-    }
-    ws = ws_addr[dev];
-  }
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // lm_argmax touches one ArgmaxWs entry per row and nothing else of a workspace (it clears the entries it uses on the stream
-  // before its kernel: the array keeps whatever the last call left); the size given here only has to pass its general check
-  return lm_argmax(logits, dtype, rows, vocab, row_stride, out_tokens, ws, lm_workspace_bytes(rows, vocab), st);
+  const int rc = argmax_args_ok(logits, dtype, rows, vocab, row_stride, out_tokens);
+  if (rc != LM_OK || rows == 0) return rc;
+  if (rows > LM_ARGMAX_STATIC_MAX_ROWS) return LM_E_UNSUPPORTED;
+  return lm_argmax(logits, dtype, rows, vocab, row_stride, out_tokens, nullptr, 0, stream);
 }
 
 // The merge's thread geometry and the FP64 reciprocal of a scalar temperature, once per call on the host.
@@ -317,7 +240,7 @@ int lm_sample(const lm_sample_args* a) {
     return sample_clusters(P, sms, st);
   if (fast) {
     const size_t rows_bytes = align256(static_cast<size_t>(a->rows) * sizeof(uint32_t));
-    char* ws = static_cast<char*>(a->workspace) + align256(static_cast<size_t>(a->rows) * sizeof(ArgmaxWs));
+    char* ws = static_cast<char*>(a->workspace) + align256(static_cast<size_t>(a->rows) * 16);
     int* redo = reinterpret_cast<int*>(ws);                                // rows for the generic kernel
     int* list_other = reinterpret_cast<int*>(ws + rows_bytes);             // rows that are not the top-k kernel's
     int* list_left = reinterpret_cast<int*>(ws + 2 * rows_bytes);          // rows the top-k kernel left

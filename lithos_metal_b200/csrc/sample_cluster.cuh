@@ -1352,7 +1352,7 @@ __global__ void __launch_bounds__(B, kPerSM) sample_cluster_kernel(const __grid_
   }
   __syncthreads();
   if (rank == 0 && tid == 0) {
-    P.out_tokens[row] = s.o_token;
+    store_token(P.out_tokens, P.flags, row, s.o_token);
     if (P.out_tau) P.out_tau[row] = s.o_tau;
     if (P.out_stats) { P.out_stats[2 * row] = s.vmax; P.out_stats[2 * row + 1] = static_cast<float>(kept_mass); }
     if (P.out_vmax) P.out_vmax[row] = s.vmax;

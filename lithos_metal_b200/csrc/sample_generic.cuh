@@ -155,7 +155,7 @@ static __device__ void sample_row_generic(const SampleDev& P, int row, GenericSm
 
   if (V <= 0 || !(T >= 0.0f)) {                                          // empty row or a bad temperature: no token
     if (tid == 0) {
-      P.out_tokens[row] = -1;
+      store_token(P.out_tokens, P.flags, row, -1);
       if (P.out_tau) P.out_tau[row] = -INFINITY;
       if (P.out_stats) { P.out_stats[2 * row] = 0.0f; P.out_stats[2 * row + 1] = 0.0f; }
       if (P.out_vmax) P.out_vmax[row] = -INFINITY;
@@ -203,7 +203,7 @@ static __device__ void sample_row_generic(const SampleDev& P, int row, GenericSm
       for (int i = tid; i < V; i += static_cast<int>(blockDim.x)) pr[i] = (i == arg) ? 1.0f : 0.0f;
     }
     if (tid == 0) {
-      P.out_tokens[row] = arg;
+      store_token(P.out_tokens, P.flags, row, arg);
       if (P.out_tau) P.out_tau[row] = -INFINITY;
       if (P.out_stats) { P.out_stats[2 * row] = vmax; P.out_stats[2 * row + 1] = 1.0f; }
       if (P.out_vmax) P.out_vmax[row] = vmax;
@@ -323,7 +323,7 @@ static __device__ void sample_row_generic(const SampleDev& P, int row, GenericSm
     }
   }
   if (tid == 0) {
-    P.out_tokens[row] = token;
+    store_token(P.out_tokens, P.flags, row, token);
     if (P.out_tau) P.out_tau[row] = tau;
     if (P.out_stats) { P.out_stats[2 * row] = vmax; P.out_stats[2 * row + 1] = static_cast<float>(kept_mass); }
     if (P.out_vmax) P.out_vmax[row] = vmax;

@@ -675,7 +675,7 @@ static __device__ void sample_row_hist(const SampleDev& P, int row, int next, Hi
     }
     best = block_max_u64(best, s.scratch);
     if (tid == 0) {
-      P.out_tokens[row] = static_cast<int>(best_index(best));
+      store_token(P.out_tokens, P.flags, row, static_cast<int>(best_index(best)));
       if (P.out_tau) P.out_tau[row] = -INFINITY;
       if (P.out_status) P.out_status[row] = (best_value(best) != best_value(best)) ? LM_STATUS_NAN : 0u;
       if (P.out_vmax) P.out_vmax[row] = best_value(best);
@@ -899,7 +899,7 @@ static __device__ void sample_row_hist(const SampleDev& P, int row, int next, Hi
   }
   // ---- phase 7: outputs ----------------------------------------------------------------------------------------------------------
   if (tid == 0) {
-    P.out_tokens[row] = token;
+    store_token(P.out_tokens, P.flags, row, token);
     if (P.out_tau) P.out_tau[row] = tau;
     if (P.out_status) P.out_status[row] = status;
     if (P.out_vmax) P.out_vmax[row] = vmax;

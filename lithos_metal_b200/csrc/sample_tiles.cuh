@@ -257,7 +257,7 @@ static __global__ void __launch_bounds__(kTB, kTopkPerSM) tile_finish_kernel(Sam
     const float T = P.temperature ? P.temperature[row] : P.temperature_s;
     if (T == 0.0f && !(st->flags & kTileDeclined) && (st->flags & 4u)) {     // greedy: the running argmax
       if (tid == 0) {
-        P.out_tokens[row] = static_cast<int>(best_index(st->best));
+        store_token(P.out_tokens, P.flags, row, static_cast<int>(best_index(st->best)));
         if (P.out_tau) P.out_tau[row] = -INFINITY;
         if (P.out_status) P.out_status[row] = 0u;
         if (P.out_vmax) P.out_vmax[row] = best_value(st->best);
@@ -297,7 +297,7 @@ static __global__ void __launch_bounds__(kTB, kTopkPerSM) tile_finish_kernel(Sam
       __syncthreads();
     }
     if (!ok && tid == 0) {
-      P.out_tokens[row] = -1;
+      store_token(P.out_tokens, P.flags, row, -1);
       if (P.out_tau) P.out_tau[row] = -INFINITY;
       if (P.out_status) P.out_status[row] = LM_STATUS_TILE_DECLINED;
       if (P.out_vmax) P.out_vmax[row] = (st->flags & 4u) ? static_cast<float>(st->m) : -INFINITY;

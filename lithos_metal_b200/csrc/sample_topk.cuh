@@ -617,7 +617,7 @@ static __device__ bool topk_finish(const SampleDev& P, int row, TopkSmem& c, uin
     }
   }
   if (tid == 0) {
-    P.out_tokens[row] = token;
+    store_token(P.out_tokens, P.flags, row, token);
     if (P.out_tau) P.out_tau[row] = tau;
     if (P.out_status) P.out_status[row] = status;
     if (P.out_vmax) P.out_vmax[row] = vmax;

@@ -340,7 +340,7 @@ static __device__ void merge_tail_one_warp(const VpMergeDev& P, int row, Smem& s
     }
   }
   if (lane == 0 && P.out_tokens) {
-    P.out_tokens[row] = token;
+    store_token(P.out_tokens, P.flags, row, token);
     if (P.out_tau) P.out_tau[row] = tau;
     if (P.out_status) P.out_status[row] = status;
     if (P.out_vmax) P.out_vmax[row] = vmax;
@@ -360,7 +360,7 @@ static __device__ bool vocab_merge_row(const VpMergeDev& P, int row, VpMergeSmem
   const double T64 = static_cast<double>(T), inv_t = P.temperature ? 1.0 / T64 : P.inv_t_s;
   uint32_t edge = 0u;
   if (!(T > 0.0f)) {                                                     // a per-row temperature the host could not check: no token
-    if (tid == 0) { P.out_tokens[row] = -1; if (P.out_tau) P.out_tau[row] = -INFINITY; if (P.out_status) P.out_status[row] = kStatusBadParam; }
+    if (tid == 0) { store_token(P.out_tokens, P.flags, row, -1); if (P.out_tau) P.out_tau[row] = -INFINITY; if (P.out_status) P.out_status[row] = kStatusBadParam; }
     return true;
   }
   // ---- One round of loads. This thread's share of the candidates (a group of threads per shard, slot j of the record to thread
@@ -441,7 +441,7 @@ static __device__ bool vocab_merge_row(const VpMergeDev& P, int row, VpMergeSmem
   // across GPUs, where such a row reports LM_STATUS_NAN and token -1.
   if ((s.status & LM_STATUS_NAN) || !(fabsf(s.vmax) < INFINITY)) {
     if (P.hand_on) return false;
-    if (tid == 0) { P.out_tokens[row] = -1; if (P.out_tau) P.out_tau[row] = -INFINITY; if (P.out_status) P.out_status[row] = s.status | LM_STATUS_NAN; }
+    if (tid == 0) { store_token(P.out_tokens, P.flags, row, -1); if (P.out_tau) P.out_tau[row] = -INFINITY; if (P.out_status) P.out_status[row] = s.status | LM_STATUS_NAN; }
     __syncthreads();
     return true;
   }
@@ -476,7 +476,7 @@ static __device__ bool vocab_merge_row(const VpMergeDev& P, int row, VpMergeSmem
   const uint32_t status0 = s.status;
   if ((status0 & kStatusOverflow) && P.hand_on) return false;             // single GPU: the caller gives the row to the generic path
   if ((status0 & kStatusOverflow) || N == 0) {
-    if (tid == 0) { P.out_tokens[row] = -1; if (P.out_tau) P.out_tau[row] = -INFINITY; if (P.out_status) P.out_status[row] = status0; }
+    if (tid == 0) { store_token(P.out_tokens, P.flags, row, -1); if (P.out_tau) P.out_tau[row] = -INFINITY; if (P.out_status) P.out_status[row] = status0; }
     __syncthreads();
     return true;
   }
@@ -572,7 +572,7 @@ static __device__ bool vocab_merge_row(const VpMergeDev& P, int row, VpMergeSmem
   }
   __syncthreads();
   if (tid == 0) {
-    P.out_tokens[row] = s.token;
+    store_token(P.out_tokens, P.flags, row, s.token);
     if (P.out_tau) P.out_tau[row] = tau;
     if (P.out_status) P.out_status[row] = status;
     if (P.out_vmax) P.out_vmax[row] = vmax;

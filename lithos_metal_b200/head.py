@@ -16,6 +16,9 @@ def lm_head(hidden: torch.Tensor, weight: torch.Tensor, norm_weight: Optional[to
     """``bf16(x @ weightᵀ)`` with FP32 accumulation; ``x = hidden`` or, with ``norm_weight``, ``bf16(rms_norm(hidden) * (1 + norm_weight))``
     (``one_plus=False``: ``* norm_weight``), as monolith/nn/oracle.py:20-32 defines both. ``hidden`` [rows <= 8, H] and ``weight`` [V, H]
     bfloat16 CUDA tensors with unit stride along H; returns [rows, V] bfloat16."""
+    r = _lib.host().lm_head(hidden, weight, norm_weight, eps, one_plus, out)
+    if r is not None:
+        return r
     if hidden.dim() != 2 or weight.dim() != 2 or hidden.shape[1] != weight.shape[1]:
         raise ValueError("lm_head: hidden [rows, H] and weight [V, H]")
     if hidden.dtype != torch.bfloat16 or weight.dtype != torch.bfloat16 or not hidden.is_cuda or weight.device != hidden.device:

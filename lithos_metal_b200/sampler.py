@@ -125,6 +125,12 @@ def sample(logits: torch.Tensor, params: Optional[SamplingParams] = None, *, his
     p = params if params is not None else SamplingParams(**knobs)
     if params is not None and knobs:
         raise TypeError("pass either params or knob keyword arguments, not both")
+    if step_state is None:
+        # the ordinary call in native code (csrc/host_ext.cpp): 4 us of host time instead of 25 for a single row; None: not that case
+        r = _lib.host().sample(logits, p, history, uniforms, step, row_offset, (1 if return_tau else 0) | (2 if return_stats else 0) |
+                               (4 if return_probs else 0) | (8 if return_status else 0) | (16 if return_vmax else 0), out)
+        if r is not None:
+            return r
     logits = _check_logits(logits)
     rows, vocab = logits.shape
     dev = logits.device
@@ -192,14 +198,15 @@ def sample(logits: torch.Tensor, params: Optional[SamplingParams] = None, *, his
 
 def argmax(logits: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Greedy pick of every row: int32 [rows], ties -> lowest index."""
+    r = _lib.host().argmax(logits, out, False)
+    if r is not None:
+        return r
     logits = _check_logits(logits)
     rows, vocab = logits.shape
     tokens = out if out is not None else torch.empty(rows, dtype=torch.int32, device=logits.device)
-    L = _lib.lib()
-    ws = _workspace(logits.device, L.lm_workspace_bytes(rows, vocab))
     with torch.cuda.device(logits.device):
-        _lib.check(L.lm_argmax(logits.data_ptr(), _dtype_code(logits), rows, vocab, _row_stride(logits), tokens.data_ptr(), ws.data_ptr(), ws.numel(),
-                               torch.cuda.current_stream(logits.device).cuda_stream), "lm_argmax")
+        _lib.check(_lib.lib().lm_argmax(logits.data_ptr(), _dtype_code(logits), rows, vocab, _row_stride(logits), tokens.data_ptr(), None, 0,
+                                        torch.cuda.current_stream(logits.device).cuda_stream), "lm_argmax")
     return tokens
 
 
@@ -211,7 +218,8 @@ class GreedySampler:
         self.prefix = prefix
 
     def forward(self, logits: torch.Tensor) -> torch.Tensor:
-        return argmax(logits).to(torch.int64)
+        r = _lib.host().argmax(logits, None, True)
+        return r if r is not None else argmax(logits).to(torch.int64)
 
     __call__ = forward
 
@@ -232,7 +240,8 @@ class StochasticSampler:
         return SamplingParams(self.temperature, self.top_k, self.top_p, self.min_p, self.seed, self.topp_in_topk, draw="gumbel")
 
     def forward(self, logits: torch.Tensor, step: int = 0) -> torch.Tensor:
-        return sample(logits, self.params(), step=step).tokens.to(torch.int64)
+        r = _lib.host().stochastic(logits, self.temperature, self.top_k, self.top_p, self.min_p, self.seed, self.topp_in_topk, step)
+        return r if r is not None else sample(logits, self.params(), step=step).tokens.to(torch.int64)
 
     __call__ = forward
 

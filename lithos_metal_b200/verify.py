@@ -33,6 +33,10 @@ def draft_q(logits: torch.Tensor, *, temperature: float, seed: int = 0, step: in
     (``logits`` [rows, V] bfloat16/float32, rows <= 16): ``argmax_i(z_i * float32(1/T) + gumbel(seed, step, 2000 + position, i))``,
     the unfiltered softmax at ``temperature`` as the reference's drafter samples it. ``step_state`` = ``(StepStateLayout, state)``
     takes seed and step from the device-side state instead (nothing is written once it is done). Asynchronous on the current stream."""
+    if step_state is None:
+        r = _lib.host().draft_q(logits, temperature, seed, step, first_position, copy_logits)
+        if r is not None:
+            return r
     if not temperature > 0:
         raise ValueError("temperature must be positive")
     logits = _check_logits(logits)
@@ -91,6 +95,12 @@ def verify(target_logits: torch.Tensor, draft_ids: Optional[torch.Tensor], draft
     """
     if mode not in ("greedy", "stochastic"):
         raise ValueError("mode must be 'greedy' or 'stochastic'")
+    if commit is None and step_state is None and not wait_limit and not selftest and residual_draw in ("inverse_cdf", "gumbel"):
+        r = _lib.host().verify(target_logits, draft_ids, draft_probs, uniforms, u_resample, mode == "stochastic", temperature, tau, bool(return_p_draft),
+                               draft_logits, None if draft_stats is None else draft_stats.vmax, None if draft_stats is None else draft_stats.mass, seed, step,
+                               residual_draw == "gumbel", out, target_vmax, target_mass)
+        if r is not None:
+            return r
     target_logits = _check_logits(target_logits)
     dev = target_logits.device
     if residual_draw not in ("inverse_cdf", "gumbel"):
