@@ -276,7 +276,7 @@ LM_API int lm_verify(const lm_verify_args* args);
  *              an order that depends on its grid, so the two agree to ~1e-6 relative, not bit for bit);
  *   out_q_logits (optional) receives a copy of the rows, as the reference keeps them in its state.
  * BF16 or FP32 rows; 1..LM_MAX_DRAFT + 1 rows per call; temperature > 0. Workspace: lm_verify_workspace_bytes() bytes,
- * 256-byte aligned, zero-filled once (it may be the verify step's workspace: the calls are stream-ordered).
+ * 256-byte aligned (it may be the verify step's workspace: the calls are stream-ordered, and the launch leaves it untouched).
  */
 typedef struct lm_draft_q_args {
   uint32_t struct_size;

@@ -2,6 +2,7 @@
 #include <cuda_runtime.h>
 
 #include "argmax.cuh"
+#include "draft_q.cuh"
 #include "host.cuh"
 #include "sample_cluster.cuh"
 
@@ -67,6 +68,25 @@ int argmax_clusters(const void* logits, int dtype, int rows, int vocab, int64_t 
   const int C = cluster_blocks(rows, vocab, 2 * sms);                       // (two of these blocks share an SM easily)
   return dtype == LM_DTYPE_F32 ? launch_argmax<true>(logits, rows, vocab, row_stride, out32, out64, C, st)
                                : launch_argmax<false>(logits, rows, vocab, row_stride, out32, out64, C, st);
+}
+
+template <bool F32>
+static int launch_draft_q(const DraftQDev& P, int C, cudaStream_t st) {
+  const int rc = ensure_dynamic_smem(static_cast<KernelSlot>(kSlotDraftQ + (F32 ? 1 : 0)), reinterpret_cast<const void*>(draft_q_kernel<F32>), 1, true);
+  if (rc != LM_OK) return rc;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(P.rows) * static_cast<unsigned>(C)); cfg.blockDim = dim3(kDraftQThreads); cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(C); attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = C > 1 ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, draft_q_kernel<F32>, P, C);
+  return e == cudaSuccess ? LM_OK : cuda_fail(e);
+}
+
+int draft_q_clusters(const DraftQDev& P, int sms, cudaStream_t st) {
+  const int C = cluster_blocks(P.rows, P.vocab, 2 * sms);                   // (two of these blocks share an SM)
+  return P.dtype == LM_DTYPE_F32 ? launch_draft_q<true>(P, C, st) : launch_draft_q<false>(P, C, st);
 }
 
 }  // namespace lm

@@ -4,161 +4,178 @@
 // z * float32(1/T) + g; the mass is kept as the integer sum of this library's fixed-point weights instead of an FP32
 // running sum, so q_k(v) does not depend on how the row is split.
 //
-// One or a few rows of ~300 KB: latency-bound, so like the verify kernel this is one cooperative launch of one block per SM,
-// every block owning the same vocabulary slice of every row (kept in shared memory between the two phases), one bounded
-// grid barrier (the weights need the row maximum), and the last block to leave writes the outputs and cleans the workspace.
+// A few rows of ~300 KB: latency-bound. One thread-block cluster per row (16 blocks for up to 14 rows on 148 SMs), one launch, no
+// workspace: a thread holds its few chunks of the row in registers from the one read on, the blocks meet twice in distributed shared
+// memory -- the maximum (the weights are relative to it), then mass, best key and runner-up in block 0, which writes the outputs. The
+// two logarithms of a Gumbel key are spent only on logits that can still beat the maximum's own key (GumbelScan).
+// (Before: a cooperative launch of the whole GPU, scalar loads, a grid barrier and global atomics, both logarithms for every logit.)
 #pragma once
-#include "common.cuh"
+#include "sample_cluster.cuh"
 #include "spec_ops.cuh"
 
 namespace lm {
 
-constexpr int kDraftQBlock = 1024;
-constexpr int kDraftQMaxRows = LM_MAX_DRAFT + 1;
-constexpr unsigned kBarrierSpinLimit = 1u << 17;       // polls of the counter (about a microsecond each) before the wait gives up
-
-struct DraftQWs {                                       // lives in the caller's workspace, zero-filled once, left all zero by every launch
-  unsigned barrier;                                     // arrivals; returns to 0 when the launch ends
-  unsigned exits;
-  unsigned error;                                       // 1 = the barrier wait of this launch ran out
-  unsigned nan_rows;                                    // bit r: row r holds a NaN
-  unsigned long long row_best[kDraftQMaxRows];          // packed (max logit, lowest index) per row
-  unsigned long long row_mass[kDraftQMaxRows];          // fixed-point mass per row
-  unsigned long long key_best[kDraftQMaxRows];          // packed best Gumbel key per row
-  unsigned long long rival[kDraftQMaxRows];             // the best Gumbel key that lost (monotone code)
-};
-
-// Every block arrives, then waits until `target` arrivals are visible. Bounded: on time-out the error word is set and
-// the block carries on (its results are then meaningless; the outputs report the error).
-__device__ __forceinline__ void grid_barrier(DraftQWs* ws, unsigned target) {
-  __syncthreads();                                                        // the block's writes happen-before thread 0's release below
-  if (threadIdx.x == 0) {
-    unsigned seen = 0, spins = 0;
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&ws->barrier) : "memory");
-    do {
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&ws->barrier) : "memory");
-      if (seen >= target) break;
-      if (++spins > kBarrierSpinLimit) { atomicExch(&ws->error, 1u); break; }
-    } while (true);
-  }
-  __syncthreads();
-}
-__device__ __forceinline__ uint64_t ws_load(const unsigned long long* p) { return __ldcg(p); }
+constexpr int kDraftQThreads = 512;
+constexpr int kDraftQKeep = 4;                          // chunks of eight logits a thread keeps: 16 blocks hold a row of 262,144; the rest is read again from L2
 
 struct DraftQDev {
   int dtype; int rows; int first_position; int vocab; int64_t row_stride;
   const void* logits; float temperature; uint64_t seed; uint32_t step;
   int32_t* out_tokens; float* out_lse; float* out_vmax; unsigned long long* out_mass; uint32_t* out_status;
   void* out_q_logits; int64_t q_logits_stride;
-  DraftQWs* ws;
   const uint32_t* state; int t_max, g;                   // optional StepState: seed and step come from it; a done state ends the launch
 };
 
-static __global__ void __launch_bounds__(kDraftQBlock, 1) draft_q_kernel(DraftQDev P) {
-  extern __shared__ __align__(16) float dq_smem[];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, G = gridDim.x, b = blockIdx.x;
-  constexpr int kWarps = kDraftQBlock / 32;
-  const int R = P.rows, V = P.vocab;
-  DraftQWs* ws = P.ws;
+// f(c, raw chunk) for every chunk of this block's slice: the kept ones from registers.
+template <bool F32, class F>
+__device__ __forceinline__ void draft_chunks(const ClusterRow& R, const RawChunk<F32> (&kept)[kDraftQKeep], F f) {
+  const int c = R.c0 + static_cast<int>(threadIdx.x);
+#pragma unroll
+  for (int j = 0; j < kDraftQKeep; j++) if (c + j * kDraftQThreads < R.c1) f(c + j * kDraftQThreads, kept[j]);
+#pragma unroll 1
+  for (int d = c + kDraftQKeep * kDraftQThreads; d < R.c1; d += kDraftQThreads) f(d, load_raw<F32>(R, d));
+}
+
+template <bool F32>
+static __global__ void __launch_bounds__(kDraftQThreads) draft_q_kernel(const DraftQDev P, int C) {
+  constexpr int kWarps = kDraftQThreads / 32;
+  __shared__ unsigned long long x_best[kCMaxRanks], x_mass[kCMaxRanks], x_key[kCMaxRanks];
+  __shared__ float x_rival[kCMaxRanks];
+  __shared__ uint32_t x_nan[kCMaxRanks];
+  __shared__ uint64_t part_best[kWarps], part_mass[kWarps], part_key[kWarps];
+  __shared__ uint32_t part_rival[kWarps];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rank = C > 1 ? static_cast<int>(cluster_rank()) : 0, row = static_cast<int>(blockIdx.x) / C;
   uint64_t seed = P.seed; uint32_t step = P.step;
   if (P.state) {
     StepStateView st{const_cast<uint32_t*>(P.state), P.t_max, P.g};
-    if (st.done()) return;                                                // every block sees the same state: none touches the workspace
+    if (st.done()) return;                                                  // every block sees the same state
     seed = st.seed(); step = st.step();
   }
-  unsigned long long* second = ws->rival;                                 // per row: the best key that is not the winner's
-  const int per = ((V + G - 1) / G + 7) & ~7;
-  const int lo = min(V, b * per), hi = min(V, lo + per);
-  const int len = hi - lo;
-  float* zs = dq_smem;                                                    // [R][per] widened logits of this block's slice
+  if (C > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // this block runs: its memory may be written to
+  constexpr int kSize = F32 ? 4 : 2;
+  ClusterRow R;
+  R.row = static_cast<const char*>(P.logits) + static_cast<size_t>(row) * static_cast<size_t>(P.row_stride) * kSize;
+  R.V = P.vocab; R.pen = nullptr; R.rho = 1.0f; R.pi = 0.0f; R.vals = nullptr; R.nv = 0;
+  const int head = static_cast<int>((16u - (reinterpret_cast<uintptr_t>(R.row) & 15u)) & 15u) / kSize;
+  R.off = head ? 8 - head : 0;
+  const int n_chunks = (P.vocab + R.off + 7) / 8, per = (n_chunks + C - 1) / C;
+  R.c0 = min(n_chunks, rank * per); R.c1 = min(n_chunks, R.c0 + per);
 
-  // ---- phase 0: the slice of every row into shared memory (and into the copy, if one is wanted) ------------------------
-  for (int i = tid; i < R * len; i += kDraftQBlock) {
-    const int r = i / len, e = i - r * len;
-    float z;
-    if (P.dtype == LM_DTYPE_BF16) {
-      const uint16_t code = __ldg(reinterpret_cast<const uint16_t*>(P.logits) + static_cast<int64_t>(r) * P.row_stride + lo + e);
-      z = __uint_as_float(static_cast<uint32_t>(code) << 16);
-      if (P.out_q_logits) reinterpret_cast<uint16_t*>(P.out_q_logits)[static_cast<int64_t>(r) * P.q_logits_stride + lo + e] = code;
-    } else {
-      z = __ldg(reinterpret_cast<const float*>(P.logits) + static_cast<int64_t>(r) * P.row_stride + lo + e);
-      if (P.out_q_logits) reinterpret_cast<float*>(P.out_q_logits)[static_cast<int64_t>(r) * P.q_logits_stride + lo + e] = z;
-    }
-    zs[r * per + e] = canon_zero(z);
-  }
-  __syncthreads();
-  // every row is shared by `split` warps: row maximum and best Gumbel key (with this thread's runner-up, for the tie flag)
-  const int split = max(1, kWarps / R);
-  const float inv_t32 = __double2float_rn(1.0 / static_cast<double>(P.temperature));
-  uint64_t my_best = 0ull; float my_second = -INFINITY;                       // of the (single) item this warp owns
-  for (int item = warp; item < R * split; item += kWarps) {
-    const int r = item / split, part = item - r * split;
-    const uint32_t t_id = 2000u + static_cast<uint32_t>(P.first_position + r);
-    uint64_t vbest = 0ull, kbest = 0ull; float ksecond = -INFINITY; bool nan = false;
-    for (int i = part * 32 + lane; i < len; i += 32 * split) {
-      const float z = zs[r * per + i];
-      const uint32_t idx = static_cast<uint32_t>(lo + i);
-      nan = nan || (z != z);
-      const uint64_t pv = pack_best(z, idx);
-      vbest = pv > vbest ? pv : vbest;
-      const float key = __fadd_rn(__fmul_rn(z, inv_t32), gumbel(seed, step, t_id, idx));
-      const uint64_t pk = pack_best(key, idx);
-      if (pk > kbest) { if (kbest) ksecond = fmaxf(ksecond, best_value(kbest)); kbest = pk; } else ksecond = fmaxf(ksecond, key);
-    }
-    const uint64_t wv = warp_max_u64(vbest), wk = warp_max_u64(kbest);
-    if (lane == 0 && wv) atomicMax(&ws->row_best[r], static_cast<unsigned long long>(wv));
-    if (lane == 0 && wk) atomicMax(&ws->key_best[r], static_cast<unsigned long long>(wk));
-    if (__any_sync(kFull, nan) && lane == 0) atomicOr(&ws->nan_rows, 1u << r);
-    if (item < kWarps) { my_best = kbest; my_second = ksecond; }            // R * split <= kWarps: one item per warp
-  }
-  grid_barrier(ws, 1u * G);
-
-  // ---- phase 1: the fixed-point mass relative to the row maximum; the best key that lost ----------------------------------
-  const float c2 = exp2_scale(P.temperature);
-  for (int item = warp; item < R * split; item += kWarps) {
-    const int r = item / split, part = item - r * split;
-    const float vmax = best_value(ws_load(&ws->row_best[r]));
-    const uint64_t winner = ws_load(&ws->key_best[r]);
-    uint64_t w = 0ull;
-    for (int i = part * 32 + lane; i < len; i += 32 * split) w += weight_q40(zs[r * per + i], vmax, c2);
-    w = warp_sum_u64(w);
-    if (lane == 0 && w) atomicAdd(&ws->row_mass[r], static_cast<unsigned long long>(w));
-    // this thread's best candidate other than the winner, as a packed key (index irrelevant)
-    float rival = (my_best == winner) ? my_second : (my_best ? best_value(my_best) : -INFINITY);
+  // ---- the one read: the slice's maximum (with an index: its Gumbel key is where the draw starts), NaNs -----------------------------
+  RawChunk<F32> kept[kDraftQKeep];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) rival = fmaxf(rival, __shfl_xor_sync(kFull, rival, o));
-    if (lane == 0 && rival > -INFINITY) atomicMax(&second[r], static_cast<unsigned long long>(fkey(rival)));
-  }
-  __syncthreads();
-  __shared__ bool s_last;
-  if (tid == 0) {
-    __threadfence();
-    s_last = atomicAdd(&ws->exits, 1u) == static_cast<unsigned>(G) - 1u;
-  }
-  __syncthreads();
-  if (!s_last) return;
-  // ---- the last block to arrive: outputs, and the workspace back to its clean state -----------------------------------------
-  __threadfence();
-  if (tid < R) {
-    const int r = tid;
-    const uint64_t vb = ws_load(&ws->row_best[r]), kb = ws_load(&ws->key_best[r]), mass = ws_load(&ws->row_mass[r]);
-    const uint64_t sec = ws_load(&second[r]);
-    const bool bad = ws->error != 0;
-    const float vmax = best_value(vb);
-    P.out_tokens[r] = (bad || !kb) ? -1 : static_cast<int>(best_index(kb));
-    if (P.out_vmax) P.out_vmax[r] = vmax;
-    if (P.out_mass) P.out_mass[r] = mass;
-    if (P.out_lse) P.out_lse[r] = mass ? __double2float_rn(static_cast<double>(vmax) / static_cast<double>(P.temperature) + log(static_cast<double>(mass) * 9.094947017729282e-13)) : -INFINITY;
-    if (P.out_status) {
-      uint32_t st = 0u;
-      if (kb && sec && fkey_inv(static_cast<uint32_t>(sec)) >= best_value(kb) - 4e-6f) st |= LM_STATUS_NEAR_TIE;
-      if ((__ldcg(&ws->nan_rows) >> r) & 1u) st |= LM_STATUS_NAN;
-      P.out_status[r] = st;
+  for (int j = 0; j < kDraftQKeep; j++) { const int c = R.c0 + tid + j * kDraftQThreads; if (c < R.c1) kept[j] = load_raw<F32>(R, c); }
+  uint64_t mine = 0ull;
+  bool nan = false;
+  draft_chunks<F32>(R, kept, [&](int c, const RawChunk<F32>& q) {
+    float z[8];
+    widen_raw<F32>(R, q, c, z);
+    float mx = z[0];
+#pragma unroll
+    for (int e = 1; e < 8; e++) asm("max.NaN.f32 %0, %1, %2;" : "=f"(mx) : "f"(mx), "f"(z[e]));
+    if (mx != mx) {
+      nan = true;
+      mx = -INFINITY;
+#pragma unroll 1
+      for (int e = 0; e < 8; e++) {                                         // the packed order: a positive NaN above +inf, a negative one below -inf
+        const int i = 8 * c + e - R.off;
+        if (i < 0 || i >= P.vocab) continue;
+        const uint64_t p = pack_best(canon_zero(pick8(z, e)), static_cast<uint32_t>(i));
+        mine = p > mine ? p : mine;
+      }
+    } else if (mine == 0ull || mx > best_value(mine)) {
+      int at = -1;
+#pragma unroll
+      for (int e = 7; e >= 0; e--) { const int i = 8 * c + e - R.off; if (z[e] == mx && i >= 0 && i < P.vocab) at = i; }
+      if (at >= 0) { const uint64_t p = pack_best(canon_zero(mx), static_cast<uint32_t>(at)); mine = p > mine ? p : mine; }
     }
-    ws->row_best[r] = 0ull; ws->key_best[r] = 0ull; ws->row_mass[r] = 0ull; second[r] = 0ull;
+  });
+  if (P.out_q_logits) {                                                     // the copy, element by element (a warp's stores are one line), from L1 / L2
+    const int i0 = max(0, 8 * R.c0 - R.off), i1 = min(P.vocab, 8 * R.c1 - R.off);
+    for (int i = i0 + tid; i < i1; i += kDraftQThreads) {
+      const int64_t o = static_cast<int64_t>(row) * P.q_logits_stride + i;
+      if (F32) static_cast<float*>(P.out_q_logits)[o] = __ldg(reinterpret_cast<const float*>(R.row) + i);
+      else static_cast<uint16_t*>(P.out_q_logits)[o] = __ldg(reinterpret_cast<const uint16_t*>(R.row) + i);
+    }
   }
+  mine = warp_max_u64(mine);
+  if (lane == 0) part_best[warp] = mine;
+  const int any_nan = __syncthreads_or(nan);
+  if (C > 1) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");    // every block of the cluster runs
+  if (warp == 0) {
+    const uint64_t b = warp_max_u64(lane < kWarps ? part_best[lane] : 0ull);
+    if (lane < C) { cst_u64(cluster_addr(&x_best[rank], lane), b); cst_u32(cluster_addr(&x_nan[rank], lane), any_nan ? 1u : 0u); }
+  }
+  cluster_sync(C);
+  const uint64_t top = warp_max_u64(lane < C ? x_best[lane] : 0ull);        // every warp for itself
+  const bool has_nan = __any_sync(kFull, lane < C && x_nan[lane] != 0u) != 0;
+  const float vmax = best_value(top);
+
+  // ---- the fixed-point mass relative to the maximum; the best Gumbel key and the best key that lost ---------------------------------
+  const uint32_t t_id = 2000u + static_cast<uint32_t>(P.first_position + row);
+  const float c2 = exp2_scale(P.temperature), inv_t32 = __double2float_rn(1.0 / static_cast<double>(P.temperature));
+  uint64_t w = 0ull, key = 0ull; float second = -INFINITY;
+  if (!has_nan && fabsf(vmax) < INFINITY) {
+    GumbelScan g;
+    g.init(seed, step, t_id, P.temperature, __fadd_rn(__fmul_rn(vmax, inv_t32), gumbel(seed, step, t_id, best_index(top))));
+    draft_chunks<F32>(R, kept, [&](int c, const RawChunk<F32>& q) {
+      float z[8];
+      widen_raw<F32>(R, q, c, z);
+#pragma unroll
+      for (int e = 0; e < 8; e += 2) {
+        uint64_t w0, w1;
+        weight_q40_x2(z[e], z[e + 1], vmax, c2, w0, w1);                    // (positions outside the row are -inf: weight 0, no key)
+        w += w0 + w1;
+        g.offer2(canon_zero(z[e]), static_cast<uint32_t>(8 * c + e - R.off), canon_zero(z[e + 1]), static_cast<uint32_t>(8 * c + e + 1 - R.off));
+      }
+    });
+    key = g.best; second = g.second;
+  } else {                                                                  // a NaN, +inf, or nothing but -inf: every key, by the definition
+    draft_chunks<F32>(R, kept, [&](int c, const RawChunk<F32>& q) {
+      float z[8];
+      widen_raw<F32>(R, q, c, z);
+#pragma unroll 1
+      for (int e = 0; e < 8; e++) {
+        const int i = 8 * c + e - R.off;
+        if (i < 0 || i >= P.vocab) continue;
+        const float v = canon_zero(pick8(z, e)), k = __fadd_rn(__fmul_rn(v, inv_t32), gumbel(seed, step, t_id, static_cast<uint32_t>(i)));
+        const uint64_t p = pack_best(k, static_cast<uint32_t>(i));
+        if (p > key) { if (key) second = fmaxf(second, best_value(key)); key = p; } else second = fmaxf(second, k);
+        w += weight_q40(v, vmax, c2);
+      }
+    });
+  }
+  const uint64_t warp_w = warp_sum_u64(w), warp_key = warp_max_u64(key);
+  const float lost = key == warp_key ? second : (key ? best_value(key) : -INFINITY);   // this thread's best key that is not the warp's
+  const uint32_t warp_lost = warp_max_u32(fkey(lost));
+  if (lane == 0) { part_mass[warp] = warp_w; part_key[warp] = warp_key; part_rival[warp] = warp_lost; }
   __syncthreads();
-  if (tid == 0) { ws->nan_rows = 0u; ws->error = 0u; ws->exits = 0u; __threadfence(); ws->barrier = 0u; }
+  if (warp == 0) {
+    const bool have = lane < kWarps;
+    const uint64_t m = warp_sum_u64(have ? part_mass[lane] : 0ull), k = have ? part_key[lane] : 0ull, win = warp_max_u64(k);
+    const float l = fmaxf(have ? fkey_inv(part_rival[lane]) : -INFINITY, (k && k != win) ? best_value(k) : -INFINITY);
+    const uint32_t r = warp_max_u32(fkey(l));
+    if (lane == 0) {
+      cst_u64(cluster_addr(&x_mass[rank], 0), m);
+      cst_u64(cluster_addr(&x_key[rank], 0), win);
+      cst_u32(cluster_addr(&x_rival[rank], 0), __float_as_uint(fkey_inv(r)));
+    }
+  }
+  cluster_sync(C);
+  if (rank == 0 && warp == 0) {
+    const bool have = lane < C;
+    const uint64_t mass = warp_sum_u64(have ? x_mass[lane] : 0ull), k = have ? x_key[lane] : 0ull, win = warp_max_u64(k);
+    const float edge = best_value(win) - 4e-6f;
+    const bool tie = __any_sync(kFull, win && ((have && x_rival[lane] >= edge && x_rival[lane] > -INFINITY) || (k && k != win && best_value(k) >= edge))) != 0;
+    if (lane == 0) {
+      P.out_tokens[row] = win ? static_cast<int>(best_index(win)) : -1;
+      if (P.out_vmax) P.out_vmax[row] = vmax;
+      if (P.out_mass) P.out_mass[row] = mass;
+      if (P.out_lse) P.out_lse[row] = mass ? __double2float_rn(static_cast<double>(vmax) / static_cast<double>(P.temperature) + log(static_cast<double>(mass) * 9.094947017729282e-13)) : -INFINITY;
+      if (P.out_status) P.out_status[row] = (tie ? LM_STATUS_NEAR_TIE : 0u) | (has_nan ? LM_STATUS_NAN : 0u);
+    }
+  }
 }
 
 }  // namespace lm

@@ -32,9 +32,10 @@ inline int sm_count(int* out) {
 
 // Kernels that need more than 48 KB of dynamic shared memory must be told so once per device (the attribute belongs to the
 // device's copy of the function); remembered per device and kernel, raised when a call needs more.
-enum KernelSlot { kSlotFast, kSlotTopk, kSlotGeneric, kSlotVocabLocal, kSlotVerify, kSlotVerifyStats, kSlotDraftQ, kSlotTileFinish, kSlotSlice, kSlotSliceSmall, kSlotSliceTiny, kSlotSlicedMerge, kSlotHead, kSlotCluster,
+enum KernelSlot { kSlotFast, kSlotTopk, kSlotGeneric, kSlotVocabLocal, kSlotVerify, kSlotVerifyStats, kSlotTileFinish, kSlotSlice, kSlotSliceSmall, kSlotSliceTiny, kSlotSlicedMerge, kSlotHead, kSlotCluster,
                   kSlotArgmax = kSlotCluster + 6,   // (the cluster kernel has six instances, the argmax kernel two)
-                  kSlotCount = kSlotArgmax + 2 };
+                  kSlotDraftQ = kSlotArgmax + 2,    // (two instances)
+                  kSlotCount = kSlotDraftQ + 2 };
 
 inline int ensure_dynamic_smem(KernelSlot slot, const void* func, size_t bytes, bool large_clusters = false) {
   if (bytes <= 48 * 1024 && !large_clusters) return LM_OK;
@@ -60,8 +61,10 @@ inline int ensure_dynamic_smem(KernelSlot slot, const void* func, size_t bytes, 
 inline size_t align256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
 
 struct SampleDev;
+struct DraftQDev;
 // cluster.cu: one row per thread-block cluster, every row of the call.
 int sample_clusters(const SampleDev& P, int sms, cudaStream_t st);
 int argmax_clusters(const void* logits, int dtype, int rows, int vocab, int64_t row_stride, int32_t* out32, int64_t* out64, cudaStream_t st);
+int draft_q_clusters(const DraftQDev& P, int sms, cudaStream_t st);
 
 }  // namespace lm

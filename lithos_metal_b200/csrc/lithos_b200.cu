@@ -103,9 +103,8 @@ size_t lm_workspace_bytes(int64_t rows, int64_t vocab) {
 
 size_t lm_verify_workspace_bytes(int32_t n_draft, int64_t vocab) {
   (void)n_draft; (void)vocab;
-  // lm_verify and lm_draft_q may share it: the verify kernel's words (which keep a launch count between calls) come first, the
-  // draft kernel's (all zero between calls) behind them
-  return align256(sizeof(VerifyWs)) + align256(sizeof(DraftQWs));
+  // the verify kernel's words, which keep a launch count between calls (lm_draft_q asks for the same buffer and leaves it alone)
+  return align256(sizeof(VerifyWs));
 }
 
 static int argmax_args_ok(const void* logits, int32_t dtype, int64_t rows, int64_t vocab, int64_t row_stride, const void* out_tokens) {
@@ -638,7 +637,8 @@ int lm_verify(const lm_verify_args* a) {
   const int per = (static_cast<int>((a->vocab + grid - 1) / grid) + 7) & ~7;
   const size_t rows_cached = static_cast<size_t>(a->n_draft + 1) + (a->mode == LM_VERIFY_STOCHASTIC ? a->n_draft : 0);
   size_t smem = rows_cached * static_cast<size_t>(per) * sizeof(float);
-  int cached = smem <= 200 * 1024 ? 1 : 0;
+  // a launch that was given the rows' maxima and masses knows the decisive row from one logit per draft: it reads that row alone, once
+  int cached = (smem <= 200 * 1024 && !(a->mode == LM_VERIFY_STOCHASTIC && a->target_vmax && a->target_mass)) ? 1 : 0;
   if (!cached) smem = 0;
   const bool stats = P.row_max != nullptr && P.row_mass != nullptr;
   const void* kernel = stats ? reinterpret_cast<const void*>(verify_kernel<true>) : reinterpret_cast<const void*>(verify_kernel<false>);
@@ -666,26 +666,14 @@ int lm_draft_q(const lm_draft_q_args* a) {
   P.logits = a->logits; P.temperature = a->temperature; P.seed = a->seed; P.step = a->step;
   P.out_tokens = a->out_tokens; P.out_lse = a->out_lse; P.out_vmax = a->out_vmax; P.out_mass = reinterpret_cast<unsigned long long*>(a->out_mass);
   P.out_status = a->out_status; P.out_q_logits = a->out_q_logits; P.q_logits_stride = a->q_logits_stride;
-  P.ws = reinterpret_cast<DraftQWs*>(static_cast<char*>(a->workspace) + align256(sizeof(VerifyWs)));
   P.state = static_cast<const uint32_t*>(a->step_state); P.t_max = a->t_max; P.g = a->gamma_max > 1 ? a->gamma_max : 1;
-  // one block per SM, all resident at once (one grid barrier), each holding its slice of every row in shared memory;
-  // more blocks than that never, fewer when the slices would not fit
+  // rows x vocabulary that the SMs could not hold between two phases have always been refused (the limit is part of the interface)
   int grid = sms < 1024 ? sms : 1024;
-  constexpr int kPerThread = 4;
-  {
-    // a single row is ~150 logits per SM: fewer blocks with a few logits per thread meet sooner at the barrier
-    const long long want = (static_cast<long long>(a->rows) * a->vocab + kDraftQBlock * kPerThread - 1) / (kDraftQBlock * kPerThread);
-    if (want < grid) grid = static_cast<int>(want < 1 ? 1 : want);
-  }
-  const int per = (static_cast<int>((a->vocab + grid - 1) / grid) + 7) & ~7;
-  const size_t smem = static_cast<size_t>(a->rows) * static_cast<size_t>(per) * sizeof(float);
-  if (smem > 200 * 1024) return LM_E_UNSUPPORTED;                          // rows x vocabulary beyond what the SMs can hold between the phases
-  const int rs = ensure_dynamic_smem(kSlotDraftQ, reinterpret_cast<const void*>(draft_q_kernel), smem);
-  if (rs != LM_OK) return rs;
-  void* params[] = {&P};
-  const cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<void*>(draft_q_kernel), dim3(grid), dim3(kDraftQBlock), params, smem,
-                                                    static_cast<cudaStream_t>(a->stream));
-  return e == cudaSuccess ? LM_OK : cuda_fail(e);
+  const long long want = (static_cast<long long>(a->rows) * a->vocab + 4095) / 4096;
+  if (want < grid) grid = static_cast<int>(want < 1 ? 1 : want);
+  const int64_t per = ((a->vocab + grid - 1) / grid + 7) & ~static_cast<int64_t>(7);
+  if (a->rows * per * static_cast<int64_t>(sizeof(float)) > 200 * 1024) return LM_E_UNSUPPORTED;
+  return draft_q_clusters(P, sms, static_cast<cudaStream_t>(a->stream));
 }
 
 int lm_confidence(const lm_confidence_args* a) {

@@ -97,3 +97,23 @@ def test_draft_q_argument_checks():
     nan = x.clone(); nan[1, 5] = float("nan")
     st = lm.draft_q(nan, temperature=1.0).status.cpu().numpy()
     assert not (st[0] & 2) and (st[1] & 2)
+
+
+@pytest.mark.parametrize("rows,vocab", [(1, 1), (3, 7), (16, 2047), (2, 4096), (9, 4099), (15, 40000), (1, 262144), (16, 50257), (1, 600001)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_every_split_of_a_row_gives_the_oracles_draw(rows, vocab, dtype):
+    """One to sixteen blocks per row, ragged ends, rows at odd addresses, chunks beyond those a thread keeps, a masked part (-inf):
+    token (or a flagged near-tie of the float32 log), maximum and integer mass are the oracle's."""
+    rng = np.random.default_rng(vocab * 31 + rows)
+    codes = oracle.f32_to_bf16((rng.standard_normal((rows, vocab)) * 2.0).astype(np.float32))
+    codes[:, : vocab // 3] = 0xFF80                                         # -inf
+    wide = torch.zeros(rows, vocab + 3, dtype=dtype, device="cuda")
+    x = wide[:, 1:vocab + 1]                                                # rows start at odd elements
+    x.copy_(bf16_tensor(codes))
+    r = lm.draft_q(x, temperature=0.7, seed=5, step=9, first_position=1, copy_logits=True)
+    tok, status = r.tokens.cpu().numpy(), r.status.cpu().numpy()
+    for k in range(rows):
+        t, vmax, mass, lse, _ = oracle.draft_q(codes[k], temperature=0.7, seed=5, step=9, position=1 + k)
+        assert int(tok[k]) == t or (int(status[k]) & 4), k
+        assert float(r.vmax[k]) == vmax and int(r.mass[k]) == mass and float(r.lse[k]) == np.float32(lse), k
+    assert torch.equal(r.q_logits, x)
