@@ -302,14 +302,6 @@ static __device__ void hist_walk(HistSmem& s, uint32_t k_target, double m_target
 }
 
 // ---- the draws -----------------------------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t kept_mask8(const uint4 q, uint32_t tau_code2) {
-  const __nv_bfloat162 t2 = *reinterpret_cast<const __nv_bfloat162*>(&tau_code2);
-  const uint32_t m0 = __hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&q.x), t2), m1 = __hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&q.y), t2);
-  const uint32_t m2 = __hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&q.z), t2), m3 = __hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&q.w), t2);
-  if ((m0 | m1 | m2 | m3) == 0u) return 0u;
-  return (m0 & 1u) | ((m0 >> 15) & 2u) | ((m1 & 1u) << 2) | ((m1 >> 13) & 8u) | ((m2 & 1u) << 4) | ((m2 >> 11) & 32u) | ((m3 & 1u) << 6) | ((m3 >> 9) & 128u);
-}
-
 // 8-bit mask of the logits of a chunk whose BF16 code equals `code` (zero = true: whose value is zero, either sign).
 __device__ __forceinline__ uint32_t equal_mask8(const uint4 q, uint32_t code2, bool zero) {
   const uint32_t strip = zero ? 0x7FFF7FFFu : 0xFFFFFFFFu;

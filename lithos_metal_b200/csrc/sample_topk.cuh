@@ -47,7 +47,7 @@ struct TopkSmem {
     uint32_t side_id[kTopkHist];           // before either: the distinct history ids
   };
   uint32_t pen[kTopkMaxVocab / 32];        // bitmap of the row's distinct history ids
-  uint32_t hitlist[2048];                  // (chunk << 8 | 8-bit mask) of the chunks that hold a logit >= cutoff
+  uint32_t hitlist[2048];                  // the chunks that hold a logit >= cutoff
   uint32_t bins[kTopkBins];                // candidates per BF16 code, relative to the cutoff code
   uint32_t off[kTopkBins];                 // candidates in the bins above each bin
   uint64_t scratch[32];
@@ -241,6 +241,10 @@ static __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem&
       const uint32_t key = warp_max_u32(fkey(fmaxf(__low2float(mx), __high2float(mx))));
       if (lane == 0) atomicMax(&c.ref_key, key);
     }
+    // A few candidates more than wanted cost less than another round: a cut is good enough at twice the count wanted while that is small (the
+    // list has room for 2048 candidates), at half as much again in between; a large top_k gets the closest cut.
+    const uint32_t enough = want < 24u ? 2u * want : want < 48u ? want + want / 2u : want;
+    uint32_t n_lo = 0xFFFFFFFFu;                                            // count(sample >= lo), once it is known
     uint32_t lo = 0x0000u, hi = 0x7F7Fu;                                    // invariant: count(sample >= lo) >= want, or lo is still 0 (handed back below)
     const uint32_t prev = c.prev_cut[cls];
     uint32_t n3[3];
@@ -248,21 +252,21 @@ static __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem&
       const uint32_t blo = max(prev, 0x0090u) - 16u, bhi = min(prev + 15u, 0x7F7Eu), mid = (blo + bhi + 1u) >> 1;
       count3(blo, mid, bhi + 1u, n3);
       if (n3[0] < want) hi = blo - 1u;
-      else if (n3[2] >= want) lo = bhi + 1u;
-      else if (n3[1] >= want) { lo = mid; hi = bhi; }
-      else { lo = blo; hi = mid - 1u; }
+      else if (n3[2] >= want) { lo = bhi + 1u; n_lo = n3[2]; }
+      else if (n3[1] >= want) { lo = mid; hi = bhi; n_lo = n3[1]; }
+      else { lo = blo; hi = mid - 1u; n_lo = n3[0]; }
     }
-    while (lo < hi && probe + 3 <= kMaxProbes) {                            // three cuts per round: the range shrinks fourfold
+    while (lo < hi && n_lo > enough && probe + 3 <= kMaxProbes) {          // three cuts per round: the range shrinks fourfold
       const uint32_t span = hi - lo;
       const uint32_t q1 = lo + (span + 3u) / 4u, q2 = lo + (2u * span + 3u) / 4u, q3 = lo + (3u * span + 3u) / 4u;   // lo < q1 <= q2 <= q3 <= hi
       count3(q1, q2, q3, n3);
-      if (n3[2] >= want) lo = q3;
-      else if (n3[1] >= want) { lo = q2; hi = q3 - 1u; }
-      else if (n3[0] >= want) { lo = q1; hi = q2 - 1u; }
+      if (n3[2] >= want) { lo = q3; n_lo = n3[2]; }
+      else if (n3[1] >= want) { lo = q2; hi = q3 - 1u; n_lo = n3[1]; }
+      else if (n3[0] >= want) { lo = q1; hi = q2 - 1u; n_lo = n3[0]; }
       else hi = q1 - 1u;
     }
     cut_code = lo;
-    if (cut_code < 0x0080u || lo < hi) { cp_async_wait<0>(); return false; }   // fewer positive logits than candidates wanted: not this kernel's row
+    if (cut_code < 0x0080u || (lo < hi && n_lo > enough)) { cp_async_wait<0>(); return false; }   // fewer positive logits than candidates wanted: not this kernel's row
                                                                             // (the copies in flight must land before the slots are used again)
     if (tid == 0) c.prev_cut[cls] = cut_code;
   }
@@ -273,12 +277,17 @@ static __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem&
   const float nb = -M * c2a;
   float2 sacc = make_float2(0.0f, 0.0f);
   uint32_t nan_seen = 0u;
+  // A bit per step: this thread's chunk held a logit >= cutoff. The list of those chunks is written behind the pass, one reservation per
+  // warp: nearly every step some lane has one, and a reservation per step was a quarter of the pass's instructions (4096 penalised rows, three in four with a top_k:
+  // 857 -> 797 us; 64 rows of 262,144, top_k 50: 51 -> 45).
+  static_assert(kTopkMaxVocab / kChunk <= 64 * kTB, "a bit for every step");
+  unsigned long long hits = 0ull;
   {
     const uint32_t cut2 = cut_code | (cut_code << 16);
     const __nv_bfloat162 t2 = *reinterpret_cast<const __nv_bfloat162*>(&cut2);
     const uint4 pad = make_uint4(0xFF80FF80u, 0xFF80FF80u, 0xFF80FF80u, 0xFF80FF80u);   // -inf
 #pragma unroll 4
-    for (int it = 0; it < n_it; it++) {                                     // uniform trip count: warp votes inside
+    for (int it = 0; it < n_it; it++) {
       {
         const int ahead = it + kStages - 1, ca = ahead * kTB + tid;         // refill the slot read one step ago
         if (ca < n_chunks) cp_async16(&c.ring[ahead % kStages][tid], p4 + ca);
@@ -286,24 +295,11 @@ static __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem&
       }
       cp_async_wait<kStages - 1>();                                         // this step's chunk has landed
       const int cc = it * kTB + tid;
-      const bool live = cc < n_chunks;                                      // warp-uniform control flow below: votes inside
-      const uint4 q = live ? c.ring[it % kStages][tid] : pad;
+      const uint4 q = cc < n_chunks ? c.ring[it % kStages][tid] : pad;
       const uint32_t w[4] = {q.x, q.y, q.z, q.w};
       const uint32_t m0 = __hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&w[0]), t2), m1 = __hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&w[1]), t2);
       const uint32_t m2 = __hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&w[2]), t2), m3 = __hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&w[3]), t2);
-      const bool hit = live && (m0 | m1 | m2 | m3) != 0u;
-      const uint32_t votes = __ballot_sync(kFull, hit);
-      if (votes) {                                                          // one reservation per warp for all its hit chunks
-        uint32_t base = 0u;
-        if (lane == 0) base = atomicAdd(&c.n_hit, __popc(votes));
-        base = __shfl_sync(kFull, base, 0);
-        if (hit) {
-          const uint32_t mask = (m0 & 1u) | ((m0 >> 15) & 2u) | ((m1 & 1u) << 2) | ((m1 >> 13) & 8u) | ((m2 & 1u) << 4) | ((m2 >> 11) & 32u) |
-                                ((m3 & 1u) << 6) | ((m3 >> 9) & 128u);
-          const uint32_t slot = base + __popc(votes & ((1u << lane) - 1u));
-          if (slot < 2048u) c.hitlist[slot] = (static_cast<uint32_t>(cc) << 8) | mask;
-        }
-      }
+      hits = (hits << 1) | ((m0 | m1 | m2 | m3) != 0u ? 1ull : 0ull);       // (the padding is below every cutoff)
       if (need_z) {                                                         // (the padding is -inf: weight 0; a NaN or +inf logit poisons the sum)
 #pragma unroll
         for (int k = 0; k < 4; k++) {                                         // two logits per packed multiply-add and per packed add
@@ -318,6 +314,11 @@ static __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem&
       }
     }
     cp_async_wait<0>();
+  }
+  {
+    uint32_t slot = warp_reserve(&c.n_hit, static_cast<uint32_t>(__popcll(hits)));
+    for (unsigned long long m = hits; m; m &= m - 1ull, slot++)
+      if (slot < 2048u) c.hitlist[slot] = static_cast<uint32_t>((n_it - __ffsll(static_cast<long long>(m))) * kTB + tid);
   }
   // a NaN or +inf logit (or a logit far above the sampled maximum) has made this thread's sum NaN or infinite: the exact path
   // takes such rows and reports them
@@ -351,14 +352,12 @@ static __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem&
     for (int j = 0; j < kExpand; j++) {
       const uint32_t e = e0 + j * kTB + tid;
       ents[j] = (e < n_hit) ? c.hitlist[e] : 0u;
-      qq[j] = (e < n_hit) ? __ldg(p4 + (ents[j] >> 8)) : make_uint4(0u, 0u, 0u, 0u);
+      qq[j] = (e < n_hit) ? __ldg(p4 + ents[j]) : make_uint4(0u, 0u, 0u, 0u);   // (zeros: below every cutoff)
     }
 #pragma unroll
     for (int j = 0; j < kExpand; j++) {
       if (e0 + j * kTB >= n_hit) break;                                     // block-uniform
-      const uint32_t ent = ents[j];
-      uint32_t mask = ent & 0xFFu;
-      const uint32_t cc = ent >> 8;
+      const uint32_t cc = ents[j], mask = kept_mask8(qq[j], cut_code | (cut_code << 16));
       const uint32_t keep = pen_on ? mask & ~((c.pen[cc >> 2] >> ((cc & 3u) * 8u)) & 0xFFu) : mask;   // penalised positions come from the list
       uint32_t slot = warp_reserve(&c.n, __popc(keep));
       for (uint32_t m = keep; m; m &= m - 1u) {                             // usually one bit
