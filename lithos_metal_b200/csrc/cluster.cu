@@ -8,10 +8,26 @@
 
 namespace lm {
 
-// Blocks per row of the cluster kernels: as many as keep every SM busy (16 needs an opt-in; seven such clusters of blocks with an SM
-// each are resident at once, fifteen of eight), slices of at least 2048 logits.
-static int cluster_blocks(int64_t rows, int64_t vocab, int sms) {
-  int c = rows * 20 <= sms ? 16 : rows * 8 <= sms ? 8 : rows * 4 <= sms ? 4 : rows * 2 <= sms ? 2 : 1;
+// Blocks per row of the argmax and the draft draw: as many as keep `slots` places busy (16 needs an opt-in), slices of at least 2048 logits.
+static int cluster_blocks(int64_t rows, int64_t vocab, int slots) {
+  int c = rows * 20 <= slots ? 16 : rows * 8 <= slots ? 8 : rows * 4 <= slots ? 4 : rows * 2 <= slots ? 2 : 1;
+  while (c > 1 && vocab < 2048LL * c) c >>= 1;
+  return c;
+}
+
+// Blocks per row of the sampler. A cluster lies within one group of 16 to 18 SMs, so with a block per SM 148 SMs hold seven clusters of 16,
+// fifteen of 8 and thirty-two of 4 at once, and one row more waits for a second round (16 rows of 151,936, top_k 20: 41 us with 8 blocks
+// each, 29 us with 4). Beyond that the blocks share SMs, and a row without a top_k takes several times as long as one with: smaller pieces
+// even that out where the slices stay long (binary32 rows with mixed knobs, us with 1 / 2 / 4 blocks: 96 rows of 151,936 198 / 184 / 126,
+// 96 of 65,536 96 / 78 / 87, 400 of 50,257 193 / 175 / 280, 400 of 24,576 119 / 136 / 243). `listed`: every row has a top_k and a short list.
+static int sample_blocks(int64_t rows, int64_t vocab, int sms, bool listed) {
+  int c = 1;
+  if (rows * 20 <= sms) c = 16;
+  else if (rows * 48 <= 5LL * sms) c = 8;
+  else if (rows * 9 <= 2LL * sms) c = 4;
+  else if (!listed && rows <= 2LL * sms && vocab >= (rows * 3 <= sms ? 49152 : 98304)) c = 4;
+  else if (rows * 2 <= sms) c = 2;
+  else if (listed ? rows <= 2LL * sms && vocab >= 65536 : rows * 3 <= 2LL * sms || (rows <= 3LL * sms && vocab >= 40000)) c = 2;
   while (c > 1 && vocab < 2048LL * c) c >>= 1;
   return c;
 }
@@ -32,7 +48,7 @@ static int launch_cluster(const SampleDev& P, int C, size_t smem, int instance, 
 }
 
 int sample_clusters(const SampleDev& P, int sms, cudaStream_t st) {
-  const int C = cluster_blocks(P.rows, P.vocab, sms);
+  const int C = sample_blocks(P.rows, P.vocab, sms, P.top_k == nullptr && P.top_k_s >= 1 && P.top_k_s <= kCListK && !(P.flags & LM_FLAG_EXACT_ONLY));
   const size_t per = (static_cast<size_t>((P.vocab + 14) / 8) + C - 1) / C;    // chunks of a slice, for any alignment of the row
   const bool pen = P.history != nullptr && P.hist_len > 0;
   const size_t head = cluster_smem_head(), marks = pen ? (per + 15) / 16 * 16 : 0;

@@ -230,6 +230,17 @@ __device__ __forceinline__ void bin_add_u64(uint32_t* lo, uint32_t* hi, uint32_t
   if (wl) { const uint32_t old = atomicAdd(&lo[b], wl); wh += (old + wl < old) ? 1u : 0u; }
   if (wh) atomicAdd(&hi[b], wh);
 }
+// Four at once: the low words' replies (the carries) are all awaited together, one trip to the shared memory's atomic unit instead of four.
+__device__ __forceinline__ void bin_add4_u64(uint32_t* lo, uint32_t* hi, const uint32_t (&b)[4], const uint64_t (&w)[4]) {
+  uint32_t old[4];
+#pragma unroll
+  for (int e = 0; e < 4; e++) { const uint32_t wl = static_cast<uint32_t>(w[e]); old[e] = 0u; if (wl) old[e] = atomicAdd(&lo[b[e]], wl); }
+#pragma unroll
+  for (int e = 0; e < 4; e++) {
+    const uint32_t wl = static_cast<uint32_t>(w[e]), wh = static_cast<uint32_t>(w[e] >> 32) + (old[e] + wl < old[e] ? 1u : 0u);
+    if (wh) atomicAdd(&hi[b[e]], wh);
+  }
+}
 
 // ---- Gumbel keys, the two logarithms only where they can matter --------------------------------------------------------------------
 // key = z / T + g, g = -ln(-ln u), u = (h + 1/2) / 2^23 from 23 bits of the hash. key >= B needs -ln u <= exp(z / T - B), and 1 - u <=
@@ -643,31 +654,47 @@ static __device__ __noinline__ void sweep_bins(ClusterSmem& s, uint32_t kinds) {
     const float deep = 31.0f * s.T;                                         // logits this far below the maximum: their fixed-point softmass is 0
     sweep<F32, CACHED>(R, [&](int, const float (&z)[8]) {
 #pragma unroll
-      for (int e = 0; e < 8; e++) {
-        if (!(z[e] > -INFINITY)) continue;
-        const uint32_t b = bins.coarse(z[e]);
-        if (use_cnt) atomicAdd(&s.cnt[b], 1u);
-        if (use_w) { const uint64_t w = weight_q40(z[e], vmax, c2); if (w) bin_add_u64(s.lo[1], s.hi[1], b, w); }
-        if (vmax - z[e] < deep) {
-          const double2 t = s.bin_exp[b];
-          const double d = (static_cast<double>(z[e]) - vmax64) - t.y;
-          bin_add_u64(s.lo[0], s.hi[0], b, fixed43(t.x * __fma_rn(__fma_rn(__fma_rn(__fma_rn(a4, d, a3), d, a2), d, inv_t), d, 1.0)));
+      for (int h = 0; h < 8; h += 4) {
+        uint32_t b[4]; uint64_t m[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+          const float v = z[h + e];
+          b[e] = bins.coarse(v);
+          const double2 t = s.bin_exp[b[e]];
+          const double d = (static_cast<double>(v) - vmax64) - t.y;
+          m[e] = fixed43(t.x * __fma_rn(__fma_rn(__fma_rn(__fma_rn(a4, d, a3), d, a2), d, inv_t), d, 1.0));
+          if (!(vmax - v < deep)) m[e] = 0ull;                              // (also -inf, whose polynomial means nothing)
         }
+        if (use_cnt) {
+#pragma unroll
+          for (int e = 0; e < 4; e++) if (z[h + e] > -INFINITY) atomicAdd(&s.cnt[b[e]], 1u);
+        }
+        if (use_w) {
+          uint64_t w[4];
+          weight_q40_x2(z[h], z[h + 1], vmax, c2, w[0], w[1]);
+          weight_q40_x2(z[h + 2], z[h + 3], vmax, c2, w[2], w[3]);
+          bin_add4_u64(s.lo[1], s.hi[1], b, w);
+        }
+        bin_add4_u64(s.lo[0], s.hi[0], b, m);
       }
     });
     return;
   }
   sweep<F32, CACHED>(R, [&](int, const float (&z)[8]) {
 #pragma unroll
-    for (int e = 0; e < 8; e += 2) {
-      const uint32_t b0 = bins.coarse(z[e]), b1 = bins.coarse(z[e + 1]);
-      const bool in0 = z[e] > -INFINITY, in1 = z[e + 1] > -INFINITY;
-      if (use_cnt) { if (in0) atomicAdd(&s.cnt[b0], 1u); if (in1) atomicAdd(&s.cnt[b1], 1u); }
+    for (int h = 0; h < 8; h += 4) {
+      uint32_t b[4];
+#pragma unroll
+      for (int e = 0; e < 4; e++) b[e] = bins.coarse(z[h + e]);
+      if (use_cnt) {
+#pragma unroll
+        for (int e = 0; e < 4; e++) if (z[h + e] > -INFINITY) atomicAdd(&s.cnt[b[e]], 1u);
+      }
       if (use_w) {
-        uint64_t w0, w1;
-        weight_q40_x2(z[e], z[e + 1], vmax, c2, w0, w1);
-        if (in0 && w0) bin_add_u64(s.lo[1], s.hi[1], b0, w0);
-        if (in1 && w1) bin_add_u64(s.lo[1], s.hi[1], b1, w1);
+        uint64_t w[4];
+        weight_q40_x2(z[h], z[h + 1], vmax, c2, w[0], w[1]);                // (-inf: weight 0)
+        weight_q40_x2(z[h + 2], z[h + 3], vmax, c2, w[2], w[3]);
+        bin_add4_u64(s.lo[1], s.hi[1], b, w);
       }
     }
   });

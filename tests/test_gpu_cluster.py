@@ -127,3 +127,13 @@ def test_a_top_p_boundary_inside_the_error_bound_is_decided_in_fp64():
         for k in (0, 1000):
             knobs = dict(temperature=1.0, top_k=np.full(n, k, np.int32), top_p=np.array(rows, np.float32), min_p=0.0)
             _check(_tensor(host), host, knobs, draw="inverse_cdf")
+
+
+# the edges of the rule for the blocks per row on 148 SMs (16 / 8 / 4 / 2 / 1 of them), by rows and by the length of a row
+@pytest.mark.parametrize("rows,vocab", [(7, 33001), (15, 33001), (16, 33001), (32, 20011), (33, 49153), (49, 49153), (50, 98305), (75, 98305), (98, 20011), (99, 40001), (297, 40001)])
+@pytest.mark.parametrize("draw", ["inverse_cdf", "gumbel"])
+def test_every_split_of_a_batch(rows, vocab, draw):
+    rng = np.random.default_rng(rows + vocab)
+    host = (rng.standard_normal((rows, vocab)) * 2).astype(np.float32)
+    _check(_tensor(host), host, _mixed(rng, rows), draw=draw)
+    _check(_tensor(host), host, dict(temperature=0.8, top_k=30, top_p=0.9, min_p=0.0), draw=draw)   # one top_k for every row
