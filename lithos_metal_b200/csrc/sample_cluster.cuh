@@ -242,52 +242,6 @@ __device__ __forceinline__ void bin_add4_u64(uint32_t* lo, uint32_t* hi, const u
   }
 }
 
-// ---- Gumbel keys, the two logarithms only where they can matter --------------------------------------------------------------------
-// key = z / T + g, g = -ln(-ln u), u = (h + 1/2) / 2^23 from 23 bits of the hash. key >= B needs -ln u <= exp(z / T - B), and 1 - u <=
-// -ln u: a logit with (2^23 - h) > 2^23 exp(z / T - B) + 1 cannot reach B. One hash and one ex2 per logit decide that; the few that pass
-// get the exact key. B is a key already seen, less the 4e-6 of the near-tie flag and the rounding of the test itself (kSlack).
-struct GumbelScan {
-  unsigned long long base; float inv_t32, c, kb; uint64_t best; float second;
-  __device__ __forceinline__ void init(uint64_t seed, uint32_t step, uint32_t t_id, float T, float key0) {
-    base = seed + static_cast<uint64_t>(step) * 0x9E3779B97F4A7C15ull + static_cast<uint64_t>(t_id) * 0xC2B2AE3D27D4EB4Full;
-    inv_t32 = __double2float_rn(1.0 / static_cast<double>(T));
-    c = 1.44269504f * inv_t32;
-    best = 0ull; second = -INFINITY; kb = INFINITY;
-    raise(key0);
-  }
-  __device__ __forceinline__ void raise(float key) {                        // |z c|, |B| 1.44 up to 2^k round to 2^(k-24): far below the slack
-    const float b2 = key * 1.44269504f;
-    kb = fminf(kb, (23.0f + 0.02f + fabsf(b2) * 4e-6f) - b2);
-  }
-  __device__ __forceinline__ uint32_t bits(uint32_t i) const {
-    uint64_t x = base + static_cast<uint64_t>(i) * 0x165667B19E3779F9ull;
-    x ^= x >> 30; x *= 0xBF58476D1CE4E5B9ull; x ^= x >> 27; x *= 0x94D049BB133111EBull; x ^= x >> 31;
-    return static_cast<uint32_t>(x >> 41) & 0x7FFFFFu;
-  }
-  // 2^23 exp(z / T - B) + 1: a logit whose 2^23 - h is larger cannot reach B
-  __device__ __forceinline__ bool within(float z, uint32_t h) const {
-    return 16777216.0f - __uint_as_float(0x4B000000u | h) <= ex2_approx(__fmaf_rn(z, c, kb)) + 1.0f;
-  }
-  __device__ __forceinline__ void take(float z, uint32_t i, uint32_t h) {
-    const float u = (static_cast<float>(h) + 0.5f) * (1.0f / 8388608.0f);
-    const float key = __fadd_rn(__fmul_rn(z, inv_t32), -logf(-logf(u)));
-    const uint64_t p = pack_best(key, i);
-    if (p > best) { if (best) second = fmaxf(second, best_value(best)); best = p; raise(key); } else second = fmaxf(second, key);
-  }
-  // two logits at once (their hashes are independent chains); z = -inf: none
-  __device__ __forceinline__ void offer2(float z0, uint32_t i0, float z1, uint32_t i1) {
-    const uint32_t h0 = bits(i0), h1 = bits(i1);
-    bool first = within(z0, h0) && z0 > -INFINITY;
-    const bool second_too = within(z1, h1) && z1 > -INFINITY;
-#pragma unroll 1
-    for (bool more = first || second_too; more;) {                          // (the logarithms' code once)
-      take(first ? z0 : z1, first ? i0 : i1, first ? h0 : h1);
-      more = first && second_too;
-      first = false;
-    }
-  }
-};
-
 // ---- block-wide reductions whose second stage is one warp's (a shuffle costs every warp that issues it: one per cycle and SM) ---------
 __device__ __forceinline__ double cblock_sum_f64(double v, uint64_t* scratch) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;

@@ -70,7 +70,7 @@ struct HistSmem {
   int sel_g, last_g;
   uint32_t base_c; double base_m;
   float res_tau; uint32_t res_cum_c; double res_cum_m, res_excl_m;
-  int token;
+  int token; uint32_t key_bound;
   // followed by the bitmap of the row's distinct history ids: (vocab + 127) / 128 * 16 bytes
 };
 
@@ -513,19 +513,23 @@ static __device__ int hist_draw_inverse_cdf(const SampleDev& P, HistSmem& s, con
 
 // The Gumbel-max draw over the kept set (monolith/nn/sampling_ref.py:55-62; kernels/common/sample.metal:164-198): the sweeps
 // skip the penalised positions (bitmap), whose values come from the list afterwards. *near_tie: another key within 4e-6 of the
-// winner's. Every thread calls; every thread gets the token.
+// winner's. Every thread calls; every thread gets the token. The best key of any thread so far (s.key_bound) is every thread's bound: after
+// its first chunk a thread spends a hash on a logit and the two logarithms on next to none.
 static __device__ int hist_draw_gumbel(const SampleDev& P, HistSmem& s, const uint32_t* pen, const uint16_t* rowp, int n_chunks, float tau, float T, uint32_t t_id, bool* near_tie) {
   const int tid = threadIdx.x;
-  const float inv_t32 = __double2float_rn(1.0 / static_cast<double>(T));
   const uint32_t tc = hceil_code(tau), tau2 = tc | (tc << 16);
   const uint4* p4 = reinterpret_cast<const uint4*>(rowp);
-  uint64_t b1 = 0ull; float second = -INFINITY;
-  auto offer = [&](float z, uint32_t i) {
-    const float key = __fadd_rn(__fmul_rn(z, inv_t32), gumbel(P.seed, P.step, t_id, i));
-    const uint64_t p = pack_best(key, i);
-    if (p > b1) { if (b1) second = fmaxf(second, best_value(b1)); b1 = p; } else second = fmaxf(second, key);
+  GumbelScan g;
+  g.init(P.seed, P.step, t_id, T, -INFINITY);
+  uint32_t told = 0u;                                                       // the best key this thread has made known, or knows of
+  auto share = [&]() {
+    const uint32_t mine = static_cast<uint32_t>(g.best >> 32);              // (a packed key's upper half is its monotone code)
+    if (mine > told) { atomicMax(&s.key_bound, mine); told = mine; }
+    const uint32_t b = *const_cast<volatile uint32_t*>(&s.key_bound);
+    if (b > told) { told = b; g.raise(fkey_inv(b)); }
   };
-  constexpr int kU = 4;
+  constexpr int kU = 2;
+#pragma unroll 1
   for (int c0 = tid; c0 < n_chunks; c0 += kHB * kU) {
     uint4 q[kU];
 #pragma unroll
@@ -539,14 +543,17 @@ static __device__ int hist_draw_gumbel(const SampleDev& P, HistSmem& s, const ui
       if (!mask) continue;
       const uint32_t words[4] = {q[j].x, q[j].y, q[j].z, q[j].w};
 #pragma unroll
-      for (int e = 0; e < kChunk; e++) if ((mask >> e) & 1u)
-        offer(canon_zero((e & 1) ? bf16_hi(words[e >> 1]) : bf16_lo(words[e >> 1])), static_cast<uint32_t>(c * kChunk + e));
+      for (int k = 0; k < 4; k++, mask >>= 2)
+        if (mask & 3u) g.offer2((mask & 1u) ? canon_zero(bf16_lo(words[k])) : -INFINITY, static_cast<uint32_t>(c * kChunk + 2 * k),
+                                (mask & 2u) ? canon_zero(bf16_hi(words[k])) : -INFINITY, static_cast<uint32_t>(c * kChunk + 2 * k + 1));
+      share();
     }
   }
   for (uint32_t i = tid; i < s.n_side; i += kHB) {
     const float v = penalised_value(s.side_raw[i], P.rho, P.pi);
-    if (v >= tau) offer(v, s.ids[i]);
+    if (v >= tau) g.offer2(v, s.ids[i], -INFINITY, 0u);
   }
+  const uint64_t b1 = g.best; const float second = g.second;
   const uint64_t win = block_max_u64(b1, s.scratch);
   bool tie = false; int token = -1;
   if (win) {
@@ -590,7 +597,7 @@ static __device__ void sample_row_hist(const SampleDev& P, int row, int next, Hi
 
   // ---- phase 0: clear; the history's distinct ids as a bitmap and as a list -------------------------------------------------
   const bool stochastic = T > 0.0f;
-  if (tid == 0) { s.n_side = 0u; s.n_b = 0u; s.cz = 0u; s.cninf = 0u; s.pz = 0u; s.pninf = 0u; s.oob = 0u; s.top_pos = 0xFFFFFFFFu; s.token = -1; }
+  if (tid == 0) { s.n_side = 0u; s.n_b = 0u; s.cz = 0u; s.cninf = 0u; s.pz = 0u; s.pninf = 0u; s.oob = 0u; s.top_pos = 0xFFFFFFFFu; s.token = -1; s.key_bound = 0u; }
   if (stochastic) {
     const uint4 z4 = make_uint4(0u, 0u, 0u, 0u);
     uint4* h4 = reinterpret_cast<uint4*>(s.hist);

@@ -137,3 +137,16 @@ def test_every_split_of_a_batch(rows, vocab, draw):
     host = (rng.standard_normal((rows, vocab)) * 2).astype(np.float32)
     _check(_tensor(host), host, _mixed(rng, rows), draw=draw)
     _check(_tensor(host), host, dict(temperature=0.8, top_k=30, top_p=0.9, min_p=0.0), draw=draw)   # one top_k for every row
+
+
+# BF16 rows that the streaming kernels take: a row per SM, two, more, and enough for one kernel behind the other
+@pytest.mark.parametrize("rows", [38, 148, 149, 296, 297, 741])
+@pytest.mark.parametrize("draw", ["inverse_cdf", "gumbel"])
+@pytest.mark.parametrize("penalised", [False, True])
+def test_streaming_batches_of_every_geometry(rows, draw, penalised):
+    vocab = 32776                                                           # the last chunk of a step is alone
+    rng = np.random.default_rng(rows)
+    host = oracle.f32_to_bf16((rng.standard_normal((rows, vocab)) * 2).astype(np.float32))
+    kw = dict(history=rng.integers(0, vocab, (rows, 700)).astype(np.int32), rho=1.1, pi=0.5) if penalised else {}
+    _check(_tensor(host), host, _mixed(rng, rows, (0, 0, 20, 50, 1000)), draw=draw, **kw)
+    _check(_tensor(host), host, dict(temperature=0.9, top_k=0, top_p=0.9, min_p=0.0), draw=draw, **kw)
