@@ -911,7 +911,8 @@ static __device__ void sample_row_hist(const SampleDev& P, int row, int next, Hi
 // stride; a block always holds the item after its current one too, so that it can pull that row's history into L2 while it
 // works. With a row list (written by the top-k kernel: the rows it left) the items are entries of the list, without one they
 // are the rows themselves.
-static __global__ void __launch_bounds__(kHB, 2) sample_hist_kernel(SampleDev P, const int* list, const int* n_list, int* next_item, int* redo, int* n_redo) {
+static __global__ void __launch_bounds__(kHB, 2) sample_hist_kernel(SampleDev P, const int* list, const int* n_list, int* next_item, int* redo, int* n_redo,
+                                                                     const int* left, const int* n_left, int* next_left) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   HistSmem& s = *reinterpret_cast<HistSmem*>(smem_raw);
   uint32_t* pen = reinterpret_cast<uint32_t*>(smem_raw + ((sizeof(HistSmem) + 15) & ~static_cast<size_t>(15)));
@@ -920,24 +921,33 @@ static __global__ void __launch_bounds__(kHB, 2) sample_hist_kernel(SampleDev P,
   // reads nothing this kernel writes) may take every SM a block of this grid has left, instead of waiting for the whole grid.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   apply_step_state(P);
-  const int n = list ? min(*n_list, P.rows) : P.rows;
-  // many items per block: hold the next item too and claim the one after it at the start of a row (the counter's round trip
-  // hides behind the row); few items per block: claim an item only when it is needed, so that no block sits on work
-  const bool ahead = n >= 4 * static_cast<int>(gridDim.x);
-  if (threadIdx.x == 0) { item[0] = atomicAdd(next_item, 1); item[1] = (ahead && item[0] < n) ? atomicAdd(next_item, 1) : n; }
-  __syncthreads();
-  for (;;) {
-    const int i = item[0], in = item[1];
-    if (i >= n) break;
-    int fetched = n;
-    if (threadIdx.x == 0 && in < n) fetched = atomicAdd(next_item, 1);
-    const int row = list ? list[i] : i;
-    int next = in < n ? (list ? list[in] : in) : -1;
-    if (next >= P.rows) next = -1;
-    if (row >= 0 && row < P.rows) sample_row_hist(P, row, next, s, pen, redo, n_redo);   // (a list entry is a row index by construction)
+#pragma unroll 1
+  for (int pass = 0; pass < 2; pass++) {
+    // Launched that way itself, behind the top-k kernel, this grid works on its own rows first and meets that grid's end here: the rows it
+    // handed on are complete then, and the stream takes the end of this grid for the end of both.
+    if (pass == 1) { asm volatile("griddepcontrol.wait;" ::: "memory"); if (left == nullptr) break; }
+    const int* rows = pass ? left : list;
+    int* next_row = pass ? next_left : next_item;
+    const int n = rows ? min(*(pass ? n_left : n_list), P.rows) : P.rows;
+    // many items per block: hold the next item too and claim the one after it at the start of a row (the counter's round trip
+    // hides behind the row); few items per block: claim an item only when it is needed, so that no block sits on work
+    const bool ahead = n >= 4 * static_cast<int>(gridDim.x);
+    if (threadIdx.x == 0) { item[0] = atomicAdd(next_row, 1); item[1] = (ahead && item[0] < n) ? atomicAdd(next_row, 1) : n; }
     __syncthreads();
-    if (threadIdx.x == 0) { item[0] = ahead ? in : atomicAdd(next_item, 1); item[1] = fetched; }
-    __syncthreads();
+    for (;;) {
+      const int i = item[0], in = item[1];
+      if (i >= n) break;
+      int fetched = n;
+      if (threadIdx.x == 0 && in < n) fetched = atomicAdd(next_row, 1);
+      const int row = rows ? rows[i] : i;
+      int next = in < n ? (rows ? rows[in] : in) : -1;
+      if (next >= P.rows) next = -1;
+      if (row >= 0 && row < P.rows) sample_row_hist(P, row, next, s, pen, redo, n_redo);   // (a list entry is a row index by construction)
+      __syncthreads();
+      if (threadIdx.x == 0) { item[0] = ahead ? in : atomicAdd(next_row, 1); item[1] = fetched; }
+      __syncthreads();
+    }
+    __syncthreads();                                                        // (everyone has read item[] for the last time)
   }
 }
 

@@ -626,12 +626,14 @@ static __device__ bool topk_finish(const SampleDev& P, int row, TopkSmem& c, uin
 }
 
 // Rows are handed out through a counter in the workspace (counters[0], zeroed by the host before the launch): a block takes
-// the next row, passes over it if it is not this kernel's (listing it if `list_others`), and else either finishes it or appends it to `list` (length in
-// counters[1]) for the histogram kernel. The order of the list varies from run to run; what is computed per row does not.
-static __global__ void __launch_bounds__(kTB, kTopkPerSM) sample_topk_kernel(SampleDev P, int* list, int* counters, int list_others) {
+// the next row, passes over it if it is not this kernel's (sample_classify_kernel has listed it), and else either finishes it or appends it to
+// `list` (length in counters[1]) for the histogram kernel. The order of the list varies from run to run; what is computed per row does not.
+static __global__ void __launch_bounds__(kTB, kTopkPerSM) sample_topk_kernel(SampleDev P, int* list, int* counters) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   TopkSmem& c = *reinterpret_cast<TopkSmem*>(smem_raw);
   __shared__ int item[2];                                                   // the row in hand and the one after it
+  // (a histogram kernel launched behind this one with programmatic stream serialization takes over the SMs as this grid's blocks leave them)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   apply_step_state(P);
   if (threadIdx.x < 8) c.prev_cut[threadIdx.x] = 0u;
   // With many rows per block a block holds the row after its current one too (it pulls that row into L2 while it works) and
@@ -645,9 +647,7 @@ static __global__ void __launch_bounds__(kTB, kTopkPerSM) sample_topk_kernel(Sam
     if (row >= P.rows) break;
     int fetched = P.rows;
     if (threadIdx.x == 0 && next < P.rows) fetched = atomicAdd(&counters[0], 1);
-    if (!topk_row_eligible(P, row)) {                                       // not this kernel's row: listed here, or already by sample_classify_kernel
-      if (list_others && threadIdx.x == 0) list[atomicAdd(&counters[1], 1)] = row;
-    } else {
+    if (topk_row_eligible(P, row)) {
       const bool done = topk_row(P, row, next < P.rows ? next : -1, c);
       if (threadIdx.x == 0 && !done) list[atomicAdd(&counters[1], 1)] = row;
     }
