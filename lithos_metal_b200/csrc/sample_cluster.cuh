@@ -114,24 +114,6 @@ __device__ __forceinline__ void cluster_sync(int C) {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// ---- exp(y) for y <= 0 in FP64: the table-driven exponential (P. T. P. Tang, ACM TOMS 15(2), 1989) -----------------------------
-// y = (64 m + j) ln2 / 64 + r, |r| <= ln2 / 128; exp(y) = 2^m 2^(j/64) e^r, e^r by its Taylor polynomial of degree 5 (remainder
-// r^6 / 720 <= 3.6e-17), the reduction in two parts so that r carries no more than its own rounding. Below -690: 0.
-__device__ __forceinline__ double exp64(double y, const double* tab) {
-  if (!(y > -690.0)) return 0.0;
-  const double t = __fma_rn(y, 0x1.71547652b82fep+6, 0x1.8p52);            // 64 / ln2; the integer sits in the low bits
-  const int n = __double2loint(t);
-  const double k = __dadd_rn(t, -0x1.8p52);
-  double r = __fma_rn(k, -0x1.62e42fef00000p-7, y);                        // ln2 / 64, its first 33 bits ...
-  r = __fma_rn(k, -0x1.473de6af278edp-40, r);                              // ... and the rest
-  double p = __fma_rn(r, 1.0 / 120.0, 1.0 / 24.0);
-  p = __fma_rn(p, r, 1.0 / 6.0);
-  p = __fma_rn(p, r, 0.5);
-  p = __fma_rn(p, r, 1.0);
-  p = __fma_rn(p, r, 1.0);
-  p = __dmul_rn(p, tab[n & 63]);
-  return __hiloint2double(__double2hiint(p) + ((n >> 6) << 20), __double2loint(p));
-}
 // 2^43 * e rounded to the nearest integer, 0 <= e <= 1: adding 2^9 leaves an ulp of 2^-43 in the sum's low bits.
 __device__ __forceinline__ unsigned long long fixed43(double e) {
   return static_cast<unsigned long long>(__double_as_longlong(__dadd_rn(e, 512.0)) - 0x4080000000000000ll);

@@ -67,7 +67,8 @@ static_assert(kTopkPerSM * (sizeof(TopkSmem) + 1024) <= 233472, "the blocks of t
 // sum_i 2^(z_i c + shift'), the exact mass relative to a maximum vmax is z_tilde * 2^(shift - vmax c); z_raw is the part of it
 // that was accumulated in FP32 (sequences of acc_terms additions), z_corr what was added and removed term by term (penalties);
 // ref is the logit the exponents were taken relative to (a logit of the row at or near its maximum).
-struct RowMass { bool need; double z_tilde, z_raw, z_corr, shift, acc_terms; float ref; };
+// row: its BF16 codes, n_chunks of eight, where the mass can be formed again in FP64 (c.pen marks the penalised positions); nullptr: the logits are gone.
+struct RowMass { bool need; double z_tilde, z_raw, z_corr, shift, acc_terms; float ref; const uint16_t* row; int n_chunks; bool penalised; };
 
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst))), "l"(gmem_src) : "memory");
@@ -277,7 +278,8 @@ static __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem&
   float2 sacc = make_float2(0.0f, 0.0f);
   uint32_t nan_seen = 0u;
   // A bit per step: this thread's chunk held a logit >= cutoff. The list of those chunks is written behind the pass, one reservation per
-  // warp: nearly every step some lane has one, and a reservation per step was a quarter of the pass's instructions (4096 penalised rows, three in four with a top_k:
+  // warp: nearly every step some lane has one, and a reservation per step was a quarter of the pass's instructions (4096 penalised rows, three in four with a
+  // top_k:
   // 857 -> 797 us; 64 rows of 262,144, top_k 50: 51 -> 45).
   static_assert(kTopkMaxVocab / kChunk <= 64 * kTB, "a bit for every step");
   unsigned long long hits = 0ull;
@@ -406,8 +408,33 @@ static __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem&
   __syncthreads();
   RowMass zm;
   zm.need = need_z; zm.z_tilde = z_tilde; zm.z_raw = z_raw; zm.z_corr = z_sub + z_add; zm.shift = -static_cast<double>(nb);
-  zm.ref = M; zm.acc_terms = 4.0 * n_it + 1.0;
+  zm.ref = M; zm.acc_terms = 4.0 * n_it + 1.0; zm.row = rowp; zm.n_chunks = n_chunks; zm.penalised = pen_on;
   return topk_finish(P, row, c, cut_code, zm);
+}
+
+// The row's softmass in FP64, for the rare row (one in a few hundred) whose top-p boundary the FP32 mass cannot decide. ~15 FP64 operations per
+// logit from L2: less than the histogram kernel would take for the whole row, and behind no other launch. The candidates' keys are dead.
+static __device__ double topk_exact_mass(const SampleDev& P, TopkSmem& c, const RowMass& zm, float vmax, double inv_t) {
+  double* tab = reinterpret_cast<double*>(c.key);
+  const int tid = threadIdx.x;
+  __syncthreads();
+  if (tid < 64) tab[tid] = exp2(static_cast<double>(tid) * 0.015625);
+  __syncthreads();
+  const uint4* p4 = reinterpret_cast<const uint4*>(zm.row);
+  const double vmax64 = static_cast<double>(vmax);
+  double m = 0.0;
+#pragma unroll 1
+  for (int cc = tid; cc < zm.n_chunks; cc += kTB) {
+    const uint4 q = __ldg(p4 + cc);
+    const uint32_t bits = zm.penalised ? (c.pen[cc >> 2] >> ((cc & 3) * 8)) & 0xFFu : 0u, w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int e = 0; e < kChunk; e++) {
+      float z = (e & 1) ? bf16_hi(w[e >> 1]) : bf16_lo(w[e >> 1]);
+      if ((bits >> e) & 1u) z = penalise(z, P.rho, P.pi);
+      m += exp64((static_cast<double>(z) - vmax64) * inv_t, tab);
+    }
+  }
+  return block_sum_f64(m, c.scratch);
 }
 
 // The exact phases of the candidate path, on what the pass (or a producer of logits tiles, sample_tiles.cuh) has left in shared
@@ -506,22 +533,34 @@ static __device__ bool topk_finish(const SampleDev& P, int row, TopkSmem& c, uin
       // These are relative to the mass the pass summed (z_raw), which holds the penalised positions at their raw values. The penalised
       // logits then enter as z_raw - z_sub + z_add, every term of z_sub and z_add with the per-term errors above (FMA, ex2, c2a on a
       // single term: 1.6e-6 covers them for |x| < 32); when penalised tokens carried most of the raw mass the band grows with them.
-      // The band is this bound with a quarter added. A boundary of the cumulative mass inside it is decided by the exact path.
+      // The band is this bound with a quarter added. A boundary of the cumulative mass inside it is decided by the FP64 mass.
       const double u = 5.9604644775390625e-8;
       const double D = fmax(0.0, (static_cast<double>(vmax) - static_cast<double>(zm.ref)) * c64);
       const double rel = u * (12.5 + 1.3862943611198906 * D) + 6.6e-7 + 4.0 * u + zm.acc_terms * u;
       err = 1.25 * (rel * zm.z_raw + 1.6e-6 * zm.z_corr) * (total / zm.z_tilde);
     }
-    const double target = static_cast<double>(top_p) * total;
-    bool amb = false;
-    for (int i = tid; i < n_sel; i += kTB) {
-      const bool run_end = (i == n_sel - 1) || ((c.sel[i + 1] >> 32) != (c.sel[i] >> 32));
-      if (!run_end) continue;
-      const double cm = c.cum[i];
-      if (cm >= target) atomicMin(&c.hit, i);
-      if (i < n_topk - 1 && fabs(cm - target) <= err && fkey_inv(static_cast<uint32_t>(c.sel[i] >> 32)) > tau_k) amb = true;
+    double target;
+    bool edge = false;
+#pragma unroll 1
+    for (bool exact = false;; exact = true) {
+      target = static_cast<double>(top_p) * total;
+      bool amb = false;
+      for (int i = tid; i < n_sel; i += kTB) {
+        const bool run_end = (i == n_sel - 1) || ((c.sel[i + 1] >> 32) != (c.sel[i] >> 32));
+        if (!run_end) continue;
+        const double cm = c.cum[i];
+        if (cm >= target) atomicMin(&c.hit, i);
+        if (!exact && i < n_topk - 1 && fabs(cm - target) <= err && fkey_inv(static_cast<uint32_t>(c.sel[i] >> 32)) > tau_k) amb = true;
+        if (exact && fabs(cm - target) <= 1e-12 * total) edge = true;
+      }
+      if (!__syncthreads_or(amb)) break;
+      if (zm.row == nullptr || in_topk) return false;                       // too close to call, and nothing finer to look at here
+      total = topk_exact_mass(P, c, zm, vmax, inv_t);                       // ... in FP64
+      status = 0u;
+      if (tid == 0) c.hit = kTopkCap;
+      __syncthreads();
     }
-    if (__syncthreads_or(amb)) return false;                               // too close to call in FP32: the exact path decides
+    if (__syncthreads_or(edge)) status |= LM_STATUS_TOPP_EDGE;
     if (c.hit < kTopkCap) {
       const float tau_p = fkey_inv(static_cast<uint32_t>(c.sel[c.hit] >> 32));
       if (static_cast<double>(tau_p) > tau64) tau64 = tau_p;

@@ -120,3 +120,29 @@ def test_draw_over_runs_of_equal_logits_from_both_sources(exact_only):
         pen_ids = np.unique(hist[i])
         mixed += int(np.isin(same, pen_ids).any() and (~np.isin(same, pen_ids)).any())
     assert mixed >= 3, mixed
+
+
+def test_penalised_rows_inside_the_fp32_decision_band_are_decided_in_fp64():
+    """As above with penalties: the candidate kernel forms the mass again in FP64, penalised positions at their penalised values."""
+    rng = np.random.default_rng(31)
+    vocab, T, rho, pi = 40008, np.float32(0.7), 1.2, 0.4
+    codes = oracle.f32_to_bf16((rng.standard_normal(vocab) * 2.0).astype(np.float32))
+    hist = np.concatenate([np.argsort(-oracle.bf16_to_f32(codes))[:400:2], rng.integers(0, vocab, 500)]).astype(np.int32)
+    z = np.asarray(oracle.apply_penalties(oracle.bf16_to_f32(codes), hist, rho, pi), dtype=np.float64)
+    vals, counts = np.unique(z, return_counts=True)
+    vals, counts = vals[::-1], counts[::-1]
+    cum = np.cumsum(counts * np.exp((vals - vals[0]) / np.float64(T)))
+    top_p = np.array([cum[int(np.searchsorted(np.cumsum(counts), n))] / cum[-1] * (1.0 + d) for n in (60, 150, 250, 333, 390, 450)
+                      for d in (0.0, 1e-7, -1e-7, 4e-7, -4e-7, 1e-6, -1e-6, 1e-4)], dtype=np.float32)
+    n = len(top_p)
+    cfg = dict(logits=np.tile(codes, (n, 1)), temperature=np.full(n, T, np.float32), top_k=np.full(n, 600, np.int32), top_p=top_p)
+    u = np.linspace(0.02, 0.98, n).astype(np.float32)
+    r = lm.sample(torch.from_numpy(cfg["logits"].view(np.int16)).cuda().view(torch.bfloat16),
+                  lm.SamplingParams(draw="inverse_cdf", repetition_penalty=rho, presence_penalty=pi, **{k: torch.from_numpy(cfg[k]).cuda() for k in ("temperature", "top_k", "top_p")}),
+                  history=torch.from_numpy(np.tile(hist, (n, 1))).cuda(), uniforms=torch.from_numpy(u).cuda(), return_tau=True, return_status=True)
+    tok, tau, _ = oracle.sample_batch(cfg["logits"], temperature=cfg["temperature"], top_k=cfg["top_k"], top_p=top_p, history=np.tile(hist, (n, 1)), repetition_penalty=rho,
+                                      presence_penalty=pi, draw="inverse_cdf", uniforms=u, n_threads=THREADS)
+    np.testing.assert_array_equal(r.tau.cpu().numpy(), tau)
+    np.testing.assert_array_equal(r.tokens.cpu().numpy(), tok)
+    on_candidate_path = (r.status.cpu().numpy() & 64) != 0
+    assert on_candidate_path[7::8].all() and not on_candidate_path[::8].any()
