@@ -234,8 +234,15 @@ int lm_sample(const lm_sample_args* a) {
   if (fast && (!a->workspace || (reinterpret_cast<uintptr_t>(a->workspace) & 255u) || a->workspace_bytes < lm_workspace_bytes(a->rows, a->vocab)))
     return LM_E_WORKSPACE;
   // A row per cluster: every row the streaming kernels below do not take (binary32, ragged vocabularies, statistics), and batches too
-  // small to fill the GPU with a block per row. A call that limits its blocks stays below.
-  if (limit == 0 && a->vocab > 0 && (!fast || a->rows * 4 <= sms) && (!pen || a->hist_len <= 65536) && a->rows <= 0x7FFFFFFF / 16)
+  // small to fill the GPU with a block per row: up to SMs / 4 rows of any length, and up to SMs / 2 while the rows are short -- the line lies
+  // lower for rows that all lack a top_k, which the histogram kernel does faster from there on (60 rows, streaming / cluster, us: mixed knobs
+  // 32,768 74 / 64, 65,536 78 / 55, 151,936 96 / 118; top_k 50 32,768 37 / 22, 65,536 39 / 27; none 32,768 39 / 33, 65,536 45 / 61). With one
+  // top_k for all, short rows stay there up to a row per SM (148 rows of 32,768: 46 / 27). A call that limits its blocks stays below.
+  const bool exact = (a->flags & LM_FLAG_EXACT_ONLY) != 0;
+  const bool one_k = a->top_k == nullptr && a->top_k_s >= 1 && a->top_k_s <= kTopkMaxK;
+  const bool small_batch = a->rows * 4 <= sms || (!exact && a->rows * 2 <= sms && a->vocab <= (a->top_k != nullptr || one_k ? 65536 : 40000)) ||
+                           (!exact && one_k && a->rows <= sms && a->vocab <= 40000);
+  if (limit == 0 && a->vocab > 0 && (!fast || small_batch) && (!pen || a->hist_len <= 65536) && a->rows <= 0x7FFFFFFF / 16)
     return sample_clusters(P, sms, st);
   if (fast) {
     const size_t rows_bytes = align256(static_cast<size_t>(a->rows) * sizeof(uint32_t));
@@ -263,11 +270,11 @@ int lm_sample(const lm_sample_args* a) {
     if (limit > 0 && grid1 > limit) grid1 = limit;
     if (!topk) {
       sample_hist_kernel<<<grid, kHB, hist_smem, st>>>(P, nullptr, nullptr, counters + 2, redo, counters + 3, nullptr, nullptr, nullptr);
-    } else if (a->rows > static_cast<int64_t>(kOverlapRowsPerSM) * sms) {
-      // Many rows per SM: the top-k kernel first, the histogram kernel behind it with programmatic stream serialization: its blocks take an
-      // SM over as the top-k blocks leave it, work through the rows that a one-thread-per-row kernel has listed for it, wait for the top-k
-      // grid, and absorb the few rows that one handed on. (Behind its end: 4096 penalised rows 771 us, now
-      // 720; 800 rows 210, now 186.)
+    } else if (one_k || a->rows > static_cast<int64_t>(kOverlapRowsPerSM) * sms) {
+      // Many rows per SM, or hardly a row for the histogram kernel (one top_k for all: 148 rows 56 us side by side, 43 so): the top-k kernel first,
+      // the histogram kernel behind it with programmatic stream serialization: its blocks take an SM over as the top-k blocks leave it, work
+      // through the rows that a one-thread-per-row kernel has listed for it, wait for the top-k grid, and absorb the few rows that one handed
+      // on. (Behind its end: 4096 penalised rows 771 us, now 720; 800 rows 210, now 186.)
       sample_classify_kernel<<<static_cast<int>((a->rows + 255) / 256), 256, 0, st>>>(P, list_other, counters + 4);
       sample_topk_kernel<<<grid1, kTB, sizeof(TopkSmem), st>>>(P, list_left, counters);
       cudaError_t e = cudaGetLastError();

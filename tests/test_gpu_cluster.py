@@ -150,3 +150,14 @@ def test_streaming_batches_of_every_geometry(rows, draw, penalised):
     kw = dict(history=rng.integers(0, vocab, (rows, 700)).astype(np.int32), rho=1.1, pi=0.5) if penalised else {}
     _check(_tensor(host), host, _mixed(rng, rows, (0, 0, 20, 50, 1000)), draw=draw, **kw)
     _check(_tensor(host), host, dict(temperature=0.9, top_k=0, top_p=0.9, min_p=0.0), draw=draw, **kw)
+
+
+# BF16 batches on both sides of the lines between clusters and streaming kernels (rows per SM, length of a row)
+@pytest.mark.parametrize("rows,vocab", [(74, 40000), (74, 40008), (74, 65536), (74, 65544), (75, 40000), (148, 40000), (148, 40008), (149, 40000)])
+@pytest.mark.parametrize("top_k", ["per row", 30, 0])
+def test_batches_at_the_lines_between_the_kernels(rows, vocab, top_k):
+    rng = np.random.default_rng(rows + vocab)
+    host = oracle.f32_to_bf16((rng.standard_normal((rows, vocab)) * 2).astype(np.float32))
+    knobs = _mixed(rng, rows) if top_k == "per row" else dict(temperature=0.8, top_k=top_k, top_p=0.9, min_p=0.0)
+    hist = rng.integers(0, vocab, (rows, 400)).astype(np.int32) if top_k != 0 else None
+    _check(_tensor(host), host, knobs, draw="inverse_cdf" if top_k != 0 else "gumbel", history=hist, rho=1.1, pi=0.5)
