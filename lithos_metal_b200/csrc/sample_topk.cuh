@@ -5,8 +5,8 @@
 // (b) accumulate the softmass of the whole row in FP32 (the top-p target needs it). Everything exact then happens on the
 // candidates alone: the k-th largest value, FP64 masses, the top-p boundary, integer weights, the draw. The FP32 mass is
 // only used to decide on which side of top_p * Z a cumulative mass lies; if that is closer than the FP32 error bound (derived
-// where it is applied), or the candidates do not cover the top-k set, or anything else does not fit, the row is handed on and
-// the histogram kernel launched behind this one redoes it exactly.
+// where it is applied), the mass is formed again in FP64. If the candidates do not cover the top-k set, or anything else does not
+// fit, the row is handed on and the histogram kernel redoes it exactly.
 // Two blocks of 512 threads share an SM (~93 KB of shared memory each): the per-row phases after the pass are chains of short
 // dependent steps, and only the row in the other block can hide them.
 // No counterpart in the reference (its sampler always builds the full histogram, kernels/common/sample.metal:34-162).

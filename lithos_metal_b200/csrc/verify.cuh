@@ -7,6 +7,8 @@
 // test -> the residual's total -> the token), so the kernel is one cooperative launch of one block per SM; every block owns the
 // same vocabulary slice of every row in every phase. Phase 0 is the only one that touches HBM: it pulls the block's slice of
 // all target rows and all draft rows into shared memory (every load in flight at once); the later phases work from there.
+// (A launch that is given the rows' maxima and masses knows the decisive row from one logit per draft and reads only that one, from global
+// memory.)
 //
 // Blocks exchange their partial results through TAGGED WORDS in a small workspace: every partial is one 64-bit word whose top
 // bit says "written". A block publishes with one plain store per word and consumes by polling the words it needs, so a
