@@ -285,6 +285,11 @@ __device__ __forceinline__ double exp64(double y, const double* tab) {
 
 __device__ __forceinline__ float ex2_approx(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 
+// A row's softmass in FP32 is a sum of 2^(z c + nb), c = log2(e) / T, nb = fl32(-vmax c). The rounding of nb is a factor common to all terms and
+// is taken out afterwards -- as long as it is a fraction of a binade. At |vmax| / T of 2^20 it is 2^-4 at most; where |vmax| / T reaches 2^29 or so
+// it is 2^5 binades and more, and the largest term may overflow (or all of them vanish). Beyond this line the sum is formed in FP64.
+constexpr double kMassExponent = 0x1p20;
+
 // ---- Gumbel keys, the two logarithms only where they can matter --------------------------------------------------------------------
 // key = z / T + g, g = -ln(-ln u), u = (h + 1/2) / 2^23 from 23 bits of the hash. key >= B needs -ln u <= exp(z / T - B), and 1 - u <=
 // -ln u: a logit with (2^23 - h) > 2^23 exp(z / T - B) + 1 cannot reach B. One hash and one ex2 per logit decide that; the few that pass

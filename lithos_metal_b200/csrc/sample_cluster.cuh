@@ -950,8 +950,9 @@ static __device__ __noinline__ bool phase_top_k(ClusterSmem& s, const SampleDev&
     if (hits) pick = __shfl_sync(kFull, at, __ffs(hits) - 1);
   }
   if (pick < 0) return false;                                               // fewer groups than top_k
-  // every logit at or above the bound's bin, and (for a top-p over the row) the FP32 mass: one more look at the row
-  const bool need_z = s.has_p && !s.in_topk;
+  // every logit at or above the bound's bin, and (for a top-p over the row) the FP32 mass: one more look at the row. Not at temperatures so
+  // small that the rounding of the maximum's exponent is no fraction of a binade (kMassExponent): there the mass is formed in FP64 at once.
+  const bool whole = s.has_p && !s.in_topk, need_z = whole && static_cast<double>(fabsf(vmax)) * s.inv_t < kMassExponent;
   const float zf = pick >= kCMaxBins - 1 ? gmin : floor_of_bin(vmax, static_cast<float>(pick), mscale);
   const int n = phase_select<F32, CACHED>(s, zf, need_z);
   if (n > kCList) return false;
@@ -965,6 +966,7 @@ static __device__ __noinline__ bool phase_top_k(ClusterSmem& s, const SampleDev&
     tied = v == kFull;
   }
   double total = 0.0, err = 0.0;
+  if (whole && !need_z) total = phase_mass64<F32, CACHED>(s, -INFINITY, s.x_mass64);
   if (need_z) {
     for (int q = 0; q < C; q++) total += s.x_mass[q];
     const double un = 5.9604644775390625e-8;                                // sample_topk.cuh derives this bound (the reference point here is the maximum itself)
@@ -977,7 +979,7 @@ static __device__ __noinline__ bool phase_top_k(ClusterSmem& s, const SampleDev&
     VpMergeDev M;
     M.flags = s.flags; M.draw = P.draw; M.uniforms = P.uniforms; M.seed = s.seed; M.step = s.step; M.row_offset = P.row_offset;
     M.out_tokens = s.rank == 0 ? P.out_tokens : nullptr; M.out_tau = P.out_tau; M.out_status = P.out_status; M.out_vmax = P.out_vmax; M.out_mass = P.out_mass;
-    M.hand_on = 1; M.path_status = LM_STATUS_CANDIDATE_PATH;
+    M.hand_on = 1; M.path_status = whole && !need_z ? 0u : LM_STATUS_CANDIDATE_PATH;
     *written = true;
 #pragma unroll 1
     for (int pass = 0; pass < 2; pass++) {
@@ -997,7 +999,7 @@ static __device__ __noinline__ bool phase_top_k(ClusterSmem& s, const SampleDev&
   }
   // thresholds
   double tau64 = tau_k;
-  uint32_t status = s.want_stats ? 0u : LM_STATUS_CANDIDATE_PATH;
+  uint32_t status = s.want_stats || (whole && !need_z) ? 0u : LM_STATUS_CANDIDATE_PATH;
   if (s.has_p) {
     for (int i = tid; i < n_topk; i += B) s.cum[i] = exp64((static_cast<double>(list_value(s, i)) - static_cast<double>(vmax)) * s.inv_t, s.exp_tab);
     __syncthreads();

@@ -161,3 +161,19 @@ def test_batches_at_the_lines_between_the_kernels(rows, vocab, top_k):
     knobs = _mixed(rng, rows) if top_k == "per row" else dict(temperature=0.8, top_k=top_k, top_p=0.9, min_p=0.0)
     hist = rng.integers(0, vocab, (rows, 400)).astype(np.int32) if top_k != 0 else None
     _check(_tensor(host), host, knobs, draw="inverse_cdf" if top_k != 0 else "gumbel", history=hist, rho=1.1, pi=0.5)
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+def test_thresholds_at_very_small_temperatures(dtype):
+    """top-p next to a top_k where the exponent of the maximum, vmax log2(e) / T, is far beyond what binary32 resolves: the kept set is the
+    maximum (and its ties) alone. Up to 64 candidates and more, the clusters and the streaming kernels; and a maximum of 1e10."""
+    rng = np.random.default_rng(13)
+    for rows in (40, 80):
+        z = (rng.standard_normal((rows, 40008)) * 2).astype(np.float32)
+        z[1, 500], z[1, 7000] = 13.0, 13.0
+        z[2, 123] = 1e10
+        host = oracle.f32_to_bf16(z) if dtype == "bf16" else z
+        for t in (1e-6, 1e-8, 3e-9, 1e-9, 1e-12):
+            for k in (50, 200):
+                knobs = dict(temperature=np.full(rows, t, np.float32), top_k=np.full(rows, k, np.int32), top_p=np.full(rows, 0.9, np.float32), min_p=0.0)
+                _check(_tensor(host), host, knobs, draw="gumbel" if k == 50 else "inverse_cdf")
