@@ -170,7 +170,7 @@ static __global__ void __launch_bounds__(B) slice_local_kernel(SliceDev P) {
   const float vmax = best_value(best);
   const double inv_t = 1.0 / static_cast<double>(P.temperature_rows ? P.temperature_rows[row] : P.temperature);
   double mass = 0.0;
-  if (P.need_mass && P.exact_mass && vmax > -INFINITY) {
+  if (P.need_mass && (P.exact_mass || static_cast<double>(fabsf(vmax)) * inv_t >= kMassExponent) && vmax > -INFINITY) {   // (or a temperature too small for what follows)
     double m = 0.0;
     for (int j = tid; j < n; j += B) m += softmass(vals[j], vmax, inv_t);
     mass = block_sum_f64(m, scratch);

@@ -201,3 +201,16 @@ def test_random_configurations_equal_the_exact_kernels():
             assert fast.tau.cpu().numpy().tobytes() == tau.tobytes() and np.all((fast.tokens.cpu().numpy() == tok) | tie), trial
             checked_with_oracle += 1
     assert checked_with_oracle >= 2
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+def test_thresholds_at_very_small_temperatures(dtype):
+    """Where the exponent of a slice's maximum is beyond what binary32 resolves the slices form their masses in FP64."""
+    x, host = _rows(4, 40000, 11, dtype, spikes=2)
+    for t in (1e-6, 3e-9, 1e-9, 1e-12):
+        _check(x, host, draw="gumbel", temperature=float(np.float32(t)), top_k=50, top_p=0.9)
+    x, host = _rows(3, 40000, 12, dtype, spikes=0)
+    x[1, 77] = 1e10
+    host[1, 77] = oracle.f32_to_bf16(np.array([1e10], np.float32))[0] if dtype == "bf16" else np.float32(1e10)
+    for t in (0.8, 1e-9):
+        _check(x, host, draw="inverse_cdf", temperature=float(np.float32(t)), top_k=20, top_p=0.95)
