@@ -460,8 +460,8 @@ struct FoundKeys {
 };
 
 // The first look at the row: maximum, its lowest index, smallest finite logit, odd values; the group maxima; the slice's copy.
-// BF16: a value whose magnitude lies outside 2^-39 .. 2^25 and is not 0 or -inf makes the row odd, as in the histogram kernel
-// (one packed test per two logits covers NaN and +inf too); binary32: NaN is looked for, +inf shows in the maximum.
+// BF16: a NaN or a magnitude below 2^-39 that is not 0 makes the row odd (one packed test per two logits passes the codes of 2^-39 .. 2^25; a mask
+// of -1e9 or the type's lowest value fails it and is looked at closely); binary32: NaN is looked for. +inf shows in the maximum.
 template <bool F32, bool CACHED, int B>
 static __device__ __noinline__ void phase_load(ClusterSmem& s) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -496,7 +496,7 @@ static __device__ __noinline__ void phase_load(ClusterSmem& s) {
 #pragma unroll
             for (int h = 0; h < 2; h++) {
               const uint32_t code = h ? w[k] >> 16 : w[k] & 0xFFFFu, mag = code & 0x7FFFu;
-              odd = odd || (mag != 0u && code != 0xFF80u && (mag < 0x2C00u || mag >= 0x4C00u));
+              odd = odd || (mag != 0u && mag < 0x2C00u) || mag > 0x7F80u;
             }
           }
         }

@@ -177,3 +177,23 @@ def test_thresholds_at_very_small_temperatures(dtype):
             for k in (50, 200):
                 knobs = dict(temperature=np.full(rows, t, np.float32), top_k=np.full(rows, k, np.int32), top_p=np.full(rows, 0.9, np.float32), min_p=0.0)
                 _check(_tensor(host), host, knobs, draw="gumbel" if k == 50 else "inverse_cdf")
+
+
+def _masked(rng, rows, vocab, mask, dtype):
+    """Logits of which a third and the first eighth carry a mask's value."""
+    z = (rng.standard_normal((rows, vocab)) * 2).astype(np.float32)
+    z[rng.random((rows, vocab)) < 1 / 3] = mask
+    z[:, : vocab // 8] = mask
+    return oracle.f32_to_bf16(z) if dtype == "bf16" else z
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("mask", [-1e4, -1e9, -3.3e38])
+def test_a_large_negative_mask_is_no_reason_for_the_generic_algorithm(dtype, mask):
+    rng = np.random.default_rng(41)
+    host = _masked(rng, 8, 40008, mask, dtype)
+    for k, p in ((0, 0.9), (50, 0.9), (1000, 0.9)):
+        for draw in ("inverse_cdf", "gumbel"):
+            knobs = dict(temperature=np.full(8, 0.8, np.float32), top_k=np.full(8, k, np.int32), top_p=np.full(8, p, np.float32), min_p=0.0)
+            _, status = _check(_tensor(host), host, knobs, draw=draw)
+            assert not np.any(status & 1), (k, draw, status)
