@@ -197,3 +197,16 @@ def test_a_large_negative_mask_is_no_reason_for_the_generic_algorithm(dtype, mas
             knobs = dict(temperature=np.full(8, 0.8, np.float32), top_k=np.full(8, k, np.int32), top_p=np.full(8, p, np.float32), min_p=0.0)
             _, status = _check(_tensor(host), host, knobs, draw=draw)
             assert not np.any(status & 1), (k, draw, status)
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("mask", [-1e3, -1e4, -1e9, -3.3e38])
+@pytest.mark.parametrize("rows,vocab", [(1, 2048), (8, 40008), (50, 30011), (100, 16395)])
+def test_a_masked_row_keeps_the_list_of_its_top_k(dtype, mask, rows, vocab):
+    """Groups of nothing but masked logits do not spoil the bound of the top_k-th logit: the row stays on the list (status 64)."""
+    rng = np.random.default_rng(rows + vocab)
+    host = _masked(rng, rows, vocab, mask, dtype)
+    for k in (1, 50, 200):
+        knobs = dict(temperature=np.full(rows, 0.8, np.float32), top_k=np.full(rows, k, np.int32), top_p=np.full(rows, 0.9, np.float32), min_p=0.0)
+        _, status = _check(_tensor(host), host, knobs, draw="gumbel")
+        assert np.count_nonzero(status & 64) >= rows - 1, (k, status)       # (a top-p boundary inside the FP32 mass's band leaves it)
