@@ -195,12 +195,26 @@ __device__ __forceinline__ void sweep(const ClusterRow& R, F f) {
 // The bin of a logit: 0 at the maximum, growing downwards; non-increasing in z because every step of it is monotone (explicitly
 // rounded operations: every call site gives the same bin). The integer is read out of the sum with 2^23. With a window, only the
 // logits of one such bin are looked at, and the bins divide it once more (kCBins: a logit outside the window).
+constexpr int kLogBins = -2;             // ClusterBins::window: bins by the depth's exponent and four bits (2^-32 .. 2^32; what lies beyond shares the end bins)
+constexpr uint32_t kLogBase = (127u - 32u) << 4;
+__device__ __forceinline__ float log_bin_edge(uint32_t b) { return b == 0u ? 0.0f : b >= static_cast<uint32_t>(kCBins) ? INFINITY : __uint_as_float((b + kLogBase) << 19); }
 struct ClusterBins {
-  float vmax, scale; int window;                                            // window < 0: none
+  float vmax, scale; int window;                                            // -1: none; kLogBins; 0 .. kCBins - 1: a linear bin; kCBins + b: bin b of those by exponent
   __device__ __forceinline__ float depth(float z) const { return fminf(__fmul_rn(__fsub_rn(vmax, z), scale), static_cast<float>(kCBins - 1)); }
   __device__ __forceinline__ uint32_t coarse(float z) const { return __float_as_uint(__fadd_rn(depth(z), 8388608.0f)) & static_cast<uint32_t>(kCBins - 1); }
+  __device__ __forceinline__ uint32_t by_exponent(float z) const {
+    return min(max(__float_as_uint(__fsub_rn(vmax, z)) >> 19, kLogBase) - kLogBase, static_cast<uint32_t>(kCBins - 1));
+  }
   __device__ __forceinline__ uint32_t of(float z) const {
-    if (window < 0) return coarse(z);
+    if (window == -1) return coarse(z);
+    if (window == kLogBins) return by_exponent(z);
+    if (window >= kCBins) {
+      const uint32_t lb = static_cast<uint32_t>(window - kCBins);
+      if (by_exponent(z) != lb) return kCBins;
+      const float lo = log_bin_edge(lb), width = log_bin_edge(lb + 1u) - lo;   // (an infinite width, or a NaN product of it: bin 0)
+      const float t = __fmul_rn(__fsub_rn(__fsub_rn(vmax, z), lo), __fdiv_rn(static_cast<float>(kCBins - 1), width));
+      return __float_as_uint(__fadd_rn(fminf(fmaxf(t, 0.0f), static_cast<float>(kCBins - 1)), 8388608.0f)) & static_cast<uint32_t>(kCBins - 1);
+    }
     if (coarse(z) != static_cast<uint32_t>(window)) return kCBins;
     const float t = __fmul_rn(__fsub_rn(depth(z), static_cast<float>(window) - 0.5f), static_cast<float>(kCBins - 1));
     return __float_as_uint(__fadd_rn(fminf(fmaxf(t, 0.0f), static_cast<float>(kCBins - 1)), 8388608.0f)) & static_cast<uint32_t>(kCBins - 1);
@@ -571,7 +585,7 @@ static __device__ __noinline__ void sweep_bins(ClusterSmem& s, uint32_t kinds) {
   const double inv_t = s.inv_t, vmax64 = static_cast<double>(s.vmax);
   const ClusterBins bins{s.vmax, s.scale, s.window};
   const float vmax = s.vmax, c2 = s.c2;
-  if (bins.window >= 0) {                                                   // (rare: a bin that more logits share than a list holds)
+  if (bins.window != -1) {                                                  // (rare: a bin that more logits share than a list holds)
     sweep<F32, CACHED>(R, [&](int, const float (&z)[8]) {
 #pragma unroll
       for (int e = 0; e < 8; e++) {
@@ -645,7 +659,7 @@ static __device__ __noinline__ void phase_bins(ClusterSmem& s, uint32_t kinds, b
     cluster_sync(C);                                                        // (the lists that lie over the bins are no longer read)
     for (int i = tid; i < kCBins; i += B) { s.cnt[i] = 0u; s.lo[0][i] = 0u; s.lo[1][i] = 0u; s.hi[0][i] = 0u; s.hi[1][i] = 0u; }
   }
-  if (use_m && s.window < 0) {
+  if (use_m && s.window == -1) {
     const double step = 1.0 / static_cast<double>(s.scale);
     for (int b = tid; b < kCBins; b += B) { const double d = -(static_cast<double>(b) * step); s.bin_exp[b] = make_double2(exp64(d * s.inv_t, s.exp_tab), d); }
   }
@@ -722,9 +736,17 @@ __device__ __forceinline__ int end_list(ClusterSmem& s, uint32_t counter) {
 template <bool F32, bool CACHED, int B>
 static __device__ __noinline__ int phase_bin_list(ClusterSmem& s, uint32_t b, int turn) {
   const ClusterBins bins{s.vmax, s.scale, s.window};
-  const uint32_t cb = bins.window < 0 ? b : static_cast<uint32_t>(bins.window);
-  const float zl = cb >= static_cast<uint32_t>(kCBins - 1) ? -FLT_MAX : floor_of_bin(bins.vmax, static_cast<float>(cb), bins.scale);
-  const float zh = cb > 0u ? ceil_of_bin(bins.vmax, static_cast<float>(cb), bins.scale) : bins.vmax;
+  float zl, zh;
+  if (bins.window == kLogBins || bins.window >= kCBins) {                    // (the depth's rounding is half a unit in its last place)
+    const uint32_t lb = bins.window == kLogBins ? b : static_cast<uint32_t>(bins.window - kCBins);
+    const float near = log_bin_edge(lb), far = log_bin_edge(lb + 1u);
+    zl = far == INFINITY ? -FLT_MAX : (bins.vmax - far) - (fabsf(bins.vmax) + far) * 4e-7f;
+    zh = fminf((bins.vmax - near) + (fabsf(bins.vmax) + near) * 4e-7f, bins.vmax);
+  } else {
+    const uint32_t cb = bins.window < 0 ? b : static_cast<uint32_t>(bins.window);
+    zl = cb >= static_cast<uint32_t>(kCBins - 1) ? -FLT_MAX : floor_of_bin(bins.vmax, static_cast<float>(cb), bins.scale);
+    zh = cb > 0u ? ceil_of_bin(bins.vmax, static_cast<float>(cb), bins.scale) : bins.vmax;
+  }
   FoundKeys found;
   found.init(s, begin_list(s, turn));
   {
@@ -1114,13 +1136,14 @@ static __device__ __noinline__ bool phase_search(ClusterSmem& s, bool dirty) {
     }
     above_n = 0u; above_m = above_w = 0ull;
     bool refill = !fresh, empty = false, again = false;
+    int base = -1;                                                          // the bins of level 0: linear, or (kLogBins) by exponent
 #pragma unroll 1
     for (int level = 0;; level++) {
       if (refill) {
-        if (level == 0 && tid == 0) s.window = -1;                          // (phase_bins has a barrier before it reads this)
+        if (level == 0 && tid == 0) s.window = base;                        // (phase_bins has a barrier before it reads this)
         if (level == 0) __syncthreads();
         phase_bins<F32, CACHED, B>(s, kinds | (level ? 1u : 0u), dirty);
-        dirty = true; fresh = level == 0; list_tag = -1; refill = false;
+        dirty = true; fresh = level == 0 && base == -1; list_tag = -1; refill = false;
       }
       if (level == 0 && step == kMass) {
         const double row_total = static_cast<double>(sums[kCBins - 1]) * unit;
@@ -1150,16 +1173,27 @@ static __device__ __noinline__ bool phase_search(ClusterSmem& s, bool dirty) {
         b = s.pick;
         if (b >= static_cast<uint32_t>(kCBins)) { empty = true; break; }
       }
+      // with the counts at hand a list that could not hold the bin is not begun
+      const uint32_t in_bin = (kinds & 1u) || level ? s.r_cnt[b + 1] - s.r_cnt[b] : 0u;
+      // A count can cross where the linear bins do not tell: beyond their range (which is that of the weights), or so near the maximum that a
+      // masked logit has stretched them over everything else. The bins by exponent do.
+      if (step == kCount && level == 0 && base == -1 && in_bin > static_cast<uint32_t>(kCList) && (b < 4u || b == static_cast<uint32_t>(kCBins - 1))) {
+        base = kLogBins; level = -1; refill = true;
+        continue;
+      }
       if ((kinds & 1u) || level) above_n += s.r_cnt[b];
       if (b && (kinds & 2u)) above_m += s.r_sum[0][b - 1];
       if (b && (kinds & 4u)) above_w += s.r_sum[1][b - 1];
       if (level == 0 && list_tag == static_cast<int>(b)) break;             // the list in hand
-      list_len = phase_bin_list<F32, CACHED, B>(s, b, turn);
-      turn = (turn & 1) ? 2 : 1;                                            // (> 0: a list has come before)
-      if (list_len <= kCList) { list_tag = level ? -1 : static_cast<int>(b); break; }
+      list_len = static_cast<int>(in_bin);
+      if (in_bin <= static_cast<uint32_t>(kCList)) {
+        list_len = phase_bin_list<F32, CACHED, B>(s, b, turn);
+        turn = (turn & 1) ? 2 : 1;                                          // (> 0: a list has come before)
+      }
+      if (list_len <= kCList) { list_tag = level || base != -1 ? -1 : static_cast<int>(b); break; }
       if (level == 1) return false;                                         // more equal logits than a list holds
       fresh = false; refill = true;
-      if (tid == 0) s.window = static_cast<int>(b);
+      if (tid == 0) s.window = base == -1 ? static_cast<int>(b) : kCBins + static_cast<int>(b);
       __syncthreads();
     }
     if (empty) { list_len = 0; list_tag = -1; }

@@ -210,3 +210,20 @@ def test_a_masked_row_keeps_the_list_of_its_top_k(dtype, mask, rows, vocab):
         knobs = dict(temperature=np.full(rows, 0.8, np.float32), top_k=np.full(rows, k, np.int32), top_p=np.full(rows, 0.9, np.float32), min_p=0.0)
         _, status = _check(_tensor(host), host, knobs, draw="gumbel")
         assert np.count_nonzero(status & 64) >= rows - 1, (k, status)       # (a top-p boundary inside the FP32 mass's band leaves it)
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("mask", [0.0, -1e4, -1e9, -3.3e38])
+def test_a_count_is_found_wherever_it_crosses(dtype, mask):
+    """A top_k beyond the list, and exact_only: the k-th logit next to a mask's value that stretches the bins, and deeper than the weights
+    reach (a low temperature). More equal logits at the crossing than a list holds are left to the generic algorithm."""
+    rng = np.random.default_rng(43)
+    host = _masked(rng, 6, 65543, mask, dtype) if mask else _masked(rng, 6, 65543, 0.5, dtype)
+    for k, exact in ((2000, False), (9000, False), (50, True)):
+        for t, p in ((0.8, 0.0), (0.8, 0.9), (0.05, 0.9), (1e-9, 0.0)):
+            for draw in ("inverse_cdf", "gumbel"):
+                knobs = dict(temperature=np.full(6, t, np.float32), top_k=np.full(6, k, np.int32), top_p=np.full(6, p, np.float32), min_p=0.0)
+                _, status = _check(_tensor(host), host, knobs, draw=draw, exact_only=exact)
+                assert not np.any(status & 1) or (not mask and k == 9000), (k, t, p, draw, status)
+    knobs = dict(temperature=np.full(6, 0.8, np.float32), top_k=np.full(6, 60000, np.int32), top_p=np.full(6, 0.9, np.float32), min_p=0.0)
+    _check(_tensor(host), host, knobs, draw="inverse_cdf", exact_only=True)  # the k-th is one of the masked
