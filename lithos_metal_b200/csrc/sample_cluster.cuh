@@ -925,69 +925,83 @@ static __device__ __noinline__ void pick_in_list(ClusterSmem& s, int n, float ta
   }
 }
 
+// The group maxima counted in bins of their depth below the row's maximum (16-bit counts pushed to every block, added up there): the bin of the
+// top_k-th of them (-1: there are fewer), and how many lie down to that bin, the bin included. kExponent: bins by the depth's exponent and one bit.
+template <bool kExponent, int B>
+__device__ __forceinline__ int bound_of_maxima(ClusterSmem& s, float mscale, uint32_t* through) {
+  const int tid = threadIdx.x, lane = tid & 31, C = s.C;
+  const float vmax = s.vmax;
+  {
+    const ClusterBins mb{vmax, mscale, -1};
+    const int mine = (s.R.c1 - s.R.c0 - tid + B - 1) / B, groups = (mine + s.every - 1) / s.every;   // (mine may be negative: no group)
+    for (int g = 0; g < groups; g++) {
+      const float m = s.gmax[g * B + tid];
+      if (m > -INFINITY) atomicAdd(&s.max_cnt[kExponent ? __float_as_uint(__fsub_rn(vmax, m)) >> 22 : min(mb.coarse(m), static_cast<uint32_t>(kCMaxBins - 1))], 1u);
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < C * (kCMaxBins / 2); i += B) {                     // (at most 4096 groups a block: 16 bits)
+    const int q = i / (kCMaxBins / 2), w = i - q * (kCMaxBins / 2);
+    cst_u32(cluster_addr(&s.x_max[s.rank][w], q), s.max_cnt[2 * w] | (s.max_cnt[2 * w + 1] << 16));
+  }
+  cluster_sync(C);
+  if (tid < kCMaxBins / 2) {
+    uint32_t n0 = 0u, n1 = 0u;
+    for (int q = 0; q < C; q++) { const uint32_t w = s.x_max[q][tid]; n0 += w & 0xFFFFu; n1 += w >> 16; }
+    s.totals[2 * tid] = n0; s.totals[2 * tid + 1] = n1;
+  }
+  __syncthreads();
+  // every warp for itself: lane l holds 16 bins
+  uint32_t v[kCMaxBins / 32], sum = 0u;
+#pragma unroll
+  for (int j = 0; j < kCMaxBins / 32; j += 4) {
+    const uint4 q = *reinterpret_cast<const uint4*>(&s.totals[lane * (kCMaxBins / 32) + j]);
+    v[j] = q.x; v[j + 1] = q.y; v[j + 2] = q.z; v[j + 3] = q.w; sum += q.x + q.y + q.z + q.w;
+  }
+  uint32_t incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) { const uint32_t t = __shfl_up_sync(kFull, incl, o); if (lane >= o) incl += t; }
+  const uint32_t k = static_cast<uint32_t>(s.top_k);
+  uint32_t run = incl - sum, reached = 0u; int at = -1;
+#pragma unroll
+  for (int j = 0; j < kCMaxBins / 32; j++) { run += v[j]; if (at < 0 && run >= k) { at = lane * (kCMaxBins / 32) + j; reached = run; } }
+  const uint32_t hits = __ballot_sync(kFull, at >= 0);
+  if (!hits) return -1;
+  *through = __shfl_sync(kFull, reached, __ffs(hits) - 1);
+  return __shfl_sync(kFull, at, __ffs(hits) - 1);
+}
+
+// The bound again where something far below the rest (a group of nothing but masked logits) has stretched the linear bins until the bin of the
+// top_k-th holds far more than top_k: bins by exponent find the range that matters, linear ones divide that. (4 rows of 151,936, a third at
+// -1e4, top_k 50: 63 us by the search that an overflowing list leads to, 25 us so; without a mask 19.)
+template <int B>
+static __device__ __noinline__ int narrower_bound(ClusterSmem& s, float* mscale) {
+  auto again = [&]() {
+    cluster_sync(s.C);                                                      // (the counts of the pass before are no longer read)
+    for (int i = threadIdx.x; i < kCMaxBins; i += B) s.max_cnt[i] = 0u;
+    __syncthreads();
+  };
+  uint32_t through;
+  again();
+  const int e = bound_of_maxima<true, B>(s, 0.0f, &through);
+  // (the top_k-th lies above the lower edge of its bin by exponent: in the first 511 of the linear bins down to that edge)
+  *mscale = fminf(static_cast<float>(kCMaxBins - 2) / __uint_as_float(static_cast<uint32_t>(e + 1) << 22), FLT_MAX);
+  again();
+  return bound_of_maxima<false, B>(s, *mscale, &through);
+}
+
 // With a top_k: its whole set as an ordered list, then everything on the list. Returns false when there is no such list.
 // *written: the outputs are written (the caller has nothing left to do).
 template <bool F32, bool CACHED, int B>
 static __device__ __noinline__ bool phase_top_k(ClusterSmem& s, const SampleDev& P, bool* written) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, C = s.C;
   *written = false;
-  // the bound: bins of the group maxima (16-bit counts pushed to every block, added up there). Linear ones down to the smallest maximum; where
-  // something far below the rest (a group of nothing but masked logits) has stretched these until the bin of the k-th holds far more than k,
-  // bins by the depth's exponent and one bit find the range that matters and linear ones divide that (4 rows of 151,936, a third at -1e4,
-  // top_k 50: 63 us by the search that an overflowing list leads to, 25 us so; without a mask 19).
+  // the bound: bins of the group maxima, down to the smallest of them
   const float vmax = s.vmax, gmin = s.gmin;
-  const uint32_t k = static_cast<uint32_t>(s.top_k);
   float mscale = static_cast<float>(kCMaxBins - 1) / (vmax > gmin ? vmax - gmin : 1.0f);
-  int pick = -1;
-#pragma unroll 1
-  for (int pass = 0;; pass++) {                                             // 0: linear, 1: by exponent, 2: linear down to what that found
-    if (pass) {
-      cluster_sync(C);                                                      // (the counts of the pass before are no longer read)
-      for (int i = tid; i < kCMaxBins; i += B) s.max_cnt[i] = 0u;
-      __syncthreads();
-    }
-    {
-      const ClusterBins mb{vmax, mscale, -1};
-      const int mine = (s.R.c1 - s.R.c0 - tid + B - 1) / B, groups = (mine + s.every - 1) / s.every;   // (mine may be negative: no group)
-      for (int g = 0; g < groups; g++) {
-        const float m = s.gmax[g * B + tid];
-        if (m > -INFINITY) atomicAdd(&s.max_cnt[pass == 1 ? __float_as_uint(__fsub_rn(vmax, m)) >> 22 : min(mb.coarse(m), static_cast<uint32_t>(kCMaxBins - 1))], 1u);
-      }
-    }
-    __syncthreads();
-    for (int i = tid; i < C * (kCMaxBins / 2); i += B) {                   // (at most 4096 groups a block: 16 bits)
-      const int q = i / (kCMaxBins / 2), w = i - q * (kCMaxBins / 2);
-      cst_u32(cluster_addr(&s.x_max[s.rank][w], q), s.max_cnt[2 * w] | (s.max_cnt[2 * w + 1] << 16));
-    }
-    cluster_sync(C);
-    if (tid < kCMaxBins / 2) {
-      uint32_t n0 = 0u, n1 = 0u;
-      for (int q = 0; q < C; q++) { const uint32_t w = s.x_max[q][tid]; n0 += w & 0xFFFFu; n1 += w >> 16; }
-      s.totals[2 * tid] = n0; s.totals[2 * tid + 1] = n1;
-    }
-    __syncthreads();
-    uint32_t through = 0u;                                                  // the maxima down to the bin of the k-th, that bin included
-    {                                                                       // every warp for itself: lane l holds 16 bins
-      uint32_t v[kCMaxBins / 32], sum = 0u;
-#pragma unroll
-      for (int j = 0; j < kCMaxBins / 32; j += 4) {
-        const uint4 q = *reinterpret_cast<const uint4*>(&s.totals[lane * (kCMaxBins / 32) + j]);
-        v[j] = q.x; v[j + 1] = q.y; v[j + 2] = q.z; v[j + 3] = q.w; sum += q.x + q.y + q.z + q.w;
-      }
-      uint32_t incl = sum;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) { const uint32_t t = __shfl_up_sync(kFull, incl, o); if (lane >= o) incl += t; }
-      uint32_t run = incl - sum; int at = -1;
-#pragma unroll
-      for (int j = 0; j < kCMaxBins / 32; j++) { run += v[j]; if (at < 0 && run >= k) { at = lane * (kCMaxBins / 32) + j; through = run; } }
-      const uint32_t hits = __ballot_sync(kFull, at >= 0);
-      pick = -1;
-      if (hits) { const int who = __ffs(hits) - 1; pick = __shfl_sync(kFull, at, who); through = __shfl_sync(kFull, through, who); }
-    }
-    if (pick < 0 || pass == 2 || (pass == 0 && through <= 2u * k + 64u)) break;
-    // (the k-th lies above the lower edge of its bin by exponent: in the first 511 of the linear bins down to that edge)
-    if (pass == 1) mscale = fminf(static_cast<float>(kCMaxBins - 2) / __uint_as_float(static_cast<uint32_t>(pick + 1) << 22), FLT_MAX);
-  }
+  uint32_t through = 0u;
+  int pick = bound_of_maxima<false, B>(s, mscale, &through);
+  if (pick >= 0 && through > 2u * static_cast<uint32_t>(s.top_k) + 64u) pick = narrower_bound<B>(s, &mscale);
   if (pick < 0) return false;                                               // fewer groups than top_k
   // every logit at or above the bound's bin, and (for a top-p over the row) the FP32 mass: one more look at the row. Not at temperatures so
   // small that the rounding of the maximum's exponent is no fraction of a binade (kMassExponent): there the mass is formed in FP64 at once.
