@@ -81,3 +81,10 @@ def test_host_hash_equals_the_oracle():
     L = _lib.lib()
     for args in [(0, 0, 0, 0), (12345, 7, 3001, 0), (2**63 + 5, 1, 4000, 151935)]:
         assert L.lm_uniform01(*args) == oracle.uniform01(*args)
+
+
+def test_translation_units_are_compiled_whole():
+    """With split compilation the same source gave one kernel or another from build to build, up to 17 % apart in time."""
+    from lithos_metal_b200 import build
+    text = open(build.__file__).read()
+    assert not any("split-compile" in flag for flag in build.NVCC_FLAGS) and '"-split-compile' not in text
