@@ -241,9 +241,11 @@ static __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem&
       const uint32_t key = warp_max_u32(fkey(fmaxf(__low2float(mx), __high2float(mx))));
       if (lane == 0) atomicMax(&c.ref_key, key);
     }
-    // A few candidates more than wanted cost less than another round: a cut is good enough at twice the count wanted while that is small (the
-    // list has room for 2048 candidates), at half as much again in between; a large top_k gets the closest cut.
-    const uint32_t enough = want < 24u ? 2u * want : want < 48u ? want + want / 2u : want;
+    // A few candidates more than wanted cost less than another round: a cut is good enough at twice the count wanted while that is small, at half
+    // as much again in between; a large top_k gets the closest cut. Never more than stand for 1500 candidates in the row: the list holds 2048,
+    // and at the largest vocabularies a sampled logit stands for 32 (512 rows of 262,144, top_k 1000: 60 rows handed on without that bound, 8 with it).
+    const uint32_t most = static_cast<uint32_t>(1500ll * kSampleChunks * kTB * kChunk / V);
+    const uint32_t enough = max(want, min(want < 24u ? 2u * want : want < 48u ? want + want / 2u : want, most));
     uint32_t n_lo = 0xFFFFFFFFu;                                            // count(sample >= lo), once it is known
     uint32_t lo = 0x0000u, hi = 0x7F7Fu;                                    // invariant: count(sample >= lo) >= want, or lo is still 0 (handed back below)
     const uint32_t prev = c.prev_cut[cls];

@@ -146,3 +146,14 @@ def test_penalised_rows_inside_the_fp32_decision_band_are_decided_in_fp64():
     np.testing.assert_array_equal(r.tokens.cpu().numpy(), tok)
     on_candidate_path = (r.status.cpu().numpy() & 64) != 0
     assert on_candidate_path[7::8].all() and not on_candidate_path[::8].any()
+
+
+@pytest.mark.parametrize("top_k", [850, 1000])
+def test_large_top_ks_at_the_largest_vocabularies_stay_on_the_candidate_path(top_k):
+    """The cutoff accepts no more sampled logits than its list of candidates has room for (one stands for 32 here): of 256 rows of N(0, 2^2)
+    about 1.5 % meet an unlucky sample and are handed on, where an eighth of them was when half as many samples again were accepted."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(3)
+    x = torch.cat([(torch.randn(64, 262144, generator=g, device="cuda") * 2).to(torch.bfloat16) for _ in range(4)])
+    r = lm.sample(x, lm.SamplingParams(temperature=0.8, top_k=top_k, top_p=0.9, seed=2), return_status=True)
+    assert int((r.status & 64 == 0).sum()) <= 12                             # binomial(256, 0.015): beyond 12 in 1e-4 of all seeds
