@@ -55,7 +55,7 @@ extern "C" {
 #define LM_FLAG_TOPP_IN_TOPK 1u /* top-p over the top-k set's renormalised mass (the Hugging Face warpers' order) */
 #define LM_FLAG_EXACT_ONLY 2u /* skip the one-pass candidate kernel for rows with a top_k: every row takes the histogram path (same results) */
 #define LM_FLAG_TOKENS_I64 4u /* lm_sample: out_tokens points to int64_t entries (what the reference's sampler modules return) */
-#define LM_FLAG_GRID_LIMIT(n) (((uint32_t)(n) & 0xFFu) << 8) /* at most n thread blocks (0 = one per SM): leaves SMs to other streams */
+#define LM_FLAG_GRID_LIMIT(n) (((uint32_t)(n) & 0xFFu) << 8) /* lm_sample: at most n thread blocks at any time (0 = one per SM): leaves SMs to other streams; a call cut into slices is not limited */
 
 /* per-row status bits written to lm_sample_args.out_status (optional) */
 #define LM_STATUS_GENERIC_PATH 1u /* the row was handled by the generic multi-pass path, or the call asked for statistics or probabilities */

@@ -268,6 +268,9 @@ int lm_sample(const lm_sample_args* a) {
     if (limit > 0 && grid > limit) grid = limit;
     int grid1 = static_cast<int>(a->rows < static_cast<long long>(kTopkPerSM) * sms ? a->rows : static_cast<long long>(kTopkPerSM) * sms);
     if (limit > 0 && grid1 > limit) grid1 = limit;
+    int grid_list = static_cast<int>((a->rows + 255) / 256);
+    if (limit > 0 && grid_list > limit) grid_list = limit;
+    const unsigned overlap = limit > 0 ? 0u : 1u;                          // (launch attributes: two grids at once would be more blocks than the call was allowed)
     if (!topk) {
       sample_hist_kernel<<<grid, kHB, hist_smem, st>>>(P, nullptr, nullptr, counters + 2, redo, counters + 3, nullptr, nullptr, nullptr);
     } else if (one_k || a->rows > static_cast<int64_t>(kOverlapRowsPerSM) * sms) {
@@ -275,7 +278,7 @@ int lm_sample(const lm_sample_args* a) {
       // the histogram kernel behind it with programmatic stream serialization: its blocks take an SM over as the top-k blocks leave it, work
       // through the rows that a one-thread-per-row kernel has listed for it, wait for the top-k grid, and absorb the few rows that one handed
       // on. (Behind its end: 4096 penalised rows 771 us, now 720; 800 rows 210, now 186.)
-      sample_classify_kernel<<<static_cast<int>((a->rows + 255) / 256), 256, 0, st>>>(P, list_other, counters + 4);
+      sample_classify_kernel<<<grid_list, 256, 0, st>>>(P, list_other, counters + 4);
       sample_topk_kernel<<<grid1, kTB, sizeof(TopkSmem), st>>>(P, list_left, counters);
       cudaError_t e = cudaGetLastError();
       if (e != cudaSuccess) return cuda_fail(e);
@@ -284,7 +287,7 @@ int lm_sample(const lm_sample_args* a) {
       cudaLaunchAttribute attr[1];
       attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
       attr[0].val.programmaticStreamSerializationAllowed = 1;
-      cfg.attrs = attr; cfg.numAttrs = 1;
+      cfg.attrs = attr; cfg.numAttrs = overlap;
       e = cudaLaunchKernelEx(&cfg, sample_hist_kernel, P, static_cast<const int*>(list_other), static_cast<const int*>(counters + 4), counters + 2, redo, counters + 3,
                              static_cast<const int*>(list_left), static_cast<const int*>(counters + 1), counters + 5);
       if (e != cudaSuccess) return cuda_fail(e);
@@ -294,13 +297,14 @@ int lm_sample(const lm_sample_args* a) {
       // kernel lists for it; the top-k kernel is launched behind it with programmatic stream serialization and takes the SMs
       // as the histogram kernel's blocks leave them (at once, for the SMs it has no rows for); a second launch of the histogram
       // kernel takes what the top-k kernel handed on (usually nothing: it leaves at once).
-      sample_classify_kernel<<<static_cast<int>((a->rows + 255) / 256), 256, 0, st>>>(P, list_other, counters + 4);
+      sample_classify_kernel<<<grid_list, 256, 0, st>>>(P, list_other, counters + 4);
       // With at most kAloneRowsPerSM rows per SM the histogram kernel's blocks ask for so much shared memory that nothing else fits
       // beside them: a long row then has its SM to itself, and the blocks that find no row leave their SM to the top-k kernel at
       // once (256 rows of the benchmark mix: 112 -> 106 us per call; from 3 rows per SM on it costs time).
       size_t hist_smem_first = hist_smem; int grid_first = grid;
       if (a->rows <= static_cast<int64_t>(kAloneRowsPerSM) * sms && hist_smem < kAloneSmemBytes) {
         hist_smem_first = kAloneSmemBytes; grid_first = static_cast<int>(a->rows < sms ? a->rows : sms);
+        if (limit > 0 && grid_first > limit) grid_first = limit;
         rc = ensure_dynamic_smem(kSlotFast, reinterpret_cast<const void*>(sample_hist_kernel), hist_smem_first);
         if (rc != LM_OK) return rc;
       }
@@ -312,7 +316,7 @@ int lm_sample(const lm_sample_args* a) {
       cudaLaunchAttribute attr[1];
       attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
       attr[0].val.programmaticStreamSerializationAllowed = 1;
-      cfg.attrs = attr; cfg.numAttrs = 1;
+      cfg.attrs = attr; cfg.numAttrs = overlap;
       e = cudaLaunchKernelEx(&cfg, sample_topk_kernel, P, list_left, counters);
       if (e != cudaSuccess) return cuda_fail(e);
       sample_hist_kernel<<<grid, kHB, hist_smem, st>>>(P, list_left, counters + 1, counters + 5, redo, counters + 3, nullptr, nullptr, nullptr);
@@ -325,7 +329,8 @@ int lm_sample(const lm_sample_args* a) {
   rc = ensure_dynamic_smem(kSlotGeneric, reinterpret_cast<const void*>(sample_generic_kernel), smem);
   if (rc != LM_OK) return rc;
   const long long cap = fast ? sms : 8LL * sms;
-  const int grid = static_cast<int>(a->rows < cap ? a->rows : cap);
+  int grid = static_cast<int>(a->rows < cap ? a->rows : cap);
+  if (limit > 0 && grid > limit) grid = limit;
   sample_generic_kernel<<<grid, kBlock, smem, st>>>(P, redo_list, redo_n);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? LM_OK : cuda_fail(e);

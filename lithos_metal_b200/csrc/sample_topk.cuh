@@ -120,11 +120,11 @@ __device__ __forceinline__ bool topk_row_eligible(const SampleDev& P, int row) {
          (reinterpret_cast<uintptr_t>(rowp) & 15u) == 0 && !(P.history != nullptr && P.hist_len > kTopkHist);
 }
 
-// The rows that are not the top-k kernel's, listed for the histogram kernel (one thread per row).
+// The rows that are not the top-k kernel's, listed for the histogram kernel (a thread per row, or per few rows).
 static __global__ void sample_classify_kernel(SampleDev P, int* list, int* n_list) {
   apply_step_state(P);
-  const int row = blockIdx.x * blockDim.x + threadIdx.x;
-  if (row < P.rows && !topk_row_eligible(P, row)) list[atomicAdd(n_list, 1)] = row;
+  for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < P.rows; row += gridDim.x * blockDim.x)
+    if (!topk_row_eligible(P, row)) list[atomicAdd(n_list, 1)] = row;
 }
 
 struct TopkSmem;

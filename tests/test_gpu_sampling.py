@@ -8,7 +8,7 @@ import torch
 
 import oracle
 import lithos_metal_b200 as lm
-from tests import inputs
+from tests import inputs, routes
 
 pytestmark = pytest.mark.gpu
 
@@ -513,3 +513,28 @@ def test_row_maxima_come_out_of_every_kernel_and_feed_the_verify_step():
                 total = C.c_uint64()
                 oracle.lib().lmo_sample_invcdf(z[i].ctypes.data_as(C.POINTER(C.c_float)), z.shape[1], float(r.tau[i]), np.float32(0.8), np.float32(0.3), C.byref(total))
                 assert int(r.mass[i]) == total.value, (draw, knobs, i)
+
+
+@pytest.mark.parametrize("rows", [40, 200, 800])
+def test_a_call_with_a_grid_limit_keeps_to_it(rows):
+    """``grid_limit`` = n: no launch of the call has more than n blocks and none runs beside another, in either order of the two kernels and
+    for rows that neither takes. Without a limit the kernels do overlap."""
+    V = 32768
+    cfg = inputs.config3(rows=rows, vocab=V, hist_len=64, seed=19)
+    x = bf16_tensor(cfg["logits"])
+    knobs = {k: torch.from_numpy(cfg[k]).cuda() for k in ("temperature", "top_k", "top_p")}
+    u = torch.from_numpy(cfg["uniforms"]).cuda()
+    out = torch.empty(rows, dtype=torch.int32, device="cuda")
+
+    def call(logits, limit, **kw):
+        return routes.kernels(lambda: lm.sample(logits, lm.SamplingParams(draw="inverse_cdf", grid_limit=limit, **{**knobs, **kw}), uniforms=u, out=out))[0]
+
+    for kw in ({}, {"top_k": 50}, {"top_k": 0}):
+        launched = call(x, 2, **kw)
+        assert all(grid <= 2 and not beside for _, grid, beside in launched), launched
+        assert launched[-1][0] == "sample_generic_kernel" and any(k == "sample_hist_kernel" for k, _, _ in launched)
+    assert all(grid <= 2 for _, grid, _ in call(x.float(), 2))              # binary32 rows with a limit: the generic kernel
+    a = lm.sample(x, lm.SamplingParams(draw="inverse_cdf", grid_limit=2, **knobs), uniforms=u).tokens
+    assert torch.equal(a, lm.sample(x, lm.SamplingParams(draw="inverse_cdf", **knobs), uniforms=u).tokens)
+    if rows > 74:
+        assert any(beside for _, _, beside in call(x, 0))
