@@ -17,6 +17,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <map>
+#include <mutex>
 #include <tuple>
 
 #include "../../include/lithos_b200.h"
@@ -93,10 +94,12 @@ bool as_u64(PyObject* o, uint64_t* v) {                                     // a
 }
 
 // The stream's scratch (one per device, kind and stream; made and owned by the Python layer, which keeps it for its own calls too).
-// Remembered here with a reference of its own; asked for again when it is too small.
-struct Scratch { at::Tensor t; };
+// Remembered here with a reference of its own; asked for again when it is too small. A call is several launches that pass rows on in this
+// scratch, and it runs without the GIL: two threads on one stream take turns.
+struct Scratch { at::Tensor t; std::mutex turn; };
 std::map<std::tuple<int, int, void*>, Scratch> scratches;
-bool scratch(const at::Device& dev, void* stream, int kind, size_t bytes, void** p, size_t* n) {
+struct Lease { at::Tensor t; std::mutex* turn = nullptr; };                  // (holds the buffer: another thread may replace it meanwhile)
+bool scratch(const at::Device& dev, void* stream, int kind, size_t bytes, Lease* lease, void** p, size_t* n) {
   Scratch& s = scratches[std::make_tuple(static_cast<int>(dev.index()), kind, stream)];
   if (!s.t.defined() || static_cast<size_t>(s.t.numel()) < bytes) {
     Ref d(THPVariable_Wrap(at::detail::empty_cuda({0}, at::kByte, dev, c10::nullopt)));
@@ -109,9 +112,24 @@ bool scratch(const at::Device& dev, void* stream, int kind, size_t bytes, void**
     if (!t) { PyErr_SetString(PyExc_TypeError, "workspace"); return false; }
     s.t = *t;
   }
+  lease->t = s.t; lease->turn = &s.turn;
   *p = ptr(s.t);
   *n = static_cast<size_t>(s.t.numel());
   return true;
+}
+
+// An ABI call, without the GIL as a ctypes call is: a launch can wait (a full launch queue, the first use of a kernel).
+struct NoGil {
+  PyThreadState* state = PyEval_SaveThread();
+  ~NoGil() { PyEval_RestoreThread(state); }
+};
+template <class F>
+int call(const at::Device& dev, std::mutex* turn, F f) {
+  const NoGil released;                                                     // (taken back last, also when the guard throws)
+  std::unique_lock<std::mutex> lock;
+  if (turn) lock = std::unique_lock<std::mutex>(*turn);
+  const c10::cuda::CUDAGuard guard(dev);
+  return f();
 }
 
 PyObject* failed(int rc, const char* what) {                                // the Python layer's exception for an ABI error code
@@ -148,9 +166,9 @@ PyObject* run_sample(lm_sample_args& a, const at::Tensor& x, PyObject* out, int 
   }
   void* stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
   a.stream = stream;
-  if (!scratch(dev, stream, 0, abi.workspace_bytes(rows, vocab), &a.workspace, &a.workspace_bytes)) return nullptr;
-  int rc;
-  { const c10::cuda::CUDAGuard guard(dev); rc = abi.sample(&a); }
+  Lease lease;
+  if (!scratch(dev, stream, 0, abi.workspace_bytes(rows, vocab), &lease, &a.workspace, &a.workspace_bytes)) return nullptr;
+  const int rc = call(dev, lease.turn, [&] { return abi.sample(&a); });
   if (rc != LM_OK) return failed(rc, "lm_sample");
   if (want & kI64) return THPVariable_Wrap(tokens);
   auto wrap = [](const at::Tensor& t) { if (t.defined()) return THPVariable_Wrap(t); Py_INCREF(Py_None); return Py_None; };
@@ -242,12 +260,10 @@ PyObject* py_argmax(PyObject*, PyObject* const* args, Py_ssize_t n) {
     tokens = *t;
   }
   void* stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
-  int rc;
-  {
-    const c10::cuda::CUDAGuard guard(dev);
-    if (i64) rc = abi.argmax_i64(ptr(*x), dtype_code(*x), rows, vocab, row_stride(*x), static_cast<int64_t*>(ptr(tokens)), stream);
-    else rc = abi.argmax(ptr(*x), dtype_code(*x), rows, vocab, row_stride(*x), static_cast<int32_t*>(ptr(tokens)), nullptr, 0, stream);
-  }
+  const int rc = call(dev, nullptr, [&] {
+    return i64 ? abi.argmax_i64(ptr(*x), dtype_code(*x), rows, vocab, row_stride(*x), static_cast<int64_t*>(ptr(tokens)), stream)
+               : abi.argmax(ptr(*x), dtype_code(*x), rows, vocab, row_stride(*x), static_cast<int32_t*>(ptr(tokens)), nullptr, 0, stream);
+  });
   if (rc != LM_OK) return failed(rc, "lm_argmax");
   if (args[1] != Py_None) { Py_INCREF(args[1]); return args[1]; }
   return THPVariable_Wrap(tokens);
@@ -275,9 +291,9 @@ PyObject* py_draft_q(PyObject*, PyObject* const* args, Py_ssize_t n) {
   a.out_mass = static_cast<uint64_t*>(ptr(mass)); a.out_status = static_cast<uint32_t*>(ptr(status));
   void* stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
   a.stream = stream;
-  if (!scratch(dev, stream, 1, abi.verify_workspace_bytes(static_cast<int32_t>(rows), vocab), &a.workspace, &a.workspace_bytes)) return nullptr;
-  int rc;
-  { const c10::cuda::CUDAGuard guard(dev); rc = abi.draft_q(&a); }
+  Lease lease;
+  if (!scratch(dev, stream, 1, abi.verify_workspace_bytes(static_cast<int32_t>(rows), vocab), &lease, &a.workspace, &a.workspace_bytes)) return nullptr;
+  const int rc = call(dev, lease.turn, [&] { return abi.draft_q(&a); });
   if (rc != LM_OK) return failed(rc, "lm_draft_q");
   Ref fields(PyTuple_New(6));
   if (!fields.p) return nullptr;
@@ -355,9 +371,9 @@ PyObject* py_verify(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   if (want_p) { p_draft = make({n}, at::kFloat, dev); a.out_p_draft = static_cast<float*>(ptr(p_draft)); }
   void* stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
   a.stream = stream;
-  if (!scratch(dev, stream, 1, abi.verify_workspace_bytes(static_cast<int32_t>(n), vocab), &a.workspace, &a.workspace_bytes)) return nullptr;
-  int rc;
-  { const c10::cuda::CUDAGuard guard(dev); rc = abi.verify(&a); }
+  Lease lease;
+  if (!scratch(dev, stream, 1, abi.verify_workspace_bytes(static_cast<int32_t>(n), vocab), &lease, &a.workspace, &a.workspace_bytes)) return nullptr;
+  const int rc = call(dev, lease.turn, [&] { return abi.verify(&a); });
   if (rc != LM_OK) return failed(rc, "lm_verify");
   Ref res(PyTuple_New(want_p ? 4 : 3));
   if (!res.p) return nullptr;
@@ -394,8 +410,7 @@ PyObject* py_lm_head(PyObject*, PyObject* const* args, Py_ssize_t n) {
   a.eps = static_cast<float>(PyFloat_AS_DOUBLE(args[3])); a.one_plus = args[4] == Py_True ? 1 : 0;
   a.logits = ptr(out); a.logits_stride = rows > 1 ? out.stride(0) : V;
   a.stream = c10::cuda::getCurrentCUDAStream(x->device().index()).stream();
-  int rc;
-  { const c10::cuda::CUDAGuard guard(x->device()); rc = abi.head(&a); }
+  const int rc = call(x->device(), nullptr, [&] { return abi.head(&a); });
   if (rc != LM_OK) return failed(rc, "lm_head");
   if (args[5] != Py_None) { Py_INCREF(args[5]); return args[5]; }
   return THPVariable_Wrap(out);
