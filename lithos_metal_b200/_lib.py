@@ -6,6 +6,7 @@ import ctypes as C
 import importlib
 import importlib.util
 import os
+import warnings
 
 from . import build as _build
 
@@ -134,7 +135,7 @@ def lib():
     """The loaded library (built on first use if the in-tree shared object is missing or older than its sources)."""
     global _lib
     if _lib is None:
-        path = _build.build() if os.environ.get("LITHOS_B200_NO_BUILD") != "1" else _build.OUT
+        path = _build.build_library() if os.environ.get("LITHOS_B200_NO_BUILD") != "1" else _build.OUT
         if not os.path.exists(path):
             raise RuntimeError(f"lithos_metal_b200: CUDA library {path} is missing; run `python -m lithos_metal_b200.build`")
         L = C.CDLL(path)
@@ -191,19 +192,32 @@ def lib():
     return _lib
 
 
+class _NoHost:
+    """In the place of the native call path where it cannot be had: leaves every call to the Python layer (ctypes)."""
+
+    def _leave(self, *args):
+        return None
+
+    sample = stochastic = argmax = draft_q = verify = lm_head = _leave
+
+
 def host():
-    """The native call path (csrc/host_ext.cpp), handed the addresses of the loaded library's functions and the types it returns."""
+    """The native call path (csrc/host_ext.cpp), handed the addresses of the loaded library's functions and the types it returns. Without
+    a compiler for it, or if it does not load, the calls take the Python layer's way to the same library (about 20 us more of host time each)."""
     global _host
     if _host is None:
         L = lib()
-        spec = importlib.util.spec_from_file_location("lithos_host", _build.HOST_OUT)
-        if not os.path.exists(_build.HOST_OUT):
-            raise RuntimeError(f"lithos_metal_b200: native host layer {_build.HOST_OUT} is missing; run `python -m lithos_metal_b200.build`")
-        m = importlib.util.module_from_spec(spec)
-        spec.loader.exec_module(m)
-        sampler, verify = (importlib.import_module(f"{__package__}.{n}") for n in ("sampler", "verify"))
-        names = ("lm_sample", "lm_argmax", "lm_argmax_i64", "lm_verify", "lm_draft_q", "lm_head", "lm_workspace_bytes", "lm_verify_workspace_bytes")
-        m.init({n: C.cast(getattr(L, n), C.c_void_p).value for n in names}, sampler.SamplingParams, sampler.SampleOutput, verify.DraftQ, check, sampler._workspace)
+        try:
+            path = _build.build_host() if os.environ.get("LITHOS_B200_NO_BUILD") != "1" else _build.HOST_OUT
+            spec = importlib.util.spec_from_file_location("lithos_host", path)
+            m = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(m)
+            sampler, verify = (importlib.import_module(f"{__package__}.{n}") for n in ("sampler", "verify"))
+            names = ("lm_sample", "lm_argmax", "lm_argmax_i64", "lm_verify", "lm_draft_q", "lm_head", "lm_workspace_bytes", "lm_verify_workspace_bytes")
+            m.init({n: C.cast(getattr(L, n), C.c_void_p).value for n in names}, sampler.SamplingParams, sampler.SampleOutput, verify.DraftQ, check, sampler._workspace)
+        except (ImportError, OSError, RuntimeError) as e:
+            warnings.warn(f"lithos_metal_b200: no native call path ({e}); calls go through ctypes", RuntimeWarning, stacklevel=3)
+            m = _NoHost()
         _host = m
     return _host
 

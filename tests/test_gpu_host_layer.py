@@ -87,3 +87,63 @@ def test_threads_that_share_a_stream_take_turns_with_its_workspace():
     for t in threads:
         t.join()
     assert not wrong
+
+
+def test_calls_give_the_same_with_and_without_the_native_path(monkeypatch):
+    """What host_ext.cpp takes, what it leaves to Python (other types, layouts and knobs) and what both refuse."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(8)
+    x = (torch.randn(8, 40000, generator=g, device="cuda") * 2).to(torch.bfloat16)
+    hist = torch.randint(0, 40000, (8, 100), generator=g, device="cuda")
+    u = torch.rand(8, generator=g, device="cuda")
+    w = torch.randn(1000, 128, generator=g, device="cuda").to(torch.bfloat16)
+    h = torch.randn(8, 128, generator=g, device="cuda").to(torch.bfloat16)
+    ids = torch.randint(0, 40000, (7,), generator=g, device="cuda")
+    q = torch.softmax(x[:7].float(), -1)
+    K = torch.arange(8, device="cuda")
+
+    def flat(r):
+        r = list(vars(r).values()) if isinstance(r, lm.SampleOutput) else list(r) if isinstance(r, tuple) else [r]
+        return [t for t in r if isinstance(t, torch.Tensor)]
+
+    def out_of(call):
+        try:
+            return [t.clone() for t in flat(call())]
+        except (ValueError, TypeError, RuntimeError) as e:
+            return type(e), str(e)
+
+    everything = dict(return_tau=True, return_stats=True, return_probs=True, return_status=True, return_vmax=True)
+    draft = lm.draft_q(x[:7], temperature=0.9, seed=4)
+    calls = [
+        lambda: lm.sample(x, temperature=0.8, top_k=20, top_p=0.9, seed=2, step=3, row_offset=5, **everything),
+        lambda: lm.sample(x, temperature=1, top_k=20.0, seed=-1, step=-1, **everything),                            # knobs of other types, masked to 64 and 32 bits
+        lambda: lm.sample(x, temperature=u + 0.3, top_k=K, top_p=u.double(), min_p=0.01, seed=1 << 70, **everything),   # per-row knobs that need a conversion
+        lambda: lm.sample(x, temperature=u + 0.3, top_k=K.int(), top_p=u, history=hist, repetition_penalty=1.2, draw="inverse_cdf", uniforms=u, **everything),
+        lambda: lm.sample(x, temperature=0.8, history=hist.int(), presence_penalty=0.5, draw="inverse_cdf", uniforms=u.cpu(), **everything),
+        lambda: lm.sample(x[:, ::2], temperature=0.8, top_p=0.9, **everything),                                     # a stride along the vocabulary
+        lambda: lm.sample(x[2:3].expand(4, -1), temperature=0.8),                                                   # refused: rows on top of one another
+        lambda: lm.sample(x[3:4, 5:999], temperature=0.8, top_p=0.9, **everything),
+        lambda: lm.sample(x[:0], temperature=0.8, **everything),
+        lambda: lm.sample(x, temperature=0.8, out=torch.empty(8, dtype=torch.int32, device="cuda")),
+        lambda: lm.sample(x, temperature=0.8, out=torch.empty(7, dtype=torch.int32, device="cuda")),
+        lambda: lm.sample(x, temperature=float("nan")), lambda: lm.sample(x, temperature=-0.5), lambda: lm.sample(x.half(), temperature=1.0), lambda: lm.sample(x.cpu(), temperature=1.0),
+        lambda: lm.sample(x, temperature=0.8, draw="other"), lambda: lm.sample(x, temperature=0.8, draw="inverse_cdf"), lambda: lm.sample(x, temperature=0.8, top_k=K[:3]),
+        lambda: lm.sample(x, temperature=0.8, repetition_penalty=0.0), lambda: lm.sample(x, temperature=0.8, history=hist[:3]), lambda: lm.sample(x[0], temperature=0.8),
+        lambda: lm.argmax(x), lambda: lm.argmax(x.float()), lambda: lm.argmax(x.t()), lambda: lm.argmax(x, out=torch.empty(8, dtype=torch.int32, device="cuda")), lambda: lm.argmax(x[0]),
+        lambda: lm.GreedySampler().forward(x), lambda: lm.StochasticSampler(0.7, 20, 0.9, seed=3).forward(x, 4), lambda: lm.StochasticSampler(0.7, 20, 0.9).forward(x.float()[:, ::2]),
+        lambda: lm.draft_q(x[:7], temperature=0.9, seed=4, step=2, first_position=3), lambda: lm.draft_q(x[:7], temperature=0.9, copy_logits=True), lambda: lm.draft_q(x, temperature=0.0),
+        lambda: lm.draft_q(torch.cat([x] * 3), temperature=0.5),
+        lambda: lm.verify(x, ids), lambda: lm.verify(x, ids.int(), q, u[:7], u[:1], "stochastic", temperature=0.9, return_p_draft=True),
+        lambda: lm.verify(x, ids, None, u[:7].cpu(), 0.3 * u[:1], "stochastic", temperature=0.9, draft_logits=x[:7], draft_stats=draft, seed=3, step=1, residual_draw="gumbel"),
+        lambda: lm.verify(x, ids, None, None, None, "stochastic"), lambda: lm.verify(x, ids[:3]), lambda: lm.verify(x, ids, q[:3], mode="stochastic"), lambda: lm.verify(x, ids, mode="other"),
+        lambda: lm.lm_head(h, w), lambda: lm.lm_head(h, w, h[0], eps=1, one_plus=False), lambda: lm.lm_head(h, w[:, :64]), lambda: lm.lm_head(torch.cat([h, h]), w), lambda: lm.lm_head(h.float(), w),
+    ]
+    native = [out_of(c) for c in calls]
+    monkeypatch.setattr(_lib, "_host", _lib._NoHost())
+    for i, (a, c) in enumerate(zip(native, calls)):
+        b = out_of(c)
+        if isinstance(a, tuple):
+            assert a == b, i
+        else:
+            assert isinstance(b, list) and len(a) == len(b), (i, b)
+            assert all(s.dtype == t.dtype and s.shape == t.shape and torch.equal(s, t) for s, t in zip(a, b)), i
