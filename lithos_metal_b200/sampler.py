@@ -240,7 +240,9 @@ class StochasticSampler:
         return SamplingParams(self.temperature, self.top_k, self.top_p, self.min_p, self.seed, self.topp_in_topk, draw="gumbel")
 
     def forward(self, logits: torch.Tensor, step: int = 0) -> torch.Tensor:
-        r = _lib.host().stochastic(logits, self.temperature, self.top_k, self.top_p, self.min_p, self.seed, self.topp_in_topk, step)
+        r = None
+        if type(self).params is StochasticSampler.params:                    # (a subclass may form its knobs itself)
+            r = _lib.host().stochastic(logits, self.temperature, self.top_k, self.top_p, self.min_p, self.seed, self.topp_in_topk, step)
         return r if r is not None else sample(logits, self.params(), step=step).tokens.to(torch.int64)
 
     __call__ = forward

@@ -147,3 +147,14 @@ def test_calls_give_the_same_with_and_without_the_native_path(monkeypatch):
         else:
             assert isinstance(b, list) and len(a) == len(b), (i, b)
             assert all(s.dtype == t.dtype and s.shape == t.shape and torch.equal(s, t) for s, t in zip(a, b)), i
+
+
+def test_a_subclass_of_the_stochastic_sampler_forms_its_own_knobs():
+    class Annealed(lm.StochasticSampler):
+        def params(self):
+            p = super().params()
+            p.top_k = 1
+            return p
+
+    x = (torch.randn(4, 4096, device="cuda") * 2).to(torch.bfloat16)
+    assert torch.equal(Annealed(temperature=2.0, seed=5).forward(x), x.float().argmax(-1))
