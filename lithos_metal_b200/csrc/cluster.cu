@@ -32,41 +32,71 @@ static int sample_blocks(int64_t rows, int64_t vocab, int sms, bool listed) {
   return c;
 }
 
+// The instances of the sampler: FP32 / BF16 rows, the slices cached in shared memory or not, and then one block per SM or two.
+constexpr size_t kMostSmem = 227 * 1024, kHalfSmem = kMostSmem / 2 - 1024;
+struct ClusterPlan { int C; size_t smem; bool cached, two; };
+
 template <bool F32, bool CACHED, int kPerSM>
-static int launch_cluster(const SampleDev& P, int C, size_t smem, int instance, cudaStream_t st) {
+static int cluster_ready(int instance, int C, bool* fits) {
   const void* fn = reinterpret_cast<const void*>(sample_cluster_kernel<F32, CACHED, kClusterBlock, kPerSM>);
-  const int rc = ensure_dynamic_smem(static_cast<KernelSlot>(kSlotCluster + instance), fn, smem, true);
-  if (rc != LM_OK) return rc;
+  const KernelSlot slot = static_cast<KernelSlot>(kSlotCluster + instance);
+  const size_t most = kPerSM == 2 ? kHalfSmem : kMostSmem;                  // (what any call of the instance may need: one answer for all of them)
+  const int rc = ensure_dynamic_smem(slot, fn, most, true);
+  *fits = rc == LM_OK && (C == 1 || cluster_fits(slot, fn, kClusterBlock, most, C));
+  return rc;
+}
+static int cluster_ready(bool f32, const ClusterPlan& p, bool* fits) {
+  if (p.cached) return f32 ? cluster_ready<true, true, 1>(0, p.C, fits) : cluster_ready<false, true, 1>(1, p.C, fits);
+  if (p.two) return f32 ? cluster_ready<true, false, 2>(2, p.C, fits) : cluster_ready<false, false, 2>(3, p.C, fits);
+  return f32 ? cluster_ready<true, false, 1>(4, p.C, fits) : cluster_ready<false, false, 1>(5, p.C, fits);
+}
+
+template <bool F32, bool CACHED, int kPerSM>
+static int launch_cluster(const SampleDev& P, const ClusterPlan& p, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(P.rows) * static_cast<unsigned>(C)); cfg.blockDim = dim3(kClusterBlock); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cfg.gridDim = dim3(static_cast<unsigned>(P.rows) * static_cast<unsigned>(p.C)); cfg.blockDim = dim3(kClusterBlock); cfg.dynamicSmemBytes = p.smem; cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = static_cast<unsigned>(C); attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr; cfg.numAttrs = C > 1 ? 1 : 0;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, sample_cluster_kernel<F32, CACHED, kClusterBlock, kPerSM>, P, C);
+  attr[0].val.clusterDim.x = static_cast<unsigned>(p.C); attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = p.C > 1 ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, sample_cluster_kernel<F32, CACHED, kClusterBlock, kPerSM>, P, p.C);
   return e == cudaSuccess ? LM_OK : cuda_fail(e);
 }
 
 int sample_clusters(const SampleDev& P, int sms, cudaStream_t st) {
-  const int C = sample_blocks(P.rows, P.vocab, sms, P.top_k == nullptr && P.top_k_s >= 1 && P.top_k_s <= kCListK && !(P.flags & LM_FLAG_EXACT_ONLY));
-  const size_t per = (static_cast<size_t>((P.vocab + 14) / 8) + C - 1) / C;    // chunks of a slice, for any alignment of the row
-  const bool pen = P.history != nullptr && P.hist_len > 0;
-  const size_t head = cluster_smem_head(), marks = pen ? (per + 15) / 16 * 16 : 0;
+  const bool pen = P.history != nullptr && P.hist_len > 0, f32 = P.dtype == LM_DTYPE_F32;
+  const size_t head = cluster_smem_head();
   const size_t generic = sizeof(GenericSmem) + (pen ? static_cast<size_t>((P.vocab + 31) / 32) * 4 : 0) + 16;
-  constexpr size_t kMost = 227 * 1024;
-  const bool cached = head + per * 32 + marks <= kMost && C > 1;             // (a block per row reads its row from L2: two of them share an SM)
-  size_t smem = head + (cached ? per * 32 : 0) + marks;
-  if (smem < generic) smem = generic;
-  const bool f32 = P.dtype == LM_DTYPE_F32, two = static_cast<long long>(P.rows) * C > sms && smem <= kMost / 2 - 1024;   // two blocks per SM
-  if (cached) return f32 ? launch_cluster<true, true, 1>(P, C, smem, 0, st) : launch_cluster<false, true, 1>(P, C, smem, 1, st);
-  if (two) return f32 ? launch_cluster<true, false, 2>(P, C, smem, 2, st) : launch_cluster<false, false, 2>(P, C, smem, 3, st);
-  return f32 ? launch_cluster<true, false, 1>(P, C, smem, 4, st) : launch_cluster<false, false, 1>(P, C, smem, 5, st);
+  auto plan = [&](int C) {
+    const size_t per = (static_cast<size_t>((P.vocab + 14) / 8) + C - 1) / C;    // chunks of a slice, for any alignment of the row
+    const size_t marks = pen ? (per + 15) / 16 * 16 : 0;
+    ClusterPlan p;
+    p.C = C;
+    p.cached = head + per * 32 + marks <= kMostSmem && C > 1;              // (a block per row reads its row from L2: two of them share an SM)
+    p.smem = head + (p.cached ? per * 32 : 0) + marks;
+    if (p.smem < generic) p.smem = generic;
+    p.two = static_cast<long long>(P.rows) * C > sms && p.smem <= kHalfSmem;   // two blocks per SM
+    return p;
+  };
+  int rc = LM_OK;
+  bool fits = false;
+  const int most = sample_blocks(P.rows, P.vocab, sms, P.top_k == nullptr && P.top_k_s >= 1 && P.top_k_s <= kCListK && !(P.flags & LM_FLAG_EXACT_ONLY));
+  const int C = cluster_that_fits(most, [&](int c) { rc = cluster_ready(f32, plan(c), &fits); return fits || rc != LM_OK; });
+  const ClusterPlan p = plan(C);
+  if (rc == LM_OK && C == 1) rc = cluster_ready(f32, p, &fits);
+  if (rc != LM_OK) return rc;
+  if (p.cached) return f32 ? launch_cluster<true, true, 1>(P, p, st) : launch_cluster<false, true, 1>(P, p, st);
+  if (p.two) return f32 ? launch_cluster<true, false, 2>(P, p, st) : launch_cluster<false, false, 2>(P, p, st);
+  return f32 ? launch_cluster<true, false, 1>(P, p, st) : launch_cluster<false, false, 1>(P, p, st);
 }
 
 template <bool F32>
 static int launch_argmax(const void* logits, int rows, int vocab, int64_t row_stride, int32_t* out32, int64_t* out64, int C, cudaStream_t st) {
-  const int rc = ensure_dynamic_smem(static_cast<KernelSlot>(kSlotArgmax + (F32 ? 1 : 0)), reinterpret_cast<const void*>(argmax_cluster_kernel<F32>), 1, true);
+  const KernelSlot slot = static_cast<KernelSlot>(kSlotArgmax + (F32 ? 1 : 0));
+  const void* fn = reinterpret_cast<const void*>(argmax_cluster_kernel<F32>);
+  const int rc = ensure_dynamic_smem(slot, fn, 1, true);
   if (rc != LM_OK) return rc;
+  C = cluster_that_fits(C, [&](int c) { return cluster_fits(slot, fn, kArgmaxThreads, 0, c); });
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(rows) * static_cast<unsigned>(C)); cfg.blockDim = dim3(kArgmaxThreads); cfg.stream = st;
   cudaLaunchAttribute attr[1];
@@ -88,8 +118,11 @@ int argmax_clusters(const void* logits, int dtype, int rows, int vocab, int64_t 
 
 template <bool F32>
 static int launch_draft_q(const DraftQDev& P, int C, cudaStream_t st) {
-  const int rc = ensure_dynamic_smem(static_cast<KernelSlot>(kSlotDraftQ + (F32 ? 1 : 0)), reinterpret_cast<const void*>(draft_q_kernel<F32>), 1, true);
+  const KernelSlot slot = static_cast<KernelSlot>(kSlotDraftQ + (F32 ? 1 : 0));
+  const void* fn = reinterpret_cast<const void*>(draft_q_kernel<F32>);
+  const int rc = ensure_dynamic_smem(slot, fn, 1, true);
   if (rc != LM_OK) return rc;
+  C = cluster_that_fits(C, [&](int c) { return cluster_fits(slot, fn, kDraftQThreads, 0, c); });
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(P.rows) * static_cast<unsigned>(C)); cfg.blockDim = dim3(kDraftQThreads); cfg.stream = st;
   cudaLaunchAttribute attr[1];

@@ -58,6 +58,37 @@ inline int ensure_dynamic_smem(KernelSlot slot, const void* func, size_t bytes, 
   return LM_OK;
 }
 
+// The largest cluster of at most `want` blocks (a power of two) of which `fits` says that the device can hold one; 1 needs no cluster.
+template <class Fits> inline int cluster_that_fits(int want, Fits fits) {
+  while (want > 1 && !fits(want)) want >>= 1;
+  return want;
+}
+
+// Whether the device (a partition of it, a context limited in its SMs) can hold a cluster of C such blocks at all: 16 are beyond what every
+// device guarantees, and a cluster lies within one group of SMs. Asked once per device, kernel and C. The kernel has been let have `smem`.
+inline bool cluster_fits(KernelSlot slot, const void* func, int threads, size_t smem, int C) {
+  constexpr int kMaxDevices = 64;
+  static std::mutex mutex;
+  static unsigned char yes[kMaxDevices][kSlotCount] = {}, no[kMaxDevices][kSlotCount] = {};   // a bit per log2 C
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return C <= 8;
+  unsigned char bit = 1;
+  for (int c = C; c > 1; c >>= 1) bit = static_cast<unsigned char>(bit << 1);
+  std::lock_guard<std::mutex> lock(mutex);
+  if (yes[dev][slot] & bit) return true;
+  if (no[dev][slot] & bit) return false;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(C)); cfg.blockDim = dim3(static_cast<unsigned>(threads)); cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(C); attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, func, &cfg) != cudaSuccess) { n = 0; (void)cudaGetLastError(); }
+  (n > 0 ? yes : no)[dev][slot] |= bit;
+  return n > 0;
+}
+
 inline size_t align256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
 
 struct SampleDev;

@@ -7,6 +7,7 @@ import subprocess
 import tempfile
 
 from lithos_metal_b200 import _lib
+from lithos_metal_b200 import build as _build
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 HEADER = os.path.join(ROOT, "include", "lithos_b200.h")
@@ -85,6 +86,18 @@ def test_host_hash_equals_the_oracle():
 
 def test_translation_units_are_compiled_whole():
     """With split compilation the same source gave one kernel or another from build to build, up to 17 % apart in time."""
-    from lithos_metal_b200 import build
-    text = open(build.__file__).read()
-    assert not any("split-compile" in flag for flag in build.NVCC_FLAGS) and '"-split-compile' not in text
+    text = open(_build.__file__).read()
+    assert not any("split-compile" in flag for flag in _build.NVCC_FLAGS) and '"-split-compile' not in text
+
+
+def test_a_cluster_that_does_not_fit_is_halved():
+    """The rule for devices (partitions, SM-limited contexts) that cannot hold a cluster of 16 blocks: the largest power of two that fits."""
+    src = '#include <cstdio>\n#include "host.cuh"\nint main(){int asked=0;for(int most: {16, 8, 4, 2, 1, 0})for(int want: {16, 4, 1})' \
+          'printf("%d ", lm::cluster_that_fits(want, [&](int c) { asked++; return c <= most; }));printf("%d\\n", asked);return 0;}\n'
+    with tempfile.TemporaryDirectory() as d:
+        open(os.path.join(d, "t.cpp"), "w").write(src)
+        cuda = os.path.dirname(os.path.dirname(os.path.realpath(_build._nvcc())))
+        subprocess.run(["g++", "-std=c++17", "-O1", "-I", os.path.join(ROOT, "lithos_metal_b200", "csrc"), "-I", os.path.join(cuda, "include"), "-o", os.path.join(d, "t"),
+                        os.path.join(d, "t.cpp"), "-L", os.path.join(cuda, "lib64"), "-lcudart"], check=True)
+        out = subprocess.run([os.path.join(d, "t")], capture_output=True, text=True, check=True, env={**os.environ, "LD_LIBRARY_PATH": os.path.join(cuda, "lib64")}).stdout.split()
+    assert [int(x) for x in out[:-1]] == [min(want, max(most, 1)) for most in (16, 8, 4, 2, 1, 0) for want in (16, 4, 1)]
