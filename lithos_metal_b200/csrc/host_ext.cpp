@@ -97,7 +97,7 @@ bool as_u64(PyObject* o, uint64_t* v) {                                     // a
 // Remembered here with a reference of its own; asked for again when it is too small. A call is several launches that pass rows on in this
 // scratch, and it runs without the GIL: two threads on one stream take turns.
 struct Scratch { at::Tensor t; std::mutex turn; };
-std::map<std::tuple<int, int, void*>, Scratch> scratches;
+auto& scratches = *new std::map<std::tuple<int, int, void*>, Scratch>;     // (never destroyed: at exit the allocator may be gone before it)
 struct Lease { at::Tensor t; std::mutex* turn = nullptr; };                  // (holds the buffer: another thread may replace it meanwhile)
 bool scratch(const at::Device& dev, void* stream, int kind, size_t bytes, Lease* lease, void** p, size_t* n) {
   Scratch& s = scratches[std::make_tuple(static_cast<int>(dev.index()), kind, stream)];
