@@ -137,6 +137,13 @@ def warped_probabilities(z: np.ndarray, *, temperature: float = 1.0, top_k: int 
     return out
 
 
+def kept_mass(z: np.ndarray, tau: float, temperature: float) -> int:
+    """The kept set's integer mass: the fixed-point weights of the logits >= tau."""
+    z, total = _f32(z), C.c_uint64()
+    lib().lmo_sample_invcdf_index(_p(z, C.c_float), z.size, np.float32(tau), np.float32(temperature), np.float32(0.0), C.byref(total))
+    return total.value
+
+
 def sample_invcdf(z: np.ndarray, u: float, *, temperature: float = 1.0, top_k: int = 0, top_p: float = 0.0, min_p: float = 0.0,
                   topp_in_topk: bool = False) -> int:
     z = _f32(z)

@@ -26,12 +26,18 @@ def _check(x, host, knobs, *, draw, history=None, rho=1.0, pi=0.0, seed=3, step=
                                        row_offset=row_offset, topp_in_topk=topp_in_topk, n_threads=8, **knobs)
     status = r.status.cpu().numpy()
     np.testing.assert_array_equal(r.tau.cpu().numpy(), tau)
+    vmax, mass = r.vmax.cpu().numpy(), r.mass.cpu().numpy()
+    z = oracle.bf16_to_f32(host) if host.dtype == np.uint16 else host
+    for i in range(rows):                                                   # what the verification takes over: the maximum and the kept integer mass
+        zi = z[i] if history is None else oracle.apply_penalties(z[i], history[i], rho, pi)
+        t = knobs["temperature"][i] if isinstance(knobs["temperature"], np.ndarray) else knobs["temperature"]
+        assert vmax[i] == zi.max(), i
+        assert t == 0 or int(mass[i]) == oracle.kept_mass(zi, tau[i], t), i
     assert np.all((r.tokens.cpu().numpy() == tok) | ((status & 4) != 0)), np.nonzero(r.tokens.cpu().numpy() != tok)
     if stats:
         np.testing.assert_allclose(r.stats.cpu().numpy(), st, rtol=1e-6)
         pr = r.probs.cpu().numpy().astype(np.float64)
         np.testing.assert_allclose(pr.sum(-1), 1.0, rtol=1e-5)
-        z = oracle.bf16_to_f32(host) if host.dtype == np.uint16 else host
         for i in range(rows):
             zi = z[i] if history is None else oracle.apply_penalties(z[i], history[i], rho, pi)
             t = knobs["temperature"][i] if isinstance(knobs["temperature"], np.ndarray) else knobs["temperature"]

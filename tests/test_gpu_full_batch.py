@@ -9,7 +9,7 @@ import torch
 import bench
 import lithos_metal_b200 as lm
 import oracle
-from tests import inputs
+from tests import inputs, routes
 from tests.test_gpu_sampling import bf16_tensor
 
 pytestmark = pytest.mark.gpu
@@ -54,10 +54,10 @@ def test_every_row_of_the_benchmark_workload():
 
 
 def test_rows_on_the_edge_of_the_fp32_decision_band():
-    """The candidate kernel knows the row's mass only in FP32 and hands a row on when a cumulative-mass boundary lies inside its
+    """The candidate kernel knows the row's mass only in FP32 and forms it again in FP64 when a cumulative-mass boundary lies inside its
     error band around top_p * Z. Here top_p is placed at relative distances 0 .. 1e-4 on both sides of an exact boundary inside the
-    top-k set: whichever kernel finishes the row, the threshold must be the oracle's (FP64). Far from the boundary the candidate
-    kernel must keep the row (the band is narrow)."""
+    top-k set: however the row is decided, the threshold must be the oracle's (FP64). Far from the boundary the FP32 mass must do
+    (the band is narrow)."""
     base = inputs.config3(rows=8, seed=77)
     deltas = np.array([0.0, 3e-7, -3e-7, 1e-6, -1e-6, 3e-6, -3e-6, 1e-5, -1e-5, 3e-5, -3e-5, 1e-4, -1e-4])
     rows = []
@@ -122,8 +122,10 @@ def test_draw_over_runs_of_equal_logits_from_both_sources(exact_only):
     assert mixed >= 3, mixed
 
 
-def test_penalised_rows_inside_the_fp32_decision_band_are_decided_in_fp64():
-    """As above with penalties: the candidate kernel forms the mass again in FP64, penalised positions at their penalised values."""
+@pytest.mark.parametrize("copies,one_k,kernel", [(1, False, "sample_cluster_kernel"), (2, False, "sample_topk_kernel"), (2, True, "sample_topk_kernel")])
+def test_penalised_rows_inside_the_fp32_decision_band_are_decided_in_fp64(copies, one_k, kernel):
+    """As above with penalties: the mass is formed again in FP64, penalised positions at their penalised values; by the cluster kernel (48 rows)
+    and by the candidate kernel (96), beside the histogram kernel's rows or, with one top_k for all, ahead of them."""
     rng = np.random.default_rng(31)
     vocab, T, rho, pi = 40008, np.float32(0.7), 1.2, 0.4
     codes = oracle.f32_to_bf16((rng.standard_normal(vocab) * 2.0).astype(np.float32))
@@ -133,13 +135,18 @@ def test_penalised_rows_inside_the_fp32_decision_band_are_decided_in_fp64():
     vals, counts = vals[::-1], counts[::-1]
     cum = np.cumsum(counts * np.exp((vals - vals[0]) / np.float64(T)))
     top_p = np.array([cum[int(np.searchsorted(np.cumsum(counts), n))] / cum[-1] * (1.0 + d) for n in (60, 150, 250, 333, 390, 450)
-                      for d in (0.0, 1e-7, -1e-7, 4e-7, -4e-7, 1e-6, -1e-6, 1e-4)], dtype=np.float32)
+                      for d in (0.0, 1e-7, -1e-7, 4e-7, -4e-7, 1e-6, -1e-6, 1e-4)] * copies, dtype=np.float32)
     n = len(top_p)
     cfg = dict(logits=np.tile(codes, (n, 1)), temperature=np.full(n, T, np.float32), top_k=np.full(n, 600, np.int32), top_p=top_p)
     u = np.linspace(0.02, 0.98, n).astype(np.float32)
-    r = lm.sample(torch.from_numpy(cfg["logits"].view(np.int16)).cuda().view(torch.bfloat16),
-                  lm.SamplingParams(draw="inverse_cdf", repetition_penalty=rho, presence_penalty=pi, **{k: torch.from_numpy(cfg[k]).cuda() for k in ("temperature", "top_k", "top_p")}),
-                  history=torch.from_numpy(np.tile(hist, (n, 1))).cuda(), uniforms=torch.from_numpy(u).cuda(), return_tau=True, return_status=True)
+    x, h, ut = bf16_tensor(cfg["logits"]), torch.from_numpy(np.tile(hist, (n, 1))).cuda(), torch.from_numpy(u).cuda()
+    knobs = {k: torch.from_numpy(cfg[k]).cuda() for k in ("temperature", "top_k", "top_p")}
+    if one_k:
+        knobs["top_k"] = 600
+    p = lm.SamplingParams(draw="inverse_cdf", repetition_penalty=rho, presence_penalty=pi, **knobs)
+    launched = routes.names(lambda: lm.sample(x, p, history=h, uniforms=ut))
+    assert kernel in launched and (len(launched) == 1) == (copies == 1), launched
+    r = lm.sample(x, p, history=h, uniforms=ut, return_tau=True, return_status=True)
     tok, tau, _ = oracle.sample_batch(cfg["logits"], temperature=cfg["temperature"], top_k=cfg["top_k"], top_p=top_p, history=np.tile(hist, (n, 1)), repetition_penalty=rho,
                                       presence_penalty=pi, draw="inverse_cdf", uniforms=u, n_threads=THREADS)
     np.testing.assert_array_equal(r.tau.cpu().numpy(), tau)

@@ -108,15 +108,20 @@ def test_config1_single_fp32_row(golden):
 
 
 def run_both(cfg, draw, rows, seed=77, step=3, row_offset=0, **extra):
-    """The same batch through the CUDA library and through the CPU oracle."""
+    """The same batch through the CUDA library and through the CPU oracle. Statistics are asked for: the cluster kernel takes the call, or
+    with a grid limit the generic one."""
     x = bf16_tensor(cfg["logits"][:rows]) if cfg["logits"].dtype == np.uint16 else torch.from_numpy(cfg["logits"][:rows]).cuda()
     knobs = {k: torch.from_numpy(cfg[k][:rows]).cuda() for k in ("temperature", "top_k", "top_p") if k in cfg}
     hist = cfg.get("history")
-    r = lm.sample(x, lm.SamplingParams(seed=seed, draw=draw, repetition_penalty=cfg.get("repetition_penalty", 1.0),
-                                       presence_penalty=cfg.get("presence_penalty", 0.0), **knobs, **extra),
-                  history=None if hist is None else torch.from_numpy(hist[:rows]).cuda(),
-                  uniforms=torch.from_numpy(cfg["uniforms"][:rows]).cuda(), step=step, row_offset=row_offset,
-                  return_tau=True, return_stats=True, return_status=True)
+    p = lm.SamplingParams(seed=seed, draw=draw, repetition_penalty=cfg.get("repetition_penalty", 1.0), presence_penalty=cfg.get("presence_penalty", 0.0), **knobs, **extra)
+    h = None if hist is None else torch.from_numpy(hist[:rows]).cuda()
+    u = torch.from_numpy(cfg["uniforms"][:rows]).cuda()
+
+    def call():
+        return lm.sample(x, p, history=h, uniforms=u, step=step, row_offset=row_offset, return_tau=True, return_stats=True, return_status=True)
+
+    assert routes.names(call) == ["sample_generic_kernel" if extra.get("grid_limit") else "sample_cluster_kernel"]
+    r = call()
     tok, tau, stats = oracle.sample_batch(cfg["logits"][:rows], temperature=cfg["temperature"][:rows], top_k=cfg["top_k"][:rows],
                                           top_p=cfg["top_p"][:rows], history=None if hist is None else hist[:rows],
                                           repetition_penalty=cfg.get("repetition_penalty", 1.0), presence_penalty=cfg.get("presence_penalty", 0.0),
@@ -126,11 +131,13 @@ def run_both(cfg, draw, rows, seed=77, step=3, row_offset=0, **extra):
 
 
 @pytest.mark.parametrize("draw", ["inverse_cdf", "gumbel"])
-def test_penalised_batch_equals_the_oracle(draw):
-    """Benchmark configuration 3 (per-row knobs, 2048-id histories, both penalties) on its first rows."""
+@pytest.mark.parametrize("limit", [0, 255])
+def test_penalised_batch_equals_the_oracle(draw, limit):
+    """Benchmark configuration 3 (per-row knobs, 2048-id histories, both penalties) on its first rows; statistics are asked for, which the
+    cluster kernel forms, or (``limit``: a grid limit) the generic one."""
     rows = 24
     cfg = inputs.config3(rows=rows)
-    r, tok, tau, stats = run_both(cfg, draw, rows, row_offset=1000)
+    r, tok, tau, stats = run_both(cfg, draw, rows, row_offset=1000, grid_limit=limit)
     np.testing.assert_array_equal(r.tau.cpu().numpy(), tau)
     status = r.status.cpu().numpy()
     got = r.tokens.cpu().numpy()
@@ -143,7 +150,8 @@ def test_penalised_batch_equals_the_oracle(draw):
 
 @pytest.mark.parametrize("vocab,rows", [(300, 5), (1000, 7), (8191, 3), (32768, 4)])
 @pytest.mark.parametrize("dtype", ["bf16", "f32"])
-def test_small_and_ragged_vocabularies(vocab, rows, dtype):
+@pytest.mark.parametrize("limit", [0, 255])
+def test_small_and_ragged_vocabularies(vocab, rows, dtype, limit):
     rng = np.random.default_rng(vocab)
     z = (rng.standard_normal((rows, vocab)) * 3).astype(np.float32)
     cfg = dict(logits=oracle.f32_to_bf16(z) if dtype == "bf16" else z, temperature=rng.uniform(0.3, 1.5, rows).astype(np.float32),
@@ -151,14 +159,15 @@ def test_small_and_ragged_vocabularies(vocab, rows, dtype):
                history=rng.integers(-2, vocab + 2, (rows, 64)).astype(np.int32), uniforms=rng.random(rows).astype(np.float32),
                repetition_penalty=1.3, presence_penalty=0.25)
     for draw in ("inverse_cdf", "gumbel"):
-        r, tok, tau, stats = run_both(cfg, draw, rows, min_p=0.01)
+        r, tok, tau, stats = run_both(cfg, draw, rows, min_p=0.01, grid_limit=limit)
         np.testing.assert_array_equal(r.tau.cpu().numpy(), tau)
         status = r.status.cpu().numpy()
         assert np.all((r.tokens.cpu().numpy() == tok) | ((status & 4) != 0))
         np.testing.assert_allclose(r.stats.cpu().numpy(), stats, rtol=1e-5)
 
 
-def test_ties_duplicates_and_degenerate_rows():
+@pytest.mark.parametrize("limit", [0, 255])
+def test_ties_duplicates_and_degenerate_rows(limit):
     V = 4096
     z = np.zeros((4, V), dtype=np.float32)                                 # row 0: every logit equal
     z[1, :] = -np.inf; z[1, 17] = 0.5; z[1, 99] = 0.5                      # row 1: a masked row with two survivors
@@ -166,7 +175,7 @@ def test_ties_duplicates_and_degenerate_rows():
     z[3, :] = np.linspace(-5, 5, V, dtype=np.float32)
     cfg = dict(logits=oracle.f32_to_bf16(z), temperature=np.array([1.0, 0.5, 0.8, 1.2], np.float32), top_k=np.array([10, 0, 12, 3], np.int32),
                top_p=np.array([0.9, 0.95, 0.5, 0.0], np.float32), uniforms=np.array([0.999999, 0.5, 0.0, 0.3], np.float32))
-    r, tok, tau, stats = run_both(cfg, "inverse_cdf", 4)
+    r, tok, tau, stats = run_both(cfg, "inverse_cdf", 4, grid_limit=limit)
     np.testing.assert_array_equal(r.tau.cpu().numpy(), tau)
     np.testing.assert_array_equal(r.tokens.cpu().numpy(), tok)
     np.testing.assert_allclose(r.stats.cpu().numpy(), stats, rtol=1e-5)
@@ -213,8 +222,8 @@ def test_invalid_arguments_raise_before_launch():
 
 
 def test_streaming_and_generic_paths_agree():
-    """BF16 rows that only ask for tokens take the one-pass streaming kernel; asking for statistics routes the same rows
-    through the generic kernel. Same tokens, same thresholds; rows the streaming kernel cannot take fall back by themselves."""
+    """BF16 rows that only ask for tokens take the streaming kernels; asking for statistics with a grid limit routes the same rows
+    through the generic kernel. Same tokens, same thresholds; rows the streaming kernels cannot take fall back by themselves."""
     rows = 40
     cfg = inputs.config3(rows=rows, seed=31)
     cfg["logits"][5, :70000] = 0xFF80                                      # a masked row: 70000 x -inf (counted apart from the codes: stays)
@@ -225,11 +234,15 @@ def test_streaming_and_generic_paths_agree():
     x = bf16_tensor(cfg["logits"])
     knobs = {k: torch.from_numpy(cfg[k]).cuda() for k in ("temperature", "top_k", "top_p")}
     hist, u = torch.from_numpy(cfg["history"]).cuda(), torch.from_numpy(cfg["uniforms"]).cuda()
+    plain = lm.SamplingParams(seed=5, **knobs)
+    assert {"sample_topk_kernel", "sample_hist_kernel"} <= set(routes.names(lambda: lm.sample(x, plain)))
+    assert routes.names(lambda: lm.sample(x, lm.SamplingParams(seed=5, grid_limit=255, **knobs), return_stats=True)) == ["sample_generic_kernel"]
     for draw in ("inverse_cdf", "gumbel"):
         for extra in (dict(), dict(min_p=0.02), dict(topp_in_topk=True)):
             p = lm.SamplingParams(seed=5, draw=draw, repetition_penalty=1.1, presence_penalty=0.5, **knobs, **extra)
             fast = lm.sample(x, p, history=hist, uniforms=u, step=1, return_tau=True, return_status=True)
-            slow = lm.sample(x, p, history=hist, uniforms=u, step=1, return_tau=True, return_status=True, return_stats=True)
+            slow_p = lm.SamplingParams(seed=5, draw=draw, repetition_penalty=1.1, presence_penalty=0.5, grid_limit=255, **knobs, **extra)
+            slow = lm.sample(x, slow_p, history=hist, uniforms=u, step=1, return_tau=True, return_status=True, return_stats=True)
             fs, ss = fast.status.cpu().numpy(), slow.status.cpu().numpy()
             assert np.all(ss & 1) and not (fs[5] & 1) and (fs[6] & 1) and np.count_nonzero(fs & 1) <= 3, fs   # the degenerate row, at most a stray dense one
             assert torch.equal(fast.tau, slow.tau), (draw, extra)
@@ -287,17 +300,19 @@ def test_candidate_path_equals_the_oracle(draw):
         got = r.tokens.cpu().numpy()
         assert np.all((got == tok) | ((status & 4) != 0)), (extra, np.nonzero(got != tok))
         # and the same rows through the histogram path alone: identical
-        q = lm.SamplingParams(seed=5, draw=draw, repetition_penalty=1.1, presence_penalty=0.5, exact_only=True, **knobs, **extra)
+        q = lm.SamplingParams(seed=5, draw=draw, repetition_penalty=1.1, presence_penalty=0.5, exact_only=True, grid_limit=255, **knobs, **extra)
+        assert routes.names(lambda: lm.sample(x, q, history=hist, uniforms=u)) == ["sample_hist_kernel", "sample_generic_kernel"]
         h = lm.sample(x, q, history=hist, uniforms=u, step=2, return_tau=True, return_status=True)
         assert not np.any(h.status.cpu().numpy() & 64)
         assert torch.equal(h.tau, r.tau) and torch.equal(h.tokens, r.tokens)
 
 
-def test_streaming_draw_over_wide_kept_sets():
+@pytest.mark.parametrize("copies", [1, 4])
+def test_streaming_draw_over_wide_kept_sets(copies):
     """Rows without a top_k draw through the histogram kernel: kept sets that stay in the
     positive codes, reach into the negative ones (no filter at all, a loose min_p, a row shifted below zero) or
     lie many binades apart must all give the oracle's token. Row 5 holds magnitudes below the kernel's code window
-    (2^-39): it is handed to the generic kernel, with the same result."""
+    (2^-39): it is handed to the generic kernel, with the same result. (Twelve rows alone go to the cluster kernel, which leaves row 5 likewise.)"""
     rows, V = 12, 151936
     rng = np.random.default_rng(23)
     z = (rng.standard_normal((rows, V)) * 2).astype(np.float32)
@@ -309,15 +324,18 @@ def test_streaming_draw_over_wide_kept_sets():
                top_k=np.zeros(rows, np.int32), top_p=np.float32([0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.9, 0.999, 0.97, 0.5, 1.0]),
                history=rng.integers(0, V, (rows, 64)).astype(np.int32), uniforms=rng.random(rows).astype(np.float32),
                repetition_penalty=1.2, presence_penalty=0.3)
+    cfg = {k: np.concatenate([v] * copies) if isinstance(v, np.ndarray) else v for k, v in cfg.items()}
+    cfg["uniforms"] = rng.random(rows * copies).astype(np.float32)
     x = bf16_tensor(cfg["logits"])
     knobs = {k: torch.from_numpy(cfg[k]).cuda() for k in ("temperature", "top_k", "top_p")}
+    assert ("sample_hist_kernel" if copies > 1 else "sample_cluster_kernel") in routes.names(lambda: lm.sample(x, lm.SamplingParams(**knobs)))
     for extra in (dict(), dict(min_p=1e-6), dict(min_p=0.01)):
         r = lm.sample(x, lm.SamplingParams(draw="inverse_cdf", repetition_penalty=1.2, presence_penalty=0.3, **knobs, **extra),
                       history=torch.from_numpy(cfg["history"]).cuda(), uniforms=torch.from_numpy(cfg["uniforms"]).cuda(), return_tau=True, return_status=True)
         tok, tau, _ = oracle.sample_batch(cfg["logits"], temperature=cfg["temperature"], top_k=cfg["top_k"], top_p=cfg["top_p"], history=cfg["history"],
                                           repetition_penalty=1.2, presence_penalty=0.3, draw="inverse_cdf", uniforms=cfg["uniforms"], n_threads=8, **extra)
         generic = (r.status.cpu().numpy() & 1) != 0
-        assert generic.tolist() == [row == 5 for row in range(rows)], r.status   # all but row 5 through the histogram kernel
+        assert generic.tolist() == [row % rows == 5 for row in range(rows * copies)], r.status   # all but row 5
         np.testing.assert_array_equal(r.tau.cpu().numpy(), tau)
         np.testing.assert_array_equal(r.tokens.cpu().numpy(), tok)
 
@@ -392,11 +410,12 @@ def test_sampling_call_in_a_cuda_graph(rows):
 
 
 @pytest.mark.parametrize("draw", ["inverse_cdf", "gumbel"])
-def test_top_k_kernel_edge_rows(draw):
+@pytest.mark.parametrize("copies,limit", [(1, 0), (7, 0), (1, 3)])
+def test_top_k_kernel_edge_rows(draw, copies, limit):
     """Rows built to stress the one-pass top-k kernel at a vocabulary it accepts (32768): ties through the k-th rank, more
     ties than it can hold, every logit equal, a -inf mask over most of the row, a +inf logit, a tiny temperature, one
     repeated history id, penalised values crowding the top. Whatever kernel ends up finishing a row, tokens and thresholds
-    are the oracle's."""
+    are the oracle's. (Twelve rows alone go to the cluster kernel; 84, or a grid limit, to the top-k kernel.)"""
     V, rows = 32768, 12
     rng = np.random.default_rng(123)
     z = (rng.standard_normal((rows, V)) * 2).astype(np.float32)
@@ -415,30 +434,38 @@ def test_top_k_kernel_edge_rows(draw):
     cfg = dict(logits=codes, temperature=np.float32([0.7, 1.0, 0.9, 1.1, 1.0, 0.02, 0.8, 1.0, 0.9, 1.3, 1.0, 0.6]),
                top_k=np.int32([20, 1000, 5, 50, 20, 50, 20, 7, 50, 1024, 20, 1]), top_p=np.float32([0.9, 0.95, 0.5, 0.9, 0.9, 0.99, 0.8, 0.0, 0.97, 0.9, 0.9, 0.3]),
                history=hist, uniforms=rng.random(rows).astype(np.float32))
+    cfg = {k: np.concatenate([v] * copies) for k, v in cfg.items()}
+    codes, hist, rows = cfg["logits"], cfg["history"], rows * copies
     x = bf16_tensor(codes)
+    assert ("sample_cluster_kernel" if copies == 1 and not limit else "sample_topk_kernel") in routes.names(
+        lambda: lm.sample(x, lm.SamplingParams(temperature=0.8, top_k=torch.full((rows,), 20, dtype=torch.int32, device="cuda"), grid_limit=limit)))
     knobs = {k: torch.from_numpy(cfg[k]).cuda() for k in ("temperature", "top_k", "top_p")}
     for extra in (dict(), dict(min_p=0.01), dict(topp_in_topk=True)):
-        r = lm.sample(x, lm.SamplingParams(seed=9, draw=draw, repetition_penalty=1.3, presence_penalty=0.4, **knobs, **extra),
+        r = lm.sample(x, lm.SamplingParams(seed=9, draw=draw, repetition_penalty=1.3, presence_penalty=0.4, grid_limit=limit, **knobs, **extra),
                       history=torch.from_numpy(hist).cuda(), uniforms=torch.from_numpy(cfg["uniforms"]).cuda(), step=4, return_tau=True, return_status=True)
         tok, tau, _ = oracle.sample_batch(codes, temperature=cfg["temperature"], top_k=cfg["top_k"], top_p=cfg["top_p"], history=hist,
                                           repetition_penalty=1.3, presence_penalty=0.4, draw=draw, uniforms=cfg["uniforms"], seed=9, step=4, n_threads=8, **extra)
         status = r.status.cpu().numpy()
-        keep = np.arange(rows) != 4                                         # the +inf row: weights are NaN by definition, only the threshold is compared
+        keep = np.arange(rows) % 12 != 4                                    # the +inf row: weights are NaN by definition, only the threshold is compared
         np.testing.assert_array_equal(r.tau.cpu().numpy(), tau)
         got = r.tokens.cpu().numpy()
         assert np.all((got == tok)[keep] | ((status & 4) != 0)[keep]), (extra, got, tok, status)
-        assert np.count_nonzero(status & 64) >= 5                           # the ordinary rows did go through the top-k kernel
+        assert np.count_nonzero(status & 64) >= 5 * copies                  # the ordinary rows were finished from their candidates
 
 
-def test_penalised_rows_equal_the_reference(golden):
+@pytest.mark.parametrize("limit", [0, 255])
+def test_penalised_rows_equal_the_reference(golden, limit):
     """16 penalised rows of the batched configuration: the thresholds and Gumbel tokens the reference's own sampling_ref gives on
-    the penalised rows (tests/golden), through the candidate kernel and through the histogram kernel alone."""
+    the penalised rows (tests/golden), through the cluster kernel and (with a grid limit) through the candidate kernel, and through
+    either's exact form alone."""
     g = golden["penalised"]
     cfg = inputs.config3(rows=g["rows"], seed=3)
     x = bf16_tensor(cfg["logits"])
     knobs = {k: torch.from_numpy(cfg[k]).cuda() for k in ("temperature", "top_k", "top_p")}
     for exact_only in (False, True):
-        p = lm.SamplingParams(seed=12345, draw="gumbel", repetition_penalty=1.1, presence_penalty=0.5, exact_only=exact_only, **knobs)
+        p = lm.SamplingParams(seed=12345, draw="gumbel", repetition_penalty=1.1, presence_penalty=0.5, exact_only=exact_only, grid_limit=limit, **knobs)
+        launched = routes.names(lambda: lm.sample(x, p, step=1))
+        assert ("sample_topk_kernel" in launched) == bool(limit and not exact_only) and ("sample_cluster_kernel" in launched) == (not limit)
         r = lm.sample(x, p, history=torch.from_numpy(cfg["history"]).cuda(), step=1, return_tau=True, return_status=True)
         status = r.status.cpu().numpy()
         assert not np.any(status & 1)
@@ -450,13 +477,15 @@ def test_penalised_rows_equal_the_reference(golden):
 def test_two_streams_sample_at_once_with_their_own_workspaces():
     """Calls that can overlap on the GPU must not share scratch: the host layer keeps one workspace per stream. Two streams run
     different batches again and again, side by side; each gets what it gets alone."""
-    cfgs = [inputs.config3(rows=48, vocab=32768, hist_len=256, seed=s) for s in (71, 72)]
+    cfgs = [inputs.config3(rows=80, vocab=32768, hist_len=256, seed=s) for s in (71, 72)]
     streams = [torch.cuda.Stream(), torch.cuda.Stream()]
     work = []
     for cfg in cfgs:
         knobs = {k: torch.from_numpy(cfg[k]).cuda() for k in ("temperature", "top_k", "top_p")}
         work.append((bf16_tensor(cfg["logits"]), lm.SamplingParams(draw="inverse_cdf", repetition_penalty=1.1, presence_penalty=0.5, **knobs),
                      torch.from_numpy(cfg["history"]).cuda(), torch.from_numpy(cfg["uniforms"]).cuda()))
+    x, p, h, u = work[0]
+    assert "sample_topk_kernel" in routes.names(lambda: lm.sample(x, p, history=h, uniforms=u))    # (calls that pass rows on in a workspace)
     alone = [lm.sample(x, p, history=h, uniforms=u).tokens.clone() for x, p, h, u in work]
     torch.cuda.synchronize()
     got = [[], []]
@@ -482,7 +511,8 @@ def test_row_maxima_come_out_of_every_kernel_and_feed_the_verify_step():
     t = torch.from_numpy(np.where(np.arange(rows) % 5 == 0, 0.0, 0.9).astype(np.float32))   # greedy rows among them
     k = torch.from_numpy(np.where(np.arange(rows) % 2 == 0, 0, 30).astype(np.int32))        # histogram-kernel and candidate-kernel rows
     p = lm.SamplingParams(temperature=t, top_k=k, top_p=0.9, repetition_penalty=1.2, presence_penalty=0.3, seed=3)
-    for extra in ({}, {"return_stats": True}):                                             # the streaming kernels; the generic kernel
+    for limit, extra in ((0, {}), (0, {"return_stats": True}), (255, {"return_stats": True})):   # the streaming kernels; the cluster kernel; the generic kernel
+        p.grid_limit = limit
         r = lm.sample(x, p, history=torch.from_numpy(hist).cuda(), return_vmax=True, **extra)
         np.testing.assert_array_equal(r.vmax.cpu().numpy(), want.astype(np.float32))
     few = lm.sample(x[:3], lm.SamplingParams(temperature=0.9, top_k=30, top_p=0.9, seed=3), return_vmax=True, return_status=True)   # the sliced path
@@ -506,9 +536,15 @@ def test_row_maxima_come_out_of_every_kernel_and_feed_the_verify_step():
             assert [v.cpu().tolist() for v in a] == [v.cpu().tolist() for v in b], (draw, u[0])
     # the masses themselves, from every kernel and both of the sampler's draws: the integer sum the oracle forms
     z = oracle.bf16_to_f32(target)
+    k50, k0, u = torch.full((8,), 50, dtype=torch.int32, device="cuda"), torch.zeros(8, dtype=torch.int32, device="cuda"), torch.full((8,), 0.3, device="cuda")
     for draw in ("inverse_cdf", "gumbel"):
-        for knobs in (dict(top_k=torch.full((8,), 50, dtype=torch.int32)), dict(top_k=torch.zeros(8, dtype=torch.int32)), dict(top_k=50)):
-            r = lm.sample(xt, lm.SamplingParams(temperature=0.8, top_p=0.95, seed=1, draw=draw, **knobs), uniforms=torch.full((8,), 0.3), return_tau=True, return_vmax=True)
+        for kernel, logits, knobs in (("sample_cluster_kernel", xt, dict(top_k=k50)), ("sample_cluster_kernel", xt, dict(top_k=k0)), ("sample_cluster_kernel", xt.float(), dict(top_k=700)),
+                                      ("slice_local_kernel", xt, dict(top_k=50)), ("sample_topk_kernel", xt, dict(top_k=k50, grid_limit=255)),
+                                      ("sample_topk_kernel", xt, dict(top_k=700, grid_limit=255)), ("sample_hist_kernel", xt, dict(top_k=0, grid_limit=255)),
+                                      ("sample_generic_kernel", xt.float(), dict(top_k=0, grid_limit=255))):
+            p = lm.SamplingParams(temperature=0.8, top_p=0.95, seed=1, draw=draw, **knobs)
+            assert kernel in routes.names(lambda: lm.sample(logits, p, uniforms=u)), kernel
+            r = lm.sample(logits, p, uniforms=u, return_tau=True, return_vmax=True)
             for i in range(8):
                 total = C.c_uint64()
                 oracle.lib().lmo_sample_invcdf(z[i].ctypes.data_as(C.POINTER(C.c_float)), z.shape[1], float(r.tau[i]), np.float32(0.8), np.float32(0.3), C.byref(total))

@@ -155,7 +155,7 @@ def test_rows_that_do_not_start_on_a_16_byte_boundary():
 
 def test_random_configurations_equal_the_exact_kernels():
     """A sweep of seeded random calls (rows, vocabulary, dtype, knobs, draw, penalties, -inf masks, planted ties): the few-row path
-    against the same library with LM_FLAG_EXACT_ONLY (the generic kernel, which the other tests hold to the oracle), bit for bit;
+    against the same library with LM_FLAG_EXACT_ONLY (the cluster kernel's searches, which its own tests hold to the oracle), bit for bit;
     a sample of the calls against the oracle itself."""
     rng = np.random.default_rng(2024)
     checked_with_oracle = 0

@@ -1,8 +1,8 @@
 """The allocation-free greedy entry point (lm_argmax_static) against the ordinary one (lm_argmax).
 
 Some callers of the library are given tensors and a stream but may not allocate device memory (a plug-in inside a
-frozen decode loop, a step running while the engine's allocator is locked): lm_argmax_static keeps the scratch
-that lm_argmax takes from the caller in a fixed array inside the library instead. This file is collected last on
+frozen decode loop, a step running while the engine's allocator is locked): lm_argmax_static takes no workspace. (Neither kernel needs
+any: the blocks of a row meet in one another's shared memory.) This file is collected last on
 purpose (its name sorts after every other test file): a run that stops at the first failure has then already
 run the rest of the suite.
 """
@@ -38,7 +38,7 @@ def test_static_scratch_argmax_equals_the_workspace_one(rows, vocab, dtype):
     expect = lm.argmax(x)                                                    # the existing entry point, caller-owned workspace
     assert expect.cpu().tolist() == host.argmax(-1).tolist()
     stream = torch.cuda.current_stream().cuda_stream
-    for call in range(2):                                                    # two calls in a row share the library's scratch
+    for call in range(2):
         out = torch.full((rows,), -7, dtype=torch.int32, device="cuda")
         rc = L.lm_argmax_static(x.data_ptr(), _lib.DTYPE_BF16 if dtype == "bf16" else _lib.DTYPE_F32, rows, vocab, x.stride(0) if rows > 1 else vocab,
                                 out.data_ptr(), stream)
@@ -58,12 +58,11 @@ def test_static_scratch_rejects_what_does_not_fit():
 
 
 def test_static_scratch_allocates_nothing_and_survives_a_larger_call_before_a_smaller_one():
-    """A call that splits many rows over several blocks dirties most of the library's scratch; the smaller call behind it must
-    still be right (the entry point clears what it uses), and neither call may take device memory: the free memory the driver
-    reports and the bytes torch has handed out are the same before and after."""
+    """Calls of many rows, of rows split over several blocks and of a few rows behind one another; none may take device memory: the free
+    memory the driver reports and the bytes torch has handed out are the same before and after."""
     L = _lib.lib()
     stream = torch.cuda.current_stream().cuda_stream
-    big, big_host = _logits(_lib.ARGMAX_STATIC_MAX_ROWS, 32768, 11, "bf16")   # the largest row count the scratch holds
+    big, big_host = _logits(_lib.ARGMAX_STATIC_MAX_ROWS, 32768, 11, "bf16")   # the largest row count it takes
     wide, wide_host = _logits(64, 151936, 12, "bf16")                        # 64 rows x 151936: split over several blocks per row
     small, small_host = _logits(3, 151936, 13, "f32")
     outs = [torch.full((t.shape[0],), -7, dtype=torch.int32, device="cuda") for t in (big, wide, small)]
