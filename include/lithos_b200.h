@@ -53,7 +53,7 @@ extern "C" {
 
 /* lm_sample_args.flags */
 #define LM_FLAG_TOPP_IN_TOPK 1u /* top-p over the top-k set's renormalised mass (the Hugging Face warpers' order) */
-#define LM_FLAG_EXACT_ONLY 2u /* skip the one-pass candidate kernel for rows with a top_k: every row takes the histogram path (same results) */
+#define LM_FLAG_EXACT_ONLY 2u /* no candidate lists for rows with a top_k: every row is counted out, by the histogram kernel or (few rows) the cluster kernel's searches (same results) */
 #define LM_FLAG_TOKENS_I64 4u /* lm_sample: out_tokens points to int64_t entries (what the reference's sampler modules return) */
 #define LM_FLAG_GRID_LIMIT(n) (((uint32_t)(n) & 0xFFu) << 8) /* lm_sample: at most n thread blocks at any time (0 = one per SM): leaves SMs to other streams; a call cut into slices is not limited */
 

@@ -277,7 +277,7 @@ int lm_sample(const lm_sample_args* a) {
       // Many rows per SM, or hardly a row for the histogram kernel (one top_k for all: 148 rows 56 us side by side, 43 so): the top-k kernel first,
       // the histogram kernel behind it with programmatic stream serialization: its blocks take an SM over as the top-k blocks leave it, work
       // through the rows that a one-thread-per-row kernel has listed for it, wait for the top-k grid, and absorb the few rows that one handed
-      // on. (Behind its end: 4096 penalised rows 771 us, now 720; 800 rows 210, now 186.)
+      // on. (4096 penalised rows 720 us, behind its end 771; 800 rows 186 and 210.)
       sample_classify_kernel<<<grid_list, 256, 0, st>>>(P, list_other, counters + 4);
       sample_topk_kernel<<<grid1, kTB, sizeof(TopkSmem), st>>>(P, list_left, counters);
       cudaError_t e = cudaGetLastError();
@@ -300,7 +300,7 @@ int lm_sample(const lm_sample_args* a) {
       sample_classify_kernel<<<grid_list, 256, 0, st>>>(P, list_other, counters + 4);
       // With at most kAloneRowsPerSM rows per SM the histogram kernel's blocks ask for so much shared memory that nothing else fits
       // beside them: a long row then has its SM to itself, and the blocks that find no row leave their SM to the top-k kernel at
-      // once (256 rows of the benchmark mix: 112 -> 106 us per call; from 3 rows per SM on it costs time).
+      // once (256 rows of the benchmark mix: 106 us per call, 112 without; from 3 rows per SM on it costs time).
       size_t hist_smem_first = hist_smem; int grid_first = grid;
       if (a->rows <= static_cast<int64_t>(kAloneRowsPerSM) * sms && hist_smem < kAloneSmemBytes) {
         hist_smem_first = kAloneSmemBytes; grid_first = static_cast<int>(a->rows < sms ? a->rows : sms);
@@ -662,7 +662,7 @@ int lm_verify(const lm_verify_args* a) {
   const int per = (static_cast<int>((a->vocab + grid - 1) / grid) + 7) & ~7;
   const size_t rows_cached = static_cast<size_t>(a->n_draft + 1) + (a->mode == LM_VERIFY_STOCHASTIC ? a->n_draft : 0);
   size_t smem = rows_cached * static_cast<size_t>(per) * sizeof(float);
-  // a launch that was given the rows' maxima and masses knows the decisive row from one logit per draft: it reads that row alone, once
+  // a launch that was given the rows' maxima and masses knows the decisive row from one logit per draft and reads no other: nothing to keep in shared memory
   int cached = (smem <= 200 * 1024 && !(a->mode == LM_VERIFY_STOCHASTIC && a->target_vmax && a->target_mass)) ? 1 : 0;
   if (!cached) smem = 0;
   const bool stats = P.row_max != nullptr && P.row_mass != nullptr;

@@ -1,11 +1,11 @@
 // The cluster row sampler: one row per thread-block CLUSTER, any element type, alignment, vocabulary and knobs, every output.
 //
 // A row is cut into as many contiguous slices as its cluster has blocks (16 for a handful of rows, 1 for a batch that fills the
-// GPU by itself), so one row is spread over 16 SMs and a batch of 64 over 128; the blocks exchange through distributed shared
+// GPU by itself), so one row is spread over 16 SMs and a batch of 64 over 256 blocks, two to an SM; the blocks exchange through distributed shared
 // memory and the hardware cluster barrier (well under a microsecond), in ONE launch. Per row:
 //
 //   load       every block reads its slice once (kept in shared memory as binary32 when it fits, else read again from L2): maximum,
-//              its lowest index, smallest finite logit; odd values (NaN, infinities above, see kWin*) send the row to the generic code
+//              its lowest index, smallest finite logit, maxima of groups; odd values (NaN, +inf, BF16 below 2^-39) send the row to the generic code
 //   histogram  1024 bins, linear in the logit below the row's maximum: counts (a top_k wants them), fixed-point sums of
 //              exp((z - vmax) / T) in FP64 (a top-p over binary32 values wants them), or of the draw's integer weights. The bins of
 //              the blocks are added up, a share by every block, and pushed to all of them

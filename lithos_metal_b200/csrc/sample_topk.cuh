@@ -280,9 +280,8 @@ static __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem&
   float2 sacc = make_float2(0.0f, 0.0f);
   uint32_t nan_seen = 0u;
   // A bit per step: this thread's chunk held a logit >= cutoff. The list of those chunks is written behind the pass, one reservation per
-  // warp: nearly every step some lane has one, and a reservation per step was a quarter of the pass's instructions (4096 penalised rows, three in four with a
-  // top_k:
-  // 857 -> 797 us; 64 rows of 262,144, top_k 50: 51 -> 45).
+  // warp: nearly every step some lane has one, and a reservation per step would be a quarter of the pass's instructions (4096 penalised rows, three
+  // in four with a top_k: 857 us with it, 797 without; 64 rows of 262,144, top_k 50: 51 and 45).
   static_assert(kTopkMaxVocab / kChunk <= 64 * kTB, "a bit for every step");
   unsigned long long hits = 0ull;
   {

@@ -33,8 +33,8 @@ class SamplingParams:
     repetition_penalty: float = 1.0
     presence_penalty: float = 0.0
     draw: str = "gumbel"               # "gumbel" (the reference's counter-based Gumbel-max) or "inverse_cdf" (injected uniforms)
-    exact_only: bool = False           # skip the candidate kernel for rows with a top_k (same results; for cross-checks)
-    grid_limit: int = 0                # at most this many thread blocks (0 = one per SM); leaves SMs free for other streams
+    exact_only: bool = False           # no candidate lists for rows with a top_k (same results; for cross-checks)
+    grid_limit: int = 0                # at most this many thread blocks at any time (0 = one per SM); leaves SMs free for other streams
 
 
 @dataclass
