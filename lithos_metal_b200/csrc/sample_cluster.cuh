@@ -1207,6 +1207,7 @@ static __device__ __noinline__ bool phase_search(ClusterSmem& s, bool dirty) {
       if (list_len <= kCList) { list_tag = level || base != -1 ? -1 : static_cast<int>(b); break; }
       if (level == 1) return false;                                         // more equal logits than a list holds
       fresh = false; refill = true;
+      __syncthreads();                                                      // (where no list was begun, a warp may still be looking tau's bin up with the window as it was)
       if (tid == 0) s.window = base == -1 ? static_cast<int>(b) : kCBins + static_cast<int>(b);
       __syncthreads();
     }

@@ -233,3 +233,16 @@ def test_a_count_is_found_wherever_it_crosses(dtype, mask):
                 assert not np.any(status & 1) or (not mask and k == 9000), (k, t, p, draw, status)
     knobs = dict(temperature=np.full(6, 0.8, np.float32), top_k=np.full(6, 60000, np.int32), top_p=np.full(6, 0.9, np.float32), min_p=0.0)
     _check(_tensor(host), host, knobs, draw="inverse_cdf", exact_only=True)  # the k-th is one of the masked
+
+
+def test_every_warp_looks_the_thresholds_bin_up_in_the_same_window():
+    """A bin that holds more than a list, met by the threshold's own step (no barrier of a list in between): hundreds of rows whose logits lie
+    within a few units in the last place of one another, a third of them far below, thresholds from a top_k and a top_p close to 1."""
+    rng = np.random.default_rng(47)
+    z = (rng.standard_normal((148, 4096)) * 1e-4 + 100.0).astype(np.float32)
+    z[:, ::3] -= 40.0
+    for top_p in (0.9999999, 0.95, 0.5):
+        for draw in ("gumbel", "inverse_cdf"):
+            knobs = dict(temperature=np.full(148, 50.0, np.float32), top_k=np.full(148, 1000, np.int32), top_p=np.full(148, top_p, np.float32), min_p=0.0)
+            for _ in range(5):
+                _check(_tensor(z), z, knobs, draw=draw)
