@@ -46,6 +46,8 @@ __device__ __forceinline__ uint32_t kept_chunk(const RowView& rv, int c, float t
       if ((m0 | m1 | m2 | m3) == 0u) return 0u;
       z[0] = bf16_lo(q.x); z[1] = bf16_hi(q.x); z[2] = bf16_lo(q.y); z[3] = bf16_hi(q.y);
       z[4] = bf16_lo(q.z); z[5] = bf16_hi(q.z); z[6] = bf16_lo(q.w); z[7] = bf16_hi(q.w);
+#pragma unroll
+      for (int e = 0; e < kChunk; e++) z[e] = canon_zero(z[e]);             // (a zero of either sign is one value: the keys below tell them apart)
       return (m0 & 1u) | ((m0 >> 15) & 2u) | ((m1 & 1u) << 2) | ((m1 >> 13) & 8u) | ((m2 & 1u) << 4) | ((m2 >> 11) & 32u) |
              ((m3 & 1u) << 6) | ((m3 >> 9) & 128u);
     }

@@ -574,3 +574,22 @@ def test_a_call_with_a_grid_limit_keeps_to_it(rows):
     assert torch.equal(a, lm.sample(x, lm.SamplingParams(draw="inverse_cdf", **knobs), uniforms=u).tokens)
     if rows > 74:
         assert any(beside for _, _, beside in call(x, 0))
+
+
+@pytest.mark.parametrize("limit", [0, 255])
+def test_zeros_of_either_sign_are_one_value_to_the_generic_draw(limit):
+    """-0 and +0 compare equal, so the draw orders them by index alone, whichever way a chunk is read (aligned rows, penalised logits)."""
+    rows, V = 8, 4100
+    rng = np.random.default_rng(77)
+    z = np.where(rng.random((rows, V)) < 0.5, 0.0, -0.0).astype(np.float32)
+    z[:, 5] = 1.0
+    hist = np.tile(np.arange(6, 1200, 7, dtype=np.int32), (rows, 1))
+    codes = oracle.f32_to_bf16(z)
+    u = np.linspace(0.05, 0.999, rows).astype(np.float32)
+    for h in (None, hist):
+        pen = {} if h is None else dict(repetition_penalty=1.3, presence_penalty=0.0)
+        r = lm.sample(bf16_tensor(codes), lm.SamplingParams(temperature=0.8, draw="inverse_cdf", grid_limit=limit, top_p=0.99, **pen),
+                      history=None if h is None else torch.from_numpy(h).cuda(), uniforms=torch.from_numpy(u).cuda(), return_status=True)
+        tok, _, _ = oracle.sample_batch(codes, temperature=0.8, top_k=0, top_p=0.99, draw="inverse_cdf", uniforms=u, n_threads=8, history=h, **pen)
+        assert np.all(r.status.cpu().numpy() & 1)                           # more equal logits than a list holds
+        np.testing.assert_array_equal(r.tokens.cpu().numpy(), tok)
