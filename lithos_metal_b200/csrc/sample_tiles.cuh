@@ -291,7 +291,8 @@ static __global__ void __launch_bounds__(kTB, kTopkPerSM) tile_finish_kernel(Sam
       __syncthreads();
       RowMass zm;
       zm.need = true; zm.z_tilde = st->s; zm.z_raw = st->s - st->s_pen; zm.z_corr = st->s_pen;
-      zm.shift = st->m * (1.4426950408889634 / static_cast<double>(T));
+      zm.slope = 1.4426950408889634 / static_cast<double>(T);               // (the tiles' masses are joined in FP64, relative to st->m)
+      zm.shift = st->m * zm.slope;
       zm.ref = static_cast<float>(st->m); zm.acc_terms = static_cast<double>(kTileMaxCols / kTileBlock) + 1.0; zm.row = nullptr; zm.n_chunks = 0; zm.penalised = false;
       ok = topk_finish(P, row, c, cut_code, zm);
       __syncthreads();

@@ -68,7 +68,7 @@ static_assert(kTopkPerSM * (sizeof(TopkSmem) + 1024) <= 233472, "the blocks of t
 // that was accumulated in FP32 (sequences of acc_terms additions), z_corr what was added and removed term by term (penalties);
 // ref is the logit the exponents were taken relative to (a logit of the row at or near its maximum).
 // row: its BF16 codes, n_chunks of eight, where the mass can be formed again in FP64 (c.pen marks the penalised positions); nullptr: the logits are gone.
-struct RowMass { bool need; double z_tilde, z_raw, z_corr, shift, acc_terms; float ref; const uint16_t* row; int n_chunks; bool penalised; };
+struct RowMass { bool need; double z_tilde, z_raw, z_corr, shift, slope, acc_terms; float ref; const uint16_t* row; int n_chunks; bool penalised; };
 
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst))), "l"(gmem_src) : "memory");
@@ -408,7 +408,7 @@ static __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem&
   if (need_z && !(z_tilde > 0.0)) return false;                             // nothing left after the corrections (cancellation): the exact path
   __syncthreads();
   RowMass zm;
-  zm.need = need_z; zm.z_tilde = z_tilde; zm.z_raw = z_raw; zm.z_corr = z_sub + z_add; zm.shift = -static_cast<double>(nb);
+  zm.need = need_z; zm.z_tilde = z_tilde; zm.z_raw = z_raw; zm.z_corr = z_sub + z_add; zm.shift = -static_cast<double>(nb); zm.slope = static_cast<double>(c2a);
   zm.ref = M; zm.acc_terms = 4.0 * n_it + 1.0; zm.row = rowp; zm.n_chunks = n_chunks; zm.penalised = pen_on;
   return topk_finish(P, row, c, cut_code, zm);
 }
@@ -521,13 +521,15 @@ static __device__ bool topk_finish(const SampleDev& P, int row, TopkSmem& c, uin
       // The FP32 mass of the whole row, moved to the exact maximum. z_tilde approximates sum_i 2^(z_i c2a + nb); nb's own rounding
       // is a common factor and is taken out exactly here (zm.shift is the true -nb, not M c2a).
       const double c64 = 1.4426950408889634 * inv_t;
-      total = zm.z_tilde * exp2(zm.shift - static_cast<double>(vmax) * c64);
+      // With the slope that the terms were formed with: log2(e) / T in FP64 instead would leave the factor 2^(vmax (c2a - c)), which no
+      // bound below holds (a maximum of 105 at T 0.3: 2e-5).
+      total = zm.z_tilde * exp2(zm.shift - static_cast<double>(vmax) * zm.slope);
       // What separates it from sum_i 2^((z_i - vmax) c), relative, first order, worst case (u = 2^-24, the FP32 unit roundoff):
       //   - c2a = fl32(c): every term is off by a factor 2^(x_i delta), |delta| <= u, x_i = (z_i - M) c; weighted by the terms that is
       //     ln2 u E_w|x| <= u (ln V + 2 ln2 D): E_w[-x ln2] = H - ln Z <= ln V (H the entropy of the softmax, Z >= 1 relative to the
       //     row maximum, V <= 2^18: ln V <= 12.5), and the terms above the sampled maximum have 0 < x <= D = (vmax - M) c;
-      //   - the FMA rounds its result: half an ulp of |x| < 32 is at most 2^-20, a factor 2^(2^-20) = 1 + 6.6e-7 on the term; the terms
-      //     with |x| >= 32 weigh less than V 2^-32 altogether;
+      //   - the FMA rounds its result: half an ulp of |x| < 32 is at most 2^-20, a factor 2^(2^-20) = 1 + 6.6e-7 on the term, and D / 16 times
+      //     that for the terms up to D above the sampled maximum; the terms below -32 weigh less than V 2^-32 altogether;
       //   - ex2.approx.ftz.f32: 2 ulp = 4 u;
       //   - each lane accumulates 4 n_it terms one after the other in FP32, then two accumulators and the lanes meet in FP64:
       //     (4 n_it + 1) u (zm.acc_terms);
@@ -537,7 +539,7 @@ static __device__ bool topk_finish(const SampleDev& P, int row, TopkSmem& c, uin
       // The band is this bound with a quarter added. A boundary of the cumulative mass inside it is decided by the FP64 mass.
       const double u = 5.9604644775390625e-8;
       const double D = fmax(0.0, (static_cast<double>(vmax) - static_cast<double>(zm.ref)) * c64);
-      const double rel = u * (12.5 + 1.3862943611198906 * D) + 6.6e-7 + 4.0 * u + zm.acc_terms * u;
+      const double rel = u * (12.5 + 1.3862943611198906 * D) + 6.6e-7 * fmax(1.0, D * 0.0625) + 4.0 * u + zm.acc_terms * u;
       err = 1.25 * (rel * zm.z_raw + 1.6e-6 * zm.z_corr) * (total / zm.z_tilde);
     }
     double target;

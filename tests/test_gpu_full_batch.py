@@ -164,3 +164,25 @@ def test_large_top_ks_at_the_largest_vocabularies_stay_on_the_candidate_path(top
     x = torch.cat([(torch.randn(64, 262144, generator=g, device="cuda") * 2).to(torch.bfloat16) for _ in range(4)])
     r = lm.sample(x, lm.SamplingParams(temperature=0.8, top_k=top_k, top_p=0.9, seed=2), return_status=True)
     assert int((r.status & 64 == 0).sum()) <= 12                             # binomial(256, 0.015): beyond 12 in 1e-4 of all seeds
+
+
+def test_the_fp32_mass_of_rows_far_from_zero():
+    """Logits around 100: the candidate kernel's mass must not carry the rounding of the slope log2(e) / T times the maximum (2e-5 at T 0.3), which
+    its band does not hold. top_p a few 1e-6 on either side of a boundary of the cumulative mass inside the top-k set."""
+    rng = np.random.default_rng(67)
+    rows = []
+    for r in range(16):
+        T = np.float32(rng.uniform(0.25, 0.5))
+        codes = oracle.f32_to_bf16((100.0 + 2.0 * rng.standard_normal(40000)).astype(np.float32))
+        vals, counts = np.unique(oracle.bf16_to_f32(codes).astype(np.float64), return_counts=True)
+        vals, counts = vals[::-1], counts[::-1]
+        cum = np.cumsum(counts * np.exp((vals - vals[0]) / np.float64(T)))
+        i = int(np.searchsorted(np.cumsum(counts), 100))
+        for d in (0.0, 3e-6, -3e-6, 6e-6, -6e-6, 1.2e-5, -1.2e-5, 1e-4):
+            rows.append((codes, T, np.float32(cum[i] / cum[-1] * (1.0 + d))))
+    n = len(rows)
+    cfg = dict(logits=np.stack([c for c, _, _ in rows]), temperature=np.array([t for _, t, _ in rows], np.float32), top_k=np.full(n, 500, np.int32),
+               top_p=np.array([p for _, _, p in rows], np.float32), uniforms=np.linspace(0.02, 0.98, n).astype(np.float32))
+    r, tok, tau = gpu_and_oracle(cfg)
+    np.testing.assert_array_equal(r.tau.cpu().numpy(), tau)
+    np.testing.assert_array_equal(r.tokens.cpu().numpy(), tok)
