@@ -25,13 +25,16 @@ constexpr uint32_t kFull = 0xFFFFFFFFu;
 __device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
 
+// A bit per logit of a chunk from the masks of packed compares.
+__device__ __forceinline__ uint32_t mask8(uint32_t m0, uint32_t m1, uint32_t m2, uint32_t m3) {
+  return (m0 & 1u) | ((m0 >> 15) & 2u) | ((m1 & 1u) << 2) | ((m1 >> 13) & 8u) | ((m2 & 1u) << 4) | ((m2 >> 11) & 32u) | ((m3 & 1u) << 6) | ((m3 >> 9) & 128u);
+}
 // 8-bit mask of the logits of a chunk of BF16 codes that are at or above the code in both halves of tau_code2.
 __device__ __forceinline__ uint32_t kept_mask8(const uint4 q, uint32_t tau_code2) {
   const __nv_bfloat162 t2 = *reinterpret_cast<const __nv_bfloat162*>(&tau_code2);
   const uint32_t m0 = __hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&q.x), t2), m1 = __hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&q.y), t2);
   const uint32_t m2 = __hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&q.z), t2), m3 = __hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&q.w), t2);
-  if ((m0 | m1 | m2 | m3) == 0u) return 0u;
-  return (m0 & 1u) | ((m0 >> 15) & 2u) | ((m1 & 1u) << 2) | ((m1 >> 13) & 8u) | ((m2 & 1u) << 4) | ((m2 >> 11) & 32u) | ((m3 & 1u) << 6) | ((m3 >> 9) & 128u);
+  return (m0 | m1 | m2 | m3) == 0u ? 0u : mask8(m0, m1, m2, m3);
 }
 
 // Monotone 32-bit key of a float: a > b  <=>  fkey(a) > fkey(b) (for non-NaN, with -0 canonicalised to +0 first).

@@ -16,7 +16,7 @@
 // The walks are two-level: 258 groups of 64 window positions (block scan), then one warp inside the group where the target
 // falls. The inverse-CDF draw (descending value order, equal values by ascending index) is decided by the same walks on integer
 // weights, down to the value; its second look at the row (from L2) only counts the logits equal to that value, in 256-logit
-// segments from the nearer end of the row, and stops at the segment that holds the one it wants.
+// segments from the nearer end of the row, and stops after the batch of segments that holds the one it wants.
 //
 // Rows this kernel cannot take go to the generic kernel through the `redo` list: a logit outside the window other than 0
 // and -inf (NaN, +inf, |z| >= 2^25, 0 < |z| < 2^-39), more than 65535 equal logits, more than kPenCap distinct penalised ids
@@ -45,8 +45,12 @@ constexpr uint32_t kPosNinf = 2u * kWinCodes + 1u;//   8193..16384 negative, 163
 constexpr int kPenCap = 2048;                     // distinct penalised ids per row
 constexpr int kSegChunks = 32;                    // the draw's segments: 32 chunks = 256 logits, one warp-wide load
 constexpr int kMaxSegs = kHistMaxVocab / (kSegChunks * kChunk);
-constexpr int kDrawIters = 4;                     // segments per warp and batch of the draw
+constexpr int kDrawIters = 10;                    // segments per warp and batch of the draw ...
+constexpr int kDrawDeep = 5;                      // ... and how many of them are in flight
 constexpr int kBatchSegs = kDrawIters * kHW;
+constexpr int kMaxBatches = (kMaxSegs + kBatchSegs - 1) / kBatchSegs;
+static_assert(kBatchSegs % 32 == 0 && kDrawIters % kDrawDeep == 0, "whole warps walk a batch's counts");
+static_assert(kHB == 2 * static_cast<int>(kSlots) / kGrpSlots, "two threads count a group");
 
 struct HistSmem {
   uint32_t hist[kSlots / 2];                      // 32 KB: 16-bit counters of the unpenalised logits, slot s in half (s & 1) of word s >> 1
@@ -59,14 +63,16 @@ struct HistSmem {
   float b_val[kPenCap];                           // distinct penalised values, descending
   uint16_t b_ins[kPenCap];                        // the window position each is inserted before: the smallest p with value(p) <= b_val
   uint16_t b_cnt[kPenCap];                        // how many logits carry each value; from phase 4 on the running sum (inclusive)
-  unsigned long long seg_fix[kMaxSegs];           // draw: per segment (as 32-bit counters), its penalised logits equal to the drawn value
-  unsigned long long batch_sum[2][kBatchSegs];    // draw: (as 32-bit counters) segment counts of the batch in hand, double-buffered
+  uint32_t seg_pen[kMaxSegs];                     // draw: per segment, its penalised logits equal to the drawn value
+  uint32_t batch_cnt[kBatchSegs];                 // draw: the logits equal to the drawn value per segment of the batch in hand ...
+  uint32_t batch_total[kMaxBatches];              // ... and per batch
+  uint16_t g_b0[kGroupsH], g_b1[kGroupsH];        // the penalised values inserted inside each group: [g_b0, g_b1) of the list
   double g_mass[kGroupsH + 2];
   uint32_t g_cnt[kGroupsH + 2];
   uint64_t scratch[32];
   double warp_m[kHW];
   uint32_t warp_c[kHW];
-  uint32_t n_side, n_b, cz, cninf, pz, pninf, oob, top_pos;    // cz / cninf: unpenalised zeros and -inf; pz / pninf: penalised ones
+  uint32_t n_side, n_b, cz, cninf, pz, pninf, oob, top_pos, top_group;    // cz / cninf: unpenalised zeros and -inf; pz / pninf: penalised ones
   int sel_g, last_g;
   uint32_t base_c; double base_m;
   float res_tau; uint32_t res_cum_c; double res_cum_m, res_excl_m;
@@ -178,9 +184,8 @@ __device__ __forceinline__ uint32_t hblock_scan_u32(uint32_t v, uint32_t* warp_c
   return __shfl_sync(kFull, winc - w, warp) + incl - v;
 }
 
-// first index j in [0, n) with a[j] >= key (a ascending)
-__device__ __forceinline__ uint32_t lower_bound_u16(const uint16_t* a, uint32_t n, uint32_t key) {
-  uint32_t lo = 0u, hi = n;
+// first index j in [lo, hi) with a[j] >= key (a ascending; hi: none)
+__device__ __forceinline__ uint32_t lower_bound_u16(const uint16_t* a, uint32_t lo, uint32_t hi, uint32_t key) {
   while (lo < hi) { const uint32_t mid = (lo + hi) >> 1; if (a[mid] < key) lo = mid + 1u; else hi = mid; }
   return lo;
 }
@@ -191,6 +196,13 @@ __device__ __forceinline__ uint32_t b_count_range(const HistSmem& s, uint32_t j0
 }
 __device__ __forceinline__ double b_mass_range(const HistSmem& s, uint32_t j0, uint32_t j1) {
   return j1 > j0 ? s.b_mass[j1 - 1u] - (j0 ? s.b_mass[j0 - 1u] : 0.0) : 0.0;
+}
+
+// The penalised values of group g that are inserted before position q0, and before q0 + 1: [ja, jb) and [jb, jc) of the list (single: a group of one position).
+__device__ __forceinline__ void group_items(const HistSmem& s, int g, uint32_t q0, bool single, uint32_t& ja, uint32_t& jb, uint32_t& jc) {
+  const uint32_t b0 = s.g_b0[g], b1 = s.g_b1[g];
+  ja = lower_bound_u16(s.b_ins, b0, b1, q0); jb = lower_bound_u16(s.b_ins, ja, b1, q0 + 1u);
+  jc = single ? jb : lower_bound_u16(s.b_ins, jb, b1, q0 + 2u);
 }
 
 // ---- the threshold walk ------------------------------------------------------------------------------------------------------
@@ -234,12 +246,8 @@ static __device__ void hist_walk(HistSmem& s, uint32_t k_target, double m_target
     const bool single = g == kZeroGroup || g == kNinfGroup;
     const uint32_t q0 = p0 + 2u * lane, q1 = q0 + 1u;
     const bool own = !single || lane == 0;
-    const uint32_t nb = s.n_b;
     uint32_t ja = 0u, jb = 0u, jc = 0u;
-    if (own) {
-      ja = lower_bound_u16(s.b_ins, nb, q0); jb = lower_bound_u16(s.b_ins, nb, q0 + 1u);
-      jc = single ? jb : lower_bound_u16(s.b_ins, nb, q0 + 2u);
-    }
+    if (own) group_items(s, g, q0, single, ja, jb, jc);
     const uint32_t ca0 = own ? cnt_of_pos(s, q0) : 0u, ca1 = (own && !single) ? cnt_of_pos(s, q1) : 0u;
     const float va0 = val_of_pos(q0), va1 = val_of_pos(q1);
     const double ma0 = (MASS && ca0) ? static_cast<double>(ca0) * softmass(va0, vmax, inv_t) : 0.0;
@@ -302,34 +310,29 @@ static __device__ void hist_walk(HistSmem& s, uint32_t k_target, double m_target
 }
 
 // ---- the draws -----------------------------------------------------------------------------------------------------------------
-// 8-bit mask of the logits of a chunk whose BF16 code equals `code` (zero = true: whose value is zero, either sign).
-__device__ __forceinline__ uint32_t equal_mask8(const uint4 q, uint32_t code2, bool zero) {
-  const uint32_t strip = zero ? 0x7FFF7FFFu : 0xFFFFFFFFu;
-  const uint32_t m0 = __vcmpeq2(q.x & strip, code2), m1 = __vcmpeq2(q.y & strip, code2), m2 = __vcmpeq2(q.z & strip, code2), m3 = __vcmpeq2(q.w & strip, code2);
-  if ((m0 | m1 | m2 | m3) == 0u) return 0u;
-  return (m0 & 1u) | ((m0 >> 15) & 2u) | ((m1 & 1u) << 2) | ((m1 >> 13) & 8u) | ((m2 & 1u) << 4) | ((m2 >> 11) & 32u) | ((m3 & 1u) << 6) | ((m3 >> 9) & 128u);
-}
-
 // The inverse-CDF draw: the kept set in descending value order, equal values by ascending index. Equal values have equal
 // weights, so the histograms decide almost everything: the total weight S, hence the target; the group of 64 window positions
 // where the cumulative weight crosses it (a block scan over the groups' weights); inside the group one warp walks the merged
 // sequence of window positions and distinct penalised values down to the value v where the crossing lies. What is left is the
 // floor((target - weight above v) / w(v))-th smallest index among the logits equal to v: the row is looked at again (L2) only to
-// COUNT them -- segments of 256 logits from whichever end is nearer, a batch of kBatchSegs per barrier, packed 16-bit compares
-// against v's raw code, the penalised logits equal to v as per-segment corrections (s.seg_fix) -- and the warp that holds the
-// segment locates the token. Every thread calls; every thread gets the token (-1: the kept set has no weight).
+// COUNT them -- segments of 256 logits from whichever end is nearer, packed compares against v (most segments have none and cost a
+// vote), the penalised logits equal to v added per segment (s.seg_pen) -- and one warp locates the token in the segment that holds it.
+// A batch of 160 segments ends with one barrier: with 64 to a batch, a scan of the counts by every warp behind each, the counting took
+// 7.4 us of a row alone on its SM and 11.3 beside another one (151,936 logits); 3.7 and 6.2 so.
+// Every thread calls; every thread gets the token (-1: the kept set has no weight).
 static __device__ int hist_draw_inverse_cdf(const SampleDev& P, HistSmem& s, const uint32_t* pen, const uint16_t* rowp, int n_chunks, float tau, float vmax, float T, float u,
                                      uint64_t* out_total, bool total_only = false) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const float c2 = exp2_scale(T);
   const uint32_t n_side = s.n_side, n_b = s.n_b;
+  const int g_last = tau > -INFINITY ? group_of_pos(ins_pos(tau)) : kGroupsH;   // groups below that hold nothing at or above tau
   unsigned long long* g_w = reinterpret_cast<unsigned long long*>(s.g_mass);   // the groups' weights take the place of their masses
   auto kept_weight = [&](float v, uint32_t n) -> uint64_t { return (n && v >= tau) ? static_cast<uint64_t>(n) * weight_q40(v, vmax, c2) : 0ull; };
   // ---- the weight of every group: window positions ...
   for (int sg = warp; sg < static_cast<int>(kSlots) / kGrpSlots; sg += kHW) {
     const int g = sg < kSignGroups ? kSignGroups - 1 - sg : sg + 1;
     uint64_t w = 0ull;
-    if (s.g_cnt[g] != 0u) {                                                // (warp-uniform)
+    if (g <= g_last && s.g_cnt[g] != 0u) {                                 // (warp-uniform)
       const uint32_t h = s.hist[sg * 32 + lane];
       if (h) {
         const uint32_t slot = static_cast<uint32_t>(sg) * kGrpSlots + 2u * lane;
@@ -374,10 +377,7 @@ static __device__ int hist_draw_inverse_cdf(const SampleDev& P, HistSmem& s, con
     const uint32_t q0 = p0 + 2u * lane, q1 = q0 + 1u;
     const bool own = !single || lane == 0;
     uint32_t ja = 0u, jb = 0u, jc = 0u;
-    if (own) {
-      ja = lower_bound_u16(s.b_ins, n_b, q0); jb = lower_bound_u16(s.b_ins, n_b, q0 + 1u);
-      jc = single ? jb : lower_bound_u16(s.b_ins, n_b, q0 + 2u);
-    }
+    if (own) group_items(s, g, q0, single, ja, jb, jc);
     const uint32_t ca0 = own ? cnt_of_pos(s, q0) : 0u, ca1 = (own && !single) ? cnt_of_pos(s, q1) : 0u;
     const float va0 = val_of_pos(q0), va1 = val_of_pos(q1);
     const uint32_t n_items = (jc - ja) + 2u;
@@ -422,89 +422,99 @@ static __device__ int hist_draw_inverse_cdf(const SampleDev& P, HistSmem& s, con
   const uint32_t n_raw = s.res_cum_c, n_pen = s.base_c, members = n_raw + n_pen;
   const uint64_t each = weight_q40(v_star, vmax, c2);
   const uint32_t want = static_cast<uint32_t>((target - *reinterpret_cast<const unsigned long long*>(&s.res_cum_m)) / each);   // < members
-  // ---- the penalised logits equal to the value, per segment
-  unsigned int* seg_cnt = reinterpret_cast<unsigned int*>(s.seg_fix);      // (cleared with seg_fix at the start of the row)
+  // ---- the penalised logits equal to the value, per segment (cleared at the start of the row)
   if (n_pen) {
-    for (uint32_t i = tid; i < n_side; i += kHB) if (penalised_value(s.side_raw[i], P.rho, P.pi) == v_star) atomicAdd(&seg_cnt[s.ids[i] >> 8], 1u);
+    for (uint32_t i = tid; i < n_side; i += kHB) if (penalised_value(s.side_raw[i], P.rho, P.pi) == v_star) atomicAdd(&s.seg_pen[s.ids[i] >> 8], 1u);
+    __syncthreads();
   }
-  // the raw code of the value, if a window position carries it (0xFFFFFFFF: none -- every member is a penalised logit)
-  const bool zero = v_star == 0.0f;
-  const uint32_t code = n_raw ? (zero ? 0u : (__float_as_uint(v_star) >> 16)) : 0xFFFFFFFFu;
-  const uint32_t code2 = code | (code << 16);
+  // v as a packed pair, if a window position carries it (n_raw > 0; else every member is a penalised logit). The compare takes zeros of either sign.
+  const uint32_t code = n_raw ? (__float_as_uint(v_star) >> 16) : 0xFF80u, code2 = code | (code << 16);
+  const __nv_bfloat162 v2 = *reinterpret_cast<const __nv_bfloat162*>(&code2);
   const bool forward = want < members - want;
   const uint32_t tt = forward ? want : members - 1u - want;               // the first segment, in scan order, whose running count exceeds tt
-  __syncthreads();                                                        // seg_cnt is complete
   // ---- the segments, a batch at a time, from the nearer end
   const uint4* p4 = reinterpret_cast<const uint4*>(rowp);
   const int n_seg = (n_chunks + kSegChunks - 1) / kSegChunks;
-  uint32_t run = 0u, before_cnt = 0u, found_total = 0u;
-  int found = -1, found_b0 = 0, buf = 0;
-  unsigned int* batch_cnt = reinterpret_cast<unsigned int*>(s.batch_sum);  // [2][kBatchSegs]
-  for (int b0 = 0; b0 < n_seg && found < 0; b0 += kBatchSegs, buf ^= 1) {
-    uint4 q[kDrawIters];                                                  // the warp's chunks of this batch, all in flight at once
+  uint32_t run = 0u;
+  int b0 = 0;
+#pragma unroll 1
+  for (int batch = 0;; batch++, b0 += kBatchSegs) {
+    uint32_t mine = 0u;                                                   // lane i: what the warp's i-th segment holds
+    if (n_raw) {
 #pragma unroll
-    for (int it = 0; it < kDrawIters; it++) {
-      const int k = b0 + it * kHW + warp, seg = forward ? k : n_seg - 1 - k, cc = seg * kSegChunks + lane;
-      q[it] = (n_raw && k < n_seg && cc < n_chunks) ? __ldg(p4 + cc) : make_uint4(0xFF80FF80u, 0xFF80FF80u, 0xFF80FF80u, 0xFF80FF80u);
-    }
+      for (int h = 0; h < kDrawIters; h += kDrawDeep) {
+        uint4 q[kDrawDeep];
 #pragma unroll
-    for (int it = 0; it < kDrawIters; it++) {
-      const int k = b0 + it * kHW + warp, seg = forward ? k : n_seg - 1 - k, cc = seg * kSegChunks + lane;
-      uint32_t mask = (n_raw && k < n_seg && cc < n_chunks) ? equal_mask8(q[it], code2, zero) : 0u;
-      if (mask && pen != nullptr) mask &= ~((pen[cc >> 2] >> ((cc & 3) * 8)) & 0xFFu);
-      const uint32_t cnt = warp_sum_u32(__popc(mask));
-      if (lane == 0) batch_cnt[buf * kBatchSegs + it * kHW + warp] = k < n_seg ? cnt + seg_cnt[seg] : 0u;
+        for (int j = 0; j < kDrawDeep; j++) {
+          const int k = b0 + (h + j) * kHW + warp, cc = (forward ? k : n_seg - 1 - k) * kSegChunks + lane;
+          q[j] = (k < n_seg && cc < n_chunks) ? __ldg(p4 + cc) : make_uint4(0xFF80FF80u, 0xFF80FF80u, 0xFF80FF80u, 0xFF80FF80u);   // (-inf is never drawn)
+        }
+#pragma unroll
+        for (int j = 0; j < kDrawDeep; j++) {
+          const uint32_t m0 = __heq2_mask(*reinterpret_cast<const __nv_bfloat162*>(&q[j].x), v2), m1 = __heq2_mask(*reinterpret_cast<const __nv_bfloat162*>(&q[j].y), v2);
+          const uint32_t m2 = __heq2_mask(*reinterpret_cast<const __nv_bfloat162*>(&q[j].z), v2), m3 = __heq2_mask(*reinterpret_cast<const __nv_bfloat162*>(&q[j].w), v2);
+          if (!__any_sync(kFull, (m0 | m1 | m2 | m3) != 0u)) continue;
+          uint32_t mask = mask8(m0, m1, m2, m3);
+          if (pen != nullptr && mask) {
+            const int k = b0 + (h + j) * kHW + warp, cc = (forward ? k : n_seg - 1 - k) * kSegChunks + lane;
+            mask &= ~((pen[cc >> 2] >> ((cc & 3) * 8)) & 0xFFu);
+          }
+          const uint32_t cnt = warp_sum_u32(__popc(mask));
+          if (lane == h + j) mine = cnt;
+        }
+      }
     }
+    if (lane < kDrawIters) {
+      const int k = b0 + lane * kHW + warp;
+      if (n_pen && k < n_seg) mine += s.seg_pen[forward ? k : n_seg - 1 - k];
+      s.batch_cnt[lane * kHW + warp] = mine;
+    }
+    const uint32_t held = warp_sum_u32(mine);
+    if (lane == 0 && held) atomicAdd(&s.batch_total[batch], held);
     __syncthreads();
-    // every warp scans the batch's counts for itself: no second barrier (the next batch writes the other buffer)
-    const uint32_t a = batch_cnt[buf * kBatchSegs + 2 * lane], b = batch_cnt[buf * kBatchSegs + 2 * lane + 1];
-    uint32_t incl = a + b;
+    const uint32_t total_b = s.batch_total[batch];
+    if (run + total_b > tt) break;
+    run += total_b;
+    if (b0 + kBatchSegs >= n_seg) return -1;                              // cannot happen: the segments hold `members` logits
+  }
+  // ---- the segment, and the logit inside it: one warp
+  if (warp == 0) {
+    constexpr int kPer = kBatchSegs / 32;
+    uint32_t c[kPer], sum = 0u;
+#pragma unroll
+    for (int j = 0; j < kPer; j++) { c[j] = s.batch_cnt[lane * kPer + j]; sum += c[j]; }
+    uint32_t incl = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) { const uint32_t t = __shfl_up_sync(kFull, incl, o); if (lane >= o) incl += t; }
-    const uint32_t excl = run + incl - a - b;
-    const bool hit_a = excl + a > tt, hit_b = excl + a + b > tt;
-    const uint32_t hits = __ballot_sync(kFull, hit_b);
-    if (hits) {
-      const int src = __ffs(hits) - 1;
-      const int idx = __shfl_sync(kFull, hit_a ? 2 * lane : 2 * lane + 1, src);
-      before_cnt = __shfl_sync(kFull, hit_a ? excl : excl + a, src);
-      found_total = __shfl_sync(kFull, hit_a ? a : b, src);
-      found = b0 + idx; found_b0 = b0;
+    uint32_t before = run + incl - sum, held = 0u; int idx = -1;
+#pragma unroll
+    for (int j = 0; j < kPer; j++) {
+      if (idx < 0 && before + c[j] > tt) { idx = lane * kPer + j; held = c[j]; }
+      if (idx < 0) before += c[j];
     }
-    run += __shfl_sync(kFull, incl, 31);
-  }
-  if (found < 0) return -1;                                               // cannot happen: the segments hold `members` logits
-  // ---- inside the segment: the (local)-th logit equal to the value, in index order, by the warp that counted the segment (its
-  // chunk comes back from L2: keeping a batch of chunks alive across the loop would cost the kernel registers it does not have)
-  {
-    const int idx = found - found_b0;                                     // position of the segment in its batch: it * kHW + warp
-    if (warp == idx % kHW) {
-      const int seg = forward ? found : n_seg - 1 - found;
-      const uint32_t prefix = forward ? before_cnt : members - before_cnt - found_total;   // members before the segment
-      const uint32_t local = want - prefix;
-      const int cc = seg * kSegChunks + lane;
-      const uint4 qf = cc < n_chunks ? __ldg(p4 + cc) : make_uint4(0xFF80FF80u, 0xFF80FF80u, 0xFF80FF80u, 0xFF80FF80u);
-      const uint32_t bits = (pen != nullptr && cc < n_chunks) ? ((pen[cc >> 2] >> ((cc & 3) * 8)) & 0xFFu) : 0u;
-      const uint32_t words[4] = {qf.x, qf.y, qf.z, qf.w};
-      uint32_t hit = 0u;
+    const int src = __ffs(static_cast<int>(__ballot_sync(kFull, idx >= 0))) - 1;   // (there is one: the batch's total says so)
+    idx = __shfl_sync(kFull, idx, src); before = __shfl_sync(kFull, before, src); held = __shfl_sync(kFull, held, src);
+    const int seg = forward ? b0 + idx : n_seg - 1 - (b0 + idx);
+    const uint32_t local = want - (forward ? before : members - before - held);   // the logit's rank, in index order, inside the segment
+    const int cc = seg * kSegChunks + lane;
+    const uint4 qf = cc < n_chunks ? __ldg(p4 + cc) : make_uint4(0xFF80FF80u, 0xFF80FF80u, 0xFF80FF80u, 0xFF80FF80u);
+    const uint32_t bits = (pen != nullptr && cc < n_chunks) ? ((pen[cc >> 2] >> ((cc & 3) * 8)) & 0xFFu) : 0u;
+    const uint32_t words[4] = {qf.x, qf.y, qf.z, qf.w};
+    uint32_t hit = 0u;
 #pragma unroll
-      for (int e = 0; e < kChunk; e++) {
-        const uint32_t cde = (e & 1) ? (words[e >> 1] >> 16) : (words[e >> 1] & 0xFFFFu);
-        const bool is_pen = (bits >> e) & 1u;
-        const bool m = cc < n_chunks && (is_pen ? (n_pen && penalised_value(cde, P.rho, P.pi) == v_star)
-                                               : (n_raw && (zero ? (cde & 0x7FFFu) == 0u : cde == code)));
-        hit |= m ? (1u << e) : 0u;
-      }
-      const uint32_t mine = __popc(hit);
-      uint32_t incl = mine;
+    for (int e = 0; e < kChunk; e++) {
+      const uint32_t cde = (e & 1) ? (words[e >> 1] >> 16) : (words[e >> 1] & 0xFFFFu);
+      const bool m = ((bits >> e) & 1u) ? (n_pen && penalised_value(cde, P.rho, P.pi) == v_star) : (n_raw && hcode_val(cde) == v_star);
+      hit |= (m && cc < n_chunks) ? (1u << e) : 0u;
+    }
+    const uint32_t here = __popc(hit);
+    uint32_t upto = here;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) { const uint32_t t = __shfl_up_sync(kFull, incl, o); if (lane >= o) incl += t; }
-      const uint32_t excl = incl - mine;
-      if (excl <= local && local < incl) {
-        uint32_t r = excl;
+    for (int o = 1; o < 32; o <<= 1) { const uint32_t t = __shfl_up_sync(kFull, upto, o); if (lane >= o) upto += t; }
+    if (upto - here <= local && local < upto) {
+      uint32_t r = upto - here;
 #pragma unroll
-        for (int e = 0; e < kChunk; e++) if ((hit >> e) & 1u) { if (r == local) { s.token = cc * kChunk + e; break; } r++; }
-      }
+      for (int e = 0; e < kChunk; e++) if ((hit >> e) & 1u) { if (r == local) { s.token = cc * kChunk + e; break; } r++; }
     }
   }
   __syncthreads();
@@ -597,7 +607,7 @@ static __device__ void sample_row_hist(const SampleDev& P, int row, int next, Hi
 
   // ---- phase 0: clear; the history's distinct ids as a bitmap and as a list -------------------------------------------------
   const bool stochastic = T > 0.0f;
-  if (tid == 0) { s.n_side = 0u; s.n_b = 0u; s.cz = 0u; s.cninf = 0u; s.pz = 0u; s.pninf = 0u; s.oob = 0u; s.top_pos = 0xFFFFFFFFu; s.token = -1; s.key_bound = 0u; }
+  if (tid == 0) { s.n_side = 0u; s.n_b = 0u; s.cz = 0u; s.cninf = 0u; s.pz = 0u; s.pninf = 0u; s.oob = 0u; s.top_pos = 0xFFFFFFFFu; s.top_group = 0xFFFFFFFFu; s.token = -1; s.key_bound = 0u; }
   if (stochastic) {
     const uint4 z4 = make_uint4(0u, 0u, 0u, 0u);
     uint4* h4 = reinterpret_cast<uint4*>(s.hist);
@@ -607,9 +617,10 @@ static __device__ void sample_row_hist(const SampleDev& P, int row, int next, Hi
       for (int i = tid; i < static_cast<int>(kSlots) / 16; i += kHB) ph4[i] = z4;
     }
     if (P.draw == LM_DRAW_INVERSE_CDF) {
-      uint4* f4 = reinterpret_cast<uint4*>(s.seg_fix);
-      for (int i = tid; i < (n_chunks / kSegChunks + 2) / 2; i += kHB) f4[i] = z4;
+      for (int i = tid; i < kMaxSegs; i += kHB) s.seg_pen[i] = 0u;
+      if (tid < kMaxBatches) s.batch_total[tid] = 0u;
     }
+    if (tid < kGroupsH) { s.g_b0[tid] = 0u; s.g_b1[tid] = 0u; }
   }
   if (pen_on) {
     uint4* b4 = reinterpret_cast<uint4*>(pen);
@@ -722,23 +733,25 @@ static __device__ void sample_row_hist(const SampleDev& P, int row, int next, Hi
   }
   if (s.oob) { hand_on(); return; }
   // ---- phase 3: group counts and the top position of the main histogram; the penalised histogram compacted into a list --------
-  for (int sg = warp; sg < static_cast<int>(kSlots) / kGrpSlots; sg += kHW) {
-    const uint32_t w = s.hist[sg * 32 + lane];
-    const uint32_t tot = warp_sum_u32((w & 0xFFFFu) + (w >> 16));
-    const int g = sg < kSignGroups ? kSignGroups - 1 - sg : sg + 1;
-    if (lane == 0) s.g_cnt[g] = tot;
-    if (tot) {
-      const uint32_t slot = static_cast<uint32_t>(sg) * kGrpSlots + 2u * lane;
-      uint32_t p = 0xFFFFFFFFu;
-      if (w & 0xFFFFu) p = pos_of_slot(slot);
-      if (w >> 16) p = min(p, pos_of_slot(slot + 1u));
-      p = warp_min_u32(p);
-      if (lane == 0) atomicMin(&s.top_pos, p);
+  // Two threads to a group, sixteen words each, one packed add per word (the words of neighbouring threads in turn: no bank is met
+  // twice). A warp per group with a reduction by shuffles took 7.2 us of a row alone on its SM and 10.3 beside another; 3.4 and 4.7 so.
+  {
+    const uint4* h4 = reinterpret_cast<const uint4*>(s.hist);
+    uint32_t tot = 0u;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const uint4 w = h4[tid * 4 + ((j + (tid >> 1)) & 3)];
+      tot = __dp2a_lo(w.x, 0x0101u, tot); tot = __dp2a_lo(w.y, 0x0101u, tot); tot = __dp2a_lo(w.z, 0x0101u, tot); tot = __dp2a_lo(w.w, 0x0101u, tot);
     }
+    tot += __shfl_xor_sync(kFull, tot, 1);
+    const int sg = tid >> 1, g = sg < kSignGroups ? kSignGroups - 1 - sg : sg + 1;
+    if (!(tid & 1)) s.g_cnt[g] = tot;
+    const uint32_t first = warp_min_u32(tot ? static_cast<uint32_t>(g) : 0xFFFFFFFFu);
+    if (lane == 0 && first != 0xFFFFFFFFu) atomicMin(&s.top_group, first);
   }
   if (tid == 0) {
     s.g_cnt[kZeroGroup] = s.cz; s.g_cnt[kNinfGroup] = s.cninf;
-    if (s.cz) atomicMin(&s.top_pos, kPosZero); else if (s.cninf) atomicMin(&s.top_pos, kPosNinf);
+    if (s.cz) atomicMin(&s.top_group, static_cast<uint32_t>(kZeroGroup)); else if (s.cninf) atomicMin(&s.top_group, static_cast<uint32_t>(kNinfGroup));
   }
   if (pen_on) {
     // thread t reads 32 counters in walk order: slots 8191 - 32 t downwards (positive values), then 8192 + 32 (t - 256) upwards
@@ -746,12 +759,14 @@ static __device__ void sample_row_hist(const SampleDev& P, int row, int next, Hi
     const uint32_t first = posv ? kWinCodes - 32u - 32u * tid : kWinCodes + 32u * (tid - kHB / 2);   // lowest slot of the 32
     const uint4 a = reinterpret_cast<const uint4*>(s.pen_hist)[first / 16u], b = reinterpret_cast<const uint4*>(s.pen_hist)[first / 16u + 1u];
     const uint32_t w8[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-    uint32_t nz = 0u, sb = 0u;
+    uint32_t occupied = 0u, sb = 0u;                                      // a bit per counter that is not zero; their sum
 #pragma unroll
-    for (int k = 0; k < 8; k++) if (w8[k]) {
-#pragma unroll
-      for (int e = 0; e < 4; e++) { const uint32_t c = (w8[k] >> (8 * e)) & 0xFFu; nz += c ? 1u : 0u; sb += c; }
+    for (int k = 0; k < 8; k++) {
+      const uint32_t w = w8[k], top = (((w & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | w) & 0x80808080u;
+      occupied |= (((top >> 7) * 0x01020408u) >> 24) << (4 * k);           // (the four top bits side by side)
+      sb = __dp4a(w, 0x01010101u, sb);
     }
+    uint32_t nz = __popc(occupied);
     // the penalised zeros sit between the positive and the negative codes, the penalised -inf at the very end (marker slots)
     const uint32_t zeros = tid == kHB / 2 ? s.pz : 0u, ninfs = tid == kHB - 1 ? s.pninf : 0u;
     nz += (zeros ? 1u : 0u) + (ninfs ? 1u : 0u); sb += zeros + ninfs;
@@ -760,21 +775,13 @@ static __device__ void sample_row_hist(const SampleDev& P, int row, int next, Hi
     if ((tot >> 16) != n_side) s.oob = 1u;                                 // an 8-bit counter wrapped
     if (tid == 0) s.n_b = tot & 0xFFFFu;
     if (zeros) { s.b_ins[off] = 0xFFFFu; s.b_cnt[off] = static_cast<uint16_t>(zeros); off++; }
-    if (nz) {                                                             // (slot, count) pairs, descending value order; the values follow below
-#pragma unroll
-      for (int k = 0; k < 8; k++) {
-        const int kk = posv ? 7 - k : k;
-        const uint32_t w = w8[kk];
-        if (!w) continue;
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-          const int ee = posv ? 3 - e : e;
-          const uint32_t c = (w >> (8 * ee)) & 0xFFu;
-          if (!c) continue;
-          s.b_ins[off] = static_cast<uint16_t>(first + static_cast<uint32_t>(4 * kk + ee)); s.b_cnt[off] = static_cast<uint16_t>(c);
-          off++;
-        }
-      }
+    const uint8_t* counters = reinterpret_cast<const uint8_t*>(s.pen_hist) + first;
+#pragma unroll 1
+    while (occupied) {                                                    // (slot, count) pairs, descending value order; the values follow below
+      const int b = posv ? 31 - __clz(static_cast<int>(occupied)) : __ffs(static_cast<int>(occupied)) - 1;
+      occupied ^= 1u << b;
+      s.b_ins[off] = static_cast<uint16_t>(first + static_cast<uint32_t>(b)); s.b_cnt[off] = counters[b];
+      off++;
     }
     if (ninfs) { s.b_ins[off] = 0xFFFEu; s.b_cnt[off] = static_cast<uint16_t>(ninfs); }
   }
@@ -785,6 +792,18 @@ static __device__ void sample_row_hist(const SampleDev& P, int row, int next, Hi
     const uint32_t slot = s.b_ins[j];
     const float v = penalised_value(slot == 0xFFFFu ? 0x0000u : (slot == 0xFFFEu ? 0xFF80u : code_of_slot(slot)), P.rho, P.pi);
     s.b_val[j] = v; s.b_ins[j] = static_cast<uint16_t>(ins_pos(v));
+  }
+  if (warp == kHW - 1) {                                                  // the highest occupied position, in its group
+    const uint32_t g = s.top_group;
+    if (g == kZeroGroup || g == kNinfGroup) { if (lane == 0) s.top_pos = g == kZeroGroup ? kPosZero : kPosNinf; }
+    else if (g < kGroupsH) {
+      const uint32_t slot = (g < kZeroGroup ? static_cast<uint32_t>(kSignGroups) - 1u - g : g - 1u) * kGrpSlots + 2u * lane, w = s.hist[slot >> 1];
+      uint32_t p = 0xFFFFFFFFu;
+      if (w & 0xFFFFu) p = pos_of_slot(slot);
+      if (w >> 16) p = min(p, pos_of_slot(slot + 1u));
+      p = warp_min_u32(p);
+      if (lane == 0) s.top_pos = p;
+    }
   }
   __syncthreads();
   const float top_a = s.top_pos != 0xFFFFFFFFu ? val_of_pos(s.top_pos) : -INFINITY;
@@ -811,6 +830,11 @@ static __device__ void sample_row_hist(const SampleDev& P, int row, int next, Hi
     if (tid == 0) { s.g_mass[kZeroGroup] = s.cz ? static_cast<double>(s.cz) * softmass(0.0f, vmax, inv_t) : 0.0; s.g_mass[kNinfGroup] = 0.0; }
   }
   if (n_b) {
+    for (uint32_t j = tid; j < n_b; j += kHB) {                           // where each group's penalised values begin and end
+      const int g = group_of_pos(s.b_ins[j]);
+      if (j == 0u || group_of_pos(s.b_ins[j - 1u]) != g) s.g_b0[g] = static_cast<uint16_t>(j);
+      if (j + 1u == n_b || group_of_pos(s.b_ins[j + 1u]) != g) s.g_b1[g] = static_cast<uint16_t>(j + 1u);
+    }
     // counts and masses of the penalised values become running sums over the list (thread t owns a few consecutive entries):
     // any run of the list is then a difference of two entries
     constexpr int kPer = kPenCap / kHB;
@@ -842,12 +866,9 @@ static __device__ void sample_row_hist(const SampleDev& P, int row, int next, Hi
     }
   }
   __syncthreads();
-  for (uint32_t j = tid; j < n_b; j += kHB) {                             // the last entry of each group's run adds the run to the group
-    const int g = group_of_pos(s.b_ins[j]);
-    if (j + 1u < n_b && group_of_pos(s.b_ins[j + 1u]) == g) continue;
-    const uint32_t start = lower_bound_u16(s.b_ins, n_b, first_pos_of_group(g));
-    s.g_cnt[g] += b_count_range(s, start, j + 1u);
-    if (has_p) s.g_mass[g] += b_mass_range(s, start, j + 1u);
+  if (n_b && tid < kGroupsH) {                                            // each group's run joins the group
+    const uint32_t j0 = s.g_b0[tid], j1 = s.g_b1[tid];
+    if (j1 > j0) { s.g_cnt[tid] += b_count_range(s, j0, j1); if (has_p) s.g_mass[tid] += b_mass_range(s, j0, j1); }
   }
   __syncthreads();
   {

@@ -186,3 +186,25 @@ def test_the_fp32_mass_of_rows_far_from_zero():
     r, tok, tau = gpu_and_oracle(cfg)
     np.testing.assert_array_equal(r.tau.cpu().numpy(), tau)
     np.testing.assert_array_equal(r.tokens.cpu().numpy(), tok)
+
+
+@pytest.mark.parametrize("vocab", [8, 264, 256 * 160, 256 * 160 + 8, 2 * 256 * 160 + 264, 262144])
+@pytest.mark.parametrize("penalised", [False, True])
+def test_the_histogram_draw_at_the_edges_of_its_batches(vocab, penalised):
+    """The inverse-CDF draw counts equal logits in batches of 160 segments of 256, from the nearer end of the row. Runs of thousands of equal logits
+    (multiples of 1/2) put the drawn one into any batch and segment; vocabularies of one batch, a chunk more, two batches and a ragged segment."""
+    rows = 48
+    rng = np.random.default_rng(vocab)
+    codes = oracle.f32_to_bf16((np.round(rng.standard_normal((rows, vocab)) * 4.0) / 2.0).astype(np.float32))
+    u = np.concatenate([[0.0, 1.0 - 2.0 ** -24], np.linspace(0.01, 0.99, rows - 2)]).astype(np.float32)
+    hist = rng.integers(0, vocab, (rows, min(vocab, 1500))).astype(np.int32) if penalised else None
+    pen = dict(repetition_penalty=2.0, presence_penalty=0.5) if penalised else {}
+    T = rng.uniform(0.5, 3.0, rows).astype(np.float32)
+    p = lm.SamplingParams(draw="inverse_cdf", exact_only=True, temperature=torch.from_numpy(T).cuda(), top_p=0.97, **pen)
+    x, ut, h = bf16_tensor(codes), torch.from_numpy(u).cuda(), torch.from_numpy(hist).cuda() if penalised else None
+    assert "sample_hist_kernel" in routes.names(lambda: lm.sample(x, p, history=h, uniforms=ut))
+    r = lm.sample(x, p, history=h, uniforms=ut, return_tau=True, return_status=True)
+    tok, tau, _ = oracle.sample_batch(codes, temperature=T, top_p=0.97, history=hist, draw="inverse_cdf", uniforms=u, n_threads=THREADS, **pen)
+    np.testing.assert_array_equal(r.tau.cpu().numpy(), tau)
+    np.testing.assert_array_equal(r.tokens.cpu().numpy(), tok)
+    assert not np.any(r.status.cpu().numpy() & 1)                            # none handed on to the generic algorithm
