@@ -22,6 +22,7 @@ static __global__ void __launch_bounds__(kArgmaxThreads) argmax_cluster_kernel(c
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int rank = C > 1 ? static_cast<int>(cluster_rank()) : 0, row = C > 1 ? static_cast<int>(blockIdx.x) / C : static_cast<int>(blockIdx.x);
   if (C > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+  after_predecessor();
   ClusterRow R;
   R.row = static_cast<const char*>(logits) + static_cast<size_t>(row) * static_cast<size_t>(row_stride) * (F32 ? 4 : 2);
   R.V = vocab; R.pen = nullptr; R.rho = 1.0f; R.pi = 0.0f; R.vals = nullptr; R.nv = 0;

@@ -34,7 +34,7 @@ static int sample_blocks(int64_t rows, int64_t vocab, int sms, bool listed) {
 
 // The instances of the sampler: FP32 / BF16 rows, the slices cached in shared memory or not, and then one block per SM or two.
 constexpr size_t kMostSmem = 227 * 1024, kHalfSmem = kMostSmem / 2 - 1024;
-struct ClusterPlan { int C; size_t smem; bool cached, two; };
+struct ClusterPlan { int C; size_t smem; bool cached, two, ordered; };
 
 template <bool F32, bool CACHED, int kPerSM>
 static int cluster_ready(int instance, int C, bool* fits) {
@@ -53,14 +53,8 @@ static int cluster_ready(bool f32, const ClusterPlan& p, bool* fits) {
 
 template <bool F32, bool CACHED, int kPerSM>
 static int launch_cluster(const SampleDev& P, const ClusterPlan& p, cudaStream_t st) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(P.rows) * static_cast<unsigned>(p.C)); cfg.blockDim = dim3(kClusterBlock); cfg.dynamicSmemBytes = p.smem; cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = static_cast<unsigned>(p.C); attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr; cfg.numAttrs = p.C > 1 ? 1 : 0;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, sample_cluster_kernel<F32, CACHED, kClusterBlock, kPerSM>, P, p.C);
-  return e == cudaSuccess ? LM_OK : cuda_fail(e);
+  return launch_beside(sample_cluster_kernel<F32, CACHED, kClusterBlock, kPerSM>, dim3(static_cast<unsigned>(P.rows) * static_cast<unsigned>(p.C)), kClusterBlock,
+                       p.smem, p.C, st, P, p.C, p.ordered ? 1 : 0);
 }
 
 int sample_clusters(const SampleDev& P, int sms, cudaStream_t st) {
@@ -76,6 +70,7 @@ int sample_clusters(const SampleDev& P, int sms, cudaStream_t st) {
     p.smem = head + (p.cached ? per * 32 : 0) + marks;
     if (p.smem < generic) p.smem = generic;
     p.two = static_cast<long long>(P.rows) * C > sms && p.smem <= kHalfSmem;   // two blocks per SM
+    p.ordered = P.top_k != nullptr && P.rows <= kOrderRows && static_cast<long long>(P.rows) * C > (p.two ? 2LL : 1LL) * sms;   // (more clusters than run at once)
     return p;
   };
   int rc = LM_OK;
@@ -97,14 +92,8 @@ static int launch_argmax(const void* logits, int rows, int vocab, int64_t row_st
   const int rc = ensure_dynamic_smem(slot, fn, 1, true);
   if (rc != LM_OK) return rc;
   C = cluster_that_fits(C, [&](int c) { return cluster_fits(slot, fn, kArgmaxThreads, 0, c); });
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(rows) * static_cast<unsigned>(C)); cfg.blockDim = dim3(kArgmaxThreads); cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = static_cast<unsigned>(C); attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr; cfg.numAttrs = C > 1 ? 1 : 0;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, argmax_cluster_kernel<F32>, logits, vocab, row_stride, out32, out64, C);
-  return e == cudaSuccess ? LM_OK : cuda_fail(e);
+  return launch_beside(argmax_cluster_kernel<F32>, dim3(static_cast<unsigned>(rows) * static_cast<unsigned>(C)), kArgmaxThreads, 0, C, st, logits, vocab, row_stride,
+                       out32, out64, C);
 }
 
 int argmax_clusters(const void* logits, int dtype, int rows, int vocab, int64_t row_stride, int32_t* out32, int64_t* out64, cudaStream_t st) {
@@ -123,14 +112,7 @@ static int launch_draft_q(const DraftQDev& P, int C, cudaStream_t st) {
   const int rc = ensure_dynamic_smem(slot, fn, 1, true);
   if (rc != LM_OK) return rc;
   C = cluster_that_fits(C, [&](int c) { return cluster_fits(slot, fn, kDraftQThreads, 0, c); });
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(P.rows) * static_cast<unsigned>(C)); cfg.blockDim = dim3(kDraftQThreads); cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = static_cast<unsigned>(C); attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr; cfg.numAttrs = C > 1 ? 1 : 0;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, draft_q_kernel<F32>, P, C);
-  return e == cudaSuccess ? LM_OK : cuda_fail(e);
+  return launch_beside(draft_q_kernel<F32>, dim3(static_cast<unsigned>(P.rows) * static_cast<unsigned>(C)), kDraftQThreads, 0, C, st, P, C);
 }
 
 int draft_q_clusters(const DraftQDev& P, int sms, cudaStream_t st) {

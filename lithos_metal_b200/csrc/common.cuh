@@ -20,6 +20,11 @@ constexpr int kWarps = kBlock / 32;
 constexpr int kChunk = 8;              // consecutive logits one thread takes per step (one 128-bit load of BF16)
 constexpr uint32_t kFull = 0xFFFFFFFFu;
 
+// A kernel that may be launched beside its predecessor in the stream (launch_beside, host.cuh): here that one is complete and what it wrote is
+// visible. Every thread calls this before it touches device memory, and before it returns. What is launched behind this kernel the same way may
+// then be made ready (its blocks wait here in turn).
+__device__ __forceinline__ void after_predecessor() { asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- element access ----------------------------------------------------------------------------------------
 
 __device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }

@@ -48,6 +48,7 @@ static __global__ void __launch_bounds__(kDraftQThreads) draft_q_kernel(const Dr
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int rank = C > 1 ? static_cast<int>(cluster_rank()) : 0, row = static_cast<int>(blockIdx.x) / C;
   uint64_t seed = P.seed; uint32_t step = P.step;
+  after_predecessor();
   if (P.state) {
     StepStateView st{const_cast<uint32_t*>(P.state), P.t_max, P.g};
     if (st.done()) return;                                                  // every block sees the same state

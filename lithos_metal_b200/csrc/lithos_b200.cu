@@ -203,11 +203,11 @@ int lm_sample(const lm_sample_args* a) {
       rc = ensure_dynamic_smem(threads == kSliceBlockBig ? kSlotSlice : (threads == kSliceBlockSmall ? kSlotSliceSmall : kSlotSliceTiny), slice_fn, slice_smem);
       if (rc == LM_OK) rc = ensure_dynamic_smem(kSlotSlicedMerge, reinterpret_cast<const void*>(sliced_merge_kernel), gsmem);
       if (rc != LM_OK) return rc;
-      if (threads == kSliceBlockBig) slice_local_kernel<kSliceBlockBig><<<dim3(S.slices, P.rows), kSliceBlockBig, slice_smem, st>>>(S);
-      else if (threads == kSliceBlockSmall) slice_local_kernel<kSliceBlockSmall><<<dim3(S.slices, P.rows), kSliceBlockSmall, slice_smem, st>>>(S);
-      else slice_local_kernel<kSliceBlockTiny><<<dim3(S.slices, P.rows), kSliceBlockTiny, slice_smem, st>>>(S);
-      cudaError_t e = cudaGetLastError();
-      if (e != cudaSuccess) return cuda_fail(e);
+      const dim3 slice_grid(static_cast<unsigned>(S.slices), static_cast<unsigned>(P.rows));
+      rc = threads == kSliceBlockBig ? launch_beside(slice_local_kernel<kSliceBlockBig>, slice_grid, kSliceBlockBig, slice_smem, 1, st, S)
+         : threads == kSliceBlockSmall ? launch_beside(slice_local_kernel<kSliceBlockSmall>, slice_grid, kSliceBlockSmall, slice_smem, 1, st, S)
+                                       : launch_beside(slice_local_kernel<kSliceBlockTiny>, slice_grid, kSliceBlockTiny, slice_smem, 1, st, S);
+      if (rc != LM_OK) return rc;
       VpMergeDev M;
       M.bases = nullptr; M.pieces = 1;
       M.records = S.records; M.shards = S.slices; M.rows = P.rows; M.cap = S.cap; M.record_bytes = S.record_bytes;
@@ -218,14 +218,8 @@ int lm_sample(const lm_sample_args* a) {
       M.hand_on = 1; M.path_status = LM_STATUS_SLICED_PATH;
       merge_geometry(M);
       M.mass_band = S.need_mass ? slice_mass_band(S.slice_len, threads) : 0.0;
-      // the merge is launched with programmatic stream serialization: its blocks are resident and waiting when the slices complete
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-      attr[0].val.programmaticStreamSerializationAllowed = 1;
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(P.rows); cfg.blockDim = dim3(kVpMaxCandidates); cfg.dynamicSmemBytes = gsmem; cfg.stream = st; cfg.attrs = attr; cfg.numAttrs = 1;
-      e = cudaLaunchKernelEx(&cfg, sliced_merge_kernel, M, P);
-      return e == cudaSuccess ? LM_OK : cuda_fail(e);
+      // (the merge's blocks are resident and waiting when the slices complete)
+      return launch_beside(sliced_merge_kernel, dim3(static_cast<unsigned>(P.rows)), kVpMaxCandidates, gsmem, 1, st, M, P);
     }
   }
   const bool fast = a->dtype == LM_DTYPE_BF16 && a->out_stats == nullptr && a->out_probs == nullptr && a->vocab <= kHistMaxVocab &&

@@ -45,6 +45,7 @@ constexpr int kCGroups = 4096;           // group maxima per block
 constexpr int kCMaxBins = 512;           // bins of the group maxima
 constexpr int kCMaxRanks = 16;           // blocks of one cluster
 constexpr int kCQueue = 128;             // logits a warp's queue of the Gumbel draw holds
+constexpr int kOrderRows = 2048;         // rows whose order a block looks up (row_in_order)
 constexpr int kCRankOrder = 320;         // a list up to this long is ordered by counting larger keys, a longer one by bins first
 constexpr double kCMassBand = 1e-11;     // relative error of a logit's fixed-point softmass beyond its rounding: 7e-12 of the polynomial, a few 1e-16
 // Threads per block: a block-wide reduction costs shuffles in proportion to its warps (1024 threads: 0.5 us each, measured), so no more
@@ -1288,15 +1289,62 @@ static __device__ __noinline__ void phase_probs(const ClusterSmem& s, const Samp
   }
 }
 
+// The row that cluster `at` takes when there are more clusters than run at once: the long rows (no list of a top_k) first, then those with a
+// large top_k, so that no long one is begun when the rest are done. At most kOrderRows rows. (64 FP32 rows of 151,936 with mixed knobs, four blocks
+// each and one to an SM: 93.8 us in the order of the batch, 72.9 so; 48 BF16 rows of 50,257 53.0 and 47.0; 300 FP32 rows of 50,257 131 and 120.)
+template <int B>
+static __device__ __noinline__ int row_in_order(const SampleDev& P, int rows, int at, ClusterSmem& s) {
+  const int tid = threadIdx.x, lane = tid & 31;
+  uint32_t* count = s.fill;                                                 // [2][rows / 32]: the first two kinds per 32 rows (the bins, cleared above, lie elsewhere)
+  constexpr int kGroups = kOrderRows / 32;
+  auto kind_of = [&](int r) {
+    if (r >= rows) return 3;
+    const int k = P.top_k[r];
+    const float T = P.temperature ? P.temperature[r] : P.temperature_s;
+    return !(T > 0.0f) ? 2 : (k <= 0 || k > kCListK || (P.flags & LM_FLAG_EXACT_ONLY)) ? 0 : k > 64 ? 1 : 2;
+  };
+  for (int r = tid; r - lane < rows; r += B) {
+    const int kind = kind_of(r);
+    const uint32_t a = __ballot_sync(kFull, kind == 0), b = __ballot_sync(kFull, kind == 1);
+    if (lane == 0) { count[r >> 5] = __popc(a); count[kGroups + (r >> 5)] = __popc(b); }
+  }
+  __syncthreads();
+  const int groups = (rows + 31) >> 5;
+  uint32_t n0 = 0u, n1 = 0u;                                                // every warp for itself
+  for (int g = lane; g < groups; g += 32) { n0 += count[g]; n1 += count[kGroups + g]; }
+  n0 = warp_sum_u32(n0); n1 = warp_sum_u32(n1);
+  for (int r = tid; r - lane < rows; r += B) {
+    const int kind = kind_of(r), mine = r >> 5;
+    uint32_t b0 = 0u, b1 = 0u;
+    for (int g = lane; g < mine; g += 32) { b0 += count[g]; b1 += count[kGroups + g]; }
+    b0 = warp_sum_u32(b0); b1 = warp_sum_u32(b1);
+    const uint32_t a = __ballot_sync(kFull, kind == 0), b = __ballot_sync(kFull, kind == 1), below = (1u << lane) - 1u;
+    const uint32_t p0 = b0 + __popc(a & below), p1 = b1 + __popc(b & below);
+    const uint32_t place = kind == 0 ? p0 : kind == 1 ? n0 + p1 : n0 + n1 + static_cast<uint32_t>(r) - p0 - p1;
+    if (kind < 3 && place == static_cast<uint32_t>(at)) s.row = r;
+  }
+  __syncthreads();
+  const int row = s.row;
+  __syncthreads();                                                          // (the count lies over what is cleared next)
+  for (int i = tid; i < 2 * kGroups; i += B) count[i] = 0u;
+  return row;
+}
+
 __host__ __device__ inline size_t cluster_smem_head() { return (sizeof(ClusterSmem) + 127) & ~static_cast<size_t>(127); }
 
 // CACHED: the slices of the row fit the blocks' shared memory.
 template <bool F32, bool CACHED, int B, int kPerSM>
-__global__ void __launch_bounds__(B, kPerSM) sample_cluster_kernel(const __grid_constant__ SampleDev P, int C) {
+__global__ void __launch_bounds__(B, kPerSM) sample_cluster_kernel(const __grid_constant__ SampleDev P, int C, int ordered) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   ClusterSmem& s = *reinterpret_cast<ClusterSmem*>(smem_raw);
   const int tid = threadIdx.x;
-  const int rank = C > 1 ? static_cast<int>(cluster_rank()) : 0, row = C > 1 ? static_cast<int>(blockIdx.x) / C : static_cast<int>(blockIdx.x);
+  const int rank = C > 1 ? static_cast<int>(cluster_rank()) : 0;
+  int row = C > 1 ? static_cast<int>(blockIdx.x) / C : static_cast<int>(blockIdx.x);
+  // what needs no device memory comes first, beside the kernel in front of this one
+  for (int i = tid; i < kCBins; i += B) { s.cnt[i] = 0u; s.lo[0][i] = 0u; s.lo[1][i] = 0u; s.hi[0][i] = 0u; s.hi[1][i] = 0u; }
+  for (int i = tid; i < kCMaxBins; i += B) s.max_cnt[i] = 0u;
+  if (tid < 64) s.exp_tab[tid] = exp2(static_cast<double>(tid) * 0.015625);
+  after_predecessor();
   int rows = P.rows; uint64_t seed = P.seed; uint32_t noise_step = P.step;
   if (P.state) {                                                            // (as apply_step_state)
     StepStateView st{const_cast<uint32_t*>(P.state), P.t_max, P.g};
@@ -1304,6 +1352,7 @@ __global__ void __launch_bounds__(B, kPerSM) sample_cluster_kernel(const __grid_
     rows = active < rows ? active : rows; seed = st.seed(); noise_step = st.step();
   }
   if (row >= rows) return;                                                  // (uniform over the cluster)
+  if (ordered) row = row_in_order<B>(P, rows, row, s);
   const int V = P.vocab;
   const float T = P.temperature ? P.temperature[row] : P.temperature_s;
   const bool pen_on = P.history != nullptr && P.hist_len > 0;
@@ -1332,14 +1381,11 @@ __global__ void __launch_bounds__(B, kPerSM) sample_cluster_kernel(const __grid_
     s.list_n[0] = 0u; s.list_n[1] = 0u;
     s.o_tau = -INFINITY; s.o_token = -1; s.o_weight = 0ull; s.o_status = s.want_stats ? LM_STATUS_GENERIC_PATH : 0u;   // (what such calls have always reported)
   }
-  for (int i = tid; i < kCBins; i += B) { s.cnt[i] = 0u; s.lo[0][i] = 0u; s.lo[1][i] = 0u; s.hi[0][i] = 0u; s.hi[1][i] = 0u; }
-  for (int i = tid; i < kCMaxBins; i += B) s.max_cnt[i] = 0u;
-  if (tid < 64) s.exp_tab[tid] = exp2(static_cast<double>(tid) * 0.015625);
+  {                                                                         // the slice starts its way into L2 (a thread's loads have two chunks in flight)
+    const int lo_b = max(0, 8 * c0 - off) * (F32 ? 4 : 2), hi_b = min(V, 8 * c1 - off) * (F32 ? 4 : 2);
+    for (int l = lo_b + tid * 128; l < hi_b; l += B * 128) prefetch_l2_line(rowp + l);
+  }
   if (pen_on) {
-    {                                                                       // the slice starts its way into L2 while the history is read
-      const int lo_b = max(0, 8 * c0 - off) * (F32 ? 4 : 2), hi_b = min(V, 8 * c1 - off) * (F32 ? 4 : 2);
-      for (int l = lo_b + tid * 128; l < hi_b; l += B * 128) prefetch_l2_line(rowp + l);
-    }
     uint32_t* w = reinterpret_cast<uint32_t*>(pen);
     for (int i = tid; i < (per + 3) / 4; i += B) w[i] = 0u;
     __syncthreads();

@@ -110,8 +110,7 @@ static __global__ void __launch_bounds__(B) slice_local_kernel(SliceDev P) {
   __shared__ uint64_t scratch[32];
   __shared__ uint32_t pick[2];
   __shared__ uint32_t s_n, s_flags, s_ninf;
-  // the merge may be made resident while the slices are at work; it waits for this grid
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  after_predecessor();                                                      // (the merge may be made resident while the slices are at work)
   const int tid = threadIdx.x, slice = blockIdx.x, row = blockIdx.y;
   if (tid == 0) { s_n = 0u; s_flags = 0u; s_ninf = 0xFFFFFFFFu; }
   if (P.state) {
@@ -229,7 +228,7 @@ static __global__ void __launch_bounds__(B) slice_local_kernel(SliceDev P) {
 static __global__ void __launch_bounds__(kVpMaxCandidates, 1) sliced_merge_kernel(VpMergeDev M, SampleDev P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ VpMergeSmem s;
-  asm volatile("griddepcontrol.wait;" ::: "memory");                      // the records are complete behind this
+  after_predecessor();                                                      // the records are complete behind this
   SampleDev Q = P;                                                         // with a StepState: the noise seed, the step and the active rows come from it
   apply_step_state(Q);
   VpMergeDev N = M;

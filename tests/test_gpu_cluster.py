@@ -246,3 +246,49 @@ def test_every_warp_looks_the_thresholds_bin_up_in_the_same_window():
             knobs = dict(temperature=np.full(148, 50.0, np.float32), top_k=np.full(148, 1000, np.int32), top_p=np.full(148, top_p, np.float32), min_p=0.0)
             for _ in range(5):
                 _check(_tensor(z), z, knobs, draw=draw)
+
+
+@pytest.mark.parametrize("rows,vocab", [(48, 49157), (300, 1003), (2048, 515), (2049, 515)])
+def test_more_clusters_than_run_at_once_take_every_row_once(rows, vocab):
+    """Batches of more clusters than the device holds take their rows by kind (no top_k, a large one, the rest, greedy), up to 2048 rows of them: every
+    row's token and threshold are its own, whatever the mixture and the number of rows."""
+    rng = np.random.default_rng(rows)
+    z = (rng.standard_normal((rows, vocab)) * 2.0).astype(np.float32)
+    top_k = rng.choice(np.array([0, 0, 20, 64, 65, 1000, 1025, 2000], np.int32), rows)
+    T = np.where(rng.random(rows) < 0.1, 0.0, rng.uniform(0.3, 1.5, rows)).astype(np.float32)
+    u = rng.random(rows).astype(np.float32)
+    out = torch.full((rows,), -7, dtype=torch.int32, device="cuda")
+    p = lm.SamplingParams(draw="inverse_cdf", temperature=torch.from_numpy(T).cuda(), top_k=torch.from_numpy(top_k).cuda(), top_p=0.9)
+    r = lm.sample(torch.from_numpy(z).cuda(), p, uniforms=torch.from_numpy(u).cuda(), return_tau=True, out=out)
+    tok, tau, _ = oracle.sample_batch(z, temperature=T, top_k=top_k, top_p=0.9, draw="inverse_cdf", uniforms=u, n_threads=8)
+    np.testing.assert_array_equal(out.cpu().numpy(), tok)
+    np.testing.assert_array_equal(r.tau.cpu().numpy(), tau)
+
+
+@pytest.mark.parametrize("rows", [1, 4])
+def test_calls_in_a_row_see_what_the_one_before_them_left(rows):
+    """Calls of few rows are made ready beside the kernel in front of them in the stream and wait for it: each of these looks at logits that the one
+    before it decided."""
+    vocab = 40960
+    g = torch.Generator(device="cuda")
+    g.manual_seed(rows)
+    x = (torch.randn(rows, vocab, generator=g, device="cuda") * 2).to(torch.bfloat16)
+    p = lm.SamplingParams(temperature=0.8, top_p=0.9, seed=3)
+    q = lm.SamplingParams(temperature=0.8, top_k=20, top_p=0.9, seed=3)
+
+    def run(wait):
+        y, found = x.clone(), []
+        for step in range(24):
+            greedy = lm.argmax(y)
+            found.append(greedy.clone())
+            y.scatter_(1, greedy.long()[:, None], -5.0)
+            for params in (p, q):
+                t = lm.sample(y, params, step=step).tokens
+                found.append(t.clone())
+                y.scatter_(1, t.long()[:, None], -4.0)
+                found.append(lm.sample(y, params, step=step).tokens)
+            if wait:
+                torch.cuda.synchronize()
+        return torch.stack([f.long() for f in found])
+
+    assert torch.equal(run(False), run(True))
