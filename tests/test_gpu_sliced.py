@@ -3,6 +3,10 @@
 The reference's sampler dispatches run on the T <= 8 rows of one decode step (monolith/kernels.py:720-775); its own CPU-runnable
 configuration is a single FP32 row. The results must be the ones of the row-per-block kernels and of the oracle, bit for bit.
 """
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
@@ -214,3 +218,12 @@ def test_thresholds_at_very_small_temperatures(dtype):
     host[1, 77] = oracle.f32_to_bf16(np.array([1e10], np.float32))[0] if dtype == "bf16" else np.float32(1e10)
     for t in (0.8, 1e-9):
         _check(x, host, draw="inverse_cdf", temperature=float(np.float32(t)), top_k=20, top_p=0.95)
+
+
+def test_the_first_call_of_a_process_may_need_just_under_48_kb_a_slice():
+    """A slice of 700,000 / 64 logits and the kernel's static arrays are more shared memory than a kernel has without being told."""
+    code = ("import torch, lithos_metal_b200 as lm\n"
+            "x = torch.randn(2, 700000, device='cuda', generator=torch.Generator('cuda').manual_seed(1)).to(torch.bfloat16)\n"
+            "p = lm.SamplingParams(temperature=0.9, top_k=1, seed=3)\n"
+            "assert lm.sample(x, p).tokens.tolist() == lm.argmax(x).tolist()\n")
+    subprocess.run([sys.executable, "-c", code], check=True, timeout=300, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
