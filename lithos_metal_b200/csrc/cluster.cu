@@ -19,13 +19,15 @@ static int cluster_blocks(int64_t rows, int64_t vocab, int slots) {
 // fifteen of 8 and thirty-two of 4 at once, and one row more waits for a second round (16 rows of 151,936, top_k 20: 41 us with 8 blocks
 // each, 29 us with 4). Beyond that the blocks share SMs, and a row without a top_k takes several times as long as one with: smaller pieces
 // even that out where the slices stay long (binary32 rows with mixed knobs, us with 1 / 2 / 4 blocks: 96 rows of 151,936 198 / 184 / 126,
-// 96 of 65,536 96 / 78 / 87, 400 of 50,257 193 / 175 / 280, 400 of 24,576 119 / 136 / 243). `listed`: every row has a top_k and a short list.
+// 96 of 65,536 96 / 78 / 87, 400 of 50,257 193 / 175 / 280, 400 of 24,576 119 / 136 / 243). `listed`: every row has a top_k and a short list
+// (BF16, top_k 50, us with 2 / 4 blocks: 64 rows of 151,936 27 / 36, of 262,144 39 / 37, 74 of those 40 / 58).
 static int sample_blocks(int64_t rows, int64_t vocab, int sms, bool listed) {
   int c = 1;
   if (rows * 20 <= sms) c = 16;
   else if (rows * 48 <= 5LL * sms) c = 8;
   else if (rows * 9 <= 2LL * sms) c = 4;
   else if (!listed && rows <= 2LL * sms && vocab >= (rows * 3 <= sms ? 49152 : 98304)) c = 4;
+  else if (listed && rows * 16 <= 7LL * sms && vocab >= 196608) c = 4;
   else if (rows * 2 <= sms) c = 2;
   else if (listed ? rows <= 2LL * sms && vocab >= 65536 : rows * 3 <= 2LL * sms || (rows <= 3LL * sms && vocab >= 40000)) c = 2;
   while (c > 1 && vocab < 2048LL * c) c >>= 1;
@@ -34,7 +36,7 @@ static int sample_blocks(int64_t rows, int64_t vocab, int sms, bool listed) {
 
 // The instances of the sampler: FP32 / BF16 rows, the slices cached in shared memory or not, and then one block per SM or two.
 constexpr size_t kMostSmem = 227 * 1024, kHalfSmem = kMostSmem / 2 - 1024;
-struct ClusterPlan { int C; size_t smem; bool cached, two, ordered; };
+struct ClusterPlan { int C; size_t smem; bool cached, two, ordered, few; };
 
 template <bool F32, bool CACHED, int kPerSM>
 static int cluster_ready(int instance, int C, bool* fits) {
@@ -54,10 +56,10 @@ static int cluster_ready(bool f32, const ClusterPlan& p, bool* fits) {
 template <bool F32, bool CACHED, int kPerSM>
 static int launch_cluster(const SampleDev& P, const ClusterPlan& p, cudaStream_t st) {
   return launch_beside(sample_cluster_kernel<F32, CACHED, kClusterBlock, kPerSM>, dim3(static_cast<unsigned>(P.rows) * static_cast<unsigned>(p.C)), kClusterBlock,
-                       p.smem, p.C, st, P, p.C, p.ordered ? 1 : 0);
+                       p.smem, p.C, st, P, p.C, (p.ordered ? kCallOrdered : 0u) | (p.few ? kCallFew : 0u));
 }
 
-int sample_clusters(const SampleDev& P, int sms, cudaStream_t st) {
+int sample_clusters(const SampleDev& P, int sms, cudaStream_t st, bool few) {
   const bool pen = P.history != nullptr && P.hist_len > 0, f32 = P.dtype == LM_DTYPE_F32;
   const size_t head = cluster_smem_head();
   const size_t generic = sizeof(GenericSmem) + (pen ? static_cast<size_t>((P.vocab + 31) / 32) * 4 : 0) + 16;
@@ -65,7 +67,7 @@ int sample_clusters(const SampleDev& P, int sms, cudaStream_t st) {
     const size_t per = (static_cast<size_t>((P.vocab + 14) / 8) + C - 1) / C;    // chunks of a slice, for any alignment of the row
     const size_t marks = pen ? (per + 15) / 16 * 16 : 0;
     ClusterPlan p;
-    p.C = C;
+    p.C = C; p.few = few;
     p.cached = head + per * 32 + marks <= kMostSmem && C > 1;              // (a block per row reads its row from L2: two of them share an SM)
     p.smem = head + (p.cached ? per * 32 : 0) + marks;
     if (p.smem < generic) p.smem = generic;

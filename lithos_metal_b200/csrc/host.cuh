@@ -118,7 +118,7 @@ inline size_t align256(size_t x) { return (x + 255) & ~static_cast<size_t>(255);
 struct SampleDev;
 struct DraftQDev;
 // cluster.cu: one row per thread-block cluster, every row of the call.
-int sample_clusters(const SampleDev& P, int sms, cudaStream_t st);
+int sample_clusters(const SampleDev& P, int sms, cudaStream_t st, bool few = false);   // few: the rows report LM_STATUS_SLICED_PATH
 int argmax_clusters(const void* logits, int dtype, int rows, int vocab, int64_t row_stride, int32_t* out32, int64_t* out64, cudaStream_t st);
 int draft_q_clusters(const DraftQDev& P, int sms, cudaStream_t st);
 

@@ -178,8 +178,13 @@ int lm_sample(const lm_sample_args* a) {
                       a->workspace != nullptr && (reinterpret_cast<uintptr_t>(a->workspace) & 255u) == 0 && a->workspace_bytes >= ws_base + kSlicedWsBytes;
   if (sliced) {
     SliceDev S;
-    // a record holds twice the top_k (16 at least): only a slice with that many logits at or above its own bound overflows it
+    // As many slices as there are SMs for, so that each has a block of 1024 threads to itself: 64, 32 or 16 to a row (8 rows of 151,936, top_k 50:
+    // 20.5 us with 64 slices of 128 threads, 16.0 so; 4 rows 18.5 and 14.6). More rows than that go to clusters of 4 to 16 blocks, in one launch
+    // (12 rows 24.7 / 17.4 us, 16 of 262,144 30.1 / 25.1, 32 of 32,768 30.8 / 15.8; at 9 rows the two are even).
     S.slices = kSlices;
+    while (S.slices > 16 && static_cast<long long>(S.slices) * a->rows > sms && a->vocab <= static_cast<int64_t>(S.slices / 2) * (kSliceMaxLen - 8)) S.slices >>= 1;
+    if (static_cast<long long>(S.slices) * a->rows > sms) return sample_clusters(P, sms, st, true);
+    // a record holds twice the top_k (16 at least): only a slice with that many logits at or above its own bound overflows it
     S.cap = a->top_k_s <= 8 ? 16 : 2 * a->top_k_s;
     S.slice_len = static_cast<int>(((a->vocab + S.slices - 1) / S.slices + 7) / 8 * 8);
     if (S.slice_len <= kSliceMaxLen) {
@@ -193,20 +198,10 @@ int lm_sample(const lm_sample_args* a) {
       const size_t gsmem = sizeof(GenericSmem) + (pen ? static_cast<size_t>((a->vocab + 31) / 32) * 4 : 0) + 16;   // a row handed on to the generic algorithm
       S.need_mass = (a->top_p != nullptr || (a->top_p_s > 0.0f && a->top_p_s < 1.0f)) && !(a->flags & LM_FLAG_TOPP_IN_TOPK);
       const size_t slice_smem = slice_smem_bytes(S.slice_len);
-      // threads per slice: 1024 when every slice has an SM to itself (the latency of one or two rows), else 128 (or 256 for a large
-      // top_k, whose bound needs more threads' maxima to stay close): with several slices per SM the launch is bound by instruction
-      // issue, and the per-warp work of the selection is most of a slice's instructions
-      const int threads = static_cast<long long>(S.slices) * P.rows <= sms ? kSliceBlockBig : (a->top_k_s <= kSliceTinyMaxK ? kSliceBlockTiny : kSliceBlockSmall);
-      const void* slice_fn = threads == kSliceBlockBig ? reinterpret_cast<const void*>(slice_local_kernel<kSliceBlockBig>)
-                           : threads == kSliceBlockSmall ? reinterpret_cast<const void*>(slice_local_kernel<kSliceBlockSmall>)
-                                                         : reinterpret_cast<const void*>(slice_local_kernel<kSliceBlockTiny>);
-      rc = ensure_dynamic_smem(threads == kSliceBlockBig ? kSlotSlice : (threads == kSliceBlockSmall ? kSlotSliceSmall : kSlotSliceTiny), slice_fn, slice_smem);
+      rc = ensure_dynamic_smem(kSlotSlice, reinterpret_cast<const void*>(slice_local_kernel<kSliceBlockBig>), slice_smem);
       if (rc == LM_OK) rc = ensure_dynamic_smem(kSlotSlicedMerge, reinterpret_cast<const void*>(sliced_merge_kernel), gsmem);
       if (rc != LM_OK) return rc;
-      const dim3 slice_grid(static_cast<unsigned>(S.slices), static_cast<unsigned>(P.rows));
-      rc = threads == kSliceBlockBig ? launch_beside(slice_local_kernel<kSliceBlockBig>, slice_grid, kSliceBlockBig, slice_smem, 1, st, S)
-         : threads == kSliceBlockSmall ? launch_beside(slice_local_kernel<kSliceBlockSmall>, slice_grid, kSliceBlockSmall, slice_smem, 1, st, S)
-                                       : launch_beside(slice_local_kernel<kSliceBlockTiny>, slice_grid, kSliceBlockTiny, slice_smem, 1, st, S);
+      rc = launch_beside(slice_local_kernel<kSliceBlockBig>, dim3(static_cast<unsigned>(S.slices), static_cast<unsigned>(P.rows)), kSliceBlockBig, slice_smem, 1, st, S);
       if (rc != LM_OK) return rc;
       VpMergeDev M;
       M.bases = nullptr; M.pieces = 1;
@@ -217,7 +212,7 @@ int lm_sample(const lm_sample_args* a) {
       M.out_tokens = a->out_tokens; M.out_tau = a->out_tau; M.out_status = a->out_status; M.out_vmax = a->out_vmax; M.out_mass = reinterpret_cast<unsigned long long*>(a->out_mass);
       M.hand_on = 1; M.path_status = LM_STATUS_SLICED_PATH;
       merge_geometry(M);
-      M.mass_band = S.need_mass ? slice_mass_band(S.slice_len, threads) : 0.0;
+      M.mass_band = S.need_mass ? slice_mass_band(S.slice_len, kSliceBlockBig) : 0.0;
       // (the merge's blocks are resident and waiting when the slices complete)
       return launch_beside(sliced_merge_kernel, dim3(static_cast<unsigned>(P.rows)), kVpMaxCandidates, gsmem, 1, st, M, P);
     }
@@ -231,10 +226,11 @@ int lm_sample(const lm_sample_args* a) {
   // small to fill the GPU with a block per row: up to SMs / 4 rows of any length, and up to SMs / 2 while the rows are short -- the line lies
   // lower for rows that all lack a top_k, which the histogram kernel does faster from there on (60 rows, streaming / cluster, us: mixed knobs
   // 32,768 74 / 64, 65,536 78 / 55, 151,936 96 / 118; top_k 50 32,768 37 / 22, 65,536 39 / 27; none 32,768 39 / 33, 65,536 45 / 61). With one
-  // top_k for all, short rows stay there up to a row per SM (148 rows of 32,768: 46 / 27). A call that limits its blocks stays below.
+  // top_k for all, rows of any length stay there while two blocks to a row fill the GPU (64 rows of 262,144, top_k 50 42 / 37, top_k 1000 92 / 53; 74 of
+  // 151,936 36 / 28 and 70 / 45; 100 of them 37 / 40), short rows up to a row per SM (148 rows of 32,768: 46 / 27). A call that limits its blocks stays below.
   const bool exact = (a->flags & LM_FLAG_EXACT_ONLY) != 0;
   const bool one_k = a->top_k == nullptr && a->top_k_s >= 1 && a->top_k_s <= kTopkMaxK;
-  const bool small_batch = a->rows * 4 <= sms || (!exact && a->rows * 2 <= sms && a->vocab <= (a->top_k != nullptr || one_k ? 65536 : 40000)) ||
+  const bool small_batch = a->rows * 4 <= sms || (!exact && one_k && a->rows * 2 <= sms) || (!exact && a->rows * 2 <= sms && a->vocab <= (a->top_k != nullptr || one_k ? 65536 : 40000)) ||
                            (!exact && one_k && a->rows <= sms && a->vocab <= 40000);
   if (limit == 0 && a->vocab > 0 && (!fast || small_batch) && (!pen || a->hist_len <= 65536) && a->rows <= 0x7FFFFFFF / 16)
     return sample_clusters(P, sms, st);

@@ -45,6 +45,7 @@ constexpr int kCGroups = 4096;           // group maxima per block
 constexpr int kCMaxBins = 512;           // bins of the group maxima
 constexpr int kCMaxRanks = 16;           // blocks of one cluster
 constexpr int kCQueue = 128;             // logits a warp's queue of the Gumbel draw holds
+constexpr uint32_t kCallOrdered = 1u, kCallFew = 2u;   // of a launch: the rows are taken by kind; the rows report LM_STATUS_SLICED_PATH
 constexpr int kOrderRows = 2048;         // rows whose order a block looks up (row_in_order)
 constexpr int kCRankOrder = 320;         // a list up to this long is ordered by counting larger keys, a longer one by bins first
 constexpr double kCMassBand = 1e-11;     // relative error of a logit's fixed-point softmass beyond its rounding: 7e-12 of the polynomial, a few 1e-16
@@ -90,7 +91,7 @@ struct ClusterSmem {
   ClusterRow R;
   uint64_t seed; uint32_t step;
   double inv_t; float T, top_p, min_p, c2, vmax, vmin, gmin, scale; int top_k, arg, row, rank, C, window, every, per;
-  uint32_t draw, flags; bool has_k, has_p, has_m, in_topk, inverse, want_w, want_stats, fallback;
+  uint32_t draw, flags; bool few, has_k, has_p, has_m, in_topk, inverse, want_w, want_stats, fallback;
   uint32_t t_id; float u;
   // results
   float o_tau; int o_token; uint32_t o_status; uint64_t o_weight;
@@ -1033,7 +1034,7 @@ static __device__ __noinline__ bool phase_top_k(ClusterSmem& s, const SampleDev&
     VpMergeDev M;
     M.flags = s.flags; M.draw = P.draw; M.uniforms = P.uniforms; M.seed = s.seed; M.step = s.step; M.row_offset = P.row_offset;
     M.out_tokens = s.rank == 0 ? P.out_tokens : nullptr; M.out_tau = P.out_tau; M.out_status = P.out_status; M.out_vmax = P.out_vmax; M.out_mass = P.out_mass;
-    M.hand_on = 1; M.path_status = whole && !need_z ? 0u : LM_STATUS_CANDIDATE_PATH;
+    M.hand_on = 1; M.path_status = s.few ? LM_STATUS_SLICED_PATH : whole && !need_z ? 0u : LM_STATUS_CANDIDATE_PATH;
     *written = true;
 #pragma unroll 1
     for (int pass = 0; pass < 2; pass++) {
@@ -1047,13 +1048,13 @@ static __device__ __noinline__ bool phase_top_k(ClusterSmem& s, const SampleDev&
       if (!s.amb) break;
       total = phase_mass64<F32, CACHED>(s, -INFINITY, s.x_mass64);          // too close to call in FP32: the row's mass again, in FP64
       err = 0.0;
-      M.path_status = 0u;
+      if (!s.few) M.path_status = 0u;
     }
     return true;
   }
   // thresholds
   double tau64 = tau_k;
-  uint32_t status = s.want_stats || (whole && !need_z) ? 0u : LM_STATUS_CANDIDATE_PATH;
+  uint32_t status = s.want_stats || s.few || (whole && !need_z) ? 0u : LM_STATUS_CANDIDATE_PATH;
   if (s.has_p) {
     for (int i = tid; i < n_topk; i += B) s.cum[i] = exp64((static_cast<double>(list_value(s, i)) - static_cast<double>(vmax)) * s.inv_t, s.exp_tab);
     __syncthreads();
@@ -1334,7 +1335,7 @@ __host__ __device__ inline size_t cluster_smem_head() { return (sizeof(ClusterSm
 
 // CACHED: the slices of the row fit the blocks' shared memory.
 template <bool F32, bool CACHED, int B, int kPerSM>
-__global__ void __launch_bounds__(B, kPerSM) sample_cluster_kernel(const __grid_constant__ SampleDev P, int C, int ordered) {
+__global__ void __launch_bounds__(B, kPerSM) sample_cluster_kernel(const __grid_constant__ SampleDev P, int C, uint32_t call) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   ClusterSmem& s = *reinterpret_cast<ClusterSmem*>(smem_raw);
   const int tid = threadIdx.x;
@@ -1352,7 +1353,7 @@ __global__ void __launch_bounds__(B, kPerSM) sample_cluster_kernel(const __grid_
     rows = active < rows ? active : rows; seed = st.seed(); noise_step = st.step();
   }
   if (row >= rows) return;                                                  // (uniform over the cluster)
-  if (ordered) row = row_in_order<B>(P, rows, row, s);
+  if (call & kCallOrdered) row = row_in_order<B>(P, rows, row, s);
   const int V = P.vocab;
   const float T = P.temperature ? P.temperature[row] : P.temperature_s;
   const bool pen_on = P.history != nullptr && P.hist_len > 0;
@@ -1379,7 +1380,8 @@ __global__ void __launch_bounds__(B, kPerSM) sample_cluster_kernel(const __grid_
     const int n_it = (c1 - c0 + B - 1) / B;
     s.every = max(1, (n_it * B + kCGroups - 1) / kCGroups);
     s.list_n[0] = 0u; s.list_n[1] = 0u;
-    s.o_tau = -INFINITY; s.o_token = -1; s.o_weight = 0ull; s.o_status = s.want_stats ? LM_STATUS_GENERIC_PATH : 0u;   // (what such calls have always reported)
+    s.o_tau = -INFINITY; s.o_token = -1; s.o_weight = 0ull; s.few = (call & kCallFew) != 0u;
+    s.o_status = (s.want_stats ? LM_STATUS_GENERIC_PATH : 0u) | (s.few ? LM_STATUS_SLICED_PATH : 0u);   // (what such calls have always reported)
   }
   {                                                                         // the slice starts its way into L2 (a thread's loads have two chunks in flight)
     const int lo_b = max(0, 8 * c0 - off) * (F32 ? 4 : 2), hi_b = min(V, 8 * c1 - off) * (F32 ? 4 : 2);

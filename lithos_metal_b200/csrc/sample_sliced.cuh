@@ -4,7 +4,7 @@
 // one block walking 150k logits several times. The decode step of a single stream is exactly that call (the reference's sampler
 // dispatches run on T <= 8 rows per step, monolith/kernels.py:720-775). Here the slices of a row go to different SMs:
 //
-//   slice_local_kernel  (64 slices x rows blocks)  reads its slice ONCE into shared memory (BF16 or FP32, widened; the penalties of
+//   slice_local_kernel  (16 to 64 slices x rows blocks)  reads its slice ONCE into shared memory (BF16 or FP32, widened; the penalties of
 //                       the history ids that fall into the slice applied), and leaves a record: the slice's maximum, its FP64
 //                       softmass relative to that maximum, and every logit at or above a lower bound of the slice's own k-th
 //                       largest (the k-th largest of the threads' own maxima, to 22 key bits);
@@ -23,14 +23,14 @@
 
 namespace lm {
 
-constexpr int kSliceBlockBig = 1024;     // threads per slice when every slice has an SM to itself (latency), else kSliceBlockSmall
+constexpr int kSliceBlockBig = 1024;     // threads per slice when every slice has an SM to itself (latency); else (vocab-parallel pieces) kSliceBlockSmall
 constexpr int kSliceBlockSmall = 256;   // ... and kSliceBlockTiny when the top_k leaves its record room (fewer warps: fewer instructions per slice)
 constexpr int kSliceBlockTiny = 128;
 constexpr int kSliceTinyMaxK = 50;        // largest top_k for kSliceBlockTiny: about 62 of a record's 100 slots filled then
 constexpr int kSliceMaxLen = 32768;       // logits of one slice (128 KB of shared memory as binary32)
 constexpr int kSlicedMaxRows = 32;        // rows per call on this path
 constexpr int kSlicedMinVocab = 16384;
-constexpr int kSlices = 64;               // slices per row
+constexpr int kSlices = 64;               // slices per row at most
 constexpr int kSliceMaxCap = 128;         // candidates in one slice's record: twice the largest top_k
 constexpr size_t kSlicedWsBytes = static_cast<size_t>(kSlicedMaxRows) * kSlices * (kVpHeader + 8 * kSliceMaxCap);
 

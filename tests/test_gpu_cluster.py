@@ -292,3 +292,19 @@ def test_calls_in_a_row_see_what_the_one_before_them_left(rows):
         return torch.stack([f.long() for f in found])
 
     assert torch.equal(run(False), run(True))
+
+
+@pytest.mark.parametrize("rows,vocab,top_k", [(38, 66001, 50), (64, 262144, 50), (65, 262144, 1000), (74, 151936, 1)])
+def test_one_top_k_for_all_rows_of_half_the_gpu(rows, vocab, top_k):
+    """BF16 batches of up to half a row per SM with one top_k: two or four blocks to a row, whatever its length."""
+    rng = np.random.default_rng(vocab)
+    host = oracle.f32_to_bf16((rng.standard_normal((rows, vocab)) * 2).astype(np.float32))
+    knobs = dict(temperature=np.float32(0.8), top_k=top_k, top_p=np.float32(0.9), min_p=np.float32(0.0))
+    u = rng.random(rows).astype(np.float32)
+    for draw in ("inverse_cdf", "gumbel"):
+        p = lm.SamplingParams(draw=draw, seed=5, **{k: v if k == "top_k" else float(v) for k, v in knobs.items()})
+        r = lm.sample(_tensor(host), p, uniforms=torch.from_numpy(u).cuda(), return_tau=True, return_status=True)
+        tok, tau, _ = oracle.sample_batch(host, draw=draw, seed=5, uniforms=u, n_threads=8, **knobs)
+        near = r.status.cpu().numpy() & 4
+        np.testing.assert_array_equal(r.tau.cpu().numpy(), tau)
+        assert np.all((r.tokens.cpu().numpy() == tok) | (near != 0))

@@ -220,6 +220,38 @@ def test_thresholds_at_very_small_temperatures(dtype):
         _check(x, host, draw="inverse_cdf", temperature=float(np.float32(t)), top_k=20, top_p=0.95)
 
 
+@pytest.mark.parametrize("rows,vocab,top_k,dtype", [(3, 16384, 20, "bf16"), (4, 151936, 64, "f32"), (5, 151937, 20, "f32"), (9, 151936, 50, "bf16"), (10, 151936, 50, "bf16"),
+                                                    (10, 16384, 1, "f32"), (18, 50257, 64, "f32"), (32, 262144, 33, "bf16"), (9, 600000, 20, "bf16"), (5, 1000000, 20, "bf16")])
+def test_slices_to_a_row_by_how_many_rows_there_are(rows, vocab, top_k, dtype):
+    """64, 32 or 16 slices to a row while each has an SM, then a cluster of blocks per row: the same tokens and thresholds, reported the same way."""
+    x, host = _rows(rows, vocab, rows, dtype)
+    for draw in ("inverse_cdf", "gumbel"):
+        _check(x, host, draw=draw, temperature=0.8, top_k=top_k, top_p=0.95, min_p=0.001)
+    rng = np.random.default_rng(rows)
+    hist = rng.integers(0, vocab, (rows, 300)).astype(np.int32)
+    _check(x, host, draw="inverse_cdf", temperature=1.2, top_k=top_k, history=hist, rho=1.2, pi=0.3)
+
+
+@pytest.mark.parametrize("rows", [8, 12])
+def test_runs_of_equal_logits_and_masks_in_a_few_rows(rows):
+    """More equal logits than a record, or a list, holds; a vocabulary masked but for a few logits: whoever decides such a row, it is the oracle's."""
+    vocab = 65536
+    rng = np.random.default_rng(5)
+    z = (rng.standard_normal((rows, vocab)) * 2).astype(np.float32)
+    z[0, ::7] = 9.0
+    z[1, 1000:1500] = 9.0
+    z[2, 30:] = -np.inf
+    z[3, 100:] = -1e9
+    z[4] = 1.5
+    codes = oracle.f32_to_bf16(z)
+    u = np.linspace(0.03, 0.97, rows).astype(np.float32)
+    p = lm.SamplingParams(temperature=0.8, top_k=50, top_p=0.9, draw="inverse_cdf")
+    r = lm.sample(torch.from_numpy(codes.view(np.int16)).cuda().view(torch.bfloat16), p, uniforms=torch.from_numpy(u).cuda(), return_tau=True, return_status=True)
+    tok, tau, _ = oracle.sample_batch(codes, temperature=0.8, top_k=50, top_p=0.9, draw="inverse_cdf", uniforms=u, n_threads=8)
+    assert r.tokens.cpu().tolist() == tok.tolist() and r.tau.cpu().tolist() == tau.tolist()
+    assert np.all(r.status.cpu().numpy() & (SLICED | GENERIC))
+
+
 def test_the_first_call_of_a_process_may_need_just_under_48_kb_a_slice():
     """A slice of 700,000 / 64 logits and the kernel's static arrays are more shared memory than a kernel has without being told."""
     code = ("import torch, lithos_metal_b200 as lm\n"
