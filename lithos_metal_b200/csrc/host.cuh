@@ -89,28 +89,33 @@ inline bool cluster_fits(KernelSlot slot, const void* func, int threads, size_t 
   return n > 0;
 }
 
-// A launch in clusters of C blocks that may begin while the kernel in front of it in the stream is still at work (programmatic stream
-// serialization): its blocks are made ready, set up what needs no device memory, and wait (after_predecessor, common.cuh). Only a grid of no more
+// A launch in clusters of C blocks; beside: it may begin while the kernel in front of it in the stream is still at work (programmatic stream
+// serialization): its blocks are made ready, set up what needs no device memory, and wait (after_predecessor, common.cuh).
+template <class... K, class... A>
+inline int launch_stream(bool beside, void (*kernel)(K...), dim3 grid, int threads, size_t smem, int C, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = dim3(static_cast<unsigned>(threads)); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = beside ? 1 : 0;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = static_cast<unsigned>(C); attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = C > 1 ? 2 : 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...);
+  return e == cudaSuccess ? LM_OK : cuda_fail(e);
+}
+
+// ... of a call of few rows, beside its predecessor: only a grid of no more
 // blocks than SMs, or of blocks that need an SM each: placed while others are at work, many small blocks pile up on the SMs that happen to be
 // free (a speculative round's 512 slices: the round 49.2 us so, 45.2 behind the predecessor's end). Calls in a row, us per call so / behind the predecessor's end: greedy,
 // one row 5.9 / 6.2; 4 nucleus rows 32.3 / 33.5; probabilities of 4 rows 21.8 / 23.2; one FP32 row with a top_k 13.5 / 14.5; 64 FP32 rows
 // with mixed knobs 72.9 / 74.8.
 template <class... K, class... A>
 inline int launch_beside(void (*kernel)(K...), dim3 grid, int threads, size_t smem, int C, cudaStream_t st, A... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid; cfg.blockDim = dim3(static_cast<unsigned>(threads)); cfg.dynamicSmemBytes = smem; cfg.stream = st;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = static_cast<unsigned>(C); attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
   int sms = 0;
   const int rc = sm_count(&sms);
   if (rc != LM_OK) return rc;
-  if (static_cast<long long>(grid.x) * grid.y > sms && smem < 114 * 1024) attr[0].val.programmaticStreamSerializationAllowed = 0;
-  cfg.attrs = attr; cfg.numAttrs = C > 1 ? 2 : 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...);
-  return e == cudaSuccess ? LM_OK : cuda_fail(e);
+  return launch_stream(static_cast<long long>(grid.x) * grid.y <= sms || smem >= 114 * 1024, kernel, grid, threads, smem, C, st, args...);
 }
 
 inline size_t align256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }

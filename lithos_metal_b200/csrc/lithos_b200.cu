@@ -28,6 +28,7 @@ __global__ void __launch_bounds__(kBlock, 1) sample_generic_kernel(SampleDev P, 
   extern __shared__ __align__(16) unsigned char smem_raw[];
   GenericSmem& s = *reinterpret_cast<GenericSmem*>(smem_raw);
   uint32_t* pen_bits = reinterpret_cast<uint32_t*>(smem_raw + sizeof(GenericSmem));
+  after_predecessor();
   apply_step_state(P);
   const int n = list ? min(*n_list, P.rows) : P.rows;
   for (int i = blockIdx.x; i < n; i += gridDim.x) {
@@ -249,70 +250,55 @@ int lm_sample(const lm_sample_args* a) {
     if (rc != LM_OK) return rc;
     const bool topk = !(a->flags & LM_FLAG_EXACT_ONLY) && a->vocab >= kTopkMinVocab && (a->top_k != nullptr || (a->top_k_s >= 1 && a->top_k_s <= kTopkMaxK)) &&
                       (a->temperature != nullptr || a->temperature_s > 0.0f) && (!pen || a->hist_len <= kTopkHist);
-    {
-      const cudaError_t e = cudaMemsetAsync(counters, 0, 8 * sizeof(int), st);
-      if (e != cudaSuccess) return cuda_fail(e);
-    }
     const long long hist_per_sm = 2 * (hist_smem + 1024) <= 233472 ? 2 : 1;   // blocks of the histogram kernel that fit one SM's shared memory
     int grid = static_cast<int>(a->rows < hist_per_sm * sms ? a->rows : hist_per_sm * sms);
     if (limit > 0 && grid > limit) grid = limit;
     int grid1 = static_cast<int>(a->rows < static_cast<long long>(kTopkPerSM) * sms ? a->rows : static_cast<long long>(kTopkPerSM) * sms);
     if (limit > 0 && grid1 > limit) grid1 = limit;
-    int grid_list = static_cast<int>((a->rows + 255) / 256);
-    if (limit > 0 && grid_list > limit) grid_list = limit;
-    const unsigned overlap = limit > 0 ? 0u : 1u;                          // (launch attributes: two grids at once would be more blocks than the call was allowed)
+    const bool beside = limit == 0;                                        // (two grids at once would be more blocks than the call was allowed)
+    const int* none = nullptr; int* none_mut = nullptr;
     if (!topk) {
-      sample_hist_kernel<<<grid, kHB, hist_smem, st>>>(P, nullptr, nullptr, counters + 2, redo, counters + 3, nullptr, nullptr, nullptr);
-    } else if (one_k || a->rows > static_cast<int64_t>(kOverlapRowsPerSM) * sms) {
-      // Many rows per SM, or hardly a row for the histogram kernel (one top_k for all: 148 rows 56 us side by side, 43 so): the top-k kernel first,
-      // the histogram kernel behind it with programmatic stream serialization: its blocks take an SM over as the top-k blocks leave it, work
-      // through the rows that a one-thread-per-row kernel has listed for it, wait for the top-k grid, and absorb the few rows that one handed
-      // on. (4096 penalised rows 720 us, behind its end 771; 800 rows 186 and 210.)
-      sample_classify_kernel<<<grid_list, 256, 0, st>>>(P, list_other, counters + 4);
-      sample_topk_kernel<<<grid1, kTB, sizeof(TopkSmem), st>>>(P, list_left, counters);
-      cudaError_t e = cudaGetLastError();
+      const cudaError_t e = cudaMemsetAsync(counters, 0, kCounters * sizeof(int), st);
       if (e != cudaSuccess) return cuda_fail(e);
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(grid); cfg.blockDim = dim3(kHB); cfg.dynamicSmemBytes = hist_smem; cfg.stream = st;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-      attr[0].val.programmaticStreamSerializationAllowed = 1;
-      cfg.attrs = attr; cfg.numAttrs = overlap;
-      e = cudaLaunchKernelEx(&cfg, sample_hist_kernel, P, static_cast<const int*>(list_other), static_cast<const int*>(counters + 4), counters + 2, redo, counters + 3,
-                             static_cast<const int*>(list_left), static_cast<const int*>(counters + 1), counters + 5);
-      if (e != cudaSuccess) return cuda_fail(e);
+      rc = launch_stream(false, sample_hist_kernel, grid, kHB, hist_smem, 1, st, P, none, none, counters + 2, redo, counters + 3, none, none, none_mut);
+      if (rc != LM_OK) return rc;
     } else {
-      // Few rows per SM: the length of a launch is the length of its longest rows, so the two kernels, which work on different
-      // rows, share the GPU. The histogram kernel (long rows, one block per SM) goes first on the rows a one-thread-per-row
-      // kernel lists for it; the top-k kernel is launched behind it with programmatic stream serialization and takes the SMs
-      // as the histogram kernel's blocks leave them (at once, for the SMs it has no rows for); a second launch of the histogram
-      // kernel takes what the top-k kernel handed on (usually nothing: it leaves at once).
-      sample_classify_kernel<<<grid_list, 256, 0, st>>>(P, list_other, counters + 4);
-      // With at most kAloneRowsPerSM rows per SM the histogram kernel's blocks ask for so much shared memory that nothing else fits
-      // beside them: a long row then has its SM to itself, and the blocks that find no row leave their SM to the top-k kernel at
-      // once (256 rows of the benchmark mix: 106 us per call, 112 without; from 3 rows per SM on it costs time).
-      size_t hist_smem_first = hist_smem; int grid_first = grid;
-      if (a->rows <= static_cast<int64_t>(kAloneRowsPerSM) * sms && hist_smem < kAloneSmemBytes) {
-        hist_smem_first = kAloneSmemBytes; grid_first = static_cast<int>(a->rows < sms ? a->rows : sms);
-        if (limit > 0 && grid_first > limit) grid_first = limit;
-        rc = ensure_dynamic_smem(kSlotFast, reinterpret_cast<const void*>(sample_hist_kernel), hist_smem_first);
+      // Every launch of the call waits on the device for what it needs of the one in front, so that none of them begins with a gap (us per call so /
+      // with a memset and gaps: 256 penalised rows 92.8 / 102.8, 128 rows of 262,144 with a top_k 37.3 / 42.8, 4096 penalised rows 668 / 674).
+      rc = launch_stream(beside, sample_prep_kernel, 1, kPrepThreads, 0, 1, st, P, list_other, counters);
+      if (rc != LM_OK) return rc;
+      if (one_k || a->rows > static_cast<int64_t>(kOverlapRowsPerSM) * sms) {
+        // Many rows per SM, or hardly a row for the histogram kernel (one top_k for all: 148 rows 56 us side by side, 43 so): the top-k kernel first,
+        // the histogram kernel behind it with programmatic stream serialization: its blocks take an SM over as the top-k blocks leave it, work
+        // through the rows that the preparation has listed for it, wait for the top-k grid, and absorb the few rows that one handed
+        // on. (4096 penalised rows 720 us, behind its end 771; 800 rows 186 and 210.)
+        rc = launch_stream(beside, sample_topk_kernel, grid1, kTB, sizeof(TopkSmem), 1, st, P, list_left, counters, 1);
+        if (rc == LM_OK) rc = launch_stream(beside, sample_hist_kernel, grid, kHB, hist_smem, 1, st, P, list_other, counters + kCounterOther, counters + 2, redo, counters + 3,
+                                            list_left, counters + 1, counters + 5);
+        if (rc != LM_OK) return rc;
+      } else {
+        // Few rows per SM: the length of a launch is the length of its longest rows, so the two kernels, which work on different
+        // rows, share the GPU. The histogram kernel (long rows, one block per SM) goes first on the rows that the preparation has listed
+        // for it; the top-k kernel is launched behind it with programmatic stream serialization and takes the SMs
+        // as the histogram kernel's blocks leave them (at once, for the SMs it has no rows for); a second launch of the histogram
+        // kernel takes what the top-k kernel handed on (usually nothing: it leaves at once).
+        // With at most kAloneRowsPerSM rows per SM the histogram kernel's blocks ask for so much shared memory that nothing else fits
+        // beside them: a long row then has its SM to itself, and the blocks that find no row leave their SM to the top-k kernel at
+        // once (256 rows of the benchmark mix: 106 us per call, 112 without; from 3 rows per SM on it costs time).
+        size_t hist_smem_first = hist_smem; int grid_first = grid;
+        if (a->rows <= static_cast<int64_t>(kAloneRowsPerSM) * sms && hist_smem < kAloneSmemBytes) {
+          hist_smem_first = kAloneSmemBytes; grid_first = static_cast<int>(a->rows < sms ? a->rows : sms);
+          if (limit > 0 && grid_first > limit) grid_first = limit;
+          rc = ensure_dynamic_smem(kSlotFast, reinterpret_cast<const void*>(sample_hist_kernel), hist_smem_first);
+          if (rc != LM_OK) return rc;
+        }
+        rc = launch_stream(beside, sample_hist_kernel, grid_first, kHB, hist_smem_first, 1, st, P, list_other, counters + kCounterOther, counters + 2, redo, counters + 3,
+                           none, none, none_mut);
+        if (rc == LM_OK) rc = launch_stream(beside, sample_topk_kernel, grid1, kTB, sizeof(TopkSmem), 1, st, P, list_left, counters, 0);
+        if (rc == LM_OK) rc = launch_stream(beside, sample_hist_kernel, grid, kHB, hist_smem, 1, st, P, list_left, counters + 1, counters + 5, redo, counters + 3, none, none, none_mut);
         if (rc != LM_OK) return rc;
       }
-      sample_hist_kernel<<<grid_first, kHB, hist_smem_first, st>>>(P, list_other, counters + 4, counters + 2, redo, counters + 3, nullptr, nullptr, nullptr);
-      cudaError_t e = cudaGetLastError();
-      if (e != cudaSuccess) return cuda_fail(e);
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(grid1); cfg.blockDim = dim3(kTB); cfg.dynamicSmemBytes = sizeof(TopkSmem); cfg.stream = st;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-      attr[0].val.programmaticStreamSerializationAllowed = 1;
-      cfg.attrs = attr; cfg.numAttrs = overlap;
-      e = cudaLaunchKernelEx(&cfg, sample_topk_kernel, P, list_left, counters);
-      if (e != cudaSuccess) return cuda_fail(e);
-      sample_hist_kernel<<<grid, kHB, hist_smem, st>>>(P, list_left, counters + 1, counters + 5, redo, counters + 3, nullptr, nullptr, nullptr);
     }
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return cuda_fail(e);
     redo_list = redo; redo_n = counters + 3;
   }
   const size_t smem = sizeof(GenericSmem) + (pen ? static_cast<size_t>((a->vocab + 31) / 32) * 4 : 0) + 16;
@@ -321,9 +307,7 @@ int lm_sample(const lm_sample_args* a) {
   const long long cap = fast ? sms : 8LL * sms;
   int grid = static_cast<int>(a->rows < cap ? a->rows : cap);
   if (limit > 0 && grid > limit) grid = limit;
-  sample_generic_kernel<<<grid, kBlock, smem, st>>>(P, redo_list, redo_n);
-  const cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? LM_OK : cuda_fail(e);
+  return launch_stream(redo_list != nullptr && limit == 0, sample_generic_kernel, grid, kBlock, smem, 1, st, P, redo_list, redo_n);
 }
 
 static size_t tile_lists_offset(int64_t rows) { return align256(static_cast<size_t>(rows) * sizeof(TileRow)); }

@@ -939,8 +939,9 @@ static __global__ void __launch_bounds__(kHB, 2) sample_hist_kernel(SampleDev P,
   uint32_t* pen = reinterpret_cast<uint32_t*>(smem_raw + ((sizeof(HistSmem) + 15) & ~static_cast<size_t>(15)));
   __shared__ int item[2];
   // A kernel launched behind this one with programmatic stream serialization (the top-k kernel, which works on other rows and
-  // reads nothing this kernel writes) may take every SM a block of this grid has left, instead of waiting for the whole grid.
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // reads nothing this kernel writes) may take every SM a block of this grid has left, instead of waiting for the whole grid. This kernel itself
+  // begins when its predecessor is complete, but for the grid that runs beside the top-k kernel and meets its end below.
+  if (left == nullptr) after_predecessor(); else asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   apply_step_state(P);
 #pragma unroll 1
   for (int pass = 0; pass < 2; pass++) {

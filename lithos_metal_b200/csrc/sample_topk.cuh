@@ -120,11 +120,26 @@ __device__ __forceinline__ bool topk_row_eligible(const SampleDev& P, int row) {
          (reinterpret_cast<uintptr_t>(rowp) & 15u) == 0 && !(P.history != nullptr && P.hist_len > kTopkHist);
 }
 
-// The rows that are not the top-k kernel's, listed for the histogram kernel (a thread per row, or per few rows).
-static __global__ void sample_classify_kernel(SampleDev P, int* list, int* n_list) {
+// What the row kernels of a call share in the workspace: the counters begin at zero, the rows that are not the top-k kernel's are listed for the
+// histogram kernel. One block: it clears and counts without a memset of its own in front (2 us of every call).
+constexpr int kPrepThreads = 1024, kCounters = 8, kCounterOther = 4;
+static __global__ void __launch_bounds__(kPrepThreads) sample_prep_kernel(SampleDev P, int* list, int* counters) {
+  __shared__ int n;
+  if (threadIdx.x == 0) n = 0;
+  after_predecessor();
   apply_step_state(P);
-  for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < P.rows; row += gridDim.x * blockDim.x)
-    if (!topk_row_eligible(P, row)) list[atomicAdd(n_list, 1)] = row;
+  __syncthreads();
+  if (threadIdx.x < kCounters && threadIdx.x != kCounterOther) counters[threadIdx.x] = 0;
+  constexpr int kU = 4;                                                     // rows of a thread whose knobs are in flight
+  for (int r0 = threadIdx.x; r0 < P.rows; r0 += kU * kPrepThreads) {
+    bool other[kU];
+#pragma unroll
+    for (int j = 0; j < kU; j++) { const int row = r0 + j * kPrepThreads; other[j] = row < P.rows && !topk_row_eligible(P, row); }
+#pragma unroll
+    for (int j = 0; j < kU; j++) if (other[j]) list[atomicAdd(&n, 1)] = r0 + j * kPrepThreads;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) counters[kCounterOther] = n;
 }
 
 struct TopkSmem;
@@ -668,14 +683,15 @@ static __device__ bool topk_finish(const SampleDev& P, int row, TopkSmem& c, uin
 }
 
 // Rows are handed out through a counter in the workspace (counters[0], zeroed by the host before the launch): a block takes
-// the next row, passes over it if it is not this kernel's (sample_classify_kernel has listed it), and else either finishes it or appends it to
+// the next row, passes over it if it is not this kernel's (sample_prep_kernel has listed it), and else either finishes it or appends it to
 // `list` (length in counters[1]) for the histogram kernel. The order of the list varies from run to run; what is computed per row does not.
-static __global__ void __launch_bounds__(kTB, kTopkPerSM) sample_topk_kernel(SampleDev P, int* list, int* counters) {
+static __global__ void __launch_bounds__(kTB, kTopkPerSM) sample_topk_kernel(SampleDev P, int* list, int* counters, int first) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   TopkSmem& c = *reinterpret_cast<TopkSmem*>(smem_raw);
   __shared__ int item[2];                                                   // the row in hand and the one after it
-  // (a histogram kernel launched behind this one with programmatic stream serialization takes over the SMs as this grid's blocks leave them)
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // A histogram kernel launched behind this one with programmatic stream serialization takes over the SMs as this grid's blocks leave them.
+  // first: this is the call's first kernel behind sample_prep_kernel, whose counters it needs; else a histogram kernel has begun before it.
+  if (first) after_predecessor(); else asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   apply_step_state(P);
   if (threadIdx.x < 8) c.prev_cut[threadIdx.x] = 0u;
   // With many rows per block a block holds the row after its current one too (it pulls that row into L2 while it works) and

@@ -265,24 +265,25 @@ def test_more_clusters_than_run_at_once_take_every_row_once(rows, vocab):
     np.testing.assert_array_equal(r.tau.cpu().numpy(), tau)
 
 
-@pytest.mark.parametrize("rows", [1, 4])
+@pytest.mark.parametrize("rows", [1, 4, 100, 760])
 def test_calls_in_a_row_see_what_the_one_before_them_left(rows):
-    """Calls of few rows are made ready beside the kernel in front of them in the stream and wait for it: each of these looks at logits that the one
-    before it decided."""
+    """Kernels are made ready beside the one in front of them in the stream and wait for it: each of these calls (few rows; streaming kernels with
+    one top_k, none, or the rows' own) looks at logits that the one before it decided."""
     vocab = 40960
     g = torch.Generator(device="cuda")
     g.manual_seed(rows)
     x = (torch.randn(rows, vocab, generator=g, device="cuda") * 2).to(torch.bfloat16)
     p = lm.SamplingParams(temperature=0.8, top_p=0.9, seed=3)
     q = lm.SamplingParams(temperature=0.8, top_k=20, top_p=0.9, seed=3)
+    own = lm.SamplingParams(temperature=0.8, top_k=torch.tensor([0, 20, 700], dtype=torch.int32, device="cuda").repeat(rows // 3 + 1)[:rows].contiguous(), top_p=0.9, seed=3)
 
     def run(wait):
         y, found = x.clone(), []
-        for step in range(24):
+        for step in range(12):
             greedy = lm.argmax(y)
             found.append(greedy.clone())
             y.scatter_(1, greedy.long()[:, None], -5.0)
-            for params in (p, q):
+            for params in (p, q, own):
                 t = lm.sample(y, params, step=step).tokens
                 found.append(t.clone())
                 y.scatter_(1, t.long()[:, None], -4.0)
