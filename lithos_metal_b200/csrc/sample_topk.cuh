@@ -15,6 +15,7 @@
 
 #include "common.cuh"
 #include "sample_generic.cuh"
+#include "vocab_parallel.cuh"
 
 namespace lm {
 
@@ -27,7 +28,9 @@ constexpr int kTopkMaxK = 1024;            // largest top_k this kernel takes
 constexpr int kTopkHist = 2048;            // longest history it takes
 constexpr int kTopkMaxVocab = 1 << 18;
 constexpr int kMaxProbes = 30;             // counters of the cutoff search per row: three per round, one round for the bracket + eight for the whole code range
-constexpr int kBinSortMax = 256;           // a code bin with more candidates than this must already be in order (all equal)
+constexpr int kBinSortMax = 256;           // most candidates of one code bin whose values are no BF16 values (penalised ones)
+constexpr int kFew = 64;                   // this many candidates down to the top-k crossing are finished by one warp
+constexpr uint32_t kRefineFrom = 44u;      // sampled logits wanted from which on the cutoff is corrected by as many samples again
 constexpr int kSampleChunks = 1024 / kTB;   // chunks per thread in the cutoff sample: 1024 chunks = 8192 logits
 constexpr int kTopkMinVocab = 32768;
 
@@ -77,23 +80,21 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void prefetch_l2_line(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
-// Inclusive FP64 prefix sum over v[0 .. n) in place, index order; every thread calls. warp_d: one entry per warp.
+// Inclusive FP64 prefix sum over v[0 .. n) in place, n <= kTopkCap, index order; every thread calls (a thread takes consecutive entries).
 __device__ __forceinline__ void scan_f64(double* v, int n, double* warp_d) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
-  double carry = 0.0;
-  for (int base = 0; base < n; base += blockDim.x) {
-    const int i = base + tid;
-    double x = (i < n) ? v[i] : 0.0;
+  constexpr int kPer = kTopkCap / kTB;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  double x[kPer], sum = 0.0;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) { const double t = __shfl_up_sync(kFull, x, o); if (lane >= o) x += t; }
-    __syncthreads();
-    if (lane == 31) warp_d[warp] = x;
-    __syncthreads();
-    double wsum = 0.0, tot = 0.0;
-    for (int w = 0; w < nw; w++) { if (w < warp) wsum += warp_d[w]; tot += warp_d[w]; }
-    if (i < n) v[i] = carry + wsum + x;
-    carry += tot;
-  }
+  for (int j = 0; j < kPer; j++) { const int i = tid * kPer + j; sum += i < n ? v[i] : 0.0; x[j] = sum; }
+  double incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) { const double t = __shfl_up_sync(kFull, incl, o); if (lane >= o) incl += t; }
+  if (lane == 31) warp_d[warp] = incl;
+  __syncthreads();
+  const double before = warp_sum_f64(lane < warp ? warp_d[lane] : 0.0) + (incl - sum);
+#pragma unroll
+  for (int j = 0; j < kPer; j++) { const int i = tid * kPer + j; if (i < n) v[i] = before + x[j]; }
   __syncthreads();
 }
 
@@ -108,6 +109,15 @@ __device__ __forceinline__ uint32_t warp_reserve(uint32_t* counter, uint32_t min
   if (lane == 0 && total) base = atomicAdd(counter, total);
   base = __shfl_sync(kFull, base, 0);
   return base + incl - mine;
+}
+
+// ... of at most one entry a lane.
+__device__ __forceinline__ uint32_t warp_reserve_one(uint32_t* counter, bool mine) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t votes = __ballot_sync(kFull, mine);
+  uint32_t base = 0u;
+  if (lane == 0 && votes) base = atomicAdd(counter, __popc(votes));
+  return __shfl_sync(kFull, base, 0) + __popc(votes & ((1u << lane) - 1u));
 }
 
 // Whether a row is this kernel's at all, from its knobs and address alone (no look at the logits).
@@ -185,6 +195,14 @@ static __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem&
   uint4 qs[kSampleChunks];
 #pragma unroll
   for (int j = 0; j < kSampleChunks; j++) qs[j] = __ldg(p4 + tid + j * (n_chunks / kSampleChunks));
+  // The sampled logits wanted at or above the cutoff: what the top_k stands for in the sample (lam), and so many more that one row in 10^5 has fewer
+  // than top_k candidates (4.3 standard deviations of a Poisson count, and 6 for the small ones); what stands for 1536 candidates at most.
+  const float lam = static_cast<float>(top_k) * (static_cast<float>(kSampleChunks * kTB * kChunk) / static_cast<float>(V));
+  const uint32_t want = static_cast<uint32_t>(fminf(ceilf(lam + 4.3f * sqrtf(lam) + 6.0f), 1536.0f * (static_cast<float>(kSampleChunks * kTB * kChunk) / static_cast<float>(V))));
+  const bool refine = want >= kRefineFrom;
+  uint4 qr[kSampleChunks];                                                  // as many again, between the others
+#pragma unroll
+  for (int j = 0; j < kSampleChunks; j++) qr[j] = refine ? __ldg(p4 + tid + (2 * j + 1) * (n_chunks / (2 * kSampleChunks))) : make_uint4(0xFF80FF80u, 0xFF80FF80u, 0xFF80FF80u, 0xFF80FF80u);
   constexpr int kHistPer = kTopkHist / kTB;
   int hid[kHistPer];                                                        // this thread's share of the history, in flight with the sample
 #pragma unroll
@@ -209,58 +227,60 @@ static __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem&
       const uint32_t bit = 1u << (id & 31);
       fresh = (atomicOr(&c.pen[id >> 5], bit) & bit) == 0u;
     }
-    const uint32_t slot = warp_reserve(&c.n_side, fresh ? 1u : 0u);
+    const uint32_t slot = warp_reserve_one(&c.n_side, fresh);
     if (fresh) c.side_id[slot] = static_cast<uint32_t>(id);
   }
   // ---- the cutoff: the largest positive BF16 code with at least `want` of the 8192 sampled logits at or above it ---------
-  // (about 1.3 k + 150 candidates expected in the whole row, at most ~1500)
   // A bisection over the codes, one barrier per probe; it starts from a bracket around the cutoff of the block's last
   // row of the same size class, which usually holds (rows of one batch come from one model), and costs ~7 probes then.
   uint32_t cut_code;
   {
-    const int n_target = min(1500, top_k + top_k / 3 + 150);
-    const uint32_t want = max(8u, static_cast<uint32_t>((static_cast<long long>(n_target) * kSampleChunks * kTB * kChunk + V - 1) / V));
     const int cls = min(31 - __clz(want), 7);
     int probe = 0;
     // sampled logits at or above each of three codes, with one barrier; every thread calls
-    auto count3 = [&](uint32_t a, uint32_t b, uint32_t d, uint32_t out[3]) {
-      const uint32_t codes[3] = {a, b, d};
-      uint32_t cnt[3] = {0u, 0u, 0u};
+    auto count_in = [&](const uint4 (&q)[kSampleChunks], uint32_t code) {
+      const uint32_t m2 = code | (code << 16);
+      const __nv_bfloat162 t2 = *reinterpret_cast<const __nv_bfloat162*>(&m2);
+      uint32_t n = 0u;                                                      // 16 mask bits per logit
+#pragma unroll
+      for (int j = 0; j < kSampleChunks; j++) {
+        n += __popc(__hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&q[j].x), t2)) + __popc(__hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&q[j].y), t2)) +
+             __popc(__hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&q[j].z), t2)) + __popc(__hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&q[j].w), t2));
+      }
+      return n >> 4;
+    };
+    auto meet3 = [&](const uint32_t (&mine)[3], uint32_t out[3]) {
 #pragma unroll
       for (int t = 0; t < 3; t++) {
-        const uint32_t m2 = codes[t] | (codes[t] << 16);
-        const __nv_bfloat162 t2 = *reinterpret_cast<const __nv_bfloat162*>(&m2);
-#pragma unroll
-        for (int j = 0; j < kSampleChunks; j++) {
-          cnt[t] += __popc(__hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&qs[j].x), t2)) + __popc(__hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&qs[j].y), t2)) +
-                    __popc(__hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&qs[j].z), t2)) + __popc(__hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&qs[j].w), t2));
-        }
-        cnt[t] = warp_sum_u32(cnt[t] >> 4);                     // 16 mask bits per logit
-        if (lane == 0 && cnt[t]) atomicAdd(&c.probe_cnt[probe + t], cnt[t]);
+        const uint32_t n = warp_sum_u32(mine[t]);
+        if (lane == 0 && n) atomicAdd(&c.probe_cnt[probe + t], n);
       }
       __syncthreads();
 #pragma unroll
       for (int t = 0; t < 3; t++) out[t] = c.probe_cnt[probe + t];
       probe += 3;
     };
+    auto count3 = [&](uint32_t a, uint32_t b, uint32_t d, uint32_t out[3]) {
+      const uint32_t mine[3] = {count_in(qs, a), count_in(qs, b), count_in(qs, d)};
+      meet3(mine, out);
+    };
     // the largest sampled logit: the reference point of the FP32 softmass (any value near the row maximum will do); it
-    // travels with the first probe's barrier
-    if (need_z) {
-      __nv_bfloat162 mx = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&qs[0].x), *reinterpret_cast<const __nv_bfloat162*>(&qs[0].y));
-      mx = __hmax2(mx, __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&qs[0].z), *reinterpret_cast<const __nv_bfloat162*>(&qs[0].w)));
+    // travels with the first barrier
+    __nv_bfloat162 mx = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&qs[0].x), *reinterpret_cast<const __nv_bfloat162*>(&qs[0].y));
+    mx = __hmax2(mx, __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&qs[0].z), *reinterpret_cast<const __nv_bfloat162*>(&qs[0].w)));
 #pragma unroll
-      for (int j = 1; j < kSampleChunks; j++) {
-        mx = __hmax2(mx, __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&qs[j].x), *reinterpret_cast<const __nv_bfloat162*>(&qs[j].y)));
-        mx = __hmax2(mx, __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&qs[j].z), *reinterpret_cast<const __nv_bfloat162*>(&qs[j].w)));
-      }
-      const uint32_t key = warp_max_u32(fkey(fmaxf(__low2float(mx), __high2float(mx))));
-      if (lane == 0) atomicMax(&c.ref_key, key);
+    for (int j = 1; j < kSampleChunks; j++) {
+      mx = __hmax2(mx, __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&qs[j].x), *reinterpret_cast<const __nv_bfloat162*>(&qs[j].y)));
+      mx = __hmax2(mx, __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&qs[j].z), *reinterpret_cast<const __nv_bfloat162*>(&qs[j].w)));
     }
+    const float mine_max = fmaxf(__low2float(mx), __high2float(mx));
+    const uint32_t max_key = warp_max_u32(fkey(mine_max));
+    if (lane == 0) atomicMax(&c.ref_key, max_key);
     // A few candidates more than wanted cost less than another round: a cut is good enough at twice the count wanted while that is small, at half
-    // as much again in between; a large top_k gets the closest cut. Never more than stand for 1500 candidates in the row: the list holds 2048,
+    // as much again beyond; a large top_k's is corrected below. Never more than stand for 1500 candidates in the row: the list holds 2048,
     // and at the largest vocabularies a sampled logit stands for 32 (512 rows of 262,144, top_k 1000: 60 rows handed on without that bound, 8 with it).
     const uint32_t most = static_cast<uint32_t>(1500ll * kSampleChunks * kTB * kChunk / V);
-    const uint32_t enough = max(want, min(want < 24u ? 2u * want : want < 48u ? want + want / 2u : want, most));
+    const uint32_t enough = refine ? want + want / 4u : max(want, min(want < 24u ? 2u * want : want + want / 2u, most));
     uint32_t n_lo = 0xFFFFFFFFu;                                            // count(sample >= lo), once it is known
     uint32_t lo = 0x0000u, hi = 0x7F7Fu;                                    // invariant: count(sample >= lo) >= want, or lo is still 0 (handed back below)
     const uint32_t prev = c.prev_cut[cls];
@@ -272,6 +292,47 @@ static __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem&
       else if (n3[2] >= want) { lo = bhi + 1u; n_lo = n3[2]; }
       else if (n3[1] >= want) { lo = mid; hi = bhi; n_lo = n3[1]; }
       else { lo = blo; hi = mid - 1u; n_lo = n3[0]; }
+    }
+    else {
+      // The block's first row of its class: the want-th largest of the threads' own maxima has at least `want` samples at or above it, and seldom
+      // many more. One warp finds it (a bisection by four over the three binades below the largest, or over all codes). Without it the search
+      // began with every code: 7.9 us of a row's 40 where a block has one row (256 penalised rows), 4.8 so.
+      uint16_t* maxima = reinterpret_cast<uint16_t*>(c.off);
+      maxima[tid] = mine_max > 0.0f ? static_cast<uint16_t>(__float_as_uint(mine_max) >> 16) : static_cast<uint16_t>(0u);
+      __syncthreads();
+      const uint32_t top_code = c.ref_key & 0x80000000u ? min((c.ref_key & 0x7FFFFFFFu) >> 16, 0x7F7Fu) : 0u;   // (a NaN or +inf maximum: handed on by the pass)
+      if (warp == 0) {
+        const uint4 a = reinterpret_cast<const uint4*>(maxima)[2 * lane], b = reinterpret_cast<const uint4*>(maxima)[2 * lane + 1];
+        const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        auto at_or_above = [&](uint32_t code) {                            // per lane; two packed counts
+          const uint32_t m2 = code | (code << 16);
+          const __nv_bfloat162 t2 = *reinterpret_cast<const __nv_bfloat162*>(&m2);
+          uint32_t n = 0u;
+#pragma unroll
+          for (int k = 0; k < 8; k++) n += __hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&w[k]), t2) & 0x00010001u;
+          return (n & 0xFFFFu) + (n >> 16);
+        };
+        uint32_t first = top_code > 0x0080u + 383u ? top_code - 383u : 0x0080u, last = max(top_code, 0x0080u);
+        if (warp_sum_u32(at_or_above(first)) < want) { last = first; first = 0x0080u; }
+#pragma unroll 1
+        while (first < last) {
+          const uint32_t span = last - first, q1 = first + (span + 3u) / 4u, q2 = first + (2u * span + 3u) / 4u, q3 = first + (3u * span + 3u) / 4u;
+          const uint32_t n = warp_sum_u32(at_or_above(q1) | (at_or_above(q2) << 10) | (at_or_above(q3) << 20));   // (512 at most each)
+          if ((n >> 20) >= want) first = q3;
+          else if (((n >> 10) & 1023u) >= want) { first = q2; last = q3 - 1u; }
+          else if ((n & 1023u) >= want) { first = q1; last = q2 - 1u; }
+          else last = q1 - 1u;
+        }
+        if (lane == 0) c.cross_bin = first;
+      }
+      __syncthreads();
+      lo = c.cross_bin; hi = max(top_code, lo);
+      const uint32_t q2 = min(lo + 6u, hi), q3 = min(lo + 18u, hi);
+      count3(lo, q2, q3, n3);
+      if (n3[2] >= want) { lo = q3; n_lo = n3[2]; }
+      else if (n3[1] >= want) { lo = q2; hi = q3 - 1u; n_lo = n3[1]; }
+      else if (n3[0] >= want) { hi = q2 - 1u; n_lo = n3[0]; }
+      else lo = hi = 0u;                                                    // fewer positive samples than wanted
     }
     while (lo < hi && n_lo > enough && probe + 3 <= kMaxProbes) {          // three cuts per round: the range shrinks fourfold
       const uint32_t span = hi - lo;
@@ -285,6 +346,16 @@ static __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem&
     cut_code = lo;
     if (cut_code < 0x0080u || (lo < hi && n_lo > enough)) { cp_async_wait<0>(); return false; }   // fewer positive logits than candidates wanted: not this kernel's row
                                                                             // (the copies in flight must land before the slots are used again)
+    // A large top_k has little room on either side (1536 candidates for 1000, of 2048): the cutoff is moved to where both samples together put it.
+    // (One row in 400 with a top_k of 1000 missed with one sample, and made a call of 256 rows 60 us longer.)
+    if (refine && probe + 3 <= kMaxProbes && cut_code >= 0x0090u) {
+      const uint32_t mine[3] = {count_in(qs, cut_code - 2u) + count_in(qr, cut_code - 2u), count_in(qs, cut_code) + count_in(qr, cut_code),
+                                count_in(qs, cut_code + 2u) + count_in(qr, cut_code + 2u)};
+      meet3(mine, n3);
+      const float per_code = fmaxf(1.0f, 0.25f * static_cast<float>(n3[0] - n3[2]));
+      const float by = rintf((static_cast<float>(n3[1]) - 2.0f * static_cast<float>(want)) / per_code);
+      cut_code = static_cast<uint32_t>(static_cast<int>(cut_code) + static_cast<int>(fminf(fmaxf(by, -6.0f), 6.0f)));
+    }
     if (tid == 0) c.prev_cut[cls] = cut_code;
   }
   const float cut_val = __uint_as_float(cut_code << 16);
@@ -373,7 +444,7 @@ static __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem&
     }
 #pragma unroll
     for (int j = 0; j < kExpand; j++) {
-      if (e0 + j * kTB >= n_hit) break;                                     // block-uniform
+      if (e0 + j * kTB + warp * 32 >= n_hit) break;                         // warp-uniform
       const uint32_t cc = ents[j], mask = kept_mask8(qq[j], cut_code | (cut_code << 16));
       const uint32_t keep = pen_on ? mask & ~((c.pen[cc >> 2] >> ((cc & 3u) * 8u)) & 0xFFu) : mask;   // penalised positions come from the list
       uint32_t slot = warp_reserve(&c.n, __popc(keep));
@@ -394,7 +465,7 @@ static __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem&
 #pragma unroll
     for (int j = 0; j < kGather; j++) {
       const uint32_t i = j * kTB + tid;
-      if (j * kTB >= n_side) break;                                         // block-uniform
+      if (j * kTB + warp * 32 >= n_side) break;                             // warp-uniform
       float v = -INFINITY;
       if (i < n_side) {
         const float raw = __uint_as_float(static_cast<uint32_t>(raws[j]) << 16);
@@ -402,7 +473,7 @@ static __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem&
         if (need_z) { zadd += static_cast<double>(ex2_approx(__fmaf_rn(v, c2a, nb))); zsub += static_cast<double>(ex2_approx(__fmaf_rn(raw, c2a, nb))); }
       }
       const bool cand = v >= cut_val;
-      const uint32_t slot = warp_reserve(&c.n, cand ? 1u : 0u);
+      const uint32_t slot = warp_reserve_one(&c.n, cand);
       if (cand) {
         if (slot < kTopkCap) c.key[slot] = (static_cast<unsigned long long>(fkey(v)) << 32) | (0xFFFFFFFFu - ids[j]);
         const uint32_t rel = (__float_as_uint(v) >> 16) - cut_code;
@@ -417,7 +488,11 @@ static __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem&
     __syncthreads();
     if (lane == 0) { sd[warp] = zsum; sd[kTW + warp] = zadd; c.warp_d[warp] = zsub; }
     __syncthreads();
-    for (int w = 0; w < kTW; w++) { z_raw += sd[w]; z_add += sd[kTW + w]; z_sub += c.warp_d[w]; }
+    static_assert(kTW == 16, "two of the three sums side by side in a warp");
+    double two = sd[lane], third = lane < kTW ? c.warp_d[lane] : 0.0;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) { two += __shfl_xor_sync(kFull, two, o); third += __shfl_xor_sync(kFull, third, o); }
+    z_raw = __shfl_sync(kFull, two, 0); z_add = __shfl_sync(kFull, two, 16); z_sub = __shfl_sync(kFull, third, 0);
   }
   const double z_tilde = z_raw - z_sub + z_add;
   if (need_z && !(z_tilde > 0.0)) return false;                             // nothing left after the corrections (cancellation): the exact path
@@ -453,6 +528,86 @@ static __device__ double topk_exact_mass(const SampleDev& P, TopkSmem& c, const 
   return block_sum_f64(m, c.scratch);
 }
 
+// The FP32 mass of the whole row, moved to the exact maximum, and how far it can be from the exact one (the bound with a quarter added).
+__device__ __forceinline__ double topk_row_total(const RowMass& zm, float vmax, double inv_t, double* err) {
+  // z_tilde approximates sum_i 2^(z_i c2a + nb); nb's own rounding is a common factor and is taken out exactly here (zm.shift is the true -nb,
+  // not M c2a).
+  const double c64 = 1.4426950408889634 * inv_t;
+  // With the slope that the terms were formed with: log2(e) / T in FP64 instead would leave the factor 2^(vmax (c2a - c)), which no
+  // bound below holds (a maximum of 105 at T 0.3: 2e-5).
+  const double total = zm.z_tilde * exp2(zm.shift - static_cast<double>(vmax) * zm.slope);
+  // What separates it from sum_i 2^((z_i - vmax) c), relative, first order, worst case (u = 2^-24, the FP32 unit roundoff):
+  //   - c2a = fl32(c): every term is off by a factor 2^(x_i delta), |delta| <= u, x_i = (z_i - M) c; weighted by the terms that is
+  //     ln2 u E_w|x| <= u (ln V + 2 ln2 D): E_w[-x ln2] = H - ln Z <= ln V (H the entropy of the softmax, Z >= 1 relative to the
+  //     row maximum, V <= 2^18: ln V <= 12.5), and the terms above the sampled maximum have 0 < x <= D = (vmax - M) c;
+  //   - the FMA rounds its result: half an ulp of |x| < 32 is at most 2^-20, a factor 2^(2^-20) = 1 + 6.6e-7 on the term, and D / 16 times
+  //     that for the terms up to D above the sampled maximum; the terms below -32 weigh less than V 2^-32 altogether;
+  //   - ex2.approx.ftz.f32: 2 ulp = 4 u;
+  //   - each lane accumulates 4 n_it terms one after the other in FP32, then two accumulators and the lanes meet in FP64:
+  //     (4 n_it + 1) u (zm.acc_terms);
+  // These are relative to the mass the pass summed (z_raw), which holds the penalised positions at their raw values. The penalised
+  // logits then enter as z_raw - z_sub + z_add, every term of z_sub and z_add with the per-term errors above (FMA, ex2, c2a on a
+  // single term: 1.6e-6 covers them for |x| < 32); when penalised tokens carried most of the raw mass the band grows with them.
+  // A boundary of the cumulative mass inside the band is decided by the FP64 mass.
+  const double u = 5.9604644775390625e-8;
+  const double D = fmax(0.0, (static_cast<double>(vmax) - static_cast<double>(zm.ref)) * c64);
+  const double rel = u * (12.5 + 1.3862943611198906 * D) + 6.6e-7 * fmax(1.0, D * 0.0625) + 4.0 * u + zm.acc_terms * u;
+  *err = 1.25 * (rel * zm.z_raw + 1.6e-6 * zm.z_corr) * (total / zm.z_tilde);
+  return total;
+}
+
+// At most kFew candidates down to the top-k crossing: ordered by rank, then one warp does the rest with shuffles and votes
+// (vocab_parallel.cuh) where the block-wide code needs a barrier per step. Every thread calls. (Rows of 151,936 with a top_k of 20, two blocks to an
+// SM: 9.3 us of 32.7 by the block, 5.6 so.)
+static __device__ bool topk_finish_few(const SampleDev& P, int row, TopkSmem& c, uint32_t cut_code, const RowMass& zm, int n, uint32_t cross, int n_sel) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid < kFew) c.off[tid] = 0u;                                          // (the ranks; everyone has read what was there)
+  for (int i = tid; i < n; i += kTB) {
+    const unsigned long long k = c.key[i];
+    const uint32_t rel = (__float_as_uint(fkey_inv(static_cast<uint32_t>(k >> 32))) >> 16) - cut_code;
+    if (rel >= cross) c.sel[atomicAdd(&c.n_hit, 1u)] = k;                   // (n_sel of them)
+  }
+  __syncthreads();
+  {
+    const int e = tid % kFew;
+    if (e < n_sel) {
+      const unsigned long long k = c.sel[e];
+      uint32_t r = 0u;
+      for (int j = tid / kFew; j < n_sel; j += kTB / kFew) r += c.sel[j] > k ? 1u : 0u;
+      if (r) atomicAdd(&c.off[e], r);
+    }
+  }
+  __syncthreads();
+  if (tid < n_sel) c.w[c.off[tid]] = c.sel[tid];
+  __syncthreads();
+  const float T = P.temperature ? P.temperature[row] : P.temperature_s, top_p = P.top_p ? P.top_p[row] : P.top_p_s, min_p = P.min_p ? P.min_p[row] : P.min_p_s;
+  const int top_k = P.top_k ? P.top_k[row] : P.top_k_s;
+  const double inv_t = 1.0 / static_cast<double>(T);
+  const bool has_p = top_p > 0.0f && top_p < 1.0f, in_topk = (P.flags & LM_FLAG_TOPP_IN_TOPK) && has_p;
+  MergeTail t;
+  t.key = c.w; t.vmax = fkey_inv(static_cast<uint32_t>(c.w[0] >> 32)); t.z_total = 0.0;
+  double exact = 0.0;
+#pragma unroll 1
+  for (int pass = 0; pass < 2; pass++) {
+    if (warp == 0) {
+      VpMergeDev M;
+      M.flags = P.flags; M.draw = P.draw; M.uniforms = P.uniforms; M.seed = P.seed; M.step = P.step; M.row_offset = P.row_offset;
+      M.out_tokens = P.out_tokens; M.out_tau = P.out_tau; M.out_status = P.out_status; M.out_vmax = P.out_vmax; M.out_mass = P.out_mass;
+      M.hand_on = 1; M.path_status = pass ? 0u : LM_STATUS_CANDIDATE_PATH; M.mass_band = 0.0;
+      t.amb = 0;
+      if (pass) t.z_total = exact;
+      else if (has_p && !in_topk) { double err; t.z_total = topk_row_total(zm, t.vmax, inv_t, &err); M.mass_band = err / t.z_total; }
+      merge_tail_one_warp<2>(M, row, t, n_sel, T, top_k, top_p, min_p, inv_t, 0u);
+      if (lane == 0) c.wide = static_cast<uint32_t>(t.amb);
+    }
+    __syncthreads();
+    if (!c.wide) break;
+    if (zm.row == nullptr) return false;                                    // too close to call, and nothing finer to look at here
+    exact = topk_exact_mass(P, c, zm, t.vmax, inv_t);                       // ... in FP64
+  }
+  return true;
+}
+
 // The exact phases of the candidate path, on what the pass (or a producer of logits tiles, sample_tiles.cuh) has left in shared
 // memory: c.key[0 .. c.n) = every logit of the row at or above the cutoff code as (monotone value key << 32) | ~index, c.bins[b] =
 // how many of them have BF16 code cut_code + b, c.wide set if one lies beyond the bins. `zm` is what is known about the mass of
@@ -482,12 +637,14 @@ static __device__ bool topk_finish(const SampleDev& P, int row, TopkSmem& c, uin
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) { const uint32_t t = __shfl_up_sync(kFull, incl, o); if (lane >= o) incl += t; }
     if (lane == 31) c.warp_u[warp] = incl;
+    if (tid == 0) c.n_hit = 0u;
     __syncthreads();
-    for (int w = 0; w < warp; w++) run += c.warp_u[w];
+    run = warp_sum_u32(lane < warp ? c.warp_u[lane] : 0u);
     uint32_t acc = run + incl - mine;
 #pragma unroll
     for (int j = 0; j < kPer; j++) {
       c.off[kTopkBins - 1 - (kPer * tid + j)] = acc;
+      c.hitlist[kTopkBins - 1 - (kPer * tid + j)] = 0u;                      // (dead since the candidates were expanded: see `front` below)
       if (acc < static_cast<uint32_t>(top_k) && acc + cb[j] >= static_cast<uint32_t>(top_k)) c.cross_bin = static_cast<uint32_t>(kTopkBins - 1 - (kPer * tid + j));
       acc += cb[j];
     }
@@ -496,19 +653,20 @@ static __device__ bool topk_finish(const SampleDev& P, int row, TopkSmem& c, uin
   const uint32_t cross = c.cross_bin;
   const int n_sel = static_cast<int>(c.off[cross] + c.bins[cross]);
   __syncthreads();                                                          // the counts are consumed below
+  if (n_sel <= kFew) return topk_finish_few(P, row, c, cut_code, zm, n, cross, n_sel);
+  // In a bin, the values that are no BF16 values (penalised logits) lie above those that are, which are all equal: they fill their bin from its
+  // front, the others from its end, and only they have to be put in order.
+  uint32_t* front = c.hitlist;
   for (int i = tid; i < n; i += kTB) {
     const unsigned long long k = c.key[i];
-    const uint32_t rel = (__float_as_uint(fkey_inv(static_cast<uint32_t>(k >> 32))) >> 16) - cut_code;
-    if (rel >= cross) c.sel[c.off[rel] + atomicSub(&c.bins[rel], 1u) - 1u] = k;
+    const uint32_t bits = __float_as_uint(fkey_inv(static_cast<uint32_t>(k >> 32))), rel = (bits >> 16) - cut_code;
+    if (rel >= cross) c.sel[c.off[rel] + ((bits & 0xFFFFu) ? atomicAdd(&front[rel], 1u) : atomicSub(&c.bins[rel], 1u) - 1u)] = k;
   }
   __syncthreads();
   for (uint32_t b = cross + tid; b < kTopkBins; b += kTB) {
-    const uint32_t lo = c.off[b], hi = (b == cross) ? static_cast<uint32_t>(n_sel) : c.off[b - 1];
-    bool sorted = true;
-    for (uint32_t i = lo + 1u; i < hi; i++) sorted = sorted && (c.sel[i - 1u] >> 32) >= (c.sel[i] >> 32);
-    if (sorted) continue;
+    const uint32_t lo = c.off[b], hi = lo + front[b];
     if (hi - lo > static_cast<uint32_t>(kBinSortMax)) { c.wide = 1u; continue; }
-    for (uint32_t i = lo + 1u; i < hi; i++) {                               // insertion sort on the value part: equal values stay put
+    for (uint32_t i = lo + 1u; i < hi; i++) {                               // insertion sort on the value part
       const unsigned long long k = c.sel[i];
       uint32_t j = i;
       while (j > lo && (c.sel[j - 1u] >> 32) < (k >> 32)) { c.sel[j] = c.sel[j - 1u]; j--; }
@@ -517,6 +675,11 @@ static __device__ bool topk_finish(const SampleDev& P, int row, TopkSmem& c, uin
   }
   __syncthreads();
   if (c.wide) return false;                                                 // a large bin of unequal (penalised) values: the exact path takes the row
+  auto value_at = [&](int i) { return fkey_inv(static_cast<uint32_t>(c.sel[i] >> 32)); };
+  // how many of the ordered candidates lie at or above v (complete behind the next barrier; `count` held 0 before the last one)
+  auto count_prefix = [&](float v, uint32_t* count) {
+    for (int i = tid; i < n_sel; i += kTB) if (value_at(i) >= v && (i == n_sel - 1 || value_at(i + 1) < v)) *count = static_cast<uint32_t>(i + 1);
+  };
 
   // ---- exact thresholds on the sorted candidates ------------------------------------------------------------------------
   const float vmax = fkey_inv(static_cast<uint32_t>(c.sel[0] >> 32));
@@ -526,37 +689,12 @@ static __device__ bool topk_finish(const SampleDev& P, int row, TopkSmem& c, uin
   if (has_p) {
     for (int i = tid; i < n_sel; i += kTB) c.cum[i] = softmass(fkey_inv(static_cast<uint32_t>(c.sel[i] >> 32)), vmax, inv_t);
     __syncthreads();
-    scan_f64(c.cum, n_sel, c.warp_d);
-    uint64_t cnt_k = 0ull;
-    for (int i = tid; i < n_sel; i += kTB) cnt_k += fkey_inv(static_cast<uint32_t>(c.sel[i] >> 32)) >= tau_k ? 1ull : 0ull;
-    const int n_topk = static_cast<int>(block_sum_u64(cnt_k, c.scratch));
-    double total, err = 0.0;
+    count_prefix(tau_k, &c.n_hit);
+    double total = 0.0, err = 0.0;
+    if (!in_topk) total = topk_row_total(zm, vmax, inv_t, &err);
+    scan_f64(c.cum, n_sel, c.warp_d);                                       // (two barriers)
+    const int n_topk = static_cast<int>(c.n_hit);
     if (in_topk) total = c.cum[n_topk - 1];
-    else {
-      // The FP32 mass of the whole row, moved to the exact maximum. z_tilde approximates sum_i 2^(z_i c2a + nb); nb's own rounding
-      // is a common factor and is taken out exactly here (zm.shift is the true -nb, not M c2a).
-      const double c64 = 1.4426950408889634 * inv_t;
-      // With the slope that the terms were formed with: log2(e) / T in FP64 instead would leave the factor 2^(vmax (c2a - c)), which no
-      // bound below holds (a maximum of 105 at T 0.3: 2e-5).
-      total = zm.z_tilde * exp2(zm.shift - static_cast<double>(vmax) * zm.slope);
-      // What separates it from sum_i 2^((z_i - vmax) c), relative, first order, worst case (u = 2^-24, the FP32 unit roundoff):
-      //   - c2a = fl32(c): every term is off by a factor 2^(x_i delta), |delta| <= u, x_i = (z_i - M) c; weighted by the terms that is
-      //     ln2 u E_w|x| <= u (ln V + 2 ln2 D): E_w[-x ln2] = H - ln Z <= ln V (H the entropy of the softmax, Z >= 1 relative to the
-      //     row maximum, V <= 2^18: ln V <= 12.5), and the terms above the sampled maximum have 0 < x <= D = (vmax - M) c;
-      //   - the FMA rounds its result: half an ulp of |x| < 32 is at most 2^-20, a factor 2^(2^-20) = 1 + 6.6e-7 on the term, and D / 16 times
-      //     that for the terms up to D above the sampled maximum; the terms below -32 weigh less than V 2^-32 altogether;
-      //   - ex2.approx.ftz.f32: 2 ulp = 4 u;
-      //   - each lane accumulates 4 n_it terms one after the other in FP32, then two accumulators and the lanes meet in FP64:
-      //     (4 n_it + 1) u (zm.acc_terms);
-      // These are relative to the mass the pass summed (z_raw), which holds the penalised positions at their raw values. The penalised
-      // logits then enter as z_raw - z_sub + z_add, every term of z_sub and z_add with the per-term errors above (FMA, ex2, c2a on a
-      // single term: 1.6e-6 covers them for |x| < 32); when penalised tokens carried most of the raw mass the band grows with them.
-      // The band is this bound with a quarter added. A boundary of the cumulative mass inside it is decided by the FP64 mass.
-      const double u = 5.9604644775390625e-8;
-      const double D = fmax(0.0, (static_cast<double>(vmax) - static_cast<double>(zm.ref)) * c64);
-      const double rel = u * (12.5 + 1.3862943611198906 * D) + 6.6e-7 * fmax(1.0, D * 0.0625) + 4.0 * u + zm.acc_terms * u;
-      err = 1.25 * (rel * zm.z_raw + 1.6e-6 * zm.z_corr) * (total / zm.z_tilde);
-    }
     double target;
     bool edge = false;
 #pragma unroll 1
@@ -590,9 +728,11 @@ static __device__ bool topk_finish(const SampleDev& P, int row, TopkSmem& c, uin
     if (tau_m > tau64) tau64 = tau_m;
   }
   const float tau = __double2float_rn(tau64);
-  uint64_t cnt_kept = 0ull;
-  for (int i = tid; i < n_sel; i += kTB) cnt_kept += fkey_inv(static_cast<uint32_t>(c.sel[i] >> 32)) >= tau ? 1ull : 0ull;
-  const int n_kept = static_cast<int>(block_sum_u64(cnt_kept, c.scratch));   // the kept set is the first n_kept sorted candidates
+  if (tid == 0) c.n_side = 0u;
+  __syncthreads();
+  count_prefix(tau, &c.n_side);
+  __syncthreads();
+  const int n_kept = static_cast<int>(c.n_side);                            // the kept set is the first n_kept sorted candidates
 
   // ---- the draw ----------------------------------------------------------------------------------------------------------
   int token = -1;

@@ -208,3 +208,34 @@ def test_the_histogram_draw_at_the_edges_of_its_batches(vocab, penalised):
     np.testing.assert_array_equal(r.tau.cpu().numpy(), tau)
     np.testing.assert_array_equal(r.tokens.cpu().numpy(), tok)
     assert not np.any(r.status.cpu().numpy() & 1)                            # none handed on to the generic algorithm
+
+
+@pytest.mark.parametrize("rows,vocab,top_k", [(80, 32768, 1), (80, 40008, 63), (80, 40008, 64), (80, 40008, 65), (400, 32768, 20), (400, 32768, 450), (80, 262144, 1024)])
+@pytest.mark.parametrize("draw", ["inverse_cdf", "gumbel"])
+def test_the_candidate_kernel_around_its_one_warp_finish_and_its_cutoff(rows, vocab, top_k, draw):
+    """Up to 64 candidates down to the top-k crossing one warp finishes the row, beyond that the block; the cutoff of a block's first row comes from the
+    threads' maxima, a later one's from the row before (400 rows: more than there are blocks), a large top_k's is corrected by a second sample.
+    Ties at the crossing (half the rows are coarse) and penalised logits at the top of the row put 63 .. 66 candidates there."""
+    rng = np.random.default_rng(vocab + top_k)
+    z = rng.standard_normal((rows, vocab)).astype(np.float32) * 2.0
+    z[::2] = np.round(z[::2] * 16.0) / 16.0
+    codes = oracle.f32_to_bf16(z)
+    hist = rng.integers(0, vocab, (rows, 200)).astype(np.int32)
+    hist[:, :60] = np.argsort(-z, axis=1)[:, :120:2]
+    T, top_p = rng.uniform(0.3, 1.5, rows).astype(np.float32), rng.uniform(0.5, 1.0, rows).astype(np.float32)
+    u = rng.random(rows).astype(np.float32)
+    x, h, ut = bf16_tensor(codes), torch.from_numpy(hist).cuda(), torch.from_numpy(u).cuda()
+    for extra in (dict(), dict(min_p=0.02, topp_in_topk=True)):
+        p = lm.SamplingParams(draw=draw, seed=7, temperature=torch.from_numpy(T).cuda(), top_k=top_k, top_p=torch.from_numpy(top_p).cuda(), repetition_penalty=1.2,
+                              presence_penalty=0.3, **extra)
+        assert vocab == 32768 and rows == 80 or "sample_topk_kernel" in routes.names(lambda: lm.sample(x, p, history=h, uniforms=ut))
+        r = lm.sample(x, p, history=h, uniforms=ut, return_tau=True, return_status=True, return_vmax=True)
+        tok, tau, _ = oracle.sample_batch(codes, temperature=T, top_k=top_k, top_p=top_p, history=hist, draw=draw, uniforms=u, seed=7, repetition_penalty=1.2,
+                                          presence_penalty=0.3, n_threads=THREADS, **extra)
+        status = r.status.cpu().numpy()
+        np.testing.assert_array_equal(r.tau.cpu().numpy(), tau)
+        assert np.all((r.tokens.cpu().numpy() == tok) | ((status & 4) != 0))
+        if rows == 80:
+            zf = oracle.bf16_to_f32(codes)
+            for i in range(0, rows, 9):
+                assert int(r.mass[i]) == oracle.kept_mass(oracle.apply_penalties(zf[i], hist[i], 1.2, 0.3), tau[i], T[i]), i
