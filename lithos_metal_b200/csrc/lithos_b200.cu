@@ -522,9 +522,7 @@ int lm_head(const lm_head_args* a) {
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lm_head_kernel, kHeadThreads, smem) != cudaSuccess || per_sm < 1) per_sm = 1;
   const long long tiles = (a->vocab + kHeadTile - 1) / kHeadTile, want = (tiles + kHeadWarps - 1) / kHeadWarps;
   const int grid = static_cast<int>(want < static_cast<long long>(per_sm) * sms ? want : static_cast<long long>(per_sm) * sms);
-  lm_head_kernel<<<grid, kHeadThreads, smem, static_cast<cudaStream_t>(a->stream)>>>(P);
-  const cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? LM_OK : cuda_fail(e);
+  return launch_beside(lm_head_kernel, static_cast<unsigned>(grid), kHeadThreads, smem, 1, static_cast<cudaStream_t>(a->stream), P);
 }
 
 size_t lm_step_state_bytes(int32_t t_max, int32_t gamma_max) {
