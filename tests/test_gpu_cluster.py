@@ -309,3 +309,16 @@ def test_one_top_k_for_all_rows_of_half_the_gpu(rows, vocab, top_k):
         near = r.status.cpu().numpy() & 4
         np.testing.assert_array_equal(r.tau.cpu().numpy(), tau)
         assert np.all((r.tokens.cpu().numpy() == tok) | (near != 0))
+
+
+@pytest.mark.parametrize("vocab", [16384, 40964, 151936])
+@pytest.mark.parametrize("top_k", [0, 20, 700])
+def test_probabilities_of_aligned_and_ragged_rows(vocab, top_k):
+    """The kept mass comes from the ordered top-k set where there is one, and probabilities are written 16 bytes at a time where a row's slice of the output
+    is aligned (a vocabulary of 40,964: its last chunk is not whole, and BF16 rows begin at odd offsets)."""
+    rng = np.random.default_rng(vocab + top_k)
+    z = (rng.standard_normal((3, vocab)) * 2).astype(np.float32)
+    hist = rng.integers(0, vocab, (3, 100)).astype(np.int32)
+    knobs = dict(temperature=np.float32([0.7, 1.0, 1.4]), top_k=np.full(3, top_k, np.int32), top_p=np.float32([0.95, 0.0, 0.8]), min_p=np.float32([0.0, 0.01, 0.0]))
+    for host in (z, oracle.f32_to_bf16(z)):
+        _check(_tensor(host), host, knobs, draw="inverse_cdf", history=hist, rho=1.1, pi=0.5, stats=True)
