@@ -259,3 +259,26 @@ def test_the_first_call_of_a_process_may_need_just_under_48_kb_a_slice():
             "p = lm.SamplingParams(temperature=0.9, top_k=1, seed=3)\n"
             "assert lm.sample(x, p).tokens.tolist() == lm.argmax(x).tolist()\n")
     subprocess.run([sys.executable, "-c", code], check=True, timeout=300, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+
+
+@pytest.mark.parametrize("rows", [1, 2, 9])
+@pytest.mark.parametrize("kind", ["masked", "outlier", "equal"])
+def test_the_slices_quick_bound_and_the_one_behind_it(rows, kind):
+    """The bound by linear bins lets too much through where a masked logit or one far above the rest stretches the bins, or where logits are equal: the bound
+    by the keys then keeps the row on this path, as long as that does not exceed a record either."""
+    vocab, top_k = 151936, 64
+    x, host = _rows(rows, vocab, rows + 70, "f32")
+    rng = np.random.default_rng(rows)
+    if kind == "masked":
+        host[:, rng.random(vocab) < 0.9] = -1e9                               # threads with nothing but masked logits
+    elif kind == "outlier":
+        host[:, 4321] = 3e5
+    else:
+        host[:, ::40] = 7.0                                                   # 60 to 240 a slice
+    if kind != "equal":
+        _check(torch.from_numpy(host).cuda(), host, draw="inverse_cdf", temperature=0.9, top_k=top_k, top_p=0.95)
+    else:                                                                     # (with many equal logits in a slice the row may be handed on)
+        u = np.linspace(0.1, 0.9, rows).astype(np.float32)
+        r = lm.sample(torch.from_numpy(host).cuda(), lm.SamplingParams(temperature=0.9, top_k=top_k, draw="inverse_cdf"), uniforms=torch.from_numpy(u).cuda(), return_tau=True)
+        tok, tau, _ = oracle.sample_batch(host, temperature=0.9, top_k=top_k, draw="inverse_cdf", uniforms=u, n_threads=8)
+        assert r.tokens.cpu().tolist() == tok.tolist() and r.tau.cpu().tolist() == tau.tolist()
