@@ -1324,8 +1324,12 @@ static __device__ __noinline__ void phase_probs(const ClusterSmem& s, const Samp
 template <int B>
 static __device__ __noinline__ int row_in_order(const SampleDev& P, int rows, int at, ClusterSmem& s) {
   const int tid = threadIdx.x, lane = tid & 31;
-  uint32_t* count = s.fill;                                                 // [2][rows / 32]: the first two kinds per 32 rows (the bins, cleared above, lie elsewhere)
   constexpr int kGroups = kOrderRows / 32;
+  uint32_t* count = s.r_cnt;                                                // [2][rows / 32]: the first two kinds per 32 rows
+  // (No barrier lies between the kernel's clearing of its bins and the first count: the counts have to be other words, and these are written again
+  // before anything else reads them.)
+  static_assert(2 * kGroups <= kCBins && offsetof(ClusterSmem, r_cnt) >= offsetof(ClusterSmem, max_cnt) + sizeof(ClusterSmem::max_cnt) &&
+                offsetof(ClusterSmem, r_cnt) >= offsetof(ClusterSmem, hi) + sizeof(ClusterSmem::hi), "the counts share no word with what the kernel clears first");
   auto kind_of = [&](int r) {
     if (r >= rows) return 3;
     const int k = P.top_k[r];
@@ -1360,8 +1364,7 @@ static __device__ __noinline__ int row_in_order(const SampleDev& P, int rows, in
   }
   __syncthreads();
   const int row = s.row;
-  __syncthreads();                                                          // (the count lies over what is cleared next)
-  for (int i = tid; i < 2 * kGroups; i += B) count[i] = 0u;
+  __syncthreads();                                                          // (the knobs' thread writes s.row again)
   return row;
 }
 
