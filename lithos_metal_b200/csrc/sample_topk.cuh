@@ -28,7 +28,7 @@ constexpr int kTopkMaxK = 1024;            // largest top_k this kernel takes
 constexpr int kTopkHist = 2048;            // longest history it takes
 constexpr int kTopkMaxVocab = 1 << 18;
 constexpr int kMaxProbes = 30;             // counters of the cutoff search per row: three per round, one round for the bracket + eight for the whole code range
-constexpr int kBinSortMax = 256;           // most candidates of one code bin whose values are no BF16 values (penalised ones)
+constexpr int kBinSortMax = 256;           // most candidates of one code bin whose values are no BF16 values (penalised ones), unless they are in order already (all equal)
 constexpr int kFew = 64;                   // this many candidates down to the top-k crossing are finished by one warp
 constexpr uint32_t kRefineFrom = 44u;      // sampled logits wanted from which on the cutoff is corrected by as many samples again
 constexpr int kSampleChunks = 1024 / kTB;   // chunks per thread in the cutoff sample: 1024 chunks = 8192 logits
@@ -665,8 +665,10 @@ static __device__ bool topk_finish(const SampleDev& P, int row, TopkSmem& c, uin
   __syncthreads();
   for (uint32_t b = cross + tid; b < kTopkBins; b += kTB) {
     const uint32_t lo = c.off[b], hi = lo + front[b];
-    if (hi - lo > static_cast<uint32_t>(kBinSortMax)) { c.wide = 1u; continue; }
-    for (uint32_t i = lo + 1u; i < hi; i++) {                               // insertion sort on the value part
+    uint32_t from = lo + 1u;                                                // those in order already (all, if they are equal) stay
+    while (from < hi && (c.sel[from - 1u] >> 32) >= (c.sel[from] >> 32)) from++;
+    if (from < hi && hi - lo > static_cast<uint32_t>(kBinSortMax)) { c.wide = 1u; continue; }
+    for (uint32_t i = from; i < hi; i++) {                                  // insertion sort on the value part
       const unsigned long long k = c.sel[i];
       uint32_t j = i;
       while (j > lo && (c.sel[j - 1u] >> 32) < (k >> 32)) { c.sel[j] = c.sel[j - 1u]; j--; }

@@ -123,6 +123,31 @@ def test_penalised_and_greedy_rows_arrive_in_tiles_too(draw):
     assert want.tokens.cpu().tolist() == tok.tolist()
 
 
+@pytest.mark.parametrize("draw", ["inverse_cdf", "gumbel"])
+def test_hundreds_of_equal_penalised_logits_stay_on_the_candidate_path(draw):
+    """400 history ids with one raw logit: as many equal values that are no BF16 values, in one code bin above the top_k-th logit. Equal values need no
+    order among themselves, however many they are: in tiles the row is not declined, in a batch the candidate kernel keeps it."""
+    rows, vocab, top_k = 80, 40960, 450
+    x, host = _logits(rows, vocab, 50, scale=1.0)
+    g = np.random.default_rng(51)
+    hist = np.stack([g.permutation(vocab)[:400] for _ in range(rows)]).astype(np.int32)
+    x.scatter_(1, torch.from_numpy(hist).cuda().long(), 5.0)
+    p = lm.SamplingParams(temperature=0.9, top_k=torch.full((rows,), top_k, dtype=torch.int32), top_p=0.95, repetition_penalty=1.3, presence_penalty=0.4, seed=9, draw=draw)
+    u, h = torch.from_numpy(g.random(rows).astype(np.float32)).cuda(), torch.from_numpy(hist).cuda()
+    want = lm.sample(x, p, history=h, uniforms=u, step=2, return_tau=True, return_status=True)
+    assert np.all(want.status.cpu().numpy() & _lib.STATUS_CANDIDATE_PATH)
+    ts = lm.TileSampler(rows, vocab, p, history=h)
+    _feed(ts, x, 2048)
+    got = ts.finish(uniforms=u, step=2, return_tau=True)
+    assert not np.any(got.status.cpu().numpy() & _lib.STATUS_TILE_DECLINED)
+    tok, tau, _ = oracle.sample_batch(x.view(torch.int16).cpu().numpy().view(np.uint16), temperature=0.9, top_k=top_k, top_p=0.95, history=hist, repetition_penalty=1.3,
+                                      presence_penalty=0.4, draw=draw, uniforms=u.cpu().numpy(), seed=9, step=2, n_threads=8)
+    near = (want.status.cpu().numpy() & _lib.STATUS_NEAR_TIE) != 0 if draw == "gumbel" else np.zeros(rows, bool)
+    for r in (want, got):
+        np.testing.assert_array_equal(r.tau.cpu().numpy(), tau)
+        assert np.all((r.tokens.cpu().numpy() == tok) | near)
+
+
 def test_rows_the_tile_path_does_not_take_are_declined_not_guessed():
     rows, vocab = 5, 32768
     x, _ = _logits(rows, vocab, 30)
