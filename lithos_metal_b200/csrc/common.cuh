@@ -41,6 +41,12 @@ __device__ __forceinline__ uint32_t kept_mask8(const uint4 q, uint32_t tau_code2
   const uint32_t m2 = __hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&q.z), t2), m3 = __hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&q.w), t2);
   return (m0 | m1 | m2 | m3) == 0u ? 0u : mask8(m0, m1, m2, m3);
 }
+// The same logits in no particular order: bits 0..3 and 16..19, one per logit (where they are only counted).
+__device__ __forceinline__ uint32_t kept_bits8(const uint4 q, uint32_t tau_code2) {
+  const __nv_bfloat162 t2 = *reinterpret_cast<const __nv_bfloat162*>(&tau_code2);
+  return (__hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&q.x), t2) & 0x00010001u) | (__hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&q.y), t2) & 0x00020002u) |
+         (__hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&q.z), t2) & 0x00040004u) | (__hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&q.w), t2) & 0x00080008u);
+}
 
 // Monotone 32-bit key of a float: a > b  <=>  fkey(a) > fkey(b) (for non-NaN, with -0 canonicalised to +0 first).
 __device__ __forceinline__ uint32_t fkey(float f) {

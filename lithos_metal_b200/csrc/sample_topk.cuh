@@ -27,11 +27,13 @@ constexpr int kTopkBins = 512;             // BF16 codes above the cutoff that t
 constexpr int kTopkMaxK = 1024;            // largest top_k this kernel takes
 constexpr int kTopkHist = 2048;            // longest history it takes
 constexpr int kTopkMaxVocab = 1 << 18;
-constexpr int kMaxProbes = 30;             // counters of the cutoff search per row: three per round, one round for the bracket + eight for the whole code range
+constexpr int kSearchProbes = 30;          // counters of the cutoff search per row: three per round, one round for the bracket + eight for the whole code range ...
+constexpr int kMaxProbes = kSearchProbes + 7;   // ... and seven for the looks around the cutoff (topk_settle)
 constexpr int kBinSortMax = 256;           // most candidates of one code bin whose values are no BF16 values (penalised ones), unless they are in order already (all equal)
 constexpr int kFew = 64;                   // this many candidates down to the top-k crossing are finished by one warp
 constexpr uint32_t kRefineFrom = 44u;      // sampled logits wanted from which on the cutoff is corrected by as many samples again
 constexpr int kSampleChunks = 1024 / kTB;   // chunks per thread in the cutoff sample: 1024 chunks = 8192 logits
+static_assert(kSampleChunks == 2, "topk_settle holds a bit for each logit of a thread's two samples");
 constexpr int kTopkMinVocab = 32768;
 
 constexpr int kStages = 4;                 // 16-byte asynchronous copies in flight per thread during the pass
@@ -152,6 +154,84 @@ static __global__ void __launch_bounds__(kPrepThreads) sample_prep_kernel(Sample
   if (threadIdx.x == 0) counters[kCounterOther] = n;
 }
 
+// How many logits of the row lie at or above code a (low word) and code b (high word); every thread calls.
+static __device__ __noinline__ uint64_t topk_count_row(const uint4* p4, int n_chunks, uint32_t a, uint32_t b, uint64_t* scratch) {
+  constexpr int kDeep = 8;                                                  // a thread's loads in flight
+  uint32_t na = 0u, nb = 0u;
+  for (int c0 = threadIdx.x; c0 < n_chunks; c0 += kDeep * kTB) {
+    uint4 q[kDeep];
+#pragma unroll
+    for (int j = 0; j < kDeep; j++) q[j] = c0 + j * kTB < n_chunks ? __ldg(p4 + c0 + j * kTB) : make_uint4(0xFF80FF80u, 0xFF80FF80u, 0xFF80FF80u, 0xFF80FF80u);
+#pragma unroll
+    for (int j = 0; j < kDeep; j++) { na += __popc(kept_bits8(q[j], a | (a << 16))); nb += __popc(kept_bits8(q[j], b | (b << 16))); }
+  }
+  return block_sum_u64(static_cast<uint64_t>(na) | (static_cast<uint64_t>(nb) << 32), scratch);
+}
+
+// Chunk j of a thread's second sample, between those of the first, and where it lands: the list of the chunks is written behind the pass, and the
+// history's ids fill the first half of their array at most.
+__device__ __forceinline__ int topk_second_chunk(int tid, int j, int n_chunks) { return tid + (2 * j + 1) * (n_chunks / (2 * kSampleChunks)); }
+__device__ __forceinline__ uint4* topk_second_slot(TopkSmem& c, int tid, int j) { return (j ? reinterpret_cast<uint4*>(c.cum + kTopkCap / 2) : reinterpret_cast<uint4*>(c.hitlist)) + tid; }
+
+// The cutoff that the search on one sample has found, looked at again on that sample (q0, q1) and a second one as large (staged: it has been asked
+// for). A function of its own: inline it made the rows that never come by up to 10 % slower (350 rows, top_k 100), and the second sample held in
+// registers from the start of the row did so too. lam, full: what top_k and kTopkCap logits of the row stand for in one sample. 0: no cutoff will
+// do. Every thread calls; the copies in flight have landed behind it.
+static __device__ __noinline__ uint32_t topk_settle(const uint4* p4, int n_chunks, int top_k, float lam, float full, uint32_t want, uint32_t cut, bool coarse, bool staged, bool pen_on,
+                                                    uint4 q0, uint4 q1, TopkSmem& c) {
+  const int tid = threadIdx.x, lane = tid & 31;
+  uint4 q[4] = {q0, q1};
+  cp_async_wait<0>();
+#pragma unroll
+  for (int j = 0; j < 2; j++) q[2 + j] = staged ? *topk_second_slot(c, tid, j) : __ldg(p4 + topk_second_chunk(tid, j, n_chunks));
+  auto count = [&](int slot, uint32_t code) {
+    uint32_t bits = 0u;
+#pragma unroll
+    for (int j = 0; j < 4; j++) bits |= kept_bits8(q[j], code | (code << 16)) << (4 * j);
+    const uint32_t n = warp_sum_u32(__popc(bits));
+    if (lane == 0 && n) atomicAdd(&c.probe_cnt[kSearchProbes + slot], n);
+  };
+  // How far a count lies inside of what the top_k and what the list of candidates stand for, in standard deviations.
+  auto inside = [&](uint32_t n) {
+    const float low = 2.0f * lam, high = 2.0f * full, x = static_cast<float>(n);
+    return fminf((x - low - 2.0f) * rsqrtf(low), (high - x) * rsqrtf(high));
+  };
+  if (coarse) {
+    // Coarse logits: the next code up has fewer than wanted, this one more than the usual slack. Either may be the right side of the step: the
+    // upper one where it surely has top_k logits, this one where they surely fit the list, else the row is counted. (256 rows of integers N(0, 2^2), us
+    // with one step of the cutoff on the samples alone, which hands half of them on / so: 151,936 logits, top_k 450 411 / 144, 1000 493 / 152; 262,144
+    // logits, top_k 100 239 / 51, 300 919 / 75. Counting a row takes about 10 us of it.)
+    count(0, cut); count(1, cut + 1u);
+    __syncthreads();
+    if (inside(c.probe_cnt[kSearchProbes + 1]) >= 3.0f) return cut + 1u;
+    if (inside(c.probe_cnt[kSearchProbes]) >= 3.0f) return cut;
+    const uint64_t both = topk_count_row(p4, n_chunks, cut, cut + 1u, c.scratch);
+    if (static_cast<uint32_t>(both) <= static_cast<uint32_t>(kTopkCap)) return cut;
+    if (static_cast<uint32_t>(both >> 32) >= static_cast<uint32_t>(top_k)) return cut + 1u;
+    return pen_on ? cut : 0u;                                               // (penalties may yet move some below it)
+  }
+  // A large top_k has little room on either side (1477 candidates for 1000, of 2048): of the cutoff and its neighbours the one that both samples
+  // together put nearest to what is wanted, if it is well inside, or furthest inside; four more where that is less far than it should be (of N(0, 2^2) logits
+  // with a top_k of 1000 one row in 300 of 151,936, one in 4 of 262,144). One row in 400 with a top_k of 1000 missed with one sample, and made a
+  // call of 256 rows 60 us longer; one in 600 of 262,144 does so now. (Five looks at once: 256 rows, top_k 400 42.9 us, 42.2 so.)
+  constexpr int kAt[7] = {0, -5, 5, -2, 2, -10, 10};                        // (a code is 1 to 4 % of the candidates)
+  float best = -INFINITY, best_in = 0.0f; int by = 0;
+  auto look = [&](int first, int last) {
+#pragma unroll
+    for (int t = 0; t < 7; t++) if (t >= first && t < last) count(t, cut + kAt[t]);
+    __syncthreads();
+#pragma unroll
+    for (int t = 0; t < 7; t++) if (t >= first && t < last) {
+      const uint32_t n = c.probe_cnt[kSearchProbes + t];
+      const float in = inside(n), fit = in >= 3.0f ? -fabsf(static_cast<float>(n) - 2.0f * static_cast<float>(want)) : in - 1e6f;
+      if (fit > best) { best = fit; best_in = in; by = kAt[t]; }
+    }
+  };
+  look(0, 3);
+  if (best_in < 2.5f) look(3, 7);                                           // (uniform)
+  return max(static_cast<uint32_t>(static_cast<int>(cut) + by), 0x0080u);
+}
+
 struct TopkSmem;
 static __device__ bool topk_finish(const SampleDev& P, int row, TopkSmem& c, uint32_t cut_code, const RowMass& zm);
 
@@ -196,13 +276,17 @@ static __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem&
 #pragma unroll
   for (int j = 0; j < kSampleChunks; j++) qs[j] = __ldg(p4 + tid + j * (n_chunks / kSampleChunks));
   // The sampled logits wanted at or above the cutoff: what the top_k stands for in the sample (lam), and so many more that one row in 10^5 has fewer
-  // than top_k candidates (4.3 standard deviations of a Poisson count, and 6 for the small ones); what stands for 1536 candidates at most.
-  const float lam = static_cast<float>(top_k) * (static_cast<float>(kSampleChunks * kTB * kChunk) / static_cast<float>(V));
-  const uint32_t want = static_cast<uint32_t>(fminf(ceilf(lam + 4.3f * sqrtf(lam) + 6.0f), 1536.0f * (static_cast<float>(kSampleChunks * kTB * kChunk) / static_cast<float>(V))));
-  const bool refine = want >= kRefineFrom;
-  uint4 qr[kSampleChunks];                                                  // as many again, between the others
+  // than top_k candidates (4.3 standard deviations of a Poisson count, and 6 for the small ones), but no more than lie as many of its standard deviations
+  // above that as below what the list of candidates holds (the means of square roots: the spread of a count's root is the same everywhere).
+  const float per_logit = static_cast<float>(kSampleChunks * kTB * kChunk) / static_cast<float>(V), lam = static_cast<float>(top_k) * per_logit, full = static_cast<float>(kTopkCap) * per_logit;
+  const float middle = 0.5f * (sqrtf(lam) + sqrtf(full));
+  const uint32_t want = static_cast<uint32_t>(fminf(ceilf(lam + 4.3f * sqrtf(lam) + 6.0f), middle * middle));
+  const bool refine = want >= kRefineFrom || (static_cast<float>(want) - lam - 2.0f) < 4.0f * sqrtf(lam);   // ... or less slack than usual
+  if (refine) {                                                             // as many samples again, between the others, land where nothing else does before the pass
 #pragma unroll
-  for (int j = 0; j < kSampleChunks; j++) qr[j] = refine ? __ldg(p4 + tid + (2 * j + 1) * (n_chunks / (2 * kSampleChunks))) : make_uint4(0xFF80FF80u, 0xFF80FF80u, 0xFF80FF80u, 0xFF80FF80u);
+    for (int j = 0; j < kSampleChunks; j++) cp_async16(topk_second_slot(c, tid, j), p4 + topk_second_chunk(tid, j, n_chunks));
+    cp_async_commit();
+  }
   constexpr int kHistPer = kTopkHist / kTB;
   int hid[kHistPer];                                                        // this thread's share of the history, in flight with the sample
 #pragma unroll
@@ -239,30 +323,22 @@ static __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem&
     int probe = 0;
     // sampled logits at or above each of three codes, with one barrier; every thread calls
     auto count_in = [&](const uint4 (&q)[kSampleChunks], uint32_t code) {
-      const uint32_t m2 = code | (code << 16);
-      const __nv_bfloat162 t2 = *reinterpret_cast<const __nv_bfloat162*>(&m2);
-      uint32_t n = 0u;                                                      // 16 mask bits per logit
+      uint32_t bits = 0u;                                                   // a bit per logit, gathered first: a count of bits takes four times as long as a logical operation
 #pragma unroll
-      for (int j = 0; j < kSampleChunks; j++) {
-        n += __popc(__hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&q[j].x), t2)) + __popc(__hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&q[j].y), t2)) +
-             __popc(__hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&q[j].z), t2)) + __popc(__hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&q[j].w), t2));
-      }
-      return n >> 4;
+      for (int j = 0; j < kSampleChunks; j++) bits |= kept_bits8(q[j], code | (code << 16)) << (4 * j);
+      return static_cast<uint32_t>(__popc(bits));
     };
-    auto meet3 = [&](const uint32_t (&mine)[3], uint32_t out[3]) {
+    auto count3 = [&](uint32_t a, uint32_t b, uint32_t d, uint32_t out[3]) {
+      const uint32_t codes[3] = {a, b, d};
 #pragma unroll
       for (int t = 0; t < 3; t++) {
-        const uint32_t n = warp_sum_u32(mine[t]);
+        const uint32_t n = warp_sum_u32(count_in(qs, codes[t]));
         if (lane == 0 && n) atomicAdd(&c.probe_cnt[probe + t], n);
       }
       __syncthreads();
 #pragma unroll
       for (int t = 0; t < 3; t++) out[t] = c.probe_cnt[probe + t];
       probe += 3;
-    };
-    auto count3 = [&](uint32_t a, uint32_t b, uint32_t d, uint32_t out[3]) {
-      const uint32_t mine[3] = {count_in(qs, a), count_in(qs, b), count_in(qs, d)};
-      meet3(mine, out);
     };
     // the largest sampled logit: the reference point of the FP32 softmass (any value near the row maximum will do); it
     // travels with the first barrier
@@ -281,17 +357,17 @@ static __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem&
     // and at the largest vocabularies a sampled logit stands for 32 (512 rows of 262,144, top_k 1000: 60 rows handed on without that bound, 8 with it).
     const uint32_t most = static_cast<uint32_t>(1500ll * kSampleChunks * kTB * kChunk / V);
     const uint32_t enough = refine ? want + want / 4u : max(want, min(want < 24u ? 2u * want : want + want / 2u, most));
-    uint32_t n_lo = 0xFFFFFFFFu;                                            // count(sample >= lo), once it is known
+    uint32_t n_lo = 0xFFFFFFFFu, n_up = 0u;                                 // count(sample >= lo), once it is known; count(sample >= hi + 1)
     uint32_t lo = 0x0000u, hi = 0x7F7Fu;                                    // invariant: count(sample >= lo) >= want, or lo is still 0 (handed back below)
     const uint32_t prev = c.prev_cut[cls];
     uint32_t n3[3];
     if (prev >= 0x0080u) {                                                  // both ends of the bracket and its middle in one round
       const uint32_t blo = max(prev, 0x0090u) - 16u, bhi = min(prev + 15u, 0x7F7Eu), mid = (blo + bhi + 1u) >> 1;
       count3(blo, mid, bhi + 1u, n3);
-      if (n3[0] < want) hi = blo - 1u;
+      if (n3[0] < want) { hi = blo - 1u; n_up = n3[0]; }
       else if (n3[2] >= want) { lo = bhi + 1u; n_lo = n3[2]; }
-      else if (n3[1] >= want) { lo = mid; hi = bhi; n_lo = n3[1]; }
-      else { lo = blo; hi = mid - 1u; n_lo = n3[0]; }
+      else if (n3[1] >= want) { lo = mid; hi = bhi; n_lo = n3[1]; n_up = n3[2]; }
+      else { lo = blo; hi = mid - 1u; n_lo = n3[0]; n_up = n3[1]; }
     }
     else {
       // The block's first row of its class: the want-th largest of the threads' own maxima has at least `want` samples at or above it, and seldom
@@ -330,31 +406,26 @@ static __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem&
       const uint32_t q2 = min(lo + 6u, hi), q3 = min(lo + 18u, hi);
       count3(lo, q2, q3, n3);
       if (n3[2] >= want) { lo = q3; n_lo = n3[2]; }
-      else if (n3[1] >= want) { lo = q2; hi = q3 - 1u; n_lo = n3[1]; }
-      else if (n3[0] >= want) { hi = q2 - 1u; n_lo = n3[0]; }
+      else if (n3[1] >= want) { lo = q2; hi = q3 - 1u; n_lo = n3[1]; n_up = n3[2]; }
+      else if (n3[0] >= want) { hi = q2 - 1u; n_lo = n3[0]; n_up = n3[1]; }
       else lo = hi = 0u;                                                    // fewer positive samples than wanted
     }
-    while (lo < hi && n_lo > enough && probe + 3 <= kMaxProbes) {          // three cuts per round: the range shrinks fourfold
+    while (lo < hi && n_lo > enough && probe + 3 <= kSearchProbes) {          // three cuts per round: the range shrinks fourfold
       const uint32_t span = hi - lo;
       const uint32_t q1 = lo + (span + 3u) / 4u, q2 = lo + (2u * span + 3u) / 4u, q3 = lo + (3u * span + 3u) / 4u;   // lo < q1 <= q2 <= q3 <= hi
       count3(q1, q2, q3, n3);
       if (n3[2] >= want) { lo = q3; n_lo = n3[2]; }
-      else if (n3[1] >= want) { lo = q2; hi = q3 - 1u; n_lo = n3[1]; }
-      else if (n3[0] >= want) { lo = q1; hi = q2 - 1u; n_lo = n3[0]; }
-      else hi = q1 - 1u;
+      else if (n3[1] >= want) { lo = q2; hi = q3 - 1u; n_lo = n3[1]; n_up = n3[2]; }
+      else if (n3[0] >= want) { lo = q1; hi = q2 - 1u; n_lo = n3[0]; n_up = n3[1]; }
+      else { hi = q1 - 1u; n_up = n3[0]; }
     }
     cut_code = lo;
     if (cut_code < 0x0080u || (lo < hi && n_lo > enough)) { cp_async_wait<0>(); return false; }   // fewer positive logits than candidates wanted: not this kernel's row
                                                                             // (the copies in flight must land before the slots are used again)
-    // A large top_k has little room on either side (1536 candidates for 1000, of 2048): the cutoff is moved to where both samples together put it.
-    // (One row in 400 with a top_k of 1000 missed with one sample, and made a call of 256 rows 60 us longer.)
-    if (refine && probe + 3 <= kMaxProbes && cut_code >= 0x0090u) {
-      const uint32_t mine[3] = {count_in(qs, cut_code - 2u) + count_in(qr, cut_code - 2u), count_in(qs, cut_code) + count_in(qr, cut_code),
-                                count_in(qs, cut_code + 2u) + count_in(qr, cut_code + 2u)};
-      meet3(mine, n3);
-      const float per_code = fmaxf(1.0f, 0.25f * static_cast<float>(n3[0] - n3[2]));
-      const float by = rintf((static_cast<float>(n3[1]) - 2.0f * static_cast<float>(want)) / per_code);
-      cut_code = static_cast<uint32_t>(static_cast<int>(cut_code) + static_cast<int>(fminf(fmaxf(by, -6.0f), 6.0f)));
+    const bool coarse = n_lo > enough;                                      // the next code up has too few, this one more than the usual slack
+    if (coarse || refine) {
+      cut_code = topk_settle(p4, n_chunks, top_k, lam, full, want, cut_code, coarse, refine, pen_on, qs[0], qs[1], c);
+      if (cut_code == 0u) return false;
     }
     if (tid == 0) c.prev_cut[cls] = cut_code;
   }
