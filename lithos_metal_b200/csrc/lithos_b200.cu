@@ -185,8 +185,10 @@ int lm_sample(const lm_sample_args* a) {
     S.slices = kSlices;
     while (S.slices > 16 && static_cast<long long>(S.slices) * a->rows > sms && a->vocab <= static_cast<int64_t>(S.slices / 2) * (kSliceMaxLen - 8)) S.slices >>= 1;
     if (static_cast<long long>(S.slices) * a->rows > sms) return sample_clusters(P, sms, st, true);
-    // a record holds twice the top_k (16 at least): only a slice with that many logits at or above its own bound overflows it
-    S.cap = a->top_k_s <= 8 ? 16 : 2 * a->top_k_s;
+    // A record holds twice the top_k (16 at least), and as many times that as a slice is longer than one of 64: only a slice with that many logits at or
+    // above its own bound overflows it. (8 rows of 151,936 integers N(0, 2^2), top_k 50: 464 us with records for twice the top_k, 17 so.)
+    const int usual = a->top_k_s <= 8 ? 16 : 2 * a->top_k_s;
+    S.cap = usual * (kSlices / S.slices);
     S.slice_len = static_cast<int>(((a->vocab + S.slices - 1) / S.slices + 7) / 8 * 8);
     if (S.slice_len <= kSliceMaxLen) {
       char* ws = static_cast<char*>(a->workspace) + ws_base;
@@ -206,7 +208,7 @@ int lm_sample(const lm_sample_args* a) {
       if (rc != LM_OK) return rc;
       VpMergeDev M;
       M.bases = nullptr; M.pieces = 1;
-      M.records = S.records; M.shards = S.slices; M.rows = P.rows; M.cap = S.cap; M.record_bytes = S.record_bytes;
+      M.records = S.records; M.shards = S.slices; M.rows = P.rows; M.cap = S.cap; M.ahead = usual; M.record_bytes = S.record_bytes;
       M.temperature = nullptr; M.temperature_s = a->temperature_s; M.top_k = nullptr; M.top_k_s = a->top_k_s;
       M.top_p = a->top_p; M.top_p_s = a->top_p_s; M.min_p = a->min_p; M.min_p_s = a->min_p_s;
       M.flags = a->flags; M.draw = a->draw; M.uniforms = a->uniforms; M.seed = a->seed; M.step = a->step; M.row_offset = a->row_offset;
@@ -481,7 +483,7 @@ int lm_vocab_merge(const lm_vocab_args* a) {
   if (a->draw == LM_DRAW_INVERSE_CDF && a->uniforms == nullptr) return LM_E_INVALID;
   if (a->shards > kVpMaxShards || a->cap > kVpPerThread * (kVpMaxCandidates / a->shards) || a->rows > 0x7FFFFFFF) return LM_E_UNSUPPORTED;
   VpMergeDev P;
-  P.records = static_cast<const unsigned char*>(a->records); P.shards = a->shards; P.rows = static_cast<int>(a->rows); P.cap = a->cap;
+  P.records = static_cast<const unsigned char*>(a->records); P.shards = a->shards; P.rows = static_cast<int>(a->rows); P.cap = a->cap; P.ahead = a->cap;
   P.bases = static_cast<const unsigned long long*>(a->record_ptrs); P.pieces = a->pieces > 0 ? a->pieces : 1;
   if (P.bases && (a->shards % P.pieces) != 0) return LM_E_INVALID;
   P.record_bytes = static_cast<int64_t>(lm_vocab_record_bytes(a->cap));

@@ -13,7 +13,7 @@
 //                       the row's maximum and mass, thresholds, draw.
 //
 // The record format is the vocab-parallel one, a slice standing for a shard. Rows with a top_k of 1 .. 64 only: a slice's record
-// has room for twice the top_k (16 at least), so that only a slice with that many logits at or above its bound (ties at its own
+// has room for twice the top_k (16 at least) with 64 slices, four times as much with 16, so that only a slice with that many logits at or above its bound (ties at its own
 // k-th value) overflows it; the merge's block then runs the generic row algorithm on such a row itself.
 #pragma once
 #include "common.cuh"
@@ -31,7 +31,8 @@ constexpr int kSliceMaxLen = 32768;       // logits of one slice (128 KB of shar
 constexpr int kSlicedMaxRows = 32;        // rows per call on this path
 constexpr int kSlicedMinVocab = 16384;
 constexpr int kSlices = 64;               // slices per row at most
-constexpr int kSliceMaxCap = 128;         // candidates in one slice's record: twice the largest top_k
+constexpr int kSliceMaxCap = 128;         // candidates in one slice's record: twice the largest top_k (of 64 slices; more of fewer, as many in all)
+static_assert(kSlices * kSliceMaxCap <= kVpMergeCap, "the merge takes in every slot of a row's records");
 constexpr size_t kSlicedWsBytes = static_cast<size_t>(kSlicedMaxRows) * kSlices * (kVpHeader + 8 * kSliceMaxCap);
 
 struct SliceDev {

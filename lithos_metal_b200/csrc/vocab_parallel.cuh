@@ -171,6 +171,7 @@ struct VpMergeDev {
   const unsigned long long* bases;   // per GPU, the address of its [pieces][rows] records (its own memory or a peer's, read in place); or null
   int pieces;                        // with `bases`: records per row and GPU (shard s of the merge = piece s % pieces of GPU s / pieces)
   int shards; int rows; int cap; int64_t record_bytes;
+  int ahead;                         // slots of a record that are asked for before its header says how many are filled (more are so only where logits are equal)
   const float* temperature; float temperature_s; const int32_t* top_k; int32_t top_k_s;
   const float* top_p; float top_p_s; const float* min_p; float min_p_s;
   uint32_t flags; int draw; const float* uniforms; uint64_t seed; uint32_t step; int64_t row_offset;
@@ -382,7 +383,7 @@ static __device__ bool vocab_merge_row(const VpMergeDev& P, int row, VpMergeSmem
 #pragma unroll
     for (int i = 0; i < kVpPerThread; i++) {
       const int j = r + i * per;
-      if (j < P.cap) { pv[i] = rv[j]; pi[i] = ri[j]; }
+      if (j < P.ahead) { pv[i] = rv[j]; pi[i] = ri[j]; }
     }
   }
   __syncthreads();                                                        // (the shared fields above are set)
@@ -424,6 +425,16 @@ static __device__ bool vocab_merge_row(const VpMergeDev& P, int row, VpMergeSmem
   }
   // ---- keys of the filled slots and their span
   uint32_t keys[kVpPerThread];
+  if (cnt > P.ahead) {
+    const unsigned char* rec = merge_record(P, g, row);
+    const float* rv = reinterpret_cast<const float*>(rec + kVpHeader);
+    const int32_t* ri = reinterpret_cast<const int32_t*>(rec + kVpHeader + 4 * static_cast<size_t>(P.cap));
+#pragma unroll
+    for (int i = 0; i < kVpPerThread; i++) {
+      const int j = r + i * per;
+      if (j >= P.ahead && j < cnt) { pv[i] = rv[j]; pi[i] = ri[j]; }
+    }
+  }
   {
     uint32_t kmin = 0xFFFFFFFFu, kmax = 0u;
 #pragma unroll

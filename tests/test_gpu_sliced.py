@@ -14,6 +14,7 @@ import torch
 import oracle
 import lithos_metal_b200 as lm
 from lithos_metal_b200 import _lib
+from tests import routes
 
 pytestmark = pytest.mark.gpu
 SLICED, GENERIC = _lib.STATUS_SLICED_PATH, 1
@@ -230,6 +231,27 @@ def test_slices_to_a_row_by_how_many_rows_there_are(rows, vocab, top_k, dtype):
     rng = np.random.default_rng(rows)
     hist = rng.integers(0, vocab, (rows, 300)).astype(np.int32)
     _check(x, host, draw="inverse_cdf", temperature=1.2, top_k=top_k, history=hist, rho=1.2, pi=0.3)
+
+
+@pytest.mark.parametrize("rows,top_k", [(3, 64), (4, 64), (5, 50), (8, 20), (8, 50), (9, 64)])
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+def test_longer_slices_have_longer_records(rows, top_k, dtype):
+    """Integer-valued logits: a hundred of them and more share the value of a slice's k-th. With 32 or 16 slices to a row a record holds two or four times
+    as many candidates as with 64, and the merge takes them all in."""
+    vocab = 151936
+    z = np.round(np.random.default_rng(rows + top_k).standard_normal((rows, vocab)) * 2).astype(np.float32)
+    host = oracle.f32_to_bf16(z) if dtype == "bf16" else z
+    x = torch.from_numpy(host.view(np.int16)).cuda().view(torch.bfloat16) if dtype == "bf16" else torch.from_numpy(host).cuda()
+    u = np.random.default_rng(5).random(rows).astype(np.float32)
+    ut = torch.from_numpy(u).cuda()
+    for draw in ("inverse_cdf", "gumbel"):
+        p = lm.SamplingParams(temperature=0.8, top_k=top_k, top_p=0.9, seed=4, draw=draw)
+        assert routes.names(lambda: lm.sample(x, p, uniforms=ut)) == ["slice_local_kernel", "sliced_merge_kernel"]
+        r = lm.sample(x, p, uniforms=ut, return_tau=True, return_status=True)
+        tok, tau, _ = oracle.sample_batch(host, temperature=0.8, top_k=top_k, top_p=0.9, draw=draw, uniforms=u, seed=4, n_threads=8)
+        st = r.status.cpu().numpy()
+        assert r.tau.cpu().tolist() == tau.tolist() and np.all((r.tokens.cpu().numpy() == tok) | ((st & 4) != 0))
+        assert np.all(st & SLICED), st
 
 
 @pytest.mark.parametrize("rows", [8, 12])
