@@ -19,15 +19,22 @@ static int cluster_blocks(int64_t rows, int64_t vocab, int slots) {
 // fifteen of 8 and thirty-two of 4 at once, and one row more waits for a second round (16 rows of 151,936, top_k 20: 41 us with 8 blocks
 // each, 29 us with 4). Beyond that the blocks share SMs, and a row without a top_k takes several times as long as one with: smaller pieces
 // even that out where the slices stay long (binary32 rows with mixed knobs, us with 1 / 2 / 4 blocks: 96 rows of 151,936 198 / 184 / 126,
-// 96 of 65,536 96 / 78 / 87, 400 of 50,257 193 / 175 / 280, 400 of 24,576 119 / 136 / 243). `listed`: every row has a top_k and a short list
-// (BF16, top_k 50, us with 2 / 4 blocks: 64 rows of 151,936 27 / 36, of 262,144 39 / 37, 74 of those 40 / 58).
-static int sample_blocks(int64_t rows, int64_t vocab, int sms, bool listed) {
+// 96 of 65,536 96 / 78 / 87, 400 of 50,257 193 / 175 / 280, 400 of 24,576 119 / 136 / 243).
+// `listed_k`: the top_k that every row has, with a list (0: they differ, or have none). Two blocks to a row then, but for the longest rows of 33 to 64, whose
+// quarters no longer fit shared memory and so lie two to an SM, twice thirty-two clusters at once: us with 2 / 4 blocks,
+//   BF16, top_k 50: 64 rows of 151,936 25.0 / 35.4, of 196,608 29.9 / 30.9, of 229,376 33.9 / 33.2, of 262,144 38.7 / 37.0; of 262,144 40 rows 34.1 / 34.9, 48 34.7 / 34.9,
+//   56 37.0 / 35.0, 74 39.8 / 57.5; top_k 512: 64 rows of 196,608 38.2 / 39.0, of 245,760 44.6 / 42.9, 40 of those 39.8 / 41.0 (the line: 80,000 logits to an SM);
+//   a longer list sooner: top_k 700, of 180,224 40 rows 38.6 / 39.0, 64 40.9 / 42.4, of 196,608 41.5 / 39.3 and 42.3 / 41.7; 1000, 64 rows of those 48.5 / 45.9;
+//   binary32, top_k 20: of 172,032 40 rows 29.4 / 30.2, of 196,608 32.3 / 30.8, 64 35.5 / 37.0, of 229,376 39.5 / 39.6, of 262,144 42.4 / 41.1.
+static int sample_blocks(int64_t rows, int64_t vocab, int sms, bool f32, int listed_k) {
+  const bool listed = listed_k > 0;
   int c = 1;
   if (rows * 20 <= sms) c = 16;
   else if (rows * 48 <= 5LL * sms) c = 8;
   else if (rows * 9 <= 2LL * sms) c = 4;
   else if (!listed && rows <= 2LL * sms && vocab >= (rows * 3 <= sms ? 49152 : 98304)) c = 4;
-  else if (listed && rows * 16 <= 7LL * sms && vocab >= 196608) c = 4;
+  else if (listed && rows * 16 <= 7LL * sms && vocab >= 196608 &&
+           (listed_k > 512 || (f32 ? rows * 8 <= 3LL * sms || vocab >= 229376 : vocab >= 229376 && rows * vocab >= 80000LL * sms))) c = 4;
   else if (rows * 2 <= sms) c = 2;
   else if (listed ? rows <= 2LL * sms && vocab >= 65536 : rows * 3 <= 2LL * sms || (rows <= 3LL * sms && vocab >= 40000)) c = 2;
   while (c > 1 && vocab < 2048LL * c) c >>= 1;
@@ -77,7 +84,7 @@ int sample_clusters(const SampleDev& P, int sms, cudaStream_t st, bool few) {
   };
   int rc = LM_OK;
   bool fits = false;
-  const int most = sample_blocks(P.rows, P.vocab, sms, P.top_k == nullptr && P.top_k_s >= 1 && P.top_k_s <= kCListK && !(P.flags & LM_FLAG_EXACT_ONLY));
+  const int most = sample_blocks(P.rows, P.vocab, sms, f32, P.top_k == nullptr && P.top_k_s <= kCListK && !(P.flags & LM_FLAG_EXACT_ONLY) ? P.top_k_s : 0);
   const int C = cluster_that_fits(most, [&](int c) { rc = cluster_ready(f32, plan(c), &fits); return fits || rc != LM_OK; });
   const ClusterPlan p = plan(C);
   if (rc == LM_OK && C == 1) rc = cluster_ready(f32, p, &fits);

@@ -7,6 +7,7 @@ import torch
 
 import oracle
 import lithos_metal_b200 as lm
+from tests import routes
 
 pytestmark = pytest.mark.gpu
 
@@ -310,6 +311,22 @@ def test_one_top_k_for_all_rows_of_half_the_gpu(rows, vocab, top_k):
         near = r.status.cpu().numpy() & 4
         np.testing.assert_array_equal(r.tau.cpu().numpy(), tau)
         assert np.all((r.tokens.cpu().numpy() == tok) | (near != 0))
+
+
+@pytest.mark.parametrize("rows,vocab,top_k,dtype,blocks", [(64, 196608, 50, "bf16", 2), (64, 196608, 1000, "bf16", 4), (48, 229376, 50, "bf16", 2), (56, 229376, 50, "bf16", 4),
+                                                           (40, 262144, 50, "bf16", 2), (65, 262144, 50, "bf16", 2), (40, 196608, 20, "f32", 4), (64, 196608, 20, "f32", 2)])
+def test_blocks_to_a_row_with_one_top_k(rows, vocab, top_k, dtype, blocks):
+    """33 to 64 long rows with one top_k: two blocks to a row, or four where those measured faster (the line is made for 148 SMs); the same results."""
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the lines depend on the number of SMs")
+    g = torch.Generator(device="cuda")
+    g.manual_seed(rows)
+    x = torch.randn(rows, vocab, generator=g, device="cuda") * 2
+    x = x.to(torch.bfloat16) if dtype == "bf16" else x
+    p, e = (lm.SamplingParams(temperature=0.8, top_k=top_k, top_p=0.9, seed=5, exact_only=exact) for exact in (False, True))
+    assert [k[:2] for k in routes.kernels(lambda: lm.sample(x, p))[0]] == [("sample_cluster_kernel", rows * blocks)]
+    r, q = (lm.sample(x, params, return_tau=True, return_status=True) for params in (p, e))
+    assert torch.equal(r.tau, q.tau) and bool(torch.all((r.tokens == q.tokens) | (((r.status | q.status) & 4) != 0)))
 
 
 @pytest.mark.parametrize("vocab", [16384, 40964, 151936])
