@@ -30,15 +30,15 @@ inline int sm_count(int* out) {
   return LM_OK;
 }
 
-// Kernels that need more than 48 KB of shared memory, their static arrays (up to 13 KB) included, must be told so once per device (the attribute
-// belongs to the device's copy of the function); remembered per device and kernel, raised when a call needs more.
+// Kernels that need more than 48 KB of shared memory, their static arrays included, must be told so once per device (the attribute belongs to the
+// device's copy of the function). They are told whatever they ask for, so that nothing here has to know their arrays; remembered per device and kernel,
+// raised when a call needs more.
 enum KernelSlot { kSlotFast, kSlotTopk, kSlotGeneric, kSlotVocabLocal, kSlotVerify, kSlotVerifyStats, kSlotTileFinish, kSlotSlice, kSlotSliceSmall, kSlotSliceTiny, kSlotSlicedMerge, kSlotHead, kSlotCluster,
                   kSlotArgmax = kSlotCluster + 6,   // (the cluster kernel has six instances, the argmax kernel two)
                   kSlotDraftQ = kSlotArgmax + 2,    // (two instances)
                   kSlotCount = kSlotDraftQ + 2 };
 
 inline int ensure_dynamic_smem(KernelSlot slot, const void* func, size_t bytes, bool large_clusters = false) {
-  if (bytes <= 32 * 1024 && !large_clusters) return LM_OK;
   constexpr int kMaxDevices = 64;
   static std::mutex mutex;
   static size_t granted[kMaxDevices][kSlotCount] = {};
