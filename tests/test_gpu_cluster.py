@@ -269,32 +269,49 @@ def test_more_clusters_than_run_at_once_take_every_row_once(rows, vocab):
 
 @pytest.mark.parametrize("rows", [1, 4, 100, 760])
 def test_calls_in_a_row_see_what_the_one_before_them_left(rows):
-    """Kernels are made ready beside the one in front of them in the stream and wait for it: each of these calls (few rows; streaming kernels with
-    one top_k, none, or the rows' own) looks at logits that the one before it decided."""
-    vocab = 40960
+    """Kernels are made ready beside the one in front of them in the stream and wait for it. Chains of this library's calls with no other kernel in between
+    (few rows; streaming kernels with one top_k, none, or the rows' own): each reads what the one right before it wrote -- its tokens as a history, its
+    logits -- or writes over what that one read, and all share one workspace. The same as with the device idle between any two."""
+    vocab, H = 40960, 512
     g = torch.Generator(device="cuda")
     g.manual_seed(rows)
     x = (torch.randn(rows, vocab, generator=g, device="cuda") * 2).to(torch.bfloat16)
-    p = lm.SamplingParams(temperature=0.8, top_p=0.9, seed=3)
-    q = lm.SamplingParams(temperature=0.8, top_k=20, top_p=0.9, seed=3)
-    own = lm.SamplingParams(temperature=0.8, top_k=torch.tensor([0, 20, 700], dtype=torch.int32, device="cuda").repeat(rows // 3 + 1)[:rows].contiguous(), top_p=0.9, seed=3)
+    pen = dict(repetition_penalty=1.3, presence_penalty=4.0)
+    p = lm.SamplingParams(temperature=0.8, top_p=0.9, seed=3, **pen)
+    q = lm.SamplingParams(temperature=0.8, top_k=20, top_p=0.9, seed=3, **pen)
+    own = lm.SamplingParams(temperature=0.8, top_k=torch.tensor([0, 20, 700], dtype=torch.int32, device="cuda").repeat(rows // 3 + 1)[:rows].contiguous(), top_p=0.9, seed=3, **pen)
+    few = min(rows, 8)
+    hidden = [(torch.randn(few, H, generator=g, device="cuda") * (i + 1)).to(torch.bfloat16) for i in range(3)]
+    weight = (torch.randn(vocab, H, generator=g, device="cuda") * 0.05).to(torch.bfloat16)
+    first = torch.zeros(rows, dtype=torch.int32, device="cuda")
+    steps = 12
+    tokens = [[torch.empty(rows, dtype=torch.int32, device="cuda") for _ in range(7 * steps)] for _ in range(2)]
+    drawn = [[torch.empty(few, dtype=torch.int32, device="cuda") for _ in range(6 * steps)] for _ in range(2)]
+    logits = torch.empty(few, vocab, dtype=torch.bfloat16, device="cuda")
+    torch.cuda.synchronize()
 
-    def run(wait):
-        y, found = x.clone(), []
-        for step in range(12):
-            greedy = lm.argmax(y)
-            found.append(greedy.clone())
-            y.scatter_(1, greedy.long()[:, None], -5.0)
-            for params in (p, q, own):
-                t = lm.sample(y, params, step=step).tokens
-                found.append(t.clone())
-                y.scatter_(1, t.long()[:, None], -4.0)
-                found.append(lm.sample(y, params, step=step).tokens)
+    def run(arm, wait):
+        def then(_):
             if wait:
                 torch.cuda.synchronize()
-        return torch.stack([f.long() for f in found])
+        last, t, d = first, iter(tokens[arm]), iter(drawn[arm])
+        for step in range(steps):
+            for params in (p, q, own, q, p, own):                           # the last call's tokens are this one's history
+                now = next(t)
+                then(lm.sample(x, params, history=last[:, None], step=step, out=now))
+                last = now
+            then(lm.argmax(x, out=next(t)))
+            for h in hidden:                                                # logits written over as soon as they have been drawn from
+                then(lm.lm_head(h, weight, out=logits))
+                then(lm.sample(logits, q if step % 2 else p, history=last[:few, None], step=step, out=next(d)))
+                then(lm.argmax(logits, out=next(d)))
 
-    assert torch.equal(run(False), run(True))
+    run(0, False)
+    torch.cuda.synchronize()
+    run(1, True)
+    for a, b in zip(tokens[0] + drawn[0], tokens[1] + drawn[1]):
+        assert torch.equal(a, b)
+    assert len({tuple(v.tolist()) for v in tokens[1][::7]}) > 1             # (the chain moves)
 
 
 @pytest.mark.parametrize("rows,vocab,top_k", [(38, 66001, 50), (64, 262144, 50), (65, 262144, 1000), (74, 151936, 1)])
