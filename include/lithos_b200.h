@@ -55,7 +55,7 @@ extern "C" {
 #define LM_FLAG_TOPP_IN_TOPK 1u /* top-p over the top-k set's renormalised mass (the Hugging Face warpers' order) */
 #define LM_FLAG_EXACT_ONLY 2u /* no candidate lists for rows with a top_k: every row is counted out, by the histogram kernel or (few rows) the cluster kernel's searches (same results) */
 #define LM_FLAG_TOKENS_I64 4u /* lm_sample: out_tokens points to int64_t entries (what the reference's sampler modules return) */
-#define LM_FLAG_GRID_LIMIT(n) (((uint32_t)(n) & 0xFFu) << 8) /* lm_sample: at most n thread blocks at any time (0 = one per SM): leaves SMs to other streams; a call cut into slices is not limited */
+#define LM_FLAG_GRID_LIMIT(n) (((uint32_t)(n) & 0xFFu) << 8) /* lm_sample: at most n thread blocks at any time (0 = one per SM): leaves SMs to other streams; a call of a few rows with one top_k (LM_STATUS_SLICED_PATH) is not limited */
 
 /* per-row status bits written to lm_sample_args.out_status (optional) */
 #define LM_STATUS_GENERIC_PATH 1u /* the row was handled by the generic multi-pass path, or the call asked for statistics or probabilities */
@@ -63,7 +63,8 @@ extern "C" {
 #define LM_STATUS_NEAR_TIE 4u     /* Gumbel draw: best and second-best key closer than 4e-6 (float32 log is library-specific) */
 #define LM_STATUS_TOPP_EDGE 8u    /* top-p: cumulative mass within 1e-12 (relative) of the target at the boundary */
 #define LM_STATUS_CANDIDATE_PATH 64u /* the row was finished by the one-pass candidate path (informational) */
-#define LM_STATUS_SLICED_PATH 256u /* the row was cut into slices over the whole GPU (calls of a few rows; informational) */
+#define LM_STATUS_SLICED_PATH 256u /* a row of a call of at most 32 rows with one top_k of 1 .. 64, finished in pieces by several blocks: slices and a merge (a few rows) or
+                                      the blocks of a cluster (more); instead of LM_STATUS_CANDIDATE_PATH, and not where the generic path took the row (informational) */
 #define LM_STATUS_TILE_DECLINED 128u /* lm_tile_finish only: the row was not sampled (token -1); materialise it and call lm_sample */
 
 #define LM_MAX_VOCAB 1048576

@@ -107,9 +107,9 @@ inline int launch_stream(bool beside, void (*kernel)(K...), dim3 grid, int threa
 
 // ... of a call of few rows, beside its predecessor: only a grid of no more
 // blocks than SMs, or of blocks that need an SM each: placed while others are at work, many small blocks pile up on the SMs that happen to be
-// free (a speculative round's 512 slices: the round 49.2 us so, 45.2 behind the predecessor's end). Calls in a row, us per call so / behind the predecessor's end: greedy,
-// one row 5.9 / 6.2; 4 nucleus rows 32.3 / 33.5; probabilities of 4 rows 21.8 / 23.2; one FP32 row with a top_k 13.5 / 14.5; 64 FP32 rows
-// with mixed knobs 72.9 / 74.8.
+// free (512 blocks of 128 threads behind a draft draw: a speculative round 49 us so, 45 behind the predecessor's end). Calls in a row, us per call so / behind the
+// predecessor's end: 4 nucleus rows 32.5 / 34.0; probabilities of 4 rows 17.8 / 19.6; one FP32 row with a top_k 12.9 / 16.4 (two launches); a
+// speculative round 41.1 / 45.3; 64 FP32 rows with mixed knobs 71.2 / 73.4; the projection of 8 rows 206.9 / 207.7.
 template <class... K, class... A>
 inline int launch_beside(void (*kernel)(K...), dim3 grid, int threads, size_t smem, int C, cudaStream_t st, A... args) {
   int sms = 0;
@@ -123,7 +123,7 @@ inline size_t align256(size_t x) { return (x + 255) & ~static_cast<size_t>(255);
 struct SampleDev;
 struct DraftQDev;
 // cluster.cu: one row per thread-block cluster, every row of the call.
-int sample_clusters(const SampleDev& P, int sms, cudaStream_t st, bool few = false);   // few: the rows report LM_STATUS_SLICED_PATH
+int sample_clusters(const SampleDev& P, int sms, cudaStream_t st, bool few = false);   // few: a call of a few rows with one top_k (LM_STATUS_SLICED_PATH)
 int argmax_clusters(const void* logits, int dtype, int rows, int vocab, int64_t row_stride, int32_t* out32, int64_t* out64, cudaStream_t st);
 int draft_q_clusters(const DraftQDev& P, int sms, cudaStream_t st);
 

@@ -45,7 +45,7 @@ constexpr int kCGroups = 4096;           // group maxima per block
 constexpr int kCMaxBins = 512;           // bins of the group maxima
 constexpr int kCMaxRanks = 16;           // blocks of one cluster
 constexpr int kCQueue = 128;             // logits a warp's queue of the Gumbel draw holds
-constexpr uint32_t kCallOrdered = 1u, kCallFew = 2u;   // of a launch: the rows are taken by kind; the rows report LM_STATUS_SLICED_PATH
+constexpr uint32_t kCallOrdered = 1u, kCallFew = 2u;   // of a launch: the rows are taken by kind; a call of a few rows with one top_k (LM_STATUS_SLICED_PATH)
 constexpr int kOrderRows = 2048;         // rows whose order a block looks up (row_in_order)
 constexpr int kCRankOrder = 320;         // a list up to this long is ordered by counting larger keys, a longer one by bins first
 constexpr double kCMassBand = 1e-11;     // relative error of a logit's fixed-point softmass beyond its rounding: 7e-12 of the polynomial, a few 1e-16
@@ -1418,7 +1418,7 @@ __global__ void __launch_bounds__(B, kPerSM) sample_cluster_kernel(const __grid_
     s.every = max(1, (n_it * B + kCGroups - 1) / kCGroups);
     s.list_n[0] = 0u; s.list_n[1] = 0u;
     s.o_tau = -INFINITY; s.o_token = -1; s.o_weight = 0ull; s.few = (call & kCallFew) != 0u;
-    s.o_status = (s.want_stats ? LM_STATUS_GENERIC_PATH : 0u) | (s.few ? LM_STATUS_SLICED_PATH : 0u);   // (what such calls have always reported)
+    s.o_status = (s.want_stats ? LM_STATUS_GENERIC_PATH : 0u) | (s.few ? LM_STATUS_SLICED_PATH : 0u);   // (statistics: what such calls have always reported)
   }
   {                                                                         // the slice starts its way into L2 (a thread's loads have two chunks in flight)
     const int lo_b = max(0, 8 * c0 - off) * (F32 ? 4 : 2), hi_b = min(V, 8 * c1 - off) * (F32 ? 4 : 2);

@@ -1,4 +1,5 @@
-"""Calls of a few rows: lm_sample cuts every row into slices over the whole GPU (one block per slice, one merge per row).
+"""Calls of at most 32 rows with one top_k: lm_sample cuts every row into slices over the whole GPU (one block per slice, one merge per row) or, from 10 rows on,
+gives it to a cluster of blocks. Either reports STATUS_SLICED_PATH; which kernels run where is asserted below.
 
 The reference's sampler dispatches run on the T <= 8 rows of one decode step (monolith/kernels.py:720-775); its own CPU-runnable
 configuration is a single FP32 row. The results must be the ones of the row-per-block kernels and of the oracle, bit for bit.
@@ -224,8 +225,16 @@ def test_thresholds_at_very_small_temperatures(dtype):
 @pytest.mark.parametrize("rows,vocab,top_k,dtype", [(3, 16384, 20, "bf16"), (4, 151936, 64, "f32"), (5, 151937, 20, "f32"), (9, 151936, 50, "bf16"), (10, 151936, 50, "bf16"),
                                                     (10, 16384, 1, "f32"), (18, 50257, 64, "f32"), (32, 262144, 33, "bf16"), (9, 600000, 20, "bf16"), (5, 1000000, 20, "bf16")])
 def test_slices_to_a_row_by_how_many_rows_there_are(rows, vocab, top_k, dtype):
-    """64, 32 or 16 slices to a row while each has an SM, then a cluster of blocks per row: the same tokens and thresholds, reported the same way."""
+    """64, 32 or 16 slices to a row while each has an SM (and holds its share of the vocabulary), then a cluster of blocks per row: the same tokens and
+    thresholds, reported the same way."""
     x, host = _rows(rows, vocab, rows, dtype)
+    slices = 64
+    while slices > 16 and slices * rows > torch.cuda.get_device_properties(0).multi_processor_count and vocab <= slices // 2 * 32760:
+        slices //= 2
+    cut = slices * rows <= torch.cuda.get_device_properties(0).multi_processor_count
+    p = lm.SamplingParams(temperature=0.8, top_k=top_k, top_p=0.95, seed=3)
+    found = [k[:2] for k in routes.kernels(lambda: lm.sample(x, p))[0]]
+    assert found == [("slice_local_kernel", slices * rows), ("sliced_merge_kernel", rows)] if cut else [k for k, _ in found] == ["sample_cluster_kernel"], found
     for draw in ("inverse_cdf", "gumbel"):
         _check(x, host, draw=draw, temperature=0.8, top_k=top_k, top_p=0.95, min_p=0.001)
     rng = np.random.default_rng(rows)
