@@ -266,14 +266,14 @@ int lm_sample(const lm_sample_args* a) {
       if (rc != LM_OK) return rc;
     } else {
       // Every launch of the call waits on the device for what it needs of the one in front, so that none of them begins with a gap (us per call so /
-      // with a memset and gaps: 256 penalised rows 92.8 / 102.8, 128 rows of 262,144 with a top_k 37.3 / 42.8, 4096 penalised rows 668 / 674).
+      // one after the other: 256 penalised rows 82 / 132, 4096 635 / 703; a memset and gaps in place of the preparation alone were 10 and 6 of it).
       rc = launch_stream(beside, sample_prep_kernel, 1, kPrepThreads, 0, 1, st, P, list_other, counters);
       if (rc != LM_OK) return rc;
       if (one_k || a->rows > static_cast<int64_t>(kOverlapRowsPerSM) * sms) {
         // Many rows per SM, or hardly a row for the histogram kernel (one top_k for all: 148 rows 56 us side by side, 43 so): the top-k kernel first,
         // the histogram kernel behind it with programmatic stream serialization: its blocks take an SM over as the top-k blocks leave it, work
         // through the rows that the preparation has listed for it, wait for the top-k grid, and absorb the few rows that one handed
-        // on. (4096 penalised rows 720 us, behind its end 771; 800 rows 186 and 210.)
+        // on. (4096 penalised rows 635 us, behind its end 700; 800 rows 156 and 193.)
         rc = launch_stream(beside, sample_topk_kernel, grid1, kTB, sizeof(TopkSmem), 1, st, P, list_left, counters, 1);
         if (rc == LM_OK) rc = launch_stream(beside, sample_hist_kernel, grid, kHB, hist_smem, 1, st, P, list_other, counters + kCounterOther, counters + 2, redo, counters + 3,
                                             list_left, counters + 1, counters + 5);
@@ -286,7 +286,7 @@ int lm_sample(const lm_sample_args* a) {
         // kernel takes what the top-k kernel handed on (usually nothing: it leaves at once).
         // With at most kAloneRowsPerSM rows per SM the histogram kernel's blocks ask for so much shared memory that nothing else fits
         // beside them: a long row then has its SM to itself, and the blocks that find no row leave their SM to the top-k kernel at
-        // once (256 rows of the benchmark mix: 106 us per call, 112 without; from 3 rows per SM on it costs time).
+        // once (256 rows of the benchmark mix: 82 us per call, 86 without; from 3 rows per SM on it costs time).
         size_t hist_smem_first = hist_smem; int grid_first = grid;
         if (a->rows <= static_cast<int64_t>(kAloneRowsPerSM) * sms && hist_smem < kAloneSmemBytes) {
           hist_smem_first = kAloneSmemBytes; grid_first = static_cast<int>(a->rows < sms ? a->rows : sms);

@@ -928,7 +928,7 @@ static __device__ void sample_row_hist(const SampleDev& P, int row, int next, Hi
 }
 
 // One block per row in hand, two blocks per SM (vocabularies up to ~200k; one above). Rows cost very different amounts (the
-// draw scales with the kept set), so blocks take them from a counter (`next_item`, zeroed by the host) instead of a fixed
+// draw scales with the kept set), so blocks take them from a counter (`next_item`, zeroed by sample_prep_kernel or a memset) instead of a fixed
 // stride; a block always holds the item after its current one too, so that it can pull that row's history into L2 while it
 // works. With a row list (written by the top-k kernel: the rows it left) the items are entries of the list, without one they
 // are the rows themselves.
@@ -940,7 +940,9 @@ static __global__ void __launch_bounds__(kHB, 2) sample_hist_kernel(SampleDev P,
   __shared__ int item[2];
   // A kernel launched behind this one with programmatic stream serialization (the top-k kernel, which works on other rows and
   // reads nothing this kernel writes) may take every SM a block of this grid has left, instead of waiting for the whole grid. This kernel itself
-  // begins when its predecessor is complete, but for the grid that runs beside the top-k kernel and meets its end below.
+  // begins when its predecessor is complete, but for the grid that runs beside the top-k kernel and meets its end below. What that grid reads before is
+  // sample_prep_kernel's list and counter: the top-k kernel's blocks signal behind their own wait for that grid, so it is complete, and what it wrote
+  // visible, by the time this one can begin.
   if (left == nullptr) after_predecessor(); else asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   apply_step_state(P);
 #pragma unroll 1

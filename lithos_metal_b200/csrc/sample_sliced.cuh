@@ -7,7 +7,8 @@
 //   slice_local_kernel  (16 to 64 slices x rows blocks)  reads its slice ONCE into shared memory (BF16 or FP32, widened; the penalties of
 //                       the history ids that fall into the slice applied), and leaves a record: the slice's maximum, its FP64
 //                       softmass relative to that maximum, and every logit at or above a lower bound of the slice's own k-th
-//                       largest (the k-th largest of the threads' own maxima, to 22 key bits);
+//                       largest (the k-th largest of the threads' own maxima, to a bin of 2047 between the smallest and the largest of
+//                       them; to 22 key bits where that lets through too many);
 //   sliced_merge_kernel (one block per row) the merge that joins the shards of the vocab-parallel mode (vocab_parallel.cuh):
 //                       gathers the candidates of all slices, puts those at or above the row's top-k bound in order, rebuilds
 //                       the row's maximum and mass, thresholds, draw.

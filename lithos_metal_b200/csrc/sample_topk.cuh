@@ -895,7 +895,7 @@ static __device__ bool topk_finish(const SampleDev& P, int row, TopkSmem& c, uin
   return true;
 }
 
-// Rows are handed out through a counter in the workspace (counters[0], zeroed by the host before the launch): a block takes
+// Rows are handed out through a counter in the workspace (counters[0], zeroed by sample_prep_kernel): a block takes
 // the next row, passes over it if it is not this kernel's (sample_prep_kernel has listed it), and else either finishes it or appends it to
 // `list` (length in counters[1]) for the histogram kernel. The order of the list varies from run to run; what is computed per row does not.
 static __global__ void __launch_bounds__(kTB, kTopkPerSM) sample_topk_kernel(SampleDev P, int* list, int* counters, int first) {
