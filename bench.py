@@ -49,22 +49,22 @@ def peaks():
 
 def ncu_traffic():
     """DRAM bytes per row of one sampling call: dram__bytes_read.sum + dram__bytes_write.sum of the top-k kernel and of the
-    histogram kernel, from one ncu capture of the 4096-row workload itself (a call's traffic is this times its rows). The
+    histogram kernel, from one ncu capture of 800 rows of the workload's mix, 243 MB of logits (a call's traffic is this times its rows). The
     figures are typed in from that capture; `captured_at` names the commit whose kernels were captured."""
     return TRAFFIC
 
 
-# (top-k kernel read + write) + (histogram kernel read + write) over the 4096 rows of one call
-TRAFFIC = {"dram_bytes_per_row": (1038539000 + 5840384 + 397207000 + 37092864) / 4096, "captured_at": "89b19b4"}
+# (top-k kernel read + write) + (histogram kernel read + write) over the 800 rows of one call
+TRAFFIC = {"dram_bytes_per_row": (199198976 + 7932416 + 56063232 + 110592) / 800, "captured_at": "0a83bed"}
 
 
 def launches_per_call(lm, rows: int) -> int:
-    """Kernels one lm_sample call launches on this workload (per rank): top-k kernel, histogram kernel, generic kernel; with at
-    most 5 rows per SM the two sampler kernels run side by side and a row-listing kernel plus a second (usually empty) launch
-    of the histogram kernel join them (the rule is lm_sample's, lithos_metal_b200/csrc/lithos_b200.cu)."""
+    """Kernels one lm_sample call launches on this workload (per rank): preparation, top-k kernel, histogram kernel, generic kernel; with at
+    most 5 rows per SM the two sampler kernels run side by side and a second (usually empty) launch of the histogram kernel
+    joins them (the rule is lm_sample's, lithos_metal_b200/csrc/lithos_b200.cu)."""
     from lithos_metal_b200 import _lib
     sms = _lib.lib().lm_device_sm_count()
-    return 3 if rows > 5 * max(sms, 1) else 5
+    return 4 if rows > 5 * max(sms, 1) else 5
 
 
 class ClockSampler:
@@ -319,8 +319,8 @@ def main() -> None:
                         "frac_of_nominal_8TBs": achieved / 8000.0, "algorithmic_bytes_per_row": ROW_BYTES,
                         "traffic": (traffic["dram_bytes_per_row"] * rows if traffic else None)},
            "gpu_launches": launches_per_call(lm, rows) * args.steps, "clocks": clocks.summary()}
-    out["roofline"]["launch"] = ("one sampling call = sample_topk_kernel (rows with a top_k) + sample_hist_kernel (the other rows) + "
-                                 "sample_generic_kernel (rows handed on: none here)" + (" + the row-listing kernel and a second sample_hist_kernel launch "
+    out["roofline"]["launch"] = ("one sampling call = sample_prep_kernel (lists the rows) + sample_topk_kernel (rows with a top_k) + sample_hist_kernel (the other rows) + "
+                                 "sample_generic_kernel (rows handed on: none here)" + (" + a second sample_hist_kernel launch "
                                  "(side-by-side order up to 5 rows per SM)" if launches_per_call(lm, rows) == 5 else "") + "; duration = CUDA events around the call")
 
     if not args.skip_extras:
