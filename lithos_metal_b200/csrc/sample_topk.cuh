@@ -911,6 +911,12 @@ static __global__ void __launch_bounds__(kTB, kTopkPerSM) sample_topk_kernel(Sam
   // claims the one after that at the start of a row, so the counter's round trip hides behind the row. With few rows per block
   // claiming ahead would leave blocks without work while others hold two rows: a block then claims a row when it needs one.
   const bool ahead = P.rows >= 4 * static_cast<int>(gridDim.x);
+  // Up to three eighths more rows than blocks, all of them this kernel's: the second half of the blocks, which share the SMs of the first (blocks go to all
+  // SMs before any has two), leave after a row each, so that a row of the second round has an SM to itself. Else whichever block is done takes the next
+  // row, and the two of an SM are done at about the same time. (One top_k for all, us per call so / else: 310 rows, top_k 50 52.3 / 58.3; 350 rows, 50
+  // 58.4 / 61.0, 100 56.8 / 59.6, 350 63.2 / 67.2; 400 rows, 100 58.4 / 61.9, 400 64.7 / 68.3, 1000 69.8 / 70.2; with half as many again the first half is too
+  // few: 440 rows, top_k 400 74.2 / 64.9.)
+  const bool once = first && P.rows * 8LL <= gridDim.x * 11LL && blockIdx.x >= (gridDim.x + 1u) / 2u;
   if (threadIdx.x == 0) { item[0] = atomicAdd(&counters[0], 1); item[1] = (ahead && item[0] < P.rows) ? atomicAdd(&counters[0], 1) : P.rows; }
   __syncthreads();
   for (;;) {
@@ -923,7 +929,7 @@ static __global__ void __launch_bounds__(kTB, kTopkPerSM) sample_topk_kernel(Sam
       if (threadIdx.x == 0 && !done) list[atomicAdd(&counters[1], 1)] = row;
     }
     __syncthreads();                                                        // nobody reads item[] any more
-    if (threadIdx.x == 0) { item[0] = ahead ? next : atomicAdd(&counters[0], 1); item[1] = fetched; }
+    if (threadIdx.x == 0) { item[0] = once ? P.rows : ahead ? next : atomicAdd(&counters[0], 1); item[1] = fetched; }
     __syncthreads();
   }
   // This grid may have been started before the grid launched ahead of it had finished (programmatic stream serialization). The

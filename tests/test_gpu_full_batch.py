@@ -184,6 +184,20 @@ def test_coarse_logits_stay_on_the_candidate_path(vocab, grid, top_k):
     assert torch.equal(r.tau, exact.tau) and bool(torch.all((r.tokens == exact.tokens) | near))
 
 
+@pytest.mark.parametrize("rows,grid_limit", [(295, 0), (296, 0), (297, 0), (407, 0), (408, 0), (20, 16), (22, 16), (23, 16)])
+def test_every_row_is_taken_where_half_the_blocks_leave_after_one(rows, grid_limit):
+    """Rows up to, and just beyond, eleven eighths of the candidate kernel's blocks (two to each of 148 SMs, or a grid limit): each one is sampled, once and as
+    by the exact kernels."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(rows)
+    x = (torch.randn(rows, 40960, generator=g, device="cuda") * 2).to(torch.bfloat16)
+    p, e = (lm.SamplingParams(temperature=0.8, top_k=30, top_p=0.9, seed=5, exact_only=exact, grid_limit=grid_limit) for exact in (False, True))
+    assert "sample_topk_kernel" in routes.names(lambda: lm.sample(x, p)) or rows < 75
+    out = torch.full((rows,), -7, dtype=torch.int32, device="cuda")
+    r, q = lm.sample(x, p, return_tau=True, return_status=True, out=out), lm.sample(x, e, return_tau=True, return_status=True)
+    assert torch.equal(r.tau, q.tau) and bool(torch.all((r.tokens == q.tokens) | (((r.status | q.status) & 4) != 0)))
+
+
 def test_the_fp32_mass_of_rows_far_from_zero():
     """Logits around 100: the candidate kernel's mass must not carry the rounding of the slope log2(e) / T times the maximum (2e-5 at T 0.3), which
     its band does not hold. top_p a few 1e-6 on either side of a boundary of the cumulative mass inside the top-k set."""
