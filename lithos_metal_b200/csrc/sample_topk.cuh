@@ -357,17 +357,17 @@ static __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem&
     // and at the largest vocabularies a sampled logit stands for 32 (512 rows of 262,144, top_k 1000: 60 rows handed on without that bound, 8 with it).
     const uint32_t most = static_cast<uint32_t>(1500ll * kSampleChunks * kTB * kChunk / V);
     const uint32_t enough = refine ? want + want / 4u : max(want, min(want < 24u ? 2u * want : want + want / 2u, most));
-    uint32_t n_lo = 0xFFFFFFFFu, n_up = 0u;                                 // count(sample >= lo), once it is known; count(sample >= hi + 1)
+    uint32_t n_lo = 0xFFFFFFFFu;                                            // count(sample >= lo), once it is known
     uint32_t lo = 0x0000u, hi = 0x7F7Fu;                                    // invariant: count(sample >= lo) >= want, or lo is still 0 (handed back below)
     const uint32_t prev = c.prev_cut[cls];
     uint32_t n3[3];
     if (prev >= 0x0080u) {                                                  // both ends of the bracket and its middle in one round
       const uint32_t blo = max(prev, 0x0090u) - 16u, bhi = min(prev + 15u, 0x7F7Eu), mid = (blo + bhi + 1u) >> 1;
       count3(blo, mid, bhi + 1u, n3);
-      if (n3[0] < want) { hi = blo - 1u; n_up = n3[0]; }
+      if (n3[0] < want) hi = blo - 1u;
       else if (n3[2] >= want) { lo = bhi + 1u; n_lo = n3[2]; }
-      else if (n3[1] >= want) { lo = mid; hi = bhi; n_lo = n3[1]; n_up = n3[2]; }
-      else { lo = blo; hi = mid - 1u; n_lo = n3[0]; n_up = n3[1]; }
+      else if (n3[1] >= want) { lo = mid; hi = bhi; n_lo = n3[1]; }
+      else { lo = blo; hi = mid - 1u; n_lo = n3[0]; }
     }
     else {
       // The block's first row of its class: the want-th largest of the threads' own maxima has at least `want` samples at or above it, and seldom
@@ -406,8 +406,8 @@ static __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem&
       const uint32_t q2 = min(lo + 6u, hi), q3 = min(lo + 18u, hi);
       count3(lo, q2, q3, n3);
       if (n3[2] >= want) { lo = q3; n_lo = n3[2]; }
-      else if (n3[1] >= want) { lo = q2; hi = q3 - 1u; n_lo = n3[1]; n_up = n3[2]; }
-      else if (n3[0] >= want) { hi = q2 - 1u; n_lo = n3[0]; n_up = n3[1]; }
+      else if (n3[1] >= want) { lo = q2; hi = q3 - 1u; n_lo = n3[1]; }
+      else if (n3[0] >= want) { hi = q2 - 1u; n_lo = n3[0]; }
       else lo = hi = 0u;                                                    // fewer positive samples than wanted
     }
     while (lo < hi && n_lo > enough && probe + 3 <= kSearchProbes) {          // three cuts per round: the range shrinks fourfold
@@ -415,9 +415,9 @@ static __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem&
       const uint32_t q1 = lo + (span + 3u) / 4u, q2 = lo + (2u * span + 3u) / 4u, q3 = lo + (3u * span + 3u) / 4u;   // lo < q1 <= q2 <= q3 <= hi
       count3(q1, q2, q3, n3);
       if (n3[2] >= want) { lo = q3; n_lo = n3[2]; }
-      else if (n3[1] >= want) { lo = q2; hi = q3 - 1u; n_lo = n3[1]; n_up = n3[2]; }
-      else if (n3[0] >= want) { lo = q1; hi = q2 - 1u; n_lo = n3[0]; n_up = n3[1]; }
-      else { hi = q1 - 1u; n_up = n3[0]; }
+      else if (n3[1] >= want) { lo = q2; hi = q3 - 1u; n_lo = n3[1]; }
+      else if (n3[0] >= want) { lo = q1; hi = q2 - 1u; n_lo = n3[0]; }
+      else hi = q1 - 1u;
     }
     cut_code = lo;
     if (cut_code < 0x0080u || (lo < hi && n_lo > enough)) { cp_async_wait<0>(); return false; }   // fewer positive logits than candidates wanted: not this kernel's row
@@ -434,6 +434,9 @@ static __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem&
   // ---- the one pass: note the chunks that hold a logit >= cutoff; FP32 softmass relative to the sampled maximum ----------
   const float M = need_z ? fkey_inv(c.ref_key) : 0.0f;
   const float nb = -M * c2a;
+  // A chunk's terms are added up before they join the thread's sum: as many additions as one after the other, but a term goes through a fourth of them, and
+  // their rounding is most of the band inside which a boundary takes the FP64 mass, 35 us more for its row (151,936 logits: the band is 5.5e-6 of the mass so, 1.4e-5 one
+  // after the other; of 60 calls of 256 penalised rows ten had such a row, now two, and the calls' mean went from 72.1 to 67.5 us). Finer sums -- chunks in fours, or the steps in turn on two or four accumulators -- cost the pass 0.5 to 2 % (4096 penalised rows, us: 634 so, 638, 640 and 647).
   float2 sacc = make_float2(0.0f, 0.0f);
   uint32_t nan_seen = 0u;
   // A bit per step: this thread's chunk held a logit >= cutoff. The list of those chunks is written behind the pass, one reservation per
@@ -460,11 +463,14 @@ static __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem&
       const uint32_t m2 = __hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&w[2]), t2), m3 = __hge2_mask(*reinterpret_cast<const __nv_bfloat162*>(&w[3]), t2);
       hits = (hits << 1) | ((m0 | m1 | m2 | m3) != 0u ? 1ull : 0ull);       // (the padding is below every cutoff)
       if (need_z) {                                                         // (the padding is -inf: weight 0; a NaN or +inf logit poisons the sum)
+        float2 t;
 #pragma unroll
-        for (int k = 0; k < 4; k++) {                                         // two logits per packed multiply-add and per packed add
+        for (int k = 0; k < 4; k++) {
           const float2 x = __ffma2_rn(make_float2(bf16_lo(w[k]), bf16_hi(w[k])), make_float2(c2a, c2a), make_float2(nb, nb));
-          sacc = __fadd2_rn(sacc, make_float2(ex2_approx(x.x), ex2_approx(x.y)));
+          const float2 e = make_float2(ex2_approx(x.x), ex2_approx(x.y));
+          t = k ? __fadd2_rn(t, e) : e;
         }
+        sacc = __fadd2_rn(sacc, t);
       } else {                                                              // no mass wanted: the NaN check on its own
         const __nv_bfloat162 a = __hmax2_nan(*reinterpret_cast<const __nv_bfloat162*>(&w[0]), *reinterpret_cast<const __nv_bfloat162*>(&w[1]));
         const __nv_bfloat162 b = __hmax2_nan(*reinterpret_cast<const __nv_bfloat162*>(&w[2]), *reinterpret_cast<const __nv_bfloat162*>(&w[3]));
@@ -570,7 +576,7 @@ static __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem&
   __syncthreads();
   RowMass zm;
   zm.need = need_z; zm.z_tilde = z_tilde; zm.z_raw = z_raw; zm.z_corr = z_sub + z_add; zm.shift = -static_cast<double>(nb); zm.slope = static_cast<double>(c2a);
-  zm.ref = M; zm.acc_terms = 4.0 * n_it + 1.0; zm.row = rowp; zm.n_chunks = n_chunks; zm.penalised = pen_on;
+  zm.ref = M; zm.acc_terms = n_it + 5.0; zm.row = rowp; zm.n_chunks = n_chunks; zm.penalised = pen_on;
   return topk_finish(P, row, c, cut_code, zm);
 }
 
@@ -585,9 +591,11 @@ static __device__ double topk_exact_mass(const SampleDev& P, TopkSmem& c, const 
   const uint4* p4 = reinterpret_cast<const uint4*>(zm.row);
   const double vmax64 = static_cast<double>(vmax);
   double m = 0.0;
+  uint4 ahead = tid < zm.n_chunks ? __ldg(p4 + tid) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll 1
   for (int cc = tid; cc < zm.n_chunks; cc += kTB) {
-    const uint4 q = __ldg(p4 + cc);
+    const uint4 q = ahead;
+    if (cc + kTB < zm.n_chunks) ahead = __ldg(p4 + cc + kTB);
     const uint32_t bits = zm.penalised ? (c.pen[cc >> 2] >> ((cc & 3) * 8)) & 0xFFu : 0u, w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
     for (int e = 0; e < kChunk; e++) {
@@ -614,8 +622,8 @@ __device__ __forceinline__ double topk_row_total(const RowMass& zm, float vmax, 
   //   - the FMA rounds its result: half an ulp of |x| < 32 is at most 2^-20, a factor 2^(2^-20) = 1 + 6.6e-7 on the term, and D / 16 times
   //     that for the terms up to D above the sampled maximum; the terms below -32 weigh less than V 2^-32 altogether;
   //   - ex2.approx.ftz.f32: 2 ulp = 4 u;
-  //   - each lane accumulates 4 n_it terms one after the other in FP32, then two accumulators and the lanes meet in FP64:
-  //     (4 n_it + 1) u (zm.acc_terms);
+  //   - each lane adds its terms up in FP32, then the lanes meet in FP64: the additions that a term goes through, times u (zm.acc_terms: the
+  //     pass's 3 in a chunk, one a step, the two halves, and one to spare);
   // These are relative to the mass the pass summed (z_raw), which holds the penalised positions at their raw values. The penalised
   // logits then enter as z_raw - z_sub + z_add, every term of z_sub and z_add with the per-term errors above (FMA, ex2, c2a on a
   // single term: 1.6e-6 covers them for |x| < 32); when penalised tokens carried most of the raw mass the band grows with them.
