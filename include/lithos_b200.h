@@ -238,9 +238,10 @@ typedef struct lm_verify_args {
    * prefill branch). A state whose rows do not fit (verify_len > n_draft, t_this_step > n_draft + 1) gets error 4 and done = 1. */
   const void* step_state;
   int32_t t_max, gamma_max;
-  uint32_t wait_limit;         /* polls before a wait between thread blocks gives up; 0 = the default (about 0.1 s) */
-  uint32_t selftest;           /* LM_VERIFY_SELFTEST_WITHHOLD: block 0 withholds its row maxima, so every wait of the launch runs
-                                  out and the error path can be exercised (with a small wait_limit) without hanging anything */
+  uint32_t wait_limit;         /* polls of a row's result before the last of the launch's clusters gives up; 0 = the default (about 0.1 s) */
+  uint32_t selftest;           /* LM_VERIFY_SELFTEST_WITHHOLD: the first row's cluster does not say what it found, so that wait runs
+                                  out and the error path can be exercised (with a small wait_limit) without hanging anything (a launch that
+                                  is given target_vmax and target_mass has no such wait) */
   const float* target_vmax;    /* stochastic mode, optional: [n_draft + 1] (with a step_state: [t_max], indexed like the rows) the exact
                                   maximum of every target row, as the sampler that produced `tau` knows it (the reference's verify
                                   kernels take it from there too: KEPT_STATS, kernels/common/sample.metal:273-303). The launch then

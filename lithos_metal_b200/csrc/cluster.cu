@@ -5,6 +5,7 @@
 #include "draft_q.cuh"
 #include "host.cuh"
 #include "sample_cluster.cuh"
+#include "verify.cuh"
 
 namespace lm {
 
@@ -42,6 +43,7 @@ static int sample_blocks(int64_t rows, int64_t vocab, int sms, bool f32, int lis
 }
 
 // The instances of the sampler: FP32 / BF16 rows, the slices cached in shared memory or not, and then one block per SM or two.
+constexpr size_t kAloneSmem = 116 * 1024;                                  // more than half of an SM's shared memory
 constexpr size_t kMostSmem = 227 * 1024, kHalfSmem = kMostSmem / 2 - 1024;
 struct ClusterPlan { int C; size_t smem; bool cached, two, ordered, few; };
 
@@ -127,6 +129,44 @@ static int launch_draft_q(const DraftQDev& P, int C, cudaStream_t st) {
 int draft_q_clusters(const DraftQDev& P, int sms, cudaStream_t st) {
   const int C = cluster_blocks(P.rows, P.vocab, 2 * sms);                   // (two of these blocks share an SM)
   return P.dtype == LM_DTYPE_F32 ? launch_draft_q<true>(P, C, st) : launch_draft_q<false>(P, C, st);
+}
+
+// The verification: a cluster per target row, as many blocks each as let all of them run at once.
+template <bool F32, int Q>
+static int launch_verify(const VerifyDev& P, int sms, cudaStream_t st) {
+  const KernelSlot slot = static_cast<KernelSlot>(kSlotVerify + (F32 ? 3 : 0) + Q), slot_alone = static_cast<KernelSlot>(kSlotVerify + 6 + (F32 ? 3 : 0) + Q);
+  const void* fn = reinterpret_cast<const void*>(verify_kernel<F32, Q>);
+  static_assert(kVerifySmem < kAloneSmem, "one grant for both");
+  const int rc = ensure_dynamic_smem(slot, fn, kAloneSmem, true);
+  if (rc != LM_OK) return rc;
+  const int rows = P.n_draft + 1;
+  const bool given = P.row_max != nullptr && P.row_mass != nullptr, lean = given && P.draw != LM_DRAW_GUMBEL, few = lean && P.tau != nullptr;
+  auto chunks = [&](int c) { return (static_cast<size_t>((P.vocab + 14) / 8) + c - 1) / c; };   // of a slice, for any alignment of the row
+  auto z_bytes = [&](int c) { return chunks(c) * (lean && !F32 ? 16 : 32) + (chunks(c) + 1) / 2 * 16; };   // (logits, then weights; the chunks' sums)
+  // Where few logits are weighed, a block has its SM to itself (as the draft draw's: the two follow one another in a speculative round), eight to a row where
+  // sixteen would not all run at once (the round of 7 drafts 38.7 us either way). Where the masses are given all but the decisive row's blocks leave early, and
+  // a row gets all the blocks that a cluster can have.
+  int most = cluster_blocks(given ? 1 : rows, P.vocab, 2 * sms);
+  bool alone = false;
+  if (few) {
+    const int c = cluster_that_fits(most, [&](int n) { return clusters_at_once(slot_alone, fn, kVerifyThreads, kAloneSmem, n) >= rows; });
+    alone = c * 2 >= most && z_bytes(c) <= kVerifySmem;
+    if (alone) most = c;
+  }
+  const int at_once = given ? 1 : rows;
+  const int C = cluster_that_fits(most, [&](int c) { return clusters_at_once(slot, fn, kVerifyThreads, kVerifySmem, c) >= at_once; });
+  const size_t z = z_bytes(C), q = Q == 0 || few ? 0 : chunks(C) * 32;       // (the drafter's row, then the residual's weights)
+  const bool z_cached = z <= kVerifySmem, q_cached = q != 0 && (z_cached ? z : 0) + q <= kVerifySmem;
+  const size_t smem = alone ? kAloneSmem : (z_cached ? z : 0) + (q_cached ? q : 0);
+  const unsigned grid = static_cast<unsigned>(rows) * static_cast<unsigned>(C);
+  return launch_stream(given || static_cast<int>(grid) <= sms, verify_kernel<F32, Q>, dim3(grid), kVerifyThreads, smem, C, st, P, C, z_cached ? 1 : 0, q_cached ? 1 : 0);
+}
+
+int verify_clusters(const VerifyDev& P, int sms, cudaStream_t st) {
+  const bool f32 = P.dtype == LM_DTYPE_F32;
+  if (P.mode != LM_VERIFY_STOCHASTIC) return f32 ? launch_verify<true, 0>(P, sms, st) : launch_verify<false, 0>(P, sms, st);
+  if (P.q) return f32 ? launch_verify<true, 1>(P, sms, st) : launch_verify<false, 1>(P, sms, st);
+  return f32 ? launch_verify<true, 2>(P, sms, st) : launch_verify<false, 2>(P, sms, st);
 }
 
 }  // namespace lm

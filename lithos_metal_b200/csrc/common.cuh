@@ -150,17 +150,16 @@ __device__ __forceinline__ uint64_t weight_q40(float z, float vmax, float c) {
   return __float2ull_rz(__fmul_rn(spec_exp2(x), 1099511627776.0f));
 }
 // Two weights at once on the packed binary32 instructions of sm_100 (fma.rn.f32x2 and friends): element for element the
-// operations of weight_q40, so the same bits. (z - vmax is formed as z + (-vmax); the two exact power-of-two scalings, by 2^n
-// and by 2^40, are one multiplication by 2^(n + 40).)
-__device__ __forceinline__ void weight_q40_x2(float z0, float z1, float vmax, float c, uint64_t& w0, uint64_t& w1) {
+// operations of weight_q40 up to its conversion, so the same bits: a weight is the floor of what this returns. (z - vmax is formed as z + (-vmax); the two
+// exact power-of-two scalings, by 2^n and by 2^40, are one multiplication by 2^(n + 40).)
+__device__ __forceinline__ float2 weight_f2(float z0, float z1, float vmax, float c) {
   const float2 x = __fmul2_rn(__fadd2_rn(make_float2(z0, z1), make_float2(-vmax, -vmax)), make_float2(c, c));
-  const float x0 = fminf(x.x, 0.0f), x1 = fminf(x.y, 0.0f);
+  const float x0 = fminf(fmaxf(x.x, -100.0f), 0.0f), x1 = fminf(fmaxf(x.y, -100.0f), 0.0f);   // (at -100 and below, and for a NaN, 2^-60: floor 0, as spec_exp2 has it)
   // round to nearest (ties to even) by adding and subtracting 1.5 * 2^23: for -100 < x <= 0 the sum has an ulp of 1, so this is
   // rintf(x) exactly, and the integer sits in the low bits of the sum (no conversion instructions, which run at a quarter of the rate)
   const float kMagic = 12582912.0f;
   const float2 t = __fadd2_rn(make_float2(x0, x1), make_float2(kMagic, kMagic));
   const float2 n = __fadd2_rn(t, make_float2(-kMagic, -kMagic));
-  const int n0 = __float_as_int(t.x) - 0x4B400000, n1 = __float_as_int(t.y) - 0x4B400000;
   const float2 f = __fadd2_rn(make_float2(x0, x1), make_float2(-n.x, -n.y));
   float2 p = make_float2(0x1.5bba20p-10f, 0x1.5bba20p-10f);
   p = __ffma2_rn(p, f, make_float2(0x1.3cea88p-7f, 0x1.3cea88p-7f));
@@ -168,10 +167,34 @@ __device__ __forceinline__ void weight_q40_x2(float z0, float z1, float vmax, fl
   p = __ffma2_rn(p, f, make_float2(0x1.ebf9bcp-3f, 0x1.ebf9bcp-3f));
   p = __ffma2_rn(p, f, make_float2(0x1.62e42ap-1f, 0x1.62e42ap-1f));
   p = __ffma2_rn(p, f, make_float2(1.0f, 1.0f));
-  const float2 r = __fmul2_rn(p, make_float2(__int_as_float((n0 + 167) << 23), __int_as_float((n1 + 167) << 23)));
-  w0 = (x.x > -100.0f) ? __float2ull_rz(r.x) : 0ull;                        // also NaN: weight 0
-  w1 = (x.y > -100.0f) ? __float2ull_rz(r.y) : 0ull;
+  // (t's bits are 0x4B400000 + n: shifted by 23, the constant is gone and n + 167 is an exponent)
+  return __fmul2_rn(p, make_float2(__int_as_float((__float_as_int(t.x) << 23) + (167 << 23)), __int_as_float((__float_as_int(t.y) << 23) + (167 << 23))));
 }
+__device__ __forceinline__ void weight_q40_x2(float z0, float z1, float vmax, float c, uint64_t& w0, uint64_t& w1) {
+  const float2 r = weight_f2(z0, z1, vmax, c);
+  w0 = __float2ull_rz(r.x); w1 = __float2ull_rz(r.y);
+}
+// The floors of two binary32 x, 0 <= x <= 2^40, without the conversion to 64 bits (which runs at an eighth of the rate): 2^-17 x and what is left of x are
+// rounded down against 2^23, so that the integers lie in the sums' low bits. `top`, `low`: their bit patterns, each less 0x4B000000 an integer; floor =
+// top << 17 | low. Returned: the floors as binary32 where they fit 24 bits (they do for a weight: one below 2^24 is an integer below that, a larger one is x).
+__device__ __forceinline__ float2 floor2(float2 x, uint2& top, uint2& low) {
+  const float2 t = __fadd2_rd(__fmul2_rn(x, make_float2(0x1p-17f, 0x1p-17f)), make_float2(8388608.0f, 8388608.0f));
+  const float2 h = __fadd2_rn(t, make_float2(-8388608.0f, -8388608.0f));
+  const float2 u = __fadd2_rd(__ffma2_rn(h, make_float2(-131072.0f, -131072.0f), x), make_float2(8388608.0f, 8388608.0f));
+  top = make_uint2(__float_as_uint(t.x), __float_as_uint(t.y)); low = make_uint2(__float_as_uint(u.x), __float_as_uint(u.y));
+  return __ffma2_rn(h, make_float2(131072.0f, 131072.0f), __fadd2_rn(u, make_float2(-8388608.0f, -8388608.0f)));
+}
+// A sum of such floors, eight at most at a time (2^26 and 2^20 in all).
+struct FloorSum {
+  uint32_t top = 0u, low = 0u, n = 0u;
+  __device__ __forceinline__ float2 add(float2 x) {
+    uint2 t, l;
+    const float2 w = floor2(x, t, l);
+    top += t.x + t.y; low += l.x + l.y; n += 2u;
+    return w;
+  }
+  __device__ __forceinline__ uint64_t sum() const { return (static_cast<uint64_t>(top - n * 0x4B000000u) << 17) + (low - n * 0x4B000000u); }
+};
 // floor(floor(u * 2^24) * total / 2^24), u clamped to [0, 1 - 2^-24]
 __device__ __forceinline__ uint64_t cdf_target(float u, uint64_t total) {
   long long u24 = (u > 0.0f) ? __float2ll_rz(__fmul_rn(u, 16777216.0f)) : 0ll;
@@ -308,6 +331,7 @@ constexpr double kMassExponent = 0x1p20;
 // key = z / T + g, g = -ln(-ln u), u = (h + 1/2) / 2^23 from 23 bits of the hash. key >= B needs -ln u <= exp(z / T - B), and 1 - u <=
 // -ln u: a logit with (2^23 - h) > 2^23 exp(z / T - B) + 1 cannot reach B. One hash and one ex2 per logit decide that; the few that pass
 // get the exact key. B is a key already seen, less the 4e-6 of the near-tie flag and the rounding of the test itself (kSlack).
+constexpr uint64_t kHashStep = 0x165667B19E3779F9ull;   // (uniform01: what one index adds)
 struct GumbelScan {
   unsigned long long base; float inv_t32, c, kb; uint64_t best; float second;
   __device__ __forceinline__ void init(uint64_t seed, uint32_t step, uint32_t t_id, float T, float key0) {
@@ -321,8 +345,9 @@ struct GumbelScan {
     const float b2 = key * 1.44269504f;
     kb = fminf(kb, (23.0f + 0.02f + fabsf(b2) * 4e-6f) - b2);
   }
-  __device__ __forceinline__ uint32_t bits(uint32_t i) const {
-    uint64_t x = base + static_cast<uint64_t>(i) * 0x165667B19E3779F9ull;
+  __device__ __forceinline__ uint64_t first(int64_t i) const { return base + static_cast<uint64_t>(i) * kHashStep; }   // (i may lie in front of the row)
+  __device__ __forceinline__ uint32_t bits(uint32_t i) const { return bits_of(first(i)); }
+  static __device__ __forceinline__ uint32_t bits_of(uint64_t x) {
     x ^= x >> 30; x *= 0xBF58476D1CE4E5B9ull; x ^= x >> 27; x *= 0x94D049BB133111EBull; x ^= x >> 31;
     return static_cast<uint32_t>(x >> 41) & 0x7FFFFFu;
   }
@@ -337,8 +362,10 @@ struct GumbelScan {
     if (p > best) { if (best) second = fmaxf(second, best_value(best)); best = p; raise(key); } else second = fmaxf(second, key);
   }
   // two logits at once (their hashes are independent chains); z = -inf: none
-  __device__ __forceinline__ void offer2(float z0, uint32_t i0, float z1, uint32_t i1) {
-    const uint32_t h0 = bits(i0), h1 = bits(i1);
+  __device__ __forceinline__ void offer2(float z0, uint32_t i0, float z1, uint32_t i1) { offer2_bits(z0, i0, bits(i0), z1, i1, bits(i1)); }
+  // ... neighbours i, i + 1 whose hashes' arguments (first) are at hand
+  __device__ __forceinline__ void offer2_at(float z0, uint64_t x0, float z1, uint64_t x1, uint32_t i) { offer2_bits(z0, i, bits_of(x0), z1, i + 1u, bits_of(x1)); }
+  __device__ __forceinline__ void offer2_bits(float z0, uint32_t i0, uint32_t h0, float z1, uint32_t i1, uint32_t h1) {
     bool first = within(z0, h0) && z0 > -INFINITY;
     const bool second_too = within(z1, h1) && z1 > -INFINITY;
 #pragma unroll 1
@@ -347,6 +374,40 @@ struct GumbelScan {
       more = first && second_too;
       first = false;
     }
+  }
+};
+
+// The Gumbel-max draw over a residual r > 0 in the place of exp(z / T): key = ln r + g, the logarithms only where 1 - u <= r exp(-B) leaves room for a key of B (a key
+// already seen, less 2e-3 for the rounding of the test).
+struct ResidualScan {
+  unsigned long long base; float room; uint64_t best;                       // room: 2^23 exp(-B)
+  __device__ __forceinline__ void init(uint64_t seed, uint32_t step, uint32_t t_id) {
+    base = seed + static_cast<uint64_t>(step) * 0x9E3779B97F4A7C15ull + static_cast<uint64_t>(t_id) * 0xC2B2AE3D27D4EB4Full;
+    best = 0ull; room = INFINITY;
+  }
+  // Four neighbours i .. i + 3 (room is infinite at first; a residual that is not positive has no key).
+  __device__ __forceinline__ void offer4(const float (&r)[4], int i) {
+    const uint64_t x = base + static_cast<uint64_t>(static_cast<int64_t>(i)) * kHashStep;
+    uint32_t h[4], m = 0u;
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+      h[e] = GumbelScan::bits_of(x + static_cast<uint64_t>(e) * kHashStep);
+      if (r[e] > 0.0f && 16777216.0f - __uint_as_float(0x4B000000u | h[e]) <= __fmaf_rn(r[e], room, 1.0f)) m |= 1u << e;
+    }
+#pragma unroll 1
+    for (; m; m &= m - 1u) {                                                // (the logarithms' code once)
+      const int e = __ffs(static_cast<int>(m)) - 1;
+      const float re = (e & 2) ? ((e & 1) ? r[3] : r[2]) : ((e & 1) ? r[1] : r[0]);
+      const uint32_t he = (e & 2) ? ((e & 1) ? h[3] : h[2]) : ((e & 1) ? h[1] : h[0]);
+      const float u = (static_cast<float>(he) + 0.5f) * (1.0f / 8388608.0f);
+      const uint64_t p = pack_best(__fadd_rn(logf(re), -logf(-logf(u))), static_cast<uint32_t>(i + e));
+      if (p > best) best = p;
+    }
+  }
+  // The best key so far of the whole warp bounds what its lanes look at. `before`: what this lane had.
+  __device__ __forceinline__ void share(uint64_t before) {
+    if (!__any_sync(kFull, best != before)) return;
+    room = fminf(room, 8388608.0f * ex2_approx((2e-3f - best_value(warp_max_u64(best))) * 1.44269504f));
   }
 };
 

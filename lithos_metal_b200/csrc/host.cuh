@@ -33,10 +33,11 @@ inline int sm_count(int* out) {
 // Kernels that need more than 48 KB of shared memory, their static arrays included, must be told so once per device (the attribute belongs to the
 // device's copy of the function). They are told whatever they ask for, so that nothing here has to know their arrays; remembered per device and kernel,
 // raised when a call needs more.
-enum KernelSlot { kSlotFast, kSlotTopk, kSlotGeneric, kSlotVocabLocal, kSlotVerify, kSlotVerifyStats, kSlotTileFinish, kSlotSlice, kSlotSliceSmall, kSlotSliceTiny, kSlotSlicedMerge, kSlotHead, kSlotCluster,
+enum KernelSlot { kSlotFast, kSlotTopk, kSlotGeneric, kSlotVocabLocal, kSlotTileFinish, kSlotSlice, kSlotSliceSmall, kSlotSliceTiny, kSlotSlicedMerge, kSlotHead, kSlotCluster,
                   kSlotArgmax = kSlotCluster + 6,   // (the cluster kernel has six instances, the argmax kernel two)
                   kSlotDraftQ = kSlotArgmax + 2,    // (two instances)
-                  kSlotCount = kSlotDraftQ + 2 };
+                  kSlotVerify = kSlotDraftQ + 2,    // (six, and six for blocks that have an SM to themselves)
+                  kSlotCount = kSlotVerify + 12 };
 
 inline int ensure_dynamic_smem(KernelSlot slot, const void* func, size_t bytes, bool large_clusters = false) {
   constexpr int kMaxDevices = 64;
@@ -64,19 +65,18 @@ template <class Fits> inline int cluster_that_fits(int want, Fits fits) {
   return want;
 }
 
-// Whether the device (a partition of it, a context limited in its SMs) can hold a cluster of C such blocks at all: 16 are beyond what every
-// device guarantees, and a cluster lies within one group of SMs. Asked once per device, kernel and C. The kernel has been let have `smem`.
-inline bool cluster_fits(KernelSlot slot, const void* func, int threads, size_t smem, int C) {
+// How many clusters of C such blocks the device (a partition of it, a context limited in its SMs) can hold at once: 16 are beyond what every
+// device guarantees, and a cluster lies within one group of SMs. Asked once per device, kernel and C (a power of two up to 16). The kernel has been let
+// have `smem`.
+inline int clusters_at_once(KernelSlot slot, const void* func, int threads, size_t smem, int C) {
   constexpr int kMaxDevices = 64;
   static std::mutex mutex;
-  static unsigned char yes[kMaxDevices][kSlotCount] = {}, no[kMaxDevices][kSlotCount] = {};   // a bit per log2 C
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return C <= 8;
-  unsigned char bit = 1;
-  for (int c = C; c > 1; c >>= 1) bit = static_cast<unsigned char>(bit << 1);
+  static int known[kMaxDevices][kSlotCount][5] = {};                        // by log2 C: the number and one more (0: not asked yet)
+  int dev = 0, log2 = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return C <= 8 ? 1 : 0;
+  for (int c = C; c > 1; c >>= 1) log2++;
   std::lock_guard<std::mutex> lock(mutex);
-  if (yes[dev][slot] & bit) return true;
-  if (no[dev][slot] & bit) return false;
+  if (known[dev][slot][log2]) return known[dev][slot][log2] - 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(C)); cfg.blockDim = dim3(static_cast<unsigned>(threads)); cfg.dynamicSmemBytes = smem;
   cudaLaunchAttribute attr[1];
@@ -85,9 +85,10 @@ inline bool cluster_fits(KernelSlot slot, const void* func, int threads, size_t 
   cfg.attrs = attr; cfg.numAttrs = 1;
   int n = 0;
   if (cudaOccupancyMaxActiveClusters(&n, func, &cfg) != cudaSuccess) { n = 0; (void)cudaGetLastError(); }
-  (n > 0 ? yes : no)[dev][slot] |= bit;
-  return n > 0;
+  known[dev][slot][log2] = n + 1;
+  return n;
 }
+inline bool cluster_fits(KernelSlot slot, const void* func, int threads, size_t smem, int C) { return clusters_at_once(slot, func, threads, smem, C) > 0; }
 
 // A launch in clusters of C blocks; beside: it may begin while the kernel in front of it in the stream is still at work (programmatic stream
 // serialization): its blocks are made ready, set up what needs no device memory, and wait (after_predecessor, common.cuh).
@@ -96,11 +97,14 @@ inline int launch_stream(bool beside, void (*kernel)(K...), dim3 grid, int threa
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid; cfg.blockDim = dim3(static_cast<unsigned>(threads)); cfg.dynamicSmemBytes = smem; cfg.stream = st;
   cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = beside ? 1 : 0;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = static_cast<unsigned>(C); attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
-  cfg.attrs = attr; cfg.numAttrs = C > 1 ? 2 : 1;
+  unsigned n = 0;
+  attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[n++].val.programmaticStreamSerializationAllowed = beside ? 1 : 0;
+  if (C > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = static_cast<unsigned>(C); attr[n].val.clusterDim.y = 1; attr[n++].val.clusterDim.z = 1;
+  }
+  cfg.attrs = attr; cfg.numAttrs = n;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...);
   return e == cudaSuccess ? LM_OK : cuda_fail(e);
 }
@@ -122,9 +126,11 @@ inline size_t align256(size_t x) { return (x + 255) & ~static_cast<size_t>(255);
 
 struct SampleDev;
 struct DraftQDev;
+struct VerifyDev;
 // cluster.cu: one row per thread-block cluster, every row of the call.
 int sample_clusters(const SampleDev& P, int sms, cudaStream_t st, bool few = false);   // few: a call of a few rows with one top_k (LM_STATUS_SLICED_PATH)
 int argmax_clusters(const void* logits, int dtype, int rows, int vocab, int64_t row_stride, int32_t* out32, int64_t* out64, cudaStream_t st);
 int draft_q_clusters(const DraftQDev& P, int sms, cudaStream_t st);
+int verify_clusters(const VerifyDev& P, int sms, cudaStream_t st);
 
 }  // namespace lm

@@ -628,24 +628,7 @@ int lm_verify(const lm_verify_args* a) {
                          reinterpret_cast<unsigned long long*>(c->ring), c->ring_cap, EosSet{c->eos, c->eos_list, c->n_eos}, c->log, c->log_cap,
                          c->ctx_cap, c->lm};
   }
-  // one block per SM, all resident at once (the blocks wait for one another's partial results): a cooperative launch guarantees it
-  // (the same grid for every call on a device, whatever the vocabulary: the workspace's launch count is in units of it; blocks
-  // beyond a small vocabulary hold empty slices)
-  const int grid = sms < 256 ? sms : 256;                                  // consume_rows holds rows x grid words in kConsumeSlots per thread
-  // the block's slices of all rows in shared memory when they fit (they do for every vocabulary up to ~700k at 148 SMs)
-  const int per = (static_cast<int>((a->vocab + grid - 1) / grid) + 7) & ~7;
-  const size_t rows_cached = static_cast<size_t>(a->n_draft + 1) + (a->mode == LM_VERIFY_STOCHASTIC ? a->n_draft : 0);
-  size_t smem = rows_cached * static_cast<size_t>(per) * sizeof(float);
-  // a launch that was given the rows' maxima and masses knows the decisive row from one logit per draft and reads no other: nothing to keep in shared memory
-  int cached = (smem <= 200 * 1024 && !(a->mode == LM_VERIFY_STOCHASTIC && a->target_vmax && a->target_mass)) ? 1 : 0;
-  if (!cached) smem = 0;
-  const bool stats = P.row_max != nullptr && P.row_mass != nullptr;
-  const void* kernel = stats ? reinterpret_cast<const void*>(verify_kernel<true>) : reinterpret_cast<const void*>(verify_kernel<false>);
-  rc = ensure_dynamic_smem(stats ? kSlotVerifyStats : kSlotVerify, kernel, smem);
-  if (rc != LM_OK) return rc;
-  void* params[] = {&P, &cached};
-  const cudaError_t e = cudaLaunchCooperativeKernel(const_cast<void*>(kernel), dim3(grid), dim3(kVerifyBlock), params, smem, static_cast<cudaStream_t>(a->stream));
-  return e == cudaSuccess ? LM_OK : cuda_fail(e);
+  return verify_clusters(P, sms, static_cast<cudaStream_t>(a->stream));
 }
 
 int lm_draft_q(const lm_draft_q_args* a) {

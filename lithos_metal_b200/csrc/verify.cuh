@@ -3,52 +3,45 @@
 // probability min(1, p/q), replace the first rejected one by a draw from max(p - q, 0) (kernels/common/sample.metal:273-347),
 // on the integer fixed-point weights so the outcome is independent of how the vocabulary is split between blocks.
 //
-// The step is latency-bound (a few MB of input, a chain of three data dependencies: row maxima -> row masses and the accept
-// test -> the residual's total -> the token), so the kernel is one cooperative launch of one block per SM; every block owns the
-// same vocabulary slice of every row in every phase. Phase 0 is the only one that touches HBM: it pulls the block's slice of
-// all target rows and all draft rows into shared memory (every load in flight at once); the later phases work from there.
-// (A launch that is given the rows' maxima and masses knows the decisive row from one logit per draft and reads only that one, from global
-// memory.)
+// The step is latency-bound (a few MB of input and a chain of dependencies: row maximum -> row mass and accept test -> the
+// residual's total -> the token). A row's chain is its own business but for one bit, whether its draft is accepted. So every target row has a
+// thread-block CLUSTER (16 blocks for up to 14 rows, 8 beyond): its slices of the row and of the drafter's row land in shared memory by asynchronous
+// copies, all in flight at once; the blocks meet in distributed shared memory, a cluster barrier to a dependency; and every row that could be the
+// decisive one -- its own draft rejected, or the bonus row -- draws its token without waiting for the rows before it. What a row found is one word in
+// the workspace; the cluster that arrives last picks the first rejected row and writes the outputs, so no block waits for another cluster.
+// A launch that is given the rows' maxima and masses knows the decisive row from one logit per draft: every block finds it for itself, the
+// other rows' clusters leave, and the decisive one writes the outputs.
+// (All rows cut over all 148 SMs by a cooperative launch, partial results exchanged as polled words in L2, three trips for the step of 7 drafts; us a call so /
+// by clusters, first draft rejected: V = 151,936, drafter's probabilities 25.0 / 18.8, given the maxima 21.0 / 17.6, and the masses 14.0 / 12.9, drafter's logits 27.3 / 20.5, given
+// maxima, masses and thresholds 14.3 / 11.3, greedy 10.3 / 7.4; 13 drafts 31.4 / 22.4; 50,257 24.8 / 13.7; 248,320 29.3 / 22.2, but, of the decisive row alone on 16 SMs, given
+// maxima and masses without thresholds 14.4 / 15.8, and the reference's draw with every draft rejected 29.4 / 32.3. A cooperative launch of the clusters is not made
+// ready beside its predecessor: 1.1 us more. One cluster of 1024 threads a block for the decisive row alone, its slices loaded behind the tests: 1 us more.)
 //
-// Blocks exchange their partial results through TAGGED WORDS in a small workspace: every partial is one 64-bit word whose top
-// bit says "written". A block publishes with one plain store per word and consumes by polling the words it needs, so a
-// dependency costs one trip to L2 and back -- no counter, no fence, no second read. The words live in one of two BANKS. A launch
-// uses the bank its number selects, and every block clears its own words of the other bank while its loads are in flight, so
-// the next launch finds a clean bank and nobody tidies up at the end. The launch number is the count of blocks that have ever
-// left, divided by the grid size: a block adds itself on its way out (no reply awaited), and the quotient cannot change before
-// the last block of the launch has read it. The workspace starts all zero and belongs to one device (one grid size). Every poll
-// is bounded: when it runs out the launch reports an error through its outputs (and through the StepState when it commits); the
-// GPU is never left waiting.
+// A word carries the launch's number, which the last cluster counts up: were one missing, the wait for it is bounded, and the launch reports an error through
+// its outputs (and through the StepState when it commits); the GPU is never left waiting.
 //
 // With a StepState given, the kernel takes the round from it on the device, as the reference's kernels do
 // (kernels/common/sample.metal:283-296): verify length, drafts (pending_tokens), seed, step, and it leaves at once when the
 // state is done. The accept uniforms then come from the reference's stream 3000 + r of the counter-based noise.
 #pragma once
-#include "common.cuh"
+#include "sample_cluster.cuh"
 #include "spec_ops.cuh"
 
 namespace lm {
 
-constexpr int kVerifyBlock = 1024;
-constexpr int kVerifyWarps = kVerifyBlock / 32;
+constexpr int kVerifyThreads = 512;
+constexpr int kVerifyWarps = kVerifyThreads / 32;
 constexpr int kVerifyMaxRows = LM_MAX_DRAFT + 1;
-constexpr int kVerifyMaxGrid = 1024;                    // far above any SM count
-constexpr unsigned kVerifyWaitLimit = 1u << 17;         // polls of one word before a wait gives up: about 0.1 s
-constexpr unsigned long long kTagged = 1ull << 63;
+constexpr unsigned kVerifyWaitLimit = 1u << 17;         // polls of one word before the last cluster gives up: about 0.1 s
+constexpr size_t kVerifySmem = 110 * 1024;              // most shared memory of a block (two to an SM)
 
-struct VerifyBank {
-  unsigned error;                                       // a wait of the launch that used this bank ran out
-  unsigned pad[3];
-  unsigned long long draft_w[kVerifyMaxRows];           // tagged: fixed-point weight of draft r in row r (0 if not kept)
-  unsigned long long best[kVerifyMaxRows][kVerifyMaxGrid];   // tagged: per row and block, the slice's packed (max logit, lowest index)
-  unsigned long long mass[kVerifyMaxRows][kVerifyMaxGrid];   // tagged: per row and block, the slice's fixed-point mass
-  unsigned long long resid[2][kVerifyMaxGrid];          // tagged: per block, the slice's residual mass / its best draw keys
-};
 struct VerifyWs {                                       // lives in the caller's workspace, zero-filled once
-  unsigned long long exits;                             // blocks that have ever left: grid size x launches so far
-  unsigned long long pad;
-  VerifyBank bank[2];
+  unsigned long long launches;                          // so far
+  unsigned arrived, pad;                                // rows of this launch that have been through (0 between launches)
+  unsigned long long row[kVerifyMaxRows];               // what a row's cluster found: launch number << 24 | kFound | rejected << 21 | token + 1
 };
+constexpr unsigned long long kFound = 1ull << 22, kRejected = 1ull << 21;
+static_assert(LM_MAX_VOCAB < (1 << 21), "a token and 'none' fit 21 bits");
 
 struct VerifyDev {
   int mode; int dtype; int n_draft; int vocab; int64_t row_stride; int draw;
@@ -56,69 +49,41 @@ struct VerifyDev {
   const uint16_t* q_logits; int64_t q_logits_stride; const float* q_vmax; const unsigned long long* q_mass;   // q from the drafter's BF16 logits when q is null
   const float* tau; const float* u_accept; const float* u_final;
   const float* row_max;                                  // stochastic mode, optional: the exact maxima of the step's rows (from the sampler): spares the first exchange
-  const unsigned long long* row_mass;                    // ... and their kept sets' fixed-point masses (needs row_max): the accept test needs no exchange at all
+  const unsigned long long* row_mass;                    // ... and their kept sets' fixed-point masses (needs row_max): the decisive row is known at once
   uint64_t seed; uint32_t step;
   int32_t* out_accept; int32_t* out_final; int32_t* out_tokens; float* out_p_draft;
   VerifyWs* ws;
   uint32_t* state; int t_max, g;                          // StepState (optional): the round is read from it
   int commit; AcceptDev accept;                          // commit != 0: close the round on the StepState as accept_scan would
-  unsigned wait_limit; unsigned withhold;                // self-test of the bounded waits: block 0 publishes no row maxima
+  unsigned wait_limit; unsigned withhold;                // self-test of the bounded wait: the first row's cluster does not say what it found
 };
 
-// ---- tagged words ------------------------------------------------------------------------------------------------------------
-// The 52-bit packed (value, lowest index) of the row maxima: indices stay below 2^20 (LM_MAX_VOCAB).
-__device__ __forceinline__ uint64_t pack52(float v, uint32_t idx) { return (static_cast<uint64_t>(fkey(v)) << 20) | (0xFFFFFu - idx); }
-__device__ __forceinline__ float pack52_value(uint64_t p) { return fkey_inv(static_cast<uint32_t>(p >> 20)); }
-__device__ __forceinline__ uint32_t pack52_index(uint64_t p) { return 0xFFFFFu - static_cast<uint32_t>(p & 0xFFFFFu); }
-
-__device__ __forceinline__ void publish(unsigned long long* p, uint64_t v) {
-  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(static_cast<unsigned long long>(v) | kTagged) : "memory");
-}
-__device__ __forceinline__ unsigned long long peek(const unsigned long long* p) {
-  unsigned long long v;
-  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
-}
-// Polls one word until its tag is set; gives up after `limit` polls (then *failed is set and 0 returned). `first`: a value
-// already read from the word.
-__device__ __forceinline__ uint64_t consume(const unsigned long long* p, unsigned limit, bool* failed, unsigned long long first = 0ull) {
-  unsigned long long v = first;
-  for (unsigned spins = 0;; spins++) {
-    if (v & kTagged) return v & ~kTagged;
-    if (spins >= limit) { *failed = true; return 0ull; }
-    if (spins > 64u) __nanosleep(100);                                    // a long wait: leave the memory system to the blocks still working
-    v = peek(p);
+// The binary32 probabilities of weights: fl32(double(w) / double(k)) (prob_q40), two at a time and without FP64. A weight is a binary32 value; 1 / k is split in two of
+// them, so that w * 1 / k is a sum p0 + p1 that is off by less than 2^-46 of it (the product's rounding is taken along by a multiply-add). Where p0 + p1 rounds
+// to the same binary32 with 2^-44 more and less, every value in between does, the quotient and its FP64 rounding among them; else (one in half a million) FP64
+// decides. Nothing is subnormal: w >= 1 or 0, k < 2^64.
+struct ProbScale {
+  float hi, lo; unsigned long long k;
+  __device__ __forceinline__ void init(unsigned long long mass) {
+    k = mass;
+    const double inv = mass ? 1.0 / __ull2double_rn(mass) : 0.0;
+    hi = __double2float_rn(inv); lo = __double2float_rn(inv - static_cast<double>(hi));
   }
-}
-
-__device__ __forceinline__ float verify_load(const VerifyDev& P, int row, int i) {
-  const char* base = static_cast<const char*>(P.target);
-  const float z = (P.dtype == LM_DTYPE_BF16)
-                      ? __uint_as_float(static_cast<uint32_t>(__ldg(reinterpret_cast<const uint16_t*>(base) + static_cast<int64_t>(row) * P.row_stride + i)) << 16)
-                      : __ldg(reinterpret_cast<const float*>(base) + static_cast<int64_t>(row) * P.row_stride + i);
-  return canon_zero(z);
-}
-
-// q_r(v): the drafter's probability of token v at draft position r, as given or from the drafter's logits and row statistics.
-__device__ __forceinline__ float q_from_code(uint32_t code, float vmax, unsigned long long mass, float c2) {
-  return mass ? prob_q40(weight_q40(canon_zero(__uint_as_float(code << 16)), vmax, c2), mass) : 0.0f;
-}
-__device__ __forceinline__ float verify_q(const VerifyDev& P, int r, int i, float c2) {
-  if (P.q) return __ldg(P.q + static_cast<int64_t>(r) * P.q_stride + i);
-  return q_from_code(__ldg(P.q_logits + static_cast<int64_t>(r) * P.q_logits_stride + i), __ldg(P.q_vmax + r), __ldg(P.q_mass + r), c2);
-}
-
-// The block's view of its slice: shared-memory copies when they fit, global memory otherwise. Target rows are step rows
-// (row0 + r), draft rows are draft positions r.
-struct VerifySlice {
-  const VerifyDev* P; const float* zs; const float* qs; int per, lo, row0; float c2;
-  __device__ __forceinline__ float z(int r, int i) const { return zs ? zs[r * per + i] : verify_load(*P, row0 + r, lo + i); }
-  __device__ __forceinline__ float q(int r, int i) const { return qs ? qs[r * per + i] : verify_q(*P, r, lo + i, c2); }
+  static __device__ __noinline__ float exact(float w, unsigned long long k) { return __double2float_rn(__ddiv_rn(static_cast<double>(w), __ull2double_rn(k))); }
+  __device__ __forceinline__ float2 of(float2 w) const {
+    const float2 h = make_float2(hi, hi), l = make_float2(lo, lo);
+    const float2 p0 = __fmul2_rn(w, h), p1 = __ffma2_rn(w, l, __ffma2_rn(w, h, make_float2(-p0.x, -p0.y)));
+    float2 a = __fadd2_rn(p0, __ffma2_rn(p0, make_float2(0x1p-44f, 0x1p-44f), p1));
+    const float2 b = __fadd2_rn(p0, __ffma2_rn(p0, make_float2(-0x1p-44f, -0x1p-44f), p1));
+    if (a.x != b.x) a.x = exact(w.x, k);
+    if (a.y != b.y) a.y = exact(w.y, k);
+    return a;
+  }
 };
 
 // The round's bookkeeping, by the warp whose lane 0 has just written out_tokens: the accept scan on those tokens
 // (kernels/common/spec_ops.metal:148-195). A prefill chunk takes the scan's prefill branch, which reads no token. All 32 lanes call.
-__device__ __forceinline__ void verify_commit(const VerifyDev& P, bool failed) {
+static __device__ __noinline__ void verify_commit(const VerifyDev& P, bool failed) {
   if (!P.commit) return;
   __syncwarp();
   StepStateView st{P.accept.state, P.accept.t_max, P.accept.g};
@@ -132,554 +97,671 @@ __device__ __forceinline__ void verify_commit(const VerifyDev& P, bool failed) {
   round_close(P.accept);
 }
 
-constexpr int kConsumeSlots = 4;                        // words one thread may hold: rows x grid (rounded up to 32) <= 4096
+// What a launch verifies: from its arguments, or from the StepState.
+struct VerifyRound { int L, row0; uint64_t seed; uint32_t step; bool idle, mismatch, prefill; };   // idle: the state is done, or this step is a prefill chunk
 
-// Consumes words[r][g] for r < R, g < G (row stride kVerifyMaxGrid) and reduces each row over g (SUM false: maximum, true:
-// sum) into out[r] (shared memory). Warps take 32 consecutive blocks of one row at a time. The values a thread consumed stay
-// in vals[] (0 where it had none), vals[k] belonging to word k * kVerifyBlock + tid of the R x Gp index space. Every thread calls.
-template <bool SUM>
-__device__ __forceinline__ void consume_rows(const unsigned long long* words, int R, int G, unsigned long long* out, uint64_t (*red)[32],
-                                             unsigned limit, bool* failed, uint64_t vals[kConsumeSlots]) {
-  const int tid = threadIdx.x, lane = tid & 31;
-  const int Gp = (G + 31) & ~31, n = R * Gp;
-  // Every word of this thread is in flight at once, on the first look and on every further one: a word that is not there yet
-  // costs one more round trip for all of the thread's words together, not one each.
-  const unsigned long long* addr[kConsumeSlots];
-  unsigned long long got[kConsumeSlots];
-#pragma unroll
-  for (int k = 0; k < kConsumeSlots; k++) {
-    const int idx = k * kVerifyBlock + tid, r = idx / Gp, g = idx - r * Gp;
-    addr[k] = (idx < n && g < G) ? words + static_cast<size_t>(r) * kVerifyMaxGrid + g : nullptr;
-    got[k] = addr[k] ? peek(addr[k]) : kTagged;
-  }
-  for (unsigned spins = 0;; spins++) {
-    bool all = true;
-#pragma unroll
-    for (int k = 0; k < kConsumeSlots; k++) all = all && (got[k] & kTagged) != 0ull;
-    if (all) break;
-    if (spins >= limit) { *failed = true; break; }
-    if (spins > 64u) __nanosleep(100);                                    // a long wait: leave the memory system to the blocks still working
-#pragma unroll
-    for (int k = 0; k < kConsumeSlots; k++) if (!(got[k] & kTagged)) got[k] = peek(addr[k]);
-  }
-#pragma unroll
-  for (int k = 0; k < kConsumeSlots; k++) {
-    const int idx = k * kVerifyBlock + tid, r = idx / Gp, g = idx - r * Gp;
-    const uint64_t v = (got[k] & kTagged) ? (got[k] & ~kTagged) : 0ull;
-    vals[k] = v;
-    if (k * kVerifyBlock < n) {                                           // block-uniform
-      const uint64_t w = SUM ? warp_sum_u64(v) : warp_max_u64(v);
-      if (lane == 0 && idx < n) red[r][g >> 5] = w;
-    }
-  }
-  __syncthreads();
-  if (tid < R) {
-    uint64_t acc = 0ull;
-    for (int k = 0; k < Gp / 32; k++) { const uint64_t x = red[tid][k]; acc = SUM ? acc + x : (x > acc ? x : acc); }
-    out[tid] = acc;
-  }
-  __syncthreads();
+__device__ __forceinline__ int verify_draft(const VerifyDev& P, const VerifyRound& rd, int r) {
+  return P.state ? StepStateView{P.state, P.t_max, P.g}.pending(rd.row0 + r + 1) : P.drafts[r];
 }
 
-// kStats: the launch was given the rows' maxima and masses (compiled apart: the launch that has to find them runs code that is
-// laid out as if the other did not exist, and the step is short enough for that to show).
-template <bool kStats>
-__global__ void __launch_bounds__(kVerifyBlock, 1) verify_kernel(VerifyDev P, int cached) {
-  extern __shared__ __align__(16) float v_smem[];
-  __shared__ uint64_t scratch[32];
-  __shared__ uint64_t s_red[kVerifyMaxRows][32];
-  __shared__ int s_j, s_token, s_j2;
-  __shared__ unsigned long long s_pre2;
-  __shared__ int s_drafts[kVerifyMaxRows];
-  __shared__ unsigned long long s_best[kVerifyMaxRows], s_mass[kVerifyMaxRows], s_own[kVerifyMaxRows];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, G = gridDim.x, b = blockIdx.x;
-  const int V = P.vocab;
-  const bool stochastic = P.mode == LM_VERIFY_STOCHASTIC;
-  const bool gumbel_draw = stochastic && P.draw == LM_DRAW_GUMBEL;
-  // the bank of this launch (the load is in flight under phase 0; its value is first needed when the row maxima are published)
-  unsigned long long launches;
-  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(launches) : "l"(&P.ws->exits) : "memory");
-  const unsigned bank_id = static_cast<unsigned>((launches / static_cast<unsigned long long>(G)) & 1ull);
-  VerifyBank* ws = &P.ws->bank[bank_id];
+// The outputs, by one warp, and the round closed on them.
+static __device__ __noinline__ void verify_outputs(const VerifyDev& P, const VerifyRound& rd, bool bad, int accept, int token) {
+  const int lane = threadIdx.x & 31;
+  if (lane == 0) { P.out_accept[0] = bad ? -1 : accept; P.out_final[0] = bad ? -1 : token; }
+  if (P.out_tokens && lane <= rd.L) P.out_tokens[rd.row0 + lane] = bad ? -1 : (lane < accept ? verify_draft(P, rd, lane) : (lane == accept ? token : -1));
+  verify_commit(P, bad);
+}
+
+// A row is through (one warp of its cluster): what it found, and if it is the last of the launch the outputs.
+static __device__ __noinline__ void verify_arrive(const VerifyDev& P, const VerifyRound& rd, int r, unsigned long long launch, bool rejected, int token) {
+  const int lane = threadIdx.x & 31;
+  VerifyWs* ws = P.ws;
+  unsigned before = 0u;
+  if (lane == 0) {
+    if (!(P.withhold && r == 0))
+      asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(&ws->row[r]),
+                   "l"((launch << 24) | kFound | (rejected ? kRejected : 0ull) | static_cast<unsigned long long>(static_cast<uint32_t>(token + 1))) : "memory");
+    asm volatile("atom.add.relaxed.gpu.global.u32 %0, [%1], 1;" : "=r"(before) : "l"(&ws->arrived) : "memory");
+  }
+  if (__shfl_sync(kFull, before, 0) != static_cast<unsigned>(rd.L)) return;
+  // every row of the launch has been through: a lane per row (a word says itself that it is there, so nothing has to be ordered by fences: they cost 1.3 us)
   const unsigned limit = P.wait_limit ? P.wait_limit : kVerifyWaitLimit;
-  bool failed = false;
+  unsigned long long word = 0ull;
+  bool late = false;
+  if (lane <= rd.L) for (unsigned spins = 0;; spins++) {
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(word) : "l"(&ws->row[lane]) : "memory");
+    if ((word >> 24) == launch && (word & kFound)) break;
+    if (spins >= limit) { late = true; break; }
+    if (spins > 64u) __nanosleep(100);
+  }
+  const bool bad = __any_sync(kFull, late) != 0;
+  const uint32_t rejects = __ballot_sync(kFull, lane < rd.L && (word & kRejected));
+  const int j = rejects ? __ffs(static_cast<int>(rejects)) - 1 : rd.L;
+  const int drawn = __shfl_sync(kFull, static_cast<int>(word & (kRejected - 1ull)) - 1, j);
+  if (lane == 0) { ws->arrived = 0u; ws->launches = launch + 1ull; }
+  verify_outputs(P, rd, bad, j, drawn);
+}
 
-  // ---- the round: from the arguments, or from the StepState ---------------------------------------------------------------
-  int L = P.n_draft, row0 = 0;
-  uint64_t seed = P.seed; uint32_t step = P.step;
-  bool idle = false, mismatch = false;                                    // idle: the state is done, or this step is a prefill chunk
-  bool prefill = false;
-  if (P.state) {
-    StepStateView st{P.state, P.t_max, P.g};
-    if (st.done()) idle = true;
-    else if (st.prefill_left() > 0u) { idle = true; prefill = true; }
-    else {
-      const uint32_t len = st.verify_len(), rows = st.t_this_step();
-      if (len > static_cast<uint32_t>(P.n_draft) || rows < len + 1u || rows > static_cast<uint32_t>(P.n_draft) + 1u) mismatch = true;
-      else { L = static_cast<int>(len); row0 = static_cast<int>(rows - 1u - len); }
-    }
-    seed = st.seed(); step = st.step();
-  }
-  const int R = L + 1;
-  // this block's words of the other bank (the previous launch's) are cleared for the next launch; block 0 also clears the shared ones
-  auto clean_other_bank = [&]() {
-    VerifyBank* other = &P.ws->bank[bank_id ^ 1u];
-    if (tid < kVerifyMaxRows) { other->best[tid][b] = 0ull; other->mass[tid][b] = 0ull; }
-    if (tid < 2) other->resid[tid][b] = 0ull;
-    if (b == 0 && tid < kVerifyMaxRows) other->draft_w[tid] = 0ull;
-    if (b == 0 && tid == 0) other->error = 0u;
-  };
-  if (idle || mismatch) {
-    clean_other_bank();                                                   // (the launch still counts: the banks keep alternating)
-    // nothing is verified; block 0 still closes a prefill chunk (the scan's prefill branch) or reports the caller's error
-    if (b == 0 && warp == 0) {
-      if (mismatch) {
-        if (lane == 0) { P.out_accept[0] = -1; P.out_final[0] = -1; StepStateView st{P.state, P.t_max, P.g}; fail_state(st, kErrRoundMismatch); }
-      } else if (prefill) verify_commit(P, false);
-    }
-  } else {
-  // this block's vocabulary slice, a multiple of 8 elements
-  const int per = ((V + G - 1) / G + 7) & ~7;
-  const int lo = min(V, b * per), hi = min(V, lo + per);
-  const int len = hi - lo;
-  const int chunks = (len + 7) / 8;                                        // 8-element load items of one row of the slice
-  float* zs = cached ? v_smem : nullptr;
-  float* qs = (cached && stochastic) ? v_smem + (P.n_draft + 1) * per : nullptr;
-  const float c2 = stochastic ? exp2_scale(P.temperature) : 0.0f;
-  VerifySlice S{&P, zs, qs, per, lo, row0, c2};
-
-  const bool given_max = kStats || (stochastic && P.row_max != nullptr);              // the sampler already knows the rows' maxima: nothing to find or exchange
-  const bool given_mass = kStats;                                         // ... and the masses of their kept sets: only the draw is left to do together
-
-  // ---- phase 0: the only HBM pass. Slices of every target row and every draft row into shared memory.
-  // The scalars the accept test needs later are fetched now, so their latency hides behind the slice loads.
-  int my_draft = -1; float my_q = 0.0f, my_u = 0.0f;
-  if (tid < L) {
-    my_draft = P.state ? StepStateView{P.state, P.t_max, P.g}.pending(row0 + tid + 1) : P.drafts[tid];
-    s_drafts[tid] = my_draft;
-  }
-  if (stochastic && tid < L) {
-    my_u = P.u_accept ? P.u_accept[tid] : uniform01(seed, step, 3000u + static_cast<uint32_t>(tid), 0u);
-    if (my_draft >= 0 && my_draft < V) my_q = verify_q(P, tid, my_draft, c2);
-  }
-  unsigned long long my_mass = 0ull; float my_zd = -INFINITY;              // given the masses: the row's mass and the draft's own logit, fetched now too
-  if (given_mass) {
-    if (tid < R) my_mass = P.row_mass[row0 + tid];
-    if (tid < L && my_draft >= 0 && my_draft < V) my_zd = verify_load(P, row0 + tid, my_draft);
-  }
-  if (cached) {
-    // 8 elements per load item (one 16-byte load of BF16 logits, two of FP32 logits or draft probabilities), every item of
-    // a thread issued before the first is used: the whole slice arrives in one memory round trip
-    const int n_q = stochastic ? L : 0;
-    const bool z_vec = (P.dtype == LM_DTYPE_BF16 ? (P.row_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(P.target) & 15u) == 0)
-                                                 : (P.row_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(P.target) & 15u) == 0));
-    const bool q_vec = n_q == 0 || (P.q ? (P.q_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(P.q) & 15u) == 0)
-                                        : (P.q_logits_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(P.q_logits) & 15u) == 0));
-    const int n_items = (R + n_q) * chunks;
-    constexpr int kItems = 3;                                             // items in flight per thread
-    for (int i0 = 0; i0 < n_items; i0 += kItems * kVerifyBlock) {
-      float4 va[kItems], vb[kItems];
+// Half h (four elements) of chunk c of a binary32 row, the whole chunk of a BF16 row, from global memory: rows that do not fit shared memory, and first or last
+// chunks. Positions outside the row: -inf of a target row, nothing of a drafter's.
+template <bool F32>
+static __device__ __noinline__ uint4 verify_far(const char* row, int off, int V, int c, int h, bool vec, uint32_t outside) {
+  const int base = 8 * c - off + (F32 ? 4 * h : 0);
+  if (vec && base >= 0 && base + (F32 ? 4 : 8) <= V) return __ldg(reinterpret_cast<const uint4*>(row + static_cast<int64_t>(base) * (F32 ? 4 : 2)));
+  uint32_t w[4];
 #pragma unroll
-      for (int k = 0; k < kItems; k++) {
-        const int item = i0 + k * kVerifyBlock + tid;
-        va[k] = make_float4(0.f, 0.f, 0.f, 0.f); vb[k] = va[k];
-        const int r = item / chunks, ci = item - r * chunks, c8 = ci * 8;
-        if (item >= n_items) continue;
-        const bool full = c8 + 8 <= len;
-        if (r < R) {
-          if (P.dtype == LM_DTYPE_BF16) {
-            const uint16_t* src = reinterpret_cast<const uint16_t*>(P.target) + static_cast<int64_t>(row0 + r) * P.row_stride + lo + c8;
-            if (full && z_vec) va[k] = __ldg(reinterpret_cast<const float4*>(src));      // eight BF16 codes, widened below
-          } else {
-            const float* src = reinterpret_cast<const float*>(P.target) + static_cast<int64_t>(row0 + r) * P.row_stride + lo + c8;
-            if (full && z_vec) { va[k] = __ldg(reinterpret_cast<const float4*>(src)); vb[k] = __ldg(reinterpret_cast<const float4*>(src) + 1); }
-          }
-        } else if (P.q) {
-          const float* src = P.q + static_cast<int64_t>(r - R) * P.q_stride + lo + c8;
-          if (full && q_vec) { va[k] = __ldg(reinterpret_cast<const float4*>(src)); vb[k] = __ldg(reinterpret_cast<const float4*>(src) + 1); }
-        } else {
-          const uint16_t* src = P.q_logits + static_cast<int64_t>(r - R) * P.q_logits_stride + lo + c8;
-          if (full && q_vec) va[k] = __ldg(reinterpret_cast<const float4*>(src));          // eight BF16 codes of the drafter's row
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < kItems; k++) {
-        const int item = i0 + k * kVerifyBlock + tid;
-        if (item >= n_items) continue;
-        const int r = item / chunks, ci = item - r * chunks, c8 = ci * 8;
-        const bool full = c8 + 8 <= len;
-        float* dst = (r < R ? zs + r * per : qs + (r - R) * per) + c8;
-        const bool vec = full && (r < R ? z_vec : q_vec);
-        if (!vec) {                                                       // a ragged last chunk or an unaligned tensor: element by element
-          for (int e = 0; e < 8 && c8 + e < len; e++)
-            dst[e] = r < R ? verify_load(P, row0 + r, lo + c8 + e) : verify_q(P, r - R, lo + c8 + e, c2);
-          continue;
-        }
-        float4 x = va[k], y = vb[k];
-        if (r >= R && !P.q) {                                             // the drafter's logits: probabilities from the row statistics
-          const float qv = __ldg(P.q_vmax + (r - R)); const unsigned long long qm = __ldg(P.q_mass + (r - R));
-          const uint32_t w0 = __float_as_uint(va[k].x), w1 = __float_as_uint(va[k].y), w2 = __float_as_uint(va[k].z), w3 = __float_as_uint(va[k].w);
-          x = make_float4(q_from_code(w0 & 0xFFFFu, qv, qm, c2), q_from_code(w0 >> 16, qv, qm, c2), q_from_code(w1 & 0xFFFFu, qv, qm, c2), q_from_code(w1 >> 16, qv, qm, c2));
-          y = make_float4(q_from_code(w2 & 0xFFFFu, qv, qm, c2), q_from_code(w2 >> 16, qv, qm, c2), q_from_code(w3 & 0xFFFFu, qv, qm, c2), q_from_code(w3 >> 16, qv, qm, c2));
-        }
-        if (r < R && P.dtype == LM_DTYPE_BF16) {
-          const uint32_t w0 = __float_as_uint(va[k].x), w1 = __float_as_uint(va[k].y), w2 = __float_as_uint(va[k].z), w3 = __float_as_uint(va[k].w);
-          x = make_float4(bf16_lo(w0), bf16_hi(w0), bf16_lo(w1), bf16_hi(w1));
-          y = make_float4(bf16_lo(w2), bf16_hi(w2), bf16_lo(w3), bf16_hi(w3));
-        }
-        if (r < R) {
-          x = make_float4(canon_zero(x.x), canon_zero(x.y), canon_zero(x.z), canon_zero(x.w));
-          y = make_float4(canon_zero(y.x), canon_zero(y.y), canon_zero(y.z), canon_zero(y.w));
-        }
-        reinterpret_cast<float4*>(dst)[0] = x; reinterpret_cast<float4*>(dst)[1] = y;
-      }
-    }
-    __syncthreads();
+  for (int k = 0; k < 4; k++) {
+    auto at = [&](int i) {
+      if (i < 0 || i >= V) return outside;
+      return F32 ? __ldg(reinterpret_cast<const uint32_t*>(row) + i) : static_cast<uint32_t>(__ldg(reinterpret_cast<const uint16_t*>(row) + i));
+    };
+    w[k] = F32 ? at(base + k) : at(base + 2 * k) | (at(base + 2 * k + 1) << 16);
   }
-  // ---- row maxima of the slice (lowest index on ties: the greedy pick), published one word per row -----------------------
-  // A block of 1024 threads keeps every scheduler of the SM busy, so what counts is the total number of instructions: the rows
-  // are walked four elements per shared-memory load, a warp staying inside one row (rows padded to 32 groups of four), and only
-  // the warps that hold data reduce.
-  const int n4 = (len + 3) / 4, n4p = (n4 + 31) & ~31;                      // groups of four elements per row of the slice
-  const int split = max(1, kVerifyWarps / R);                              // without the shared-memory copy every row is shared by `split` warps
-  const int n_red = cached ? n4p / 32 : split;                             // partial results per row in s_red
-  if (given_max) {
-    if (tid < R) s_best[tid] = pack52(canon_zero(P.row_max[row0 + tid]), 0u);
-  } else if (cached) {
-    // stochastic: the value alone (a 32-bit key); greedy: value and lowest index together (the 52-bit pack)
-    for (int i0 = 0; i0 < R * n4p; i0 += kVerifyBlock) {
-      const int r0 = (i0 + (tid & ~31)) / n4p;
-      if (r0 >= R) break;                                                 // warp-uniform
-      const int item = i0 + tid, c4 = item - r0 * n4p;
-      const int left = len - 4 * c4;                                      // 4 except in a ragged last group
-      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (c4 < n4) x = reinterpret_cast<const float4*>(zs + r0 * per)[c4];
-      if (stochastic) {
-        uint32_t key = 0u;
-        if (c4 < n4) {
-          key = fkey(x.x);
-          if (left > 1) key = max(key, fkey(x.y));
-          if (left > 2) key = max(key, fkey(x.z));
-          if (left > 3) key = max(key, fkey(x.w));
-        }
-        key = warp_max_u32(key);
-        if (lane == 0) s_red[r0][c4 >> 5] = static_cast<uint64_t>(key) << 20;
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// What a row's chunks are weighed with; kept in shared memory for verify_half.
+struct VerifyRow {
+  const char* q_row; uint4* qs; int off, V, per; bool q_cached, q_vec, cut; float c2, tau, qv; ProbScale p_of, q_of;
+};
+struct VerifySmem {
+  unsigned long long x_best[kCMaxRanks], x_own[kCMaxRanks], x_res[kCMaxRanks];   // what the blocks of the cluster leave in one another's copy
+  uint64_t best[kVerifyWarps], own[kVerifyWarps], res[kVerifyWarps];             // this block's, per warp
+  VerifyRow row; int j; bool reject;
+};
+
+// The logits of half h of a chunk in pairs (v: the half of a binary32 row, the chunk of a BF16 row), -0 as +0; -inf outside the row.
+template <bool F32>
+__device__ __forceinline__ void verify_pairs(uint4 v, int h, float2 (&z)[2]) {
+  if (F32) { z[0] = make_float2(__uint_as_float(v.x), __uint_as_float(v.y)); z[1] = make_float2(__uint_as_float(v.z), __uint_as_float(v.w)); }
+  else {
+    const uint32_t a = h ? v.z : v.x, b = h ? v.w : v.y;
+    z[0] = make_float2(bf16_lo(a), bf16_hi(a)); z[1] = make_float2(bf16_lo(b), bf16_hi(b));
+  }
+#pragma unroll
+  for (int k = 0; k < 2; k++) z[k] = __fadd2_rn(z[k], make_float2(0.0f, 0.0f));
+}
+
+// What half a chunk weighs in the draw, before the floors: the kept set's weights (what lies outside the row is -inf: 0), or with `residual` what max(p - q, 0)
+// leaves of them (what is not kept has weight 0, hence p = 0 and nothing left). stored: v holds the floors of the weights already. For what is rare: slices that do
+// not fit shared memory, and the second look where a residual is empty.
+template <bool F32, int Q>
+static __device__ __noinline__ float4 verify_half(const VerifyRow& x, uint4 v, int c, int h, bool stored, bool residual, float vmax) {
+  float2 w[2];
+  if (stored) { w[0] = make_float2(__uint_as_float(v.x), __uint_as_float(v.y)); w[1] = make_float2(__uint_as_float(v.z), __uint_as_float(v.w)); }
+  else {
+    float2 z[2];
+    verify_pairs<F32>(v, h, z);
+    const float tau = x.tau, c2 = x.c2;
+    if (x.cut && !(fmaxf(fmaxf(z[0].x, z[0].y), fmaxf(z[1].x, z[1].y)) >= tau)) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      const float2 y = weight_f2(z[k].x, z[k].y, vmax, c2);
+      w[k] = make_float2(z[k].x >= tau ? y.x : 0.0f, z[k].y >= tau ? y.y : 0.0f);
+    }
+  }
+  if (Q == 0 || !residual || !(__float_as_uint(w[0].x) | __float_as_uint(w[0].y) | __float_as_uint(w[1].x) | __float_as_uint(w[1].y))) return make_float4(w[0].x, w[0].y, w[1].x, w[1].y);
+  uint2 t, l;
+  float2 q[2];
+  const uint4 qr = x.q_cached ? x.qs[(Q == 1 && h ? x.per : 0) + c] : verify_far<Q == 1>(x.q_row, x.off, x.V, c, h, x.q_vec, Q == 1 ? 0u : 0xFF80u);
+  if (Q == 1) { q[0] = make_float2(__uint_as_float(qr.x), __uint_as_float(qr.y)); q[1] = make_float2(__uint_as_float(qr.z), __uint_as_float(qr.w)); }
+  else {
+    verify_pairs<false>(qr, h, q);
+    const ProbScale q_of = x.q_of;
+#pragma unroll
+    for (int k = 0; k < 2; k++) q[k] = q_of.of(floor2(weight_f2(q[k].x, q[k].y, x.qv, x.c2), t, l));
+  }
+  const ProbScale p_of = x.p_of;
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    if (!stored) w[k] = floor2(w[k], t, l);
+    const float2 d = __fadd2_rn(p_of.of(w[k]), make_float2(-q[k].x, -q[k].y));
+    w[k] = __fmul2_rn(make_float2(w[k].x > 0.0f ? fmaxf(d.x, 0.0f) : 0.0f, w[k].y > 0.0f ? fmaxf(d.y, 0.0f) : 0.0f), make_float2(1099511627776.0f, 1099511627776.0f));
+  }
+  return make_float4(w[0].x, w[0].y, w[1].x, w[1].y);
+}
+
+// The same of one element of the row (its index i, its logit z >= the threshold), as an integer: where few are kept, a lane takes one of them at a time.
+template <bool F32, int Q>
+static __device__ __noinline__ uint64_t verify_element(const VerifyRow& x, int i, float z, bool residual, float vmax) {
+  const uint32_t qr = !residual ? 0u : Q == 1 ? __ldg(reinterpret_cast<const uint32_t*>(x.q_row) + i) : static_cast<uint32_t>(__ldg(reinterpret_cast<const uint16_t*>(x.q_row) + i)) << 16;
+  const uint64_t w = weight_q40(z, vmax, x.c2);
+  if (!residual) return w;
+  const float p = prob_q40(w, x.p_of.k);
+  float q = __uint_as_float(qr);
+  if (Q == 2) q = x.q_of.k ? prob_q40(weight_q40(canon_zero(q), x.qv, x.c2), x.q_of.k) : 0.0f;
+  const float d = __fsub_rn(p, q);
+  return d > 0.0f ? residual_q40(d) : 0ull;
+}
+
+// Every warp for itself: the slots' sum, and the sum of the slots before slot `at`.
+__device__ __forceinline__ uint64_t verify_prefix(const unsigned long long* slots, int n, int at, uint64_t* before) {
+  const int lane = threadIdx.x & 31;
+  const uint64_t mine = lane < n ? slots[lane] : 0ull;
+  uint64_t incl = mine;
+#pragma unroll
+  for (int o = 1; o < kCMaxRanks; o <<= 1) { const uint64_t t = __shfl_up_sync(kFull, incl, o); if (lane >= o) incl += t; }
+  *before = __shfl_sync(kFull, incl - mine, at);
+  return __shfl_sync(kFull, incl, kCMaxRanks - 1);
+}
+static_assert(kVerifyWarps <= kCMaxRanks && kCMaxRanks <= 32, "slots of ranks and of warps alike, a lane each");
+
+// One row by one cluster. Q: 0 greedy, 1 the drafter's probabilities, 2 its BF16 logits and their statistics. Every part of this runs a few times a launch, so
+// code that is not in the instruction cache costs as much as what it computes: a loop's chunk is unrolled, loops are not, what has been computed is kept rather
+// than computed by a second copy of the code (the token was found in 2.5 to 3.3 us so, in 1 with the draw's weights kept), and the rare is in functions of its own.
+template <bool F32, int Q>
+__device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound& rd, int r, int rank, int C, unsigned long long launch, bool z_cached, bool q_cached,
+                                           uint4* zs, VerifySmem& s) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int kSize = F32 ? 4 : 2;
+  const int V = P.vocab, L = rd.L, row = rd.row0 + r;
+  const bool has_q = Q != 0 && r < L;
+  const bool given_max = Q != 0 && P.row_max != nullptr, given_mass = given_max && P.row_mass != nullptr;
+  // ---- this block's slice in chunks of eight; a warp's are consecutive, so that what a warp holds is a range of the row ------------------------
+  const char* z_row = static_cast<const char*>(P.target) + static_cast<size_t>(row) * static_cast<size_t>(P.row_stride) * kSize;
+  const int head = static_cast<int>((16u - (reinterpret_cast<uintptr_t>(z_row) & 15u)) & 15u) / kSize;
+  const int off = head ? 8 - head : 0, n_chunks = (V + off + 7) / 8, per = (n_chunks + C - 1) / C;
+  const int c0 = min(n_chunks, rank * per), c1 = min(n_chunks, c0 + per);
+  const int cpw = ((per + kVerifyWarps - 1) / kVerifyWarps + 7) & ~7;
+  const int w0 = min(c1, c0 + warp * cpw), w1 = min(c1, w0 + cpw);
+  // With the maxima and masses given and a threshold, few logits are kept: they are weighed one by one, and the drafter's row is read where they lie.
+  const bool gumbel = P.draw == LM_DRAW_GUMBEL, lean = given_mass && !gumbel, few = lean && P.tau != nullptr;
+  // z_cached: a chunk's logits, later the floors of its weights, in two halves; what the chunk weighs in the draw. q_cached: the drafter's row, later the
+  // residual's weights.
+  const int z_slots = lean && !F32 ? per : 2 * per;                         // (lean: the logits stay)
+  unsigned long long* sums = reinterpret_cast<unsigned long long*>(zs + z_slots) - c0;
+  uint4* qs = zs + (z_cached ? z_slots + (per + 1) / 2 : 0) - c0;
+  zs -= c0;
+  const char* q_row = !has_q ? nullptr : Q == 1 ? reinterpret_cast<const char*>(P.q + static_cast<int64_t>(r) * P.q_stride) : reinterpret_cast<const char*>(P.q_logits + static_cast<int64_t>(r) * P.q_logits_stride);
+  const bool q_vec = ((reinterpret_cast<uintptr_t>(q_row) - static_cast<uintptr_t>(off) * (Q == 1 ? 4 : 2)) & 15u) == 0u;
+  if (tid == 0) {
+    VerifyRow& x = s.row;
+    x.q_row = q_row; x.qs = qs; x.off = off; x.V = V; x.per = per; x.q_cached = q_cached; x.q_vec = q_vec;
+    x.cut = P.tau != nullptr; x.tau = P.tau ? P.tau[row] : -INFINITY; x.c2 = Q != 0 ? exp2_scale(P.temperature) : 0.0f;
+    if (given_mass) x.p_of.init(P.row_mass[row]);
+  }
+  auto whole = [&](int c) { const int base = 8 * c - off; return base >= 0 && base + 8 <= V; };
+  constexpr uint32_t kOut = F32 ? 0xFF800000u : 0xFF80u;
+  if (z_cached) {
+#pragma unroll 1
+    for (int c = w0 + lane; c < w1; c += 32) {
+      if (whole(c)) {
+        const char* src = z_row + static_cast<int64_t>(8 * c - off) * kSize;
+        cp_async16(zs + c, src);
+        if (F32) cp_async16(zs + per + c, src + 16);
       } else {
-        uint64_t best = 0ull;
-        if (c4 < n4) {
-          const uint32_t i4 = static_cast<uint32_t>(lo + 4 * c4);
-          best = pack52(x.x, i4);
-          if (left > 1) { const uint64_t p = pack52(x.y, i4 + 1u); best = p > best ? p : best; }
-          if (left > 2) { const uint64_t p = pack52(x.z, i4 + 2u); best = p > best ? p : best; }
-          if (left > 3) { const uint64_t p = pack52(x.w, i4 + 3u); best = p > best ? p : best; }
-        }
-        best = warp_max_u64(best);
-        if (lane == 0) s_red[r0][c4 >> 5] = best;
+        zs[c] = verify_far<F32>(z_row, off, V, c, 0, false, kOut);
+        if (F32) zs[per + c] = verify_far<F32>(z_row, off, V, c, 1, false, kOut);
       }
     }
-    __syncthreads();
-    if (tid < R && !(P.withhold && b == 0)) {
-      uint64_t best = 0ull;
-      for (int k = 0; k < n_red; k++) best = s_red[tid][k] > best ? s_red[tid][k] : best;
-      publish(&ws->best[tid][b], best);
+  }
+  cp_async_commit();
+  if (Q != 0 && has_q && q_cached) {
+#pragma unroll 1
+    for (int c = w0 + lane; c < w1; c += 32) {
+      if (q_vec && whole(c)) {
+        const char* src = q_row + static_cast<int64_t>(8 * c - off) * (Q == 1 ? 4 : 2);
+        cp_async16(qs + c, src);
+        if (Q == 1) cp_async16(qs + per + c, src + 16);
+      } else {
+        qs[c] = verify_far<Q == 1>(q_row, off, V, c, 0, false, Q == 1 ? 0u : 0xFF80u);
+        if (Q == 1) qs[per + c] = verify_far<Q == 1>(q_row, off, V, c, 1, false, 0u);
+      }
     }
-  } else {
-    for (int item = warp; item < R * split; item += kVerifyWarps) {
-      const int r = item / split, part = item - r * split;
-      uint64_t best = 0ull;
-      for (int i = part * 32 + lane; i < len; i += 32 * split) {
-        const uint64_t p = pack52(S.z(r, i), static_cast<uint32_t>(lo + i));
+  }
+  cp_async_commit();
+  // The scalars of the accept test go out under the copies: of this row, or of all rows where every block runs all tests. They are
+  // the last warp's, which has the fewest chunks: the target's side of row r in lane r (lane 0), the drafter's 16 lanes on.
+  const float c2 = Q != 0 ? exp2_scale(P.temperature) : 0.0f;
+  const bool tester = Q != 0 && warp == kVerifyWarps - 1;
+  const int tr = given_mass ? lane & 15 : r;
+  const bool drafter = lane >= 16, tests = tester && tr < L && (given_mass || (lane & 15) == 0);
+  const float u_final = Q != 0 && P.u_final ? P.u_final[0] : 0.0f;           // (wanted at the very end)
+  float t_u = 0.0f, t_tau = -INFINITY, t_max = 0.0f; unsigned long long t_mass = 0ull; bool t_in = false;
+  uint32_t t_bits = 0u;                                                     // (as they come: nothing waits for them before the test)
+  if (tests) {
+    const int d = verify_draft(P, rd, tr);
+    if (!drafter) {
+      if (P.tau) t_tau = P.tau[rd.row0 + tr];
+      if (given_mass) { t_max = P.row_max[rd.row0 + tr]; t_mass = P.row_mass[rd.row0 + tr]; }
+    } else {
+      t_u = P.u_accept ? P.u_accept[tr] : uniform01(rd.seed, rd.step, 3000u + static_cast<uint32_t>(tr), 0u);
+      if (Q == 2) { t_max = __ldg(P.q_vmax + tr); t_mass = __ldg(P.q_mass + tr); }
+    }
+    t_in = d >= 0 && d < V;
+    if (t_in) {
+      if (!drafter) {
+        const char* zp = static_cast<const char*>(P.target) + (static_cast<int64_t>(rd.row0 + tr) * P.row_stride + d) * kSize;
+        t_bits = F32 ? __ldg(reinterpret_cast<const uint32_t*>(zp)) : static_cast<uint32_t>(__ldg(reinterpret_cast<const uint16_t*>(zp))) << 16;
+      } else if (Q == 1) t_bits = __float_as_uint(__ldg(P.q + static_cast<int64_t>(tr) * P.q_stride + d));
+      else t_bits = static_cast<uint32_t>(__ldg(P.q_logits + static_cast<int64_t>(tr) * P.q_logits_stride + d)) << 16;
+    }
+  }
+  // p and q of the draft, side by side: a lane's probability of its logit (0 for an id outside the vocabulary)
+  auto t_prob = [&](float vmax, unsigned long long m) {
+    const float z = canon_zero(__uint_as_float(t_bits));
+    return t_in && m > 0ull ? prob_q40(z >= t_tau ? weight_q40(z, vmax, c2) : 0ull, m) : 0.0f;
+  };
+  auto keep_drafter = [&]() { if (Q == 2 && drafter && tr == r) { s.row.qv = t_max; s.row.q_of.init(t_mass); } };
+  // the target's lanes: rejected? pq: the lanes' own probabilities
+  auto test = [&](float pq, bool write) {
+    const float uq = __shfl_down_sync(kFull, __fmul_rn(t_u, Q == 1 ? __uint_as_float(t_bits) : pq), 16);   // (t_bits of an id outside the vocabulary: 0)
+    if (write && tests && !drafter && P.out_p_draft) P.out_p_draft[tr] = pq;
+    return tests && !drafter && uq >= pq;
+  };
+  // half h of a chunk as it lies in memory (BF16: the whole chunk, whichever half)
+  auto z_raw = [&](int c, int h) { return z_cached ? zs[(F32 && h ? per : 0) + c] : verify_far<F32>(z_row, off, V, c, h, true, kOut); };
+  bool joined = C == 1;                                                     // every block of the cluster runs: its shared memory may be written to
+  auto join = [&]() { if (!joined) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); joined = true; };
+  // a warp's value to every block of the cluster (or to block 0 alone)
+  auto push = [&](unsigned long long* slots, uint64_t v, bool all) { if (lane < (all ? C : 1)) cst_u64(cluster_addr(&slots[rank], lane), v); };
+
+  // ---- the row's maximum (greedy: with its lowest index) ------------------------------------------------------------------------------
+  float vmax = 0.0f;
+  cp_async_wait<1>();                                                       // (a thread reads back its own chunks: no barrier)
+  if (given_max) { vmax = canon_zero(P.row_max[row]); __syncthreads(); }
+  else {
+    // Per half its maximum alone. NaN follows the packed order (a positive NaN above +inf, a negative one below -inf): a half that holds one is compared
+    // element by element. Greedy looks for the index once, at the end.
+    float top = -INFINITY;
+    int top_c = w0 + lane < w1 ? 2 * (w0 + lane) : -1;
+    uint64_t best = 0ull;
+    auto elements = [&](int ch, bool any, float value) {                    // those of half ch & 1 of chunk ch >> 1 that are in the row and (any or they equal value)
+      const uint4 v = z_raw(ch >> 1, ch & 1);
+      float2 z[2];
+      verify_pairs<F32>(v, ch & 1, z);
+#pragma unroll 1
+      for (int e = 0; e < 4; e++) {
+        const float2 z2 = (e & 2) ? z[1] : z[0];
+        const float ze = (e & 1) ? z2.y : z2.x;
+        const int i = 4 * ch + e - off;
+        if (i < 0 || i >= V || !(any || ze == value)) continue;
+        const uint64_t p = pack_best(ze, static_cast<uint32_t>(i));
         best = p > best ? p : best;
       }
-      best = warp_max_u64(best);
-      if (lane == 0) s_red[r][part] = best;
+    };
+#pragma unroll 1
+    for (int c = w0 + lane; c < w1; c += 32) {
+      uint4 v = z_raw(c, 0);
+#pragma unroll 1
+      for (int h = 0; h < 2; h++) {
+        float mx;
+        if (F32) {
+          if (h) v = z_raw(c, 1);
+          asm("max.NaN.f32 %0, %1, %2;" : "=f"(mx) : "f"(__uint_as_float(v.x)), "f"(__uint_as_float(v.y)));
+          asm("max.NaN.f32 %0, %1, %2;" : "=f"(mx) : "f"(mx), "f"(__uint_as_float(v.z)));
+          asm("max.NaN.f32 %0, %1, %2;" : "=f"(mx) : "f"(mx), "f"(__uint_as_float(v.w)));
+        } else {
+          const uint32_t a = h ? v.z : v.x, b = h ? v.w : v.y;
+          const __nv_bfloat162 m = __hmax2_nan(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
+          const float l = __low2float(m), u = __high2float(m);
+          asm("max.NaN.f32 %0, %1, %2;" : "=f"(mx) : "f"(l), "f"(u));
+        }
+        if (mx > top) { top = mx; top_c = 2 * c + h; }
+        if (mx != mx) elements(2 * c + h, true, 0.0f);
+      }
+    }
+    if (Q == 0 && top_c >= 0) {
+      // (a row of nothing but -inf: this thread's first element that is in the row)
+      elements(top_c, false, canon_zero(top));
+      if (best == 0ull) elements(top_c + 1, false, canon_zero(top));
+    }
+    best = Q != 0 ? static_cast<uint64_t>(warp_max_u32(max(fkey(canon_zero(top)), static_cast<uint32_t>(best >> 32)))) : warp_max_u64(best);   // (stochastic: the value alone)
+    if (lane == 0) s.best[warp] = best;
+    __syncthreads();
+    join();
+    if (warp == 0) push(s.x_best, warp_max_u64(lane < kVerifyWarps ? s.best[lane] : 0ull), Q != 0);
+    cluster_sync(C);
+    if (Q == 0) {
+      if (rank == 0 && warp == 0) {
+        const int pick = static_cast<int>(best_index(warp_max_u64(lane < C ? s.x_best[lane] : 0ull)));
+        verify_arrive(P, rd, r, launch, r < L && pick != verify_draft(P, rd, r), pick);
+      }
+      return;
+    }
+    vmax = fkey_inv(warp_max_u32(lane < C ? static_cast<uint32_t>(s.x_best[lane]) : 0u));
+  }
+  if (Q == 0) return;
+
+  // ---- the kept set's mass and the accept test; given masses: all tests, and only the decisive row goes on ----------------------------------
+  const bool keep_w = z_cached && !lean && !(gumbel && !has_q);             // the weights replace the logits
+  // the logit of an element, -0 as +0; a bit for each element of a chunk that is kept and not -inf
+  auto z_at = [&](int c, int e) {
+    const uint4 a = z_raw(c, e >> 2);
+    const uint32_t w = F32 ? ((e & 2) ? ((e & 1) ? a.w : a.z) : ((e & 1) ? a.y : a.x)) : ((e & 4) ? ((e & 2) ? a.w : a.z) : ((e & 2) ? a.y : a.x));
+    return canon_zero(F32 ? __uint_as_float(w) : (e & 1) ? bf16_hi(w) : bf16_lo(w));
+  };
+  auto kept_of = [&](int c) {
+    const float tau = s.row.tau;
+    uint32_t m = 0u;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      float2 z[2];
+      verify_pairs<F32>(z_raw(c, F32 ? h : 0), h, z);
+#pragma unroll
+      for (int k = 0; k < 2; k++) m |= ((z[k].x >= tau && z[k].x > -INFINITY ? 1u : 0u) | (z[k].y >= tau && z[k].y > -INFINITY ? 2u : 0u)) << (4 * h + 2 * k);
+    }
+    return m;
+  };
+  // a chunk's weights, as floors, from its logits in shared memory; nothing kept of it costs its maximum
+  auto weigh = [&](int c, FloorSum& sum, float2 (&w)[4]) {
+    const float tau = s.row.tau;
+    float2 z[4];
+    const uint4 v = zs[c];
+    if (F32) {
+      const uint4 b = zs[per + c];
+      z[0] = make_float2(__uint_as_float(v.x), __uint_as_float(v.y)); z[1] = make_float2(__uint_as_float(v.z), __uint_as_float(v.w));
+      z[2] = make_float2(__uint_as_float(b.x), __uint_as_float(b.y)); z[3] = make_float2(__uint_as_float(b.z), __uint_as_float(b.w));
+    } else {
+      z[0] = make_float2(bf16_lo(v.x), bf16_hi(v.x)); z[1] = make_float2(bf16_lo(v.y), bf16_hi(v.y));
+      z[2] = make_float2(bf16_lo(v.z), bf16_hi(v.z)); z[3] = make_float2(bf16_lo(v.w), bf16_hi(v.w));
+    }
+    const bool none = s.row.cut && !(fmaxf(fmaxf(fmaxf(z[0].x, z[0].y), fmaxf(z[1].x, z[1].y)), fmaxf(fmaxf(z[2].x, z[2].y), fmaxf(z[3].x, z[3].y))) >= tau);
+#pragma unroll
+    for (int k = 0; k < 4; k++) w[k] = make_float2(0.0f, 0.0f);
+    if (!none) {
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        z[k] = __fadd2_rn(z[k], make_float2(0.0f, 0.0f));
+        const float2 x = weight_f2(z[k].x, z[k].y, vmax, c2);
+        w[k] = sum.add(make_float2(z[k].x >= tau ? x.x : 0.0f, z[k].y >= tau ? x.y : 0.0f));
+      }
+    }
+    if (keep_w) {
+      zs[c] = make_uint4(__float_as_uint(w[0].x), __float_as_uint(w[0].y), __float_as_uint(w[1].x), __float_as_uint(w[1].y));
+      zs[per + c] = make_uint4(__float_as_uint(w[2].x), __float_as_uint(w[2].y), __float_as_uint(w[3].x), __float_as_uint(w[3].y));
+    }
+  };
+  bool residual = false, weighed = !given_mass && keep_w;                   // weighed: the floors of the weights lie in shared memory
+  auto half_weight = [&](int c, int h, bool stored) { return verify_half<F32, Q>(s.row, stored ? zs[(h ? per : 0) + c] : z_raw(c, h), c, h, stored, residual, vmax); };
+  const bool direct = given_mass && !(P.state && P.commit);                 // (a commit changes the state that blocks of other rows may not have read yet)
+  unsigned long long mass = 0ull;
+  int j = r;
+  if (given_mass) {
+    if (tester) {
+      if (tests) keep_drafter();
+      const uint32_t rejects = __ballot_sync(kFull, test(t_prob(canon_zero(t_max), t_mass), r == 0 && rank == 0));
+      if (lane == 0) s.j = rejects ? __ffs(static_cast<int>(rejects)) - 1 : L;
     }
     __syncthreads();
-    if (tid < R && !(P.withhold && b == 0)) {
-      uint64_t best = 0ull;
-      for (int k = 0; k < n_red; k++) best = s_red[tid][k] > best ? s_red[tid][k] : best;
-      publish(&ws->best[tid][b], best);
-    }
-  }
-  clean_other_bank();
-  __syncthreads();                                                        // s_red is reused below
-
-  uint64_t vals[kConsumeSlots] = {0ull, 0ull, 0ull, 0ull};
-  const int Gp = (G + 31) & ~31;
-  if (!stochastic) {
-    // ---- greedy: block 0 gathers every row's pick and votes; the others are done --------------------------------------------
-    if (b == 0) {
-      consume_rows<false>(&ws->best[0][0], R, G, s_best, s_red, limit, &failed, vals);
-      const bool bad = __syncthreads_or(failed) != 0;
-      if (bad && tid == 0) atomicExch(&ws->error, 1u);
-      if (tid < 32) {
-        const int pick = tid < R ? static_cast<int>(pack52_index(s_best[tid])) : -1;
-        const uint32_t miss = __ballot_sync(kFull, tid < L && pick != s_drafts[tid]);
-        const int acc = miss ? (__ffs(miss) - 1) : L;
-        const int fin = __shfl_sync(kFull, pick, acc);
-        if (tid == 0) { P.out_accept[0] = bad ? -1 : acc; P.out_final[0] = bad ? -1 : fin; }
-        if (P.out_tokens && tid < R) P.out_tokens[row0 + tid] = bad ? -1 : (tid < acc ? s_drafts[tid] : (tid == acc ? fin : -1));
-        verify_commit(P, bad);
-      }
+    join();
+    j = s.j;
+    mass = P.row_mass[row];
+    if (r != j) {
+      if (!direct && rank == 0 && warp == 0) verify_arrive(P, rd, r, launch, false, -1);   // (beyond j it does not matter)
+      return;
     }
   } else {
-    // ---- phase 1: every block learns the row maxima; fixed-point mass of every row's kept set; the drafts' own weights -------
-    if (!given_max) consume_rows<false>(&ws->best[0][0], R, G, s_best, s_red, limit, &failed, vals);
-    if (given_mass) {
-      // nothing to sum: the sampler's masses, and every block evaluates the drafts' weights itself (one logit each)
-    } else if (cached) {
-      // the same walk as for the maxima: four elements per load, two packed weight evaluations, one warp sum per 128 elements
-      for (int i0 = 0; i0 < R * n4p; i0 += kVerifyBlock) {
-        const int r0 = (i0 + (tid & ~31)) / n4p;
-        if (r0 >= R) break;                                               // warp-uniform
-        const int item = i0 + tid, c4 = item - r0 * n4p;
-        uint64_t w = 0ull;
-        if (c4 < n4) {
-          const float vmax = pack52_value(s_best[r0]);
-          const float tau = P.tau ? P.tau[row0 + r0] : -INFINITY;
-          const float4 x = reinterpret_cast<const float4*>(zs + r0 * per)[c4];
-          const int left = len - 4 * c4;
-          uint64_t w0, w1, w2, w3;
-          weight_q40_x2(x.x, x.y, vmax, c2, w0, w1);
-          weight_q40_x2(x.z, x.w, vmax, c2, w2, w3);
-          if (x.x >= tau) w += w0;
-          if (left > 1 && x.y >= tau) w += w1;
-          if (left > 2 && x.z >= tau) w += w2;
-          if (left > 3 && x.w >= tau) w += w3;
+    uint64_t own = 0ull;
+#pragma unroll 1
+    for (int c = w0 + lane; c < w1; c += 32) {
+      FloorSum sum;
+      if (z_cached) {
+        float2 w[4];
+        weigh(c, sum, w);
+        sums[c] = sum.sum();
+      } else {
+#pragma unroll 1
+        for (int h = 0; h < 2; h++) { const float4 x = half_weight(c, h, false); sum.add(make_float2(x.x, x.y)); sum.add(make_float2(x.z, x.w)); }
+      }
+      own += sum.sum();
+    }
+    float t_q = 0.0f;
+    if (Q == 2 && tests && drafter) { keep_drafter(); t_q = t_prob(t_max, t_mass); }   // (the drafter's side, before the mass is known)
+    own = warp_sum_u64(own);
+    if (lane == 0) s.own[warp] = own;
+    __syncthreads();
+    join();
+    if (warp == 0) push(s.x_own, warp_sum_u64(lane < kVerifyWarps ? s.own[lane] : 0ull), true);
+    cluster_sync(C);
+    uint64_t unused;
+    mass = verify_prefix(s.x_own, C, 0, &unused);
+    if (has_q) {
+      if (tester) {
+        const bool no = test(drafter ? t_q : t_prob(vmax, mass), rank == 0);
+        if (lane == 0) { s.reject = no; s.row.p_of.init(mass); }
+      }
+      __syncthreads();
+      if (!s.reject) {
+        if (rank == 0 && warp == 0) verify_arrive(P, rd, r, launch, false, -1);
+        return;
+      }
+    }
+  }
+
+  // ---- the draw: over the residual max(p - q, 0) of a rejected draft, over p itself on the bonus row or where the residual is empty -----------
+  cp_async_wait<0>();
+  auto deliver = [&](int token) {                                           // one whole warp of the cluster
+    if (direct) verify_outputs(P, rd, false, j, token); else verify_arrive(P, rd, r, launch, r < L, token);
+  };
+  // The sums of the draw: the residual's, and where that is empty the row's own once more (the mass's sums will do where there is no draft). Or, in the reference's
+  // form (kernels/common/sample.metal:322-346), the best of ln(p - q) + noise of stream 4000, and where nothing is left the best of the row's own Gumbel keys.
+  // The best key of this thread's chunks over the residual, whose weight in the warp's range is `there` (of 2^40). A key of ln there - 1.5 is missed once in 90, and
+  // leaves four or five logits to look at closely; where none has reached it, the bar is what has been found, or lower.
+  auto best_of_rest = [&](uint64_t there) {
+    ResidualScan rest;
+    rest.init(rd.seed, rd.step, 4000u);
+    if (there == 0ull) return rest.best;
+    float bar = logf(__ull2float_rn(there) * 0x1p-40f) - 1.5f;
+#pragma unroll 1
+    for (;;) {
+      rest.room = 8388608.0f * ex2_approx((2e-3f - bar) * 1.44269504f);
+#pragma unroll 1
+      for (int b0 = 2 * w0; b0 < 2 * w1; b0 = (b0 & 1) ? b0 + 63 : b0 + 1) {  // (whole warps)
+        const int c = (b0 >> 1) + lane, h = b0 & 1;
+        float r4[4] = {0.0f, 0.0f, 0.0f, 0.0f};                             // p - q, exactly; nothing outside the row
+        if (c < w1) {
+          float4 x;
+          if (z_cached) {
+            const uint4 v = zs[(h ? per : 0) + c];
+            x = make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
+          } else x = half_weight(c, h, false);
+          r4[0] = x.x * 0x1p-40f; r4[1] = x.y * 0x1p-40f; r4[2] = x.z * 0x1p-40f; r4[3] = x.w * 0x1p-40f;
         }
-        const uint32_t wl = warp_sum_u32(static_cast<uint32_t>(w) & 0x3FFFFFu), wh = warp_sum_u32(static_cast<uint32_t>(w >> 22));
-        if (lane == 0) s_red[r0][c4 >> 5] = static_cast<uint64_t>(wl) + (static_cast<uint64_t>(wh) << 22);
+        const uint64_t had = rest.best;
+        rest.offer4(r4, 8 * c + 4 * h - off);
+        rest.share(had);
       }
-      if (tid < L) {                                                      // the drafts' own weights: the block whose slice holds the draft
-        const int d = s_drafts[tid];
-        if (d >= lo && d < hi) {
-          const float z = S.z(tid, d - lo), tau = P.tau ? P.tau[row0 + tid] : -INFINITY;
-          publish(&ws->draft_w[tid], (z >= tau) ? weight_q40(z, pack52_value(s_best[tid]), c2) : 0ull);
-        } else if ((d < 0 || d >= V) && b == 0) publish(&ws->draft_w[tid], 0ull);     // an id outside the vocabulary: probability 0
-      }
-    } else {
-    for (int item = warp; item < R * split; item += kVerifyWarps) {
-      const int r = item / split, part = item - r * split;
-      const float vmax = pack52_value(s_best[r]);
-      const float tau = P.tau ? P.tau[row0 + r] : -INFINITY;
+      const uint64_t top = warp_max_u64(rest.best);
+      if ((top && best_value(top) >= bar) || rest.room == INFINITY) return rest.best;
+      bar = top ? best_value(top) : bar - 3.0f;
+    }
+  };
+  // ... and over the row itself (the logits of a row with a draft have been written over).
+  auto best_of_row = [&]() {
+    GumbelScan own;
+    own.init(rd.seed, rd.step, static_cast<uint32_t>(row), P.temperature, -INFINITY);
+#pragma unroll 1
+    for (int b0 = 2 * w0; b0 < 2 * w1; b0 = (b0 & 1) ? b0 + 63 : b0 + 1) {
+      const int c = (b0 >> 1) + lane, h = b0 & 1, i = 8 * c + 4 * h - off;
+      float2 z[2] = {make_float2(-INFINITY, -INFINITY), make_float2(-INFINITY, -INFINITY)};
+      if (c < w1) verify_pairs<F32>(has_q ? verify_far<F32>(z_row, off, V, c, h, true, kOut) : z_raw(c, h), h, z);
+      const float tau = s.row.tau;
+#pragma unroll
+      for (int k = 0; k < 2; k++)                                           // (what is not kept, or lies outside the row, is -inf: no key)
+        own.offer2(z[k].x >= tau ? z[k].x : -INFINITY, static_cast<uint32_t>(i + 2 * k), z[k].y >= tau ? z[k].y : -INFINITY, static_cast<uint32_t>(i + 2 * k + 1));
+      const uint64_t top = warp_max_u64(own.best);
+      if (top) own.raise(best_value(top));
+    }
+    return own.best;
+  };
+  const unsigned long long *slots = s.x_own, *parts = reinterpret_cast<const unsigned long long*>(s.own);
+  uint64_t before = 0ull, there = 0ull;                                     // the weight before this block's slice; all of it
+  if (has_q || given_mass || gumbel) {
+    slots = s.x_res; parts = reinterpret_cast<const unsigned long long*>(s.res);
+    residual = has_q;
+    bool first = true;
+#pragma unroll 1
+    for (;; residual = first = false) {
       uint64_t w = 0ull;
-      for (int i = part * 32 + lane; i < len; i += 32 * split) {
-        const float z = S.z(r, i);
-        if (z >= tau) w += weight_q40(z, vmax, c2);
+      if (mass > 0ull && !(gumbel && !residual)) {
+#pragma unroll 1
+        for (int c = w0 + lane; c < w1; c += 32) {
+          FloorSum sum;
+          uint64_t v = 0ull;
+          const uint32_t kept = few ? kept_of(c) : 0u;
+          if (few && __popc(kept) <= 2) {
+#pragma unroll 1
+            for (uint32_t m = kept; m; m &= m - 1u) { const int e = __ffs(static_cast<int>(m)) - 1; v += verify_element<F32, Q>(s.row, 8 * c + e - off, z_at(c, e), residual, vmax); }
+          } else if (first && z_cached) {
+            float2 x[4];
+            if (weighed) {
+              const uint4 a = zs[c], b = zs[per + c];
+              x[0] = make_float2(__uint_as_float(a.x), __uint_as_float(a.y)); x[1] = make_float2(__uint_as_float(a.z), __uint_as_float(a.w));
+              x[2] = make_float2(__uint_as_float(b.x), __uint_as_float(b.y)); x[3] = make_float2(__uint_as_float(b.z), __uint_as_float(b.w));
+            } else weigh(c, sum, x);
+            if (has_q) {
+              sum = FloorSum();
+              uint32_t any = 0u;
+#pragma unroll
+              for (int k = 0; k < 4; k++) any |= __float_as_uint(x[k].x) | __float_as_uint(x[k].y);
+              if (any) {
+                float2 q[4];
+                uint4 a, b;
+                if (q_cached) { a = qs[c]; if (Q == 1) b = qs[per + c]; }
+                else { a = verify_far<Q == 1>(q_row, off, V, c, 0, q_vec, Q == 1 ? 0u : 0xFF80u); if (Q == 1) b = verify_far<Q == 1>(q_row, off, V, c, 1, q_vec, 0u); }
+                if (Q == 1) {
+                  q[0] = make_float2(__uint_as_float(a.x), __uint_as_float(a.y)); q[1] = make_float2(__uint_as_float(a.z), __uint_as_float(a.w));
+                  q[2] = make_float2(__uint_as_float(b.x), __uint_as_float(b.y)); q[3] = make_float2(__uint_as_float(b.z), __uint_as_float(b.w));
+                } else {
+                  const ProbScale q_of = s.row.q_of;
+                  const float qv = s.row.qv;
+                  const uint32_t u[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+                  for (int k = 0; k < 4; k++) {
+                    const float2 z = __fadd2_rn(make_float2(bf16_lo(u[k]), bf16_hi(u[k])), make_float2(0.0f, 0.0f));
+                    uint2 t, l;
+                    q[k] = q_of.of(floor2(weight_f2(z.x, z.y, qv, c2), t, l));
+                  }
+                }
+                const ProbScale p_of = s.row.p_of;
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                  const float2 d = __fadd2_rn(p_of.of(x[k]), make_float2(-q[k].x, -q[k].y));
+                  x[k] = __fmul2_rn(make_float2(x[k].x > 0.0f ? fmaxf(d.x, 0.0f) : 0.0f, x[k].y > 0.0f ? fmaxf(d.y, 0.0f) : 0.0f), make_float2(1099511627776.0f, 1099511627776.0f));
+                  sum.add(x[k]);
+                }
+              }
+            }
+            if (gumbel || q_cached) {
+              uint4* to = gumbel ? zs : qs;
+              to[c] = make_uint4(__float_as_uint(x[0].x), __float_as_uint(x[0].y), __float_as_uint(x[1].x), __float_as_uint(x[1].y));
+              to[per + c] = make_uint4(__float_as_uint(x[2].x), __float_as_uint(x[2].y), __float_as_uint(x[3].x), __float_as_uint(x[3].y));
+            }
+          } else {
+#pragma unroll 1
+            for (int h = 0; h < 2; h++) { const float4 x = half_weight(c, h, weighed); sum.add(make_float2(x.x, x.y)); sum.add(make_float2(x.z, x.w)); }
+          }
+          v += sum.sum();
+          if (z_cached) sums[c] = v;
+          w += v;
+        }
       }
       w = warp_sum_u64(w);
-      if (lane == 0) {
-        s_red[r][part] = w;
-        if (part == 0 && r < L) {
-          const int d = s_drafts[r];
-          if (d >= lo && d < hi) {
-            const float z = S.z(r, d - lo);
-            publish(&ws->draft_w[r], (z >= tau) ? weight_q40(z, vmax, c2) : 0ull);
-          } else if ((d < 0 || d >= V) && b == 0) publish(&ws->draft_w[r], 0ull);   // an id outside the vocabulary: probability 0
-        }
-      }
-    }
-    }
-    __syncthreads();
-    if (tid < R && !given_mass) {
-      uint64_t w = 0ull;
-      for (int k = 0; k < n_red; k++) w += s_red[tid][k];
-      s_own[tid] = w;
-      publish(&ws->mass[tid][b], w);
-    }
-    if (tid < R && given_mass) s_mass[tid] = my_mass;
-    __syncthreads();
-    // ---- phase 2: row masses; accept tests (every block, identically); this slice's share of the residual -------------------
-    const unsigned long long dw_first = (tid < L && !given_mass) ? peek(&ws->draft_w[tid]) : 0ull;   // in flight while the masses are consumed
-    if (!given_mass) consume_rows<true>(&ws->mass[0][0], R, G, s_mass, s_red, limit, &failed, vals);
-    if (tid < 32) {
-      bool reject = false;
-      if (tid < L) {
-        uint64_t dw;
-        if (given_mass) {                                                  // the draft's own weight, straight from its logit
-          const float tau = P.tau ? P.tau[row0 + tid] : -INFINITY;
-          dw = (my_zd >= tau) ? weight_q40(my_zd, pack52_value(s_best[tid]), c2) : 0ull;
-        } else dw = consume(&ws->draft_w[tid], limit, &failed, dw_first);
-        const uint64_t mass = s_mass[tid];
-        const float pd = (my_draft >= 0 && my_draft < V && mass > 0ull) ? prob_q40(dw, mass) : 0.0f;
-        reject = __fmul_rn(my_u, my_q) >= pd;
-        if (b == 0 && P.out_p_draft) P.out_p_draft[tid] = pd;
-      }
-      const uint32_t rejects = __ballot_sync(kFull, reject);
-      if (tid == 0) s_j = rejects ? (__ffs(rejects) - 1) : L;
-    }
-    __syncthreads();
-    const int j = s_j;
-    const float vmax_j = pack52_value(s_best[j]);
-    const float tau_j = P.tau ? P.tau[row0 + j] : -INFINITY;
-    const uint64_t mass_j = s_mass[j];
-    const bool has_q = j < L;
-    // this block's exclusive prefix over the blocks' masses of row j (the draw over p itself needs it)
-    uint64_t pre_w = 0ull;
-    if (!given_mass) {
-#pragma unroll
-      for (int k = 0; k < kConsumeSlots; k++) {
-        const int idx = k * kVerifyBlock + tid, r = idx / Gp, g = idx - r * Gp;
-        if (r == j && g < b) pre_w += vals[k];
-      }
-      pre_w = block_sum_u64(pre_w, scratch);
-    }
-    uint64_t own_w = given_mass ? 0ull : s_own[j];                         // this block's share of row j's mass (the draw over p itself)
-    // residual weight of element i of this slice (0 when not kept or not positive)
-    auto residual_of = [&](const VerifySlice& V2, int i) -> uint64_t {
-      const float z = V2.z(j, i);
-      if (!(z >= tau_j)) return 0ull;
-      const float p = prob_q40(weight_q40(z, vmax_j, c2), mass_j);
-      const float res = has_q ? __fsub_rn(p, V2.q(j, i)) : p;
-      return res > 0.0f ? residual_q40(res) : 0ull;
-    };
-    auto residual = [&](int i) -> uint64_t { return residual_of(S, i); };
-    // the token inside a slice (lo2, len2, read through V2): the first element, in index order, at which the running weight -- the
-    // residual's, or the row's own when the residual is empty -- passes the target; `base` = the weight of everything before the slice
-    auto locate = [&](const VerifySlice& V2, int lo2, int len2, uint64_t base, bool use_res, uint64_t target) -> int {
-      if (tid == 0) s_token = -2;
+      if (gumbel) w = warp_max_u64(mass == 0ull ? 0ull : residual ? best_of_rest(w) : best_of_row());
+      if (lane == 0) s.res[warp] = w;
       __syncthreads();
-      for (int i0 = 0; i0 < len2; i0 += kVerifyBlock) {                     // uniform trip count: block-wide scans inside
-        const int i = i0 + tid;
-        uint64_t w = 0ull;
-        if (i < len2) {
-          if (use_res) w = residual_of(V2, i);
-          else { const float z = V2.z(j, i); if (z >= tau_j) w = weight_q40(z, vmax_j, c2); }
-        }
-        uint64_t sweep = 0ull;
-        const uint64_t excl = block_exclusive_scan_u64(w, scratch, &sweep);
-        if (w && base + excl <= target && target < base + excl + w) s_token = lo2 + i;
-        base += sweep;
-        __syncthreads();
-        if (s_token != -2) break;
+      if (warp == 0) {
+        w = lane < kVerifyWarps ? s.res[lane] : 0ull;
+        push(s.x_res, gumbel ? warp_max_u64(w) : warp_sum_u64(w), true);
       }
-      return s_token;
-    };
-    const uint32_t t_row = static_cast<uint32_t>(row0 + j);
-    const float inv_t32 = __double2float_rn(1.0 / static_cast<double>(P.temperature));
-    uint64_t total_r = 0ull, mine_r = 0ull;
-    int token = -2;
-    if (gumbel_draw) {
-      // the reference's draws (kernels/common/sample.metal:322-346): argmax of ln(p - q) + noise of stream 4000 over the positive
-      // residual; with nothing rejected, or an empty residual, the row's own Gumbel-max draw on its stream (the sampler's token)
-      uint64_t best_res = 0ull, best_own = 0ull;
-      if (mass_j > 0ull) for (int i = tid; i < len; i += kVerifyBlock) {
-        const float z = S.z(j, i);
-        if (!(z >= tau_j)) continue;
-        const uint32_t idx = static_cast<uint32_t>(lo + i);
-        const uint64_t own = pack52(__fadd_rn(__fmul_rn(z, inv_t32), gumbel(seed, step, t_row, idx)), idx);
-        best_own = own > best_own ? own : best_own;
-        if (has_q) {
-          const float res = __fsub_rn(prob_q40(weight_q40(z, vmax_j, c2), mass_j), S.q(j, i));
-          if (res > 0.0f) { const uint64_t k = pack52(__fadd_rn(logf(res), gumbel(seed, step, 4000u, idx)), idx); best_res = k > best_res ? k : best_res; }
-        }
-      }
-      best_res = block_max_u64(best_res, scratch);
-      best_own = block_max_u64(best_own, scratch);
-      if (tid == 0) { publish(&ws->resid[0][b], best_res); publish(&ws->resid[1][b], best_own); }
-      if (b == 0) {                                                       // block 0 gathers the blocks' best keys
-        uint64_t kr = 0ull, ko = 0ull;
-        for (int g = tid; g < G; g += kVerifyBlock) {
-          const uint64_t a = consume(&ws->resid[0][g], limit, &failed), c = consume(&ws->resid[1][g], limit, &failed);
-          kr = a > kr ? a : kr; ko = c > ko ? c : ko;
-        }
-        kr = block_max_u64(kr, scratch); ko = block_max_u64(ko, scratch);
-        token = kr ? static_cast<int>(pack52_index(kr)) : (ko ? static_cast<int>(pack52_index(ko)) : -1);
-      }
-    } else if (given_mass) {
-      // ---- the one exchange of a launch that was given the masses: this slice's share of row j's mass and of its residual --------
-      uint64_t w = 0ull, wo = 0ull;
-      if (mass_j > 0ull) for (int i = tid; i < len; i += kVerifyBlock) {
-        const float z = S.z(j, i);
-        if (z >= tau_j) wo += weight_q40(z, vmax_j, c2);
-        if (has_q) w += residual(i);
-      }
-      mine_r = block_sum_u64(w, scratch); own_w = block_sum_u64(wo, scratch);
-      if (tid == 0) { publish(&ws->resid[0][b], mine_r); publish(&ws->resid[1][b], own_w); }
-      // Block 0 alone gathers the shares (148 blocks polling each other's words from the moment they have published cost more than
-      // the draw itself); it then reads the one slice that holds the crossing straight from L2. Every other block is done.
-      if (b == 0) {
-        uint64_t* a_res = &s_red[0][0];                                    // G <= 256 shares each: s_red is free from here on
-        uint64_t* a_own = &s_red[8][0];
-        uint64_t tr = 0ull;
-        for (int g = tid; g < G; g += kVerifyBlock) {
-          const uint64_t v = consume(&ws->resid[0][g], limit, &failed), o = consume(&ws->resid[1][g], limit, &failed);
-          a_res[g] = v; a_own[g] = o; tr += v;
-        }
-        total_r = block_sum_u64(tr, scratch);                              // (its barriers also publish a_res / a_own to the block)
-      }
-    } else if (has_q) {
-      // ---- the residual's total: one more exchange (skipped when every draft was accepted: the bonus row draws from p). Block 0
-      // gathers, as above; the blocks' shares of row j's mass are still in the workspace from the exchange before.
-      uint64_t w = 0ull;
-      if (mass_j > 0ull) for (int i = tid; i < len; i += kVerifyBlock) w += residual(i);
-      mine_r = block_sum_u64(w, scratch);
-      if (tid == 0) publish(&ws->resid[0][b], mine_r);
-      if (b == 0) {
-        uint64_t* a_res = &s_red[0][0];
-        uint64_t* a_own = &s_red[8][0];
-        uint64_t tr = 0ull;
-        for (int g = tid; g < G; g += kVerifyBlock) {
-          const uint64_t v = consume(&ws->resid[0][g], limit, &failed), o = consume(&ws->mass[j][g], limit, &failed);
-          a_res[g] = v; a_own[g] = o; tr += v;
-        }
-        total_r = block_sum_u64(tr, scratch);
+      cluster_sync(C);
+      there = gumbel ? warp_max_u64(lane < C ? slots[lane] : 0ull) : verify_prefix(slots, C, rank, &before);
+      if (there || !residual) break;
+      cluster_sync(C);                                                      // (everybody has read the slots)
+    }
+  } else there = verify_prefix(slots, C, rank, &before);
+  if (gumbel) {
+    if (rank == 0 && warp == 0) deliver(there ? static_cast<int>(best_index(there)) : -1);
+    return;
+  }
+  const uint64_t total = residual ? there : mass, target = cdf_target(P.u_final ? u_final : uniform01(rd.seed, rd.step, 4000u, 0u), total);
+  if (total == 0ull || target >= there) {                                   // a row with no weight at all (empty or all -inf), or a given mass that is not the row's
+    if (rank == 0 && warp == 0) deliver(-1);
+    return;
+  }
+  if (!(before <= target && target < before + slots[rank])) return;         // the crossing lies in another block's slice
+  {
+    uint64_t in_block;
+    verify_prefix(parts, kVerifyWarps, warp, &in_block);
+    before += in_block;
+  }
+  if (!(before <= target && target < before + parts[warp])) return;         // ... in another warp's range
+  // the first element, in index order, at which the running weight passes the target: the chunk from the chunks' sums, then a lane for each of its elements
+  const bool kept_values = z_cached && q_cached && (has_q || given_mass) && residual == has_q;   // the draw's weights lie in the drafter's place
+  int token = -1;
+#pragma unroll 1
+  for (int b0 = w0; b0 < w1; b0 += 32) {
+    const int c = b0 + lane;
+    uint64_t sum = 0ull;
+    if (c < w1) {
+      if (z_cached) sum = sums[c];
+      else {
+        FloorSum f;
+#pragma unroll 1
+        for (int h = 0; h < 2; h++) { const float4 x = half_weight(c, h, false); f.add(make_float2(x.x, x.y)); f.add(make_float2(x.z, x.w)); }
+        sum = f.sum();
       }
     }
-    const bool bad = __syncthreads_or(failed) != 0;
-    if (bad && tid == 0) atomicExch(&ws->error, 1u);
+    uint64_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const uint64_t t = __shfl_up_sync(kFull, incl, o); if (lane >= o) incl += t; }
+    uint64_t run = before + incl - sum;
+    const uint32_t hit = __ballot_sync(kFull, run <= target && target < run + sum);
+    if (hit) {
+      const int ch = b0 + __ffs(static_cast<int>(hit)) - 1, e = lane & 7, h = e >> 2;
+      run = __shfl_sync(kFull, run, ch - b0);
+      uint64_t v;
+      if (few) v = (kept_of(ch) >> e) & 1u ? verify_element<F32, Q>(s.row, 8 * ch + e - off, z_at(ch, e), residual, vmax) : 0ull;
+      else if (kept_values || weighed) v = __float2ull_rz(reinterpret_cast<const float*>((kept_values ? qs : zs) + (h ? per : 0) + ch)[e & 3]);
+      else {
+        const float4 x = half_weight(ch, h, weighed);
+        v = __float2ull_rz((e & 2) ? ((e & 1) ? x.w : x.z) : ((e & 1) ? x.y : x.x));
+      }
+      uint64_t upto = v;
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) { const uint64_t t = __shfl_up_sync(kFull, upto, o); if (e >= o) upto += t; }
+      const uint32_t at = __ballot_sync(kFull, run + upto - v <= target && target < run + upto) & 0xFFu;
+      if (at) token = 8 * ch + __ffs(static_cast<int>(at)) - 1 - off;
+      break;
+    }
+    before += __shfl_sync(kFull, incl, 31);
+  }
+  deliver(token);
+}
 
-    // ---- phase 3: locate the draw; the block whose slice holds it writes the outputs ---------------------------------------
-    bool writer = false;
-    if (gumbel_draw) {
-      writer = b == 0;
-    } else if (given_mass || has_q) {                                       // the shares were gathered by block 0: it draws
-      if (b == 0) {
-        writer = true;
-        const bool use_res = total_r > 0ull;                             // an empty residual: draw from the row's own kept softmax
-        const uint64_t total = use_res ? total_r : mass_j;
-        token = -1;                                                      // (a row with no weight at all: empty or all -inf)
-        if (total > 0ull && !bad) {
-          const float u = P.u_final ? P.u_final[0] : uniform01(seed, step, 4000u, 0u);
-          const uint64_t target = cdf_target(u, total);
-          // the block whose share holds the crossing: an exclusive prefix over the shares, one per thread
-          const uint64_t mine = tid < G ? (use_res ? (&s_red[0][0])[tid] : (&s_red[8][0])[tid]) : 0ull;
-          const uint64_t before = block_exclusive_scan_u64(mine, scratch, nullptr);
-          if (tid == 0) s_j2 = -1;
-          __syncthreads();
-          if (mine && before <= target && target < before + mine) { s_j2 = tid; s_pre2 = before; }
-          __syncthreads();
-          if (s_j2 >= 0) {
-            const int lo2 = min(V, s_j2 * per), len2 = min(V, lo2 + per) - lo2;
-            const VerifySlice V2{&P, (s_j2 == 0) ? zs : nullptr, (s_j2 == 0) ? qs : nullptr, per, lo2, row0, c2};   // block 0's own slice is in shared memory
-            token = locate(V2, lo2, len2, s_pre2, use_res, target);
-          }
-        }
-      }
-    } else {
-      // every draft accepted: the bonus row's own kept softmax; each block knows its share and its prefix from the masses' exchange
-      if (mass_j > 0ull) {
-        const float u = P.u_final ? P.u_final[0] : uniform01(seed, step, 4000u, 0u);
-        const uint64_t target = cdf_target(u, mass_j);
-        if (own_w > 0ull && pre_w <= target && target < pre_w + own_w) {   // the crossing lies in this block's slice
-          writer = true;
-          token = locate(S, lo, len, pre_w, false, target);
-        }
-      } else if (b == 0) { writer = true; token = -1; }                   // a row with no weight at all (empty or all -inf)
+template <bool F32, int Q>
+static __global__ void __launch_bounds__(kVerifyThreads, 2) verify_kernel(const __grid_constant__ VerifyDev P, int C, int z_cached, int q_cached) {
+  extern __shared__ __align__(16) uint4 v_smem[];
+  __shared__ VerifySmem s;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rank = C > 1 ? static_cast<int>(cluster_rank()) : 0, r = static_cast<int>(blockIdx.x) / C;
+  after_predecessor();
+  unsigned long long launch;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(launch) : "l"(&P.ws->launches) : "memory");
+  VerifyRound rd{P.n_draft, 0, P.seed, P.step, false, false, false};
+  if (P.state) {
+    StepStateView st{P.state, P.t_max, P.g};
+    if (st.done()) rd.idle = true;
+    else if (st.prefill_left() > 0u) { rd.idle = true; rd.prefill = true; }
+    else {
+      const uint32_t len = st.verify_len(), rows = st.t_this_step();
+      if (len > static_cast<uint32_t>(P.n_draft) || rows < len + 1u || rows > static_cast<uint32_t>(P.n_draft) + 1u) rd.mismatch = true;
+      else { rd.L = static_cast<int>(len); rd.row0 = static_cast<int>(rows - 1u - len); }
     }
-    if (bad) writer = b == 0;                                             // a wait ran out: block 0 reports it
-    if (writer && warp == 0) {
-      if (lane == 0) {
-        P.out_accept[0] = bad ? -1 : j; P.out_final[0] = bad ? -1 : token;
-        if (P.out_tokens) for (int r = 0; r < R; r++) P.out_tokens[row0 + r] = bad ? -1 : (r < j ? s_drafts[r] : (r == j ? token : -1));
-      }
-      verify_commit(P, bad);
+    rd.seed = st.seed(); rd.step = st.step();
+  }
+  if (rd.idle || rd.mismatch) {
+    // nothing is verified; block 0 still closes a prefill chunk (the scan's prefill branch) or reports the caller's error
+    if (blockIdx.x == 0 && warp == 0) {
+      if (rd.mismatch) {
+        if (lane == 0) { P.out_accept[0] = -1; P.out_final[0] = -1; StepStateView st{P.state, P.t_max, P.g}; fail_state(st, kErrRoundMismatch); }
+      } else if (rd.prefill) verify_commit(P, false);
     }
+  } else if (r <= rd.L) {                                                   // (a state may verify fewer rows than the launch has clusters)
+    if (C > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // this block runs, and has read the state
+    verify_row<F32, Q>(P, rd, r, rank, C, launch, z_cached != 0, q_cached != 0, v_smem, s);
   }
-  }
-  // ---- on the way out: one more block of this launch has left (nobody waits for the reply) -----------------------------------
-  __syncthreads();
-  if (tid == 0) asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(&P.ws->exits), "l"(1ull) : "memory");
 }
 
 }  // namespace lm
