@@ -124,13 +124,16 @@ static __global__ void __launch_bounds__(kDraftQThreads) draft_q_kernel(const Dr
     draft_chunks<F32>(R, kept, [&](int c, const RawChunk<F32>& q) {
       float z[8];
       widen_raw<F32>(R, q, c, z);
+      FloorSum sum;
+      const int i0 = 8 * c - R.off;
+      uint64_t x = g.first(i0);                                             // (the hash's arguments lie a constant apart)
 #pragma unroll
       for (int e = 0; e < 8; e += 2) {
-        uint64_t w0, w1;
-        weight_q40_x2(z[e], z[e + 1], vmax, c2, w0, w1);                    // (positions outside the row are -inf: weight 0, no key)
-        w += w0 + w1;
-        g.offer2(canon_zero(z[e]), static_cast<uint32_t>(8 * c + e - R.off), canon_zero(z[e + 1]), static_cast<uint32_t>(8 * c + e + 1 - R.off));
+        sum.add(weight_f2(z[e], z[e + 1], vmax, c2));                       // (positions outside the row are -inf: weight 0, no key)
+        g.offer2_at(canon_zero(z[e]), x, canon_zero(z[e + 1]), x + kHashStep, static_cast<uint32_t>(i0 + e));
+        x += 2u * kHashStep;
       }
+      w += sum.sum();
     });
     key = g.best; second = g.second;
   } else {                                                                  // a NaN, +inf, or nothing but -inf: every key, by the definition
