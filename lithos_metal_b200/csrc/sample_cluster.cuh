@@ -780,16 +780,19 @@ static __device__ __noinline__ int phase_select(ClusterSmem& s, float zf, bool n
   const float c2a = static_cast<float>(1.4426950408889634 * s.inv_t), nb = __fmul_rn(-s.vmax, c2a);
   FoundKeys found;
   found.init(s, begin_list(s, 0));
-  float acc = 0.0f;
+  float2 acc = make_float2(0.0f, 0.0f);
   {
     const ClusterRow R = s.R;
     sweep<F32, CACHED>(R, [&](int c, const float (&z)[8]) {
-      float mx = z[0];
+      const float mx = fmaxf(fmaxf(fmaxf(z[0], z[1]), fmaxf(z[2], z[3])), fmaxf(fmaxf(z[4], z[5]), fmaxf(z[6], z[7])));
+      if (need_z) {                                                         // (two at a time, a chunk's terms added up before they join the thread's sum)
+        float2 t[4];
 #pragma unroll
-      for (int e = 1; e < 8; e++) mx = fmaxf(mx, z[e]);
-      if (need_z) {
-#pragma unroll
-        for (int e = 0; e < 8; e++) acc += ex2_approx(__fmaf_rn(z[e], c2a, nb));
+        for (int k = 0; k < 4; k++) {
+          const float2 x = __ffma2_rn(make_float2(z[2 * k], z[2 * k + 1]), make_float2(c2a, c2a), make_float2(nb, nb));
+          t[k] = make_float2(ex2_approx(x.x), ex2_approx(x.y));
+        }
+        acc = __fadd2_rn(acc, __fadd2_rn(__fadd2_rn(t[0], t[1]), __fadd2_rn(t[2], t[3])));
       }
       if (mx >= zf) {
         uint32_t m = 0u;
@@ -803,7 +806,7 @@ static __device__ __noinline__ int phase_select(ClusterSmem& s, float zf, bool n
   found.flush();
   if (need_z) {
     // the common factor that nb's rounding leaves is taken out exactly
-    const double m = cblock_sum_f64(static_cast<double>(acc), s.scratch) * exp2(-(static_cast<double>(s.vmax) * static_cast<double>(c2a) + static_cast<double>(nb)));
+    const double m = cblock_sum_f64(static_cast<double>(acc.x) + static_cast<double>(acc.y), s.scratch) * exp2(-(static_cast<double>(s.vmax) * static_cast<double>(c2a) + static_cast<double>(nb)));
     if (static_cast<int>(threadIdx.x) < s.C) cst_u64(cluster_addr(&s.x_mass[s.rank], threadIdx.x), __double_as_longlong(m));
   }
   return end_list(s, found.counter);
@@ -1028,7 +1031,7 @@ static __device__ __noinline__ bool phase_top_k(ClusterSmem& s, const SampleDev&
   if (need_z) {
     for (int q = 0; q < C; q++) total += s.x_mass[q];
     const double un = 5.9604644775390625e-8;                                // sample_topk.cuh derives this bound (the reference point here is the maximum itself)
-    err = 1.25 * total * (un * (13.9 + 4.0 + 8.0 * ((s.per + B - 1) / B) + 1.0) + 6.6e-7);   // (ln V <= 13.9)
+    err = 1.25 * total * (un * (13.9 + 4.0 + static_cast<double>((s.per + B - 1) / B) + 3.0) + 6.6e-7);   // (ln V <= 13.9; a term goes through two additions in its chunk and one a step)
   }
   if (n_topk <= 64 && !s.want_stats) {
     // few candidates: one warp does the rest, with shuffles and votes (vocab_parallel.cuh); rank 0's writes the outputs
