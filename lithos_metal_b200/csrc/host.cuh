@@ -33,7 +33,7 @@ inline int sm_count(int* out) {
 // Kernels that need more than 48 KB of shared memory, their static arrays included, must be told so once per device (the attribute belongs to the
 // device's copy of the function). They are told whatever they ask for, so that nothing here has to know their arrays; remembered per device and kernel,
 // raised when a call needs more.
-enum KernelSlot { kSlotFast, kSlotTopk, kSlotGeneric, kSlotVocabLocal, kSlotTileFinish, kSlotSlice, kSlotSliceSmall, kSlotSliceTiny, kSlotSlicedMerge, kSlotHead, kSlotCluster,
+enum KernelSlot { kSlotFast, kSlotTopk, kSlotTopkOrdered, kSlotGeneric, kSlotVocabLocal, kSlotTileFinish, kSlotSlice, kSlotSliceSmall, kSlotSliceTiny, kSlotSlicedMerge, kSlotHead, kSlotCluster,
                   kSlotArgmax = kSlotCluster + 6,   // (the cluster kernel has six instances, the argmax kernel two)
                   kSlotDraftQ = kSlotArgmax + 2,    // (two instances)
                   kSlotVerify = kSlotDraftQ + 2,    // (six, and six for blocks that have an SM to themselves)

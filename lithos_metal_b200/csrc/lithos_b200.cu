@@ -97,7 +97,7 @@ float lm_uniform01(uint64_t seed, uint32_t step, uint32_t t, uint32_t index) { r
 size_t lm_workspace_bytes(int64_t rows, int64_t vocab) {
   (void)vocab;
   if (rows < 0) rows = 0;
-  // (16 bytes a row, free) | rows for the generic kernel | rows that are not the top-k kernel's | rows the top-k kernel left | counters
+  // the top-k kernel's rows in order (16 bytes a row, 4 of them used) | rows for the generic kernel | rows that are not the top-k kernel's | rows the top-k kernel left | counters
   //   | the slice records of a call of a few rows
   return align256(static_cast<size_t>(rows) * 16) + 3 * align256(static_cast<size_t>(rows) * sizeof(uint32_t)) + 256 + kSlicedWsBytes;
 }
@@ -245,10 +245,11 @@ int lm_sample(const lm_sample_args* a) {
     int* list_left = reinterpret_cast<int*>(ws + 2 * rows_bytes);          // rows the top-k kernel left
     int* counters = reinterpret_cast<int*>(ws + 3 * rows_bytes);
     // counters: 0 next row of the top-k kernel, 1 length of list_left, 2 next item of the histogram kernel, 3 length of redo,
-    //           4 length of list_other, 5 next of the rows the top-k kernel left
+    //           4 length of list_other, 5 next of the rows the top-k kernel left, 6 and 7 its rows with a large and a small top_k
     const size_t hist_smem = hist_smem_bytes(static_cast<int>(a->vocab));
     rc = ensure_dynamic_smem(kSlotFast, reinterpret_cast<const void*>(sample_hist_kernel), hist_smem);
-    if (rc == LM_OK) rc = ensure_dynamic_smem(kSlotTopk, reinterpret_cast<const void*>(sample_topk_kernel), sizeof(TopkSmem));
+    if (rc == LM_OK) rc = ensure_dynamic_smem(kSlotTopk, reinterpret_cast<const void*>(sample_topk_kernel<false>), sizeof(TopkSmem));
+    if (rc == LM_OK) rc = ensure_dynamic_smem(kSlotTopkOrdered, reinterpret_cast<const void*>(sample_topk_kernel<true>), sizeof(TopkSmem));
     if (rc != LM_OK) return rc;
     const bool topk = !(a->flags & LM_FLAG_EXACT_ONLY) && a->vocab >= kTopkMinVocab && (a->top_k != nullptr || (a->top_k_s >= 1 && a->top_k_s <= kTopkMaxK)) &&
                       (a->temperature != nullptr || a->temperature_s > 0.0f) && (!pen || a->hist_len <= kTopkHist);
@@ -267,14 +268,18 @@ int lm_sample(const lm_sample_args* a) {
     } else {
       // Every launch of the call waits on the device for what it needs of the one in front, so that none of them begins with a gap (us per call so /
       // one after the other: 256 penalised rows 82 / 132, 4096 635 / 703; a memset and gaps in place of the preparation alone were 10 and 6 of it).
-      rc = launch_stream(beside, sample_prep_kernel, 1, kPrepThreads, 0, 1, st, P, list_other, counters);
+      // Where the length of a launch is that of its longest rows, the top-k kernel takes those with a large top_k first: the last ones, which begin when others are done, are
+      // short then (256 penalised rows, 40 seeds: median 66.4 -> 60.0 us; 160 72.4 -> 62.1; 256 of 50,264 without penalties 47.6 -> 41; a claim costs a trip to the list: 200 rows 73.7 -> 74.0).
+      const bool side = !(one_k || a->rows > static_cast<int64_t>(kOverlapRowsPerSM) * sms);
+      int* order = side && a->top_k != nullptr && a->rows > grid1 / 2 ? reinterpret_cast<int*>(a->workspace) : nullptr;
+      rc = launch_stream(beside, sample_prep_kernel, 1, kPrepThreads, 0, 1, st, P, list_other, counters, order);
       if (rc != LM_OK) return rc;
-      if (one_k || a->rows > static_cast<int64_t>(kOverlapRowsPerSM) * sms) {
+      if (!side) {
         // Many rows per SM, or hardly a row for the histogram kernel (one top_k for all: 148 rows 56 us side by side, 43 so): the top-k kernel first,
         // the histogram kernel behind it with programmatic stream serialization: its blocks take an SM over as the top-k blocks leave it, work
         // through the rows that the preparation has listed for it, wait for the top-k grid, and absorb the few rows that one handed
         // on. (4096 penalised rows 635 us, behind its end 700; 800 rows 156 and 193.)
-        rc = launch_stream(beside, sample_topk_kernel, grid1, kTB, sizeof(TopkSmem), 1, st, P, list_left, counters, 1);
+        rc = launch_stream(beside, sample_topk_kernel<false>, grid1, kTB, sizeof(TopkSmem), 1, st, P, list_left, counters, 1, none);
         if (rc == LM_OK) rc = launch_stream(beside, sample_hist_kernel, grid, kHB, hist_smem, 1, st, P, list_other, counters + kCounterOther, counters + 2, redo, counters + 3,
                                             list_left, counters + 1, counters + 5);
         if (rc != LM_OK) return rc;
@@ -296,7 +301,8 @@ int lm_sample(const lm_sample_args* a) {
         }
         rc = launch_stream(beside, sample_hist_kernel, grid_first, kHB, hist_smem_first, 1, st, P, list_other, counters + kCounterOther, counters + 2, redo, counters + 3,
                            none, none, none_mut);
-        if (rc == LM_OK) rc = launch_stream(beside, sample_topk_kernel, grid1, kTB, sizeof(TopkSmem), 1, st, P, list_left, counters, 0);
+        if (rc == LM_OK) rc = order ? launch_stream(beside, sample_topk_kernel<true>, grid1, kTB, sizeof(TopkSmem), 1, st, P, list_left, counters, 0, static_cast<const int*>(order))
+                                    : launch_stream(beside, sample_topk_kernel<false>, grid1, kTB, sizeof(TopkSmem), 1, st, P, list_left, counters, 0, none);
         if (rc == LM_OK) rc = launch_stream(beside, sample_hist_kernel, grid, kHB, hist_smem, 1, st, P, list_left, counters + 1, counters + 5, redo, counters + 3, none, none, none_mut);
         if (rc != LM_OK) return rc;
       }

@@ -134,24 +134,33 @@ __device__ __forceinline__ bool topk_row_eligible(const SampleDev& P, int row) {
 
 // What the row kernels of a call share in the workspace: the counters begin at zero, the rows that are not the top-k kernel's are listed for the
 // histogram kernel. One block: it clears and counts without a memset of its own in front (2 us of every call).
-constexpr int kPrepThreads = 1024, kCounters = 8, kCounterOther = 4;
-static __global__ void __launch_bounds__(kPrepThreads) sample_prep_kernel(SampleDev P, int* list, int* counters) {
-  __shared__ int n;
-  if (threadIdx.x == 0) n = 0;
+// order: optional, the top-k kernel's own rows in the order in which its blocks take them: those with a large top_k from the front, the others from the back.
+constexpr int kPrepThreads = 1024, kCounters = 8, kCounterOther = 4, kCounterLong = 6, kCounterShort = 7;
+static __global__ void __launch_bounds__(kPrepThreads) sample_prep_kernel(SampleDev P, int* list, int* counters, int* order) {
+  __shared__ int n, n_long, n_short;
+  if (threadIdx.x == 0) n = n_long = n_short = 0;
   after_predecessor();
   apply_step_state(P);
   __syncthreads();
-  if (threadIdx.x < kCounters && threadIdx.x != kCounterOther) counters[threadIdx.x] = 0;
+  if (threadIdx.x < kCounterOther || threadIdx.x == 5) counters[threadIdx.x] = 0;
   constexpr int kU = 4;                                                     // rows of a thread whose knobs are in flight
   for (int r0 = threadIdx.x; r0 < P.rows; r0 += kU * kPrepThreads) {
-    bool other[kU];
+    bool other[kU]; int top_k[kU];
 #pragma unroll
-    for (int j = 0; j < kU; j++) { const int row = r0 + j * kPrepThreads; other[j] = row < P.rows && !topk_row_eligible(P, row); }
+    for (int j = 0; j < kU; j++) {
+      const int row = r0 + j * kPrepThreads;
+      other[j] = row < P.rows && !topk_row_eligible(P, row);
+      top_k[j] = order != nullptr && row < P.rows && P.top_k ? P.top_k[row] : 0;
+    }
 #pragma unroll
-    for (int j = 0; j < kU; j++) if (other[j]) list[atomicAdd(&n, 1)] = r0 + j * kPrepThreads;
+    for (int j = 0; j < kU; j++) {
+      const int row = r0 + j * kPrepThreads;
+      if (other[j]) list[atomicAdd(&n, 1)] = row;
+      else if (order != nullptr && row < P.rows) order[top_k[j] > kFew ? atomicAdd(&n_long, 1) : P.rows - 1 - atomicAdd(&n_short, 1)] = row;
+    }
   }
   __syncthreads();
-  if (threadIdx.x == 0) counters[kCounterOther] = n;
+  if (threadIdx.x == 0) { counters[kCounterOther] = n; counters[kCounterLong] = n_long; counters[kCounterShort] = n_short; }
 }
 
 // How many logits of the row lie at or above code a (low word) and code b (high word); every thread calls.
@@ -906,7 +915,15 @@ static __device__ bool topk_finish(const SampleDev& P, int row, TopkSmem& c, uin
 // Rows are handed out through a counter in the workspace (counters[0], zeroed by sample_prep_kernel): a block takes
 // the next row, passes over it if it is not this kernel's (sample_prep_kernel has listed it), and else either finishes it or appends it to
 // `list` (length in counters[1]) for the histogram kernel. The order of the list varies from run to run; what is computed per row does not.
-static __global__ void __launch_bounds__(kTB, kTopkPerSM) sample_topk_kernel(SampleDev P, int* list, int* counters, int first) {
+// The row that is taken as the i-th (sample_prep_kernel); rows: there is none.
+static __device__ __noinline__ int topk_row_at(const int* order, const int* counters, int rows, int i) {
+  const int n_long = __ldcg(counters + kCounterLong), n_short = __ldcg(counters + kCounterShort);   // (from L2: the preparation is two launches back, without an end between)
+  return i < n_long ? __ldcg(order + i) : i < n_long + n_short ? __ldcg(order + rows - 1 - (i - n_long)) : rows;
+}
+
+// kOrdered: the rows in the order in which they are taken; else all rows as they come (compiled apart: the look-up cost the others 0.3 %).
+template <bool kOrdered>
+static __global__ void __launch_bounds__(kTB, kTopkPerSM) sample_topk_kernel(SampleDev P, int* list, int* counters, int first, const int* order) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   TopkSmem& c = *reinterpret_cast<TopkSmem*>(smem_raw);
   __shared__ int item[2];                                                   // the row in hand and the one after it
@@ -925,19 +942,26 @@ static __global__ void __launch_bounds__(kTB, kTopkPerSM) sample_topk_kernel(Sam
   // 58.4 / 61.0, 100 56.8 / 59.6, 350 63.2 / 67.2; 400 rows, 100 58.4 / 61.9, 400 64.7 / 68.3, 1000 69.8 / 70.2; with half as many again the first half is too
   // few: 440 rows, top_k 400 74.2 / 64.9.)
   const bool once = first && P.rows * 8LL <= gridDim.x * 11LL && blockIdx.x >= (gridDim.x + 1u) / 2u;
-  if (threadIdx.x == 0) { item[0] = atomicAdd(&counters[0], 1); item[1] = (ahead && item[0] < P.rows) ? atomicAdd(&counters[0], 1) : P.rows; }
+  auto claim = [&]() {                                                      // (thread 0)
+    const int i = atomicAdd(&counters[0], 1);
+    return kOrdered ? topk_row_at(order, counters, P.rows, i) : i;
+  };
+  if (threadIdx.x == 0) {
+    item[0] = claim();
+    item[1] = (ahead && item[0] < P.rows) ? claim() : P.rows;
+  }
   __syncthreads();
   for (;;) {
     const int row = item[0], next = item[1];
     if (row >= P.rows) break;
     int fetched = P.rows;
-    if (threadIdx.x == 0 && next < P.rows) fetched = atomicAdd(&counters[0], 1);
+    if (threadIdx.x == 0 && next < P.rows) fetched = claim();
     if (topk_row_eligible(P, row)) {
       const bool done = topk_row(P, row, next < P.rows ? next : -1, c);
       if (threadIdx.x == 0 && !done) list[atomicAdd(&counters[1], 1)] = row;
     }
     __syncthreads();                                                        // nobody reads item[] any more
-    if (threadIdx.x == 0) { item[0] = once ? P.rows : ahead ? next : atomicAdd(&counters[0], 1); item[1] = fetched; }
+    if (threadIdx.x == 0) { item[0] = once ? P.rows : ahead ? next : claim(); item[1] = fetched; }
     __syncthreads();
   }
   // This grid may have been started before the grid launched ahead of it had finished (programmatic stream serialization). The
