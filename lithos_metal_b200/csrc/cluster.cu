@@ -117,7 +117,7 @@ int argmax_clusters(const void* logits, int dtype, int rows, int vocab, int64_t 
 }
 
 template <bool F32>
-static int launch_draft_q(const DraftQDev& P, int C, cudaStream_t st) {
+static int launch_draft_q(const DraftQDev& P, int C, int sms, cudaStream_t st) {
   const KernelSlot slot = static_cast<KernelSlot>(kSlotDraftQ + (F32 ? 1 : 0));
   const void* fn = reinterpret_cast<const void*>(draft_q_kernel<F32>);
   const int rc = ensure_dynamic_smem(slot, fn, kAloneSmem, true);
@@ -125,14 +125,16 @@ static int launch_draft_q(const DraftQDev& P, int C, cudaStream_t st) {
   C = cluster_that_fits(C, [&](int c) { return cluster_fits(slot, fn, kDraftQThreads, kAloneSmem, c); });
   // A block asks for more than half of an SM's shared memory, so that no two of them lie on one while others are idle: made ready beside a predecessor they
   // pile up where that has left room (7 rows of 151,936 behind the verification of the round before: the round 40.0 us, 38.7 so; 15 rows of 248,320 68 to 70 and 62). Not
-  // where all clusters would then not run at once.
-  const size_t alone = clusters_at_once(slot, fn, kDraftQThreads, kAloneSmem, C) >= P.rows ? kAloneSmem : 0;
-  return launch_beside(draft_q_kernel<F32>, dim3(static_cast<unsigned>(P.rows) * static_cast<unsigned>(C)), kDraftQThreads, alone, C, st, P, C);
+  // where all clusters would then not run at once: with a few blocks more than SMs they share some (8 rows of 151,936 12.3 us), with half as many again eight
+  // blocks to a row, an SM each, are faster (11 rows 14.4 / 12.6, 14 rows of 262,144 18.5 / 17.8).
+  auto at_once = [&](int c) { return clusters_at_once(slot, fn, kDraftQThreads, kAloneSmem, c) >= P.rows; };
+  if (C > 1 && !at_once(C) && P.rows * C * 6 > sms * 7 && at_once(C / 2)) C /= 2;
+  return launch_beside(draft_q_kernel<F32>, dim3(static_cast<unsigned>(P.rows) * static_cast<unsigned>(C)), kDraftQThreads, at_once(C) ? kAloneSmem : 0, C, st, P, C);
 }
 
 int draft_q_clusters(const DraftQDev& P, int sms, cudaStream_t st) {
   const int C = cluster_blocks(P.rows, P.vocab, 2 * sms);                   // (two of these blocks share an SM)
-  return P.dtype == LM_DTYPE_F32 ? launch_draft_q<true>(P, C, st) : launch_draft_q<false>(P, C, st);
+  return P.dtype == LM_DTYPE_F32 ? launch_draft_q<true>(P, C, sms, st) : launch_draft_q<false>(P, C, sms, st);
 }
 
 // The verification: a cluster per target row, as many blocks each as let all of them run at once.
