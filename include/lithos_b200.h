@@ -249,8 +249,8 @@ typedef struct lm_verify_args {
                                   gives unspecified tokens (never a hang). NULL: the kernel finds the maxima itself. */
   const uint64_t* target_mass; /* with target_vmax, optional: per row the fixed-point mass of its kept set {z >= tau} at `temperature`, as
                                   lm_sample_args.out_mass gives it for the same rows, thresholds and temperature (the other half of
-                                  the reference's KEPT_STATS). Every block then runs the accept test by itself and the launch has a
-                                  single exchange left (the draw). Ignored without target_vmax. */
+                                  the reference's KEPT_STATS). Every block then runs the accept test by itself, and only the
+                                  blocks of the decisive row meet again (the draw). Ignored without target_vmax. */
 } lm_verify_args;
 
 #define LM_RESIDUAL_INVERSE_CDF 0 /* final token by inverse CDF, in ascending index order, over max(p - q, 0) (over p on the bonus row) from u_final */

@@ -589,7 +589,7 @@ static __device__ bool topk_row(const SampleDev& P, int row, int next, TopkSmem&
   return topk_finish(P, row, c, cut_code, zm);
 }
 
-// The row's softmass in FP64, for the rare row (one in a few hundred) whose top-p boundary the FP32 mass cannot decide. ~15 FP64 operations per
+// The row's softmass in FP64, for the rare row (one in some 4000 of the benchmark's) whose top-p boundary the FP32 mass cannot decide. ~15 FP64 operations per
 // logit from L2: less than the histogram kernel would take for the whole row, and behind no other launch. The candidates' keys are dead.
 static __device__ double topk_exact_mass(const SampleDev& P, TopkSmem& c, const RowMass& zm, float vmax, double inv_t) {
   double* tab = reinterpret_cast<double*>(c.key);
