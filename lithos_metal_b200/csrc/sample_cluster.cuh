@@ -47,7 +47,9 @@ constexpr int kCMaxRanks = 16;           // blocks of one cluster
 constexpr int kCQueue = 128;             // logits a warp's queue of the Gumbel draw holds
 constexpr uint32_t kCallOrdered = 1u, kCallFew = 2u;   // of a launch: the rows are taken by kind; a call of a few rows with one top_k (LM_STATUS_SLICED_PATH)
 constexpr int kOrderRows = 2048;         // rows whose order a block looks up (row_in_order)
-constexpr int kCRankOrder = 160;         // a list up to this long is ordered by counting larger keys, a longer one by bins first (472 keys: 7.7 us by counting, 1.5 by bins)
+// A list up to this long is ordered by counting larger keys, a longer one by bins first (472 keys: 7.7 us by counting, 1.5 by bins). us a call of 12 FP32 rows, by counting / by bins:
+// top_k 64 15.16 / 15.44, 80 16.10 / 16.33, 100 16.38 / 16.46, 120 16.63 / 16.50, 140 16.98 / 16.58.
+constexpr int kCRankOrder = 110;
 constexpr double kCMassBand = 1e-11;     // relative error of a logit's fixed-point softmass beyond its rounding: 7e-12 of the polynomial, a few 1e-16
 // Threads per block: a block-wide reduction costs shuffles in proportion to its warps (1024 threads: 0.5 us each, measured), so no more
 // warps than the sweeps need.
