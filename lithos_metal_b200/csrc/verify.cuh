@@ -688,7 +688,8 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
   }
   if (!(before <= target && target < before + parts[warp])) return;         // ... in another warp's range
   // the first element, in index order, at which the running weight passes the target: the chunk from the chunks' sums, then a lane for each of its elements
-  const bool kept_values = z_cached && q_cached && (has_q || given_mass) && residual == has_q;   // the draw's weights lie in the drafter's place
+  // ... where the draw's weights lie: in the drafter's place, or where the row itself is drawn from in the logits' place; a residual that was not kept is formed again
+  const bool kept_values = z_cached && q_cached && (has_q || given_mass) && residual == has_q;
   int token = -1;
 #pragma unroll 1
   for (int b0 = w0; b0 < w1; b0 += 32) {
@@ -713,7 +714,7 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
       run = __shfl_sync(kFull, run, ch - b0);
       uint64_t v;
       if (few) v = (kept_of(ch) >> e) & 1u ? verify_element<F32, Q>(s.row, 8 * ch + e - off, z_at(ch, e), residual, vmax) : 0ull;
-      else if (kept_values || weighed) v = __float2ull_rz(reinterpret_cast<const float*>((kept_values ? qs : zs) + (h ? per : 0) + ch)[e & 3]);
+      else if (kept_values || (weighed && !residual)) v = __float2ull_rz(reinterpret_cast<const float*>((kept_values ? qs : zs) + (h ? per : 0) + ch)[e & 3]);
       else {
         const float4 x = half_weight(ch, h, weighed);
         v = __float2ull_rz((e & 2) ? ((e & 1) ? x.w : x.z) : ((e & 1) ? x.y : x.x));

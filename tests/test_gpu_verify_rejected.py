@@ -1,0 +1,71 @@
+"""Replacement tokens of rejected drafts (the draw over max(p - q, 0)) in every layout of the verification's slices: the drafter's row beside the target's in shared
+memory, the target's alone, neither. Every case asserts that a draft was rejected and that something of p - q is left. Against the CPU oracle (exact)."""
+import numpy as np
+import pytest
+import torch
+
+import lithos_metal_b200 as lm
+import oracle
+from tests.test_gpu_sampling import bf16_tensor
+from tests.test_gpu_verify_slices import check, on_gpu, step
+
+pytestmark = pytest.mark.gpu
+LAST = np.float32(1.0 - 2.0**-24)                                            # the largest uniform
+
+
+def rejecting(z, q, at, T=1.0, tau=None):
+    """Drafts and accept uniforms of which the one at `at` is the first to be rejected: likely tokens before it, from it on the one where q exceeds p by most."""
+    n = len(q)
+    drafts, ua = z[:n].argmax(-1).astype(np.int32), np.zeros(n, np.float32)
+    for r in range(at, n):
+        p = np.exp((z[r].astype(np.float64) - z[r].max()) / T) * (True if tau is None else z[r] >= tau[r])
+        drafts[r], ua[r] = np.argmax(q[r] - p / p.sum()), LAST
+    return drafts, ua
+
+
+# 16 blocks a row up to 13 drafts, 8 beyond: (50257, 7) holds both rows, (700001, 2) neither, the others the target's alone
+@pytest.mark.parametrize("vocab,n", [(248320, 1), (248320, 7), (262144, 7), (262143, 13), (151936, 14), (151936, 15), (50257, 7), (700001, 2)])
+@pytest.mark.parametrize("dtype", ["bf16", "fp32"])
+def test_first_rejected_draft_is_replaced(vocab, n, dtype):
+    rng, target, noisy, q = step(vocab, n, dtype, vocab + 3 * n)
+    z = oracle.bf16_to_f32(target) if dtype == "bf16" else target
+    lb = oracle.f32_to_bf16(noisy)
+    stats = lm.draft_q(bf16_tensor(lb), temperature=0.7, seed=3)
+    q2 = np.stack([oracle.draft_probs(lb[k], temperature=0.7, vmax=float(stats.vmax[k]), mass=int(stats.mass[k])) for k in range(n)])
+    tau = np.partition(z, vocab - min(300, vocab), axis=-1)[:, vocab - min(300, vocab)].astype(np.float32)
+    for at in sorted({0, n // 2, n - 1}):
+        for kept in (None, tau):
+            d, ua = rejecting(z, q, at, tau=kept)
+            acc, fin, _ = oracle.verify_stochastic(target, d, q, ua, 0.5, tau=kept)
+            assert acc == at and fin >= 0
+            for uf in (rng.random(), 0.0, LAST):
+                check(target, d, q, ua, np.float32(uf), tau=kept)
+        d, ua = rejecting(z, q2, at, 0.7)
+        assert oracle.verify_stochastic(target, d, q2, ua, 0.5, temperature=0.7)[0] == at
+        check(target, d, q2, ua, np.float32(rng.random()), gpu_q=dict(draft_logits=bf16_tensor(lb), draft_stats=stats), temperature=0.7)
+
+
+@pytest.mark.parametrize("draft_form", ["probabilities", "logits"])
+def test_replaced_in_a_round_that_closes_itself(draft_form):
+    """With a StepState that the launch reads and moves on: the state's token is the oracle's."""
+    vocab, n, at, T = 248320, 7, 3, 0.7
+    layout = lm.StepStateLayout(n + 1, n)
+    rng, target, noisy, q = step(vocab, n, "bf16", 11)
+    z = oracle.bf16_to_f32(target)
+    lb = oracle.f32_to_bf16(noisy)
+    stats = lm.draft_q(bf16_tensor(lb), temperature=T, seed=3)
+    if draft_form == "logits":
+        q = np.stack([oracle.draft_probs(lb[k], temperature=T, vmax=float(stats.vmax[k]), mass=int(stats.mass[k])) for k in range(n)])
+    d, ua = rejecting(z, q, at, T)
+    uf = np.float32(rng.random())
+    acc, fin, _ = oracle.verify_stochastic(target, d, q, ua, uf, temperature=T)
+    assert acc == at
+    st = layout.to_device(dict(step=2, verify_len=n, t_this_step=n + 1, pending_tokens=[5] + d.tolist(), position=40, kv_len=40))
+    ring = torch.zeros(64, dtype=torch.int64, device="cuda")
+    out = lm.verify(on_gpu(target), None, torch.from_numpy(q).cuda() if draft_form == "probabilities" else None, torch.from_numpy(ua).cuda(), torch.tensor([uf]), "stochastic",
+                    temperature=T, step_state=(layout, st), commit=dict(layout=layout, state=st, ring=ring),
+                    **(dict(draft_logits=bf16_tensor(lb), draft_stats=stats) if draft_form == "logits" else {}))
+    assert (int(out[0]), int(out[1])) == (acc, fin)
+    after = layout.from_device(st)
+    assert [int(t) & 0xFFFFFFFF for t in ring[:acc + 1].tolist()] == d[:acc].tolist() + [fin]
+    assert after["anchor"] == fin and after["accepted"] == at and after["step"] == 3
