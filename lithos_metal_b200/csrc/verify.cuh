@@ -541,8 +541,8 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
   auto best_of_rest = [&](uint64_t there) {
     ResidualScan rest;
     rest.init(rd.seed, rd.step, 4000u);
-    if (there == 0ull) return rest.best;
-    float bar = logf(__ull2float_rn(there) * 0x1p-40f) - 1.5f;
+    // (Floors that add up to nothing leave residuals below 2^-40, which have their keys all the same: the first is looked for without a bar.)
+    float bar = there ? logf(__ull2float_rn(there) * 0x1p-40f) - 1.5f : -INFINITY;
 #pragma unroll 1
     for (;;) {
       rest.room = 8388608.0f * ex2_approx((2e-3f - bar) * 1.44269504f);

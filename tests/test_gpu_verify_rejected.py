@@ -69,3 +69,27 @@ def test_replaced_in_a_round_that_closes_itself(draft_form):
     after = layout.from_device(st)
     assert [int(t) & 0xFFFFFFFF for t in ring[:acc + 1].tolist()] == d[:acc].tolist() + [fin]
     assert after["anchor"] == fin and after["accepted"] == at and after["step"] == 3
+
+
+# every layout again (both rows in shared memory, the target's alone, neither), a threshold that cuts nothing, statistics given or not (check)
+@pytest.mark.parametrize("vocab,n", [(151936, 7), (262144, 7), (151936, 15), (700001, 2)])
+@pytest.mark.parametrize("dtype", ["bf16", "fp32"])
+def test_residuals_below_the_fixed_point_have_their_keys(vocab, n, dtype):
+    """A flat row, and a drafter an ulp below it: p - q is less than 2^-40 everywhere. The reference's draw takes the best ln(p - q) + noise all the same (the
+    inverse CDF, on floors of 2^-40, draws from the row itself). Then with a few residuals above 2^-40 in one place, and with one positive one at the very end."""
+    host = np.zeros((n + 1, vocab), np.float32)
+    target = oracle.f32_to_bf16(host) if dtype == "bf16" else host
+    p = np.float32(1.0) / np.float32(vocab)
+    q = np.full((n, vocab), np.nextafter(p, np.float32(0.0)), np.float32)
+    d, ua = np.full(n, 77, np.int32), np.zeros(n, np.float32)
+    at = n // 2
+    q[:, 77], ua[at] = 2 * p, LAST
+    some, last = q.copy(), np.full_like(q, 1.0)
+    some[:, 5000:5003] = p - np.float32(2.0**-38)
+    last[:, vocab - 1] = np.nextafter(p, np.float32(0.0))
+    for x in (q, some, last):
+        acc, fin, _ = oracle.verify_gumbel(target, d, x, seed=17, step=5, u_accept=ua)
+        assert acc == at and 0 < p - x[at, vocab - 1] < 2.0**-40
+        for kept in (None, np.full(n + 1, -1.0, np.float32)):
+            check(target, d, x, ua, np.float32(0.3), tau=kept)
+    assert fin == vocab - 1
