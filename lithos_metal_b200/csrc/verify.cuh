@@ -234,15 +234,22 @@ static __device__ __noinline__ uint64_t verify_element(const VerifyRow& x, int i
   return d > 0.0f ? residual_q40(d) : 0ull;
 }
 
-// Every warp for itself: the slots' sum, and the sum of the slots before slot `at`.
-__device__ __forceinline__ uint64_t verify_prefix(const unsigned long long* slots, int n, int at, uint64_t* before) {
+// Every warp for itself: the slots' running sums, a lane per slot, and their sum.
+struct VerifySums { uint64_t mine, incl; };
+__device__ __forceinline__ uint64_t verify_sums(const unsigned long long* slots, int n, VerifySums& v) {
   const int lane = threadIdx.x & 31;
-  const uint64_t mine = lane < n ? slots[lane] : 0ull;
-  uint64_t incl = mine;
+  v.incl = v.mine = lane < n ? slots[lane] : 0ull;
 #pragma unroll
-  for (int o = 1; o < kCMaxRanks; o <<= 1) { const uint64_t t = __shfl_up_sync(kFull, incl, o); if (lane >= o) incl += t; }
-  *before = __shfl_sync(kFull, incl - mine, at);
-  return __shfl_sync(kFull, incl, kCMaxRanks - 1);
+  for (int o = 1; o < kCMaxRanks; o <<= 1) { const uint64_t t = __shfl_up_sync(kFull, v.incl, o); if (lane >= o) v.incl += t; }
+  return __shfl_sync(kFull, v.incl, kCMaxRanks - 1);
+}
+// The slot in which the running sum passes `left`, which then counts from that slot's start; -1: none. It is one slot at most, the same for whoever asks, whatever
+// the sums are: masses that are not the rows' can make them pass 2^64, and then more than one slot, or none, would hold the point.
+__device__ __forceinline__ int verify_slot(const VerifySums& v, uint64_t& left) {
+  const uint32_t hit = __ballot_sync(kFull, v.incl - v.mine <= left && left < v.incl);
+  const int at = __ffs(static_cast<int>(hit)) - 1;
+  left -= __shfl_sync(kFull, v.incl - v.mine, at < 0 ? 0 : at);
+  return at;
 }
 static_assert(kVerifyWarps <= kCMaxRanks && kCMaxRanks <= 32, "slots of ranks and of warps alike, a lane each");
 
@@ -476,6 +483,7 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
   auto half_weight = [&](int c, int h, bool stored) { return verify_half<F32, Q>(s.row, stored ? zs[(h ? per : 0) + c] : z_raw(c, h), c, h, stored, residual, vmax); };
   const bool direct = given_mass && !(P.state && P.commit);                 // (a commit changes the state that blocks of other rows may not have read yet)
   unsigned long long mass = 0ull;
+  VerifySums shares;                                                        // the blocks' shares of what is drawn from
   int j = r;
   if (given_mass) {
     if (tester) {
@@ -514,8 +522,7 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
     join();
     if (warp == 0) push(s.x_own, warp_sum_u64(lane < kVerifyWarps ? s.own[lane] : 0ull), true);
     cluster_sync(C);
-    uint64_t unused;
-    mass = verify_prefix(s.x_own, C, 0, &unused);
+    mass = verify_sums(s.x_own, C, shares);
     if (has_q) {
       if (tester) {
         const bool no = test(drafter ? t_q : t_prob(vmax, mass), rank == 0);
@@ -585,10 +592,10 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
     }
     return own.best;
   };
-  const unsigned long long *slots = s.x_own, *parts = reinterpret_cast<const unsigned long long*>(s.own);
-  uint64_t before = 0ull, there = 0ull;                                     // the weight before this block's slice; all of it
+  const unsigned long long* parts = reinterpret_cast<const unsigned long long*>(s.own);
+  uint64_t there = mass;                                                    // the weight of all blocks (or the best key)
   if (has_q || given_mass || gumbel) {
-    slots = s.x_res; parts = reinterpret_cast<const unsigned long long*>(s.res);
+    parts = reinterpret_cast<const unsigned long long*>(s.res);
     residual = has_q;
     bool first = true;
 #pragma unroll 1
@@ -666,33 +673,31 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
         push(s.x_res, gumbel ? warp_max_u64(w) : warp_sum_u64(w), true);
       }
       cluster_sync(C);
-      there = gumbel ? warp_max_u64(lane < C ? slots[lane] : 0ull) : verify_prefix(slots, C, rank, &before);
+      there = gumbel ? warp_max_u64(lane < C ? s.x_res[lane] : 0ull) : verify_sums(s.x_res, C, shares);
       if (there || !residual) break;
       cluster_sync(C);                                                      // (everybody has read the slots)
     }
-  } else there = verify_prefix(slots, C, rank, &before);
+  }
   if (gumbel) {
     if (rank == 0 && warp == 0) deliver(there ? static_cast<int>(best_index(there)) : -1);
     return;
   }
-  const uint64_t total = residual ? there : mass, target = cdf_target(P.u_final ? u_final : uniform01(rd.seed, rd.step, 4000u, 0u), total);
-  if (total == 0ull || target >= there) {                                   // a row with no weight at all (empty or all -inf), or a given mass that is not the row's
-    if (rank == 0 && warp == 0) deliver(-1);
+  uint64_t left = cdf_target(P.u_final ? u_final : uniform01(rd.seed, rd.step, 4000u, 0u), residual ? there : mass);
+  const int block = verify_slot(shares, left);
+  if (block != rank) {                                                      // none: a row with no weight at all (empty or all -inf), or a given mass that is not the row's
+    if (block < 0 && rank == 0 && warp == 0) deliver(-1);
     return;
   }
-  if (!(before <= target && target < before + slots[rank])) return;         // the crossing lies in another block's slice
-  {
-    uint64_t in_block;
-    verify_prefix(parts, kVerifyWarps, warp, &in_block);
-    before += in_block;
-  }
-  if (!(before <= target && target < before + parts[warp])) return;         // ... in another warp's range
+  VerifySums mine;
+  verify_sums(parts, kVerifyWarps, mine);
+  const int part = verify_slot(mine, left);
+  if (warp != max(part, 0)) return;
   // the first element, in index order, at which the running weight passes the target: the chunk from the chunks' sums, then a lane for each of its elements
   // ... where the draw's weights lie: in the drafter's place, or where the row itself is drawn from in the logits' place; a residual that was not kept is formed again
   const bool kept_values = z_cached && q_cached && (has_q || given_mass) && residual == has_q;
   int token = -1;
 #pragma unroll 1
-  for (int b0 = w0; b0 < w1; b0 += 32) {
+  for (int b0 = w0; b0 < w1 && part >= 0; b0 += 32) {
     const int c = b0 + lane;
     uint64_t sum = 0ull;
     if (c < w1) {
@@ -707,8 +712,8 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
     uint64_t incl = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) { const uint64_t t = __shfl_up_sync(kFull, incl, o); if (lane >= o) incl += t; }
-    uint64_t run = before + incl - sum;
-    const uint32_t hit = __ballot_sync(kFull, run <= target && target < run + sum);
+    uint64_t run = incl - sum;
+    const uint32_t hit = __ballot_sync(kFull, run <= left && left < incl);
     if (hit) {
       const int ch = b0 + __ffs(static_cast<int>(hit)) - 1, e = lane & 7, h = e >> 2;
       run = __shfl_sync(kFull, run, ch - b0);
@@ -722,11 +727,11 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
       uint64_t upto = v;
 #pragma unroll
       for (int o = 1; o < 8; o <<= 1) { const uint64_t t = __shfl_up_sync(kFull, upto, o); if (e >= o) upto += t; }
-      const uint32_t at = __ballot_sync(kFull, run + upto - v <= target && target < run + upto) & 0xFFu;
+      const uint32_t at = __ballot_sync(kFull, run + upto - v <= left && left < run + upto) & 0xFFu;
       if (at) token = 8 * ch + __ffs(static_cast<int>(at)) - 1 - off;
       break;
     }
-    before += __shfl_sync(kFull, incl, 31);
+    left -= __shfl_sync(kFull, incl, 31);
   }
   deliver(token);
 }

@@ -93,3 +93,39 @@ def test_residuals_below_the_fixed_point_have_their_keys(vocab, n, dtype):
         for kept in (None, np.full(n + 1, -1.0, np.float32)):
             check(target, d, x, ua, np.float32(0.3), tau=kept)
     assert fin == vocab - 1
+
+
+# (a flat row of 700,001: sums of residuals pass 2^64, so that the draw's point lies in two slices or in none)
+@pytest.mark.parametrize("residual_draw", ["inverse_cdf", "gumbel"])
+@pytest.mark.parametrize("vocab,flat", [(50257, False), (700001, True)])
+def test_masses_of_no_row_end_in_outputs(vocab, flat, residual_draw):
+    """Masses that are not the rows' give unspecified tokens, but outputs are written, the round is closed once and the launches behind it are right."""
+    n = 3
+    layout = lm.StepStateLayout(n + 1, n)
+    rng, target, _, q = step(vocab, n, "bf16", 23)
+    if flat:
+        target = np.zeros_like(target)
+    z = oracle.bf16_to_f32(target)
+    x, gq = on_gpu(target), torch.from_numpy(q).cuda()
+    vmax = torch.from_numpy(z.max(-1)).cuda()
+    right = torch.tensor([oracle.kept_mass(z[r], -np.inf, 1.0) for r in range(n + 1)], dtype=torch.int64, device="cuda")
+    drafts = torch.full((n,), -1, dtype=torch.int32, device="cuda")          # no id of the vocabulary: rejected whatever the masses
+    for mass in (1, 3, 1 << 12, 1 << 24, 1 << 36, -1):
+        for uf in (0.0, 0.01, 0.3, 0.9, LAST):
+            wrong = torch.full((n + 1,), mass, dtype=torch.int64, device="cuda")
+            kw = dict(uniforms=torch.full((n,), 0.5).cuda(), u_resample=torch.tensor([uf], dtype=torch.float32), residual_draw=residual_draw, seed=4)
+            out = torch.full((n + 3,), -7, dtype=torch.int32, device="cuda")
+            lm.verify(x, drafts, gq, mode="stochastic", out=out, target_vmax=vmax, target_mass=wrong, **kw)
+            assert int(out[0]) == 0 and -1 <= int(out[1]) < vocab, (mass, uf)
+            st = layout.to_device(dict(step=2, verify_len=n, t_this_step=n + 1, pending_tokens=[5, -1, -1, -1]))
+            ring = torch.zeros(8, dtype=torch.int64, device="cuda")
+            close = lambda **more: lm.verify(x, None, gq, mode="stochastic", out=out, target_vmax=vmax, step_state=(layout, st),   # noqa: E731
+                                             commit=dict(layout=layout, state=st, ring=ring), **kw, **more)
+            close(target_mass=wrong)
+            assert layout.from_device(st)["step"] == 3, (mass, uf)
+            out.fill_(-7)
+            close(target_mass=right)                                         # no drafts: the row's own draw
+            after = layout.from_device(st)
+            assert after["step"] == 4 and after["anchor"] == int(out[1]) and int(out[0]) == 0
+            if residual_draw == "inverse_cdf":
+                assert int(out[1]) == oracle.sample_invcdf_index_order(z[0], uf)
