@@ -193,6 +193,7 @@ struct FloorSum {
     top += t.x + t.y; low += l.x + l.y; n += 2u;
     return w;
   }
+  __device__ __forceinline__ bool beyond() const { return top - n * 0x4B000000u > 8388608u; }   // more than 2^40 in all, or an x above 2^40 (2^64 at most) among them: no sum
   __device__ __forceinline__ uint64_t sum() const { return (static_cast<uint64_t>(top - n * 0x4B000000u) << 17) + (low - n * 0x4B000000u); }
 };
 // floor(floor(u * 2^24) * total / 2^24), u clamped to [0, 1 - 2^-24]

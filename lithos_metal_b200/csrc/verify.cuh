@@ -162,7 +162,7 @@ static __device__ __noinline__ uint4 verify_far(const char* row, int off, int V,
 
 // What a row's chunks are weighed with; kept in shared memory for verify_half.
 struct VerifyRow {
-  const char* q_row; uint4* qs; int off, V, per; bool q_cached, q_vec, cut; float c2, tau, qv; ProbScale p_of, q_of;
+  const char *z_row, *q_row; uint4* qs; int off, V, per; bool q_cached, q_vec, cut; float c2, tau, qv; ProbScale p_of, q_of;
 };
 struct VerifySmem {
   unsigned long long x_best[kCMaxRanks], x_own[kCMaxRanks], x_res[kCMaxRanks];   // what the blocks of the cluster leave in one another's copy
@@ -180,6 +180,22 @@ __device__ __forceinline__ void verify_pairs(uint4 v, int h, float2 (&z)[2]) {
   }
 #pragma unroll
   for (int k = 0; k < 2; k++) z[k] = __fadd2_rn(z[k], make_float2(0.0f, 0.0f));
+}
+
+// The residual of half a chunk by the definition, from global memory: where the drafter's values are below 0, p - q may exceed 1, and a kept logit of weight 0 has one.
+template <bool F32>
+static __device__ __noinline__ float4 verify_below_zero(const VerifyRow& x, int c, int h, float vmax) {
+  const float* q = reinterpret_cast<const float*>(x.q_row);
+  float r[4];
+#pragma unroll
+  for (int e = 0; e < 4; e++) {
+    const int i = 8 * c + 4 * h + e - x.off;
+    r[e] = 0.0f;
+    if (i < 0 || i >= x.V) continue;
+    const float z = canon_zero(F32 ? __ldg(reinterpret_cast<const float*>(x.z_row) + i) : bf16_lo(__ldg(reinterpret_cast<const uint16_t*>(x.z_row) + i)));
+    if (z >= x.tau) r[e] = fmaxf(__fsub_rn(prob_q40(weight_q40(z, vmax, x.c2), x.p_of.k), __ldg(q + i)), 0.0f) * 1099511627776.0f;
+  }
+  return make_float4(r[0], r[1], r[2], r[3]);
 }
 
 // What half a chunk weighs in the draw, before the floors: the kept set's weights (what lies outside the row is -inf: 0), or with `residual` what max(p - q, 0)
@@ -200,12 +216,15 @@ static __device__ __noinline__ float4 verify_half(const VerifyRow& x, uint4 v, i
       w[k] = make_float2(z[k].x >= tau ? y.x : 0.0f, z[k].y >= tau ? y.y : 0.0f);
     }
   }
-  if (Q == 0 || !residual || !(__float_as_uint(w[0].x) | __float_as_uint(w[0].y) | __float_as_uint(w[1].x) | __float_as_uint(w[1].y))) return make_float4(w[0].x, w[0].y, w[1].x, w[1].y);
+  if (Q == 0 || !residual || (Q != 1 && !(__float_as_uint(w[0].x) | __float_as_uint(w[0].y) | __float_as_uint(w[1].x) | __float_as_uint(w[1].y))))
+    return make_float4(w[0].x, w[0].y, w[1].x, w[1].y);
   uint2 t, l;
   float2 q[2];
   const uint4 qr = x.q_cached ? x.qs[(Q == 1 && h ? x.per : 0) + c] : verify_far<Q == 1>(x.q_row, x.off, x.V, c, h, x.q_vec, Q == 1 ? 0u : 0xFF80u);
-  if (Q == 1) { q[0] = make_float2(__uint_as_float(qr.x), __uint_as_float(qr.y)); q[1] = make_float2(__uint_as_float(qr.z), __uint_as_float(qr.w)); }
-  else {
+  if (Q == 1) {
+    q[0] = make_float2(__uint_as_float(qr.x), __uint_as_float(qr.y)); q[1] = make_float2(__uint_as_float(qr.z), __uint_as_float(qr.w));
+    if (fminf(fminf(q[0].x, q[0].y), fminf(q[1].x, q[1].y)) < 0.0f) return verify_below_zero<F32>(x, c, h, vmax);
+  } else {
     verify_pairs<false>(qr, h, q);
     const ProbScale q_of = x.q_of;
 #pragma unroll
@@ -219,6 +238,11 @@ static __device__ __noinline__ float4 verify_half(const VerifyRow& x, uint4 v, i
     w[k] = __fmul2_rn(make_float2(w[k].x > 0.0f ? fmaxf(d.x, 0.0f) : 0.0f, w[k].y > 0.0f ? fmaxf(d.y, 0.0f) : 0.0f), make_float2(1099511627776.0f, 1099511627776.0f));
   }
   return make_float4(w[0].x, w[0].y, w[1].x, w[1].y);
+}
+
+// The floors' sum of residuals some of which may be above 2^40.
+static __device__ __noinline__ uint64_t verify_wide(float4 a, float4 b) {
+  return __float2ull_rz(a.x) + __float2ull_rz(a.y) + __float2ull_rz(a.z) + __float2ull_rz(a.w) + __float2ull_rz(b.x) + __float2ull_rz(b.y) + __float2ull_rz(b.z) + __float2ull_rz(b.w);
 }
 
 // The same of one element of the row (its index i, its logit z >= the threshold), as an integer: where few are kept, a lane takes one of them at a time.
@@ -283,7 +307,7 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
   const bool q_vec = ((reinterpret_cast<uintptr_t>(q_row) - static_cast<uintptr_t>(off) * (Q == 1 ? 4 : 2)) & 15u) == 0u;
   if (tid == 0) {
     VerifyRow& x = s.row;
-    x.q_row = q_row; x.qs = qs; x.off = off; x.V = V; x.per = per; x.q_cached = q_cached; x.q_vec = q_vec;
+    x.z_row = z_row; x.q_row = q_row; x.qs = qs; x.off = off; x.V = V; x.per = per; x.q_cached = q_cached; x.q_vec = q_vec;
     x.cut = P.tau != nullptr; x.tau = P.tau ? P.tau[row] : -INFINITY; x.c2 = Q != 0 ? exp2_scale(P.temperature) : 0.0f;
     if (given_mass) x.p_of.init(P.row_mass[row]);
   }
@@ -481,6 +505,17 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
   };
   bool residual = false, weighed = !given_mass && keep_w;                   // weighed: the floors of the weights lie in shared memory
   auto half_weight = [&](int c, int h, bool stored) { return verify_half<F32, Q>(s.row, stored ? zs[(h ? per : 0) + c] : z_raw(c, h), c, h, stored, residual, vmax); };
+  auto chunk_weight = [&](int c, bool stored) {
+    uint64_t v = 0ull;
+#pragma unroll 1
+    for (int h = 0; h < 2; h++) {
+      const float4 x = half_weight(c, h, stored);
+      FloorSum sum;
+      sum.add(make_float2(x.x, x.y)); sum.add(make_float2(x.z, x.w));
+      v += sum.beyond() ? verify_wide(x, make_float4(0.0f, 0.0f, 0.0f, 0.0f)) : sum.sum();
+    }
+    return v;
+  };
   const bool direct = given_mass && !(P.state && P.commit);                 // (a commit changes the state that blocks of other rows may not have read yet)
   unsigned long long mass = 0ull;
   VerifySums shares;                                                        // the blocks' shares of what is drawn from
@@ -503,16 +538,12 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
     uint64_t own = 0ull;
 #pragma unroll 1
     for (int c = w0 + lane; c < w1; c += 32) {
-      FloorSum sum;
       if (z_cached) {
+        FloorSum sum;
         float2 w[4];
         weigh(c, sum, w);
-        sums[c] = sum.sum();
-      } else {
-#pragma unroll 1
-        for (int h = 0; h < 2; h++) { const float4 x = half_weight(c, h, false); sum.add(make_float2(x.x, x.y)); sum.add(make_float2(x.z, x.w)); }
-      }
-      own += sum.sum();
+        own += sums[c] = sum.sum();
+      } else own += chunk_weight(c, false);
     }
     float t_q = 0.0f;
     if (Q == 2 && tests && drafter) { keep_drafter(); t_q = t_prob(t_max, t_mass); }   // (the drafter's side, before the mass is known)
@@ -620,9 +651,10 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
             if (has_q) {
               sum = FloorSum();
               uint32_t any = 0u;
+              bool below = false;
 #pragma unroll
               for (int k = 0; k < 4; k++) any |= __float_as_uint(x[k].x) | __float_as_uint(x[k].y);
-              if (any) {
+              if (any || Q == 1) {
                 float2 q[4];
                 uint4 a, b;
                 if (q_cached) { a = qs[c]; if (Q == 1) b = qs[per + c]; }
@@ -630,6 +662,7 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
                 if (Q == 1) {
                   q[0] = make_float2(__uint_as_float(a.x), __uint_as_float(a.y)); q[1] = make_float2(__uint_as_float(a.z), __uint_as_float(a.w));
                   q[2] = make_float2(__uint_as_float(b.x), __uint_as_float(b.y)); q[3] = make_float2(__uint_as_float(b.z), __uint_as_float(b.w));
+                  below = fminf(fminf(fminf(q[0].x, q[0].y), fminf(q[1].x, q[1].y)), fminf(fminf(q[2].x, q[2].y), fminf(q[3].x, q[3].y))) < 0.0f;
                 } else {
                   const ProbScale q_of = s.row.q_of;
                   const float qv = s.row.qv;
@@ -642,6 +675,11 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
                   }
                 }
                 const ProbScale p_of = s.row.p_of;
+                if (below) {
+                  const float4 l = verify_below_zero<F32>(s.row, c, 0, vmax), u = verify_below_zero<F32>(s.row, c, 1, vmax);
+                  x[0] = make_float2(l.x, l.y); x[1] = make_float2(l.z, l.w); x[2] = make_float2(u.x, u.y); x[3] = make_float2(u.z, u.w);
+                  v += verify_wide(l, u);
+                } else if (any)
 #pragma unroll
                 for (int k = 0; k < 4; k++) {
                   const float2 d = __fadd2_rn(p_of.of(x[k]), make_float2(-q[k].x, -q[k].y));
@@ -655,10 +693,7 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
               to[c] = make_uint4(__float_as_uint(x[0].x), __float_as_uint(x[0].y), __float_as_uint(x[1].x), __float_as_uint(x[1].y));
               to[per + c] = make_uint4(__float_as_uint(x[2].x), __float_as_uint(x[2].y), __float_as_uint(x[3].x), __float_as_uint(x[3].y));
             }
-          } else {
-#pragma unroll 1
-            for (int h = 0; h < 2; h++) { const float4 x = half_weight(c, h, weighed); sum.add(make_float2(x.x, x.y)); sum.add(make_float2(x.z, x.w)); }
-          }
+          } else v += chunk_weight(c, weighed);
           v += sum.sum();
           if (z_cached) sums[c] = v;
           w += v;
@@ -702,12 +737,7 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
     uint64_t sum = 0ull;
     if (c < w1) {
       if (z_cached) sum = sums[c];
-      else {
-        FloorSum f;
-#pragma unroll 1
-        for (int h = 0; h < 2; h++) { const float4 x = half_weight(c, h, false); f.add(make_float2(x.x, x.y)); f.add(make_float2(x.z, x.w)); }
-        sum = f.sum();
-      }
+      else sum = chunk_weight(c, false);
     }
     uint64_t incl = sum;
 #pragma unroll

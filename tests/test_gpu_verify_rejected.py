@@ -129,3 +129,25 @@ def test_masses_of_no_row_end_in_outputs(vocab, flat, residual_draw):
             assert after["step"] == 4 and after["anchor"] == int(out[1]) and int(out[0]) == 0
             if residual_draw == "inverse_cdf":
                 assert int(out[1]) == oracle.sample_invcdf_index_order(z[0], uf)
+
+
+@pytest.mark.parametrize("vocab,n", [(50257, 7), (262144, 7), (700001, 2)])
+@pytest.mark.parametrize("dtype", ["bf16", "fp32"])
+def test_draft_values_below_zero(vocab, n, dtype):
+    """What a drafter gives need not be a distribution: where q < 0 the residual may exceed 1, and the draw is still the definition's."""
+    rng, target, _, q = step(vocab, n, dtype, 7)
+    z = oracle.bf16_to_f32(target) if dtype == "bf16" else target
+    sharp = np.full_like(z, -40.0)                                           # p = 1 at one token
+    sharp[:, 1234] = 3.0
+    for t, zt in ((target, z), (oracle.f32_to_bf16(sharp) if dtype == "bf16" else sharp, sharp)):
+        d, ua = rejecting(zt, q, n // 2)
+        tau = np.partition(zt, vocab - 300, axis=-1)[:, vocab - 300].astype(np.float32)
+        for least in (-1e-7, -0.3, -3.0, -1000.0):
+            x = q.copy()
+            x[:, rng.integers(0, vocab, 40)] = np.float32(least) * rng.random(40).astype(np.float32)
+            x[:, 1234], x[:, 4321] = np.float32(least), np.float32(least)
+            x[np.arange(n), d] = q[np.arange(n), d]
+            assert oracle.verify_stochastic(t, d, x, ua, 0.5)[0] == n // 2
+            for uf in (0.0, rng.random(), rng.random(), LAST):
+                check(t, d, x, ua, np.float32(uf))
+            check(t, d, x, ua, np.float32(rng.random()), tau=tau)
