@@ -532,6 +532,7 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
     mass = P.row_mass[row];
     if (r != j) {
       if (!direct && rank == 0 && warp == 0) verify_arrive(P, rd, r, launch, false, -1);   // (beyond j it does not matter)
+      cp_async_wait<0>();                                                   // (nothing of a block is in flight when it leaves its shared memory to another)
       return;
     }
   } else {
@@ -562,6 +563,7 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
       __syncthreads();
       if (!s.reject) {
         if (rank == 0 && warp == 0) verify_arrive(P, rd, r, launch, false, -1);
+        cp_async_wait<0>();
         return;
       }
     }
