@@ -269,9 +269,12 @@ int lm_sample(const lm_sample_args* a) {
       // Every launch of the call waits on the device for what it needs of the one in front, so that none of them begins with a gap (us per call so /
       // one after the other: 256 penalised rows 82 / 132, 4096 635 / 703; a memset and gaps in place of the preparation alone were 10 and 6 of it).
       // Where the length of a launch is that of its longest rows, the top-k kernel takes those with a large top_k first: the last ones, which begin when others are done, are
-      // short then (256 penalised rows, 40 seeds: median 66.4 -> 60.0 us; 160 72.4 -> 62.1; 256 of 50,264 without penalties 47.6 -> 41; a claim costs a trip to the list: 200 rows 73.7 -> 74.0).
+      // short then. Not where all its rows have a block at once: with a quarter of the rows the histogram kernel's, an SM each, and two blocks to each other SM that is up to
+      // 1.6 rows per SM, and a claim costs a trip to the list for nothing. us as they come / ordered, means of 20 inputs with knobs of the benchmark's mix: of 50,264 logits 148 rows
+      // 36.7 / 38.4, 224 39.0 / 40.4, 256 47.9 / 43.0, 500 65.2 / 56.9, 740 81.4 / 78.2; of 151,936 with 2048 tokens of history 160 60.1 / 60.5, 224 64.9 / 65.7, 256 66.7 / 61.8, 288 81.0 / 75.7,
+      // 350 86.3 / 86.2, 600 131 / 127; of 262,144 148 65.9 / 70.7, 200 79.2 / 81.8, 256 93.8 / 92.8, 288 101.9 / 97.5, 500 156 / 163 (of all these the one to lose).
       const bool side = !(one_k || a->rows > static_cast<int64_t>(kOverlapRowsPerSM) * sms);
-      int* order = side && a->top_k != nullptr && a->rows > grid1 / 2 ? reinterpret_cast<int*>(a->workspace) : nullptr;
+      int* order = side && a->top_k != nullptr && a->rows * 5 > 8LL * sms ? reinterpret_cast<int*>(a->workspace) : nullptr;
       rc = launch_stream(beside, sample_prep_kernel, 1, kPrepThreads, 0, 1, st, P, list_other, counters, order);
       if (rc != LM_OK) return rc;
       if (!side) {

@@ -5,9 +5,9 @@ import re
 import torch
 
 
-def kernels(call, stream=None):
+def kernels(call, stream=None, full=False):
     """``call()`` captured: the launched kernels in order as (name, grid size, launched beside its predecessor) and the number of other nodes.
-    "Beside": the only edge into the node is a programmatic one (programmatic stream serialization)."""
+    "Beside": the only edge into the node is a programmatic one (programmatic stream serialization). full: mangled names, which tell a template's instances apart."""
     from cuda.bindings import driver as cu
 
     def ok(r):
@@ -45,7 +45,7 @@ def kernels(call, stream=None):
         short = re.search(r"\d+([a-z_]+_kernel)", name)
         edges = into.get(int(node), [])
         beside = bool(edges) and all(kind == 1 for kind in edges)
-        found.append((short.group(1) if short else name, p.gridDimX * p.gridDimY * p.gridDimZ, beside))
+        found.append((short.group(1) if short and not full else name, p.gridDimX * p.gridDimY * p.gridDimZ, beside))
     return found, others
 
 

@@ -26,3 +26,14 @@ def test_every_row_is_taken_once(rows, pattern):
     assert "sample_topk_kernel" in routes.names(call)
     assert torch.equal(r.tokens, exact.tokens) and torch.equal(r.tau, exact.tau)
     assert int(((r.status & 64) != 0).sum()) >= 0.9 * int((k > 0).sum())     # (by the candidate kernel, but for the rows that it hands on)
+
+
+@pytest.mark.parametrize("rows,ordered", [(75, False), (148, False), (1, True), (0, False)])
+def test_rows_are_ordered_where_some_wait_for_a_block(rows, ordered):
+    """Up to 1.6 rows per SM every row of the candidate kernel has a block at once, and the kernel that looks the order up is not launched."""
+    line = 8 * torch.cuda.get_device_properties(0).multi_processor_count // 5
+    rows = rows if rows > 1 else line + rows
+    x = torch.randn(rows, 40960, device="cuda").to(torch.bfloat16)
+    k = torch.tensor([0, 20, 50, 1000] * rows, dtype=torch.int32, device="cuda")[:rows]
+    found = [name for name, _, _ in routes.kernels(lambda: lm.sample(x, lm.SamplingParams(temperature=0.8, top_k=k, top_p=0.9)), full=True)[0] if "sample_topk_kernel" in name]
+    assert found and all(("Lb1" in name) == ordered for name in found), found
