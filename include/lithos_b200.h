@@ -238,10 +238,9 @@ typedef struct lm_verify_args {
    * prefill branch). A state whose rows do not fit (verify_len > n_draft, t_this_step > n_draft + 1) gets error 4 and done = 1. */
   const void* step_state;
   int32_t t_max, gamma_max;
-  uint32_t wait_limit;         /* polls of a row's result before the last of the launch's clusters gives up; 0 = the default (about 0.1 s) */
-  uint32_t selftest;           /* LM_VERIFY_SELFTEST_WITHHOLD: the first row's cluster does not say what it found, so that wait runs
-                                  out and the error path can be exercised (with a small wait_limit) without hanging anything (a launch that
-                                  is given target_vmax and target_mass has no such wait) */
+  uint32_t wait_limit;         /* polls of a block's result before the last of the launch's blocks gives up; 0 = the default (about 0.1 s) */
+  uint32_t selftest;           /* LM_VERIFY_SELFTEST_WITHHOLD: the first of them does not say what it found, so that wait runs
+                                  out and the error path can be exercised (with a small wait_limit) without hanging anything */
   const float* target_vmax;    /* stochastic mode, optional: [n_draft + 1] (with a step_state: [t_max], indexed like the rows) the exact
                                   maximum of every target row, as the sampler that produced `tau` knows it (the reference's verify
                                   kernels take it from there too: KEPT_STATS, kernels/common/sample.metal:273-303). The launch then
@@ -249,8 +248,9 @@ typedef struct lm_verify_args {
                                   gives unspecified tokens (never a hang). NULL: the kernel finds the maxima itself. */
   const uint64_t* target_mass; /* with target_vmax, optional: per row the fixed-point mass of its kept set {z >= tau} at `temperature`, as
                                   lm_sample_args.out_mass gives it for the same rows, thresholds and temperature (the other half of
-                                  the reference's KEPT_STATS). Every block then runs the accept test by itself, and only the
-                                  blocks of the decisive row meet again (the draw). Ignored without target_vmax. */
+                                  the reference's KEPT_STATS). Every block then runs the accept tests by itself, and all blocks
+                                  share the decisive row (the draw). Masses that are not the rows' give unspecified tokens, never a hang.
+                                  Ignored without target_vmax. */
 } lm_verify_args;
 
 #define LM_RESIDUAL_INVERSE_CDF 0 /* final token by inverse CDF, in ascending index order, over max(p - q, 0) (over p on the bonus row) from u_final */

@@ -5,7 +5,7 @@
 #include "draft_q.cuh"
 #include "host.cuh"
 #include "sample_cluster.cuh"
-#include "verify.cuh"
+#include "verify_given.cuh"
 
 namespace lm {
 
@@ -137,42 +137,47 @@ int draft_q_clusters(const DraftQDev& P, int sms, cudaStream_t st) {
   return P.dtype == LM_DTYPE_F32 ? launch_draft_q<true>(P, C, sms, st) : launch_draft_q<false>(P, C, sms, st);
 }
 
-// The verification: a cluster per target row, as many blocks each as let all of them run at once.
+// The verification given the rows' maxima and masses: the decisive row over all the blocks that it is worth, an SM each (as the draft draw's: the two follow one
+// another in a speculative round). A thread per half chunk is 256 chunks to a block; down to 64 more blocks are faster, up to some 120, beyond which their arrivals
+// cost more (us, first of 7 drafts rejected, 48 / 80 / 120 / 148 blocks: 151,936 tokens 8.84 / 8.62 / 8.31 / 9.14, 100,000 8.63 / 8.23 / 8.22 / -, 50,257 8.75 / 8.22 / 8.08 / 8.45).
 template <bool F32, int Q>
-static int launch_verify(const VerifyDev& P, int sms, cudaStream_t st) {
-  const KernelSlot slot = static_cast<KernelSlot>(kSlotVerify + (F32 ? 3 : 0) + Q), slot_alone = static_cast<KernelSlot>(kSlotVerify + 6 + (F32 ? 3 : 0) + Q);
-  const void* fn = reinterpret_cast<const void*>(verify_kernel<F32, Q>);
-  static_assert(kVerifySmem < kAloneSmem, "one grant for both");
-  const int rc = ensure_dynamic_smem(slot, fn, kAloneSmem, true);
+static int launch_verify_given(const VerifyDev& P, int sms, cudaStream_t st) {
+  const KernelSlot slot = static_cast<KernelSlot>(kSlotVerifyGiven + (F32 ? 2 : 0) + Q - 1);
+  const int rc = ensure_dynamic_smem(slot, reinterpret_cast<const void*>(verify_given_kernel<F32, Q>), kAloneSmem);
   if (rc != LM_OK) return rc;
-  const int rows = P.n_draft + 1;
-  const bool given = P.row_max != nullptr && P.row_mass != nullptr, lean = given && P.draw != LM_DRAW_GUMBEL, few = lean && P.tau != nullptr;
-  auto chunks = [&](int c) { return (static_cast<size_t>((P.vocab + 14) / 8) + c - 1) / c; };   // of a slice, for any alignment of the row
-  auto z_bytes = [&](int c) { return chunks(c) * (lean && !F32 ? 16 : 32) + (chunks(c) + 1) / 2 * 16; };   // (logits, then weights; the chunks' sums)
-  // Where few logits are weighed, a block has its SM to itself (as the draft draw's: the two follow one another in a speculative round), eight to a row where
-  // sixteen would not all run at once (the round of 7 drafts 38.7 us either way). Where the masses are given all but the decisive row's blocks leave early, and
-  // a row gets all the blocks that a cluster can have.
-  int most = cluster_blocks(given ? 1 : rows, P.vocab, 2 * sms);
-  bool alone = false;
-  if (few) {
-    const int c = cluster_that_fits(most, [&](int n) { return clusters_at_once(slot_alone, fn, kVerifyThreads, kAloneSmem, n) >= rows; });
-    alone = c * 2 >= most && z_bytes(c) <= kVerifySmem;
-    if (alone) most = c;
-  }
-  const int at_once = given ? 1 : rows;
-  const int C = cluster_that_fits(most, [&](int c) { return clusters_at_once(slot, fn, kVerifyThreads, kVerifySmem, c) >= at_once; });
-  const size_t z = z_bytes(C), q = Q == 0 || few ? 0 : chunks(C) * 32;       // (the drafter's row, then the residual's weights)
-  const bool z_cached = z <= kVerifySmem, q_cached = q != 0 && (z_cached ? z : 0) + q <= kVerifySmem;
-  const size_t smem = alone ? kAloneSmem : (z_cached ? z : 0) + (q_cached ? q : 0);
-  const unsigned grid = static_cast<unsigned>(rows) * static_cast<unsigned>(C);
-  return launch_stream(given || static_cast<int>(grid) <= sms, verify_kernel<F32, Q>, dim3(grid), kVerifyThreads, smem, C, st, P, C, z_cached ? 1 : 0, q_cached ? 1 : 0);
+  const int chunks = P.vocab / 8 + 1, least = (chunks + 255) / 256, most = sms < kVerifyParts ? sms : kVerifyParts;
+  int grid = (chunks + 63) / 64;
+  if (grid > 120) grid = least > 120 ? least : 120;
+  if (grid > most) grid = most;
+  return launch_stream(true, verify_given_kernel<F32, Q>, dim3(static_cast<unsigned>(grid)), kVerifyThreads, kAloneSmem, 1, st, P);
 }
 
-int verify_clusters(const VerifyDev& P, int sms, cudaStream_t st) {
-  const bool f32 = P.dtype == LM_DTYPE_F32;
-  if (P.mode != LM_VERIFY_STOCHASTIC) return f32 ? launch_verify<true, 0>(P, sms, st) : launch_verify<false, 0>(P, sms, st);
-  if (P.q) return f32 ? launch_verify<true, 1>(P, sms, st) : launch_verify<false, 1>(P, sms, st);
-  return f32 ? launch_verify<true, 2>(P, sms, st) : launch_verify<false, 2>(P, sms, st);
+// ... and not given: a cluster per target row, as many blocks each as let all of them run at once.
+template <bool F32, int Q>
+static int launch_verify(const VerifyDev& P, int sms, cudaStream_t st) {
+  const KernelSlot slot = static_cast<KernelSlot>(kSlotVerify + (F32 ? 3 : 0) + Q);
+  const void* fn = reinterpret_cast<const void*>(verify_kernel<F32, Q>);
+  const int rc = ensure_dynamic_smem(slot, fn, kVerifySmem, true);
+  if (rc != LM_OK) return rc;
+  const int rows = P.n_draft + 1;
+  const int C = cluster_that_fits(cluster_blocks(rows, P.vocab, 2 * sms), [&](int c) { return clusters_at_once(slot, fn, kVerifyThreads, kVerifySmem, c) >= rows; });
+  const size_t chunks = (static_cast<size_t>((P.vocab + 14) / 8) + C - 1) / C;   // of a slice, for any alignment of the row
+  const size_t z = chunks * 32 + (chunks + 1) / 2 * 16, q = Q == 0 ? 0 : chunks * 32;   // (logits, then weights; the chunks' sums; the drafter's row, then the residual's weights)
+  const bool z_cached = z <= kVerifySmem, q_cached = q != 0 && (z_cached ? z : 0) + q <= kVerifySmem;
+  const size_t smem = (z_cached ? z : 0) + (q_cached ? q : 0);
+  const unsigned grid = static_cast<unsigned>(rows) * static_cast<unsigned>(C);
+  return launch_stream(static_cast<int>(grid) <= sms, verify_kernel<F32, Q>, dim3(grid), kVerifyThreads, smem, C, st, P, C, z_cached ? 1 : 0, q_cached ? 1 : 0);
+}
+
+template <bool F32>
+static int launch_verify_rows(const VerifyDev& P, int sms, cudaStream_t st) {
+  if (P.mode != LM_VERIFY_STOCHASTIC) return launch_verify<F32, 0>(P, sms, st);
+  if (P.row_max && P.row_mass) return P.q ? launch_verify_given<F32, 1>(P, sms, st) : launch_verify_given<F32, 2>(P, sms, st);
+  return P.q ? launch_verify<F32, 1>(P, sms, st) : launch_verify<F32, 2>(P, sms, st);
+}
+
+int verify_rows(const VerifyDev& P, int sms, cudaStream_t st) {
+  return P.dtype == LM_DTYPE_F32 ? launch_verify_rows<true>(P, sms, st) : launch_verify_rows<false>(P, sms, st);
 }
 
 }  // namespace lm

@@ -36,8 +36,9 @@ inline int sm_count(int* out) {
 enum KernelSlot { kSlotFast, kSlotTopk, kSlotTopkOrdered, kSlotGeneric, kSlotVocabLocal, kSlotTileFinish, kSlotSlice, kSlotSliceSmall, kSlotSliceTiny, kSlotSlicedMerge, kSlotHead, kSlotCluster,
                   kSlotArgmax = kSlotCluster + 6,   // (the cluster kernel has six instances, the argmax kernel two)
                   kSlotDraftQ = kSlotArgmax + 2,    // (two instances)
-                  kSlotVerify = kSlotDraftQ + 2,    // (six, and six for blocks that have an SM to themselves)
-                  kSlotCount = kSlotVerify + 12 };
+                  kSlotVerify = kSlotDraftQ + 2,    // (six)
+                  kSlotVerifyGiven = kSlotVerify + 6,   // (four)
+                  kSlotCount = kSlotVerifyGiven + 4 };
 
 inline int ensure_dynamic_smem(KernelSlot slot, const void* func, size_t bytes, bool large_clusters = false) {
   constexpr int kMaxDevices = 64;
@@ -131,6 +132,6 @@ struct VerifyDev;
 int sample_clusters(const SampleDev& P, int sms, cudaStream_t st, bool few = false);   // few: a call of a few rows with one top_k (LM_STATUS_SLICED_PATH)
 int argmax_clusters(const void* logits, int dtype, int rows, int vocab, int64_t row_stride, int32_t* out32, int64_t* out64, cudaStream_t st);
 int draft_q_clusters(const DraftQDev& P, int sms, cudaStream_t st);
-int verify_clusters(const VerifyDev& P, int sms, cudaStream_t st);
+int verify_rows(const VerifyDev& P, int sms, cudaStream_t st);
 
 }  // namespace lm

@@ -637,7 +637,7 @@ int lm_verify(const lm_verify_args* a) {
                          reinterpret_cast<unsigned long long*>(c->ring), c->ring_cap, EosSet{c->eos, c->eos_list, c->n_eos}, c->log, c->log_cap,
                          c->ctx_cap, c->lm};
   }
-  return verify_clusters(P, sms, static_cast<cudaStream_t>(a->stream));
+  return verify_rows(P, sms, static_cast<cudaStream_t>(a->stream));
 }
 
 int lm_draft_q(const lm_draft_q_args* a) {

@@ -9,13 +9,11 @@
 // copies, all in flight at once; the blocks meet in distributed shared memory, a cluster barrier to a dependency; and every row that could be the
 // decisive one -- its own draft rejected, or the bonus row -- draws its token without waiting for the rows before it. What a row found is one word in
 // the workspace; the cluster that arrives last picks the first rejected row and writes the outputs, so no block waits for another cluster.
-// A launch that is given the rows' maxima and masses knows the decisive row from one logit per draft: every block finds it for itself, the
-// other rows' clusters leave, and the decisive one writes the outputs.
+// A launch that is given the rows' maxima and masses knows the decisive row from one logit per draft: verify_given.cuh.
 // (All rows cut over all 148 SMs by a cooperative launch, partial results exchanged as polled words in L2, three trips for the step of 7 drafts; us a call so /
-// by clusters, first draft rejected: V = 151,936, drafter's probabilities 25.0 / 18.8, given the maxima 21.0 / 17.6, and the masses 14.0 / 12.9, drafter's logits 27.3 / 20.5, given
-// maxima, masses and thresholds 14.3 / 11.3, greedy 10.3 / 7.4; 13 drafts 31.4 / 22.4; 50,257 24.8 / 13.7; 248,320 29.3 / 22.2, but, of the decisive row alone on 16 SMs, given
-// maxima and masses without thresholds 14.4 / 15.8, and the reference's draw with every draft rejected 29.4 / 32.3. A cooperative launch of the clusters is not made
-// ready beside its predecessor: 1.1 us more. One cluster of 1024 threads a block for the decisive row alone, its slices loaded behind the tests: 1 us more.)
+// by clusters, first draft rejected: V = 151,936, drafter's probabilities 25.0 / 18.8, given the maxima 21.0 / 17.6, drafter's logits 27.3 / 20.5, greedy 10.3 / 7.4; 13 drafts 31.4 /
+// 22.4; 50,257 24.8 / 13.7; but the reference's draw over 248,320 with every draft rejected 29.4 / 32.3. A cooperative launch of the clusters is not made ready beside
+// its predecessor: 1.1 us more.)
 //
 // A word carries the launch's number, which the last cluster counts up: were one missing, the wait for it is bounded, and the launch reports an error through
 // its outputs (and through the StepState when it commits); the GPU is never left waiting.
@@ -33,12 +31,14 @@ constexpr int kVerifyThreads = 512;
 constexpr int kVerifyWarps = kVerifyThreads / 32;
 constexpr int kVerifyMaxRows = LM_MAX_DRAFT + 1;
 constexpr unsigned kVerifyWaitLimit = 1u << 17;         // polls of one word before the last cluster gives up: about 0.1 s
+constexpr int kVerifyParts = 256;                       // most blocks that share a row (verify_given.cuh)
 constexpr size_t kVerifySmem = 110 * 1024;              // most shared memory of a block (two to an SM)
 
 struct VerifyWs {                                       // lives in the caller's workspace, zero-filled once
   unsigned long long launches;                          // so far
-  unsigned arrived, pad;                                // rows of this launch that have been through (0 between launches)
+  unsigned arrived, pad;                                // rows (or, of a launch that cuts one row, blocks) of this launch that have been through (0 between launches)
   unsigned long long row[kVerifyMaxRows];               // what a row's cluster found: launch number << 24 | kFound | rejected << 21 | token + 1
+  unsigned long long part[kVerifyParts][4];             // a block's shares (verify_given.cuh), in halves: launch number + 1 << 32 | half
 };
 constexpr unsigned long long kFound = 1ull << 22, kRejected = 1ull << 21;
 static_assert(LM_MAX_VOCAB < (1 << 21), "a token and 'none' fit 21 bits");
@@ -98,7 +98,28 @@ static __device__ __noinline__ void verify_commit(const VerifyDev& P, bool faile
 }
 
 // What a launch verifies: from its arguments, or from the StepState.
-struct VerifyRound { int L, row0; uint64_t seed; uint32_t step; bool idle, mismatch, prefill; };   // idle: the state is done, or this step is a prefill chunk
+struct VerifyRound { int L, row0; uint64_t seed; uint32_t step; };
+// False: nothing is verified, as the state is done, this step is a prefill chunk (block 0 still closes it: the scan's prefill branch), or the state's rows do not fit
+// the launch (block 0 reports the caller's error).
+__device__ __forceinline__ bool verify_begin(const VerifyDev& P, VerifyRound& rd) {
+  rd = VerifyRound{P.n_draft, 0, P.seed, P.step};
+  if (!P.state) return true;
+  StepStateView st{P.state, P.t_max, P.g};
+  rd.seed = st.seed(); rd.step = st.step();
+  const bool first = blockIdx.x == 0 && threadIdx.x < 32;
+  if (st.done()) return false;
+  if (st.prefill_left() > 0u) {
+    if (first) verify_commit(P, false);
+    return false;
+  }
+  const uint32_t len = st.verify_len(), rows = st.t_this_step();
+  if (len > static_cast<uint32_t>(P.n_draft) || rows < len + 1u || rows > static_cast<uint32_t>(P.n_draft) + 1u) {
+    if (first && threadIdx.x == 0) { P.out_accept[0] = -1; P.out_final[0] = -1; fail_state(st, kErrRoundMismatch); }
+    return false;
+  }
+  rd.L = static_cast<int>(len); rd.row0 = static_cast<int>(rows - 1u - len);
+  return true;
+}
 
 __device__ __forceinline__ int verify_draft(const VerifyDev& P, const VerifyRound& rd, int r) {
   return P.state ? StepStateView{P.state, P.t_max, P.g}.pending(rd.row0 + r + 1) : P.drafts[r];
@@ -160,14 +181,14 @@ static __device__ __noinline__ uint4 verify_far(const char* row, int off, int V,
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// What a row's chunks are weighed with; kept in shared memory for verify_half.
+// What a row's chunks are weighed with; kept in shared memory for the functions below.
 struct VerifyRow {
-  const char *z_row, *q_row; uint4* qs; int off, V, per; bool q_cached, q_vec, cut; float c2, tau, qv; ProbScale p_of, q_of;
+  const char *z_row, *q_row; int off, V; bool cut; float c2, tau, qv; ProbScale p_of, q_of;
 };
 struct VerifySmem {
   unsigned long long x_best[kCMaxRanks], x_own[kCMaxRanks], x_res[kCMaxRanks];   // what the blocks of the cluster leave in one another's copy
   uint64_t best[kVerifyWarps], own[kVerifyWarps], res[kVerifyWarps];             // this block's, per warp
-  VerifyRow row; int j; bool reject;
+  VerifyRow row; bool reject;
 };
 
 // The logits of half h of a chunk in pairs (v: the half of a binary32 row, the chunk of a BF16 row), -0 as +0; -inf outside the row.
@@ -198,33 +219,33 @@ static __device__ __noinline__ float4 verify_below_zero(const VerifyRow& x, int 
   return make_float4(r[0], r[1], r[2], r[3]);
 }
 
-// What half a chunk weighs in the draw, before the floors: the kept set's weights (what lies outside the row is -inf: 0), or with `residual` what max(p - q, 0)
-// leaves of them (what is not kept has weight 0, hence p = 0 and nothing left). stored: v holds the floors of the weights already. For what is rare: slices that do
-// not fit shared memory, and the second look where a residual is empty.
-template <bool F32, int Q>
-static __device__ __noinline__ float4 verify_half(const VerifyRow& x, uint4 v, int c, int h, bool stored, bool residual, float vmax) {
-  float2 w[2];
-  if (stored) { w[0] = make_float2(__uint_as_float(v.x), __uint_as_float(v.y)); w[1] = make_float2(__uint_as_float(v.z), __uint_as_float(v.w)); }
-  else {
-    float2 z[2];
-    verify_pairs<F32>(v, h, z);
-    const float tau = x.tau, c2 = x.c2;
-    if (x.cut && !(fmaxf(fmaxf(z[0].x, z[0].y), fmaxf(z[1].x, z[1].y)) >= tau)) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+// What half a chunk weighs, before the floors: the kept set's weights (what lies outside the row is -inf: 0). v: the half as it lies in the row. (By clusters for what
+// is rare: slices that do not fit shared memory, and the second look where a residual is empty.)
+template <bool F32>
+static __device__ __noinline__ float4 verify_weights(const VerifyRow& x, uint4 v, int h, float vmax) {
+  float2 z[2], w[2];
+  verify_pairs<F32>(v, h, z);
+  const float tau = x.tau, c2 = x.c2;
+  if (x.cut && !(fmaxf(fmaxf(z[0].x, z[0].y), fmaxf(z[1].x, z[1].y)) >= tau)) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
-    for (int k = 0; k < 2; k++) {
-      const float2 y = weight_f2(z[k].x, z[k].y, vmax, c2);
-      w[k] = make_float2(z[k].x >= tau ? y.x : 0.0f, z[k].y >= tau ? y.y : 0.0f);
-    }
+  for (int k = 0; k < 2; k++) {
+    const float2 y = weight_f2(z[k].x, z[k].y, vmax, c2);
+    w[k] = make_float2(z[k].x >= tau ? y.x : 0.0f, z[k].y >= tau ? y.y : 0.0f);
   }
-  if (Q == 0 || !residual || (Q != 1 && !(__float_as_uint(w[0].x) | __float_as_uint(w[0].y) | __float_as_uint(w[1].x) | __float_as_uint(w[1].y))))
-    return make_float4(w[0].x, w[0].y, w[1].x, w[1].y);
-  uint2 t, l;
-  float2 q[2];
-  const uint4 qr = x.q_cached ? x.qs[(Q == 1 && h ? x.per : 0) + c] : verify_far<Q == 1>(x.q_row, x.off, x.V, c, h, x.q_vec, Q == 1 ? 0u : 0xFF80u);
+  return make_float4(w[0].x, w[0].y, w[1].x, w[1].y);
+}
+// What max(p - q, 0) leaves of a half's weights f, floors (what is not kept has weight 0, hence p = 0 and nothing left), of 2^40 and before the floors. qr: the half
+// as it lies in the drafter's row.
+template <bool F32, int Q>
+static __device__ __noinline__ float4 verify_rest(const VerifyRow& x, float4 f, uint4 qr, int c, int h, float vmax) {
+  float2 w[2] = {make_float2(f.x, f.y), make_float2(f.z, f.w)}, q[2];
   if (Q == 1) {
     q[0] = make_float2(__uint_as_float(qr.x), __uint_as_float(qr.y)); q[1] = make_float2(__uint_as_float(qr.z), __uint_as_float(qr.w));
     if (fminf(fminf(q[0].x, q[0].y), fminf(q[1].x, q[1].y)) < 0.0f) return verify_below_zero<F32>(x, c, h, vmax);
-  } else {
+  }
+  if (!(__float_as_uint(f.x) | __float_as_uint(f.y) | __float_as_uint(f.z) | __float_as_uint(f.w))) return f;
+  if (Q == 2) {
+    uint2 t, l;
     verify_pairs<false>(qr, h, q);
     const ProbScale q_of = x.q_of;
 #pragma unroll
@@ -233,29 +254,28 @@ static __device__ __noinline__ float4 verify_half(const VerifyRow& x, uint4 v, i
   const ProbScale p_of = x.p_of;
 #pragma unroll
   for (int k = 0; k < 2; k++) {
-    if (!stored) w[k] = floor2(w[k], t, l);
     const float2 d = __fadd2_rn(p_of.of(w[k]), make_float2(-q[k].x, -q[k].y));
     w[k] = __fmul2_rn(make_float2(w[k].x > 0.0f ? fmaxf(d.x, 0.0f) : 0.0f, w[k].y > 0.0f ? fmaxf(d.y, 0.0f) : 0.0f), make_float2(1099511627776.0f, 1099511627776.0f));
   }
   return make_float4(w[0].x, w[0].y, w[1].x, w[1].y);
 }
+// Both, of a half that is weighed in the draw over the residual.
+template <bool F32, int Q>
+static __device__ __forceinline__ float4 verify_far_rest(const VerifyRow& x, uint4 v, bool q_vec, int c, int h, float vmax) {
+  float2 z[2];
+  verify_pairs<F32>(v, h, z);
+  const float tau = x.tau;
+  if (!(fmaxf(fmaxf(z[0].x, z[0].y), fmaxf(z[1].x, z[1].y)) >= tau)) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);   // (nothing kept: the drafter's row is not read)
+  const uint4 qr = verify_far<Q == 1>(x.q_row, x.off, x.V, c, h, q_vec, Q == 1 ? 0u : 0xFF80u);
+  const float4 w = verify_weights<F32>(x, v, h, vmax);
+  uint2 t, l;
+  const float2 a = floor2(make_float2(w.x, w.y), t, l), b = floor2(make_float2(w.z, w.w), t, l);
+  return verify_rest<F32, Q>(x, make_float4(a.x, a.y, b.x, b.y), qr, c, h, vmax);
+}
 
 // The floors' sum of residuals some of which may be above 2^40.
 static __device__ __noinline__ uint64_t verify_wide(float4 a, float4 b) {
   return __float2ull_rz(a.x) + __float2ull_rz(a.y) + __float2ull_rz(a.z) + __float2ull_rz(a.w) + __float2ull_rz(b.x) + __float2ull_rz(b.y) + __float2ull_rz(b.z) + __float2ull_rz(b.w);
-}
-
-// The same of one element of the row (its index i, its logit z >= the threshold), as an integer: where few are kept, a lane takes one of them at a time.
-template <bool F32, int Q>
-static __device__ __noinline__ uint64_t verify_element(const VerifyRow& x, int i, float z, bool residual, float vmax) {
-  const uint32_t qr = !residual ? 0u : Q == 1 ? __ldg(reinterpret_cast<const uint32_t*>(x.q_row) + i) : static_cast<uint32_t>(__ldg(reinterpret_cast<const uint16_t*>(x.q_row) + i)) << 16;
-  const uint64_t w = weight_q40(z, vmax, x.c2);
-  if (!residual) return w;
-  const float p = prob_q40(w, x.p_of.k);
-  float q = __uint_as_float(qr);
-  if (Q == 2) q = x.q_of.k ? prob_q40(weight_q40(canon_zero(q), x.qv, x.c2), x.q_of.k) : 0.0f;
-  const float d = __fsub_rn(p, q);
-  return d > 0.0f ? residual_q40(d) : 0ull;
 }
 
 // Every warp for itself: the slots' running sums, a lane per slot, and their sum.
@@ -277,6 +297,42 @@ __device__ __forceinline__ int verify_slot(const VerifySums& v, uint64_t& left) 
 }
 static_assert(kVerifyWarps <= kCMaxRanks && kCMaxRanks <= 32, "slots of ranks and of warps alike, a lane each");
 
+// The accept test of one draft, by two lanes of one warp: the target's side in lane r (or 0), the drafter's 16 lanes on.
+template <bool F32, int Q>
+struct VerifyTest {
+  float u, tau, vmax; unsigned long long mass; uint32_t bits; bool in;       // (bits as they come: nothing waits for them before the test)
+  // on: this lane has a side of row r's test. given: the target's side with the row's maximum and mass from the caller.
+  __device__ __forceinline__ void load(const VerifyDev& P, const VerifyRound& rd, bool on, bool given, int r) {
+    const bool drafter = (threadIdx.x & 16u) != 0u;
+    constexpr int kSize = F32 ? 4 : 2;
+    u = vmax = 0.0f; tau = -INFINITY; mass = 0ull; bits = 0u; in = false;
+    if (given && !drafter && r <= rd.L) { vmax = P.row_max[rd.row0 + r]; mass = P.row_mass[rd.row0 + r]; if (P.tau) tau = P.tau[rd.row0 + r]; }   // (the bonus row's too)
+    if (!on) return;
+    const int d = verify_draft(P, rd, r);
+    if (!drafter) { if (P.tau && !given) tau = P.tau[rd.row0 + r]; }
+    else {
+      u = P.u_accept ? P.u_accept[r] : uniform01(rd.seed, rd.step, 3000u + static_cast<uint32_t>(r), 0u);
+      if (Q == 2) { vmax = __ldg(P.q_vmax + r); mass = __ldg(P.q_mass + r); }
+    }
+    in = d >= 0 && d < P.vocab;
+    if (!in) return;
+    if (!drafter) {
+      const char* zp = static_cast<const char*>(P.target) + (static_cast<int64_t>(rd.row0 + r) * P.row_stride + d) * kSize;
+      bits = F32 ? __ldg(reinterpret_cast<const uint32_t*>(zp)) : static_cast<uint32_t>(__ldg(reinterpret_cast<const uint16_t*>(zp))) << 16;
+    } else if (Q == 1) bits = __float_as_uint(__ldg(P.q + static_cast<int64_t>(r) * P.q_stride + d));
+    else bits = static_cast<uint32_t>(__ldg(P.q_logits + static_cast<int64_t>(r) * P.q_logits_stride + d)) << 16;
+  }
+  // p and q of the draft, side by side: a lane's probability of its logit (0 for an id outside the vocabulary)
+  __device__ __forceinline__ float prob(float top, unsigned long long m, float c2) const {
+    const float z = canon_zero(__uint_as_float(bits));
+    return in && m > 0ull ? prob_q40(z >= tau ? weight_q40(z, top, c2) : 0ull, m) : 0.0f;
+  }
+  // for the target's lanes: rejected? pq: the lanes' own probabilities
+  __device__ __forceinline__ bool rejects(float pq) const {
+    return __shfl_down_sync(kFull, __fmul_rn(u, Q == 1 ? __uint_as_float(bits) : pq), 16) >= pq;   // (bits of an id outside the vocabulary: 0)
+  }
+};
+
 // One row by one cluster. Q: 0 greedy, 1 the drafter's probabilities, 2 its BF16 logits and their statistics. Every part of this runs a few times a launch, so
 // code that is not in the instruction cache costs as much as what it computes: a loop's chunk is unrolled, loops are not, what has been computed is kept rather
 // than computed by a second copy of the code (the token was found in 2.5 to 3.3 us so, in 1 with the draw's weights kept), and the rare is in functions of its own.
@@ -286,8 +342,8 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int kSize = F32 ? 4 : 2;
   const int V = P.vocab, L = rd.L, row = rd.row0 + r;
-  const bool has_q = Q != 0 && r < L;
-  const bool given_max = Q != 0 && P.row_max != nullptr, given_mass = given_max && P.row_mass != nullptr;
+  const bool has_q = Q != 0 && r < L, gumbel = P.draw == LM_DRAW_GUMBEL;
+  const bool given_max = Q != 0 && P.row_max != nullptr;
   // ---- this block's slice in chunks of eight; a warp's are consecutive, so that what a warp holds is a range of the row ------------------------
   const char* z_row = static_cast<const char*>(P.target) + static_cast<size_t>(row) * static_cast<size_t>(P.row_stride) * kSize;
   const int head = static_cast<int>((16u - (reinterpret_cast<uintptr_t>(z_row) & 15u)) & 15u) / kSize;
@@ -295,21 +351,17 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
   const int c0 = min(n_chunks, rank * per), c1 = min(n_chunks, c0 + per);
   const int cpw = ((per + kVerifyWarps - 1) / kVerifyWarps + 7) & ~7;
   const int w0 = min(c1, c0 + warp * cpw), w1 = min(c1, w0 + cpw);
-  // With the maxima and masses given and a threshold, few logits are kept: they are weighed one by one, and the drafter's row is read where they lie.
-  const bool gumbel = P.draw == LM_DRAW_GUMBEL, lean = given_mass && !gumbel, few = lean && P.tau != nullptr;
   // z_cached: a chunk's logits, later the floors of its weights, in two halves; what the chunk weighs in the draw. q_cached: the drafter's row, later the
   // residual's weights.
-  const int z_slots = lean && !F32 ? per : 2 * per;                         // (lean: the logits stay)
-  unsigned long long* sums = reinterpret_cast<unsigned long long*>(zs + z_slots) - c0;
-  uint4* qs = zs + (z_cached ? z_slots + (per + 1) / 2 : 0) - c0;
+  unsigned long long* sums = reinterpret_cast<unsigned long long*>(zs + 2 * per) - c0;
+  uint4* qs = zs + (z_cached ? 2 * per + (per + 1) / 2 : 0) - c0;
   zs -= c0;
   const char* q_row = !has_q ? nullptr : Q == 1 ? reinterpret_cast<const char*>(P.q + static_cast<int64_t>(r) * P.q_stride) : reinterpret_cast<const char*>(P.q_logits + static_cast<int64_t>(r) * P.q_logits_stride);
   const bool q_vec = ((reinterpret_cast<uintptr_t>(q_row) - static_cast<uintptr_t>(off) * (Q == 1 ? 4 : 2)) & 15u) == 0u;
   if (tid == 0) {
     VerifyRow& x = s.row;
-    x.z_row = z_row; x.q_row = q_row; x.qs = qs; x.off = off; x.V = V; x.per = per; x.q_cached = q_cached; x.q_vec = q_vec;
+    x.z_row = z_row; x.q_row = q_row; x.off = off; x.V = V;
     x.cut = P.tau != nullptr; x.tau = P.tau ? P.tau[row] : -INFINITY; x.c2 = Q != 0 ? exp2_scale(P.temperature) : 0.0f;
-    if (given_mass) x.p_of.init(P.row_mass[row]);
   }
   auto whole = [&](int c) { const int base = 8 * c - off; return base >= 0 && base + 8 <= V; };
   constexpr uint32_t kOut = F32 ? 0xFF800000u : 0xFF80u;
@@ -341,45 +393,13 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
     }
   }
   cp_async_commit();
-  // The scalars of the accept test go out under the copies: of this row, or of all rows where every block runs all tests. They are
-  // the last warp's, which has the fewest chunks: the target's side of row r in lane r (lane 0), the drafter's 16 lanes on.
+  // The scalars of the accept test go out under the copies. They are the last warp's, which has the fewest chunks.
   const float c2 = Q != 0 ? exp2_scale(P.temperature) : 0.0f;
   const bool tester = Q != 0 && warp == kVerifyWarps - 1;
-  const int tr = given_mass ? lane & 15 : r;
-  const bool drafter = lane >= 16, tests = tester && tr < L && (given_mass || (lane & 15) == 0);
   const float u_final = Q != 0 && P.u_final ? P.u_final[0] : 0.0f;           // (wanted at the very end)
-  float t_u = 0.0f, t_tau = -INFINITY, t_max = 0.0f; unsigned long long t_mass = 0ull; bool t_in = false;
-  uint32_t t_bits = 0u;                                                     // (as they come: nothing waits for them before the test)
-  if (tests) {
-    const int d = verify_draft(P, rd, tr);
-    if (!drafter) {
-      if (P.tau) t_tau = P.tau[rd.row0 + tr];
-      if (given_mass) { t_max = P.row_max[rd.row0 + tr]; t_mass = P.row_mass[rd.row0 + tr]; }
-    } else {
-      t_u = P.u_accept ? P.u_accept[tr] : uniform01(rd.seed, rd.step, 3000u + static_cast<uint32_t>(tr), 0u);
-      if (Q == 2) { t_max = __ldg(P.q_vmax + tr); t_mass = __ldg(P.q_mass + tr); }
-    }
-    t_in = d >= 0 && d < V;
-    if (t_in) {
-      if (!drafter) {
-        const char* zp = static_cast<const char*>(P.target) + (static_cast<int64_t>(rd.row0 + tr) * P.row_stride + d) * kSize;
-        t_bits = F32 ? __ldg(reinterpret_cast<const uint32_t*>(zp)) : static_cast<uint32_t>(__ldg(reinterpret_cast<const uint16_t*>(zp))) << 16;
-      } else if (Q == 1) t_bits = __float_as_uint(__ldg(P.q + static_cast<int64_t>(tr) * P.q_stride + d));
-      else t_bits = static_cast<uint32_t>(__ldg(P.q_logits + static_cast<int64_t>(tr) * P.q_logits_stride + d)) << 16;
-    }
-  }
-  // p and q of the draft, side by side: a lane's probability of its logit (0 for an id outside the vocabulary)
-  auto t_prob = [&](float vmax, unsigned long long m) {
-    const float z = canon_zero(__uint_as_float(t_bits));
-    return t_in && m > 0ull ? prob_q40(z >= t_tau ? weight_q40(z, vmax, c2) : 0ull, m) : 0.0f;
-  };
-  auto keep_drafter = [&]() { if (Q == 2 && drafter && tr == r) { s.row.qv = t_max; s.row.q_of.init(t_mass); } };
-  // the target's lanes: rejected? pq: the lanes' own probabilities
-  auto test = [&](float pq, bool write) {
-    const float uq = __shfl_down_sync(kFull, __fmul_rn(t_u, Q == 1 ? __uint_as_float(t_bits) : pq), 16);   // (t_bits of an id outside the vocabulary: 0)
-    if (write && tests && !drafter && P.out_p_draft) P.out_p_draft[tr] = pq;
-    return tests && !drafter && uq >= pq;
-  };
+  const bool tests = tester && has_q && (lane & 15) == 0, drafter = lane >= 16;
+  VerifyTest<F32, Q> t;
+  t.load(P, rd, tests, false, r);
   // half h of a chunk as it lies in memory (BF16: the whole chunk, whichever half)
   auto z_raw = [&](int c, int h) { return z_cached ? zs[(F32 && h ? per : 0) + c] : verify_far<F32>(z_row, off, V, c, h, true, kOut); };
   bool joined = C == 1;                                                     // every block of the cluster runs: its shared memory may be written to
@@ -454,26 +474,8 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
   }
   if (Q == 0) return;
 
-  // ---- the kept set's mass and the accept test; given masses: all tests, and only the decisive row goes on ----------------------------------
-  const bool keep_w = z_cached && !lean && !(gumbel && !has_q);             // the weights replace the logits
-  // the logit of an element, -0 as +0; a bit for each element of a chunk that is kept and not -inf
-  auto z_at = [&](int c, int e) {
-    const uint4 a = z_raw(c, e >> 2);
-    const uint32_t w = F32 ? ((e & 2) ? ((e & 1) ? a.w : a.z) : ((e & 1) ? a.y : a.x)) : ((e & 4) ? ((e & 2) ? a.w : a.z) : ((e & 2) ? a.y : a.x));
-    return canon_zero(F32 ? __uint_as_float(w) : (e & 1) ? bf16_hi(w) : bf16_lo(w));
-  };
-  auto kept_of = [&](int c) {
-    const float tau = s.row.tau;
-    uint32_t m = 0u;
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-      float2 z[2];
-      verify_pairs<F32>(z_raw(c, F32 ? h : 0), h, z);
-#pragma unroll
-      for (int k = 0; k < 2; k++) m |= ((z[k].x >= tau && z[k].x > -INFINITY ? 1u : 0u) | (z[k].y >= tau && z[k].y > -INFINITY ? 2u : 0u)) << (4 * h + 2 * k);
-    }
-    return m;
-  };
+  // ---- the kept set's mass and the accept test ---------------------------------------------------------------------------------------------
+  const bool keep_w = z_cached && !(gumbel && !has_q);                      // the weights replace the logits
   // a chunk's weights, as floors, from its logits in shared memory; nothing kept of it costs its maximum
   auto weigh = [&](int c, FloorSum& sum, float2 (&w)[4]) {
     const float tau = s.row.tau;
@@ -503,8 +505,15 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
       zs[per + c] = make_uint4(__float_as_uint(w[2].x), __float_as_uint(w[2].y), __float_as_uint(w[3].x), __float_as_uint(w[3].y));
     }
   };
-  bool residual = false, weighed = !given_mass && keep_w;                   // weighed: the floors of the weights lie in shared memory
-  auto half_weight = [&](int c, int h, bool stored) { return verify_half<F32, Q>(s.row, stored ? zs[(h ? per : 0) + c] : z_raw(c, h), c, h, stored, residual, vmax); };
+  bool residual = false;
+  auto half_weight = [&](int c, int h, bool stored) {
+    if (!stored) return residual ? verify_far_rest<F32, Q>(s.row, z_raw(c, h), q_vec, c, h, vmax) : verify_weights<F32>(s.row, z_raw(c, h), h, vmax);
+    const uint4 v = zs[(h ? per : 0) + c];
+    const float4 w = make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
+    if (!residual) return w;
+    const uint4 qr = q_cached ? qs[(Q == 1 && h ? per : 0) + c] : verify_far<Q == 1>(q_row, off, V, c, h, q_vec, Q == 1 ? 0u : 0xFF80u);
+    return verify_rest<F32, Q>(s.row, w, qr, c, h, vmax);
+  };
   auto chunk_weight = [&](int c, bool stored) {
     uint64_t v = 0ull;
 #pragma unroll 1
@@ -516,26 +525,9 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
     }
     return v;
   };
-  const bool direct = given_mass && !(P.state && P.commit);                 // (a commit changes the state that blocks of other rows may not have read yet)
-  unsigned long long mass = 0ull;
+  unsigned long long mass;
   VerifySums shares;                                                        // the blocks' shares of what is drawn from
-  int j = r;
-  if (given_mass) {
-    if (tester) {
-      if (tests) keep_drafter();
-      const uint32_t rejects = __ballot_sync(kFull, test(t_prob(canon_zero(t_max), t_mass), r == 0 && rank == 0));
-      if (lane == 0) s.j = rejects ? __ffs(static_cast<int>(rejects)) - 1 : L;
-    }
-    __syncthreads();
-    join();
-    j = s.j;
-    mass = P.row_mass[row];
-    if (r != j) {
-      if (!direct && rank == 0 && warp == 0) verify_arrive(P, rd, r, launch, false, -1);   // (beyond j it does not matter)
-      cp_async_wait<0>();                                                   // (nothing of a block is in flight when it leaves its shared memory to another)
-      return;
-    }
-  } else {
+  {
     uint64_t own = 0ull;
 #pragma unroll 1
     for (int c = w0 + lane; c < w1; c += 32) {
@@ -547,7 +539,7 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
       } else own += chunk_weight(c, false);
     }
     float t_q = 0.0f;
-    if (Q == 2 && tests && drafter) { keep_drafter(); t_q = t_prob(t_max, t_mass); }   // (the drafter's side, before the mass is known)
+    if (Q == 2 && tests && drafter) { s.row.qv = t.vmax; s.row.q_of.init(t.mass); t_q = t.prob(t.vmax, t.mass, c2); }   // (the drafter's side, before the mass is known)
     own = warp_sum_u64(own);
     if (lane == 0) s.own[warp] = own;
     __syncthreads();
@@ -557,8 +549,12 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
     mass = verify_sums(s.x_own, C, shares);
     if (has_q) {
       if (tester) {
-        const bool no = test(drafter ? t_q : t_prob(vmax, mass), rank == 0);
-        if (lane == 0) { s.reject = no; s.row.p_of.init(mass); }
+        const float pq = drafter ? t_q : t.prob(vmax, mass, c2);
+        const bool no = t.rejects(pq);
+        if (lane == 0) {
+          if (rank == 0 && P.out_p_draft) P.out_p_draft[r] = pq;
+          s.reject = no; s.row.p_of.init(mass);
+        }
       }
       __syncthreads();
       if (!s.reject) {
@@ -571,9 +567,7 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
 
   // ---- the draw: over the residual max(p - q, 0) of a rejected draft, over p itself on the bonus row or where the residual is empty -----------
   cp_async_wait<0>();
-  auto deliver = [&](int token) {                                           // one whole warp of the cluster
-    if (direct) verify_outputs(P, rd, false, j, token); else verify_arrive(P, rd, r, launch, r < L, token);
-  };
+  auto deliver = [&](int token) { verify_arrive(P, rd, r, launch, r < L, token); };   // one whole warp of the cluster
   // The sums of the draw: the residual's, and where that is empty the row's own once more (the mass's sums will do where there is no draft). Or, in the reference's
   // form (kernels/common/sample.metal:322-346), the best of ln(p - q) + noise of stream 4000, and where nothing is left the best of the row's own Gumbel keys.
   // The best key of this thread's chunks over the residual, whose weight in the warp's range is `there` (of 2^40). A key of ln there - 1.5 is missed once in 90, and
@@ -627,7 +621,7 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
   };
   const unsigned long long* parts = reinterpret_cast<const unsigned long long*>(s.own);
   uint64_t there = mass;                                                    // the weight of all blocks (or the best key)
-  if (has_q || given_mass || gumbel) {
+  if (has_q || gumbel) {
     parts = reinterpret_cast<const unsigned long long*>(s.res);
     residual = has_q;
     bool first = true;
@@ -637,21 +631,16 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
       if (mass > 0ull && !(gumbel && !residual)) {
 #pragma unroll 1
         for (int c = w0 + lane; c < w1; c += 32) {
-          FloorSum sum;
           uint64_t v = 0ull;
-          const uint32_t kept = few ? kept_of(c) : 0u;
-          if (few && __popc(kept) <= 2) {
-#pragma unroll 1
-            for (uint32_t m = kept; m; m &= m - 1u) { const int e = __ffs(static_cast<int>(m)) - 1; v += verify_element<F32, Q>(s.row, 8 * c + e - off, z_at(c, e), residual, vmax); }
-          } else if (first && z_cached) {
+          if (first && z_cached) {
             float2 x[4];
-            if (weighed) {
+            FloorSum sum;
+            {
               const uint4 a = zs[c], b = zs[per + c];
               x[0] = make_float2(__uint_as_float(a.x), __uint_as_float(a.y)); x[1] = make_float2(__uint_as_float(a.z), __uint_as_float(a.w));
               x[2] = make_float2(__uint_as_float(b.x), __uint_as_float(b.y)); x[3] = make_float2(__uint_as_float(b.z), __uint_as_float(b.w));
-            } else weigh(c, sum, x);
-            if (has_q) {
-              sum = FloorSum();
+            }
+            {
               uint32_t any = 0u;
               bool below = false;
 #pragma unroll
@@ -695,8 +684,8 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
               to[c] = make_uint4(__float_as_uint(x[0].x), __float_as_uint(x[0].y), __float_as_uint(x[1].x), __float_as_uint(x[1].y));
               to[per + c] = make_uint4(__float_as_uint(x[2].x), __float_as_uint(x[2].y), __float_as_uint(x[3].x), __float_as_uint(x[3].y));
             }
-          } else v += chunk_weight(c, weighed);
-          v += sum.sum();
+            v += sum.sum();
+          } else v = chunk_weight(c, keep_w);
           if (z_cached) sums[c] = v;
           w += v;
         }
@@ -731,7 +720,7 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
   if (warp != max(part, 0)) return;
   // the first element, in index order, at which the running weight passes the target: the chunk from the chunks' sums, then a lane for each of its elements
   // ... where the draw's weights lie: in the drafter's place, or where the row itself is drawn from in the logits' place; a residual that was not kept is formed again
-  const bool kept_values = z_cached && q_cached && (has_q || given_mass) && residual == has_q;
+  const bool kept_values = z_cached && q_cached && residual;
   int token = -1;
 #pragma unroll 1
   for (int b0 = w0; b0 < w1 && part >= 0; b0 += 32) {
@@ -750,10 +739,9 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
       const int ch = b0 + __ffs(static_cast<int>(hit)) - 1, e = lane & 7, h = e >> 2;
       run = __shfl_sync(kFull, run, ch - b0);
       uint64_t v;
-      if (few) v = (kept_of(ch) >> e) & 1u ? verify_element<F32, Q>(s.row, 8 * ch + e - off, z_at(ch, e), residual, vmax) : 0ull;
-      else if (kept_values || (weighed && !residual)) v = __float2ull_rz(reinterpret_cast<const float*>((kept_values ? qs : zs) + (h ? per : 0) + ch)[e & 3]);
+      if (kept_values || (keep_w && !residual)) v = __float2ull_rz(reinterpret_cast<const float*>((kept_values ? qs : zs) + (h ? per : 0) + ch)[e & 3]);
       else {
-        const float4 x = half_weight(ch, h, weighed);
+        const float4 x = half_weight(ch, h, keep_w);
         v = __float2ull_rz((e & 2) ? ((e & 1) ? x.w : x.z) : ((e & 1) ? x.y : x.x));
       }
       uint64_t upto = v;
@@ -772,31 +760,12 @@ template <bool F32, int Q>
 static __global__ void __launch_bounds__(kVerifyThreads, 2) verify_kernel(const __grid_constant__ VerifyDev P, int C, int z_cached, int q_cached) {
   extern __shared__ __align__(16) uint4 v_smem[];
   __shared__ VerifySmem s;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int rank = C > 1 ? static_cast<int>(cluster_rank()) : 0, r = static_cast<int>(blockIdx.x) / C;
   after_predecessor();
   unsigned long long launch;
   asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(launch) : "l"(&P.ws->launches) : "memory");
-  VerifyRound rd{P.n_draft, 0, P.seed, P.step, false, false, false};
-  if (P.state) {
-    StepStateView st{P.state, P.t_max, P.g};
-    if (st.done()) rd.idle = true;
-    else if (st.prefill_left() > 0u) { rd.idle = true; rd.prefill = true; }
-    else {
-      const uint32_t len = st.verify_len(), rows = st.t_this_step();
-      if (len > static_cast<uint32_t>(P.n_draft) || rows < len + 1u || rows > static_cast<uint32_t>(P.n_draft) + 1u) rd.mismatch = true;
-      else { rd.L = static_cast<int>(len); rd.row0 = static_cast<int>(rows - 1u - len); }
-    }
-    rd.seed = st.seed(); rd.step = st.step();
-  }
-  if (rd.idle || rd.mismatch) {
-    // nothing is verified; block 0 still closes a prefill chunk (the scan's prefill branch) or reports the caller's error
-    if (blockIdx.x == 0 && warp == 0) {
-      if (rd.mismatch) {
-        if (lane == 0) { P.out_accept[0] = -1; P.out_final[0] = -1; StepStateView st{P.state, P.t_max, P.g}; fail_state(st, kErrRoundMismatch); }
-      } else if (rd.prefill) verify_commit(P, false);
-    }
-  } else if (r <= rd.L) {                                                   // (a state may verify fewer rows than the launch has clusters)
+  VerifyRound rd;
+  if (verify_begin(P, rd) && r <= rd.L) {                                   // (a state may verify fewer rows than the launch has clusters)
     if (C > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // this block runs, and has read the state
     verify_row<F32, Q>(P, rd, r, rank, C, launch, z_cached != 0, q_cached != 0, v_smem, s);
   }

@@ -6,6 +6,7 @@ import torch
 
 import lithos_metal_b200 as lm
 import oracle
+from lithos_metal_b200 import _lib
 from tests.test_gpu_sampling import bf16_tensor
 from tests.test_gpu_verify_slices import check, on_gpu, step
 
@@ -151,3 +152,42 @@ def test_draft_values_below_zero(vocab, n, dtype):
             for uf in (0.0, rng.random(), rng.random(), LAST):
                 check(t, d, x, ua, np.float32(uf))
             check(t, d, x, ua, np.float32(rng.random()), tau=tau)
+
+
+@pytest.mark.parametrize("residual_draw", ["inverse_cdf", "gumbel"])
+def test_withheld_shares_are_reported_where_masses_are_given(residual_draw):
+    """The decisive row's shares: the first block's does not come, the launch reports an error through outputs and state, and the next one is right."""
+    vocab, n = 151936, 7
+    layout = lm.StepStateLayout(n + 1, n)
+    rng, target, _, q = step(vocab, n, "bf16", 3)
+    z = oracle.bf16_to_f32(target)
+    d, ua = rejecting(z, q, 2)
+    given = dict(target_vmax=torch.from_numpy(z.max(-1)).cuda(),
+                 target_mass=torch.tensor([oracle.kept_mass(z[r], -np.inf, 1.0) for r in range(n + 1)], dtype=torch.int64, device="cuda"))
+    st = layout.to_device(dict(step=2, verify_len=n, t_this_step=n + 1, pending_tokens=[5] + d.tolist(), position=40))
+    ring = torch.zeros(16, dtype=torch.int64, device="cuda")
+    call = lambda **kw: lm.verify(on_gpu(target), torch.from_numpy(d).cuda(), torch.from_numpy(q).cuda(), torch.from_numpy(ua).cuda(), torch.tensor([0.4]),   # noqa: E731
+                                  "stochastic", residual_draw=residual_draw, seed=9, step=4, **given, **kw)
+    out = call(commit=dict(layout=layout, state=st, ring=ring), wait_limit=300, selftest=_lib.VERIFY_SELFTEST_WITHHOLD)
+    assert int(out[0]) == -1 and out[2].tolist() == [-1] * (n + 1)
+    after = layout.from_device(st)
+    assert after["error"] == 3 and after["done"] == 1 and int(ring.abs().sum()) == 0
+    acc, fin, gap = oracle.verify_gumbel(target, d, q, seed=9, step=4, u_accept=ua) if residual_draw == "gumbel" else (*oracle.verify_stochastic(target, d, q, ua, 0.4)[:2], 1.0)
+    out = call()
+    assert int(out[0]) == acc == 2 and (int(out[1]) == fin or gap < 1e-5)
+
+
+# one block, two, as many as there are chunks of 64 for, the line of 120, several turns a block; slices whose last halves lie outside the row
+@pytest.mark.parametrize("vocab", [1, 7, 511, 513, 1027, 61439, 61448, 245761, 303105, 700003])
+@pytest.mark.parametrize("dtype", ["bf16", "fp32"])
+def test_decisive_row_over_all_blocks(vocab, dtype):
+    n = 2
+    rng, target, _, q = step(vocab, n, dtype, vocab)
+    z = oracle.bf16_to_f32(target) if dtype == "bf16" else target
+    tau = np.sort(z, axis=-1)[:, -max(1, vocab // 3)].astype(np.float32)
+    for at in (0, n - 1):
+        for kept in (None, tau):
+            d, ua = rejecting(z, q, at, tau=kept)
+            for uf in (0.0, rng.random(), LAST):
+                check(target, d, q, ua, np.float32(uf), tau=kept)
+    check(target, z[:n].argmax(-1).astype(np.int32), q, np.zeros(n, np.float32), np.float32(rng.random()))
