@@ -153,10 +153,10 @@ static int launch_verify_given(const VerifyDev& P, int sms, cudaStream_t st) {
 }
 
 // ... and not given: a cluster per target row, as many blocks each as let all of them run at once.
-template <bool F32, int Q>
+template <bool F32, int Q, bool kGumbel>
 static int launch_verify(const VerifyDev& P, int sms, cudaStream_t st) {
-  const KernelSlot slot = static_cast<KernelSlot>(kSlotVerify + (F32 ? 3 : 0) + Q);
-  const void* fn = reinterpret_cast<const void*>(verify_kernel<F32, Q>);
+  const KernelSlot slot = static_cast<KernelSlot>(kSlotVerify + (F32 ? 5 : 0) + Q + (kGumbel ? 2 : 0));
+  const void* fn = reinterpret_cast<const void*>(verify_kernel<F32, Q, kGumbel>);
   const int rc = ensure_dynamic_smem(slot, fn, kVerifySmem, true);
   if (rc != LM_OK) return rc;
   const int rows = P.n_draft + 1;
@@ -166,14 +166,15 @@ static int launch_verify(const VerifyDev& P, int sms, cudaStream_t st) {
   const bool z_cached = z <= kVerifySmem, q_cached = q != 0 && (z_cached ? z : 0) + q <= kVerifySmem;
   const size_t smem = (z_cached ? z : 0) + (q_cached ? q : 0);
   const unsigned grid = static_cast<unsigned>(rows) * static_cast<unsigned>(C);
-  return launch_stream(static_cast<int>(grid) <= sms, verify_kernel<F32, Q>, dim3(grid), kVerifyThreads, smem, C, st, P, C, z_cached ? 1 : 0, q_cached ? 1 : 0);
+  return launch_stream(static_cast<int>(grid) <= sms, verify_kernel<F32, Q, kGumbel>, dim3(grid), kVerifyThreads, smem, C, st, P, C, z_cached ? 1 : 0, q_cached ? 1 : 0);
 }
 
 template <bool F32>
 static int launch_verify_rows(const VerifyDev& P, int sms, cudaStream_t st) {
-  if (P.mode != LM_VERIFY_STOCHASTIC) return launch_verify<F32, 0>(P, sms, st);
+  if (P.mode != LM_VERIFY_STOCHASTIC) return launch_verify<F32, 0, false>(P, sms, st);
   if (P.row_max && P.row_mass) return P.q ? launch_verify_given<F32, 1>(P, sms, st) : launch_verify_given<F32, 2>(P, sms, st);
-  return P.q ? launch_verify<F32, 1>(P, sms, st) : launch_verify<F32, 2>(P, sms, st);
+  if (P.draw == LM_DRAW_GUMBEL) return P.q ? launch_verify<F32, 1, true>(P, sms, st) : launch_verify<F32, 2, true>(P, sms, st);
+  return P.q ? launch_verify<F32, 1, false>(P, sms, st) : launch_verify<F32, 2, false>(P, sms, st);
 }
 
 int verify_rows(const VerifyDev& P, int sms, cudaStream_t st) {

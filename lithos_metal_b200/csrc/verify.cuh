@@ -188,7 +188,7 @@ struct VerifyRow {
 struct VerifySmem {
   unsigned long long x_best[kCMaxRanks], x_own[kCMaxRanks], x_res[kCMaxRanks];   // what the blocks of the cluster leave in one another's copy
   uint64_t best[kVerifyWarps], own[kVerifyWarps], res[kVerifyWarps];             // this block's, per warp
-  VerifyRow row; bool reject;
+  VerifyRow row; uint64_t own_block; bool reject;
 };
 
 // The logits of half h of a chunk in pairs (v: the half of a binary32 row, the chunk of a BF16 row), -0 as +0; -inf outside the row.
@@ -333,16 +333,77 @@ struct VerifyTest {
   }
 };
 
+// The best key of the reference's draws in a block's slice (chunks w0 .. w1 are the warp's; zs: in shared memory, the residual, or the logits of a row without a
+// draft): over what is left of p - q, `weight` of it (of 2^40) in the warp's range, or over the row itself. A key of ln(the slice's weight) - 2 is missed once in
+// 1600, and leaves seven or eight logits of the slice to look at closely; where none has reached that bar, it is what has been found, or none. (A bar for each warp's
+// range leaves as many of every range, and a row without a bar a record a step at first; us a call of 7 drafts, 151,936 tokens, all of them rejected 26.4 / 25.6 so,
+// accepted 16.6 / 15.8; all SMs for the decisive row 21.2 and 19.7.)
+template <bool F32, int Q>
+static __device__ __noinline__ uint64_t verify_best_key(const VerifyDev& P, const VerifyRound& rd, VerifySmem& s, const uint4* zs, int w0, int w1, int per, int row, bool residual, bool has_q,
+                                                        bool q_vec, uint64_t weight, float vmax) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, off = s.row.off;
+  const float tau = s.row.tau;
+  if (lane == 0) s.res[warp] = weight;
+  __syncthreads();
+  const uint64_t there = residual ? warp_sum_u64(lane < kVerifyWarps ? s.res[lane] : 0ull) : s.own_block;
+  ResidualScan rest;
+  GumbelScan own;
+  rest.init(rd.seed, rd.step, 4000u);
+  own.init(rd.seed, rd.step, static_cast<uint32_t>(row), P.temperature, -INFINITY);
+  // (Floors that add up to nothing leave residuals below 2^-40, which have their keys all the same: no bar.)
+  float bar = there ? logf(__ull2float_rn(there) * 0x1p-40f) - 2.0f + (residual ? 0.0f : vmax * own.inv_t32) : -INFINITY;
+  if (!(fabsf(bar) < 1e30f)) bar = -INFINITY;
+#pragma unroll 1
+  for (;;) {
+    rest.room = 8388608.0f * ex2_approx((2e-3f - bar) * 1.44269504f);
+    own.kb = INFINITY;
+    own.raise(bar);
+#pragma unroll 1
+    for (int b0 = 2 * w0; b0 < 2 * w1; b0 = (b0 & 1) ? b0 + 63 : b0 + 1) {  // (whole warps)
+      const int c = (b0 >> 1) + lane, h = b0 & 1, i = 8 * c + 4 * h - off;
+      uint4 v = make_uint4(0u, 0u, 0u, 0u);
+      if (residual) {
+        if (c < w1) {
+          if (zs) v = zs[(h ? per : 0) + c];
+          else {
+            const float4 x = verify_far_rest<F32, Q>(s.row, verify_far<F32>(s.row.z_row, off, s.row.V, c, h, true, F32 ? 0xFF800000u : 0xFF80u), q_vec, c, h, vmax);
+            v = make_uint4(__float_as_uint(x.x), __float_as_uint(x.y), __float_as_uint(x.z), __float_as_uint(x.w));
+          }
+        }
+        const float r4[4] = {__uint_as_float(v.x) * 0x1p-40f, __uint_as_float(v.y) * 0x1p-40f, __uint_as_float(v.z) * 0x1p-40f, __uint_as_float(v.w) * 0x1p-40f};   // p - q, exactly
+        const uint64_t had = rest.best;
+        rest.offer4(r4, i);
+        rest.share(had);
+      } else {
+        float2 z[2] = {make_float2(-INFINITY, -INFINITY), make_float2(-INFINITY, -INFINITY)};
+        if (c < w1) verify_pairs<F32>(zs && !has_q ? zs[(F32 && h ? per : 0) + c] : verify_far<F32>(s.row.z_row, off, s.row.V, c, h, true, F32 ? 0xFF800000u : 0xFF80u), h, z);
+        const uint64_t had = own.best;
+#pragma unroll
+        for (int k = 0; k < 2; k++)                                         // (what is not kept, or lies outside the row, is -inf: no key)
+          own.offer2(z[k].x >= tau ? z[k].x : -INFINITY, static_cast<uint32_t>(i + 2 * k), z[k].y >= tau ? z[k].y : -INFINITY, static_cast<uint32_t>(i + 2 * k + 1));
+        if (__any_sync(kFull, own.best != had)) own.raise(best_value(warp_max_u64(own.best)));
+      }
+    }
+    const uint64_t mine = warp_max_u64(residual ? rest.best : own.best);
+    if (lane == 0) s.best[warp] = mine;
+    __syncthreads();
+    const uint64_t top = warp_max_u64(lane < kVerifyWarps ? s.best[lane] : 0ull);
+    if (bar == -INFINITY || (top && best_value(top) >= bar)) return top;
+    bar = top ? best_value(top) : -INFINITY;
+    __syncthreads();                                                        // (everybody has read the warps' best)
+  }
+}
+
 // One row by one cluster. Q: 0 greedy, 1 the drafter's probabilities, 2 its BF16 logits and their statistics. Every part of this runs a few times a launch, so
 // code that is not in the instruction cache costs as much as what it computes: a loop's chunk is unrolled, loops are not, what has been computed is kept rather
 // than computed by a second copy of the code (the token was found in 2.5 to 3.3 us so, in 1 with the draw's weights kept), and the rare is in functions of its own.
-template <bool F32, int Q>
+template <bool F32, int Q, bool kGumbel>
 __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound& rd, int r, int rank, int C, unsigned long long launch, bool z_cached, bool q_cached,
                                            uint4* zs, VerifySmem& s) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int kSize = F32 ? 4 : 2;
   const int V = P.vocab, L = rd.L, row = rd.row0 + r;
-  const bool has_q = Q != 0 && r < L, gumbel = P.draw == LM_DRAW_GUMBEL;
+  const bool has_q = Q != 0 && r < L;
   const bool given_max = Q != 0 && P.row_max != nullptr;
   // ---- this block's slice in chunks of eight; a warp's are consecutive, so that what a warp holds is a range of the row ------------------------
   const char* z_row = static_cast<const char*>(P.target) + static_cast<size_t>(row) * static_cast<size_t>(P.row_stride) * kSize;
@@ -475,7 +536,7 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
   if (Q == 0) return;
 
   // ---- the kept set's mass and the accept test ---------------------------------------------------------------------------------------------
-  const bool keep_w = z_cached && !(gumbel && !has_q);                      // the weights replace the logits
+  const bool keep_w = z_cached && !(kGumbel && !has_q);                      // the weights replace the logits
   // a chunk's weights, as floors, from its logits in shared memory; nothing kept of it costs its maximum
   auto weigh = [&](int c, FloorSum& sum, float2 (&w)[4]) {
     const float tau = s.row.tau;
@@ -544,7 +605,11 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
     if (lane == 0) s.own[warp] = own;
     __syncthreads();
     join();
-    if (warp == 0) push(s.x_own, warp_sum_u64(lane < kVerifyWarps ? s.own[lane] : 0ull), true);
+    if (warp == 0) {
+      const uint64_t block = warp_sum_u64(lane < kVerifyWarps ? s.own[lane] : 0ull);
+      push(s.x_own, block, true);
+      if (lane == 0) s.own_block = block;
+    }
     cluster_sync(C);
     mass = verify_sums(s.x_own, C, shares);
     if (has_q) {
@@ -570,65 +635,16 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
   auto deliver = [&](int token) { verify_arrive(P, rd, r, launch, r < L, token); };   // one whole warp of the cluster
   // The sums of the draw: the residual's, and where that is empty the row's own once more (the mass's sums will do where there is no draft). Or, in the reference's
   // form (kernels/common/sample.metal:322-346), the best of ln(p - q) + noise of stream 4000, and where nothing is left the best of the row's own Gumbel keys.
-  // The best key of this thread's chunks over the residual, whose weight in the warp's range is `there` (of 2^40). A key of ln there - 1.5 is missed once in 90, and
-  // leaves four or five logits to look at closely; where none has reached it, the bar is what has been found, or lower.
-  auto best_of_rest = [&](uint64_t there) {
-    ResidualScan rest;
-    rest.init(rd.seed, rd.step, 4000u);
-    // (Floors that add up to nothing leave residuals below 2^-40, which have their keys all the same: the first is looked for without a bar.)
-    float bar = there ? logf(__ull2float_rn(there) * 0x1p-40f) - 1.5f : -INFINITY;
-#pragma unroll 1
-    for (;;) {
-      rest.room = 8388608.0f * ex2_approx((2e-3f - bar) * 1.44269504f);
-#pragma unroll 1
-      for (int b0 = 2 * w0; b0 < 2 * w1; b0 = (b0 & 1) ? b0 + 63 : b0 + 1) {  // (whole warps)
-        const int c = (b0 >> 1) + lane, h = b0 & 1;
-        float r4[4] = {0.0f, 0.0f, 0.0f, 0.0f};                             // p - q, exactly; nothing outside the row
-        if (c < w1) {
-          float4 x;
-          if (z_cached) {
-            const uint4 v = zs[(h ? per : 0) + c];
-            x = make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
-          } else x = half_weight(c, h, false);
-          r4[0] = x.x * 0x1p-40f; r4[1] = x.y * 0x1p-40f; r4[2] = x.z * 0x1p-40f; r4[3] = x.w * 0x1p-40f;
-        }
-        const uint64_t had = rest.best;
-        rest.offer4(r4, 8 * c + 4 * h - off);
-        rest.share(had);
-      }
-      const uint64_t top = warp_max_u64(rest.best);
-      if ((top && best_value(top) >= bar) || rest.room == INFINITY) return rest.best;
-      bar = top ? best_value(top) : bar - 3.0f;
-    }
-  };
-  // ... and over the row itself (the logits of a row with a draft have been written over).
-  auto best_of_row = [&]() {
-    GumbelScan own;
-    own.init(rd.seed, rd.step, static_cast<uint32_t>(row), P.temperature, -INFINITY);
-#pragma unroll 1
-    for (int b0 = 2 * w0; b0 < 2 * w1; b0 = (b0 & 1) ? b0 + 63 : b0 + 1) {
-      const int c = (b0 >> 1) + lane, h = b0 & 1, i = 8 * c + 4 * h - off;
-      float2 z[2] = {make_float2(-INFINITY, -INFINITY), make_float2(-INFINITY, -INFINITY)};
-      if (c < w1) verify_pairs<F32>(has_q ? verify_far<F32>(z_row, off, V, c, h, true, kOut) : z_raw(c, h), h, z);
-      const float tau = s.row.tau;
-#pragma unroll
-      for (int k = 0; k < 2; k++)                                           // (what is not kept, or lies outside the row, is -inf: no key)
-        own.offer2(z[k].x >= tau ? z[k].x : -INFINITY, static_cast<uint32_t>(i + 2 * k), z[k].y >= tau ? z[k].y : -INFINITY, static_cast<uint32_t>(i + 2 * k + 1));
-      const uint64_t top = warp_max_u64(own.best);
-      if (top) own.raise(best_value(top));
-    }
-    return own.best;
-  };
   const unsigned long long* parts = reinterpret_cast<const unsigned long long*>(s.own);
   uint64_t there = mass;                                                    // the weight of all blocks (or the best key)
-  if (has_q || gumbel) {
+  if (has_q || kGumbel) {
     parts = reinterpret_cast<const unsigned long long*>(s.res);
     residual = has_q;
     bool first = true;
 #pragma unroll 1
     for (;; residual = first = false) {
       uint64_t w = 0ull;
-      if (mass > 0ull && !(gumbel && !residual)) {
+      if (mass > 0ull && !(kGumbel && !residual)) {
 #pragma unroll 1
         for (int c = w0 + lane; c < w1; c += 32) {
           uint64_t v = 0ull;
@@ -679,8 +695,8 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
                 }
               }
             }
-            if (gumbel || q_cached) {
-              uint4* to = gumbel ? zs : qs;
+            if (kGumbel || q_cached) {
+              uint4* to = kGumbel ? zs : qs;
               to[c] = make_uint4(__float_as_uint(x[0].x), __float_as_uint(x[0].y), __float_as_uint(x[1].x), __float_as_uint(x[1].y));
               to[per + c] = make_uint4(__float_as_uint(x[2].x), __float_as_uint(x[2].y), __float_as_uint(x[3].x), __float_as_uint(x[3].y));
             }
@@ -691,20 +707,20 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
         }
       }
       w = warp_sum_u64(w);
-      if (gumbel) w = warp_max_u64(mass == 0ull ? 0ull : residual ? best_of_rest(w) : best_of_row());
+      if (kGumbel) w = mass == 0ull ? 0ull : verify_best_key<F32, Q>(P, rd, s, z_cached ? zs : nullptr, w0, w1, per, row, residual, has_q, q_vec, residual ? w : 0ull, vmax);
       if (lane == 0) s.res[warp] = w;
       __syncthreads();
       if (warp == 0) {
         w = lane < kVerifyWarps ? s.res[lane] : 0ull;
-        push(s.x_res, gumbel ? warp_max_u64(w) : warp_sum_u64(w), true);
+        push(s.x_res, kGumbel ? warp_max_u64(w) : warp_sum_u64(w), true);
       }
       cluster_sync(C);
-      there = gumbel ? warp_max_u64(lane < C ? s.x_res[lane] : 0ull) : verify_sums(s.x_res, C, shares);
+      there = kGumbel ? warp_max_u64(lane < C ? s.x_res[lane] : 0ull) : verify_sums(s.x_res, C, shares);
       if (there || !residual) break;
       cluster_sync(C);                                                      // (everybody has read the slots)
     }
   }
-  if (gumbel) {
+  if (kGumbel) {
     if (rank == 0 && warp == 0) deliver(there ? static_cast<int>(best_index(there)) : -1);
     return;
   }
@@ -756,7 +772,7 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
   deliver(token);
 }
 
-template <bool F32, int Q>
+template <bool F32, int Q, bool kGumbel>
 static __global__ void __launch_bounds__(kVerifyThreads, 2) verify_kernel(const __grid_constant__ VerifyDev P, int C, int z_cached, int q_cached) {
   extern __shared__ __align__(16) uint4 v_smem[];
   __shared__ VerifySmem s;
@@ -767,7 +783,7 @@ static __global__ void __launch_bounds__(kVerifyThreads, 2) verify_kernel(const 
   VerifyRound rd;
   if (verify_begin(P, rd) && r <= rd.L) {                                   // (a state may verify fewer rows than the launch has clusters)
     if (C > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // this block runs, and has read the state
-    verify_row<F32, Q>(P, rd, r, rank, C, launch, z_cached != 0, q_cached != 0, v_smem, s);
+    verify_row<F32, Q, kGumbel>(P, rd, r, rank, C, launch, z_cached != 0, q_cached != 0, v_smem, s);
   }
 }
 

@@ -191,3 +191,26 @@ def test_decisive_row_over_all_blocks(vocab, dtype):
             for uf in (0.0, rng.random(), LAST):
                 check(target, d, q, ua, np.float32(uf), tau=kept)
     check(target, z[:n].argmax(-1).astype(np.int32), q, np.zeros(n, np.float32), np.float32(rng.random()))
+
+
+@pytest.mark.parametrize("vocab,n", [(16385, 2), (50257, 7), (151936, 15)])
+@pytest.mark.parametrize("dtype", ["bf16", "fp32"])
+def test_best_keys_of_rows_and_residuals(vocab, n, dtype):
+    """The reference's draw where the best key lies far above or below what a slice's weight lets expect: one token with all the weight, a flat row, a row of two
+    values, temperatures at both ends, a residual of one element; accepted and rejected rounds, many noises."""
+    rng, target, _, q = step(vocab, n, "fp32", 29)
+    rows = {"random": target, "flat": np.zeros_like(target), "one": np.where(np.arange(vocab) == vocab // 3, 9.0, -9.0) + np.zeros_like(target),
+            "two": np.where(np.arange(vocab) % 2 == 0, 1.0, -30.0) + np.zeros_like(target)}
+    for name, zf in rows.items():
+        t = oracle.f32_to_bf16(zf.astype(np.float32)) if dtype == "bf16" else zf.astype(np.float32)
+        z = oracle.bf16_to_f32(t) if dtype == "bf16" else t
+        lone = np.ones_like(q)
+        lone[:, vocab - 2] = 0.0
+        for T in (0.05, 1.0, 30.0):
+            for x, d, u in ((q, z[:n].argmax(-1), np.zeros(n)), (q, np.full(n, -1), np.full(n, LAST)), (lone, np.full(n, 5), np.full(n, LAST))):
+                d, u = d.astype(np.int32), u.astype(np.float32)
+                for seed in (0, 1, 2):
+                    acc, fin, gap = oracle.verify_gumbel(t, d, x, seed=seed, step=seed, temperature=T, u_accept=u)
+                    out = lm.verify(on_gpu(t), torch.from_numpy(d).cuda(), torch.from_numpy(x).cuda(), torch.from_numpy(u).cuda(), None, "stochastic", temperature=T,
+                                    residual_draw="gumbel", seed=seed, step=seed)
+                    assert int(out[0]) == acc and (int(out[1]) == fin or gap < 1e-5 * max(1.0, abs(z).max() / T)), (name, T, seed)
