@@ -152,29 +152,41 @@ static int launch_verify_given(const VerifyDev& P, int sms, cudaStream_t st) {
   return launch_stream(true, verify_given_kernel<F32, Q>, dim3(static_cast<unsigned>(grid)), kVerifyThreads, kAloneSmem, 1, st, P);
 }
 
-// ... and not given: a cluster per target row, as many blocks each as let all of them run at once.
-template <bool F32, int Q, bool kGumbel>
+// ... and not given: a cluster per target row, as many blocks each as let all of them run at once. In two launches, the first of them clusters for the maxima and
+// masses, where a slice does not fit shared memory (us by clusters alone / so, and by all SMs for the decisive row in a cooperative launch; first draft rejected and, in
+// brackets, all accepted: 15 drafts, 200,000 tokens 53.5 / 25.5, 32.5 (27.9 / 24.8, 24.8), the reference's draw 81.3 / 27.2, 29.4; 262,144 60.5 / 27.3, 42.2; 7 drafts, 400,000
+// 45.7 / 26.3, 28.9; but 3 of 1,000,000 85 / 35, 34 (40 / 35, 28)). And for the reference's draw from eight rows on, whose eighth cluster of sixteen shares another's SMs, where
+// rows are long (7 drafts, 151,936 tokens 23.6 / 17.3, 21.2 (14.8 / 15.3, 19.7), 65,536 15.4 / 14.6, 20.5 (10.9 / 13.0, 19.9); 15 of 100,000 27.6 / 17.8, 24.3 (18.4 / 16.2, 25.7);
+// 3 of 151,936 16.9 / 17.1, 17.6 (13.7 / 15.2, 16.7)).
+template <bool F32, int Q, int kMode>
 static int launch_verify(const VerifyDev& P, int sms, cudaStream_t st) {
-  const KernelSlot slot = static_cast<KernelSlot>(kSlotVerify + (F32 ? 5 : 0) + Q + (kGumbel ? 2 : 0));
-  const void* fn = reinterpret_cast<const void*>(verify_kernel<F32, Q, kGumbel>);
+  const KernelSlot slot = static_cast<KernelSlot>(kSlotVerify + (F32 ? 6 : 0) + (Q == 0 ? 0 : kMode == kVerifyStats ? 1 : 2 * Q + kMode));
+  const void* fn = reinterpret_cast<const void*>(verify_kernel<F32, Q, kMode>);
   const int rc = ensure_dynamic_smem(slot, fn, kVerifySmem, true);
   if (rc != LM_OK) return rc;
   const int rows = P.n_draft + 1;
   const int C = cluster_that_fits(cluster_blocks(rows, P.vocab, 2 * sms), [&](int c) { return clusters_at_once(slot, fn, kVerifyThreads, kVerifySmem, c) >= rows; });
   const size_t chunks = (static_cast<size_t>((P.vocab + 14) / 8) + C - 1) / C;   // of a slice, for any alignment of the row
-  const size_t z = chunks * 32 + (chunks + 1) / 2 * 16, q = Q == 0 ? 0 : chunks * 32;   // (logits, then weights; the chunks' sums; the drafter's row, then the residual's weights)
+  const size_t z = chunks * 32 + (chunks + 1) / 2 * 16, q = Q == 0 || kMode == kVerifyStats ? 0 : chunks * 32;   // (logits, then weights; the chunks' sums; the drafter's row, then the residual's weights)
   const bool z_cached = z <= kVerifySmem, q_cached = q != 0 && (z_cached ? z : 0) + q <= kVerifySmem;
+  if (Q != 0 && kMode != kVerifyStats && (!z_cached || (kMode == kVerifyNoise && rows * 20 > sms && P.vocab >= 98304))) {
+    const int rc1 = launch_verify<F32, 1, kVerifyStats>(P, sms, st);
+    if (rc1 != LM_OK) return rc1;
+    VerifyDev G = P;
+    G.row_max = P.ws->vmax; G.row_mass = P.ws->mass;
+    return launch_verify_given<F32, Q == 0 ? 1 : Q>(G, sms, st);
+  }
   const size_t smem = (z_cached ? z : 0) + (q_cached ? q : 0);
   const unsigned grid = static_cast<unsigned>(rows) * static_cast<unsigned>(C);
-  return launch_stream(static_cast<int>(grid) <= sms, verify_kernel<F32, Q, kGumbel>, dim3(grid), kVerifyThreads, smem, C, st, P, C, z_cached ? 1 : 0, q_cached ? 1 : 0);
+  return launch_stream(static_cast<int>(grid) <= sms, verify_kernel<F32, Q, kMode>, dim3(grid), kVerifyThreads, smem, C, st, P, C, z_cached ? 1 : 0, q_cached ? 1 : 0);
 }
 
 template <bool F32>
 static int launch_verify_rows(const VerifyDev& P, int sms, cudaStream_t st) {
-  if (P.mode != LM_VERIFY_STOCHASTIC) return launch_verify<F32, 0, false>(P, sms, st);
+  if (P.mode != LM_VERIFY_STOCHASTIC) return launch_verify<F32, 0, kVerifyDraw>(P, sms, st);
   if (P.row_max && P.row_mass) return P.q ? launch_verify_given<F32, 1>(P, sms, st) : launch_verify_given<F32, 2>(P, sms, st);
-  if (P.draw == LM_DRAW_GUMBEL) return P.q ? launch_verify<F32, 1, true>(P, sms, st) : launch_verify<F32, 2, true>(P, sms, st);
-  return P.q ? launch_verify<F32, 1, false>(P, sms, st) : launch_verify<F32, 2, false>(P, sms, st);
+  if (P.draw == LM_DRAW_GUMBEL) return P.q ? launch_verify<F32, 1, kVerifyNoise>(P, sms, st) : launch_verify<F32, 2, kVerifyNoise>(P, sms, st);
+  return P.q ? launch_verify<F32, 1, kVerifyDraw>(P, sms, st) : launch_verify<F32, 2, kVerifyDraw>(P, sms, st);
 }
 
 int verify_rows(const VerifyDev& P, int sms, cudaStream_t st) {

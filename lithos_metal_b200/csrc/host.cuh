@@ -36,8 +36,8 @@ inline int sm_count(int* out) {
 enum KernelSlot { kSlotFast, kSlotTopk, kSlotTopkOrdered, kSlotGeneric, kSlotVocabLocal, kSlotTileFinish, kSlotSlice, kSlotSliceSmall, kSlotSliceTiny, kSlotSlicedMerge, kSlotHead, kSlotCluster,
                   kSlotArgmax = kSlotCluster + 6,   // (the cluster kernel has six instances, the argmax kernel two)
                   kSlotDraftQ = kSlotArgmax + 2,    // (two instances)
-                  kSlotVerify = kSlotDraftQ + 2,    // (ten)
-                  kSlotVerifyGiven = kSlotVerify + 10,   // (four)
+                  kSlotVerify = kSlotDraftQ + 2,    // (twelve)
+                  kSlotVerifyGiven = kSlotVerify + 12,   // (four)
                   kSlotCount = kSlotVerifyGiven + 4 };
 
 inline int ensure_dynamic_smem(KernelSlot slot, const void* func, size_t bytes, bool large_clusters = false) {

@@ -1,4 +1,4 @@
-// DSpark verification of one speculative step in ONE launch: up to n_draft drafted tokens against n_draft + 1 rows of target
+// DSpark verification of one speculative step, in one launch but for the largest rows: up to n_draft drafted tokens against n_draft + 1 rows of target
 // logits. Greedy: row-wise argmax and prefix match (kernels/common/spec_ops.metal:162-165). Stochastic: accept draft r with
 // probability min(1, p/q), replace the first rejected one by a draw from max(p - q, 0) (kernels/common/sample.metal:273-347),
 // on the integer fixed-point weights so the outcome is independent of how the vocabulary is split between blocks.
@@ -9,7 +9,8 @@
 // copies, all in flight at once; the blocks meet in distributed shared memory, a cluster barrier to a dependency; and every row that could be the
 // decisive one -- its own draft rejected, or the bonus row -- draws its token without waiting for the rows before it. What a row found is one word in
 // the workspace; the cluster that arrives last picks the first rejected row and writes the outputs, so no block waits for another cluster.
-// A launch that is given the rows' maxima and masses knows the decisive row from one logit per draft: verify_given.cuh.
+// A launch that is given the rows' maxima and masses knows the decisive row from one logit per draft: verify_given.cuh. Rows whose slices do not fit shared memory
+// have their maxima and masses found by clusters and go on there in a second launch, and so does the reference's draw of long rows whose clusters share SMs.
 // (All rows cut over all 148 SMs by a cooperative launch, partial results exchanged as polled words in L2, three trips for the step of 7 drafts; us a call so /
 // by clusters, first draft rejected: V = 151,936, drafter's probabilities 25.0 / 18.8, given the maxima 21.0 / 17.6, drafter's logits 27.3 / 20.5, greedy 10.3 / 7.4; 13 drafts 31.4 /
 // 22.4; 50,257 24.8 / 13.7; but the reference's draw over 248,320 with every draft rejected 29.4 / 32.3. A cooperative launch of the clusters is not made ready beside
@@ -38,6 +39,8 @@ struct VerifyWs {                                       // lives in the caller's
   unsigned long long launches;                          // so far
   unsigned arrived, pad;                                // rows (or, of a launch that cuts one row, blocks) of this launch that have been through (0 between launches)
   unsigned long long row[kVerifyMaxRows];               // what a row's cluster found: launch number << 24 | kFound | rejected << 21 | token + 1
+  unsigned long long mass[kVerifyMaxRows];               // rows' masses and maxima, by row of the step, from a launch that finds nothing else to the one behind it
+  float vmax[kVerifyMaxRows];
   unsigned long long part[kVerifyParts][4];             // a block's shares (verify_given.cuh), in halves: launch number + 1 << 32 | half
 };
 constexpr unsigned long long kFound = 1ull << 22, kRejected = 1ull << 21;
@@ -101,12 +104,13 @@ static __device__ __noinline__ void verify_commit(const VerifyDev& P, bool faile
 struct VerifyRound { int L, row0; uint64_t seed; uint32_t step; };
 // False: nothing is verified, as the state is done, this step is a prefill chunk (block 0 still closes it: the scan's prefill branch), or the state's rows do not fit
 // the launch (block 0 reports the caller's error).
-__device__ __forceinline__ bool verify_begin(const VerifyDev& P, VerifyRound& rd) {
+// closes: this launch does that.
+__device__ __forceinline__ bool verify_begin(const VerifyDev& P, VerifyRound& rd, bool closes = true) {
   rd = VerifyRound{P.n_draft, 0, P.seed, P.step};
   if (!P.state) return true;
   StepStateView st{P.state, P.t_max, P.g};
   rd.seed = st.seed(); rd.step = st.step();
-  const bool first = blockIdx.x == 0 && threadIdx.x < 32;
+  const bool first = closes && blockIdx.x == 0 && threadIdx.x < 32;
   if (st.done()) return false;
   if (st.prefill_left() > 0u) {
     if (first) verify_commit(P, false);
@@ -219,8 +223,8 @@ static __device__ __noinline__ float4 verify_below_zero(const VerifyRow& x, int 
   return make_float4(r[0], r[1], r[2], r[3]);
 }
 
-// What half a chunk weighs, before the floors: the kept set's weights (what lies outside the row is -inf: 0). v: the half as it lies in the row. (By clusters for what
-// is rare: slices that do not fit shared memory, and the second look where a residual is empty.)
+// What half a chunk weighs, before the floors: the kept set's weights (what lies outside the row is -inf: 0). v: the half as it lies in the row. (By clusters
+// for slices that do not fit shared memory.)
 template <bool F32>
 static __device__ __noinline__ float4 verify_weights(const VerifyRow& x, uint4 v, int h, float vmax) {
   float2 z[2], w[2];
@@ -259,20 +263,6 @@ static __device__ __noinline__ float4 verify_rest(const VerifyRow& x, float4 f, 
   }
   return make_float4(w[0].x, w[0].y, w[1].x, w[1].y);
 }
-// Both, of a half that is weighed in the draw over the residual.
-template <bool F32, int Q>
-static __device__ __forceinline__ float4 verify_far_rest(const VerifyRow& x, uint4 v, bool q_vec, int c, int h, float vmax) {
-  float2 z[2];
-  verify_pairs<F32>(v, h, z);
-  const float tau = x.tau;
-  if (!(fmaxf(fmaxf(z[0].x, z[0].y), fmaxf(z[1].x, z[1].y)) >= tau)) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);   // (nothing kept: the drafter's row is not read)
-  const uint4 qr = verify_far<Q == 1>(x.q_row, x.off, x.V, c, h, q_vec, Q == 1 ? 0u : 0xFF80u);
-  const float4 w = verify_weights<F32>(x, v, h, vmax);
-  uint2 t, l;
-  const float2 a = floor2(make_float2(w.x, w.y), t, l), b = floor2(make_float2(w.z, w.w), t, l);
-  return verify_rest<F32, Q>(x, make_float4(a.x, a.y, b.x, b.y), qr, c, h, vmax);
-}
-
 // The floors' sum of residuals some of which may be above 2^40.
 static __device__ __noinline__ uint64_t verify_wide(float4 a, float4 b) {
   return __float2ull_rz(a.x) + __float2ull_rz(a.y) + __float2ull_rz(a.z) + __float2ull_rz(a.w) + __float2ull_rz(b.x) + __float2ull_rz(b.y) + __float2ull_rz(b.z) + __float2ull_rz(b.w);
@@ -337,10 +327,10 @@ struct VerifyTest {
 // draft): over what is left of p - q, `weight` of it (of 2^40) in the warp's range, or over the row itself. A key of ln(the slice's weight) - 2 is missed once in
 // 1600, and leaves seven or eight logits of the slice to look at closely; where none has reached that bar, it is what has been found, or none. (A bar for each warp's
 // range leaves as many of every range, and a row without a bar a record a step at first; us a call of 7 drafts, 151,936 tokens, all of them rejected 26.4 / 25.6 so,
-// accepted 16.6 / 15.8; all SMs for the decisive row 21.2 and 19.7.)
-template <bool F32, int Q>
+// accepted 16.6 / 15.8.)
+template <bool F32>
 static __device__ __noinline__ uint64_t verify_best_key(const VerifyDev& P, const VerifyRound& rd, VerifySmem& s, const uint4* zs, int w0, int w1, int per, int row, bool residual, bool has_q,
-                                                        bool q_vec, uint64_t weight, float vmax) {
+                                                        uint64_t weight, float vmax) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, off = s.row.off;
   const float tau = s.row.tau;
   if (lane == 0) s.res[warp] = weight;
@@ -363,20 +353,14 @@ static __device__ __noinline__ uint64_t verify_best_key(const VerifyDev& P, cons
       const int c = (b0 >> 1) + lane, h = b0 & 1, i = 8 * c + 4 * h - off;
       uint4 v = make_uint4(0u, 0u, 0u, 0u);
       if (residual) {
-        if (c < w1) {
-          if (zs) v = zs[(h ? per : 0) + c];
-          else {
-            const float4 x = verify_far_rest<F32, Q>(s.row, verify_far<F32>(s.row.z_row, off, s.row.V, c, h, true, F32 ? 0xFF800000u : 0xFF80u), q_vec, c, h, vmax);
-            v = make_uint4(__float_as_uint(x.x), __float_as_uint(x.y), __float_as_uint(x.z), __float_as_uint(x.w));
-          }
-        }
+        if (c < w1) v = zs[(h ? per : 0) + c];
         const float r4[4] = {__uint_as_float(v.x) * 0x1p-40f, __uint_as_float(v.y) * 0x1p-40f, __uint_as_float(v.z) * 0x1p-40f, __uint_as_float(v.w) * 0x1p-40f};   // p - q, exactly
         const uint64_t had = rest.best;
         rest.offer4(r4, i);
         rest.share(had);
       } else {
         float2 z[2] = {make_float2(-INFINITY, -INFINITY), make_float2(-INFINITY, -INFINITY)};
-        if (c < w1) verify_pairs<F32>(zs && !has_q ? zs[(F32 && h ? per : 0) + c] : verify_far<F32>(s.row.z_row, off, s.row.V, c, h, true, F32 ? 0xFF800000u : 0xFF80u), h, z);
+        if (c < w1) verify_pairs<F32>(!has_q ? zs[(F32 && h ? per : 0) + c] : verify_far<F32>(s.row.z_row, off, s.row.V, c, h, true, F32 ? 0xFF800000u : 0xFF80u), h, z);
         const uint64_t had = own.best;
 #pragma unroll
         for (int k = 0; k < 2; k++)                                         // (what is not kept, or lies outside the row, is -inf: no key)
@@ -394,16 +378,21 @@ static __device__ __noinline__ uint64_t verify_best_key(const VerifyDev& P, cons
   }
 }
 
+// What a launch draws from: kVerifyDraw by inverse CDF, kVerifyNoise the reference's form, kVerifyStats nothing: it leaves the rows' maxima and masses in the workspace.
+constexpr int kVerifyDraw = 0, kVerifyNoise = 1, kVerifyStats = 2;
+
 // One row by one cluster. Q: 0 greedy, 1 the drafter's probabilities, 2 its BF16 logits and their statistics. Every part of this runs a few times a launch, so
 // code that is not in the instruction cache costs as much as what it computes: a loop's chunk is unrolled, loops are not, what has been computed is kept rather
 // than computed by a second copy of the code (the token was found in 2.5 to 3.3 us so, in 1 with the draw's weights kept), and the rare is in functions of its own.
-template <bool F32, int Q, bool kGumbel>
+template <bool F32, int Q, int kMode>
 __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound& rd, int r, int rank, int C, unsigned long long launch, bool z_cached, bool q_cached,
                                            uint4* zs, VerifySmem& s) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int kSize = F32 ? 4 : 2;
+  constexpr bool kGumbel = kMode == kVerifyNoise, kStats = kMode == kVerifyStats;
+  if (Q != 0 && !kStats) z_cached = true;                                   // (else the launch is cut in two: launch_verify)
   const int V = P.vocab, L = rd.L, row = rd.row0 + r;
-  const bool has_q = Q != 0 && r < L;
+  const bool has_q = Q != 0 && !kStats && r < L;
   const bool given_max = Q != 0 && P.row_max != nullptr;
   // ---- this block's slice in chunks of eight; a warp's are consecutive, so that what a warp holds is a range of the row ------------------------
   const char* z_row = static_cast<const char*>(P.target) + static_cast<size_t>(row) * static_cast<size_t>(P.row_stride) * kSize;
@@ -536,7 +525,7 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
   if (Q == 0) return;
 
   // ---- the kept set's mass and the accept test ---------------------------------------------------------------------------------------------
-  const bool keep_w = z_cached && !(kGumbel && !has_q);                      // the weights replace the logits
+  const bool keep_w = !kStats && !(kGumbel && !has_q);                      // the weights replace the logits
   // a chunk's weights, as floors, from its logits in shared memory; nothing kept of it costs its maximum
   auto weigh = [&](int c, FloorSum& sum, float2 (&w)[4]) {
     const float tau = s.row.tau;
@@ -567,24 +556,12 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
     }
   };
   bool residual = false;
-  auto half_weight = [&](int c, int h, bool stored) {
-    if (!stored) return residual ? verify_far_rest<F32, Q>(s.row, z_raw(c, h), q_vec, c, h, vmax) : verify_weights<F32>(s.row, z_raw(c, h), h, vmax);
+  auto half_weight = [&](int c, int h) {                                    // (of the weights that replaced the logits)
     const uint4 v = zs[(h ? per : 0) + c];
     const float4 w = make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
     if (!residual) return w;
     const uint4 qr = q_cached ? qs[(Q == 1 && h ? per : 0) + c] : verify_far<Q == 1>(q_row, off, V, c, h, q_vec, Q == 1 ? 0u : 0xFF80u);
     return verify_rest<F32, Q>(s.row, w, qr, c, h, vmax);
-  };
-  auto chunk_weight = [&](int c, bool stored) {
-    uint64_t v = 0ull;
-#pragma unroll 1
-    for (int h = 0; h < 2; h++) {
-      const float4 x = half_weight(c, h, stored);
-      FloorSum sum;
-      sum.add(make_float2(x.x, x.y)); sum.add(make_float2(x.z, x.w));
-      v += sum.beyond() ? verify_wide(x, make_float4(0.0f, 0.0f, 0.0f, 0.0f)) : sum.sum();
-    }
-    return v;
   };
   unsigned long long mass;
   VerifySums shares;                                                        // the blocks' shares of what is drawn from
@@ -596,8 +573,18 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
         FloorSum sum;
         float2 w[4];
         weigh(c, sum, w);
-        own += sums[c] = sum.sum();
-      } else own += chunk_weight(c, false);
+        const uint64_t sum_c = sum.sum();
+        own += sum_c;
+        if (!kStats) sums[c] = sum_c;
+      } else {
+#pragma unroll 1
+        for (int h = 0; h < 2; h++) {
+          const float4 x = verify_weights<F32>(s.row, z_raw(c, h), h, vmax);
+          FloorSum sum;
+          sum.add(make_float2(x.x, x.y)); sum.add(make_float2(x.z, x.w));
+          own += sum.sum();
+        }
+      }
     }
     float t_q = 0.0f;
     if (Q == 2 && tests && drafter) { s.row.qv = t.vmax; s.row.q_of.init(t.mass); t_q = t.prob(t.vmax, t.mass, c2); }   // (the drafter's side, before the mass is known)
@@ -612,6 +599,10 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
     }
     cluster_sync(C);
     mass = verify_sums(s.x_own, C, shares);
+    if (kStats) {
+      if (rank == 0 && tid == 0) { P.ws->vmax[row] = vmax; P.ws->mass[row] = mass; }
+      return;
+    }
     if (has_q) {
       if (tester) {
         const float pq = drafter ? t_q : t.prob(vmax, mass, c2);
@@ -648,7 +639,7 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
 #pragma unroll 1
         for (int c = w0 + lane; c < w1; c += 32) {
           uint64_t v = 0ull;
-          if (first && z_cached) {
+          if (first) {
             float2 x[4];
             FloorSum sum;
             {
@@ -701,13 +692,21 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
               to[per + c] = make_uint4(__float_as_uint(x[2].x), __float_as_uint(x[2].y), __float_as_uint(x[3].x), __float_as_uint(x[3].y));
             }
             v += sum.sum();
-          } else v = chunk_weight(c, keep_w);
-          if (z_cached) sums[c] = v;
+          } else {
+#pragma unroll 1
+            for (int h = 0; h < 2; h++) {
+              const float4 y = half_weight(c, h);
+              FloorSum sum;
+              sum.add(make_float2(y.x, y.y)); sum.add(make_float2(y.z, y.w));
+              v += sum.sum();
+            }
+          }
+          sums[c] = v;
           w += v;
         }
       }
       w = warp_sum_u64(w);
-      if (kGumbel) w = mass == 0ull ? 0ull : verify_best_key<F32, Q>(P, rd, s, z_cached ? zs : nullptr, w0, w1, per, row, residual, has_q, q_vec, residual ? w : 0ull, vmax);
+      if (kGumbel) w = mass == 0ull ? 0ull : verify_best_key<F32>(P, rd, s, zs, w0, w1, per, row, residual, has_q, residual ? w : 0ull, vmax);
       if (lane == 0) s.res[warp] = w;
       __syncthreads();
       if (warp == 0) {
@@ -736,16 +735,13 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
   if (warp != max(part, 0)) return;
   // the first element, in index order, at which the running weight passes the target: the chunk from the chunks' sums, then a lane for each of its elements
   // ... where the draw's weights lie: in the drafter's place, or where the row itself is drawn from in the logits' place; a residual that was not kept is formed again
-  const bool kept_values = z_cached && q_cached && residual;
+  const bool kept_values = q_cached && residual;
   int token = -1;
 #pragma unroll 1
   for (int b0 = w0; b0 < w1 && part >= 0; b0 += 32) {
     const int c = b0 + lane;
     uint64_t sum = 0ull;
-    if (c < w1) {
-      if (z_cached) sum = sums[c];
-      else sum = chunk_weight(c, false);
-    }
+    if (c < w1) sum = sums[c];
     uint64_t incl = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) { const uint64_t t = __shfl_up_sync(kFull, incl, o); if (lane >= o) incl += t; }
@@ -755,9 +751,9 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
       const int ch = b0 + __ffs(static_cast<int>(hit)) - 1, e = lane & 7, h = e >> 2;
       run = __shfl_sync(kFull, run, ch - b0);
       uint64_t v;
-      if (kept_values || (keep_w && !residual)) v = __float2ull_rz(reinterpret_cast<const float*>((kept_values ? qs : zs) + (h ? per : 0) + ch)[e & 3]);
+      if (kept_values || !residual) v = __float2ull_rz(reinterpret_cast<const float*>((kept_values ? qs : zs) + (h ? per : 0) + ch)[e & 3]);
       else {
-        const float4 x = half_weight(ch, h, keep_w);
+        const float4 x = half_weight(ch, h);
         v = __float2ull_rz((e & 2) ? ((e & 1) ? x.w : x.z) : ((e & 1) ? x.y : x.x));
       }
       uint64_t upto = v;
@@ -772,7 +768,7 @@ __device__ __forceinline__ void verify_row(const VerifyDev& P, const VerifyRound
   deliver(token);
 }
 
-template <bool F32, int Q, bool kGumbel>
+template <bool F32, int Q, int kMode>
 static __global__ void __launch_bounds__(kVerifyThreads, 2) verify_kernel(const __grid_constant__ VerifyDev P, int C, int z_cached, int q_cached) {
   extern __shared__ __align__(16) uint4 v_smem[];
   __shared__ VerifySmem s;
@@ -781,9 +777,9 @@ static __global__ void __launch_bounds__(kVerifyThreads, 2) verify_kernel(const 
   unsigned long long launch;
   asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(launch) : "l"(&P.ws->launches) : "memory");
   VerifyRound rd;
-  if (verify_begin(P, rd) && r <= rd.L) {                                   // (a state may verify fewer rows than the launch has clusters)
+  if (verify_begin(P, rd, kMode != kVerifyStats) && r <= rd.L) {                                   // (a state may verify fewer rows than the launch has clusters)
     if (C > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // this block runs, and has read the state
-    verify_row<F32, Q, kGumbel>(P, rd, r, rank, C, launch, z_cached != 0, q_cached != 0, v_smem, s);
+    verify_row<F32, Q, kMode>(P, rd, r, rank, C, launch, z_cached != 0, q_cached != 0, v_smem, s);
   }
 }
 

@@ -46,10 +46,11 @@ def test_first_rejected_draft_is_replaced(vocab, n, dtype):
         check(target, d, q2, ua, np.float32(rng.random()), gpu_q=dict(draft_logits=bf16_tensor(lb), draft_stats=stats), temperature=0.7)
 
 
+@pytest.mark.parametrize("vocab,n", [(248320, 7), (400001, 7), (262144, 15)])   # (the last two in two launches)
 @pytest.mark.parametrize("draft_form", ["probabilities", "logits"])
-def test_replaced_in_a_round_that_closes_itself(draft_form):
+def test_replaced_in_a_round_that_closes_itself(draft_form, vocab, n):
     """With a StepState that the launch reads and moves on: the state's token is the oracle's."""
-    vocab, n, at, T = 248320, 7, 3, 0.7
+    at, T = 3, 0.7
     layout = lm.StepStateLayout(n + 1, n)
     rng, target, noisy, q = step(vocab, n, "bf16", 11)
     z = oracle.bf16_to_f32(target)
@@ -214,3 +215,28 @@ def test_best_keys_of_rows_and_residuals(vocab, n, dtype):
                     out = lm.verify(on_gpu(t), torch.from_numpy(d).cuda(), torch.from_numpy(x).cuda(), torch.from_numpy(u).cuda(), None, "stochastic", temperature=T,
                                     residual_draw="gumbel", seed=seed, step=seed)
                     assert int(out[0]) == acc and (int(out[1]) == fin or gap < 1e-5 * max(1.0, abs(z).max() / T)), (name, T, seed)
+
+
+@pytest.mark.parametrize("vocab", [50257, 400001])                           # in one launch, in two
+def test_states_without_a_round_are_closed_once(vocab):
+    """A prefill chunk is closed once, a finished state left alone, a state whose rows do not fit reported, also where the step takes two launches."""
+    n = 2
+    layout = lm.StepStateLayout(4, 3)
+    x, q = torch.randn(4, vocab, device="cuda").to(torch.bfloat16), torch.full((3, vocab), 1.0 / vocab, device="cuda")
+    ring = torch.zeros(8, dtype=torch.int64, device="cuda")
+
+    def after(**fields):
+        st = layout.to_device(fields)
+        out = torch.full((6,), -7, dtype=torch.int32, device="cuda")
+        lm.verify(x, None, q, torch.zeros(3).cuda(), torch.tensor([0.5]), "stochastic", step_state=(layout, st), out=out, commit=dict(layout=layout, state=st, ring=ring))
+        return layout.from_device(st), out.tolist()
+
+    got, out = after(step=5, position=40, t_this_step=4, prefill_left=9)
+    assert (got["step"], got["position"], got["n_inject"], got["done"]) == (6, 44, 4, 0) and out == [-7] * 6
+    got, out = after(step=5, position=40, t_this_step=3, verify_len=n, done=1)
+    assert (got["step"], got["position"]) == (5, 40) and out == [-7] * 6
+    got, out = after(step=5, position=40, t_this_step=1, verify_len=3)
+    assert (got["error"], got["done"], got["step"]) == (4, 1, 5) and out[:2] == [-1, -1]
+    assert int(ring.abs().sum()) == 0
+    got, out = after(step=5, position=40, t_this_step=3, verify_len=n, pending_tokens=[1, 2, 3])
+    assert got["step"] == 6 and got["ring_head"] == got["accepted"] + 1 and got["anchor"] == out[1]
