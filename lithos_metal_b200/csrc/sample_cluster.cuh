@@ -48,9 +48,9 @@ constexpr int kCQueue = 128;             // logits a warp's queue of the Gumbel 
 constexpr uint32_t kCallOrdered = 1u, kCallFew = 2u;   // of a launch: the rows are taken by kind; a call of a few rows with one top_k (LM_STATUS_SLICED_PATH)
 constexpr int kOrderRows = 2048;         // rows whose order a block looks up (row_in_order)
 // A list up to this long is ordered by counting larger keys, a longer one by bins first (472 keys: 7.7 us by counting, 1.5 by bins). us a call of 12 FP32 rows, by counting / by bins:
-// top_k 64 15.16 / 15.44, 80 16.10 / 16.33, 100 16.38 / 16.46, 120 16.63 / 16.50, 140 16.98 / 16.58. A list of few distinct values (BF16 logits of one crossing bin) fills few bins, and
+// top_k 64 15.16 / 15.44, 80 16.10 / 16.33, 100 16.38 / 16.46, 120 16.63 / 16.50, 140 16.98 / 16.58. A list of few distinct values (BF16 logits of one crossing bin, penalised or not) fills few bins, and
 // the order inside those is counted all the same: by bins from where counting has a thread per key (inverse CDF, no top_k, means of 16 inputs, by counting to 320 / to 110 / to 256: 4 rows
-// of 248,320 42.4 / 44.1 / 42.5, 45 of 53,442 53.6 / 54.7 / 53.8, one of 151,936 28.8 / 31.0 / 28.5 and, with longer lists, 32.5 / 31.5 / 31.0).
+// of 248,320 42.4 / 44.1 / 42.5, 45 of 53,442 53.6 / 54.7 / 53.8, one of 151,936 28.8 / 31.0 / 28.5 and, with longer lists, 32.5 / 31.5 / 31.0; penalised 29.4 / 31.9 / 29.2).
 constexpr int kCRankOrder = 110, kCRankOrderFew = 256;
 constexpr double kCMassBand = 1e-11;     // relative error of a logit's fixed-point softmass beyond its rounding: 7e-12 of the polynomial, a few 1e-16
 // Threads per block: a block-wide reduction costs shuffles in proportion to its warps (1024 threads: 0.5 us each, measured), so no more
@@ -780,8 +780,8 @@ static __device__ __noinline__ int phase_bin_list(ClusterSmem& s, uint32_t b, in
   // Neighbouring BF16 values of magnitude >= a lie a / 256 apart or more: four of the list's bins, where its span is no more than a. The order of equal ones
   // matters to the draw by inverse CDF alone.
   const float least = zl > 0.0f ? zl : zh < 0.0f ? -zh : 0.0f;
-  const bool few = !F32 && s.R.pen == nullptr, in_bins = few && !s.inverse && zh - zl <= least;
-  if (n <= kCList) order_list<B>(s, n, zh, fmaxf(zl, s.vmin), in_bins, few && !in_bins ? kCRankOrderFew : kCRankOrder);
+  const bool in_bins = !F32 && s.R.pen == nullptr && !s.inverse && zh - zl <= least;
+  if (n <= kCList) order_list<B>(s, n, zh, fmaxf(zl, s.vmin), in_bins, F32 || in_bins ? kCRankOrder : kCRankOrderFew);   // (few values, penalised or not)
   return n;
 }
 

@@ -27,9 +27,9 @@ def test_lists_of_every_kind(centre, dtype, draw, penalised):
         _check(_tensor(host), host, dict(temperature=0.9, top_k=0, top_p=top_p, min_p=0.0), draw=draw, history=hist, rho=1.05, pi=0.01)
 
 
-@pytest.mark.parametrize("draw,near_zero", [("inverse_cdf", False), ("gumbel", True)])
-def test_lists_of_few_values_on_both_sides_of_their_line(draw, near_zero):
-    """BF16 lists that bins alone do not put in order: of a few distinct values for the inverse CDF, and around zero."""
+@pytest.mark.parametrize("draw,near_zero,penalised", [("inverse_cdf", False, False), ("gumbel", True, False), ("gumbel", False, True), ("inverse_cdf", False, True)])
+def test_lists_of_few_values_on_both_sides_of_their_line(draw, near_zero, penalised):
+    """BF16 lists that bins alone do not put in order: of a few distinct values for the inverse CDF, around zero, and with penalties."""
     rng = np.random.default_rng(17)
     vocab, centre = 30011, 0.0 if near_zero else 1.75
     z = (centre - 4.0 - np.abs(rng.standard_normal((8, vocab)))).astype(np.float32)
@@ -38,5 +38,6 @@ def test_lists_of_few_values_on_both_sides_of_their_line(draw, near_zero):
         z[r, at[:n]] = rng.choice([-4e-3, -1e-5, 0.0, 2e-5, 3e-3] if near_zero else [1.75, 1.7578125, 1.765625], n)
         z[r, at[n:]] = centre + rng.uniform(0.5, 4.0, 3)
     host = oracle.f32_to_bf16(z)
+    hist = rng.integers(0, vocab, (8, 600)).astype(np.int32) if penalised else None
     for top_p in (0.3, 0.7, 0.95):
-        _check(_tensor(host), host, dict(temperature=0.9, top_k=0, top_p=top_p, min_p=0.0), draw=draw)
+        _check(_tensor(host), host, dict(temperature=0.9, top_k=0, top_p=top_p, min_p=0.0), draw=draw, history=hist, rho=1.05, pi=0.01)
