@@ -5,16 +5,15 @@
 //
 // The step is latency-bound (a few MB of input and a chain of dependencies: row maximum -> row mass and accept test -> the
 // residual's total -> the token). A row's chain is its own business but for one bit, whether its draft is accepted. So every target row has a
-// thread-block CLUSTER (16 blocks for up to 14 rows, 8 beyond): its slices of the row and of the drafter's row land in shared memory by asynchronous
+// thread-block CLUSTER (16 blocks for up to 14 rows, 8 beyond, fewer where slices would be below 2048 logits or the device cannot hold them all): its slices of the row and of the drafter's row land in shared memory by asynchronous
 // copies, all in flight at once; the blocks meet in distributed shared memory, a cluster barrier to a dependency; and every row that could be the
 // decisive one -- its own draft rejected, or the bonus row -- draws its token without waiting for the rows before it. What a row found is one word in
 // the workspace; the cluster that arrives last picks the first rejected row and writes the outputs, so no block waits for another cluster.
 // A launch that is given the rows' maxima and masses knows the decisive row from one logit per draft: verify_given.cuh. Rows whose slices do not fit shared memory
 // have their maxima and masses found by clusters and go on there in a second launch, and so does the reference's draw of long rows whose clusters share SMs.
 // (All rows cut over all 148 SMs by a cooperative launch, partial results exchanged as polled words in L2, three trips for the step of 7 drafts; us a call so /
-// by clusters, first draft rejected: V = 151,936, drafter's probabilities 25.0 / 18.8, given the maxima 21.0 / 17.6, drafter's logits 27.3 / 20.5, greedy 10.3 / 7.4; 13 drafts 31.4 /
-// 22.4; 50,257 24.8 / 13.7; but the reference's draw over 248,320 with every draft rejected 29.4 / 32.3. A cooperative launch of the clusters is not made ready beside
-// its predecessor: 1.1 us more.)
+// by clusters, first draft rejected: V = 151,936, drafter's probabilities 20.9 / 14.7, given the maxima 19.8 / 13.0, drafter's logits 23.2 / 15.1, greedy 8.6 / 7.8; 15
+// drafts 27 / 22.7; 50,257 22 / 10.8; 248,320 26 / 16.6. A cooperative launch of the clusters is not made ready beside its predecessor: 1.1 us more.)
 //
 // A word carries the launch's number, which the last cluster counts up: were one missing, the wait for it is bounded, and the launch reports an error through
 // its outputs (and through the StepState when it commits); the GPU is never left waiting.
@@ -33,7 +32,9 @@ constexpr int kVerifyWarps = kVerifyThreads / 32;
 constexpr int kVerifyMaxRows = LM_MAX_DRAFT + 1;
 constexpr unsigned kVerifyWaitLimit = 1u << 17;         // polls of one word before the last cluster gives up: about 0.1 s
 constexpr int kVerifyParts = 256;                       // most blocks that share a row (verify_given.cuh)
-constexpr size_t kVerifySmem = 110 * 1024;              // most shared memory of a block (two to an SM)
+// Most shared memory of a block (two to an SM). A chunk of eight logits takes 40 bytes of it (logits, then weights, in binary32; their sum), 32 more where the
+// drafter's row lies there too: both do up to 1564 chunks a block, the target's alone up to 2816 (16 blocks: 200,200 and 360,400 logits).
+constexpr size_t kVerifySmem = 110 * 1024;
 
 struct VerifyWs {                                       // lives in the caller's workspace, zero-filled once
   unsigned long long launches;                          // so far

@@ -1,4 +1,4 @@
-"""DSpark speculative verification on the GPU: one launch checks ``n`` drafted tokens against ``n + 1`` rows of
+"""DSpark speculative verification on the GPU: one launch (two for the longest rows) checks ``n`` drafted tokens against ``n + 1`` rows of
 target logits. Stands in for the accept chain of a speculative round in the reference (greedy: the prefix match of
 ``accept_scan``, kernels/common/spec_ops.metal:162-165; sampled drafts: ``spec_q_accept`` and the residual draw,
 kernels/common/sample.metal:279-347). ``draft_q`` is the drafter's side of such a round: the draw of draft k from the
@@ -90,7 +90,7 @@ def verify(target_logits: torch.Tensor, draft_ids: Optional[torch.Tensor], draft
     there, and a finished state leaves the outputs untouched. ``out`` (int32 [rows + 2]) receives accept, final and the tokens.
     ``target_vmax`` (float32, one value per target row; stochastic mode) hands the kernel the exact row maxima the sampler already knows, as the
     reference's verify kernels get them, and spares the launch one exchange between its thread blocks; ``target_mass`` (int64, the kept sets'
-    fixed-point masses for the same thresholds and temperature: ``sample(..., return_vmax=True).mass``) spares it the second.
+    fixed-point masses for the same thresholds and temperature: ``sample(..., return_vmax=True).mass``) lets every block tell the decisive row by itself, and all of them share that row.
     ``wait_limit`` / ``selftest`` exercise the kernel's bounded waits (tests only). Asynchronous on the current stream.
     """
     if mode not in ("greedy", "stochastic"):

@@ -156,5 +156,8 @@ def test_a_subclass_of_the_stochastic_sampler_forms_its_own_knobs():
             p.top_k = 1
             return p
 
-    x = (torch.randn(4, 4096, device="cuda") * 2).to(torch.bfloat16)
+    g = torch.Generator(device="cuda").manual_seed(3)                        # (rows whose largest logit is one: a top_k of 1 keeps equal ones)
+    x = (torch.randn(4, 4096, generator=g, device="cuda") * 2).to(torch.bfloat16)
+    top = x.float().topk(2).values
+    assert bool((top[:, 0] > top[:, 1]).all())
     assert torch.equal(Annealed(temperature=2.0, seed=5).forward(x), x.float().argmax(-1))

@@ -8,23 +8,12 @@ import lithos_metal_b200 as lm
 import oracle
 from lithos_metal_b200 import _lib
 from tests.test_gpu_sampling import bf16_tensor
-from tests.test_gpu_verify_slices import check, on_gpu, step
+from tests.test_gpu_verify_slices import LAST, check, on_gpu, rejecting, step
 
 pytestmark = pytest.mark.gpu
-LAST = np.float32(1.0 - 2.0**-24)                                            # the largest uniform
 
 
-def rejecting(z, q, at, T=1.0, tau=None):
-    """Drafts and accept uniforms of which the one at `at` is the first to be rejected: likely tokens before it, from it on the one where q exceeds p by most."""
-    n = len(q)
-    drafts, ua = z[:n].argmax(-1).astype(np.int32), np.zeros(n, np.float32)
-    for r in range(at, n):
-        p = np.exp((z[r].astype(np.float64) - z[r].max()) / T) * (True if tau is None else z[r] >= tau[r])
-        drafts[r], ua[r] = np.argmax(q[r] - p / p.sum()), LAST
-    return drafts, ua
-
-
-# 16 blocks a row up to 13 drafts, 8 beyond: (50257, 7) holds both rows, (700001, 2) neither, the others the target's alone
+# 16 blocks a row up to 13 drafts, 8 beyond: (50257, 7) holds both rows, (700001, 2) neither (two launches), the others the target's alone
 @pytest.mark.parametrize("vocab,n", [(248320, 1), (248320, 7), (262144, 7), (262143, 13), (151936, 14), (151936, 15), (50257, 7), (700001, 2)])
 @pytest.mark.parametrize("dtype", ["bf16", "fp32"])
 def test_first_rejected_draft_is_replaced(vocab, n, dtype):

@@ -21,6 +21,19 @@ def step(vocab, n, dtype, seed):
     return rng, target, noisy, q
 
 
+LAST = np.float32(1.0 - 2.0**-24)                                            # the largest uniform
+
+
+def rejecting(z, q, at, T=1.0, tau=None):
+    """Drafts and accept uniforms of which the one at `at` is the first to be rejected: likely tokens before it, from it on the one where q exceeds p by most."""
+    n = len(q)
+    drafts, ua = z[:n].argmax(-1).astype(np.int32), np.zeros(n, np.float32)
+    for r in range(at, n):
+        p = np.exp((z[r].astype(np.float64) - z[r].max()) / T) * (True if tau is None else z[r] >= tau[r])
+        drafts[r], ua[r] = np.argmax(q[r] - p / p.sum()), LAST
+    return drafts, ua
+
+
 def on_gpu(target):
     return bf16_tensor(target) if target.dtype == np.uint16 else torch.from_numpy(target).cuda()
 
@@ -47,8 +60,8 @@ def check(target, drafts, q, ua, uf, gpu_q=None, **kw):
         assert int(out[0]) == acc_g and (int(out[1]) == fin_g or gap < 1e-5), more.keys()
 
 
-# one block a row, a few, sixteen; vocabularies that are no multiple of 8 (rows at every alignment); slices that do not fit shared memory (binary32 of
-# 262,144 and more); one draft, and so many that a row gets eight blocks
+# one block a row, a few, sixteen; vocabularies that are no multiple of 8 (rows at every alignment); one draft, and so many that a row gets eight blocks; slices that
+# fit shared memory without the drafter's ((151936, 15), (262144, 7), (262143, 7)) and that do not fit at all ((262144, 14), (700001, 2))
 @pytest.mark.parametrize("vocab,n,dtype", [(1, 1, "bf16"), (9, 2, "fp32"), (2049, 3, "bf16"), (4095, 15, "fp32"), (32769, 1, "bf16"), (50257, 7, "bf16"), (50257, 7, "fp32"),
                                            (151936, 15, "bf16"), (151937, 13, "fp32"), (262144, 7, "bf16"), (262143, 7, "fp32"), (262144, 14, "fp32"), (700001, 2, "bf16")])
 def test_slices_of_every_shape(vocab, n, dtype):
@@ -58,6 +71,10 @@ def test_slices_of_every_shape(vocab, n, dtype):
     random, likely = rng.integers(0, vocab, n).astype(np.int32), z[:n].argmax(-1).astype(np.int32)
     for d, u in ((random, ua), (likely, np.zeros(n, np.float32)), (np.where(np.arange(n) < n // 2, likely, random).astype(np.int32), ua)):
         check(target, d, q, u, uf)
+    for at in {0, n // 2, n - 1}:                                            # and with a rejected draft for certain
+        d, u = rejecting(z, q, at)
+        assert vocab == 1 or oracle.verify_stochastic(target, d, q, u, uf)[0] == at
+        check(target, d, q, u, uf)
     acc, fin, toks = oracle.verify_greedy(target, likely)
     out = lm.verify(on_gpu(target), torch.from_numpy(likely).cuda(), mode="greedy")
     assert (int(out[0]), int(out[1])) == (acc, fin)
@@ -65,7 +82,8 @@ def test_slices_of_every_shape(vocab, n, dtype):
     lb = oracle.f32_to_bf16(noisy)
     stats = lm.draft_q(bf16_tensor(lb), temperature=0.7, seed=3)
     q2 = np.stack([oracle.draft_probs(lb[k], temperature=0.7, vmax=float(stats.vmax[k]), mass=int(stats.mass[k])) for k in range(n)])
-    check(target, random, q2, ua, uf, gpu_q=dict(draft_logits=bf16_tensor(lb), draft_stats=stats), temperature=0.7)
+    for d, u in ((random, ua), rejecting(z, q2, n // 2, 0.7)):
+        check(target, d, q2, u, uf, gpu_q=dict(draft_logits=bf16_tensor(lb), draft_stats=stats), temperature=0.7)
 
 
 @pytest.mark.parametrize("dtype", ["bf16", "fp32"])
