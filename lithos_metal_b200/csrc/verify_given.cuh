@@ -5,7 +5,8 @@
 // bound by its chain: the drafts' logits, the row's slice, an arrival, the shares, the slice again. us a call in a CUDA graph, the decisive row on the 16 SMs of its
 // cluster / so (7 drafts but where 15 are said; the first one rejected; 148 blocks that met by polled words in a cooperative launch in brackets): 151,936 tokens 12.1 / 8.3
 // (11.9), with thresholds of top_p 0.95 19.8 / 8.5 (12.1), of top_k 50 8.9 / 7.8 (10.7), drafter's logits 12.5 / 8.3 (13.0), the reference's draw 18.0 / 9.8 (10.7), 15 drafts
-// 12.9 / 8.4 (12.2); 248,320 15.0 / 8.6 (12.2), with top_p 28.5 / 8.7 (12.4); 50,257 8.5 / 8.1 (11.0); 16,384 7.7 / 7.9 (11.0), the only sizes to lose.
+// 12.9 / 8.4 (12.2); 248,320 15.0 / 8.6 (12.2), with top_p 28.5 / 8.7 (12.4); 50,257 8.5 / 8.1 (11.0); 16,384 7.7 / 7.9 (11.0): 32,000 and less
+// are the only sizes to lose.
 #pragma once
 #include "verify.cuh"
 
